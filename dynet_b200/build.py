@@ -19,7 +19,7 @@ FLAGS = [f for f in FLAGS if f != "--use_fast_math=false"]
 
 
 def _deps_mtime():
-    hdrs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
+    hdrs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
     return max(os.path.getmtime(h) for h in hdrs)
 
 
@@ -60,7 +60,7 @@ def build_host(force=False):
     """C++ host layer above the C ABI: the node classes mirroring the reference interface and
     the LSTM language-model step driver (g++, links libdyb200.so and cudart)."""
     srcs = sorted(glob.glob(os.path.join(HOST, "*.cc")))
-    deps = srcs + glob.glob(os.path.join(HOST, "*.h")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
+    deps = srcs + glob.glob(os.path.join(HOST, "*.h")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
     if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= max(os.path.getmtime(d) for d in deps):
         return HOST_LIB
     cuda_home = os.path.dirname(os.path.dirname(NVCC))

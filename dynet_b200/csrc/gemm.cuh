@@ -155,6 +155,11 @@ struct SeqPlanes { PackedOp X, Hs; };
 bool dyb200_wgrad_seq_planes(const dyb200_wgrad* w, uint32_t steps, uint32_t step, SeqPlanes* out);
 int dyb200_wgrad_seq_h0(dyb200_wgrad* w, const float* h0, const float* mh, int mh_full, dyb200_ctx* ctx, PackJobs* batch);
 void dyb200_wgrad_seq_done(dyb200_wgrad* w);
+// For kernels that run a whole sequence of equal or ragged steps (lstm_rec.cu): the first `columns` columns as K-major right
+// operands - D = dgates (K = M), X = inputs of dyb200_wgrad_pack_inputs (K = I), Hs = h inputs (K = H); null: not asked for.
+// False when X is asked for and the inputs of that many columns are not in place.  dyb200_wgrad_h_done: all Hs rows are written.
+bool dyb200_wgrad_column_planes(const dyb200_wgrad* w, uint32_t columns, PackedOp* D, PackedOp* X, PackedOp* Hs);
+void dyb200_wgrad_h_done(dyb200_wgrad* w);
 // A 2-D tensor map (CUtensorMap, 128 bytes at `map`) over a K-major plane: box = 32 floats of K x box_rows rows, 128-byte swizzle.
 int dyb200_tc_make_tmap(dyb200_ctx* ctx, void* map, float* plane, uint32_t rows, uint32_t K, uint32_t pitch, uint32_t box_rows);
 uint32_t dyb200_tc_tile_cols(uint32_t N);   // width of the output tile the tensor path uses for N columns (64 or 128)

@@ -1317,6 +1317,17 @@ void dyb200_wgrad_seq_done(dyb200_wgrad* w) {
   w->h_col = w->x_cols - w->step;   // the planes of the last step's h input are the most recent ones
   if (w->x_cols > w->kb) w->kb = w->x_cols;
 }
+bool dyb200_wgrad_column_planes(const dyb200_wgrad* w, uint32_t columns, PackedOp* D, PackedOp* X, PackedOp* Hs) {
+  if (!w || columns > w->Kcap || (X && columns > w->x_cols) || (Hs && w->N[1] == 0)) return false;
+  if (D) { *D = w->A; D->rows = columns; D->K = w->M; D->mn_major = 0; }
+  if (X) { *X = w->B[0]; X->rows = columns; X->K = w->N[0]; X->mn_major = 0; }
+  if (Hs) { *Hs = w->B[1]; Hs->rows = columns; Hs->K = w->N[1]; Hs->mn_major = 0; }
+  return true;
+}
+void dyb200_wgrad_h_done(dyb200_wgrad* w) {
+  w->h_col = 0xffffffffu;           // (no single step's planes are the latest)
+  if (w->x_cols > w->kb) w->kb = w->x_cols;
+}
 int dyb200_tc_make_tmap(dyb200_ctx* ctx, void* map, float* plane, uint32_t rows, uint32_t K, uint32_t pitch, uint32_t box_rows) {
   EncodeTiledFn enc;
   int rc = get_encoder(ctx, &enc);

@@ -1,0 +1,46 @@
+// The recurrence of an LSTM layer of moderate width over a whole sequence (equal or shrinking batches), one launch per pass for
+// one or two directions: lstm_rec.cu.  The input product Wx x + b of all steps is formed beforehand by one GEMM, and
+// dx / dWx / dWh of all steps follow as one GEMM each, so that only Wh h_{t-1} (forward) and Wh^T dgates_t (backward) remain
+// in the chain.
+#pragma once
+#include "common.cuh"
+
+struct RecDirF {
+  const float* Wh;       // 4H x H, column-major
+  float* gates;          // 4H x columns: Wx x + b on entry, gate activations on exit
+  float *c, *h;          // H x columns
+  const float *h0, *c0;  // H x N (null: zeros)
+  const float* mask;     // dropout mask of h_{t-1} (null: none)
+  float *hn_hi, *hn_lo;  // TF32 planes of h_{t-1} .* mask, one row per column (null: not wanted)
+};
+struct RecFwd {
+  RecDirF d[2];
+  uint32_t H, U, T, N, G, ncap, hn_pitch;
+  int mask_full;
+  float fb;
+  const uint32_t* prefix;   // device, T + 1 entries: step t has the columns [prefix[t], prefix[t + 1]), widths never grow (null: N each)
+};
+struct RecDirB {
+  const float* Wh;
+  const float *gates, *c, *c0;
+  float* dh;             // H x columns: dE/dh_t from outside on entry, complete on exit
+  float* dc;             // the same for dE/dc_t (null: zero from outside, not kept)
+  const float* mask;
+  float *dn_hi, *dn_lo;  // TF32 planes of dgates, one row of 4H per column
+  float* dbpart;         // [G][4H] row sums of dgates per cluster
+};
+struct RecBwd {
+  RecDirB d[2];
+  uint32_t H, U, T, N, G, ncap, dn_pitch;
+  int mask_full;
+  const uint32_t* prefix;
+};
+
+// U hidden units per CTA, C CTAs per cluster, KD / KD2 = reduction elements per lane forward / backward.
+struct RecPlan { uint32_t U, C, KD, KD2; };
+// False when the width is outside what the registers of a cluster hold.
+bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, RecPlan* out);
+// ndir directions (1 or 2) share T, N and prefix.  U, G and ncap are filled in here.
+int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir);
+// db[dir] (4H) += row sums of dgates over all columns (partial sums in scratch memory).
+int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db);

@@ -1,0 +1,34 @@
+/* Internal interface between the kernel library and the C++ drivers (host/): the LSTM recurrence of one or two directions over
+ * ragged batches in one launch per pass, with its products over all columns formed outside.  Not part of the public C ABI.
+ *
+ * Columns are laid out step after step: step t has the columns [prefix[t], prefix[t + 1]), and the widths never grow.  The
+ * inputs of all columns must have been split into the accumulator w by dyb200_wgrad_pack_inputs (step 0 or equal steps). */
+#pragma once
+#include "../../include/dyb200.h"
+#ifdef __cplusplus
+extern "C" {
+#endif
+typedef struct {
+  const float *Wh, *h0, *c0, *mask_h;   /* h0 / c0 / mask_h may be NULL: zeros / none */
+  float *gates, *c, *h;
+  float *dh, *dc;                       /* backward only; dc may be NULL (zero from outside, not kept) */
+  float *db;
+  struct dyb200_wgrad* w;               /* may be NULL in the forward pass (no operand planes wanted) */
+} dyb200i_rec_dir;
+
+/* 1 when the kernels take a layer of H units on this device (and a sequence of T steps is long enough to be worth it). */
+int dyb200i_rec_takes(dyb200_ctx* ctx, uint32_t H, uint32_t T);
+/* gates = Wx x + b over the first `columns` columns, x = the input planes of w. */
+int dyb200i_rec_inputs(dyb200_ctx* ctx, struct dyb200_wgrad* w, const float* Wx, const float* b, uint32_t I, uint32_t H, uint32_t columns,
+                       float* gates);
+int dyb200i_rec_fwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint32_t H, uint32_t T, uint32_t N, const uint32_t* prefix_dev,
+                    int mask_full, float forget_bias);
+/* columns = all of them: marks the gate-gradient planes of w as filled. */
+int dyb200i_rec_bwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint32_t H, uint32_t T, uint32_t N, const uint32_t* prefix_dev,
+                    int mask_full, uint32_t columns);
+/* dx += Wx^T dgates (.* mask_x, which repeats every `period` columns when mask_full), dgates = the planes left in w by rec_bwd. */
+int dyb200i_rec_dx(dyb200_ctx* ctx, struct dyb200_wgrad* w, const float* Wx, uint32_t I, uint32_t H, uint32_t columns, const float* mask_x,
+                   int mask_full, uint32_t period, float* dx);
+#ifdef __cplusplus
+}
+#endif

@@ -18,6 +18,7 @@
 // Values are bit for bit those of the per-step calls: the same k-blocks in the same accumulation chains (cut every
 // kChunkKB k-blocks), the same K split (k_split) reduced in split order through distributed shared memory, the same epilogue.
 #include "seq_dev.cuh"
+#include "lstm_rec_api.h"
 
 namespace {
 
@@ -516,6 +517,24 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
     if (rc) return rc;
     dyb200_wgrad_seq_done(deferred);
     return DYB200_OK;
+  }
+
+  // ---- layers of moderate width: the input products of all steps as one GEMM, then the recurrence in clusters (lstm_rec.cu) ----
+  if (!persistent && attrs->weightnoise_std == 0.f && I > 0 && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 && Wh->d[0] == G &&
+      Wh->d[1] == H && t_size(b) == G && (deferred || !attrs->dropout) &&
+      (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H)) && dyb200i_rec_takes(ctx, H, T)) {
+    if (deferred) {
+      if ((rc = dyb200i_rec_inputs(ctx, deferred, Wx->v, b->v, I, H, T * B, gates_all->v))) return rc;
+    } else {
+      { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
+      GemmPair p{Wx->v, G, 0, x_all->v, I, 0, I, nullptr, 0, 0, 1};
+      GemmEpilogue e{EPI_BIAS, gates_all->v, G, b->v, 0, 0.f, nullptr, 0, 0};
+      if ((rc = dyb200_gemm_fused(ctx, G, T * B, 1, &p, e))) return rc;
+    }
+    dyb200i_rec_dir d;
+    memset(&d, 0, sizeof(d));
+    d.Wh = Wh->v; d.h0 = h0->v; d.c0 = c0->v; d.mask_h = mh; d.gates = gates_all->v; d.c = c_all->v; d.h = h_all->v; d.w = deferred;
+    return dyb200i_rec_fwd(ctx, 1, &d, H, T, B, nullptr, mh_full, attrs->forget_gate_bias);
   }
 
   // ---- the same sequence as one call per time step ----

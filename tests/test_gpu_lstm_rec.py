@@ -1,0 +1,100 @@
+"""The cluster-resident recurrence (csrc/lstm_rec.cu) behind the sequence calls, for layers up to 384 units and sequences of at
+least 8 steps: gates, states, every gradient and the weight gradients against the oracle's node chain.  Shapes at the edges of
+its tiling: widths that are no multiple of 4, 8 or 32, one CTA / a portable cluster / a 16-CTA cluster, one column, more columns
+than one pass of a cluster carries, batch-1 masks."""
+import numpy as np
+import pytest
+
+from util import TOL_REDUCE, assert_close, glorot, randn, rng, row_floor
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def g():
+    import gpu_util
+    gpu_util.ctx()
+    return gpu_util
+
+
+@pytest.fixture(autouse=True)
+def _release(g):
+    yield
+    g.release()
+
+
+def _oracle(oracle, x, h0, c0, Wx, Wh, b, mx, mh, up):
+    """Forward and backward over the steps, node by node: (h, c, gates) per step, (dx, dh, dc) per step, dWx, dWh, db."""
+    T, B, H = len(x), x[0].shape[0], Wh.shape[0]
+    h, c, gates = [h0], [c0], []
+    for t in range(T):
+        gates.append(oracle.lstm_gates_fwd([x[t]], h[-1], Wx, Wh, b, mask_x=mx, mask_h=mh))
+        c.append(oracle.lstm_c_fwd(c[-1], gates[t]))
+        h.append(oracle.lstm_h_fwd(c[-1], gates[t]))
+    dWx, dWh, db = np.zeros_like(Wx), np.zeros_like(Wh), np.zeros_like(b)
+    dx = [np.zeros_like(v) for v in x]
+    dh = [np.zeros((B, H), np.float32)] + [u.copy() for u in up]
+    dc = [np.zeros((B, H), np.float32) for _ in range(T + 1)]
+    for t in range(T, 0, -1):
+        dg = np.zeros((B, 4 * H), np.float32)
+        oracle.lstm_h_bwd(c[t], gates[t - 1], dh[t], 0, dc[t])
+        oracle.lstm_h_bwd(c[t], gates[t - 1], dh[t], 1, dg)
+        oracle.lstm_c_bwd(c[t - 1], gates[t - 1], dc[t], 0, dc[t - 1])
+        oracle.lstm_c_bwd(c[t - 1], gates[t - 1], dc[t], 1, dg)
+        for i, tgt in enumerate((dx[t - 1], dh[t - 1], dWx, dWh, db)):
+            oracle.lstm_gates_bwd([x[t - 1]], h[t - 1], Wx, Wh, gates[t - 1], dg, i, tgt, mask_x=mx, mask_h=mh)
+    return np.concatenate(h[1:]), np.concatenate(c[1:]), np.concatenate(gates), np.concatenate(dx), np.concatenate(dh[1:]), dWx, dWh, db
+
+
+@pytest.mark.parametrize("I,H,B,T,mask", [
+    (20, 12, 5, 8, None),            # one CTA, three column blocks of one
+    (33, 33, 3, 9, "full"),          # two CTAs, the second with one unit
+    (128, 256, 1, 12, None),         # one column
+    (128, 256, 32, 10, "full"),      # two columns per cluster
+    (100, 100, 47, 8, "one"),        # batch-1 masks, a cluster of four
+    (64, 257, 9, 8, None),           # just beyond the portable cluster
+    (200, 300, 30, 9, "full"),       # fifteen CTAs
+    (48, 384, 130, 8, None),         # the widest layer, several columns per cluster
+    (16, 64, 700, 8, "full"),        # many columns per cluster
+    (16, 384, 600, 8, "full"),       # more columns than one pass of a cluster carries
+])
+def test_recurrence_matches_oracle(oracle, g, I, H, B, T, mask):
+    import torch
+    from dynet_b200 import capi
+    r = rng(900 + H + B)
+    Wx, Wh, b = glorot(r, 4 * H, I), glorot(r, 4 * H, H), randn(r, 4 * H, scale=0.1)
+    mB = B if mask == "full" else 1
+    mx = ((r.random((mB, I)) < 0.8) / 0.8).astype(np.float32) if mask else None
+    mh = ((r.random((mB, H)) < 0.8) / 0.8).astype(np.float32) if mask else None
+    x, up = [randn(r, B, I) for _ in range(T)], [randn(r, B, H) for _ in range(T)]
+    h0, c0 = randn(r, B, H, scale=0.5), randn(r, B, H, scale=0.5)
+    want = _oracle(oracle, x, h0, c0, Wx, Wh, b, mx, mh, up)
+    ctx = g.ctx()
+    at = capi.LstmGatesAttrs(1 if mask else 0, 0.0, 1.0)
+    D = {k: g.dev(v) for k, v in dict(Wx=Wx, Wh=Wh, b=b, x=np.concatenate(x), h0=h0, c0=c0, dh=np.concatenate(up)).items()}
+    tmx, tmh = (g.T(g.dev(mx)), g.T(g.dev(mh))) if mask else (None, None)
+    tWx, tWh, tb = g.T(D["Wx"], [4 * H, I], 1), g.T(D["Wh"], [4 * H, H], 1), g.T(D["b"], [4 * H], 1)
+    gates, cs, hs = (torch.full((T * B, n), 7.0, device="cuda") for n in (4 * H, H, H))
+    dc, dx, db = torch.zeros(T * B, H, device="cuda"), torch.zeros(T * B, I, device="cuda"), torch.zeros(4 * H, device="cuda")
+    dWx, dWh = torch.zeros(I, 4 * H, device="cuda"), torch.zeros(H, 4 * H, device="cuda")
+    w = ctx.wgrad_create(4 * H, I, H, T * B)
+    try:
+        l0 = ctx.launches()
+        ctx.lstm_seq_fwd(g.T(D["x"], [I], T * B), g.T(D["h0"]), g.T(D["c0"]), tWx, tWh, tb, tmx, tmh, at, g.T(gates, [4 * H], T * B),
+                         g.T(cs, [H], T * B), g.T(hs, [H], T * B), w, T)
+        ctx.lstm_seq_bwd(g.T(D["x"], [I], T * B), g.T(D["h0"]), g.T(D["c0"]), tWx, tWh, tmx, tmh, at, g.T(gates, [4 * H], T * B),
+                         g.T(cs, [H], T * B), g.T(hs, [H], T * B), g.T(D["dh"], [H], T * B), g.T(dc, [H], T * B), g.T(dx, [I], T * B),
+                         None, None, g.T(db, [4 * H], 1), w, T)
+        assert ctx.launches() - l0 < 14, "the per-step calls ran"
+        ctx.wgrad_flush(w, dWx.data_ptr(), 4 * H, dWh.data_ptr(), 4 * H)
+        torch.cuda.synchronize()
+    finally:
+        ctx.wgrad_destroy(w)
+    assert ctx.device_errors() == 0
+    for name, got, ref in zip(("h", "c", "gates"), (hs, cs, gates), want[:3]):
+        assert_close(g.host(got), ref, TOL_REDUCE, floor=0.1, what=name)
+    for name, got, ref in zip(("dx", "dh"), (dx, D["dh"]), want[3:5]):
+        assert_close(g.host(got), ref, TOL_REDUCE, floor=row_floor(ref, 1, rel=1e-2), what=name + " (per-column scale)")
+    for name, got, ref in zip(("dWx", "dWh"), (dWx, dWh), want[5:7]):
+        assert_close(g.host(got), ref, TOL_REDUCE, floor=row_floor(ref, 0, rel=1e-2), what=name + " (per-row scale)")
+    assert_close(g.host(db), want[7], TOL_REDUCE, floor=float(np.abs(want[7]).max()) * 0.02, what="db")
