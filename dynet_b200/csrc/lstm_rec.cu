@@ -9,16 +9,24 @@
 //   * Wh is held on chip for the whole sequence: CTA r of the cluster keeps the 4 gate rows of its U hidden units (forward)
 //     / the same rows as the reduction index of Wh^T (backward) in REGISTERS, up to 192 floats per thread; Wh is read once
 //     per launch and cluster instead of once per step.
-//   * h_t (forward) goes to every CTA of the cluster through distributed shared memory, double-buffered, with one hardware
-//     cluster barrier per step (no polling, no global-memory hand-over); backward, each CTA reduces over its own gate rows
-//     and sends partial sums of dE/dh_{t-1} to the CTA that owns the unit, 4 x fewer bytes than handing dgates around.
-//   * plain fp32 multiply-adds (two per instruction, fma.rn.f32x2): more accurate than the 3xTF32 products of the per-step
-//     form, and at 1 - 8 columns per cluster the tensor pipe could not be filled anyway.
+//   * h_t (forward) goes to every CTA of the cluster through distributed shared memory as 16-byte messages that complete an
+//     mbarrier of the receiver (st.async): no fence, no polling of global memory, two buffers.  A barrier of the whole cluster
+//     per step instead took 1.9 us per step at 2 - 4 columns, most of it the release of the step's global stores.  Backward,
+//     each CTA reduces over its own gate rows and sends partial sums of dE/dh_{t-1} to the CTA that owns the unit, 4 x fewer
+//     bytes than handing dgates around.
+//   * plain fp32 multiply-adds: more accurate than the 3xTF32 products of the per-step form, and at 1 - 8 columns per cluster
+//     the tensor pipe could not be filled anyway.  (Not fma.rn.f32x2: with two 64-bit register operands and a 64-bit
+//     accumulator it issued once in four cycles here, half the rate of the scalar form.)
 // The arithmetic order is fixed by the shape (cluster count, ranks, lanes): reproducible run to run.
 //
-// Thread layout, forward: 8 lanes per hidden unit (slice s of the reduction index: k = 32 j + 4 s + 0..3, so the 8 slices of
-// a unit read 128 contiguous bytes of h: no bank conflicts, the 4 units of a warp broadcast), 4 gates x KD k per lane.
-// NB columns at a time; a butterfly over the 8 lanes leaves each lane with all four gates of one column.
+// Every warp sends its own part as soon as it has it (no barrier of the CTA).  Buffers are free to be overwritten without a
+// further hand-shake: a warp sends h_t only after the h_{t-1} of every warp of the cluster has arrived, and each of those was
+// sent after that warp had read the buffer that h_t goes to.
+//
+// Thread layout, forward: 16 lanes per pair of hidden units (slice s of the reduction index: k = 64 j + 4 s + 0..3, so the
+// slices read 256 contiguous bytes of h without bank conflicts), 8 gate rows x KD k per lane - with one unit per 8 lanes the
+// loads of h took as many cycles as the multiply-adds.  NB columns at a time; a butterfly over the 16 lanes leaves each lane
+// with all four gates of one unit and column.
 // Backward: 8 lanes per group of 8 units of dE/dh_{t-1}, slices of the CTA's own 4 U gate rows in the same pattern.
 #include "lstm_rec.cuh"
 
@@ -28,18 +36,6 @@
 
 namespace {
 
-typedef unsigned long long u64;
-__device__ __forceinline__ u64 pack2(float a, float b) {
-  u64 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float sum2(u64 v) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return a + b;
-}
-__device__ __forceinline__ void fma2(u64& acc, u64 a, u64 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -51,104 +47,234 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ float xor_add(float keep, float send, int m) { return keep + __shfl_xor_sync(0xffffffffu, send, m); }
 
-// columns of this cluster that are active at a step of width B: those i < ncol with g + G (i0 + i) < B
-__device__ __forceinline__ uint32_t active_cols(uint32_t B, uint32_t g, uint32_t G, uint32_t i0, uint32_t ncol) {
-  if (B <= g) return 0;
-  const uint32_t n = (B - g + G - 1) / G;
-  return n > i0 ? min(n - i0, ncol) : 0;
+// columns of cluster g that are active at a step of width B: those i with g + G i < B
+__device__ __forceinline__ uint32_t active_cols(uint32_t B, uint32_t g, uint32_t G) { return B > g ? (B - g + G - 1) / G : 0; }
+
+// One mbarrier per buffer parity: `bytes` of st.async messages complete its phase.
+__device__ __forceinline__ void msg_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void msg_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool msg_wait(uint64_t* bar, uint32_t parity) {   // bounded
+  for (uint32_t it = 0; it < (1u << 20); ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+// 16 bytes into a CTA's shared memory, counted by its mbarrier (both addresses shared::cluster)
+__device__ __forceinline__ void send4(uint32_t addr, float4 v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(v.x), "f"(v.y),
+               "f"(v.z), "f"(v.w), "r"(bar) : "memory");
 }
 
-// grid (C, G, directions), cluster (C, 1, 1); block = 8 U threads.  Dynamic shared memory: h[2][ncap][8 KD], c[ncap][U].
-template <int KD, int NB>
+// grid (C, G, directions), cluster (C, 1, 1); block = 8 U threads.
+// Dynamic shared memory: h[2][ncap][16 KD], c[ncap][U].  NB columns per block, NF of them computed (3 of 4, or all).
+template <int KD, int NB, int NF = NB>
 __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__ RecFwd a) {
-  constexpr int HP = 8 * KD;
+  constexpr int HP = 16 * KD;
   extern __shared__ __align__(16) float rec_smem[];
+  __shared__ __align__(8) uint64_t got[2];
+  __shared__ __align__(16) float stage_all[8][NB * 4];
   const RecDirF d = blockIdx.z ? a.d[1] : a.d[0];
-  const uint32_t H = a.H, U = a.U, G = a.G, g = blockIdx.y, rank = blockIdx.x, C = gridDim.x;
-  const uint32_t tid = threadIdx.x, s = tid & 7, ul = tid >> 3, u = rank * U + ul;
+  const uint32_t H = a.H, U = a.U, G = a.G, g = blockIdx.y, rank = blockIdx.x, C = gridDim.x, ncap = a.ncap;
+  const uint32_t tid = threadIdx.x, s = tid & 15, ul0 = 2 * (tid >> 4);   // slice, first of the lane's two units
+  const uint32_t ul = ul0 + (s >> 3), u = rank * U + ul;                  // the unit this lane finishes
   const bool live_u = u < H;
   float* hbuf = rec_smem;
-  float* cbuf = rec_smem + (size_t)2 * a.ncap * HP;
+  float* cbuf = hbuf + (size_t)2 * ncap * HP;
+  float* stage = stage_all[tid >> 5];                                     // h of this warp's 4 units, column by column
+  const uint32_t lane = tid & 31, u_warp = rank * U + 4 * (tid >> 5);
+  if (tid == 0) {
+    msg_init(&got[0]);
+    msg_init(&got[1]);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   dyb_grid_dep_sync();
 
-  u64 w[4][KD / 2];
-#pragma unroll
-  for (int j = 0; j < KD / 4; ++j)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float v[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t k = 32 * j + 4 * s + i;
-        v[i] = (live_u && k < H) ? __ldg(d.Wh + (size_t)q * H + u + (size_t)4 * H * k) : 0.f;
-      }
-      w[q][2 * j] = pack2(v[0], v[1]);
-      w[q][2 * j + 1] = pack2(v[2], v[3]);
-    }
-
   // the column of a block that this lane finishes; 8 / NB lanes share one (they hold equal values; dup == 0 stores)
-  const uint32_t lc = NB == 8 ? s : NB == 4 ? s >> 1 : NB == 2 ? s >> 2 : 0;
-  const uint32_t dup = NB == 8 ? 0 : NB == 4 ? (s & 1) : NB == 2 ? (s & 3) : s;
-  constexpr uint32_t DUPS = 8 / NB;
-  const uint32_t nloc = a.N > g ? (a.N - g + G - 1) / G : 0;
+  const uint32_t lc = NB == 8 ? (s & 7) : NB == 4 ? (s & 7) >> 1 : NB == 2 ? (s & 7) >> 2 : 0;
+  const uint32_t dup = NB == 8 ? 0 : NB == 4 ? (s & 1) : NB == 2 ? (s & 3) : (s & 7);
+  const uint32_t ncol = active_cols(a.N, g, G);
+  uint32_t phase[2] = {0, 0};
+  bool ok = true;
+  uint32_t col0 = 0, B = a.prefix ? a.prefix[1] : a.N;      // first column and width of the step
+  uint32_t n = active_cols(B, g, G);
+  float pre[4], mk;
+  auto fetch = [&](uint32_t c0, uint32_t nact, uint32_t nb) {   // Wx x + b and the mask of this lane's column of a block
+    const uint32_t i = nb + lc, sc = g + G * i;
+    if (live_u && i < nact) {
+      const float* p = d.gates + u + (size_t)4 * H * (c0 + sc);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) pre[q] = p[(size_t)q * H];
+      mk = d.mask ? d.mask[u + (a.mask_full ? (size_t)H * sc : 0)] : 1.f;
+    } else {
+      pre[0] = pre[1] = pre[2] = pre[3] = mk = 0.f;
+    }
+  };
+  fetch(col0, n, 0);
 
-  for (uint32_t i0 = 0; i0 < nloc; i0 += a.ncap) {
-    const uint32_t ncol = min(a.ncap, nloc - i0);
-    // h_{-1} of this chunk's columns; zeros in the padding (both buffers)
-    for (uint32_t e = tid; e < a.ncap * HP; e += blockDim.x) {
-      const uint32_t i = e / HP, k = e % HP, sc = g + G * (i0 + i);
-      float v = 0.f;
-      if (d.h0 && i < ncol && k < H) {
-        v = d.h0[k + (size_t)H * sc];
-        if (d.mask) v *= d.mask[k + (a.mask_full ? (size_t)H * sc : 0)];
-      }
-      hbuf[e] = v;
-      hbuf[(size_t)a.ncap * HP + e] = 0.f;
-    }
-    for (uint32_t e = tid; e < ncol * U; e += blockDim.x) {
-      const uint32_t i = e / U, uu = rank * U + e % U, sc = g + G * (i0 + i);
-      cbuf[e] = (d.c0 && uu < H) ? d.c0[uu + (size_t)H * sc] : 0.f;
-    }
-    __syncthreads();
-    if (d.hn_hi)   // the planes of the first step's h input
-      for (uint32_t e = tid; e < ncol * U; e += blockDim.x) {
-        const uint32_t i = e / U, uu = rank * U + e % U, sc = g + G * (i0 + i);
-        if (uu < H) {
-          float hi, lo;
-          split_tf32(hbuf[(size_t)i * HP + uu], hi, lo);
-          d.hn_hi[(size_t)sc * a.hn_pitch + uu] = hi;
-          d.hn_lo[(size_t)sc * a.hn_pitch + uu] = lo;
+  // The CTA's rows of Wh come in as they lie in memory (16 bytes of U neighbouring units of one gate and column per lane), pass
+  // through shared memory and stay in registers.  For 128 KB: 3 000 cycles; 4-byte loads took 4 500 - 7 000 (twice that when
+  // they miss L2), 128-byte bulk copies 7 500.  Row k is shifted by the slice that reads it, so that the 16 slices meet 16
+  // pairs of banks.
+  const uint32_t WP = 4 * U + 32;
+  {
+    const bool vec = (H & 3) == 0 && aligned16(d.Wh);
+    const uint32_t nq = U / 4, total = 64 * KD * nq;
+    for (uint32_t e0 = tid; e0 < total; e0 += 8 * blockDim.x) {
+      float4 v[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const uint32_t e = e0 + x * blockDim.x, seg = e / nq, k = seg / 4, q = seg % 4, uu = rank * U + 4 * (e % nq);
+        const float* p = d.Wh + (size_t)q * H + uu + (size_t)4 * H * k;
+        v[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k < H && uu < H) {
+          if (vec) v[x] = __ldg(reinterpret_cast<const float4*>(p));
+          else {
+            v[x].x = __ldg(p);
+            if (uu + 1 < H) v[x].y = __ldg(p + 1);
+            if (uu + 2 < H) v[x].z = __ldg(p + 2);
+            if (uu + 3 < H) v[x].w = __ldg(p + 3);
+          }
         }
       }
-    cluster_arrive();
-    cluster_wait();
-
-    uint32_t col0 = 0, B = a.prefix ? a.prefix[1] : a.N;      // first column and width of the step
-    uint32_t n = active_cols(B, g, G, i0, ncol);
-    float pre[4], mk;
-    auto fetch = [&](uint32_t c0, uint32_t nact, uint32_t nb) {   // Wx x + b and the mask of this lane's column of a block
-      const uint32_t i = nb + lc, sc = g + G * (i0 + i);
-      if (live_u && i < nact) {
-        const float* p = d.gates + u + (size_t)4 * H * (c0 + sc);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pre[q] = p[(size_t)q * H];
-        mk = d.mask ? d.mask[u + (a.mask_full ? (size_t)H * sc : 0)] : 1.f;
-      } else {
-        pre[0] = pre[1] = pre[2] = pre[3] = mk = 0.f;
+      for (int x = 0; x < 8; ++x) {
+        const uint32_t e = e0 + x * blockDim.x, seg = e / nq, k = seg / 4, q = seg % 4;
+        if (e < total) {
+          float2* dst = reinterpret_cast<float2*>(rec_smem + (size_t)k * WP + 2 * (k / 4 % 16) + q * U + 4 * (e % nq));
+          dst[0] = make_float2(v[x].x, v[x].y);
+          dst[1] = make_float2(v[x].z, v[x].w);
+        }
       }
-    };
-    fetch(col0, n, 0);
-    for (uint32_t t = 0; t < a.T && n > 0; ++t) {
-      const float* hcur = hbuf + (size_t)(t & 1) * a.ncap * HP;
-      const uint32_t hnext = smem_addr(hbuf + (size_t)((t + 1) & 1) * a.ncap * HP);
-      const uint32_t col1 = col0 + B;                                          // the next step
-      const uint32_t B1 = t + 1 < a.T ? (a.prefix ? a.prefix[t + 2] - a.prefix[t + 1] : a.N) : 0;
-      const uint32_t n1 = active_cols(B1, g, G, i0, ncol);
-      float z[4], cn = 0.f, hv = 0.f, hm = 0.f;
-      uint32_t sc = 0;
-      bool mine = false;
-      auto store = [&]() {   // gates, c, h and the operand planes of the block just finished
-        if (!mine || dup) return;
+    }
+  }
+  __syncthreads();
+  float w[8][KD];   // row 4 (unit of the pair) + gate
+#pragma unroll
+  for (int x = 0; x < KD; ++x)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 v = *reinterpret_cast<const float2*>(rec_smem + (size_t)(64 * (x / 4) + 4 * s + x % 4) * WP + 2 * s + q * U + ul0);
+      w[q][x] = v.x;
+      w[4 + q][x] = v.y;
+    }
+  __syncthreads();
+
+  // h_{-1} and c_{-1} of the cluster's columns, the operand planes of the first step's h input; zeros in the padding of h
+  for (uint32_t e = tid; e < 2 * ncap * HP / 4; e += blockDim.x) reinterpret_cast<float4*>(hbuf)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+#pragma unroll 2
+  for (uint32_t e = tid; e < ncol * H; e += blockDim.x) {
+    const uint32_t i = e / H, k = e % H, sc = g + G * i;
+    const bool own = k / U == rank;
+    float v = d.h0 ? __ldg(d.h0 + k + (size_t)H * sc) : 0.f;
+    const float m = d.mask ? __ldg(d.mask + k + (a.mask_full ? (size_t)H * sc : 0)) : 1.f, c = own && d.c0 ? __ldg(d.c0 + k + (size_t)H * sc) : 0.f;
+    v *= m;
+    hbuf[(size_t)i * HP + k] = v;
+    if (own) {
+      cbuf[i * U + k % U] = c;
+      if (d.hn_hi) {
+        float hi, lo;
+        split_tf32(v, hi, lo);
+        d.hn_hi[(size_t)sc * a.hn_pitch + k] = hi;
+        d.hn_lo[(size_t)sc * a.hn_pitch + k] = lo;
+      }
+    }
+  }
+  cluster_arrive();
+  cluster_wait();
+
+  for (uint32_t t = 0; t < a.T && n > 0; ++t) {
+    const uint32_t pt = t & 1, pn = pt ^ 1;
+    const float* hcur = hbuf + (size_t)pt * ncap * HP;
+    const uint32_t hnext = smem_addr(hbuf + (size_t)pn * ncap * HP);
+    const uint32_t col1 = col0 + B;                                          // the next step
+    const uint32_t B1 = t + 1 < a.T ? (a.prefix ? a.prefix[t + 2] - a.prefix[t + 1] : a.N) : 0;
+    const uint32_t n1 = active_cols(B1, g, G);
+    if (n1 && tid == 0) msg_expect(&got[pn], n1 * C * U * 4);   // (only the columns that go on are handed over)
+    if (t > 0) {
+      ok = ok && msg_wait(&got[pt], phase[pt]);
+      phase[pt] ^= 1;
+    }
+#pragma unroll 1
+    for (uint32_t nb = 0; nb < n; nb += NB) {
+      float acc[8][NB];   // (columns NF .. NB - 1 stay zero)
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int c = 0; c < NB; ++c) acc[r][c] = 0.f;
+      const float* hp = hcur + (size_t)nb * HP + 4 * s;
+#pragma unroll
+      for (int j = 0; j < KD / 4; ++j)
+#pragma unroll
+        for (int c = 0; c < NF; ++c) {
+          const float4 hh = ld4(hp + (size_t)c * HP + 64 * j);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) acc[r][c] = fmaf(w[r][4 * j], hh.x, acc[r][c]);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) acc[r][c] = fmaf(w[r][4 * j + 1], hh.y, acc[r][c]);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) acc[r][c] = fmaf(w[r][4 * j + 2], hh.z, acc[r][c]);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) acc[r][c] = fmaf(w[r][4 * j + 3], hh.w, acc[r][c]);
+        }
+      // sum over the 16 slices: first the units, then the columns are split between the lanes; what is left is added on both
+      float z[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float v[NB];
+        const bool hi_unit = (s & 8) != 0;
+#pragma unroll
+        for (int c = 0; c < NB; ++c) {
+          const float v0 = acc[q][c], v1 = acc[4 + q][c];
+          v[c] = xor_add(hi_unit ? v1 : v0, hi_unit ? v0 : v1, 8);
+        }
+#pragma unroll
+        for (int m = 4; m >= 1; m >>= 1) {
+          const int half = NB * m / 8;            // columns each side keeps (0: one is left, added on both sides)
+          const bool up = (s & m) != 0;
+          if (half >= 1) {
+#pragma unroll
+            for (int c = 0; c < NB / 2; ++c)
+              if (c < half) v[c] = xor_add(up ? v[c + half] : v[c], up ? v[c] : v[c + half], m);
+          } else {
+            v[0] = xor_add(v[0], v[0], m);
+          }
+        }
+        z[q] = v[0];
+      }
+      const uint32_t i = nb + lc, sc = g + G * i;
+      const bool mine = live_u && i < n;
+      float cn = 0.f, hv = 0.f, hm = 0.f;
+      if (mine) {
+        z[0] = gate_sigmoid(z[0] + pre[0]);
+        z[1] = gate_sigmoid(z[1] + pre[1] + a.fb);
+        z[2] = gate_sigmoid(z[2] + pre[2]);
+        z[3] = gate_tanh(z[3] + pre[3]);
+        cn = lstm_cell_c(z[0], z[3], z[1], cbuf[i * U + ul]);
+        hv = lstm_cell_h(z[2], cn);
+        hm = hv * mk;
+      }
+      if (dup == 0) stage[lc * 4 + (ul & 3)] = hm;
+      __syncwarp();             // (also: all lanes of the unit have read the old cell state)
+      if (n1 > nb) {
+        // the warp hands its 4 units of the block over: one 16-byte message per column and CTA
+        const uint32_t n_send = min(n1 - nb, (uint32_t)NB);
+        for (uint32_t e = lane; e < NB * C; e += 32) {
+          const uint32_t c = e % NB, r = e / NB;
+          if (c < n_send)
+            send4(map_rank(hnext + 4u * ((nb + c) * HP + u_warp), r), *reinterpret_cast<const float4*>(stage + 4 * c), map_rank(smem_addr(&got[pn]), r));
+        }
+      }
+      if (mine && dup == 0) {   // gates, c, h and the operand planes of the next step's input
+        cbuf[i * U + ul] = cn;
         float* p = d.gates + u + (size_t)4 * H * (col0 + sc);
 #pragma unroll
         for (int q = 0; q < 4; ++q) p[(size_t)q * H] = z[q];
@@ -160,221 +286,193 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
           d.hn_hi[(size_t)(col1 + sc) * a.hn_pitch + u] = hi;
           d.hn_lo[(size_t)(col1 + sc) * a.hn_pitch + u] = lo;
         }
-      };
-#pragma unroll 1
-      for (uint32_t nb = 0; nb < n; nb += NB) {
-        u64 acc[4][NB];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int c = 0; c < NB; ++c) acc[q][c] = 0ull;
-        const float* hp = hcur + (size_t)nb * HP + 4 * s;
-#pragma unroll
-        for (int j = 0; j < KD / 4; ++j)
-#pragma unroll
-          for (int c = 0; c < NB; ++c) {
-            const ulonglong2 hh = *reinterpret_cast<const ulonglong2*>(hp + (size_t)c * HP + 32 * j);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) { fma2(acc[q][c], w[q][2 * j], hh.x); fma2(acc[q][c], w[q][2 * j + 1], hh.y); }
-          }
-        // sum over the 8 slices: columns are split between the lanes as long as there are several, then added on both sides
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float v[NB];
-#pragma unroll
-          for (int c = 0; c < NB; ++c) v[c] = sum2(acc[q][c]);
-#pragma unroll
-          for (int m = 4; m >= 1; m >>= 1) {
-            const int half = NB * m / 8;            // columns each side keeps (0: one is left, added on both sides)
-            const bool up = (s & m) != 0;
-            if (half >= 1) {
-#pragma unroll
-              for (int c = 0; c < NB / 2; ++c)
-                if (c < half) v[c] = xor_add(up ? v[c + half] : v[c], up ? v[c] : v[c + half], m);
-            } else {
-              v[0] = xor_add(v[0], v[0], m);
-            }
-          }
-          z[q] = v[0];
-        }
-        const uint32_t i = nb + lc;
-        mine = live_u && i < n;
-        if (mine) {
-          sc = g + G * (i0 + i);
-          z[0] = gate_sigmoid(z[0] + pre[0]);
-          z[1] = gate_sigmoid(z[1] + pre[1] + a.fb);
-          z[2] = gate_sigmoid(z[2] + pre[2]);
-          z[3] = gate_tanh(z[3] + pre[3]);
-          cn = lstm_cell_c(z[0], z[3], z[1], cbuf[i * U + ul]);
-          hv = lstm_cell_h(z[2], cn);
-          hm = hv * mk;
-        }
-        __syncwarp();   // (all lanes of the unit have read the old cell state)
-        if (mine) {
-          if (!dup) cbuf[i * U + ul] = cn;
-          const uint32_t off = hnext + 4u * (i * HP + u);
-          for (uint32_t r = dup; r < C; r += DUPS) st_cluster(map_rank(off, r), hm);
-        }
-        if (nb + NB < n) {
-          store();
-          fetch(col0, n, nb + NB);
-        }
       }
-      cluster_arrive();
-      store();                       // (the last block's results go out while the cluster meets)
-      if (n1) fetch(col1, n1, 0);
-      cluster_wait();
-      col0 = col1; B = B1; n = n1;
+      if (nb + NB < n) fetch(col0, n, nb + NB);
+      else if (n1) fetch(col1, n1, 0);
+      __syncwarp();             // (the unit's other lanes read the new cell state in the next step)
     }
-    cluster_arrive();                // nobody overwrites a neighbour's buffers before it is through with this chunk
-    cluster_wait();
+    col0 = col1; B = B1; n = n1;
   }
+  cluster_arrive();                // nobody leaves while a neighbour may still send to it
+  cluster_wait();
+  if (!ok) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
 }
 
-// grid (C, G, directions), cluster (C, 1, 1); block = 8 ceil(H / 8) threads rounded up to warps.
-// Dynamic shared memory: part[2][C][ncap][U], dg[ncap][8 KD], dcs[ncap][U].  KD = gate rows per slice: 8 KD >= 4 U.
-template <int KD, int NB>
+// grid (C, G, directions), cluster (C, 1, 1); block = C U threads rounded up to warps.  KD = gate rows per slice: 8 KD >= 4 U.
+// Dynamic shared memory: part[2][C][ncap][U], dg[ncap][8 KD], dcs[ncap][U].
+template <int KD, int NB, int NF = NB>
 __global__ void __launch_bounds__(KD == 16 ? 256 : 384, 1) k_lstm_rec_bwd(const __grid_constant__ RecBwd a) {
   constexpr int KP = 8 * KD;
   extern __shared__ __align__(16) float rec_smem[];
+  __shared__ __align__(8) uint64_t got[2];
+  __shared__ __align__(16) float stage_all[12][NB * 32];
   const RecDirB d = blockIdx.z ? a.d[1] : a.d[0];
   const uint32_t H = a.H, U = a.U, G = a.G, g = blockIdx.y, rank = blockIdx.x, C = gridDim.x, ncap = a.ncap;
   const uint32_t tid = threadIdx.x, s = tid & 7, og = tid >> 3;
   float* part = rec_smem;                                   // [parity][source rank][column][unit]
   float* dg = part + (size_t)2 * C * ncap * U;
   float* dcs = dg + (size_t)ncap * KP;
+  float* stage = stage_all[tid >> 5];                       // partial sums of this warp's 32 units, column by column
+  // message of this lane: 4 units of column lane / 8 of a block, for the CTA that owns them
+  const uint32_t lane = tid & 31, o_msg = 32 * (tid >> 5) + 4 * (lane & 7), r_msg = o_msg / U;
+  const bool msg_live = o_msg < C * U;
+  if (tid == 0) {
+    msg_init(&got[0]);
+    msg_init(&got[1]);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   dyb_grid_dep_sync();
 
   // weights: outputs o = 8 og + 0..7 (units of h_{t-1}) x this CTA's gate rows kk = q U + unit, slice s
-  u64 w[8][KD / 2];
+  float w[8][KD];
+  const bool quads = (H & 3) == 0 && aligned16(d.Wh);
 #pragma unroll
   for (int o = 0; o < 8; ++o)
 #pragma unroll
     for (int j = 0; j < KD / 4; ++j) {
-      float v[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t kk = 32 * j + 4 * s + i, q = kk / U, uu = rank * U + kk % U, oo = 8 * og + o;
-        v[i] = (q < 4 && uu < H && oo < H) ? __ldg(d.Wh + (size_t)q * H + uu + (size_t)4 * H * oo) : 0.f;
+      // (U is a multiple of 4: the four rows are one gate's rows of four neighbouring units)
+      const uint32_t kk = 32 * j + 4 * s, q = kk / U, uu = rank * U + kk % U, oo = 8 * og + o;
+      const float* p = d.Wh + (size_t)q * H + uu + (size_t)4 * H * oo;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (q < 4 && uu < H && oo < H) {
+        if (quads) v = __ldg(reinterpret_cast<const float4*>(p));
+        else {
+          v.x = __ldg(p);
+          if (uu + 1 < H) v.y = __ldg(p + 1);
+          if (uu + 2 < H) v.z = __ldg(p + 2);
+          if (uu + 3 < H) v.w = __ldg(p + 3);
+        }
       }
-      w[o][2 * j] = pack2(v[0], v[1]);
-      w[o][2 * j + 1] = pack2(v[2], v[3]);
+      w[o][4 * j] = v.x; w[o][4 * j + 1] = v.y; w[o][4 * j + 2] = v.z; w[o][4 * j + 3] = v.w;
     }
-  // after the butterfly this lane holds unit o_mine of dE/dh_{t-1}; it belongs to CTA o_mine / U
-  const uint32_t o_mine = 8 * og + s, o_rank = o_mine / U, o_ul = o_mine % U;
-  const bool o_live = o_mine < H;
-  const uint32_t o_base = map_rank(smem_addr(part), o_live ? o_rank : rank) + 4u * (rank * ncap * U + o_ul);
   // cell pass: thread -> (unit c_ul, columns c_i0, c_i0 + c_step, ...)
   const uint32_t c_step = blockDim.x / U, c_ul = tid % U, c_i0 = tid / U, c_u = rank * U + c_ul;
   const bool c_live = c_i0 < c_step && c_u < H;
   float db[4] = {0.f, 0.f, 0.f, 0.f};
-  const uint32_t nloc = a.N > g ? (a.N - g + G - 1) / G : 0;
+  uint32_t phase[2] = {0, 0};
+  bool ok = true;
 
-  for (uint32_t i0 = 0; i0 < nloc; i0 += ncap) {
-    const uint32_t ncol = min(ncap, nloc - i0);
-    for (uint32_t e = tid; e < ncap * KP; e += blockDim.x) dg[e] = 0.f;
-    for (uint32_t e = tid; e < ncap * U; e += blockDim.x) dcs[e] = 0.f;
-    cluster_arrive();
-    cluster_wait();
-    // the last step that has a column of this chunk: widths never grow, so the steps before it have one too
-    uint32_t T = a.T;
-    while (a.prefix && T > 0 && active_cols(a.prefix[T] - a.prefix[T - 1], g, G, i0, ncol) == 0) --T;
+  for (uint32_t e = tid; e < ncap * KP; e += blockDim.x) dg[e] = 0.f;
+  for (uint32_t e = tid; e < ncap * U; e += blockDim.x) dcs[e] = 0.f;
+  cluster_arrive();
+  cluster_wait();
+  // the last step that has a column of this cluster: widths never grow, so the steps before it have one too
+  uint32_t T = a.T;
+  while (a.prefix && T > 0 && active_cols(a.prefix[T] - a.prefix[T - 1], g, G) == 0) --T;
 
-    // saved values of the first (column, unit) item of the cell pass of a step, requested one step ahead
-    float gt[4], cv, cp, dhv, dcv;
-    auto fetch = [&](uint32_t t, uint32_t col, uint32_t colm1, uint32_t sc) {
-      const float* p = d.gates + c_u + (size_t)4 * H * (col + sc);
+  // saved values of the first (column, unit) item of the cell pass of a step, requested one step ahead
+  float gt[4], cv, cp, dhv, dcv;
+  auto fetch = [&](uint32_t t, uint32_t col, uint32_t colm1, uint32_t sc) {
+    const float* p = d.gates + c_u + (size_t)4 * H * (col + sc);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) gt[q] = p[(size_t)q * H];
-      cv = d.c[c_u + (size_t)H * (col + sc)];
-      cp = t ? d.c[c_u + (size_t)H * (colm1 + sc)] : (d.c0 ? d.c0[c_u + (size_t)H * sc] : 0.f);
-      dhv = d.dh[c_u + (size_t)H * (col + sc)];
-      dcv = d.dc ? d.dc[c_u + (size_t)H * (col + sc)] : 0.f;
-    };
-    auto start_of = [&](uint32_t t) { return a.prefix ? a.prefix[t] : t * a.N; };
-    uint32_t n_later = 0;            // columns that were active at step t + 1
-    uint32_t col = T ? start_of(T - 1) : 0;
-    uint32_t n = T ? active_cols(start_of(T) - col, g, G, i0, ncol) : 0;
-    if (T && c_live && c_i0 < n) fetch(T - 1, col, T > 1 ? start_of(T - 2) : 0, g + G * (i0 + c_i0));
-    for (uint32_t t = T; t-- > 0;) {
-      const uint32_t colm1 = t ? start_of(t - 1) : 0;
-      const float* pin = part + (size_t)((t + 1) & 1) * C * ncap * U;
-      // ---- gradients of the gate pre-activations of this CTA's units ----
-      if (c_live)
-        for (uint32_t i = c_i0; i < n; i += c_step) {
-          const uint32_t sc = g + G * (i0 + i);
-          if (i != c_i0) fetch(t, col, colm1, sc);
-          float dh = dhv;
-          if (i < n_later) {
-            float r = 0.f;
-            for (uint32_t q = 0; q < C; ++q) r += pin[((size_t)q * ncap + i) * U + c_ul];
-            if (d.mask) r *= d.mask[c_u + (a.mask_full ? (size_t)H * sc : 0)];
-            dh += r;
-            d.dh[c_u + (size_t)H * (col + sc)] = dh;
-          }
-          float dcp = 0.f, pr[4];
-          const float dci = dcv + dcs[i * U + c_ul];
-          if (d.dc && i < n_later) d.dc[c_u + (size_t)H * (col + sc)] = dci;
-          lstm_cell_grad(gt[0], gt[1], gt[2], gt[3], cv, cp, dh, dci, true, dcp, pr[0], pr[1], pr[2], pr[3]);
-          dcs[i * U + c_ul] = dcp;
-          float* dgi = dg + (size_t)i * KP + c_ul;
-          float* ph = d.dn_hi + (size_t)(col + sc) * a.dn_pitch + c_u;
-          float* pl = d.dn_lo + (size_t)(col + sc) * a.dn_pitch + c_u;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            dgi[q * U] = pr[q];
-            db[q] += pr[q];
-            float hi, lo;
-            split_tf32(pr[q], hi, lo);
-            ph[(size_t)q * H] = hi;
-            pl[(size_t)q * H] = lo;
-          }
+    for (int q = 0; q < 4; ++q) gt[q] = p[(size_t)q * H];
+    cv = d.c[c_u + (size_t)H * (col + sc)];
+    cp = t ? d.c[c_u + (size_t)H * (colm1 + sc)] : (d.c0 ? d.c0[c_u + (size_t)H * sc] : 0.f);
+    dhv = d.dh[c_u + (size_t)H * (col + sc)];
+    dcv = d.dc ? d.dc[c_u + (size_t)H * (col + sc)] : 0.f;
+  };
+  auto start_of = [&](uint32_t t) { return a.prefix ? a.prefix[t] : t * a.N; };
+  uint32_t n_later = 0;            // columns that were active at step t + 1
+  uint32_t col = T ? start_of(T - 1) : 0;
+  uint32_t n = T ? active_cols(start_of(T) - col, g, G) : 0;
+  if (T && c_live && c_i0 < n) fetch(T - 1, col, T > 1 ? start_of(T - 2) : 0, g + G * c_i0);
+  for (uint32_t t = T; t-- > 0;) {
+    const uint32_t colm1 = t ? start_of(t - 1) : 0, pin = (t + 1) & 1, pout = t & 1;
+    const float* from = part + (size_t)pin * C * ncap * U;
+    if (t && tid == 0) msg_expect(&got[pout], n * C * U * 4);
+    if (n_later) {
+      ok = ok && msg_wait(&got[pin], phase[pin]);
+      phase[pin] ^= 1;
+    }
+    // ---- gradients of the gate pre-activations of this CTA's units ----
+    if (c_live)
+      for (uint32_t i = c_i0; i < n; i += c_step) {
+        const uint32_t sc = g + G * i;
+        if (i != c_i0) fetch(t, col, colm1, sc);
+        float dh = dhv;
+        if (i < n_later) {
+          float r = 0.f;
+          for (uint32_t q = 0; q < C; ++q) r += from[((size_t)q * ncap + i) * U + c_ul];
+          if (d.mask) r *= d.mask[c_u + (a.mask_full ? (size_t)H * sc : 0)];
+          dh += r;
+          d.dh[c_u + (size_t)H * (col + sc)] = dh;
         }
-      if (t == 0) break;             // (no earlier state to hand dE/dh to)
-      __syncthreads();
-      const uint32_t nm1 = active_cols(col - colm1, g, G, i0, ncol);
-      if (c_live && c_i0 < nm1) fetch(t - 1, colm1, t > 1 ? start_of(t - 2) : 0, g + G * (i0 + c_i0));
-      // ---- partial sums of dE/dh_{t-1} over this CTA's gate rows ----
-      const uint32_t pout = o_base + 4u * ((t & 1) * C * ncap * U);
-#pragma unroll 1
-      for (uint32_t nb = 0; nb < n; nb += NB) {
-        u64 acc[8][NB];
+        float dcp = 0.f, pr[4];
+        const float dci = dcv + dcs[i * U + c_ul];
+        if (d.dc && i < n_later) d.dc[c_u + (size_t)H * (col + sc)] = dci;
+        lstm_cell_grad(gt[0], gt[1], gt[2], gt[3], cv, cp, dh, dci, true, dcp, pr[0], pr[1], pr[2], pr[3]);
+        dcs[i * U + c_ul] = dcp;
+        float* dgi = dg + (size_t)i * KP + c_ul;
+        float* ph = d.dn_hi + (size_t)(col + sc) * a.dn_pitch + c_u;
+        float* pl = d.dn_lo + (size_t)(col + sc) * a.dn_pitch + c_u;
 #pragma unroll
-        for (int o = 0; o < 8; ++o)
-#pragma unroll
-          for (int c = 0; c < NB; ++c) acc[o][c] = 0ull;
-        const float* gp = dg + (size_t)nb * KP + 4 * s;
-#pragma unroll
-        for (int j = 0; j < KD / 4; ++j)
-#pragma unroll
-          for (int c = 0; c < NB; ++c) {
-            const ulonglong2 hh = *reinterpret_cast<const ulonglong2*>(gp + (size_t)c * KP + 32 * j);
-#pragma unroll
-            for (int o = 0; o < 8; ++o) { fma2(acc[o][c], w[o][2 * j], hh.x); fma2(acc[o][c], w[o][2 * j + 1], hh.y); }
-          }
-#pragma unroll
-        for (int c = 0; c < NB; ++c) {
-          float v[8];
-#pragma unroll
-          for (int o = 0; o < 8; ++o) v[o] = sum2(acc[o][c]);
-#pragma unroll
-          for (int m = 4; m >= 1; m >>= 1) {
-            const bool up = (s & m) != 0;
-#pragma unroll
-            for (int o = 0; o < 4; ++o)
-              if (o < m) v[o] = xor_add(up ? v[o + m] : v[o], up ? v[o] : v[o + m], m);
-          }
-          if (o_live && nb + c < n) st_cluster(pout + 4u * ((nb + c) * U), v[0]);
+        for (int q = 0; q < 4; ++q) {
+          dgi[q * U] = pr[q];
+          db[q] += pr[q];
+          float hi, lo;
+          split_tf32(pr[q], hi, lo);
+          ph[(size_t)q * H] = hi;
+          pl[(size_t)q * H] = lo;
         }
       }
-      cluster_arrive();
-      cluster_wait();
-      n_later = n; n = nm1; col = colm1;
+    if (t == 0) break;             // (no earlier state to hand dE/dh to)
+    __syncthreads();
+    const uint32_t nm1 = active_cols(col - colm1, g, G);
+    if (c_live && c_i0 < nm1) fetch(t - 1, colm1, t > 1 ? start_of(t - 2) : 0, g + G * c_i0);
+    // ---- partial sums of dE/dh_{t-1} over this CTA's gate rows ----
+#pragma unroll 1
+    for (uint32_t nb = 0; nb < n; nb += NB) {
+      float acc[8][NB];
+#pragma unroll
+      for (int o = 0; o < 8; ++o)
+#pragma unroll
+        for (int c = 0; c < NB; ++c) acc[o][c] = 0.f;
+      const float* gp = dg + (size_t)nb * KP + 4 * s;
+#pragma unroll
+      for (int j = 0; j < KD / 4; ++j)
+#pragma unroll
+        for (int c = 0; c < NF; ++c) {
+          const float4 hh = ld4(gp + (size_t)c * KP + 32 * j);
+#pragma unroll
+          for (int o = 0; o < 8; ++o) acc[o][c] = fmaf(w[o][4 * j], hh.x, acc[o][c]);
+#pragma unroll
+          for (int o = 0; o < 8; ++o) acc[o][c] = fmaf(w[o][4 * j + 1], hh.y, acc[o][c]);
+#pragma unroll
+          for (int o = 0; o < 8; ++o) acc[o][c] = fmaf(w[o][4 * j + 2], hh.z, acc[o][c]);
+#pragma unroll
+          for (int o = 0; o < 8; ++o) acc[o][c] = fmaf(w[o][4 * j + 3], hh.w, acc[o][c]);
+        }
+#pragma unroll
+      for (int c = 0; c < NF; ++c) {
+        float v[8];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) v[o] = acc[o][c];
+#pragma unroll
+        for (int m = 4; m >= 1; m >>= 1) {
+          const bool up = (s & m) != 0;
+#pragma unroll
+          for (int o = 0; o < 4; ++o)
+            if (o < m) v[o] = xor_add(up ? v[o + m] : v[o], up ? v[o] : v[o + m], m);
+        }
+        stage[c * 32 + lane] = v[0];   // (lane 8 g + s holds unit 8 g + s of the warp's 32)
+      }
+      __syncwarp();
+      // the warp hands its sums over: 8 messages of 4 units per column, each to the CTA that owns those units
+      if (NB * 8 >= 32 || lane < NB * 8) {
+        const uint32_t c = lane >> 3;
+        if (msg_live && nb + c < n)
+          send4(map_rank(smem_addr(part + (((size_t)pout * C + rank) * ncap + nb + c) * U + o_msg % U), r_msg),
+                *reinterpret_cast<const float4*>(stage + c * 32 + 4 * (lane & 7)), map_rank(smem_addr(&got[pout]), r_msg));
+      }
+      __syncwarp();
     }
-    cluster_arrive();
-    cluster_wait();
+    n_later = n; n = nm1; col = colm1;
   }
+  cluster_arrive();                // nobody leaves while a neighbour may still send to it
+  cluster_wait();
+  if (!ok) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
   // row sums of dgates: the threads of one unit, in ascending order (part is free: every CTA is through)
+  __syncthreads();
   float* red = part;
   if (c_live)
 #pragma unroll
@@ -409,45 +507,48 @@ __global__ void __launch_bounds__(256) k_rec_db(const float* __restrict__ part0,
 // ---- host side -----------------------------------------------------------------------------------------------------------
 namespace {
 
-constexpr size_t kRecSmemMax = 208 * 1024;
-constexpr uint32_t kRecCols = 64;   // most columns a cluster carries through the sequence at once (more: one batch of them after another)
+constexpr size_t kRecSmemMax = 216 * 1024;
+// Most columns a cluster carries: at 32 - 64 columns a step takes 0.3 us per column and cluster, as much as the per-step tensor
+// products take for the whole GPU; wider batches stay with those.
+constexpr uint32_t kRecCols = 64;
 
 typedef void (*FwdKernel)(RecFwd);
 typedef void (*BwdKernel)(RecBwd);
-// (registers: 4 KD weights + 8 NB accumulator words forward, 8 KD2 + 16 NB backward, at most 255 per thread)
-FwdKernel fwd_kernel(uint32_t kd, uint32_t nb) {
-#define REC_F(K) (nb == 1 ? k_lstm_rec_fwd<K, 1> : nb == 2 ? k_lstm_rec_fwd<K, 2> : nb == 4 ? k_lstm_rec_fwd<K, 4> : k_lstm_rec_fwd<K, 8>)
+// (registers: 8 KD weights + 8 NB sums in both kernels, at most 255 per thread.  Three columns are a variant of their own: up to
+// 45 columns on the 15 clusters of 8 CTAs that fit.)
+FwdKernel fwd_kernel(uint32_t kd, uint32_t n) {
+#define REC_F4(K) n == 1 ? k_lstm_rec_fwd<K, 1> : n == 2 ? k_lstm_rec_fwd<K, 2> : n == 3 ? k_lstm_rec_fwd<K, 4, 3>
+#define REC_F(K) (REC_F4(K) : n == 4 ? k_lstm_rec_fwd<K, 4> : k_lstm_rec_fwd<K, 8>)
   switch (kd) {
+    case 4: return REC_F(4);
     case 8: return REC_F(8);
+    case 12: return REC_F(12);
     case 16: return REC_F(16);
-    case 24: return REC_F(24);
-    case 32: return REC_F(32);
-    case 40: return nb == 1 ? k_lstm_rec_fwd<40, 1> : nb == 2 ? k_lstm_rec_fwd<40, 2> : k_lstm_rec_fwd<40, 4>;
-    default: return nb == 1 ? k_lstm_rec_fwd<48, 1> : k_lstm_rec_fwd<48, 2>;
+    case 20: return REC_F4(20) : k_lstm_rec_fwd<20, 4>;
+    default: return n == 1 ? k_lstm_rec_fwd<24, 1> : k_lstm_rec_fwd<24, 2>;
   }
 #undef REC_F
+#undef REC_F4
 }
-uint32_t fwd_nb_max(uint32_t kd) { return kd <= 32 ? 8 : kd == 40 ? 4 : 2; }
 // (16 gate rows per lane: at most 256 units and threads, 255 registers each; fewer: up to 384 threads of 168 registers)
-BwdKernel bwd_kernel(uint32_t kd, uint32_t nb) {
-#define REC_B(K) (nb == 1 ? k_lstm_rec_bwd<K, 1> : nb == 2 ? k_lstm_rec_bwd<K, 2> : k_lstm_rec_bwd<K, 4>)
+BwdKernel bwd_kernel(uint32_t kd, uint32_t n) {
+#define REC_B(K) (n == 1 ? k_lstm_rec_bwd<K, 1> : n == 2 ? k_lstm_rec_bwd<K, 2> : n == 3 ? k_lstm_rec_bwd<K, 4, 3> : k_lstm_rec_bwd<K, 4>)
   switch (kd) {
     case 8: return REC_B(8);
-    case 12: return nb == 1 ? k_lstm_rec_bwd<12, 1> : k_lstm_rec_bwd<12, 2>;
+    case 12: return REC_B(12);
     default: return REC_B(16);
   }
 #undef REC_B
 }
-uint32_t bwd_nb_max(uint32_t kd) { return kd == 12 ? 2 : 4; }
-uint32_t block_cols(uint32_t n, uint32_t most) {
-  uint32_t nb = 1;
-  while (nb < n && nb < most) nb *= 2;
-  return nb;
-}
 uint32_t fwd_threads(const RecPlan& p) { return 8 * p.U; }
-uint32_t bwd_threads(uint32_t H) { return ((H + 7) / 8 * 8 + 31) / 32 * 32; }
-size_t fwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * 8 * p.KD + p.U); }
+uint32_t bwd_threads(const RecPlan& p) { return (p.C * p.U + 31) / 32 * 32; }
+// shared memory: per column carried, and for Wh on its way into registers (forward)
+size_t fwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * 16 * p.KD + p.U); }
 size_t bwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * p.C * p.U + 8 * p.KD2 + p.U); }
+size_t fwd_smem(const RecPlan& p, uint32_t ncap) {
+  const size_t cols = ncap * fwd_col_bytes(p), weights = sizeof(float) * (16 * p.KD * (4 * p.U + 32) + 32);
+  return cols > weights ? cols : weights;
+}
 
 int launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, dim3 grid, uint32_t threads, size_t smem) {
   DYB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRecSmemMax));
@@ -461,9 +562,9 @@ int launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cud
 }
 // How many clusters run side by side (remembered per context and width class): the columns are dealt out over that many.
 int clusters_that_fit(dyb200_ctx* ctx, const RecPlan& p, bool bwd, uint32_t threads) {
-  int16_t& fit = ctx->rec_fit[bwd][p.KD / 8 - 1][p.C];
+  int16_t& fit = ctx->rec_fit[bwd][p.KD / 4 - 1][p.C];
   if (fit == 0) {
-    const void* k = bwd ? (const void*)bwd_kernel(p.KD2, bwd_nb_max(p.KD2)) : (const void*)fwd_kernel(p.KD, fwd_nb_max(p.KD));
+    const void* k = bwd ? (const void*)bwd_kernel(p.KD2, 4) : (const void*)fwd_kernel(p.KD, 8);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     if (launch_cfg(ctx, k, &cfg, attr, dim3(p.C, 1, 1), threads, kRecSmemMax)) return -1;
@@ -473,40 +574,36 @@ int clusters_that_fit(dyb200_ctx* ctx, const RecPlan& p, bool bwd, uint32_t thre
   }
   return fit;
 }
-// Columns per cluster and per pass of it over the sequence.
-void deal_columns(uint32_t N, int fit, int ndir, size_t col_bytes, uint32_t* G, uint32_t* ncap) {
+// Clusters per direction and columns per cluster; false when a cluster would have to carry more than it can.
+bool deal_columns(uint32_t N, int fit, int ndir, size_t col_bytes, uint32_t* G, uint32_t* ncap) {
   const uint32_t g = fit > ndir ? (uint32_t)(fit / ndir) : 1u;
   *G = N < g ? N : g;
-  const uint32_t nloc = (N + *G - 1) / *G;
-  uint32_t most = (uint32_t)(kRecSmemMax / col_bytes) / 8 * 8;
-  if (most > kRecCols) most = kRecCols;
-  const uint32_t chunks = (nloc + most - 1) / most;
-  *ncap = ((nloc + chunks - 1) / chunks + 7) / 8 * 8;
+  *ncap = ((N + *G - 1) / *G + 7) / 8 * 8;
+  return *ncap <= kRecCols && *ncap * col_bytes <= kRecSmemMax;
 }
 
 }  // namespace
 
-bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, RecPlan* out) {
-  if (H == 0 || H > 384) return false;
+bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan* out) {
+  if (H == 0 || H > 384 || N == 0) return false;
   RecPlan p;
   // up to 256 units: 32 per CTA and at most 8 CTAs, the portable cluster size; beyond: 16 CTAs
   p.U = H <= 256 ? (H < 32 ? (H + 3) / 4 * 4 : 32u) : ((H + 15) / 16 + 3) / 4 * 4;
   p.C = (H + p.U - 1) / p.U;
-  p.KD = (H + 63) / 64 * 8;
+  p.KD = (H + 63) / 64 * 4;
   p.KD2 = p.U <= 16 ? 8 : p.U <= 24 ? 12 : 16;
-  if (clusters_that_fit(ctx, p, false, fwd_threads(p)) <= 0 || clusters_that_fit(ctx, p, true, bwd_threads(H)) <= 0) return false;
+  const int ff = clusters_that_fit(ctx, p, false, fwd_threads(p)), fb = clusters_that_fit(ctx, p, true, bwd_threads(p));
+  if (ff <= 0 || fb <= 0 || !deal_columns(N, ff, ndir, fwd_col_bytes(p), &p.Gf, &p.ncapf) || !deal_columns(N, fb, ndir, bwd_col_bytes(p), &p.Gb, &p.ncapb)) return false;
   *out = p;
   return true;
 }
 
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
-  a->U = p.U;
-  deal_columns(a->N, clusters_that_fit(ctx, p, false, fwd_threads(p)), ndir, fwd_col_bytes(p), &a->G, &a->ncap);
-  const uint32_t per_pass = a->ncap < (a->N + a->G - 1) / a->G ? a->ncap : (a->N + a->G - 1) / a->G;
-  FwdKernel k = fwd_kernel(p.KD, block_cols(per_pass, fwd_nb_max(p.KD)));
+  a->U = p.U; a->G = p.Gf; a->ncap = p.ncapf; a->flags = ctx->dev_flags;
+  FwdKernel k = fwd_kernel(p.KD, (a->N + p.Gf - 1) / p.Gf);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  int rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, a->G, ndir), fwd_threads(p), a->ncap * fwd_col_bytes(p));
+  int rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gf, ndir), fwd_threads(p), fwd_smem(p, p.ncapf));
   if (rc) return rc;
   cudaLaunchKernelEx(&cfg, k, *a);
   DYB_LAUNCHED(ctx);
@@ -514,22 +611,20 @@ int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
 }
 
 int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db) {
-  a->U = p.U;
-  deal_columns(a->N, clusters_that_fit(ctx, p, true, bwd_threads(a->H)), ndir, bwd_col_bytes(p), &a->G, &a->ncap);
-  const uint32_t per_pass = a->ncap < (a->N + a->G - 1) / a->G ? a->ncap : (a->N + a->G - 1) / a->G;
+  a->U = p.U; a->G = p.Gb; a->ncap = p.ncapb; a->flags = ctx->dev_flags;
+  const uint32_t rows = 4 * a->H;
   void* part;
-  int rc = dyb200_scratch(ctx, (size_t)ndir * a->G * 4 * a->H * sizeof(float), &part);
+  int rc = dyb200_scratch(ctx, (size_t)ndir * p.Gb * rows * sizeof(float), &part);
   if (rc) return rc;
-  for (int k = 0; k < ndir; ++k) a->d[k].dbpart = (float*)part + (size_t)k * a->G * 4 * a->H;
-  BwdKernel k = bwd_kernel(p.KD2, block_cols(per_pass, bwd_nb_max(p.KD2)));
+  for (int k = 0; k < ndir; ++k) a->d[k].dbpart = (float*)part + (size_t)k * p.Gb * rows;
+  BwdKernel k = bwd_kernel(p.KD2, (a->N + p.Gb - 1) / p.Gb);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, a->G, ndir), bwd_threads(a->H), a->ncap * bwd_col_bytes(p));
+  rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gb, ndir), bwd_threads(p), p.ncapb * bwd_col_bytes(p));
   if (rc) return rc;
   cudaLaunchKernelEx(&cfg, k, *a);
   DYB_LAUNCHED(ctx);
-  const uint32_t rows = 4 * a->H;
-  dyb_launch(k_rec_db, dim3((rows + 255) / 256, ndir), 256, 0, ctx, (const float*)a->d[0].dbpart, (const float*)a->d[ndir - 1].dbpart, a->G, rows,
+  dyb_launch(k_rec_db, dim3((rows + 255) / 256, ndir), 256, 0, ctx, (const float*)a->d[0].dbpart, (const float*)a->d[ndir - 1].dbpart, p.Gb, rows,
              db[0], db[ndir - 1]);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
@@ -556,9 +651,9 @@ constexpr uint32_t kRecMinSteps = 8;
 
 extern "C" {
 
-int dyb200i_rec_takes(dyb200_ctx* ctx, uint32_t H, uint32_t T) {
+int dyb200i_rec_takes(dyb200_ctx* ctx, uint32_t H, uint32_t T, uint32_t N, int ndir) {
   RecPlan p;
-  return ctx->seq_kernels && T >= kRecMinSteps && dyb200_rec_plan(ctx, H, &p) ? 1 : 0;
+  return ctx->seq_kernels && T >= kRecMinSteps && dyb200_rec_plan(ctx, H, N, ndir, &p) ? 1 : 0;
 }
 
 int dyb200i_rec_inputs(dyb200_ctx* ctx, dyb200_wgrad* w, const float* Wx, const float* b, uint32_t I, uint32_t H, uint32_t columns, float* gates) {
@@ -578,7 +673,7 @@ int dyb200i_rec_inputs(dyb200_ctx* ctx, dyb200_wgrad* w, const float* Wx, const 
 int dyb200i_rec_fwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint32_t H, uint32_t T, uint32_t N, const uint32_t* prefix_dev,
                     int mask_full, float forget_bias) {
   RecPlan p;
-  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, &p), "lstm recurrence: %u units are outside its range", H);
+  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, N, ndir, &p), "lstm recurrence: %u units x %u columns are outside its range", H, N);
   RecFwd a;
   memset(&a, 0, sizeof(a));
   for (int k = 0; k < ndir; ++k) {
@@ -602,7 +697,7 @@ int dyb200i_rec_bwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint
                     int mask_full, uint32_t columns) {
   { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
   RecPlan p;
-  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, &p), "lstm recurrence: %u units are outside its range", H);
+  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, N, ndir, &p), "lstm recurrence: %u units x %u columns are outside its range", H, N);
   RecBwd a;
   memset(&a, 0, sizeof(a));
   float* db[2] = {nullptr, nullptr};

@@ -19,6 +19,7 @@ struct RecFwd {
   int mask_full;
   float fb;
   const uint32_t* prefix;   // device, T + 1 entries: step t has the columns [prefix[t], prefix[t + 1]), widths never grow (null: N each)
+  uint32_t* flags;
 };
 struct RecDirB {
   const float* Wh;
@@ -34,13 +35,15 @@ struct RecBwd {
   uint32_t H, U, T, N, G, ncap, dn_pitch;
   int mask_full;
   const uint32_t* prefix;
+  uint32_t* flags;
 };
 
-// U hidden units per CTA, C CTAs per cluster, KD / KD2 = reduction elements per lane forward / backward.
-struct RecPlan { uint32_t U, C, KD, KD2; };
-// False when the width is outside what the registers of a cluster hold.
-bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, RecPlan* out);
-// ndir directions (1 or 2) share T, N and prefix.  U, G and ncap are filled in here.
+// U hidden units per CTA, C CTAs per cluster, KD / KD2 = reduction elements per lane, G clusters per direction, room for ncap
+// columns per cluster (forward, backward).
+struct RecPlan { uint32_t U, C, KD, KD2, Gf, Gb, ncapf, ncapb; };
+// False when the width is outside what the registers of a cluster hold, or N columns are more than the clusters can carry.
+bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan* out);
+// ndir directions (1 or 2) share T, N and prefix.  U, G, ncap and flags are filled in here.
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir);
 // db[dir] (4H) += row sums of dgates over all columns (partial sums in scratch memory).
 int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db);

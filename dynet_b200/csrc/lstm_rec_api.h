@@ -16,8 +16,8 @@ typedef struct {
   struct dyb200_wgrad* w;               /* may be NULL in the forward pass (no operand planes wanted) */
 } dyb200i_rec_dir;
 
-/* 1 when the kernels take a layer of H units on this device (and a sequence of T steps is long enough to be worth it). */
-int dyb200i_rec_takes(dyb200_ctx* ctx, uint32_t H, uint32_t T);
+/* 1 when the kernels take a layer of H units and N columns (of the widest step) on this device, and T steps are worth it. */
+int dyb200i_rec_takes(dyb200_ctx* ctx, uint32_t H, uint32_t T, uint32_t N, int ndir);
 /* gates = Wx x + b over the first `columns` columns, x = the input planes of w. */
 int dyb200i_rec_inputs(dyb200_ctx* ctx, struct dyb200_wgrad* w, const float* Wx, const float* b, uint32_t I, uint32_t H, uint32_t columns,
                        float* gates);

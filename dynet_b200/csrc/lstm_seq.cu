@@ -522,7 +522,7 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
   // ---- layers of moderate width: the input products of all steps as one GEMM, then the recurrence in clusters (lstm_rec.cu) ----
   if (!persistent && attrs->weightnoise_std == 0.f && I > 0 && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 && Wh->d[0] == G &&
       Wh->d[1] == H && t_size(b) == G && (deferred || !attrs->dropout) &&
-      (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H)) && dyb200i_rec_takes(ctx, H, T)) {
+      (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H)) && dyb200i_rec_takes(ctx, H, T, B, 1)) {
     if (deferred) {
       if ((rc = dyb200i_rec_inputs(ctx, deferred, Wx->v, b->v, I, H, T * B, gates_all->v))) return rc;
     } else {

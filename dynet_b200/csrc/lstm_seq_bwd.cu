@@ -666,7 +666,7 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
   if (first == T && deferred && dx_all && attrs->weightnoise_std == 0.f && I > 0 && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I &&
       Wh->nd == 2 && Wh->d[0] == G && Wh->d[1] == H && t_size(db) == G &&
       (!mx || ((mask_x->bd == B || mask_x->bd == 1) && (mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_x, 0) == I && t_dim(mask_h, 0) == H)) &&
-      dyb200i_rec_takes(ctx, H, T)) {
+      dyb200i_rec_takes(ctx, H, T, B, 1)) {
     dyb200i_rec_dir d;
     memset(&d, 0, sizeof(d));
     d.Wh = Wh->v; d.c0 = c0->v; d.mask_h = mh; d.gates = gates_all->v; d.c = c_all->v; d.dh = dh_all->v; d.dc = dc_all->v; d.db = db->v; d.w = deferred;

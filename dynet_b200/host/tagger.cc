@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "../csrc/lstm_rec_api.h"
 #include "dynet_shim.h"
 
 using namespace dynet_b200;
@@ -83,7 +84,7 @@ struct Tagger {
   float *hf, *hr, *dhf, *dhr, *pre, *th, *dth, *dpre, *logits, *dlogits, *errs, *aux, *ones, *zeros, *scalars;
   // pointer / length tables of the four mover calls (device) and their pinned host staging
   float** tbl_dev; size_t* len_dev;
-  float** tbl_host;   // pinned: 8 N pointers, N lengths, then the ids (2 N words + N tags)
+  float** tbl_host;   // pinned: 8 N pointers, N lengths, then the ids (2 N words + N tags) and the first columns of the steps
   size_t dact_off0, dact_off1;
   char* ws;
   bool time_movers = false;
@@ -96,7 +97,9 @@ struct Tagger {
   cudaStream_t stream2 = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   double host_schedule_ms = 0.0;
+  uint32_t* prefix_dev = nullptr;   // first column of every step, max_len + 1 entries
   ~Tagger() {
+    if (prefix_dev) cudaFree(prefix_dev);
     for (int k = 0; k < 2; ++k) if (d[k].wg) dyb200_wgrad_destroy(d[k].wg);
     if (tbl_host) cudaFreeHost(tbl_host);
     for (auto& e : ev) if (e) cudaEventDestroy(e);
@@ -203,8 +206,19 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   CU(cudaMemcpyAsync(m.d[0].ids, ids_f, (size_t)N * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(m.d[1].ids, ids_r, (size_t)N * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(m.aux + 2 * (size_t)N, tag_ids, (size_t)N * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  const bool rec = dyb200i_rec_takes(dev.ctx, H, Lmax, S, 2) != 0;   // the recurrence of both directions as one launch per pass
+  if (rec) {
+    uint32_t* prefix_host = ids_host + 3 * (size_t)m.max_tok;
+    std::memcpy(prefix_host, prefix.data(), (Lmax + 1) * sizeof(uint32_t));
+    CU(cudaMemcpyAsync(m.prefix_dev, prefix_host, (Lmax + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  }
   CU(cudaEventRecord(m.upload_ev, st));
   m.upload_pending = true;
+  dyb200i_rec_dir rdir[2];
+  for (int dr = 0; dr < 2; ++dr) {
+    const Dir& d = m.d[dr];
+    rdir[dr] = {m.p[P_WHF + 3 * dr], nullptr, nullptr, nullptr, d.gates, d.c, d.h, d.dh, nullptr, m.g[P_BF + 3 * dr], d.wg};
+  }
 
   Tensor tEmb(Dim({E}, V), m.p[P_EMB]);
   const dyb200_lstm_gates_attrs at = {0, 0.f, 1.f};
@@ -225,6 +239,10 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
     // steps launch no operand split of their own
     const dyb200_tensor cxall = to_c(xall);
     throw_status(dev, dyb200_wgrad_pack_inputs(d.wg, &cxall, nullptr, 0, dev.ctx));
+    if (rec) {
+      throw_status(dev, dyb200i_rec_inputs(dev.ctx, d.wg, m.p[P_WXF + 3 * dr], m.p[P_BF + 3 * dr], E, H, N, d.gates));
+      continue;
+    }
     Tensor tWx(Dim({4 * H, E}), m.p[P_WXF + 3 * dr]), tWh(Dim({4 * H, H}), m.p[P_WHF + 3 * dr]), tb(Dim({4 * H}), m.p[P_BF + 3 * dr]);
     const dyb200_tensor cWx = to_c(tWx), cWh = to_c(tWh), cb = to_c(tb);
     for (uint32_t k = 0; k < Lmax; ++k) {
@@ -238,6 +256,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   }
   CU(cudaEventRecord(m.join_ev, st2));
   CU(cudaStreamWaitEvent(st, m.join_ev, 0));
+  if (rec) throw_status(dev, dyb200i_rec_fwd(dev.ctx, 2, rdir, H, Lmax, S, m.prefix_dev, 0, at.forget_gate_bias));
   // combine_tensors: the hidden states of all tokens, token-major
   for (int dr = 0; dr < 2; ++dr) {
     if (m.time_movers) CU(cudaEventRecord(m.ev[2 * dr], st));
@@ -282,6 +301,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
     if (m.time_movers) CU(cudaEventRecord(m.ev[5 + 2 * dr], st));
   }
   Tensor gEmb(Dim({E}, V), m.g[P_EMB]);
+  if (rec) throw_status(dev, dyb200i_rec_bwd(dev.ctx, 2, rdir, H, Lmax, S, m.prefix_dev, 0, N));
   CU(cudaEventRecord(m.fork_ev, st));
   CU(cudaStreamWaitEvent(st2, m.fork_ev, 0));
   for (int dr = 0; dr < 2; ++dr) {
@@ -291,7 +311,8 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
     Tensor gb(Dim({4 * H}), m.g[P_BF + 3 * dr]);
     const dyb200_tensor cWx = to_c(tWx), cWh = to_c(tWh);
     dyb200_tensor cgb = to_c(gb);
-    for (uint32_t k = Lmax; k-- > 0;) {
+    if (rec) throw_status(dev, dyb200i_rec_dx(dev.ctx, d.wg, m.p[P_WXF + 3 * dr], E, H, N, nullptr, 0, 0, d.dx));
+    for (uint32_t k = rec ? 0 : Lmax; k-- > 0;) {
       const uint32_t B = Bk[k];
       const dyb200_tensor cx = to_c(col(d.x, E, prefix[k], B));
       const dyb200_tensor chp = to_c(k ? col(d.h, H, prefix[k - 1], B) : Tensor(Dim({H}, B), m.zeros));
@@ -371,8 +392,10 @@ int dyb200h_tagger_create(const dyb200h_tagger_config* c, float* params, float* 
   if (!rc && (cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
   for (int k = 0; k < 2 && !rc; ++k) rc = dyb200_wgrad_create(k ? m->dev2.ctx : ctx, 4 * c->H, c->E, c->H, max_tokens, &m->d[k].wg);
-  const size_t host_bytes = 8 * (size_t)max_tokens * sizeof(float*) + (size_t)max_tokens * sizeof(size_t) + 3 * (size_t)max_tokens * sizeof(uint32_t);
+  const size_t host_bytes = 8 * (size_t)max_tokens * sizeof(float*) + (size_t)max_tokens * sizeof(size_t) + 3 * (size_t)max_tokens * sizeof(uint32_t) +
+                            ((size_t)max_len + 1) * sizeof(uint32_t);
   if (!rc && cudaMallocHost((void**)&m->tbl_host, host_bytes) != cudaSuccess) { cudaGetLastError(); rc = DYB200_ENOMEM; }
+  if (!rc && cudaMalloc((void**)&m->prefix_dev, ((size_t)max_len + 1) * sizeof(uint32_t)) != cudaSuccess) { cudaGetLastError(); rc = DYB200_ENOMEM; }
   for (auto& e : m->ev) if (!rc && cudaEventCreate(&e) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc && cudaEventCreateWithFlags(&m->upload_ev, cudaEventDisableTiming) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc) rc = dyb200_fill(m->zeros, (size_t)c->H * max_sentences, 0.f, ctx);
