@@ -530,8 +530,29 @@ int dyb200_vanilla_lstm_fwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
                            t_size(gates) == (size_t)G * B &&
                            (!attrs->dropout || ((mask_x->bd == B || mask_x->bd == 1) && (mask_h->bd == B || mask_h->bd == 1) &&
                                                 t_dim(mask_x, 0) == I && t_dim(mask_h, 0) == H));
-    const uint32_t kb = (I + 31) / 32 + (H + 31) / 32;
-    (void)kb;
+    if (shapes_ok && attrs->weightnoise_std == 0.f && I > 0 && H > 0 && B > 0 && dyb200_thin_columns(B)) {
+      // few columns: one pass over the weights in fp32, c and h formed by the CTAs that hold the gates (gemm_thin.cu)
+      const float* mx = attrs->dropout ? mask_x->v : nullptr;
+      const float* mh = attrs->dropout ? mask_h->v : nullptr;
+      const int mx_full = mx ? mask_x->bd == B : 0, mh_full = mh ? mask_h->bd == B : 0;
+      GemmPair pairs[2] = {{Wx->v, G, 0, x->v, I, 0, I, mx, I, mx_full, 1}, {Wh->v, G, 0, h_tm1->v, H, 0, H, mh, H, mh_full, 1}};
+      GemmEpilogue e{EPI_LSTM_CELL, gates->v, G, b->v, H, attrs->forget_gate_bias, nullptr, 0, 0};
+      e.c_prev = c_tm1->v; e.c_out = c_t->v; e.h_out = h_t->v;
+      int rc;
+      if (deferred) {
+        DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_fwd_fused: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
+        PackedOp px, ph;
+        const bool x_pre = dyb200_wgrad_x_planes(deferred, deferred_col, B, &px), h_pre = x_pre && dyb200_wgrad_h_planes(deferred, deferred_col, B, &ph);
+        if (!(x_pre && h_pre)) {
+          PackJobs batch;
+          dyb200_tc_pack_begin(&batch);
+          if ((rc = dyb200_wgrad_push_b_at(deferred, deferred_col, B, x_pre ? nullptr : x->v, I, mx, mx_full, h_tm1->v, H, mh, mh_full, ctx, &batch))) return rc;
+          if ((rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
+        }
+        if (x_pre && dyb200_wgrad_next_h(deferred, deferred_col, B, &e)) { e.hmask = mh; e.hmask_ld = H; e.hmask_full = mh_full; }
+      }
+      return dyb200_lstm_thin(ctx, H, B, 2, pairs, 0, e);
+    }
     if (shapes_ok && attrs->weightnoise_std == 0.f && H % 32 == 0 && I > 0 && B > 0 && dyb200_tc_eligible(G, B, 2.0 * G * B * (I + H)) &&
         aligned16(gates->v) && aligned16(b->v) && aligned16(c_tm1->v) && aligned16(c_t->v) && aligned16(h_t->v)) {
       { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }

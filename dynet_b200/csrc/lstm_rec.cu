@@ -643,10 +643,6 @@ __global__ void __launch_bounds__(256) k_masked_add(const float* __restrict__ sr
   }
 }
 
-// Steps from which a sequence is worth the fixed costs of the recurrence kernels: reading Wh into registers (3 - 5 us), the
-// separate input product and the separate dx product.  Shorter ones stay on the per-step calls.
-constexpr uint32_t kRecMinSteps = 8;
-
 }  // namespace
 
 extern "C" {

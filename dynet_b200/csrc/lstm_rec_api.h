@@ -16,6 +16,9 @@ typedef struct {
   struct dyb200_wgrad* w;               /* may be NULL in the forward pass (no operand planes wanted) */
 } dyb200i_rec_dir;
 
+/* Steps from which a sequence is worth the fixed costs of the recurrence kernels: reading Wh into registers (3 - 5 us), the
+ * separate input product and the separate dx product.  Shorter ones stay on the per-step calls. */
+enum { kRecMinSteps = 8 };
 /* 1 when the kernels take a layer of H units and N columns (of the widest step) on this device, and T steps are worth it. */
 int dyb200i_rec_takes(dyb200_ctx* ctx, uint32_t H, uint32_t T, uint32_t N, int ndir);
 /* gates = Wx x + b over the first `columns` columns, x = the input planes of w. */

@@ -430,6 +430,16 @@ int seq_fwd_dispatch(SeqOp op, uint32_t bn, uint32_t S, dyb200_ctx* ctx, const T
   }
 }
 
+// gates = Wx x + b over all columns: from the accumulator's input planes, or from x itself without one (no mask then)
+int layer_inputs(dyb200_ctx* ctx, dyb200_wgrad* deferred, const float* Wx, const float* x, const float* b, uint32_t I, uint32_t H, uint32_t columns,
+                 float* gates) {
+  if (deferred) return dyb200i_rec_inputs(ctx, deferred, Wx, b, I, H, columns, gates);
+  { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
+  GemmPair p{Wx, 4 * H, 0, x, I, 0, I, nullptr, 0, 0, 1};
+  GemmEpilogue e{EPI_BIAS, gates, 4 * H, b, 0, 0.f, nullptr, 0, 0};
+  return dyb200_gemm_fused(ctx, 4 * H, columns, 1, &p, e);
+}
+
 }  // namespace
 
 extern "C" {
@@ -523,18 +533,36 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
   if (!persistent && attrs->weightnoise_std == 0.f && I > 0 && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 && Wh->d[0] == G &&
       Wh->d[1] == H && t_size(b) == G && (deferred || !attrs->dropout) &&
       (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H)) && dyb200i_rec_takes(ctx, H, T, B, 1)) {
-    if (deferred) {
-      if ((rc = dyb200i_rec_inputs(ctx, deferred, Wx->v, b->v, I, H, T * B, gates_all->v))) return rc;
-    } else {
-      { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
-      GemmPair p{Wx->v, G, 0, x_all->v, I, 0, I, nullptr, 0, 0, 1};
-      GemmEpilogue e{EPI_BIAS, gates_all->v, G, b->v, 0, 0.f, nullptr, 0, 0};
-      if ((rc = dyb200_gemm_fused(ctx, G, T * B, 1, &p, e))) return rc;
-    }
+    if ((rc = layer_inputs(ctx, deferred, Wx->v, x_all->v, b->v, I, H, T * B, gates_all->v))) return rc;
     dyb200i_rec_dir d;
     memset(&d, 0, sizeof(d));
     d.Wh = Wh->v; d.h0 = h0->v; d.c0 = c0->v; d.mask_h = mh; d.gates = gates_all->v; d.c = c_all->v; d.h = h_all->v; d.w = deferred;
     return dyb200i_rec_fwd(ctx, 1, &d, H, T, B, nullptr, mh_full, attrs->forget_gate_bias);
+  }
+
+  // ---- few columns: the input products of all steps as one GEMM, then one pass over Wh per step (gemm_thin.cu) ----
+  // (from as many steps up as the recurrence kernels; a shorter sequence keeps the per-step calls' own sums)
+  if (!persistent && ctx->seq_kernels && T >= kRecMinSteps && attrs->weightnoise_std == 0.f && I > 0 && dyb200_thin_columns(B) && Wx->nd == 2 && Wx->d[0] == G &&
+      Wx->d[1] == I && Wh->nd == 2 && Wh->d[0] == G && Wh->d[1] == H && t_size(b) == G && (deferred || !attrs->dropout) &&
+      (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H))) {
+    { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
+    if ((rc = layer_inputs(ctx, deferred, Wx->v, x_all->v, b->v, I, H, T * B, gates_all->v))) return rc;
+    if (deferred) {
+      PackJobs batch;
+      dyb200_tc_pack_begin(&batch);
+      if ((rc = dyb200_wgrad_seq_h0(deferred, h0->v, mh, mh_full, ctx, &batch))) return rc;
+      if ((rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
+    }
+    for (uint32_t t = 0; t < T; ++t) {
+      GemmPair p{Wh->v, G, 0, t ? h_all->v + (size_t)(t - 1) * HB : h0->v, H, 0, H, mh, H, mh_full, 1};
+      GemmEpilogue e{EPI_LSTM_CELL, gates_all->v + (size_t)t * 4 * HB, G, nullptr, H, attrs->forget_gate_bias, nullptr, 0, 0};
+      e.c_prev = t ? c_all->v + (size_t)(t - 1) * HB : c0->v;
+      e.c_out = c_all->v + (size_t)t * HB; e.h_out = h_all->v + (size_t)t * HB;
+      if (deferred && dyb200_wgrad_next_h(deferred, t * B, B, &e)) { e.hmask = mh; e.hmask_ld = H; e.hmask_full = mh_full; }
+      if ((rc = dyb200_lstm_thin(ctx, H, B, 1, &p, 1, e))) return rc;
+    }
+    if (deferred) dyb200_wgrad_seq_done(deferred);
+    return DYB200_OK;
   }
 
   // ---- the same sequence as one call per time step ----

@@ -312,9 +312,11 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
  * Equivalent, bit for bit, to dyb200_wgrad_pack_inputs(deferred, x_all, mask_x, batch) followed by steps calls of
  * dyb200_vanilla_lstm_fwd_fused_at with deferred_col = t * batch, h_tm1 / c_tm1 = the previous step's outputs.  When the shape
  * allows (tensor-path sizes, whole tiles, every CTA resident at once) the steps run inside ONE kernel whose CTAs stay on the
- * GPU for the whole sequence and hand h_t over through device memory; otherwise the per-step calls are made.
- * dyb200_ctx_sequence_kernels(ctx, 0) forces the per-step form.  deferred may be NULL (per-step form, nothing recorded for
- * the weight gradients). */
+ * GPU for the whole sequence and hand h_t over through device memory; otherwise the per-step calls are made.  Sequences of at
+ * least 8 steps of layers up to 384 units, or with at most 32 columns, form Wx x of all steps at once and keep only Wh h in the
+ * recurrence, in fp32: the same values to fp32 rounding (the sums associate differently), and the same bits from run to run.
+ * dyb200_ctx_sequence_kernels(ctx, 0) forces the per-step form.  deferred may be NULL (nothing recorded for the weight
+ * gradients). */
 int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0,
                                 const dyb200_tensor* Wx, const dyb200_tensor* Wh, const dyb200_tensor* b,
                                 const dyb200_tensor* mask_x, const dyb200_tensor* mask_h, const dyb200_lstm_gates_attrs* attrs,
@@ -331,7 +333,9 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
  * steps run inside ONE kernel whose CTAs stay on the GPU: the cell pass and the [Wx; Wh]^T dgates product of a step hand
  * over through counters in device memory, and every CTA alternates between two independent blocks of batch columns so that
  * one block's hand-overs hide behind the other's products (the per-step call uses the same K splits for such shapes, which
- * keeps the two forms bit-identical).  dyb200_ctx_sequence_kernels(ctx, 0) forces the per-step form. */
+ * keeps the two forms bit-identical).  Sequences of at least 8 steps of layers up to 384 units keep only Wh^T dgates in the
+ * recurrence, in fp32, and form dx of all steps at once: the same values to fp32 rounding.
+ * dyb200_ctx_sequence_kernels(ctx, 0) forces the per-step form. */
 int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0,
                                 const dyb200_tensor* Wx, const dyb200_tensor* Wh, const dyb200_tensor* mask_x,
                                 const dyb200_tensor* mask_h, const dyb200_lstm_gates_attrs* attrs, const dyb200_tensor* gates_all,
