@@ -49,6 +49,7 @@ def build(force=False, verbose=False):
     if jobs or not os.path.exists(LIB):
         subprocess.check_call([NVCC, "-shared", "-o", LIB] + objs + ["-lcudart"])
     build_host(force or bool(jobs))
+    build_call(force)
     return LIB
 
 
@@ -68,6 +69,15 @@ def build_host(force=False):
                           ["-I" + os.path.join(cuda_home, "include"), "-L" + HERE, "-ldyb200",
                            "-L" + os.path.join(cuda_home, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN"])
     return HOST_LIB
+
+
+def build_call(force=False):
+    """The CPython extension behind capi.Context (gcc)."""
+    import sysconfig
+    src, out = os.path.join(HOST, "py", "call.c"), os.path.join(HERE, "_call.so")
+    if force or not os.path.exists(out) or os.path.getmtime(out) < os.path.getmtime(src):
+        subprocess.check_call(["gcc", "-O2", "-fPIC", "-shared", "-Wall", "-o", out, src, "-I" + sysconfig.get_paths()["include"]])
+    return out
 
 
 if __name__ == "__main__":

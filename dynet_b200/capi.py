@@ -185,8 +185,7 @@ def lib():
         L.dyb200_wgrad_destroy.restype = C.c_int
         L.dyb200_wgrad_destroy.argtypes = [C.c_void_p]
         L.dyb200_wgrad_push.restype = C.c_int
-        L.dyb200_wgrad_push.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_int,
-                                        C.c_void_p, C.c_uint32, C.c_void_p, C.c_int, C.c_void_p]
+        L.dyb200_wgrad_push.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_int, C.c_void_p, C.c_uint32, C.c_void_p, C.c_int, C.c_void_p]
         L.dyb200_wgrad_flush.restype = C.c_int
         L.dyb200_wgrad_flush.argtypes = [C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p]
         L.dyb200_ctx_param_cache.restype = C.c_int
@@ -204,11 +203,9 @@ def lib():
         L.dyb200_ctx_profile_count.restype = C.c_int
         L.dyb200_ctx_profile_count.argtypes = [C.c_void_p]
         L.dyb200_ctx_profile_launch.restype = C.c_int
-        L.dyb200_ctx_profile_launch.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_uint32), C.POINTER(C.c_int), C.POINTER(C.c_float),
-                                                C.POINTER(C.c_double)]
+        L.dyb200_ctx_profile_launch.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_uint32), C.POINTER(C.c_int), C.POINTER(C.c_float), C.POINTER(C.c_double)]
         L.dyb200_lookup_accumulate_grads.restype = C.c_int
-        L.dyb200_lookup_accumulate_grads.argtypes = [C.c_uint, C.POINTER(C.c_uint32), C.c_void_p, C.c_void_p,
-                                                     C.c_void_p, C.c_uint, C.c_uint, C.c_void_p]
+        L.dyb200_lookup_accumulate_grads.argtypes = [C.c_uint, C.POINTER(C.c_uint32), C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint, C.c_uint, C.c_void_p]
         L.dyb200_lookup_accumulate_grads_noalloc.restype = C.c_int
         L.dyb200_lookup_accumulate_grads_noalloc.argtypes = L.dyb200_lookup_accumulate_grads.argtypes
         for n in ("dyb200_parallel_memcpy", "dyb200_parallel_accumulate"):
@@ -225,8 +222,7 @@ def lib():
         L.dyb200_sgd_update.restype = C.c_int
         L.dyb200_sgd_update.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_float, C.c_float, C.c_void_p, C.c_void_p]
         L.dyb200_trainer_update.restype = C.c_int
-        L.dyb200_trainer_update.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t,
-                                            C.POINTER(TrainerHyper), C.c_void_p, C.c_int, C.c_void_p]
+        L.dyb200_trainer_update.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.POINTER(TrainerHyper), C.c_void_p, C.c_int, C.c_void_p]
         L.dyb200_wgrad_pack_inputs.restype = C.c_int
         L.dyb200_wgrad_pack_inputs.argtypes = [C.c_void_p, tp, tp, C.c_uint32, C.c_void_p]
         L.dyb200_softmax_output_bwd_fused.restype = C.c_int
@@ -236,6 +232,39 @@ def lib():
                                   C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_int, C.c_uint, C.c_void_p]
         _LIB = L
     return _LIB
+
+
+try:
+    from . import _call
+    _call.setup(C.Structure, DyTensor, C.c_void_p, C.sizeof(DyTensor))
+    _native_call = _call.call
+except ImportError:         # not built (no Python headers): every call goes through ctypes
+    def _native_call(*args):
+        return NotImplemented
+
+_ADDRESS = {}
+
+
+def _address(name):
+    a = _ADDRESS.get(name)
+    if a is None:
+        a = _ADDRESS[name] = C.cast(getattr(lib(), name), C.c_void_p).value
+    return a
+
+
+def _ctypes_call(name, args):
+    """The same call through ctypes, for argument kinds the extension does not take."""
+    out = []
+    for a in args:
+        if isinstance(a, C.Structure):
+            out.append(C.byref(a))
+        elif isinstance(a, (list, tuple)):
+            out.append((DyTensor * len(a))(*a) if a else None)
+        else:
+            out.append(a)
+    f = getattr(lib(), name)
+    # (node attributes are declared void *)
+    return f(*[C.cast(o, C.c_void_p) if t is C.c_void_p and isinstance(a, C.Structure) else o for o, a, t in zip(out, args, f.argtypes)])
 
 
 class Context:
@@ -249,11 +278,20 @@ class Context:
             raise _EXC.get(rc, Dyb200Error)("dyb200_ctx_create(device=%d) failed with status %d: a B200 "
                                             "(sm_100) device is required, there is no CPU fallback" % (device, rc))
         self.h = h
+        self._hv = h.value
+        self._fwd, self._bwd = {}, {}
+
+    def _run(self, name, *args):
+        rc = _native_call(_address(name), *args, self._hv)
+        if rc is NotImplemented:
+            rc = _ctypes_call(name, args + (self._hv,))
+        if rc:
+            self.check(rc)
 
     def close(self):
         if self.h:
             self.L.dyb200_ctx_destroy(self.h)
-            self.h = None
+            self.h = self._hv = None
 
     def __del__(self):
         try:
@@ -291,23 +329,25 @@ class Context:
         self.check(self.L.dyb200_ctx_check_device_errors(self.h, C.byref(f)))
         return f.value
 
-    @staticmethod
-    def _arr(ts):
-        if not ts:
-            return None, 0
-        a = (DyTensor * len(ts))(*ts)
-        return a, len(ts)
-
     def fwd(self, node, xs, fx, attrs=None, aux=None):
-        a, n = self._arr(xs)
-        f = getattr(self.L, "dyb200_%s_fwd" % node)
-        self.check(f(a, n, C.byref(fx), C.cast(C.byref(attrs), C.c_void_p) if attrs is not None else None, aux, self.h))
+        f = self._fwd.get(node)
+        if f is None:
+            f = self._fwd[node] = _address("dyb200_%s_fwd" % node)
+        rc = _native_call(f, xs, len(xs), fx, attrs, aux, self._hv)
+        if rc is NotImplemented:
+            rc = _ctypes_call("dyb200_%s_fwd" % node, (xs, len(xs), fx, attrs, aux, self._hv))
+        if rc:
+            self.check(rc)
 
     def bwd(self, node, xs, fx, dEdf, i, dEdxi, attrs=None, aux=None):
-        a, n = self._arr(xs)
-        f = getattr(self.L, "dyb200_%s_bwd" % node)
-        self.check(f(a, n, C.byref(fx), C.byref(dEdf), i, C.byref(dEdxi),
-                     C.cast(C.byref(attrs), C.c_void_p) if attrs is not None else None, aux, self.h))
+        f = self._bwd.get(node)
+        if f is None:
+            f = self._bwd[node] = _address("dyb200_%s_bwd" % node)
+        rc = _native_call(f, xs, len(xs), fx, dEdf, i, dEdxi, attrs, aux, self._hv)
+        if rc is NotImplemented:
+            rc = _ctypes_call("dyb200_%s_bwd" % node, (xs, len(xs), fx, dEdf, i, dEdxi, attrs, aux, self._hv))
+        if rc:
+            self.check(rc)
 
     def lookup_accumulate_grads(self, ids_host, ids_dev_ptr, g_ptr, all_grads_ptr, dim_size, vocab, n=None):
         """ids_host may be empty with n given: the ids are then only read on the device."""
@@ -315,7 +355,7 @@ class Context:
         if n is None:
             n = len(ids_host)
             arr = (C.c_uint32 * n)(*[int(i) for i in ids_host]) if n else None
-        self.check(self.L.dyb200_lookup_accumulate_grads(n, arr, ids_dev_ptr, g_ptr, all_grads_ptr, dim_size, vocab, self.h))
+        self._run("dyb200_lookup_accumulate_grads", n, arr, ids_dev_ptr, g_ptr, all_grads_ptr, dim_size, vocab)
 
     def lookup_accumulate_grads_noalloc(self, ids_host, ids_dev_ptr, g_ptr, all_grads_ptr, dim_size, vocab):
         """Same as lookup_accumulate_grads, through the entry point that never allocates device memory."""
@@ -332,59 +372,38 @@ class Context:
     def gemm(self, transA, transB, M, N, K, A, lda, B, ldb, Cp, ldc, accumulate, flags=0):
         self.check(self.L.dyb200_gemm(int(transA), int(transB), M, N, K, A, lda, B, ldb, Cp, ldc, int(accumulate), flags, self.h))
 
-    @staticmethod
-    def _opt(t):
-        return C.byref(t) if t is not None else None
-
     def lstm_fwd_fused(self, x, h_tm1, c_tm1, Wx, Wh, b, mask_x, mask_h, attrs, gates, c_t, h_t):
-        o = self._opt
-        self.check(self.L.dyb200_vanilla_lstm_fwd_fused(o(x), o(h_tm1), o(c_tm1), o(Wx), o(Wh), o(b), o(mask_x), o(mask_h),
-                                                        C.byref(attrs), o(gates), o(c_t), o(h_t), self.h))
+        self._run("dyb200_vanilla_lstm_fwd_fused", x, h_tm1, c_tm1, Wx, Wh, b, mask_x, mask_h, attrs, gates, c_t, h_t)
 
     def lstm_bwd_fused(self, x, h_tm1, c_tm1, Wx, Wh, mask_x, mask_h, gates, c_t, dEdh, dEdc, dx, dh_tm1, dc_tm1, dWx, dWh, db, attrs,
                        deferred=None):
-        o = self._opt
-        self.check(self.L.dyb200_vanilla_lstm_bwd_fused(o(x), o(h_tm1), o(c_tm1), o(Wx), o(Wh), o(mask_x), o(mask_h), o(gates), o(c_t),
-                                                        o(dEdh), o(dEdc), o(dx), o(dh_tm1), o(dc_tm1), o(dWx), o(dWh), o(db),
-                                                        C.byref(attrs), deferred, self.h))
+        self._run("dyb200_vanilla_lstm_bwd_fused", x, h_tm1, c_tm1, Wx, Wh, mask_x, mask_h, gates, c_t, dEdh, dEdc, dx, dh_tm1, dc_tm1, dWx, dWh, db, attrs, deferred)
 
     WGRAD_APPEND = 0xffffffff
 
     def lstm_fwd_fused_at(self, x, h_tm1, c_tm1, Wx, Wh, b, mask_x, mask_h, attrs, gates, c_t, h_t, deferred, col):
-        o = self._opt
-        self.check(self.L.dyb200_vanilla_lstm_fwd_fused_at(o(x), o(h_tm1), o(c_tm1), o(Wx), o(Wh), o(b), o(mask_x), o(mask_h),
-                                                           C.byref(attrs), o(gates), o(c_t), o(h_t), deferred, col, self.h))
+        self._run("dyb200_vanilla_lstm_fwd_fused_at", x, h_tm1, c_tm1, Wx, Wh, b, mask_x, mask_h, attrs, gates, c_t, h_t, deferred, col)
 
     def lstm_seq_fwd(self, x_all, h0, c0, Wx, Wh, b, mask_x, mask_h, attrs, gates_all, c_all, h_all, deferred, steps):
-        o = self._opt
-        self.check(self.L.dyb200_vanilla_lstm_seq_fwd(o(x_all), o(h0), o(c0), o(Wx), o(Wh), o(b), o(mask_x), o(mask_h), C.byref(attrs),
-                                                      o(gates_all), o(c_all), o(h_all), deferred, steps, self.h))
+        self._run("dyb200_vanilla_lstm_seq_fwd", x_all, h0, c0, Wx, Wh, b, mask_x, mask_h, attrs, gates_all, c_all, h_all, deferred, steps)
 
     def lstm_seq_bwd(self, x_all, h0, c0, Wx, Wh, mask_x, mask_h, attrs, gates_all, c_all, h_all, dh_all, dc_all, dx_all, dWx, dWh, db,
                      deferred, steps):
-        o = self._opt
-        self.check(self.L.dyb200_vanilla_lstm_seq_bwd(o(x_all), o(h0), o(c0), o(Wx), o(Wh), o(mask_x), o(mask_h), C.byref(attrs),
-                                                      o(gates_all), o(c_all), o(h_all), o(dh_all), o(dc_all), o(dx_all), o(dWx), o(dWh),
-                                                      o(db), deferred, steps, self.h))
+        self._run("dyb200_vanilla_lstm_seq_bwd", x_all, h0, c0, Wx, Wh, mask_x, mask_h, attrs, gates_all, c_all, h_all, dh_all, dc_all, dx_all, dWx, dWh, db, deferred, steps)
 
     def sequence_kernels(self, enable):
         self.check(self.L.dyb200_ctx_sequence_kernels(self.h, int(enable)))
 
     def lstm_bwd_fused_at(self, x, h_tm1, c_tm1, Wx, Wh, mask_x, mask_h, gates, c_t, dEdh, dEdc, dx, dh_tm1, dc_tm1, dWx, dWh, db, attrs,
                           deferred, col):
-        o = self._opt
-        self.check(self.L.dyb200_vanilla_lstm_bwd_fused_at(o(x), o(h_tm1), o(c_tm1), o(Wx), o(Wh), o(mask_x), o(mask_h), o(gates), o(c_t),
-                                                           o(dEdh), o(dEdc), o(dx), o(dh_tm1), o(dc_tm1), o(dWx), o(dWh), o(db),
-                                                           C.byref(attrs), deferred, col, self.h))
+        self._run("dyb200_vanilla_lstm_bwd_fused_at", x, h_tm1, c_tm1, Wx, Wh, mask_x, mask_h, gates, c_t, dEdh, dEdc, dx, dh_tm1, dc_tm1, dWx, dWh, db, attrs, deferred, col)
 
     def softmax_output_bwd_fused(self, x, h, R, dEdf, aux_ptr, dR, db, dh, dx_scratch=None, flags=0):
         """Backward of PickNegLogSoftmax(affine_transform({b, R, h})) in one call (DyTensor arguments, aux_ptr: device pointer)."""
-        o = self._opt
-        self.check(self.L.dyb200_softmax_output_bwd_fused(o(x), o(h), o(R), o(dEdf), aux_ptr, o(dR), o(db), o(dh), o(dx_scratch),
-                                                          flags, self.h))
+        self._run("dyb200_softmax_output_bwd_fused", x, h, R, dEdf, aux_ptr, dR, db, dh, dx_scratch, flags)
 
     def wgrad_pack_inputs(self, w, x_all, mask_x, step):
-        self.check(self.L.dyb200_wgrad_pack_inputs(w, self._opt(x_all), self._opt(mask_x), step, self.h))
+        self._run("dyb200_wgrad_pack_inputs", w, x_all, mask_x, step)
 
     def wgrad_create(self, M, N0, N1, Kcap):
         h = C.c_void_p()
@@ -395,10 +414,10 @@ class Context:
         self.L.dyb200_wgrad_destroy(w)
 
     def wgrad_push(self, w, k, a, lda, b0, ldb0, mask0=None, mask0_full=0, b1=None, ldb1=0, mask1=None, mask1_full=0):
-        self.check(self.L.dyb200_wgrad_push(w, k, a, lda, b0, ldb0, mask0, mask0_full, b1, ldb1, mask1, mask1_full, self.h))
+        self._run("dyb200_wgrad_push", w, k, a, lda, b0, ldb0, mask0, mask0_full, b1, ldb1, mask1, mask1_full)
 
     def wgrad_flush(self, w, C0, ldc0, C1=None, ldc1=0):
-        self.check(self.L.dyb200_wgrad_flush(w, C0, ldc0, C1, ldc1, self.h))
+        self._run("dyb200_wgrad_flush", w, C0, ldc0, C1, ldc1)
 
     def squared_norm(self, x_ptr, n, out_ptr, accumulate=False):
         self.check(self.L.dyb200_squared_norm(x_ptr, n, out_ptr, int(accumulate), self.h))
@@ -409,8 +428,7 @@ class Context:
     def trainer_update(self, rule, params, grads, states, n, hyper, grad_sumsq=None, zero_grads=True):
         """rule: key of RULES; params / grads / states / grad_sumsq: device pointers (ints)."""
         st = list(states) + [None] * (3 - len(states))
-        self.check(self.L.dyb200_trainer_update(RULES[rule], params, grads, st[0], st[1], st[2], n, C.byref(hyper), grad_sumsq,
-                                                int(zero_grads), self.h))
+        self.check(self.L.dyb200_trainer_update(RULES[rule], params, grads, st[0], st[1], st[2], n, C.byref(hyper), grad_sumsq, int(zero_grads), self.h))
 
     def cluster_splitk(self, enable):
         self.check(self.L.dyb200_ctx_cluster_splitk(self.h, int(bool(enable))))

@@ -83,6 +83,7 @@ int dyb200_ctx_create(int device, void* stream, dyb200_ctx** out) {
   c->stream = (cudaStream_t)stream;
   c->sm_count = prop.multiProcessorCount;
   c->cluster_splitk = 1;
+  c->pdl = 1;
   c->seq_kernels = 1;
   if (cudaMalloc((void**)&c->dev_flags, DYB200_DEV_WORDS * 4) != cudaSuccess || cudaMemset(c->dev_flags, 0, DYB200_DEV_WORDS * 4) != cudaSuccess) {
     free(c);

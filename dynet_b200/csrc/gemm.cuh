@@ -72,7 +72,7 @@ __host__ __device__ inline EpiRow epi_row(const GemmEpilogue& e, uint32_t m) {
 int dyb200_gemm_simt(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi);
 // fp32 path for products of few columns (gemm_thin.cu): whether the dispatcher gives it a product, the product itself, and the
 // LSTM step built on it (gates, c and h; pre_in_gates: epi.C holds Wx x + b of the step and only Wh h is added).
-bool dyb200_thin_columns(uint32_t N);
+bool dyb200_thin_columns(uint32_t M, uint32_t N, uint32_t K);
 bool dyb200_thin_takes(uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi);
 int dyb200_gemm_thin(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi);
 int dyb200_lstm_thin(dyb200_ctx* ctx, uint32_t H, uint32_t B, int npairs, const GemmPair* pairs, int pre_in_gates, const GemmEpilogue& epi);

@@ -530,7 +530,7 @@ int dyb200_vanilla_lstm_fwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
                            t_size(gates) == (size_t)G * B &&
                            (!attrs->dropout || ((mask_x->bd == B || mask_x->bd == 1) && (mask_h->bd == B || mask_h->bd == 1) &&
                                                 t_dim(mask_x, 0) == I && t_dim(mask_h, 0) == H));
-    if (shapes_ok && attrs->weightnoise_std == 0.f && I > 0 && H > 0 && B > 0 && dyb200_thin_columns(B)) {
+    if (shapes_ok && attrs->weightnoise_std == 0.f && I > 0 && H > 0 && B > 0 && dyb200_thin_columns(G, B, I + H)) {
       // few columns: one pass over the weights in fp32, c and h formed by the CTAs that hold the gates (gemm_thin.cu)
       const float* mx = attrs->dropout ? mask_x->v : nullptr;
       const float* mh = attrs->dropout ? mask_h->v : nullptr;

@@ -542,7 +542,7 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
 
   // ---- few columns: the input products of all steps as one GEMM, then one pass over Wh per step (gemm_thin.cu) ----
   // (from as many steps up as the recurrence kernels; a shorter sequence keeps the per-step calls' own sums)
-  if (!persistent && ctx->seq_kernels && T >= kRecMinSteps && attrs->weightnoise_std == 0.f && I > 0 && dyb200_thin_columns(B) && Wx->nd == 2 && Wx->d[0] == G &&
+  if (!persistent && ctx->seq_kernels && T >= kRecMinSteps && attrs->weightnoise_std == 0.f && I > 0 && dyb200_thin_columns(G, B, H) && Wx->nd == 2 && Wx->d[0] == G &&
       Wx->d[1] == I && Wh->nd == 2 && Wh->d[0] == G && Wh->d[1] == H && t_size(b) == G && (deferred || !attrs->dropout) &&
       (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H))) {
     { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }

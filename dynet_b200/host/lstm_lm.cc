@@ -467,9 +467,6 @@ int dyb200h_lm_create(const dyb200h_lm_config* c, float* params, float* grads, v
   // this driver owns the parameter updates (dyb200h_lm_update -> dyb200_sgd_update), so the packed
   // copies of the weights can be reused across the time steps of a training step
   dyb200_ctx_param_cache(ctx, 1);
-  // Programmatic dependent launch measured no gain for this step (the graph replay already chains the kernels
-  // tightly: 5.95 vs 6.00 ms at batch 64, 19.9 vs 20.1 ms at batch 512), so this driver leaves it as the caller set it
-  // on the context (dyb200_ctx_dependent_launch; off by default).
   int rc = DYB200_OK;
   if (c->fused) {
     for (uint32_t l = 0; l < c->L && !rc; ++l) {

@@ -141,6 +141,7 @@ class LstmLm:
             raise capi.Dyb200Error("dyb200h_lm_create failed with status %d" % rc)
         self.h = h
         self._mask_keep = None
+        self._mask_views = None
 
     def close(self):
         if getattr(self, "h", None):
@@ -173,8 +174,14 @@ class LstmLm:
             ptr, on_dev = tokens.data_ptr(), 1 if tokens.is_cuda else 0
         mp = None
         if masks_dev is not None:
-            mp = (C.c_void_p * len(masks_dev))(*[m.data_ptr() for m in masks_dev])
+            mp = self._pointers(masks_dev)
         self._check(self.H.dyb200h_lm_forward_backward(self.h, ptr, on_dev, mp, self.loss_dev.data_ptr()))
+
+    def _pointers(self, masks):
+        own = self._mask_views
+        if own is not None and len(own) == len(masks) and all(a is b for a, b in zip(own, masks)):
+            return self._mask_ptrs          # the driver's own buffers, as draw_masks hands them out
+        return (C.c_void_p * len(masks))(*[m.data_ptr() for m in masks])
 
     def _token_ptr(self, tokens):
         if isinstance(tokens, np.ndarray):
@@ -248,6 +255,11 @@ class LstmLm:
 
     def mask_buffers(self):
         """The driver's own 2L mask buffers as torch views into the workspace (mask_x_l is [B, I_l], mask_h_l [B, H])."""
+        return list(self._masks())
+
+    def _masks(self):
+        if self._mask_views is not None:
+            return self._mask_views
         V, E, H, L, T, B = self.dims
         ptrs = (C.c_void_p * (2 * L))()
         n = self.H.dyb200h_lm_mask_buffers(self.h, ptrs, 2 * L)
@@ -256,19 +268,22 @@ class LstmLm:
             cols = (E if k == 0 else H) if k % 2 == 0 else H
             off = ptrs[k] - base
             out.append(self.workspace[off:off + 4 * B * cols].view(self.torch.float32).view(B, cols))
+        self._mask_views = out
+        self._mask_ptrs = (C.c_void_p * n)(*[m.data_ptr() for m in out])
+        # the masks' part of a draw: (tensor, vectors of four random numbers before it)
+        self._mask_plan, quads = [], 0
+        for m in out:
+            self._mask_plan.append((capi.DyTensor.of(m.data_ptr(), [m.shape[1]], m.shape[0]), quads))
+            quads += (m.numel() + 3) // 4
         return out
 
     def draw_masks(self, keep, seed, step):
         """Fresh dropout masks in the driver's buffers: RandomBernoulli(keep, 1/keep) per layer input and hidden state
         (dynet/lstm.cc:964-982), one launch per mask; `step` selects a disjoint stretch of the random stream."""
-        from . import capi
         bufs = self.mask_buffers()
-        off = 0
-        for k, mk in enumerate(bufs):
-            n = mk.numel()
-            at = capi.BernoulliAttrs(float(keep), 1.0 / float(keep), int(seed), int(step) * self._mask_quads + off)
-            self.ctx.fwd("random_bernoulli", [], capi.DyTensor.of(mk.data_ptr(), [mk.shape[1]], mk.shape[0]), at)
-            off += (n + 3) // 4
+        base, keep = int(step) * self._mask_quads, float(keep)
+        for t, off in self._mask_plan:
+            self.ctx.fwd("random_bernoulli", [], t, capi.BernoulliAttrs(keep, 1.0 / keep, int(seed), base + off))
         return bufs
 
     @property
