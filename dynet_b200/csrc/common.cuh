@@ -143,7 +143,9 @@ inline void dyb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = ctx->pdl ? 1 : 0;
+  // (not for kernels that take most of an SM's shared memory: scheduled early, they would keep other streams' work off the SMs
+  // they wait on, and their own prologue is nothing beside their run time)
+  cfg.numAttrs = ctx->pdl && smem <= 96 * 1024 ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);   // a failure is picked up by DYB_LAUNCHED (cudaGetLastError)
 }
 __device__ __forceinline__ void dyb_grid_dep_sync() {

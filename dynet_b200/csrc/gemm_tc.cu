@@ -984,11 +984,9 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     auto fits = [&](uint32_t Sc) -> bool {
@@ -1011,7 +1009,6 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       kb_per_split = (kb_total + Sc - 1) / Sc;
       cfg.gridDim = dim3(grid.x, grid.y, Sc);
       attr[0].val.clusterDim.z = Sc;
-      cfg.numAttrs = ctx->pdl ? 2 : 1;
       GemmProfScope scope(ctx, flops, 1, M, N, kb_total * BK, (uint32_t)epi.mode);
       if (bn == 64) cudaLaunchKernelEx(&cfg, k_gemm_tc<64, true>, tm, M, N, kb0, kb1, kb_per_split, epi, ctx->dev_flags);
       else cudaLaunchKernelEx(&cfg, k_gemm_tc<128, true>, tm, M, N, kb0, kb1, kb_per_split, epi, ctx->dev_flags);

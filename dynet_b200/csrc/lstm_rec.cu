@@ -557,9 +557,7 @@ int launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cud
   cfg->gridDim = grid; cfg->blockDim = dim3(threads, 1, 1); cfg->dynamicSmemBytes = smem; cfg->stream = ctx->stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = grid.x; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg->attrs = attr; cfg->numAttrs = ctx->pdl ? 2 : 1;
+  cfg->attrs = attr; cfg->numAttrs = 1;
   return DYB200_OK;
 }
 // How many clusters run side by side (remembered per context and width class): the columns are dealt out over that many.
@@ -568,9 +566,8 @@ int clusters_that_fit(dyb200_ctx* ctx, const RecPlan& p, bool bwd, uint32_t thre
   if (fit == 0) {
     const void* k = bwd ? (const void*)bwd_kernel(p.KD2, 4) : (const void*)fwd_kernel(p.KD, 8);
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     if (launch_cfg(ctx, k, &cfg, attr, dim3(p.C, 1, 1), threads, kRecSmemMax)) return -1;
-    cfg.numAttrs = 1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
     fit = (int16_t)(n > 0 ? n : -1);
@@ -605,7 +602,7 @@ int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
   a->U = p.U; a->G = p.Gf; a->ncap = p.ncapf; a->flags = ctx->dev_flags;
   FwdKernel k = fwd_kernel(p.KD, (a->N + p.Gf - 1) / p.Gf);
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];
   int rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gf, ndir), fwd_threads(p), fwd_smem(p, p.ncapf));
   if (rc) return rc;
   cudaLaunchKernelEx(&cfg, k, *a);
@@ -622,7 +619,7 @@ int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float
   for (int k = 0; k < ndir; ++k) a->d[k].dbpart = (float*)part + (size_t)k * p.Gb * rows;
   BwdKernel k = bwd_kernel(p.KD2, (a->N + p.Gb - 1) / p.Gb);
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];
   rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gb, ndir), bwd_threads(p), p.ncapb * bwd_col_bytes(p));
   if (rc) return rc;
   cudaLaunchKernelEx(&cfg, k, *a);

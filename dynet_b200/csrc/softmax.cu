@@ -204,6 +204,53 @@ __global__ void __launch_bounds__(kBlock) k_col_stream(ColArgs a) {
   }
 }
 
+// ---- a cluster of 8 CTAs per column, for few long columns: one CTA reading 10 000 rows (the logits of one token) took 4.7 us, and
+// re-read them to write the output; here each CTA keeps its eighth in registers and the eight (max, sum) pairs meet in
+// distributed shared memory, combined in rank order.
+constexpr uint32_t kColCluster = 8, kColVals = 16;   // up to 8 x 256 x 16 rows
+template <int MODE>
+__global__ void __launch_bounds__(kBlock) __cluster_dims__(8, 1, 1) k_col_cluster(ColArgs a) {
+  dyb_grid_dep_sync();
+  __shared__ float red[32];
+  __shared__ float2 part[kColCluster];
+  const uint32_t rank = blockIdx.x, per = (a.rows + kColCluster - 1) / kColCluster, lo = rank * per, hi = min(a.rows, lo + per);
+  const float* xc = a.x + (size_t)blockIdx.y * a.rows;
+  float v[kColVals], mx = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < (int)kColVals; ++k) {
+    const uint32_t r = lo + threadIdx.x + kBlock * k;
+    v[k] = r < hi ? xc[r] : -INFINITY;
+    mx = fmaxf(mx, v[k]);
+  }
+  mx = block_max(mx, red);
+  float s = 0.f;
+  const float ml = shift_log2(mx);
+#pragma unroll
+  for (int k = 0; k < (int)kColVals; ++k) s += ex2_approx(fmaf(v[k], kLog2e, -ml));
+  s = block_sum(s, red);
+  if (threadIdx.x < kColCluster) {
+    uint32_t dst;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"((uint32_t)__cvta_generic_to_shared(&part[rank])), "r"(threadIdx.x));
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst), "f"(mx), "f"(s) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  float m = -INFINITY, tot = 0.f;
+#pragma unroll
+  for (uint32_t q = 0; q < kColCluster; ++q) m = fmaxf(m, part[q].x);
+#pragma unroll
+  for (uint32_t q = 0; q < kColCluster; ++q) tot += part[q].x == -INFINITY ? 0.f : part[q].y * ex2_approx((part[q].x - m) * kLog2e);
+  finish_column<MODE>(a, blockIdx.y, m, tot, rank == 0 && threadIdx.x == 0);
+  if (MODE == M_SOFTMAX || MODE == M_LOGSOFTMAX) {
+    const float z = logf(tot) + m, inv = 1.f / tot, mall = shift_log2(m);
+    float* yc = a.y + (size_t)blockIdx.y * a.rows;
+#pragma unroll
+    for (int k = 0; k < (int)kColVals; ++k) {
+      const uint32_t r = lo + threadIdx.x + kBlock * k;
+      if (r < hi) yc[r] = MODE == M_SOFTMAX ? ex2_approx(fmaf(v[k], kLog2e, -mall)) * inv : v[k] - z;
+    }
+  }
+}
+
 template <int MODE>
 int run_columns(dyb200_ctx* ctx, ColArgs a) {
   if (a.ncols == 0 || a.rows == 0) return DYB200_OK;
@@ -212,6 +259,8 @@ int run_columns(dyb200_ctx* ctx, ColArgs a) {
     dyb_launch(k_col_warp<MODE>, stream_grid(ctx, a.ncols, kBlock / 32), kBlock, 0, ctx, a);
   } else if (a.rows <= kBlockRowsMax && a.rows % 4 == 0 && aligned16(a.x) && (a.y == nullptr || aligned16(a.y))) {
     dyb_launch(k_col_block_vec<MODE>, stream_grid(ctx, a.ncols, 1), kBlock, 0, ctx, a);
+  } else if (a.rows > 2048 && a.rows <= kColCluster * kBlock * kColVals && a.ncols * kColCluster <= (size_t)ctx->sm_count) {
+    dyb_launch(k_col_cluster<MODE>, dim3(kColCluster, (unsigned)a.ncols), kBlock, 0, ctx, a);
   } else {
     dyb_launch(k_col_stream<MODE>, stream_grid(ctx, a.ncols, 1), kBlock, 0, ctx, a);
   }

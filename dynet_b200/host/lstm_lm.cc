@@ -467,6 +467,10 @@ int dyb200h_lm_create(const dyb200h_lm_config* c, float* params, float* grads, v
   // this driver owns the parameter updates (dyb200h_lm_update -> dyb200_sgd_update), so the packed
   // copies of the weights can be reused across the time steps of a training step
   dyb200_ctx_param_cache(ctx, 1);
+  // Inside a CUDA graph the launches follow one another closely as it is, and CTAs that are scheduled early and wait keep the SMs
+  // from other streams: three models on three streams took 143 instead of 126 us per step (V 2000, H 256, batch 16), 3.30 instead
+  // of 3.16 ms (V 10000, H 1024, batch 64).
+  dyb200_ctx_dependent_launch(ctx, 0);
   int rc = DYB200_OK;
   if (c->fused) {
     for (uint32_t l = 0; l < c->L && !rc; ++l) {

@@ -97,9 +97,8 @@ struct Tagger {
   cudaStream_t stream2 = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   double host_schedule_ms = 0.0;
-  uint32_t* prefix_dev = nullptr;   // first column of every step, max_len + 1 entries
+  uint32_t* prefix_dev = nullptr;   // first column of every step, and their end
   ~Tagger() {
-    if (prefix_dev) cudaFree(prefix_dev);
     for (int k = 0; k < 2; ++k) if (d[k].wg) dyb200_wgrad_destroy(d[k].wg);
     if (tbl_host) cudaFreeHost(tbl_host);
     for (auto& e : ev) if (e) cudaEventDestroy(e);
@@ -126,6 +125,7 @@ size_t plan(const dyb200h_tagger_config& c, uint32_t S, uint32_t N, Tagger* t, c
   float* errs = a.take<float>(N); float* aux = a.take<float>(3 * (size_t)N); float* ones = a.take<float>(N);
   float* zeros = a.take<float>(H * S); float* scalars = a.take<float>(64);
   float** tbl = a.take<float*>(8 * (size_t)N); size_t* len = a.take<size_t>(N);
+  uint32_t* prefix_dev = a.take<uint32_t>((size_t)N + 1);   // (a batch has no more steps than tokens)
   // everything below is zeroed by one memset per pass
   a.off = (a.off + 255) & ~(size_t)255;
   const size_t z0 = a.off;
@@ -138,7 +138,7 @@ size_t plan(const dyb200h_tagger_config& c, uint32_t S, uint32_t N, Tagger* t, c
     for (int k = 0; k < 2; ++k) { dyb200_wgrad* keep = t->d[k].wg; t->d[k] = d[k]; t->d[k].wg = keep; }
     t->hf = hf; t->hr = hr; t->dhf = dhf; t->dhr = dhr; t->pre = pre; t->th = th; t->dth = dth; t->dpre = dpre;
     t->logits = logits; t->dlogits = dlogits; t->errs = errs; t->aux = aux; t->ones = ones; t->zeros = zeros; t->scalars = scalars;
-    t->tbl_dev = tbl; t->len_dev = len; t->dact_off0 = z0; t->dact_off1 = z1; t->ws = base;
+    t->prefix_dev = prefix_dev; t->tbl_dev = tbl; t->len_dev = len; t->dact_off0 = z0; t->dact_off1 = z1; t->ws = base;
   }
   return a.off + 256;
 }
@@ -389,13 +389,15 @@ int dyb200h_tagger_create(const dyb200h_tagger_config* c, float* params, float* 
   if (!rc && cudaStreamCreateWithFlags(&m->stream2, cudaStreamNonBlocking) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc) rc = dyb200_ctx_create(device, m->stream2, &m->dev2.ctx);
   if (!rc) dyb200_ctx_param_cache(m->dev2.ctx, 1);
+  // (two streams: a kernel scheduled early would hold SMs that the other direction's kernels could use)
+  dyb200_ctx_dependent_launch(ctx, 0);
+  if (!rc) dyb200_ctx_dependent_launch(m->dev2.ctx, 0);
   if (!rc && (cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
   for (int k = 0; k < 2 && !rc; ++k) rc = dyb200_wgrad_create(k ? m->dev2.ctx : ctx, 4 * c->H, c->E, c->H, max_tokens, &m->d[k].wg);
   const size_t host_bytes = 8 * (size_t)max_tokens * sizeof(float*) + (size_t)max_tokens * sizeof(size_t) + 3 * (size_t)max_tokens * sizeof(uint32_t) +
                             ((size_t)max_len + 1) * sizeof(uint32_t);
   if (!rc && cudaMallocHost((void**)&m->tbl_host, host_bytes) != cudaSuccess) { cudaGetLastError(); rc = DYB200_ENOMEM; }
-  if (!rc && cudaMalloc((void**)&m->prefix_dev, ((size_t)max_len + 1) * sizeof(uint32_t)) != cudaSuccess) { cudaGetLastError(); rc = DYB200_ENOMEM; }
   for (auto& e : m->ev) if (!rc && cudaEventCreate(&e) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc && cudaEventCreateWithFlags(&m->upload_ev, cudaEventDisableTiming) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc) rc = dyb200_fill(m->zeros, (size_t)c->H * max_sentences, 0.f, ctx);

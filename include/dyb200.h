@@ -84,8 +84,8 @@ int dyb200_ctx_profile_launch(dyb200_ctx* ctx, int k, uint32_t shape_out[4], int
  * parameter values (dyb200_sgd_update does it itself); in a DyNet tree that is the end of
  * Trainer::update (dynet/training.cc:195-265).  Costs up to 2x the size of each cached matrix. */
 int dyb200_ctx_param_cache(dyb200_ctx* ctx, int enable);
-/* Programmatic dependent launch (off by default).  When on, every kernel of this library is launched so that it may be
- * scheduled while its predecessor in the stream still runs; each kernel waits, before its first memory access, until that
+/* Programmatic dependent launch (on by default).  When on, the kernels of this library are launched so that they may be
+ * scheduled while their predecessor in the stream still runs; each kernel waits, before its first memory access, until that
  * predecessor has completed (griddepcontrol.wait), so results do not change - only launch latency overlaps.  Work that other
  * code puts into the same stream between two calls is ordered as usual. */
 int dyb200_ctx_dependent_launch(dyb200_ctx* ctx, int enable);

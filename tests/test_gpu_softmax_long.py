@@ -1,0 +1,31 @@
+"""Few long columns (a cluster of CTAs per column) and the lengths and column counts around it, against the oracle."""
+import numpy as np
+import pytest
+
+from util import TOL_REDUCE, assert_close, randn, rng
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,bd", [(2049, 1), (4097, 18), (10000, 1), (32767, 2), (32768, 3), (32769, 2), (5001, 40)])
+def test_long_columns(oracle, rows, bd):
+    import gpu_util as g
+    from dynet_b200 import capi
+    r = rng(rows + bd)
+    x = randn(r, bd, rows, scale=3.0)
+    ids = r.integers(0, rows, bd).astype(np.uint32)
+    ids[0] = rows - 1
+    x_ = g.dev(x)
+    y_ = g.dev(np.zeros_like(x))
+    g.ctx().fwd("softmax", [g.T(x_, [rows], bd)], g.T(y_, [rows], bd), capi.DimAttrs(0))
+    want = oracle.softmax_fwd(x.reshape(bd, 1, rows), 0).reshape(bd, rows)
+    assert_close(g.host(y_), want, TOL_REDUCE, floor=1e-7, what="softmax")
+    aux = g.dev(np.zeros(2 * bd, np.float32))
+    g.ctx().fwd("log_softmax", [g.T(x_, [rows], bd)], g.T(y_, [rows], bd), None, aux.data_ptr())
+    assert_close(g.host(y_), oracle.log_softmax_fwd(x.reshape(bd, 1, rows)).reshape(bd, rows), TOL_REDUCE, floor=1.0, what="log_softmax")
+    loss_, paux = g.dev(np.zeros(bd, np.float32)), g.dev(np.zeros(3 * bd, np.float32))
+    keep, p = g.u32(ids)
+    g.ctx().fwd("pickneglogsoftmax", [g.T(x_, [rows], bd)], g.T(loss_, [1], bd), capi.PickAttrs(p, bd), paux.data_ptr())
+    assert_close(g.host(loss_), oracle.pnls_fwd(x, ids)[0], TOL_REDUCE, floor=1.0, what="pnls")
+    assert g.ctx().device_errors() == 0
+    g.release()
