@@ -299,7 +299,8 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
 }
 
 // grid (C, G, directions), cluster (C, 1, 1); block = C U threads rounded up to warps.  KD = gate rows per slice: 8 KD >= 4 U.
-// Dynamic shared memory: part[2][C][ncap][U], dg[ncap][8 KD], dcs[ncap][U].
+// Dynamic shared memory: part[2][C][ncap][U], dg[2][ncap][8 KD], dcs[ncap][U].  (dg in two: a step's gradients are written as soon
+// as the sums of the step before have arrived, which some warps of this CTA may still be forming for other CTAs.)
 template <int KD, int NB, int NF = NB>
 __global__ void __launch_bounds__(KD == 16 ? 256 : 384, 1) k_lstm_rec_bwd(const __grid_constant__ RecBwd a) {
   constexpr int KP = 8 * KD;
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(KD == 16 ? 256 : 384, 1) k_lstm_rec_bwd(const 
   const uint32_t tid = threadIdx.x, s = tid & 7, og = tid >> 3;
   float* part = rec_smem;                                   // [parity][source rank][column][unit]
   float* dg = part + (size_t)2 * C * ncap * U;
-  float* dcs = dg + (size_t)ncap * KP;
+  float* dcs = dg + (size_t)2 * ncap * KP;
   float* stage = stage_all[tid >> 5];                       // partial sums of this warp's 32 units, column by column
   // message of this lane: 4 units of column lane / 8 of a block, for the CTA that owns them
   const uint32_t lane = tid & 31, o_msg = 32 * (tid >> 5) + 4 * (lane & 7), r_msg = o_msg / U;
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(KD == 16 ? 256 : 384, 1) k_lstm_rec_bwd(const 
   uint32_t phase[2] = {0, 0};
   bool ok = true;
 
-  for (uint32_t e = tid; e < ncap * KP; e += blockDim.x) dg[e] = 0.f;
+  for (uint32_t e = tid; e < 2 * ncap * KP; e += blockDim.x) dg[e] = 0.f;
   for (uint32_t e = tid; e < ncap * U; e += blockDim.x) dcs[e] = 0.f;
   cluster_arrive();
   cluster_wait();
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(KD == 16 ? 256 : 384, 1) k_lstm_rec_bwd(const 
         if (d.dc && i < n_later) d.dc[c_u + (size_t)H * (col + sc)] = dci;
         lstm_cell_grad(gt[0], gt[1], gt[2], gt[3], cv, cp, dh, dci, true, dcp, pr[0], pr[1], pr[2], pr[3]);
         dcs[i * U + c_ul] = dcp;
-        float* dgi = dg + (size_t)i * KP + c_ul;
+        float* dgi = dg + (size_t)((t & 1) * ncap + i) * KP + c_ul;
         float* ph = d.dn_hi + (size_t)(col + sc) * a.dn_pitch + c_u;
         float* pl = d.dn_lo + (size_t)(col + sc) * a.dn_pitch + c_u;
 #pragma unroll
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(KD == 16 ? 256 : 384, 1) k_lstm_rec_bwd(const 
       for (int o = 0; o < 8; ++o)
 #pragma unroll
         for (int c = 0; c < NB; ++c) acc[o][c] = 0.f;
-      const float* gp = dg + (size_t)nb * KP + 4 * s;
+      const float* gp = dg + (size_t)((t & 1) * ncap + nb) * KP + 4 * s;
 #pragma unroll
       for (int j = 0; j < KD / 4; ++j)
 #pragma unroll
@@ -544,7 +545,7 @@ uint32_t fwd_threads(const RecPlan& p) { return 8 * p.U; }
 uint32_t bwd_threads(const RecPlan& p) { return (p.C * p.U + 31) / 32 * 32; }
 // shared memory: per column carried, and for Wh on its way into registers (forward)
 size_t fwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * 16 * p.KD + p.U); }
-size_t bwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * p.C * p.U + 8 * p.KD2 + p.U); }
+size_t bwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * p.C * p.U + 2 * 8 * p.KD2 + p.U); }
 size_t fwd_smem(const RecPlan& p, uint32_t ncap) {
   const size_t cols = ncap * fwd_col_bytes(p), weights = sizeof(float) * (16 * p.KD * (4 * p.U + 32) + 32);
   return cols > weights ? cols : weights;

@@ -98,3 +98,36 @@ def test_recurrence_matches_oracle(oracle, g, I, H, B, T, mask):
     for name, got, ref in zip(("dWx", "dWh"), (dWx, dWh), want[5:7]):
         assert_close(g.host(got), ref, TOL_REDUCE, floor=row_floor(ref, 0, rel=1e-2), what=name + " (per-row scale)")
     assert_close(g.host(db), want[7], TOL_REDUCE, floor=float(np.abs(want[7]).max()) * 0.02, what="db")
+
+
+def test_recurrence_is_the_same_every_time(g):
+    """Widths whose warps and CTAs finish unevenly (a last CTA with two units, nine warps per CTA), many columns: twelve passes over
+    the same inputs give the same bits."""
+    import torch
+    from dynet_b200 import capi
+    I, H, B, T = 45, 262, 372, 19
+    gen = torch.Generator("cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    x, Wx, Wh, b, up = rnd(T * B, I), rnd(I, 4 * H) * 0.05, rnd(H, 4 * H) * 0.05, rnd(4 * H) * 0.1, rnd(T * B, H)
+    z, at, ctx = torch.zeros(B, H, device="cuda"), capi.LstmGatesAttrs(0, 0.0, 1.0), g.ctx()
+    w = ctx.wgrad_create(4 * H, I, H, T * B)
+    first = None
+    try:
+        for _ in range(12):
+            gates, cs, hs, dh = (torch.empty(T * B, n, device="cuda") for n in (4 * H, H, H, H))
+            dc, dx, db = torch.zeros(T * B, H, device="cuda"), torch.zeros(T * B, I, device="cuda"), torch.zeros(4 * H, device="cuda")
+            dh.copy_(up)
+            W = (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1))
+            S = (g.T(gates, [4 * H], T * B), g.T(cs, [H], T * B), g.T(hs, [H], T * B))
+            ctx.lstm_seq_fwd(g.T(x, [I], T * B), g.T(z), g.T(z), *W, g.T(b, [4 * H], 1), None, None, at, *S, w, T)
+            ctx.lstm_seq_bwd(g.T(x, [I], T * B), g.T(z), g.T(z), *W, None, None, at, *S, g.T(dh, [H], T * B), g.T(dc, [H], T * B),
+                             g.T(dx, [I], T * B), None, None, g.T(db, [4 * H], 1), w, T)
+            dWx, dWh = torch.zeros(I, 4 * H, device="cuda"), torch.zeros(H, 4 * H, device="cuda")
+            ctx.wgrad_flush(w, dWx.data_ptr(), 4 * H, dWh.data_ptr(), 4 * H)
+            torch.cuda.synchronize()
+            out = (gates, cs, hs, dh, dx, db, dWx, dWh)
+            first = first or out
+            assert all(torch.equal(p, q) for p, q in zip(first, out))
+    finally:
+        ctx.wgrad_destroy(w)
+    assert ctx.device_errors() == 0
