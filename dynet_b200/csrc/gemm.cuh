@@ -3,6 +3,8 @@
 // All matrices are column-major fp32.  Up to two (A, B) pairs accumulate into the same
 // tile, which is how the gate pre-activation Wx*x + Wh*h is formed in one kernel.
 #pragma once
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 
 struct GemmPair {
@@ -58,6 +60,32 @@ __device__ __forceinline__ void epi_emit_h(const GemmEpilogue& epi, uint32_t u, 
   *reinterpret_cast<float4*>(epi.hn_lo + (size_t)n * epi.hn_pitch + u) = lo;
 }
 #endif
+#ifdef __CUDACC__
+// ---- 2 x 11 bits in fp16 ---------------------------------------------------------------------------------------------------
+// A TF32 hi / lo pair carries 2 x 11 significand bits.  fp16 has the same 11, at twice the rate of the tensor pipe and half the
+// bytes, with 5 bits of exponent.  So an operand row (or a whole parameter) is scaled by a power of two that brings its largest
+// element to [2^14, 2^15), hi = fp16(x s), lo = fp16((x s - hi) 2^11): elements down to 2^-28 of the row's largest keep all
+// 2 x 11 bits, smaller ones an absolute error below 2^-51 of it.  Per k step: A_hi x [B_hi | B_lo] as ONE instruction of twice
+// the columns (B_lo lies right behind B_hi in shared memory), whose halves are the accumulators D1 (hi hi) and D2, then
+// A_lo x B_hi into D2; the result is (D1 + 2^-11 D2) / (s_a s_b).  A chain of D1 is one third of the accumulations of the TF32
+// chain for the same K (the tensor core truncates at each), so chains are cut every 1024 of K here.
+// A scale word is the bit pattern of the row's largest finite |x|: the scale is 2^(141 - E), E its exponent field.
+__device__ __forceinline__ int scale_field(uint32_t word) {   // E, kept where both the scale and its inverse are normal numbers
+  const int e = (int)(word >> 23);
+  return e < 27 ? 27 : e;
+}
+__device__ __forceinline__ float scale_of(uint32_t word) { return __int_as_float((268 - scale_field(word)) << 23); }
+// v 2^(Ea + Eb - 282): in two factors, so that nothing overflows on the way to a result that does not
+__device__ __forceinline__ float unscale(float v, int t) {
+  const int h = t >> 1;
+  return (v * __int_as_float((h + 127) << 23)) * __int_as_float((t - h + 127) << 23);
+}
+constexpr float kLoScale = 1.0f / 2048.0f;
+__device__ __forceinline__ void split_f16(float xs, __half& hi, __half& lo) {
+  hi = __float2half_rn(xs);
+  lo = __float2half_rn((xs - __half2float(hi)) * 2048.0f);
+}
+#endif
 // Row m of the product -> destination pointer of column 0, leading dimension and mask of that row.
 struct EpiRow { float* c; uint32_t ldc; const float* mask; uint32_t mask_ld; int mask_full; };
 __host__ __device__ inline EpiRow epi_row(const GemmEpilogue& e, uint32_t m) {
@@ -87,10 +115,32 @@ int dyb200_gemm_fused(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const
 // TF32 hi / lo planes of an operand: `rows` rows (m or n) of K values.  K-major (mn_major = 0): element (r, k) at
 // plane[r * pitch + k].  MN-major (left operands of dyb200_tc_gemm_packed only): element (r, k) at plane[k * pitch + r] -
 // the K-major planes of the transposed matrix, used as they are.
-struct PackedOp { float* hi; float* lo; uint32_t rows, K, pitch; uint32_t mn_major = 0; };
+// f16: the planes hold scaled fp16 pairs instead (below; hi / lo then point at halves, K-blocks are 64 wide) and `scale` the
+// scale words of the rows (scale_step 1) or of the whole operand (scale_step 0).
+struct PackedOp {
+  float* hi; float* lo; uint32_t rows, K, pitch; uint32_t mn_major = 0;
+  uint32_t f16 = 0; const uint32_t* scale = nullptr; uint32_t scale_step = 0;
+};
+// ---- fp16 operand planes ----
+// One operand as `lines` lines of n contiguous values (line i at src + ld i), its planes laid out alike.  Scale words: one per line
+// (F16_LINE: lines are rows of a K-major operand), one per position in the line (F16_ELEM: positions are rows of an MN-major
+// operand) or one in all (F16_ALL: planes that serve both ways).
+enum F16Scale { F16_LINE = 0, F16_ELEM = 1, F16_ALL = 2 };
+struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; };
+struct F16Jobs { F16Job job[2]; int n; };
+// Planes and scale words for a job from the scratch arena; dyb200_f16_pack fills those of up to two jobs in one pass each.
+int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
+int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
+int dyb200_f16_absmax(dyb200_ctx* ctx, const F16Jobs& jobs);       // the scale words alone
+// The same for a parameter (one scale word, so that its planes can be read both ways), from the parameter cache when it is on.
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, F16Job* job);
+PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
+// Products from here on (useful flops) use fp16 pairs.  Finding the scales adds a clear and a pass over the operands: 8.6 GFLOP
+// (512 x 4096 x 2048) took 86 us that way and 70 us with TF32 pairs, 46 GFLOP (10000 x 2240 x 1024) 205 against 255 us.
+constexpr double kF16Flops = 24.0e9;
 // A queue of packing work that one kernel launch executes (several small operands per launch).
 constexpr int kMaxPackJobs = 8;
-constexpr int kLayoutGates = 2;
+constexpr int kLayoutGates = 2, kLayoutF16 = 3;
 struct PackJob {
   const float* src; const float* mask; float* hi; float* lo;
   uint32_t ld, rows, K, mask_ld, pitch, gx, perm_H;

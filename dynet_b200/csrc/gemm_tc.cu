@@ -23,15 +23,43 @@
 // kernel still frees its TMEM and returns.
 
 #include "tc_dev.cuh"
+#include "seq_dev.cuh"
 
 namespace {
+
+// instruction descriptor: D = f32, A = B = tf32 or f16, M = 128, N = cols (bits 15 / 16: A / B is MN-major)
+__device__ __forceinline__ uint32_t tile_idesc(uint32_t cols, bool f16, uint32_t a_mn, uint32_t b_mn) {
+  return (1u << 4) | (f16 ? 0u : (2u << 7) | (2u << 10)) | ((cols >> 3) << 17) | ((uint32_t)(BM >> 4) << 24) | (a_mn ? 1u << 15 : 0u) |
+         (b_mn ? 1u << 16 : 0u);
+}
+// shared-memory descriptor of an operand tile, and what one MMA's k step adds to it (in units of 16 bytes)
+__device__ __forceinline__ uint64_t tile_desc(uint32_t addr, bool f16, uint32_t mn) {
+  return !mn ? umma_desc(addr) : f16 ? umma_desc_mn16(addr) : umma_desc_mn(addr);
+}
+__device__ __forceinline__ uint64_t mma_step(bool f16, uint32_t mn) { return !mn ? 2 : f16 ? 128 : 64; }
+// F16: the sums of row m, columns [n0, n0 + 64), divided by the scales of the row and the columns
+__device__ __forceinline__ void unscale_tile(const TmapPack& tm, float (&sum)[64], uint32_t m, uint32_t M, uint32_t n0, uint32_t N) {
+  const int ea = scale_field(__ldg(tm.sa + (size_t)min(m, M - 1) * tm.sa_step)) - 282;
+  if (tm.sb_step == 0) {
+    const int t = ea + scale_field(__ldg(tm.sb));
+#pragma unroll
+    for (int j = 0; j < 64; ++j) sum[j] = unscale(sum[j], t);
+  } else {
+    // (a lane fetches the words of two columns and hands them round)
+    const uint32_t lane = threadIdx.x & 31;
+    const int f0 = scale_field(__ldg(tm.sb + min(n0 + lane, N - 1))), f1 = scale_field(__ldg(tm.sb + min(n0 + 32 + lane, N - 1)));
+#pragma unroll
+    for (int j = 0; j < 64; ++j) sum[j] = unscale(sum[j], ea + __shfl_sync(0xffffffffu, j < 32 ? f0 : f1, j & 31));
+  }
+}
 
 // BNT = columns of the output tile: 128, or 64 for products with N <= 64 (small per-GPU batches), where a 128-wide tile
 // would spend half of every MMA and half of the B traffic on padding.
 // CLUSTER: the gridDim.z K-splits of a tile form one thread-block cluster (1 x 1 x S); every CTA parks its partial tile in
 // its own shared memory, and CTA r adds all partial tiles of its 1 / S of the columns through distributed shared memory, in
 // split order, and runs the epilogue on that slice - no workspace round trip and no second kernel.
-template <int BNT, bool CLUSTER>
+// F16: the operands are fp16 pairs (tc_dev.cuh) in k-blocks of 64; an accumulator is D1 | D2, 2 BNT columns of TMEM.
+template <int BNT, bool CLUSTER, bool F16 = false>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__ TmapPack tm, uint32_t M, uint32_t N,
                                                          uint32_t kb0, uint32_t kb1, uint32_t kb_per_split,
                                                          GemmEpilogue epi, uint32_t* flags) {
@@ -50,7 +78,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
   const KSplit ks = k_split(kb0, kb1, blockIdx.z, gridDim.z);
   const uint32_t total = ks.n0 + ks.n1;
   (void)kb_per_split;
-  const uint32_t nchunks = (total + kChunkKB - 1) / kChunkKB;
+  constexpr uint32_t kChunk = F16 ? kChunkF16 : kChunkKB, kAccCols = F16 ? 2 * BN : BN, kTmem = F16 ? 2 * kTmemCols : kTmemCols;
+  constexpr int EL = F16 ? 64 : 32;
+  const uint32_t nchunks = (total + kChunk - 1) / kChunk;
   if (!CLUSTER && gridDim.z > 1) epi.C += (size_t)blockIdx.z * epi.ldc * N;   // raw partial tile of this split (mode is EPI_STORE)
   __shared__ uint32_t split_ok;   // CLUSTER: this CTA's partial tile is complete
 
@@ -65,7 +95,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
     for (int q = 0; q < 8; ++q) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm.t[q]) : "memory");
   }
   if (warp == 1) {   // the whole warp allocates the accumulator columns
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmem) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -84,10 +114,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
         const uint32_t pair = it < ks.n0 ? 0 : 1, kblk = pair ? ks.b1 + (it - ks.n0) : ks.b0 + it;
         unsigned char* st = ring + (size_t)s * STAGE_BYTES;
         mbar_expect_tx(&full_bar[s], STAGE_TX);
-        load_a_tile(st, &tm.t[4 * pair + 0], &full_bar[s], kblk, m0, tm.a_mn);
-        load_a_tile(st + TILE_BYTES, &tm.t[4 * pair + 1], &full_bar[s], kblk, m0, tm.a_mn);
-        load_b_tile(st + 2 * TILE_BYTES, &tm.t[4 * pair + 2], &full_bar[s], kblk, n0, tm.b_mn);
-        load_b_tile(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[4 * pair + 3], &full_bar[s], kblk, n0, tm.b_mn);
+        load_a_tile<EL>(st, &tm.t[4 * pair + 0], &full_bar[s], kblk, m0, tm.a_mn);
+        load_a_tile<EL>(st + TILE_BYTES, &tm.t[4 * pair + 1], &full_bar[s], kblk, m0, tm.a_mn);
+        load_b_tile<EL>(st + 2 * TILE_BYTES, &tm.t[4 * pair + 2], &full_bar[s], kblk, n0, tm.b_mn);
+        load_b_tile<EL>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[4 * pair + 3], &full_bar[s], kblk, n0, tm.b_mn);
         if (++s == STAGES) { s = 0; ph ^= 1; }
       }
     }
@@ -104,17 +134,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
       // instruction descriptor: D = f32, A = B = tf32, both K-major, N = BNT, M = 128
       // (bits 15 / 16: A / B is MN-major)
       const uint32_t a_mn = tm.a_mn, b_mn = tm.b_mn;
-      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BNT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24) |
-                             (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
-      const uint64_t a_step = a_mn ? 64 : 2, b_step = b_mn ? 64 : 2;
+      const uint32_t idesc = tile_idesc(BNT, F16, a_mn, b_mn), idesc_wide = tile_idesc(2 * BNT, F16, a_mn, b_mn);
+      const uint64_t a_step = mma_step(F16, a_mn), b_step = mma_step(F16, b_mn);
       uint64_t d_a_hi[STAGES], d_a_lo[STAGES], d_b_hi[STAGES], d_b_lo[STAGES];
 #pragma unroll
       for (int q = 0; q < STAGES; ++q) {
         const uint32_t base = smem_u32(ring + (size_t)q * STAGE_BYTES);
-        d_a_hi[q] = a_mn ? umma_desc_mn(base) : umma_desc(base);
-        d_a_lo[q] = a_mn ? umma_desc_mn(base + TILE_BYTES) : umma_desc(base + TILE_BYTES);
-        d_b_hi[q] = b_mn ? umma_desc_mn(base + 2 * TILE_BYTES) : umma_desc(base + 2 * TILE_BYTES);
-        d_b_lo[q] = b_mn ? umma_desc_mn(base + 2 * TILE_BYTES + TILE_B_BYTES) : umma_desc(base + 2 * TILE_BYTES + TILE_B_BYTES);
+        d_a_hi[q] = tile_desc(base, F16, a_mn);
+        d_a_lo[q] = tile_desc(base + TILE_BYTES, F16, a_mn);
+        d_b_hi[q] = tile_desc(base + 2 * TILE_BYTES, F16, b_mn);
+        d_b_lo[q] = tile_desc(base + 2 * TILE_BYTES + TILE_B_BYTES, F16, b_mn);
       }
       // The tensor core truncates when it aligns addends to the accumulator, a bias that grows with the length of
       // the accumulation chain.  So the chain is cut every kChunkKB k-blocks: chunk c accumulates into TMEM buffer
@@ -130,10 +159,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
         if (s == 0) { a_hi = d_a_hi[0]; a_lo = d_a_lo[0]; b_hi = d_b_hi[0]; b_lo = d_b_lo[0]; }
         else if (s == 1) { a_hi = d_a_hi[1]; a_lo = d_a_lo[1]; b_hi = d_b_hi[1]; b_lo = d_b_lo[1]; }
         else { a_hi = d_a_hi[2]; a_lo = d_a_lo[2]; b_hi = d_b_hi[2]; b_lo = d_b_lo[2]; }
-        const uint32_t acc = tmem_base + buf * BN;
-        issue_kblock(acc, a_hi, a_lo, b_hi, b_lo, idesc, in_chunk, a_step, b_step);
+        const uint32_t acc = tmem_base + buf * kAccCols;
+        if (F16) issue_kblock_f16(acc, acc + BNT, a_hi, a_lo, b_hi, idesc_wide, idesc, in_chunk, a_step, b_step);
+        else issue_kblock(acc, a_hi, a_lo, b_hi, b_lo, idesc, in_chunk, a_step, b_step);
         umma_commit(&empty_bar[s]);   // frees the stage once these MMAs have read it
-        const bool chunk_ends = in_chunk == kChunkKB - 1 || it == total - 1;
+        const bool chunk_ends = in_chunk == kChunk - 1 || it == total - 1;
         if (chunk_ends) { umma_commit(&acc_full[buf]); in_chunk = 0; ++chunk; buf ^= 1; }
         else ++in_chunk;
         if (++s == STAGES) { s = 0; ph ^= 1; }
@@ -172,13 +202,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
       if (64 * half < BNT) {   // (with a 64-column tile the second column half does not exist)
         // (two 32-column loads: one 64-column load per flush measured slower)
         float v[32];
-        const uint32_t taddr = tmem_base + buf * BN + ((quarter * 32) << 16) + 2 * half * 32;
+        const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + 2 * half * 32;
         tmem_ld32(taddr, v);
 #pragma unroll
         for (int j = 0; j < 32; ++j) sum[j] += v[j];
         tmem_ld32(taddr + 32, v);
 #pragma unroll
         for (int j = 0; j < 32; ++j) sum[32 + j] += v[j];
+        if (F16) {
+          tmem_ld32(taddr + BNT, v);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[j] = fmaf(v[j], kLoScale, sum[j]);
+          tmem_ld32(taddr + BNT + 32, v);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[32 + j] = fmaf(v[j], kLoScale, sum[32 + j]);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -191,6 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
     // 16-byte vectors covering whole 512-byte columns of the tile.  Every epilogue warp reaches the named barrier,
     // whatever its waits did; a failed wait anywhere cancels the stores.
     float* tile = reinterpret_cast<float*>(ring);
+    if (F16 && 64 * half < BNT) unscale_tile(tm, sum, m0 + quarter * 32 + lane, M, n0 + 64 * half, N);
     if (64 * half < BNT) {
       float* col = tile + (size_t)(64 * half) * BM + quarter * 32 + lane;
 #pragma unroll
@@ -248,7 +287,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmem) : "memory");
   }
 }
 
@@ -280,7 +319,7 @@ __device__ __forceinline__ void persist_tile_coords(uint32_t tile, uint32_t tile
 }
 
 // The two single-thread roles are functions of their own: their loops pace the tensor pipe and keep their own registers.
-template <int BNT>
+template <int BNT, bool F16>
 __device__ __noinline__ void persist_producer(const TmapPack* tm, unsigned char* ring, uint64_t* full_bar, uint64_t* empty_bar,
                                               uint32_t tiles, uint32_t tiles_m, uint32_t tiles_n, uint32_t gm, uint32_t kb0,
                                               uint32_t kb1, uint32_t S, uint32_t* flags) {
@@ -300,32 +339,32 @@ __device__ __noinline__ void persist_producer(const TmapPack* tm, unsigned char*
       const uint32_t pair = g < ks.n0 ? 0 : 1, kblk = pair ? ks.b1 + (g - ks.n0) : ks.b0 + g;
       unsigned char* st = ring + (size_t)s * STAGE_BYTES;
       mbar_expect_tx(&full_bar[s], STAGE_TX);
-      load_a_tile(st, &tm->t[4 * pair + 0], &full_bar[s], kblk, m0, tm->a_mn);
-      load_a_tile(st + TILE_BYTES, &tm->t[4 * pair + 1], &full_bar[s], kblk, m0, tm->a_mn);
-      load_b_tile(st + 2 * TILE_BYTES, &tm->t[4 * pair + 2], &full_bar[s], kblk, n0, tm->b_mn);
-      load_b_tile(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm->t[4 * pair + 3], &full_bar[s], kblk, n0, tm->b_mn);
+      load_a_tile<F16 ? 64 : 32>(st, &tm->t[4 * pair + 0], &full_bar[s], kblk, m0, tm->a_mn);
+      load_a_tile<F16 ? 64 : 32>(st + TILE_BYTES, &tm->t[4 * pair + 1], &full_bar[s], kblk, m0, tm->a_mn);
+      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES, &tm->t[4 * pair + 2], &full_bar[s], kblk, n0, tm->b_mn);
+      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm->t[4 * pair + 3], &full_bar[s], kblk, n0, tm->b_mn);
       if (++s == STAGES) { s = 0; ph ^= 1; }
     }
   }
   if (fail) atomicOr(flags, DYB200_FLAG_WAIT_TIMEOUT);
 }
 
-template <int BNT>
+template <int BNT, bool F16>
 __device__ __noinline__ void persist_issue(unsigned char* ring, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* acc_full,
                                            uint64_t* acc_empty, uint32_t tmem_base, uint32_t tiles, uint32_t kb0, uint32_t kb1, uint32_t S,
                                            uint32_t a_mn, uint32_t b_mn, uint32_t* flags) {
   constexpr int TILE_B_BYTES = BNT * BK * 4;
-  const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BNT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24) |
-                         (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
-  const uint64_t a_step = a_mn ? 64 : 2, b_step = b_mn ? 64 : 2;
+  constexpr uint32_t kBufs = F16 ? kPersistBufs / 2 : kPersistBufs, kChunk = F16 ? kChunkF16 : kChunkKB, kAccCols = F16 ? 2 * BN : BN;
+  const uint32_t idesc = tile_idesc(BNT, F16, a_mn, b_mn), idesc_wide = tile_idesc(2 * BNT, F16, a_mn, b_mn);
+  const uint64_t a_step = mma_step(F16, a_mn), b_step = mma_step(F16, b_mn);
   uint64_t d_a_hi[STAGES], d_a_lo[STAGES], d_b_hi[STAGES], d_b_lo[STAGES];
 #pragma unroll
   for (int q = 0; q < STAGES; ++q) {
     const uint32_t base = smem_u32(ring + (size_t)q * STAGE_BYTES);
-    d_a_hi[q] = a_mn ? umma_desc_mn(base) : umma_desc(base);
-    d_a_lo[q] = a_mn ? umma_desc_mn(base + TILE_BYTES) : umma_desc(base + TILE_BYTES);
-    d_b_hi[q] = b_mn ? umma_desc_mn(base + 2 * TILE_BYTES) : umma_desc(base + 2 * TILE_BYTES);
-    d_b_lo[q] = b_mn ? umma_desc_mn(base + 2 * TILE_BYTES + TILE_B_BYTES) : umma_desc(base + 2 * TILE_BYTES + TILE_B_BYTES);
+    d_a_hi[q] = tile_desc(base, F16, a_mn);
+    d_a_lo[q] = tile_desc(base + TILE_BYTES, F16, a_mn);
+    d_b_hi[q] = tile_desc(base + 2 * TILE_BYTES, F16, b_mn);
+    d_b_lo[q] = tile_desc(base + 2 * TILE_BYTES + TILE_B_BYTES, F16, b_mn);
   }
   // stage, phase and chunk counters run on across tiles; an accumulation chain never crosses a tile boundary
   uint32_t s = 0, ph = 0, chunk = 0, buf = 0;
@@ -335,8 +374,8 @@ __device__ __noinline__ void persist_issue(unsigned char* ring, uint64_t* full_b
     const uint32_t kb = ks.n0 + ks.n1;
     uint32_t in_chunk = 0;
     for (uint32_t it = 0; it < kb; ++it) {
-      if (in_chunk == 0 && chunk >= kPersistBufs) {
-        if (!mbar_wait(&acc_empty[buf], ((chunk / kPersistBufs) - 1) & 1)) { fail = true; break; }
+      if (in_chunk == 0 && chunk >= kBufs) {
+        if (!mbar_wait(&acc_empty[buf], ((chunk / kBufs) - 1) & 1)) { fail = true; break; }
       }
       if (!mbar_wait(&full_bar[s], ph)) { fail = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -344,11 +383,12 @@ __device__ __noinline__ void persist_issue(unsigned char* ring, uint64_t* full_b
       if (s == 0) { a_hi = d_a_hi[0]; a_lo = d_a_lo[0]; b_hi = d_b_hi[0]; b_lo = d_b_lo[0]; }
       else if (s == 1) { a_hi = d_a_hi[1]; a_lo = d_a_lo[1]; b_hi = d_b_hi[1]; b_lo = d_b_lo[1]; }
       else { a_hi = d_a_hi[2]; a_lo = d_a_lo[2]; b_hi = d_b_hi[2]; b_lo = d_b_lo[2]; }
-      const uint32_t acc = tmem_base + buf * BN;
-      issue_kblock(acc, a_hi, a_lo, b_hi, b_lo, idesc, in_chunk, a_step, b_step);
+      const uint32_t acc = tmem_base + buf * kAccCols;
+      if (F16) issue_kblock_f16(acc, acc + BNT, a_hi, a_lo, b_hi, idesc_wide, idesc, in_chunk, a_step, b_step);
+      else issue_kblock(acc, a_hi, a_lo, b_hi, b_lo, idesc, in_chunk, a_step, b_step);
       umma_commit(&empty_bar[s]);
-      const bool chunk_ends = in_chunk == kChunkKB - 1 || it == kb - 1;
-      if (chunk_ends) { umma_commit(&acc_full[buf]); in_chunk = 0; ++chunk; buf = chunk % kPersistBufs; }
+      const bool chunk_ends = in_chunk == kChunk - 1 || it == kb - 1;
+      if (chunk_ends) { umma_commit(&acc_full[buf]); in_chunk = 0; ++chunk; buf = chunk % kBufs; }
       else ++in_chunk;
       if (++s == STAGES) { s = 0; ph ^= 1; }
     }
@@ -357,7 +397,7 @@ __device__ __noinline__ void persist_issue(unsigned char* ring, uint64_t* full_b
 }
 
 
-template <int BNT>
+template <int BNT, bool F16 = false>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_constant__ TmapPack tm, uint32_t M, uint32_t N,
                                                               uint32_t kb0, uint32_t kb1, uint32_t tiles_m, uint32_t tiles,
                                                               uint32_t gm, uint32_t S, GemmEpilogue epi, uint32_t* flags) {
@@ -386,21 +426,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) persist_producer<BNT>(&tm, ring, full_bar, empty_bar, tiles, tiles_m, (N + BNT - 1) / BNT, gm, kb0, kb1, S, flags);
+    if (lane == 0) persist_producer<BNT, F16>(&tm, ring, full_bar, empty_bar, tiles, tiles_m, (N + BNT - 1) / BNT, gm, kb0, kb1, S, flags);
   } else if (warp == 1) {
-    if (lane == 0) persist_issue<BNT>(ring, full_bar, empty_bar, acc_full, acc_empty, tmem_base, tiles, kb0, kb1, S, tm.a_mn, tm.b_mn, flags);
+    if (lane == 0) persist_issue<BNT, F16>(ring, full_bar, empty_bar, acc_full, acc_empty, tmem_base, tiles, kb0, kb1, S, tm.a_mn, tm.b_mn, flags);
   } else {
     // epilogue warps 2..9: TMEM lanes 32 (warp % 4) .. +31; warps 2-5 hold columns 0-63 of the tile, warps 6-9 columns 64-127
     const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
     const uint32_t th = (threadIdx.x - 64) & 127;   // 0..127 within this half's four warps
     const bool has_cols = 64 * half < BNT;
+    constexpr uint32_t kBufs = F16 ? kPersistBufs / 2 : kPersistBufs, kChunk = F16 ? kChunkF16 : kChunkKB, kAccCols = F16 ? 2 * BN : BN;
     uint32_t cg = 0;   // chunks drained so far (selects the TMEM buffer and the barrier phase)
     bool ok = true;
 #pragma unroll 1
     for (uint32_t w = blockIdx.x, j = 0; w < tiles * S; w += gridDim.x, ++j) {
       const uint32_t z = w / tiles, tile = w - z * tiles;
       const KSplit ks = k_split(kb0, kb1, z, S);
-      const uint32_t nchunks = (ks.n0 + ks.n1 + kChunkKB - 1) / kChunkKB;
+      const uint32_t nchunks = (ks.n0 + ks.n1 + kChunk - 1) / kChunk;
       // (K splits: epi is a plain store with ldc = M into S partial products side by side, so split z writes columns z N ..)
       const uint32_t n_shift = z * N;
       uint32_t mt, nt;
@@ -411,24 +452,33 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
       for (int q = 0; q < 64; ++q) sum[q] = 0.f;
 #pragma unroll 1
       for (uint32_t c = 0; c < nchunks; ++c, ++cg) {
-        const uint32_t buf = cg % kPersistBufs;
+        const uint32_t buf = cg % kBufs;
         if (!ok) continue;
-        if (!mbar_wait(&acc_full[buf], (cg / kPersistBufs) & 1)) { ok = false; continue; }
+        if (!mbar_wait(&acc_full[buf], (cg / kBufs) & 1)) { ok = false; continue; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (has_cols) {
           float v[32];
-          const uint32_t taddr = tmem_base + buf * BN + ((quarter * 32) << 16) + 2 * half * 32;
+          const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + 2 * half * 32;
           tmem_ld32(taddr, v);
 #pragma unroll
           for (int q = 0; q < 32; ++q) sum[q] += v[q];
           tmem_ld32(taddr + 32, v);
 #pragma unroll
           for (int q = 0; q < 32; ++q) sum[32 + q] += v[q];
+          if (F16) {
+            tmem_ld32(taddr + BNT, v);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) sum[q] = fmaf(v[q], kLoScale, sum[q]);
+            tmem_ld32(taddr + BNT + 32, v);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) sum[32 + q] = fmaf(v[q], kLoScale, sum[32 + q]);
+          }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[buf]);
       }
+      if (F16 && has_cols) unscale_tile(tm, sum, m0 + quarter * 32 + lane, M, n0, N);
       if (!has_cols) continue;   // (64-column tiles: warps 6-9 only take part in the accumulator hand-shake)
       // The staging buffer is free once the other half has written out its columns of the previous turn (128-column
       // tiles), or once this half's own warps have all left the previous pass (64-column tiles).
@@ -440,8 +490,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
       }
       {
         float* col = stage + quarter * 32 + lane;
+        const float b = tm.store_map && epi.mode == EPI_BIAS ? __ldg(epi.bias + min(m0 + quarter * 32 + lane, M - 1)) : 0.f;
 #pragma unroll
-        for (int q = 0; q < 64; ++q) col[(size_t)q * BM] = sum[q];
+        for (int q = 0; q < 64; ++q) col[(size_t)q * BM] = sum[q] + b;
+      }
+      if (tm.store_map) {
+        // A plain store: the staged 64 columns x 128 rows go out as one TMA store (rows and columns past the edge are clipped),
+        // and these warps go on to drain the next tile.  The generic pass below took longer than the tensor pipe needs for a tile
+        // of K = 512 fp16 pairs.
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        const uint32_t fine = bar_and(1u + 2u * half, 128, ok);
+        if (fine && th == 0) {
+          asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(&tm.t[4]), "r"(smem_u32(stage)),
+                       "r"((int)m0), "r"((int)n0), "r"((int)z) : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the buffer may be overwritten
+        }
+        __syncwarp();
+        if (BNT == 128) {
+          if (half == 0) bar_arrive(2, 256);
+          else if (w + gridDim.x < tiles * S) bar_arrive(4, 256);
+        }
+        continue;
       }
       float4 cprev[4];
       if (epi.mode == EPI_LSTM_CELL) {
@@ -643,6 +713,116 @@ __global__ void __launch_bounds__(256) k_pack_multi(const PackJobs jobs) {
   }
 }
 
+// ---- fp16 operand planes: the largest |x| per line, per position or in all, then the split ---------------------------------
+// Both passes read the source once; a line of a wide operand is shared by several CTAs, maxima meet by atomicMax on the bit
+// patterns (the same from run to run).  Infinities and NaNs do not count: they come through the split as they are.
+constexpr uint32_t kMaxLines = 32;   // lines per unit of work where positions have their own scale
+__device__ __forceinline__ uint32_t mag(float v) {
+  const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
+  return u < 0x7f800000u ? u : 0u;
+}
+__device__ __forceinline__ uint32_t mag4(float4 v) { return max(max(mag(v.x), mag(v.y)), max(mag(v.z), mag(v.w))); }
+__global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
+  dyb_grid_dep_sync();
+  const F16Job& j = jobs.job[blockIdx.z];
+  const bool vec = (j.ld & 3) == 0 && aligned16(j.src);
+  if (j.mode == F16_ELEM) {   // a unit is 1024 positions of kMaxLines lines, four positions per thread
+    const uint32_t xb = (j.n + 1023) / 1024, yb = (j.lines + kMaxLines - 1) / kMaxLines;
+    for (uint32_t u = blockIdx.x; u < xb * yb; u += gridDim.x) {
+      const uint32_t e = 4 * ((u % xb) * 256 + threadIdx.x), l0 = u / xb * kMaxLines;
+      if (e >= j.n) continue;
+      uint32_t m[4] = {0, 0, 0, 0};
+#pragma unroll 8
+      for (uint32_t l = l0; l < min(l0 + kMaxLines, j.lines); ++l) {
+        const float* p = j.src + (size_t)j.ld * l + e;
+        if (vec && e + 4 <= j.n) {
+          const float4 v = ld4(p);
+          m[0] = max(m[0], mag(v.x)); m[1] = max(m[1], mag(v.y)); m[2] = max(m[2], mag(v.z)); m[3] = max(m[3], mag(v.w));
+        } else {
+#pragma unroll
+          for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) m[i] = max(m[i], mag(p[i]));
+        }
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) atomicMax(j.scale + e + i, m[i]);
+    }
+    return;
+  }
+  __shared__ uint32_t red[8];
+  uint32_t all = 0;
+  const uint32_t piece = 4096, pieces = (j.n + piece - 1) / piece;
+  const uint64_t units = (uint64_t)pieces * j.lines;
+  for (uint64_t u = blockIdx.x; u < units; u += gridDim.x) {
+    const uint32_t line = (uint32_t)(u / pieces), lo = (uint32_t)(u % pieces) * piece, hi = min(j.n, lo + piece);
+    const float* p = j.src + (size_t)j.ld * line;
+    uint32_t m = 0;
+    if (vec) {
+#pragma unroll 4
+      for (uint32_t e = lo + 4 * threadIdx.x; e < hi; e += 1024) {
+        if (e + 4 <= hi) m = max(m, mag4(ld4(p + e)));
+        else for (uint32_t i = e; i < hi; ++i) m = max(m, mag(p[i]));
+      }
+    } else {
+#pragma unroll 4
+      for (uint32_t e = lo + threadIdx.x; e < hi; e += 256) m = max(m, mag(p[e]));
+    }
+    if (j.mode == F16_ALL) { all = max(all, m); continue; }
+    m = __reduce_max_sync(0xffffffffu, m);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) m = max(m, red[w]);
+      if (pieces == 1) j.scale[line] = m; else atomicMax(j.scale + line, m);
+    }
+  }
+  if (j.mode == F16_ALL) {
+    all = __reduce_max_sync(0xffffffffu, all);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = all;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) all = max(all, red[w]);
+      if (all) atomicMax(j.scale, all);
+    }
+  }
+}
+__device__ __forceinline__ void split4_f16(float4 v, float4 s, uint2& hi, uint2& lo) {
+  __half h[4], l[4];
+  split_f16(v.x * s.x, h[0], l[0]); split_f16(v.y * s.y, h[1], l[1]); split_f16(v.z * s.z, h[2], l[2]); split_f16(v.w * s.w, h[3], l[3]);
+  hi = *reinterpret_cast<const uint2*>(h);
+  lo = *reinterpret_cast<const uint2*>(l);
+}
+__global__ void __launch_bounds__(256) k_f16_split(const F16Jobs jobs) {
+  dyb_grid_dep_sync();
+  const F16Job& j = jobs.job[blockIdx.z];
+  const bool vec = (j.ld & 3) == 0 && aligned16(j.src);
+  const uint32_t q = (j.n + 3) / 4;   // items of four values per line
+  const uint64_t items = (uint64_t)q * j.lines;
+  for (uint64_t it = (uint64_t)blockIdx.x * 256 + threadIdx.x; it < items; it += (uint64_t)gridDim.x * 256) {
+    const uint32_t line = (uint32_t)(it / q), e = 4 * (uint32_t)(it % q);
+    const float* p = j.src + (size_t)j.ld * line + e;
+    float v[4] = {0.f, 0.f, 0.f, 0.f}, s[4];
+    if (vec && e + 4 <= j.n) { const float4 x = ld4(p); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+    else {
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) v[i] = p[i];
+    }
+    if (j.mode == F16_ELEM) {
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i) s[i] = scale_of(__ldg(j.scale + min(e + i, j.n - 1)));
+    } else {
+      s[0] = s[1] = s[2] = s[3] = scale_of(__ldg(j.scale + (j.mode == F16_LINE ? line : 0u)));
+    }
+    uint2 hi, lo;
+    split4_f16(make_float4(v[0], v[1], v[2], v[3]), make_float4(s[0], s[1], s[2], s[3]), hi, lo);
+    // (the pitch is a multiple of 64: the last item's padding stays inside the line's pitch)
+    *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line + e) = hi;
+    *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line + e) = lo;
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -661,12 +841,12 @@ int get_encoder(dyb200_ctx* ctx, EncodeTiledFn* fn) {
 
 // Plane of `rows` rows and K valid floats per row, row pitch `pitch` floats; box = 32 (k) x 128 (rows).
 int make_map(dyb200_ctx* ctx, EncodeTiledFn enc, CUtensorMap* map, float* plane, uint32_t rows, uint32_t K, uint32_t pitch,
-             uint32_t box_rows = BM) {
+             uint32_t box_rows = BM, bool f16 = false) {
   cuuint64_t dims[2] = {K, rows};
-  cuuint64_t strides[1] = {(cuuint64_t)pitch * sizeof(float)};
-  cuuint32_t box[2] = {BK, box_rows};
+  cuuint64_t strides[1] = {(cuuint64_t)pitch * (f16 ? 2 : 4)};
+  cuuint32_t box[2] = {f16 ? 64u : 32u, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, plane, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  CUresult r = enc(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, plane, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return dyb200_fail(ctx, DYB200_ECUDA, "cuTensorMapEncodeTiled failed with code %d (rows %u, K %u, pitch %u)", (int)r, rows, K, pitch);
   return DYB200_OK;
@@ -676,14 +856,16 @@ int make_map(dyb200_ctx* ctx, EncodeTiledFn enc, CUtensorMap* map, float* plane,
 // of 32, k, group): one box = 4 groups x 32 k x 32 m, in the 128-byte swizzle with 32-byte atoms that umma_desc_mn describes.
 // The last group may reach past `rows` into the pitch (those rows of the product are never stored).
 int make_map_mn(dyb200_ctx* ctx, EncodeTiledFn enc, CUtensorMap* map, float* plane, uint32_t rows, uint32_t K, uint32_t pitch,
-                uint32_t box_rows = BM) {
-  // (32 m, k, group of 32 m): one box brings box_rows / 32 groups x 32 k rows x 128 bytes, group after group
-  cuuint64_t dims[3] = {32, K, (rows + 31) / 32};
-  cuuint64_t strides[2] = {(cuuint64_t)pitch * sizeof(float), 128};
-  cuuint32_t box[3] = {32, BK, box_rows / 32};
+                uint32_t box_rows = BM, bool f16 = false) {
+  // (32 m, k, group of 32 m): one box brings box_rows / 32 groups x 32 k rows x 128 bytes, group after group; F16: 64 of each, in
+  // the plain 128-byte swizzle
+  const uint32_t el = f16 ? 64u : 32u;
+  cuuint64_t dims[3] = {el, K, (rows + el - 1) / el};
+  cuuint64_t strides[2] = {(cuuint64_t)pitch * (f16 ? 2 : 4), 128};
+  cuuint32_t box[3] = {el, el, box_rows / el};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, plane, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = enc(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, plane, dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, f16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return dyb200_fail(ctx, DYB200_ECUDA, "cuTensorMapEncodeTiled failed with code %d (MN-major, rows %u, K %u, pitch %u)", (int)r, rows, K, pitch);
   return DYB200_OK;
 }
@@ -735,6 +917,7 @@ int pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int layout, uint32_t ro
 inline uint32_t round_up(uint32_t x, uint32_t m) { return (x + m - 1) / m * m; }
 
 // Returns the cached packed form of a parameter matrix, packing it first if it is new or stale.
+// (k_is_fast = kLayoutF16: fp16 planes of the matrix as it lies, its scale word behind the hi plane)
 int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_fast, uint32_t rows, uint32_t K, uint32_t pitch,
                       float** hi, float** lo, const float* src2 = nullptr, uint32_t rows2 = 0) {
   const int cap = (int)(sizeof(ctx->param_pack) / sizeof(ctx->param_pack[0]));
@@ -747,7 +930,7 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     else if (victim->hi && e->last_use < victim->last_use) victim = e;
   }
   dyb200_ctx::ParamPack* e = hit ? hit : victim;
-  const size_t floats = (size_t)(rows + rows2) * pitch;
+  const size_t floats = k_is_fast == kLayoutF16 ? (size_t)rows * pitch / 2 + 64 : (size_t)(rows + rows2) * pitch;
   if (!hit) {
     if (e->hi && e->floats < floats) {   // evicted entry is too small: its buffers may still be read by queued kernels
       DYB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -766,7 +949,14 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     e->src = src; e->src2 = src2; e->rows2 = rows2; e->ld = ld; e->rows = rows; e->K = K; e->pitch = pitch; e->k_is_fast = (int)k_is_fast;
     e->version = ~0ull;
   }
-  if (e->version != ctx->param_version) {
+  if (e->version != ctx->param_version && k_is_fast == kLayoutF16) {
+    F16Jobs jobs;
+    jobs.n = 1;
+    jobs.job[0] = F16Job{src, ld, rows, K, pitch, F16_ALL, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
+    int rc = dyb200_f16_pack(ctx, &jobs);
+    if (rc) return rc;
+    e->version = ctx->param_version;
+  } else if (e->version != ctx->param_version) {
     PackJobs batch;
     dyb200_tc_pack_begin(&batch);
     int rc = pack(ctx, src, ld, k_is_fast, rows, K, nullptr, 0, 0, e->hi, e->lo, pitch, &batch);
@@ -781,6 +971,65 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
 }
 
 }  // namespace
+
+// ---- fp16 operand planes ----
+int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job) {
+  const uint32_t pitch = round_up(n, 64);
+  const size_t plane = (size_t)lines * pitch * sizeof(__half), words = mode == F16_LINE ? lines : mode == F16_ELEM ? n : 1;
+  void *h, *l, *sc;
+  int rc;
+  if ((rc = dyb200_scratch(ctx, plane, &h)) || (rc = dyb200_scratch(ctx, plane, &l)) || (rc = dyb200_scratch(ctx, words * sizeof(uint32_t), &sc))) return rc;
+  *job = F16Job{src, ld, lines, n, pitch, mode, (uint32_t*)sc, (__half*)h, (__half*)l};
+  return DYB200_OK;
+}
+int dyb200_f16_absmax(dyb200_ctx* ctx, const F16Jobs& jobs) {
+  uint32_t gx = 1;
+  for (int k = 0; k < jobs.n; ++k) {
+    const F16Job& j = jobs.job[k];
+    const bool one_store = j.mode == F16_LINE && j.n <= 4096;   // (every word is written once, no maximum to start from)
+    const size_t words = j.mode == F16_LINE ? j.lines : j.mode == F16_ELEM ? j.n : 1;
+    if (!one_store) DYB_CUDA(ctx, cudaMemsetAsync(j.scale, 0, words * sizeof(uint32_t), ctx->stream));
+    uint64_t x = j.mode == F16_ELEM ? (uint64_t)((j.n + 1023) / 1024) * ((j.lines + kMaxLines - 1) / kMaxLines) : (uint64_t)((j.n + 4095) / 4096) * j.lines;
+    if (x > 8ull * ctx->sm_count) x = 8ull * ctx->sm_count;
+    if (x > gx) gx = (uint32_t)x;
+  }
+  dyb_launch(k_f16_absmax, dim3(gx, 1, jobs.n), 256, 0, ctx, jobs);
+  DYB_LAUNCHED(ctx);
+  return DYB200_OK;
+}
+int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
+  if (jobs->n == 0) return DYB200_OK;
+  int rc = dyb200_f16_absmax(ctx, *jobs);
+  if (rc) return rc;
+  uint64_t most = 0;
+  for (int k = 0; k < jobs->n; ++k) { const uint64_t it = (uint64_t)((jobs->job[k].n + 3) / 4) * jobs->job[k].lines; if (it > most) most = it; }
+  dyb_launch(k_f16_split, dim3(stream_grid(ctx, most, 256, 16), 1, jobs->n), 256, 0, ctx, *jobs);
+  DYB_LAUNCHED(ctx);
+  return DYB200_OK;
+}
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, F16Job* job) {
+  if (!ctx->param_cache_on) {
+    F16Jobs jobs;
+    jobs.n = 1;
+    int rc = dyb200_f16_planes(ctx, src, ld, lines, n, F16_ALL, &jobs.job[0]);
+    if (!rc) rc = dyb200_f16_pack(ctx, &jobs);
+    *job = jobs.job[0];
+    return rc;
+  }
+  const uint32_t pitch = round_up(n, 64);
+  float *hi, *lo;
+  int rc = cached_param_pack(ctx, src, ld, kLayoutF16, lines, n, pitch, &hi, &lo);
+  if (rc) return rc;
+  *job = F16Job{src, ld, lines, n, pitch, F16_ALL, reinterpret_cast<uint32_t*>(hi + (size_t)lines * pitch / 2), (__half*)hi, (__half*)lo};
+  return DYB200_OK;
+}
+PackedOp dyb200_f16_op(const F16Job& j, bool mn_major) {
+  PackedOp p;
+  p.hi = (float*)j.hi; p.lo = (float*)j.lo; p.pitch = j.pitch; p.f16 = 1; p.mn_major = mn_major ? 1u : 0u;
+  p.rows = mn_major ? j.n : j.lines; p.K = mn_major ? j.lines : j.n;
+  p.scale = j.scale; p.scale_step = j.mode == F16_ALL ? 0u : 1u;
+  return p;
+}
 
 // ---- building blocks shared with the fused LSTM entry points ----------------------------------
 int dyb200_tc_pack_flush(dyb200_ctx* ctx, PackJobs* batch) { return pack_flush_impl(ctx, batch); }
@@ -927,13 +1176,20 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   if (!(ctx->func_attr_done & 1u)) {
     DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     ctx->func_attr_done |= 1u;
   }
   const uint32_t bn = tile_cols(N);
   TmapPack tm;
   memset(&tm, 0, sizeof(tm));
   double flops = 0;
-  const bool a_mn = A[0].mn_major != 0, b_mn = B[0].mn_major != 0;
+  const bool a_mn = A[0].mn_major != 0, b_mn = B[0].mn_major != 0, f16 = A[0].f16 != 0;
+  const uint32_t el = f16 ? 64u : 32u;
+  DYB_CHECK_ARG(ctx, !f16 || (npairs == 1 && B[0].f16 && A[0].scale && B[0].scale && A[0].pitch % 64 == 0 && B[0].pitch % 64 == 0),
+                "tensor GEMM: fp16 operands come in one pair, both with scale words and a pitch that is a multiple of 64");
+  DYB_CHECK_ARG(ctx, f16 || !B[0].f16, "tensor GEMM: operands of two kinds");
+  tm.sa = A[0].scale; tm.sb = B[0].scale; tm.sa_step = A[0].scale_step; tm.sb_step = B[0].scale_step;
   // (an MN-major plane is read in groups of 32 rows: its pitch covers the rows rounded up to 32)
   DYB_CHECK_ARG(ctx, !a_mn || (npairs == 1 && A[0].pitch % 32 == 0 && A[0].pitch >= M && aligned16(A[0].hi) && aligned16(A[0].lo)),
                 "tensor GEMM: an MN-major left operand needs a single pair, a pitch that is a multiple of 32 and covers the rows, and 16-byte aligned planes");
@@ -946,22 +1202,22 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
                   "tensor GEMM: packed operand shapes do not match (M %u, N %u)", M, N);
     flops += 2.0 * M * N * A[p].K;
     if (a_mn) {
-      if ((rc = make_map_mn(ctx, enc, &tm.t[0], A[0].hi, M, A[0].K, A[0].pitch))) return rc;
-      if ((rc = make_map_mn(ctx, enc, &tm.t[1], A[0].lo, M, A[0].K, A[0].pitch))) return rc;
+      if ((rc = make_map_mn(ctx, enc, &tm.t[0], A[0].hi, M, A[0].K, A[0].pitch, BM, f16))) return rc;
+      if ((rc = make_map_mn(ctx, enc, &tm.t[1], A[0].lo, M, A[0].K, A[0].pitch, BM, f16))) return rc;
     } else {
-      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 0], A[p].hi, M, A[p].K, A[p].pitch))) return rc;
-      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 1], A[p].lo, M, A[p].K, A[p].pitch))) return rc;
+      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 0], A[p].hi, M, A[p].K, A[p].pitch, BM, f16))) return rc;
+      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 1], A[p].lo, M, A[p].K, A[p].pitch, BM, f16))) return rc;
     }
     if (b_mn) {
-      if ((rc = make_map_mn(ctx, enc, &tm.t[2], B[0].hi, N, B[0].K, B[0].pitch, bn))) return rc;
-      if ((rc = make_map_mn(ctx, enc, &tm.t[3], B[0].lo, N, B[0].K, B[0].pitch, bn))) return rc;
+      if ((rc = make_map_mn(ctx, enc, &tm.t[2], B[0].hi, N, B[0].K, B[0].pitch, bn, f16))) return rc;
+      if ((rc = make_map_mn(ctx, enc, &tm.t[3], B[0].lo, N, B[0].K, B[0].pitch, bn, f16))) return rc;
     } else {
-      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 2], B[p].hi, N, B[p].K, B[p].pitch, bn))) return rc;
-      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 3], B[p].lo, N, B[p].K, B[p].pitch, bn))) return rc;
+      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 2], B[p].hi, N, B[p].K, B[p].pitch, bn, f16))) return rc;
+      if ((rc = make_map(ctx, enc, &tm.t[4 * p + 3], B[p].lo, N, B[p].K, B[p].pitch, bn, f16))) return rc;
     }
   }
   if (npairs == 1) for (int k = 0; k < 4; ++k) tm.t[4 + k] = tm.t[k];
-  uint32_t kb0 = round_up(A[0].K, 32) / BK, kb1 = npairs > 1 ? round_up(A[1].K, 32) / BK : 0;
+  uint32_t kb0 = round_up(A[0].K, el) / el, kb1 = npairs > 1 ? round_up(A[1].K, el) / el : 0;
   const uint32_t kb_total = kb0 + kb1;
   dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, 1);
   DYB_CHECK_ARG(ctx, epi.mode != EPI_LSTM_CELL || (M % BM == 0 && epi.H * 4 == M && epi.ldc % 4 == 0 && aligned16(epi.C) &&
@@ -979,6 +1235,8 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     if (!(ctx->func_attr_done & 2u)) {
       DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
       DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
       ctx->func_attr_done |= 2u;
     }
     cudaLaunchConfig_t cfg;
@@ -1009,9 +1267,9 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       kb_per_split = (kb_total + Sc - 1) / Sc;
       cfg.gridDim = dim3(grid.x, grid.y, Sc);
       attr[0].val.clusterDim.z = Sc;
-      GemmProfScope scope(ctx, flops, 1, M, N, kb_total * BK, (uint32_t)epi.mode);
-      if (bn == 64) cudaLaunchKernelEx(&cfg, k_gemm_tc<64, true>, tm, M, N, kb0, kb1, kb_per_split, epi, ctx->dev_flags);
-      else cudaLaunchKernelEx(&cfg, k_gemm_tc<128, true>, tm, M, N, kb0, kb1, kb_per_split, epi, ctx->dev_flags);
+      GemmProfScope scope(ctx, flops, 1, M, N, kb_total * el, (uint32_t)epi.mode);
+      auto kern = f16 ? (bn == 64 ? k_gemm_tc<64, true, true> : k_gemm_tc<128, true, true>) : (bn == 64 ? k_gemm_tc<64, true> : k_gemm_tc<128, true>);
+      cudaLaunchKernelEx(&cfg, kern, tm, M, N, kb0, kb1, kb_per_split, epi, ctx->dev_flags);
       DYB_LAUNCHED(ctx);
       return DYB200_OK;
     }
@@ -1040,6 +1298,8 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     if (!(ctx->func_attr_done & 4u)) {
       DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
       DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
+      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
+      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
       ctx->func_attr_done |= 4u;
     }
     // A long reduction whose tiles fill the last round badly (the deferred weight gradients: 256 tiles of 560 k-blocks on
@@ -1066,13 +1326,22 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       ppart = (float*)pw;
       pepi = GemmEpilogue{EPI_STORE, ppart, M, nullptr, 0, 0.f, nullptr, 0, 0};
     }
+    // one TMA store per finished half tile where the destination allows it
+    if (npairs == 1 && (pepi.mode == EPI_STORE || pepi.mode == EPI_BIAS) && pepi.split_m == 0 && pepi.ldc % 4 == 0 && aligned16(pepi.C)) {
+      cuuint64_t dims[3] = {M, N, Sp}, strides[2] = {(cuuint64_t)pepi.ldc * 4, (cuuint64_t)pepi.ldc * N * 4};
+      cuuint32_t box[3] = {BM, 64, 1}, estr[3] = {1, 1, 1};
+      CUresult r = enc(&tm.t[4], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, pepi.C, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      if (r != CUDA_SUCCESS) return dyb200_fail(ctx, DYB200_ECUDA, "cuTensorMapEncodeTiled failed with code %d (output %u x %u, ld %u)", (int)r, M, N, pepi.ldc);
+      tm.store_map = 1;
+    }
     {
-      GemmProfScope scope(ctx, flops * ((double)tiles_run / (grid.x * grid.y)), 1, M, N, kb_total * BK, (uint32_t)epi.mode);
+      GemmProfScope scope(ctx, flops * ((double)tiles_run / (grid.x * grid.y)), 1, M, N, kb_total * el, (uint32_t)epi.mode);
       // grouped tile order when the A operand has many row blocks (unless the last round runs apart as part of the last
       // column of tiles, which relies on the row-block-fastest order)
       const uint32_t gm = (tail_form != 1 && rows_run > 16) ? 16u : 0u;
-      if (bn == 64) dyb_launch(k_gemm_persist<64>, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb0, kb1, rows_run, tiles_run, gm, Sp, pepi, ctx->dev_flags);
-      else dyb_launch(k_gemm_persist<128>, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb0, kb1, rows_run, tiles_run, gm, Sp, pepi, ctx->dev_flags);
+      auto kern = f16 ? (bn == 64 ? k_gemm_persist<64, true> : k_gemm_persist<128, true>) : (bn == 64 ? k_gemm_persist<64> : k_gemm_persist<128>);
+      dyb_launch(kern, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb0, kb1, rows_run, tiles_run, gm, Sp, pepi, ctx->dev_flags);
       DYB_LAUNCHED(ctx);
       if (Sp > 1 && (rc = dyb200_splitk_reduce(ctx, ppart, Sp, M, N, epi))) return rc;
     }
@@ -1082,9 +1351,13 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     PackedOp A2[2], B2[2];
     for (int p = 0; p < npairs; ++p) {
       A2[p] = A[p]; A2[p].rows = M - m_off;   // (MN-major planes: the rows are the fast index)
-      A2[p].hi += a_mn ? (size_t)m_off : (size_t)m_off * A[p].pitch; A2[p].lo += a_mn ? (size_t)m_off : (size_t)m_off * A[p].pitch;
+      auto ahead = [&](float* q, size_t n) { return f16 ? (float*)((__half*)q + n) : q + n; };
+      const size_t ao = a_mn ? (size_t)m_off : (size_t)m_off * A[p].pitch, bo = b_mn ? (size_t)n_off : (size_t)n_off * B[p].pitch;
+      A2[p].hi = ahead(A[p].hi, ao); A2[p].lo = ahead(A[p].lo, ao);
+      if (f16) { A2[p].scale += (size_t)m_off * A[p].scale_step; }
       B2[p] = B[p]; B2[p].rows = N - n_off;
-      B2[p].hi += b_mn ? (size_t)n_off : (size_t)n_off * B[p].pitch; B2[p].lo += b_mn ? (size_t)n_off : (size_t)n_off * B[p].pitch;
+      B2[p].hi = ahead(B[p].hi, bo); B2[p].lo = ahead(B[p].lo, bo);
+      if (f16) { B2[p].scale += (size_t)n_off * B[p].scale_step; }
     }
     GemmEpilogue e2 = epi;
     e2.C += m_off + (size_t)epi.ldc * n_off;
@@ -1093,9 +1366,9 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   }
   {
     // times the MMA kernel (and the split-K reduction); the packing launches show up in the step time
-    GemmProfScope scope(ctx, flops, 1, M, N, kb_total * BK, (uint32_t)epi.mode);
-    if (bn == 64) dyb_launch(k_gemm_tc<64, false>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb0, kb1, kb_per_split, kepi, ctx->dev_flags);
-    else dyb_launch(k_gemm_tc<128, false>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb0, kb1, kb_per_split, kepi, ctx->dev_flags);
+    GemmProfScope scope(ctx, flops, 1, M, N, kb_total * el, (uint32_t)epi.mode);
+    auto kern = f16 ? (bn == 64 ? k_gemm_tc<64, false, true> : k_gemm_tc<128, false, true>) : (bn == 64 ? k_gemm_tc<64, false> : k_gemm_tc<128, false>);
+    dyb_launch(kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb0, kb1, kb_per_split, kepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);
     if (S > 1 && epi.mode == EPI_LSTM_CELL) {
       dyb_launch(k_splitk_reduce_cell, stream_grid(ctx, (size_t)M / 16 * N + 1, 256), 256, 0, ctx, part, S, M, N, epi);
@@ -1147,6 +1420,24 @@ int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const Ge
   for (int p = 0; p < npairs; ++p) if (pairs[p].K == 0) return DYB200_OK;
   *handled = 1;
   PackedOp A[2], B[2];
+  if (npairs == 1 && !pairs[0].maskB && flops >= kF16Flops) {
+    // Both operands as they lie: lines are rows of a K-major operand (A transposed / B not), or k of an MN-major one.  Rows have
+    // their own scale; a parameter has one, so that one set of planes serves this product and the one that uses it transposed.
+    const GemmPair& g = pairs[0];
+    const bool a_mn = g.transA == 0, b_mn = g.transB != 0;
+    F16Jobs jobs;
+    F16Job ja, jb;
+    int rc;
+    jobs.n = 0;
+    if (g.a_is_param) rc = dyb200_f16_param(ctx, g.A, g.lda, a_mn ? g.K : M, a_mn ? M : g.K, &ja);
+    else if (!(rc = dyb200_f16_planes(ctx, g.A, g.lda, a_mn ? g.K : M, a_mn ? M : g.K, a_mn ? F16_ELEM : F16_LINE, &ja))) jobs.job[jobs.n++] = ja;
+    if (rc) return rc;
+    if ((rc = dyb200_f16_planes(ctx, g.B, g.ldb, b_mn ? g.K : N, b_mn ? N : g.K, b_mn ? F16_ELEM : F16_LINE, &jb))) return rc;
+    jobs.job[jobs.n++] = jb;
+    if ((rc = dyb200_f16_pack(ctx, &jobs))) return rc;
+    A[0] = dyb200_f16_op(ja, a_mn); B[0] = dyb200_f16_op(jb, b_mn);
+    return dyb200_tc_gemm_packed(ctx, M, N, 1, A, B, epi);
+  }
   PackJobs batch;   // all operands that need packing go out in one launch
   dyb200_tc_pack_begin(&batch);
   for (int p = 0; p < npairs; ++p) {

@@ -409,12 +409,17 @@ struct ChunkOfPart {   // f(r, b) = v[r + n * b]
   __device__ float operator()(size_t r, uint32_t b) const { return v[r + n * (size_t)b]; }
 };
 
+// F16: the planes are scaled fp16 pairs (half the bytes); |d| <= |dz|, so the scale word is that of the largest |dz|.
+template <bool F16>
 __global__ void __launch_bounds__(256) k_softmax_bwd_split(const float* __restrict__ x, const float* __restrict__ z,
                                                            const float* __restrict__ dz, const uint32_t* __restrict__ ids,
                                                            uint32_t rows, uint32_t ncols, float* __restrict__ bh,
                                                            float* __restrict__ bl, uint32_t pitch_b,
-                                                           float* __restrict__ colsum_part, int vec_in) {
+                                                           float* __restrict__ colsum_part, int vec_in, const uint32_t* __restrict__ scale_word) {
   dyb_grid_dep_sync();
+  const float sc = F16 ? scale_of(__ldg(scale_word)) : 1.f;
+  __half* const hh = reinterpret_cast<__half*>(bh);
+  __half* const hl = reinterpret_cast<__half*>(bl);
   __shared__ float tile[64][65];   // [column][row]
   const uint32_t r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
   {
@@ -437,10 +442,17 @@ __global__ void __launch_bounds__(256) k_softmax_bwd_split(const float* __restri
             const uint32_t k = pick - r;
             if (k == 0) d.x -= dc; else if (k == 1) d.y -= dc; else if (k == 2) d.z -= dc; else d.w -= dc;
           }
-          float4 h, l;
-          split_tf32(d.x, h.x, l.x); split_tf32(d.y, h.y, l.y); split_tf32(d.z, h.z, l.z); split_tf32(d.w, h.w, l.w);
-          st4(bh + (size_t)c * pitch_b + r, h);
-          st4(bl + (size_t)c * pitch_b + r, l);
+          if (F16) {
+            __half h[4], l[4];
+            split_f16(d.x * sc, h[0], l[0]); split_f16(d.y * sc, h[1], l[1]); split_f16(d.z * sc, h[2], l[2]); split_f16(d.w * sc, h[3], l[3]);
+            *reinterpret_cast<uint2*>(hh + (size_t)c * pitch_b + r) = *reinterpret_cast<const uint2*>(h);
+            *reinterpret_cast<uint2*>(hl + (size_t)c * pitch_b + r) = *reinterpret_cast<const uint2*>(l);
+          } else {
+            float4 h, l;
+            split_tf32(d.x, h.x, l.x); split_tf32(d.y, h.y, l.y); split_tf32(d.z, h.z, l.z); split_tf32(d.w, h.w, l.w);
+            st4(bh + (size_t)c * pitch_b + r, h);
+            st4(bl + (size_t)c * pitch_b + r, l);
+          }
         } else {        // same arithmetic as its scalar path
           float e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -448,10 +460,9 @@ __global__ void __launch_bounds__(256) k_softmax_bwd_split(const float* __restri
             if (r + k < rows) {
               e[k] = expf(xc[r + k] - zc) * dc;
               if (r + k == pick) e[k] -= dc;
-              float h, l;
-              split_tf32(e[k], h, l);
-              bh[(size_t)c * pitch_b + r + k] = h;
-              bl[(size_t)c * pitch_b + r + k] = l;
+              const size_t o = (size_t)c * pitch_b + r + k;
+              if (F16) split_f16(e[k] * sc, hh[o], hl[o]);
+              else split_tf32(e[k], bh[o], bl[o]);
             }
           }
           d = make_float4(e[0], e[1], e[2], e[3]);
@@ -791,28 +802,51 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
   }
   int rc;
   PackedOp dA, dB, hT, RT;
-  if ((rc = dyb200_tc_planes(ctx, n, V, &dB))) return rc;   // rows = columns, reduction over the vocabulary
-  dA = dB; dA.rows = V; dA.K = n; dA.mn_major = 1;           // the same planes read with the vocabulary as rows
+  const bool f16 = flops >= kF16Flops;   // fp16 pairs, as for the single products
   const dim3 grid((V + 63) / 64, (n + 63) / 64);
+  DYB_CHECK_ARG(ctx, grid.y <= 65535u, "softmax_output_bwd_fused: too many columns (%u)", n);
   void* part;
   if ((rc = dyb200_scratch(ctx, (size_t)grid.y * V * sizeof(float), &part))) return rc;
   const int vec_in = V % 4 == 0 && aligned16(x->v);
-  DYB_CHECK_ARG(ctx, grid.y <= 65535u, "softmax_output_bwd_fused: too many columns (%u)", n);
-  dyb_launch(k_softmax_bwd_split, grid, 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, dB.hi, dB.lo, dB.pitch,
-             (float*)part, vec_in);
+  if (f16) {
+    F16Jobs jobs;
+    jobs.n = 1;
+    F16Job& jd = jobs.job[0];
+    if ((rc = dyb200_f16_planes(ctx, dEdf->v, n, n, V, F16_ALL, &jd))) return rc;   // lines = columns of x, positions = vocabulary
+    dB = dyb200_f16_op(jd, false);
+    dA = dyb200_f16_op(jd, true);
+    jd.lines = 1; jd.n = n;                                                          // (the scale word: over dE/df)
+    if ((rc = dyb200_f16_absmax(ctx, jobs))) return rc;
+    dyb_launch(k_softmax_bwd_split<true>, grid, 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, dB.hi, dB.lo, dB.pitch, (float*)part, vec_in, dB.scale);
+    // R as H lines of V values, h as n lines of H values
+    F16Job jr, jh;
+    jobs.n = 0;
+    if (flags & DYB200_GEMM_A_IS_PARAM) rc = dyb200_f16_param(ctx, R->v, V, H, V, &jr);
+    else if (!(rc = dyb200_f16_planes(ctx, R->v, V, H, V, F16_LINE, &jr))) jobs.job[jobs.n++] = jr;
+    if (rc || (rc = dyb200_f16_planes(ctx, h->v, H, n, H, F16_ELEM, &jh))) return rc;
+    jobs.job[jobs.n++] = jh;
+    if ((rc = dyb200_f16_pack(ctx, &jobs))) return rc;
+    RT = dyb200_f16_op(jr, false);
+    hT = dyb200_f16_op(jh, true);
+  } else {
+    if ((rc = dyb200_tc_planes(ctx, n, V, &dB))) return rc;   // rows = columns, reduction over the vocabulary
+    dA = dB; dA.rows = V; dA.K = n; dA.mn_major = 1;           // the same planes read with the vocabulary as rows
+    dyb_launch(k_softmax_bwd_split<false>, grid, 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, dB.hi, dB.lo, dB.pitch, (float*)part, vec_in, nullptr);
+    // h split as it lies (row = column, H values), read MN-major
+    if ((rc = dyb200_tc_pack(ctx, h->v, H, true, n, H, nullptr, 0, 0, &hT, nullptr))) return rc;
+    hT.rows = H; hT.K = n; hT.mn_major = 1;
+    if (flags & DYB200_GEMM_A_IS_PARAM) rc = dyb200_tc_param(ctx, R->v, V, true, H, V, &RT);
+    else rc = dyb200_tc_pack(ctx, R->v, V, true, H, V, nullptr, 0, 0, &RT, nullptr);
+    if (rc) return rc;
+  }
   DYB_LAUNCHED(ctx);
   if ((rc = batch_reduce_add(ctx, ChunkOfPart{(const float*)part, V}, V, grid.y, db->v))) return rc;   // db += sum over column tiles
-  // dR += d h^T : M = V, N = H, K = n; both operands MN-major (h split as it lies: row = column, H values)
-  if ((rc = dyb200_tc_pack(ctx, h->v, H, true, n, H, nullptr, 0, 0, &hT, nullptr))) return rc;
-  hT.rows = H; hT.K = n; hT.mn_major = 1;
+  // dR += d h^T : M = V, N = H, K = n; both operands MN-major
   {
     GemmEpilogue e{EPI_ACCUM, dR->v, V, nullptr, 0, 0.f, nullptr, 0, 0};
     if ((rc = dyb200_tc_gemm_packed(ctx, V, H, 1, &dA, &hT, e))) return rc;
   }
   // dh += R^T d : M = H, N = n, K = V
-  if (flags & DYB200_GEMM_A_IS_PARAM) rc = dyb200_tc_param(ctx, R->v, V, true, H, V, &RT);
-  else rc = dyb200_tc_pack(ctx, R->v, V, true, H, V, nullptr, 0, 0, &RT, nullptr);
-  if (rc) return rc;
   GemmEpilogue e{EPI_ACCUM, dh->v, H, nullptr, 0, 0.f, nullptr, 0, 0};
   return dyb200_tc_gemm_packed(ctx, H, n, 1, &RT, &dB, e);
 }

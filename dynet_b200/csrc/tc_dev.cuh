@@ -3,6 +3,7 @@
 // 12 MMAs of a k-block, and the cooperative epilogue pass over a tile parked in shared memory.
 #pragma once
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <math.h>
 
 #include "gemm.cuh"
@@ -22,13 +23,16 @@ constexpr uint32_t kTmemCols = 256;       // two 128-column accumulators, used a
 // zero); chains of 8 k-blocks 8.7e-6 at both, against 2.6e-6 .. 9.3e-6 for cuBLAS SGEMM.  Each flush costs about
 // 0.4 us of tensor-pipe time (4 % at this setting).
 constexpr uint32_t kChunkKB = 8;
+constexpr uint32_t kChunkF16 = 16;        // F16 products: k-blocks are 64 wide
 constexpr uint32_t kEpiWarps = 8;
 
 // pair p: t[4p] = A_hi, A_lo, B_hi, B_lo.  a_mn != 0 (one pair only): the A planes are MN-major - element (m, k) at
 // plane[k * pitch + m], the layout of a K x M row-major matrix - and t[0], t[1] are 3-D maps over (m within a group of 32,
 // k, group) with a box of 32 x 32 x 4; see load_a_tile / umma_desc_mn.  b_mn: the same for the B planes (t[2], t[3]; the
 // box holds as many groups as the tile has columns / 32).
-struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; };
+// F16 products (see "2 x 11 bits" in gemm.cuh): sa / sb are the operands' scale words, one per row (step 1) or one for all (step 0).
+struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; const uint32_t *sa, *sb; uint32_t sa_step, sb_step;
+  uint32_t store_map; };   // store_map: t[4] describes the output (persistent kernel, plain stores; one pair)
 
 // The k-blocks of K split z of S: [b0, b0 + n0) of pair 0, then [b1, b1 + n1) of pair 1 (each pair cut into S equal shares).
 struct KSplit { uint32_t b0, n0, b1, n1; };
@@ -100,20 +104,30 @@ __device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr) {
   return d;
 }
 // One plane of the A tile (m0 .., k-block kblk) into `st`: one box of 16 KB in either layout (MN-major: the box's innermost
-// extent is one 128-byte swizzle span = 32 m, its outermost the four groups of the tile).  k rows past the plane's extent
-// arrive as zeros.
+// extent is one 128-byte swizzle span = EL rows, its outermost the groups of the tile).  EL = elements per 128 bytes (32, F16: 64),
+// also the width of a k-block.  k rows past the plane's extent arrive as zeros.
+template <int EL = 32>
 __device__ __forceinline__ void load_a_tile(unsigned char* st, const CUtensorMap* map, uint64_t* bar, uint32_t kblk, uint32_t m0,
                                             uint32_t a_mn) {
-  if (a_mn) {
-    tma_load_3d(st, map, bar, 0, (int)(kblk * 32), (int)(m0 / 32));
-  } else {
-    tma_load_2d(st, map, bar, (int)(kblk * 32), (int)m0);
-  }
+  if (a_mn) tma_load_3d(st, map, bar, 0, (int)(kblk * EL), (int)(m0 / EL));
+  else tma_load_2d(st, map, bar, (int)(kblk * EL), (int)m0);
 }
+template <int EL = 32>
 __device__ __forceinline__ void load_b_tile(unsigned char* st, const CUtensorMap* map, uint64_t* bar, uint32_t kblk, uint32_t n0,
                                             uint32_t b_mn) {
-  if (b_mn) tma_load_3d(st, map, bar, 0, (int)(kblk * 32), (int)(n0 / 32));
-  else tma_load_2d(st, map, bar, (int)(kblk * 32), (int)n0);
+  if (b_mn) tma_load_3d(st, map, bar, 0, (int)(kblk * EL), (int)(n0 / EL));
+  else tma_load_2d(st, map, bar, (int)(kblk * EL), (int)n0);
+}
+// MN-major F16 tile: groups of 64 rows (128 bytes) x 64 k, 8192 bytes apart, in the plain 128-byte swizzle (8 k per 1024-byte
+// atom); one MMA (k = 16) advances the start address by 2048 bytes.
+__device__ __forceinline__ uint64_t umma_desc_mn16(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
+  d |= (uint64_t)(8192 >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -163,6 +177,27 @@ __device__ __forceinline__ void issue_kblock(uint32_t acc, uint64_t a_hi, uint64
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], xa, yb, %5, pt;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], xa, ya, %5, pt;\n\t}"
       ::"r"(acc), "l"(a_hi), "l"(a_lo), "l"(b_hi), "l"(b_lo), "r"(idesc), "r"(accumulate), "l"(a_step), "l"(b_step)
+      : "memory");
+}
+
+// One 64-wide k-block of an F16 product: 4 k steps of A_hi x [B_hi | B_lo] -> acc (2 x columns) and A_lo x B_hi -> acc2, its upper half.
+__device__ __forceinline__ void issue_kblock_f16(uint32_t acc, uint32_t acc2, uint64_t a_hi, uint64_t a_lo, uint64_t b, uint32_t idesc_wide,
+                                                 uint32_t idesc, uint32_t accumulate, uint64_t a_step, uint64_t b_step) {
+  asm volatile(
+      "{\n\t.reg .pred pf, pt;\n\t.reg .b64 xa, xl, yb;\n\t"
+      "setp.ne.b32 pf, %7, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %2, %4, %5, pf;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], %3, %4, %6, pt;\n\t"
+      "add.s64 xa, %2, %8;\n\tadd.s64 xl, %3, %8;\n\tadd.s64 yb, %4, %9;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], xa, yb, %5, pt;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], xl, yb, %6, pt;\n\t"
+      "add.s64 xa, xa, %8;\n\tadd.s64 xl, xl, %8;\n\tadd.s64 yb, yb, %9;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], xa, yb, %5, pt;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], xl, yb, %6, pt;\n\t"
+      "add.s64 xa, xa, %8;\n\tadd.s64 xl, xl, %8;\n\tadd.s64 yb, yb, %9;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], xa, yb, %5, pt;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], xl, yb, %6, pt;\n\t}"
+      ::"r"(acc), "r"(acc2), "l"(a_hi), "l"(a_lo), "l"(b), "r"(idesc_wide), "r"(idesc), "r"(accumulate), "l"(a_step), "l"(b_step)
       : "memory");
 }
 

@@ -119,7 +119,8 @@ size_t plan(const dyb200h_lm_config& c, Lm* m, char* base, size_t size) {
   float* dh = a.take<float>(TL * HB);
   float* dc = a.take<float>(TL * HB);
   float* dgates = a.take<float>(TL * GB);
-  size_t d1 = a.off;
+  // (the fused driver never stores the gate gradients in fp32: their part is not cleared)
+  size_t d1 = c.fused ? (size_t)((char*)dgates - base) : a.off;
   if (m) {
     m->tok = tok; m->x = x; m->gates = gates; m->cs = cs; m->hs = hs; m->r = r; m->aux = aux; m->errs = errs;
     m->zeros = zeros; m->ones = ones; m->scalars = scalars; m->dr = dr; m->dx = dx; m->dh = dh; m->dc = dc; m->dgates = dgates;
