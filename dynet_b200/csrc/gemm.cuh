@@ -104,6 +104,9 @@ bool dyb200_thin_columns(uint32_t M, uint32_t N, uint32_t K);
 bool dyb200_thin_takes(uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi);
 int dyb200_gemm_thin(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi);
 int dyb200_lstm_thin(dyb200_ctx* ctx, uint32_t H, uint32_t B, int npairs, const GemmPair* pairs, int pre_in_gates, const GemmEpilogue& epi);
+// fp32 path for products with a narrow side and a long one (gemm_narrow.cu).
+bool dyb200_narrow_takes(uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi);
+int dyb200_gemm_narrow(dyb200_ctx* ctx, uint32_t M, uint32_t N, const GemmPair& p, const GemmEpilogue& epi);
 // 3xTF32 tensor-pipe path (tcgen05 + TMEM + TMA); returns DYB200_ERUNTIME with *handled = 0
 // when the shape/alignment is outside what it supports.
 int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi,

@@ -111,6 +111,7 @@ int dyb200_gemm_fused(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const
   double flops = 0;
   for (int p = 0; p < npairs; ++p) flops += 2.0 * M * N * pairs[p].K;
   if (M && N && dyb200_thin_takes(M, N, npairs, pairs, epi)) return dyb200_gemm_thin(ctx, M, N, npairs, pairs, epi);
+  if (M && N && dyb200_narrow_takes(M, N, npairs, pairs, epi)) return dyb200_gemm_narrow(ctx, M, N, pairs[0], epi);
   int handled = 0;
   int rc = dyb200_gemm_tc(ctx, M, N, npairs, pairs, epi, &handled);
   if (handled) return rc;

@@ -659,11 +659,17 @@ __global__ void __launch_bounds__(256) k_pack_multi(const PackJobs jobs) {
   const int mask_full = job.mask_full;
   const uint32_t mask_period = job.mask_period;
   if (job.k_is_fast) {
-    const uint32_t r = unit / job.gx, bx = unit % job.gx;
-    const uint32_t mr = mask_period ? r % mask_period : r;   // batch column of the mask
     if (job.vec) {
-      const uint32_t k = (bx * 256 + threadIdx.x) * 4;
-      if (k < K) {
+      // rows end to end, 1024 float4 per CTA whatever their length: a CTA for each row of 256 values (64 of its threads at work)
+      // took 111 us for 107 000 rows
+      const uint32_t K4 = K / 4;
+      const uint64_t e0 = (uint64_t)unit * 1024;
+      const uint32_t first = (uint32_t)(e0 / K4), rem = (uint32_t)(e0 - (uint64_t)first * K4);
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t e = rem + 256 * i + threadIdx.x, r = first + e / K4, k = 4 * (e % K4);
+        if (r >= rows) break;
+        const uint32_t mr = mask_period ? r % mask_period : r;   // batch column of the mask
         float4 v = ld4(src + k + (size_t)ld * r);
         if (mask) {
           float4 mk = ld4(mask + k + (mask_full ? (size_t)mask_ld * mr : 0));
@@ -675,6 +681,7 @@ __global__ void __launch_bounds__(256) k_pack_multi(const PackJobs jobs) {
         st4(lo + k + (size_t)pitch * r, l);
       }
     } else {
+      const uint32_t r = unit / job.gx, bx = unit % job.gx, mr = mask_period ? r % mask_period : r;
       for (uint32_t k = bx * 1024 + threadIdx.x; k < min(K, (bx + 1) * 1024); k += 256) {
         float v = src[k + (size_t)ld * r];
         if (mask) v *= mask[k + (mask_full ? (size_t)mask_ld * mr : 0)];
@@ -902,7 +909,7 @@ int pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int layout, uint32_t ro
   if (k_is_fast) {
     j.vec = (K % 4 == 0) && (ld % 4 == 0) && aligned16(src) && (!mask || ((mask_ld % 4 == 0 || !mask_full) && aligned16(mask)));
     j.gx = (K + 1023) / 1024;
-    units = (uint64_t)j.gx * rows;
+    units = j.vec ? ((uint64_t)(K / 4) * rows + 1023) / 1024 : (uint64_t)j.gx * rows;
   } else {
     j.vec = 0;
     j.gx = (rows + 31) / 32;
