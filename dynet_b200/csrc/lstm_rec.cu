@@ -33,45 +33,14 @@
 #include "gemm.cuh"
 #include "lstm_cell.cuh"
 #include "lstm_rec_api.h"
+#include "lstm_rec_dev.cuh"
 
 namespace {
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ float xor_add(float keep, float send, int m) { return keep + __shfl_xor_sync(0xffffffffu, send, m); }
 
 // columns of cluster g that are active at a step of width B: those i with g + G i < B
 __device__ __forceinline__ uint32_t active_cols(uint32_t B, uint32_t g, uint32_t G) { return B > g ? (B - g + G - 1) / G : 0; }
-
-// One mbarrier per buffer parity: `bytes` of st.async messages complete its phase.
-__device__ __forceinline__ void msg_init(uint64_t* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void msg_expect(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool msg_wait(uint64_t* bar, uint32_t parity) {   // bounded
-  for (uint32_t it = 0; it < (1u << 20); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-// 16 bytes into a CTA's shared memory, counted by its mbarrier (both addresses shared::cluster)
-__device__ __forceinline__ void send4(uint32_t addr, float4 v, uint32_t bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(v.x), "f"(v.y),
-               "f"(v.z), "f"(v.w), "r"(bar) : "memory");
-}
 
 // grid (C, G, directions), cluster (C, 1, 1); block = 8 U threads.
 // Dynamic shared memory: h[2][ncap][16 KD], c[ncap][U].  NB columns per block, NF of them computed (3 of 4, or all).
@@ -519,13 +488,13 @@ typedef void (*BwdKernel)(RecBwd);
 // 45 columns on the 15 clusters of 8 CTAs that fit.)
 FwdKernel fwd_kernel(uint32_t kd, uint32_t n) {
 #define REC_F4(K) n == 1 ? k_lstm_rec_fwd<K, 1> : n == 2 ? k_lstm_rec_fwd<K, 2> : n == 3 ? k_lstm_rec_fwd<K, 4, 3>
-#define REC_F(K) (REC_F4(K) : n == 4 ? k_lstm_rec_fwd<K, 4> : k_lstm_rec_fwd<K, 8>)
+#define REC_F(K) (REC_F4(K) : k_lstm_rec_fwd<K, 4>)
   switch (kd) {
     case 4: return REC_F(4);
     case 8: return REC_F(8);
     case 12: return REC_F(12);
     case 16: return REC_F(16);
-    case 20: return REC_F4(20) : k_lstm_rec_fwd<20, 4>;
+    case 20: return REC_F(20);
     default: return n == 1 ? k_lstm_rec_fwd<24, 1> : k_lstm_rec_fwd<24, 2>;
   }
 #undef REC_F
@@ -551,8 +520,10 @@ size_t fwd_smem(const RecPlan& p, uint32_t ncap) {
   return cols > weights ? cols : weights;
 }
 
-int launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, dim3 grid, uint32_t threads, size_t smem) {
-  DYB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRecSmemMax));
+}  // namespace
+
+int dyb200_rec_launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, dim3 grid, uint32_t threads, size_t smem) {
+  DYB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (grid.x > 8) DYB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   memset(cfg, 0, sizeof(*cfg));
   cfg->gridDim = grid; cfg->blockDim = dim3(threads, 1, 1); cfg->dynamicSmemBytes = smem; cfg->stream = ctx->stream;
@@ -561,14 +532,16 @@ int launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cud
   cfg->attrs = attr; cfg->numAttrs = 1;
   return DYB200_OK;
 }
+namespace {
+
 // How many clusters run side by side (remembered per context and width class): the columns are dealt out over that many.
 int clusters_that_fit(dyb200_ctx* ctx, const RecPlan& p, bool bwd, uint32_t threads) {
   int16_t& fit = ctx->rec_fit[bwd][p.KD / 4 - 1][p.C];
   if (fit == 0) {
-    const void* k = bwd ? (const void*)bwd_kernel(p.KD2, 4) : (const void*)fwd_kernel(p.KD, 8);
+    const void* k = bwd ? (const void*)bwd_kernel(p.KD2, 4) : (const void*)fwd_kernel(p.KD, 4);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    if (launch_cfg(ctx, k, &cfg, attr, dim3(p.C, 1, 1), threads, kRecSmemMax)) return -1;
+    if (dyb200_rec_launch_cfg(ctx, k, &cfg, attr, dim3(p.C, 1, 1), threads, kRecSmemMax)) return -1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
     fit = (int16_t)(n > 0 ? n : -1);
@@ -594,17 +567,23 @@ bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan*
   p.KD = (H + 63) / 64 * 4;
   p.KD2 = p.U <= 16 ? 8 : p.U <= 24 ? 12 : 16;
   const int ff = clusters_that_fit(ctx, p, false, fwd_threads(p)), fb = clusters_that_fit(ctx, p, true, bwd_threads(p));
-  if (ff <= 0 || fb <= 0 || !deal_columns(N, ff, ndir, fwd_col_bytes(p), &p.Gf, &p.ncapf) || !deal_columns(N, fb, ndir, bwd_col_bytes(p), &p.Gb, &p.ncapb)) return false;
+  const bool sf = ff > 0 && deal_columns(N, ff, ndir, fwd_col_bytes(p), &p.Gf, &p.ncapf), sb = fb > 0 && deal_columns(N, fb, ndir, bwd_col_bytes(p), &p.Gb, &p.ncapb);
+  // More than four columns per cluster: the tensor pipe, where the width lets it (256 units, a step: 1.8 us here at 3 columns,
+  // 8.0 at 37; there KERNEL_STEP_US up to 48)
+  p.tcf = !(sf && (N + p.Gf - 1) / p.Gf <= 4) && dyb200_rec_tc_plan(ctx, false, H, N, ndir, &p.tf);
+  p.tcb = !(sb && (N + p.Gb - 1) / p.Gb <= 4) && dyb200_rec_tc_plan(ctx, true, H, N, ndir, &p.tb);
+  if (!(sf || p.tcf) || !(sb || p.tcb)) return false;
   *out = p;
   return true;
 }
 
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
+  if (p.tcf) return dyb200_rec_tc_fwd(ctx, p.tf, a, ndir);
   a->U = p.U; a->G = p.Gf; a->ncap = p.ncapf; a->flags = ctx->dev_flags;
   FwdKernel k = fwd_kernel(p.KD, (a->N + p.Gf - 1) / p.Gf);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  int rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gf, ndir), fwd_threads(p), fwd_smem(p, p.ncapf));
+  int rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gf, ndir), fwd_threads(p), fwd_smem(p, p.ncapf));
   if (rc) return rc;
   cudaLaunchKernelEx(&cfg, k, *a);
   DYB_LAUNCHED(ctx);
@@ -612,20 +591,24 @@ int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
 }
 
 int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db) {
-  a->U = p.U; a->G = p.Gb; a->ncap = p.ncapb; a->flags = ctx->dev_flags;
-  const uint32_t rows = 4 * a->H;
+  const uint32_t rows = 4 * a->H, G = p.tcb ? p.tb.G : p.Gb;
+  a->U = p.U; a->G = G; a->ncap = p.ncapb; a->flags = ctx->dev_flags;
   void* part;
-  int rc = dyb200_scratch(ctx, (size_t)ndir * p.Gb * rows * sizeof(float), &part);
+  int rc = dyb200_scratch(ctx, (size_t)ndir * G * rows * sizeof(float), &part);
   if (rc) return rc;
-  for (int k = 0; k < ndir; ++k) a->d[k].dbpart = (float*)part + (size_t)k * p.Gb * rows;
-  BwdKernel k = bwd_kernel(p.KD2, (a->N + p.Gb - 1) / p.Gb);
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  rc = launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gb, ndir), bwd_threads(p), p.ncapb * bwd_col_bytes(p));
-  if (rc) return rc;
-  cudaLaunchKernelEx(&cfg, k, *a);
-  DYB_LAUNCHED(ctx);
-  dyb_launch(k_rec_db, dim3((rows + 255) / 256, ndir), 256, 0, ctx, (const float*)a->d[0].dbpart, (const float*)a->d[ndir - 1].dbpart, p.Gb, rows,
+  for (int k = 0; k < ndir; ++k) a->d[k].dbpart = (float*)part + (size_t)k * G * rows;
+  if (p.tcb) {
+    if ((rc = dyb200_rec_tc_bwd(ctx, p.tb, a, ndir))) return rc;
+  } else {
+    BwdKernel k = bwd_kernel(p.KD2, (a->N + p.Gb - 1) / p.Gb);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gb, ndir), bwd_threads(p), p.ncapb * bwd_col_bytes(p));
+    if (rc) return rc;
+    cudaLaunchKernelEx(&cfg, k, *a);
+    DYB_LAUNCHED(ctx);
+  }
+  dyb_launch(k_rec_db, dim3((rows + 255) / 256, ndir), 256, 0, ctx, (const float*)a->d[0].dbpart, (const float*)a->d[ndir - 1].dbpart, G, rows,
              db[0], db[ndir - 1]);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;

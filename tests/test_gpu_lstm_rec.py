@@ -1,4 +1,4 @@
-"""The cluster-resident recurrence (csrc/lstm_rec.cu) behind the sequence calls, for layers up to 384 units and sequences of at
+"""The cluster-resident recurrence (csrc/lstm_rec.cu, csrc/lstm_rec_tc.cu) behind the sequence calls, for layers up to 384 units and sequences of at
 least 8 steps: gates, states, every gradient and the weight gradients against the oracle's node chain.  Shapes at the edges of
 its tiling: widths that are no multiple of 4, 8 or 32, one CTA / a portable cluster / a 16-CTA cluster, one column, as many
 columns as its clusters carry, batch-1 masks."""
@@ -57,6 +57,14 @@ def _oracle(oracle, x, h0, c0, Wx, Wh, b, mx, mh, up):
     (48, 384, 130, 8, None),         # the widest layer, several columns per cluster
     (16, 64, 700, 8, "full"),        # many columns per cluster
     (16, 384, 280, 8, "full"),       # the most columns its clusters carry, or nearly
+    # on the tensor pipe (csrc/lstm_rec_tc.cu)
+    (24, 256, 70, 9, "full"),        # five columns per cluster
+    (24, 256, 301, 8, None),         # twenty-one
+    (16, 250, 500, 8, "full"),       # three groups of columns forward; backward more blocks than clusters; a last CTA with 26 units
+    (16, 225, 1001, 8, "one"),       # more blocks than clusters both ways; a last CTA with one unit
+    (16, 130, 600, 8, None),         # five CTAs, two row tiles
+    (16, 97, 1500, 9, "full"),       # four CTAs, one row tile, the second block of the reduction nearly empty
+    (8, 31, 3000, 8, None),          # one CTA
 ])
 def test_recurrence_matches_oracle(oracle, g, I, H, B, T, mask):
     import torch
@@ -100,12 +108,12 @@ def test_recurrence_matches_oracle(oracle, g, I, H, B, T, mask):
     assert_close(g.host(db), want[7], TOL_REDUCE, floor=float(np.abs(want[7]).max()) * 0.02, what="db")
 
 
-def test_recurrence_is_the_same_every_time(g):
-    """Widths whose warps and CTAs finish unevenly (a last CTA with two units, nine warps per CTA), many columns: twelve passes over
-    the same inputs give the same bits."""
+@pytest.mark.parametrize("I,H,B,T", [(45, 262, 372, 19), (45, 230, 777, 19)])
+def test_recurrence_is_the_same_every_time(g, I, H, B, T):
+    """Widths whose warps and CTAs finish unevenly (a last CTA with two or six units, nine warps per CTA), many columns: twelve passes
+    over the same inputs give the same bits."""
     import torch
     from dynet_b200 import capi
-    I, H, B, T = 45, 262, 372, 19
     gen = torch.Generator("cuda").manual_seed(5)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
     x, Wx, Wh, b, up = rnd(T * B, I), rnd(I, 4 * H) * 0.05, rnd(H, 4 * H) * 0.05, rnd(4 * H) * 0.1, rnd(T * B, H)

@@ -193,7 +193,8 @@ def _split(lens, words, tags):
             [[int(v) for v in tags[off[s]:off[s + 1]]] for s in range(len(lens))])
 
 
-@pytest.mark.parametrize("dims,S,lo,hi", [((50, 16, 8, 6, 5), 7, 1, 6), ((2000, 128, 256, 32, 45), 48, 5, 30)])
+@pytest.mark.parametrize("dims,S,lo,hi", [((50, 16, 8, 6, 5), 7, 1, 6), ((2000, 128, 256, 32, 45), 48, 5, 30),
+                                          ((400, 24, 200, 8, 9), 350, 1, 14)])   # (the last: more blocks of sentences than clusters)
 def test_tagger_driver_matches_per_sentence_oracle(oracle, dims, S, lo, hi):
     """The C++ driver (autobatched schedule, deferred weight-gradient products, folded embedding scatter) against the oracle
     running every sentence on its own: loss and all 12 gradient tensors, every row at its own scale.  Two passes in a row:
