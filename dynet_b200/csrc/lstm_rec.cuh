@@ -16,7 +16,7 @@ struct RecDirF {
 struct RecFwd {
   RecDirF d[2];
   uint32_t H, U, T, N, G, ncap, hn_pitch;
-  uint32_t ndir, contiguous;   // lstm_rec_tc.cu: directions in the grid; whether a cluster's columns are neighbours or every G-th
+  uint32_t ndir;   // directions in the grid of lstm_rec_tc.cu, whose clusters take blocks of ncap neighbouring columns (lstm_rec.cu: every G-th)
   int mask_full;
   float fb;
   const uint32_t* prefix;   // device, T + 1 entries: step t has the columns [prefix[t], prefix[t + 1]), widths never grow (null: N each)
@@ -34,14 +34,14 @@ struct RecDirB {
 struct RecBwd {
   RecDirB d[2];
   uint32_t H, U, T, N, G, ncap, dn_pitch;
-  uint32_t ndir, contiguous;
+  uint32_t ndir;
   int mask_full;
   const uint32_t* prefix;
   uint32_t* flags;
 };
 
-// lstm_rec_tc.cu: columns per cluster / 16, blocks of columns per direction, neighbours or every G-th.
-struct RecTcPlan { uint32_t nch, G, contiguous; };
+// lstm_rec_tc.cu: columns per cluster / 16, blocks of columns per direction.
+struct RecTcPlan { uint32_t nch, G; };
 // U hidden units per CTA, C CTAs per cluster, KD / KD2 = reduction elements per lane, G clusters per direction, room for ncap
 // columns per cluster (forward, backward).  tcf / tcb: the pass runs on the tensor pipe.
 struct RecPlan { uint32_t U, C, KD, KD2, Gf, Gb, ncapf, ncapb; bool tcf, tcb; RecTcPlan tf, tb; };
