@@ -16,7 +16,7 @@ struct RecDirF {
 struct RecFwd {
   RecDirF d[2];
   uint32_t H, U, T, N, G, ncap, hn_pitch;
-  uint32_t ndir;   // directions in the grid of lstm_rec_tc.cu, whose clusters take blocks of ncap neighbouring columns (lstm_rec.cu: every G-th)
+  uint32_t ndir;   // directions in the grid of lstm_rec_tc.cu, whose groups take neighbouring columns (lstm_rec.cu: every G-th)
   int mask_full;
   float fb;
   const uint32_t* prefix;   // device, T + 1 entries: step t has the columns [prefix[t], prefix[t + 1]), widths never grow (null: N each)
@@ -40,18 +40,18 @@ struct RecBwd {
   uint32_t* flags;
 };
 
-// lstm_rec_tc.cu: columns per cluster / 16, blocks of columns per direction.
+// lstm_rec_tc.cu: columns per group / 16, clusters per direction.
 struct RecTcPlan { uint32_t nch, G; };
 // U hidden units per CTA, C CTAs per cluster, KD / KD2 = reduction elements per lane, G clusters per direction, room for ncap
 // columns per cluster (forward, backward).  tcf / tcb: the pass runs on the tensor pipe.
 struct RecPlan { uint32_t U, C, KD, KD2, Gf, Gb, ncapf, ncapb; bool tcf, tcb; RecTcPlan tf, tb; };
 // False when the width is outside what the registers of a cluster hold, or N columns are more than the clusters can carry.
-bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan* out);
+bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, bool ragged, RecPlan* out);
 // ndir directions (1 or 2) share T, N and prefix.  U, G, ncap and flags are filled in here.
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir);
 // db[dir] (4H) += row sums of dgates over all columns (partial sums in scratch memory).
 int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db);
 int dyb200_rec_launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, dim3 grid, uint32_t threads, size_t smem);
-bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int ndir, RecTcPlan* out);
+bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int ndir, bool ragged, RecTcPlan* out);
 int dyb200_rec_tc_fwd(dyb200_ctx* ctx, const RecTcPlan& p, RecFwd* a, int ndir);
 int dyb200_rec_tc_bwd(dyb200_ctx* ctx, const RecTcPlan& p, RecBwd* a, int ndir);

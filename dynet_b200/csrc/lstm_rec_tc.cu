@@ -6,8 +6,8 @@
 // half of the TMEM for the whole sequence; TF32 pairs of the same precision would need all of it.  (From shared memory the 32 MMAs of
 // a step took 2400 cycles, each waiting for its 4 KB of Wh.)  A step is a chain of product, cell pass and one trip through the cluster.
 //
-// Columns: a cluster takes up to 16 NCH.  More than the clusters that fit run one after the other (no cluster waits for another);
-// ragged batches are then dealt out in blocks of neighbours, longest first, so that every block ends with its own longest sentence.
+// Columns: a cluster takes two groups of 16 NCH neighbours.  More clusters than fit run one after the other (no cluster waits for another):
+// ragged batches come longest first, so every group ends with its own longest sentence.
 //
 // Cells: a warp's lanes are the CTA's 32 units of one column, so that every access to gates, states and operand planes is a full
 // 128-byte line (8 units x 4 columns per access took four requests each: 3400 of a step's 9000 cycles went into the stores alone).
@@ -28,8 +28,11 @@
 
 namespace {
 
-// Warp 0 issues the products and the copies (the oldest warp of its scheduler goes first), warps 1 .. 16 are the cell warps.
-constexpr uint32_t kCellThreads = 512, kTcThreads = kCellThreads + 32;
+// Two groups of columns per CTA, each with its own loop, barriers and buffers (only Wh is shared): one's cell pass runs beside the other's
+// product and messages.  Warps 0 and 1 issue the groups' products and copies (the oldest warps of their schedulers go first), 2 .. 9
+// and 10 .. 17 are the groups' cell warps.
+constexpr uint32_t kGroups = 2, kGroupWarps = 8, kGroupThreads = 32 * kGroupWarps;
+constexpr uint32_t kCellThreads = kGroups * kGroupThreads, kTcThreads = kCellThreads + 32 * kGroups;
 constexpr uint32_t kTcUnits = 32;      // hidden units per CTA
 
 // Positions of a column's K-major operand row: byte offset of element k (even or odd) of row r in a plane block of `rows` rows per 64 k.
@@ -85,6 +88,12 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
                "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// one lane of a converged warp, in a form that lets the compiler keep the MMAs' operands in uniform registers
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(e)::"memory");
+  return e != 0;
+}
 // element `col * step` floats behind p
 __device__ __forceinline__ float* at(float* p, uint32_t col, uint32_t step) { return p + (uint64_t)col * step; }
 __device__ __forceinline__ const float* at(const float* p, uint32_t col, uint32_t step) { return p + (uint64_t)col * step; }
@@ -92,58 +101,55 @@ __device__ __forceinline__ const float* at(const float* p, uint32_t col, uint32_
 __device__ __forceinline__ uint32_t tc_active(uint32_t B, uint32_t base, uint32_t ncap) { return B > base ? min(B - base, ncap) : 0; }
 __device__ __forceinline__ uint32_t tmem_cols(uint32_t need) { return need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512; }
 
-// One k-block of 64: A_hi x [B_hi | B_lo] -> acc (2 NC columns), A_lo x B_hi -> its upper half, four k steps of 16.  A in TMEM: lane = row,
-// a column holds two k.  b0 / b1: descriptors of the right operand's first and second 32 k.
+// One k step of 16: A_hi x [B_hi | B_lo] -> wide (2 NC columns), A_lo x B_hi -> narrow.  A in TMEM: lane = row, a column holds two k.
 template <int NC>
-__device__ __forceinline__ void tc_kblock(uint32_t acc, uint32_t a_hi, uint32_t a_lo, uint64_t b0, uint64_t b1, uint32_t accumulate) {
+__device__ __forceinline__ void tc_kstep(uint32_t wide, uint32_t narrow, uint32_t a_hi, uint32_t a_lo, uint64_t b, uint32_t add_wide, uint32_t add_narrow) {
   constexpr uint32_t base = (1u << 4) | ((uint32_t)(BM >> 4) << 24);   // fp32 accumulator, fp16 operands, both K-major
-  constexpr uint32_t wide = base | ((uint32_t)(2 * NC >> 3) << 17), narrow = base | ((uint32_t)(NC >> 3) << 17);
   asm volatile(
-      "{\n\t.reg .pred pf, pt;\n\t.reg .b32 xa, xl;\n\t.reg .b64 yb;\n\t"
-      "setp.ne.b32 pf, %8, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %4, %6, pf;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [%3], %4, %7, pt;\n\t"
-      "add.u32 xa, %2, 8;\n\tadd.u32 xl, %3, 8;\n\tadd.s64 yb, %4, 2;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [xa], yb, %6, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [xl], yb, %7, pt;\n\t"
-      "add.u32 xa, xa, 8;\n\tadd.u32 xl, xl, 8;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [xa], %5, %6, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [xl], %5, %7, pt;\n\t"
-      "add.u32 xa, xa, 8;\n\tadd.u32 xl, xl, 8;\n\tadd.s64 yb, %5, 2;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [xa], yb, %6, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [xl], yb, %7, pt;\n\t}"
-      ::"r"(acc), "r"(acc + NC), "r"(a_hi), "r"(a_lo), "l"(b0), "l"(b1), "r"(wide), "r"(narrow), "r"(accumulate)
+      "{\n\t.reg .pred pw, pn;\n\t"
+      "setp.ne.b32 pw, %7, 0;\n\tsetp.ne.b32 pn, %8, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %4, %5, pw;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], [%3], %4, %6, pn;\n\t}"
+      ::"r"(wide), "r"(narrow), "r"(a_hi), "r"(a_lo), "l"(b), "r"(base | ((uint32_t)(2 * NC >> 3) << 17)), "r"(base | ((uint32_t)(NC >> 3) << 17)),
+        "r"(add_wide), "r"(add_narrow)
       : "memory");
 }
 
-// grid (C, blocks x directions), cluster (C, 1, 1).  Dynamic shared memory (1024-byte aligned):
+// grid (C, clusters x directions), cluster (C, 1, 1).  Dynamic shared memory (1024-byte aligned), for each group:
 // h [2][2 KB blocks of 32 units][NC hi rows, NC lo rows][64 bytes]; gates on their way [NC][4][32]; KB = ceil(H / 64).
-// TMEM: accumulators (2 NC columns), Wh_hi and Wh_lo (32 KB columns each).
+// TMEM: each group's accumulators (3 NC columns: A_hi B_hi, A_hi B_lo, A_lo B_hi - the last apart, so that the chain of one waits on
+// the other's MMAs, not on its own), Wh_hi and Wh_lo (32 KB columns each).
 template <int NCH>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_constant__ RecFwd a) {
   constexpr uint32_t NC = 16 * NCH, kBlock = 2 * NC * 64;   // bytes of a CTA's part of h
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t got[2], acc_full, h_ready;
-  __shared__ uint32_t tmem_slot, hword[2], wmax[128];
-  const uint32_t ndir = a.ndir, dir = blockIdx.y % ndir, g = blockIdx.y / ndir;
+  __shared__ __align__(8) uint64_t got_[kGroups][2], acc_full_[kGroups], h_ready_[kGroups];
+  __shared__ uint32_t tmem_slot, hword_[kGroups][2], wmax[128];
+  const uint32_t ndir = a.ndir, dir = blockIdx.y % ndir;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t grp = warp < kGroups ? warp : (warp - kGroups) / kGroupWarps, gw = (warp - kGroups) % kGroupWarps;   // (gw: cell warps)
   const RecDirF d = dir ? a.d[1] : a.d[0];
   const uint32_t H = a.H, rank = blockIdx.x, C = gridDim.x, KB = (H + 63) / 64;
-  const uint32_t base = g * NC;
-  unsigned char* hbuf = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const uint32_t base = (blockIdx.y / ndir * kGroups + grp) * NC;
   const uint32_t hbytes = 2 * KB * kBlock;
-  float* exch = reinterpret_cast<float*>(hbuf + 2 * hbytes);
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned char* hall = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* hbuf = hall + grp * 2 * hbytes;
+  float* exch = reinterpret_cast<float*>(hall + kGroups * 2 * hbytes) + grp * NC * 128;
+  uint64_t *got = got_[grp], &acc_full = acc_full_[grp], &h_ready = h_ready_[grp];
+  uint32_t* hword = hword_[grp];
   if (tid == 0) {
-    msg_init(&got[0]);
-    msg_init(&got[1]);
-    mbar_init(&acc_full, 1);
-    mbar_init(&h_ready, kCellThreads / 32);
-    hword[0] = hword[1] = 0;
+    for (uint32_t k = 0; k < kGroups; ++k) {
+      msg_init(&got_[k][0]);
+      msg_init(&got_[k][1]);
+      mbar_init(&acc_full_[k], 1);
+      mbar_init(&h_ready_[k], kGroupWarps);
+      hword_[k][0] = hword_[k][1] = 0;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (tid < 128) wmax[tid] = 0;
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols(2 * NC + 64 * KB)) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols(kGroups * 3 * NC + 64 * KB)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   dyb_grid_dep_sync();
@@ -155,9 +161,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
 
   // Wh of this CTA: lane = unit (128 contiguous bytes per load), a warp has 64 k of one gate.  The scale of a row is that of its largest
   // value.
-  if (warp > 0) {
+  if (warp >= kGroups) {
     float v[64];
-    const uint32_t u = rank * kTcUnits + lane, q = warp & 3, kb = (warp - 1) >> 2, row = 32 * q + lane;
+    const uint32_t u = rank * kTcUnits + lane, q = warp & 3, kb = (warp - kGroups) >> 2, row = 32 * q + lane;
     const float* src = d.Wh + (size_t)q * H + u;
     uint32_t m = 0;
 #pragma unroll
@@ -171,7 +177,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     bar_sync(1, kCellThreads);
     if (kb < KB) {
       const float scale = scale_of(wmax[row]);
-      const uint32_t to = tmem + 2 * NC + 32 * kb + ((32 * q) << 16);
+      const uint32_t to = tmem + kGroups * 3 * NC + 32 * kb + ((32 * q) << 16);
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         uint32_t hi[8], lo[8];
@@ -185,10 +191,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     tc_before();
   }
   // scales of h: the largest dropout factor (1 without); of the initial state: its largest value
-  for (uint32_t e = tid; e < 2 * hbytes / 16; e += kTcThreads) reinterpret_cast<uint4*>(hbuf)[e] = make_uint4(0, 0, 0, 0);
-  if (d.mask || d.h0) {
+  for (uint32_t e = tid; e < kGroups * 2 * hbytes / 16; e += kTcThreads) reinterpret_cast<uint4*>(hall)[e] = make_uint4(0, 0, 0, 0);
+  const uint32_t gt0 = gw * 32 + lane;   // (cell warps: thread of the group)
+  if (warp >= kGroups && (d.mask || d.h0)) {
     uint32_t m0 = 0, m1 = 0;
-    for (uint32_t e = tid; e < ncol * H; e += kTcThreads) {
+    for (uint32_t e = gt0; e < ncol * H; e += kGroupThreads) {
       const uint32_t i = e / H, k = e % H, sc = base + i;
       const float m = d.mask ? __ldg(d.mask + k + (a.mask_full ? (size_t)H * sc : 0)) : 1.f;
       m1 = max(m1, finite_mag(m));
@@ -199,9 +206,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
   }
   __syncthreads();
   const uint32_t word0 = hword[0], word1 = d.mask ? hword[1] : 0x3f800000u;
-  {
+  if (warp >= kGroups) {
     const float s0 = scale_of(word0);
-    for (uint32_t e = tid; e < ncol * H; e += kTcThreads) {
+    for (uint32_t e = gt0; e < ncol * H; e += kGroupThreads) {
       const uint32_t i = e / H, k = e % H, sc = base + i;
       float v = 0.f;
       if (d.h0) v = __ldg(d.h0 + k + (size_t)H * sc) * (d.mask ? __ldg(d.mask + k + (a.mask_full ? (size_t)H * sc : 0)) : 1.f);
@@ -225,9 +232,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
   auto start_of = [&](uint32_t t) { t = min(t, a.T); return a.prefix ? a.prefix[t] : t * a.N; };
   uint32_t col0 = 0, col1 = start_of(1), col2 = start_of(2), n = tc_active(col1, base, NC);
   bool ok = true;
-  if (warp == 0) {
+  if (warp < kGroups) {
     uint32_t phase[2] = {0, 0};
-    const uint32_t whi = tmem + 2 * NC, wlo = whi + 32 * KB;
+    const uint32_t whi = tmem + kGroups * 3 * NC, wlo = whi + 32 * KB, acc = tmem + grp * 3 * NC;
     for (uint32_t t = 0; t < a.T && n > 0; ++t) {
       const uint32_t pt = t & 1, pn = pt ^ 1, col3 = start_of(t + 3), n1 = tc_active(col2 - col1, base, NC);
       unsigned char* h = hbuf + pt * hbytes;
@@ -242,43 +249,47 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
         ok = ok && msg_wait(&got[pt], phase[pt]);
         phase[pt] ^= 1;
       }
-      if (lane == 0) {
+      if (elect_one()) {
         fence_async();
         tc_after();
         const uint32_t hb = smem_u32(h);
-        for (uint32_t kb = 0; kb < KB; ++kb)
-          tc_kblock<NC>(tmem, whi + kb * 32, wlo + kb * 32, umma_desc64(hb + 2 * kb * kBlock), umma_desc64(hb + (2 * kb + 1) * kBlock), kb);
+        for (uint32_t blk = 0; blk < 2 * KB; ++blk) {
+          const uint64_t bd = umma_desc64(hb + blk * kBlock);
+          tc_kstep<NC>(acc, acc + 2 * NC, whi + 16 * blk, wlo + 16 * blk, bd, blk, blk);
+          tc_kstep<NC>(acc, acc + 2 * NC, whi + 16 * blk + 8, wlo + 16 * blk + 8, bd + 2, 1, 1);
+        }
         umma_commit(&acc_full);
       }
       __syncwarp();
       col1 = col2; col2 = col3; n = n1;
     }
   } else {
-    // reads gate `quad` of the columns 16 j + c4 .. + 3, finishes column 16 j + c4 + quad; lane = unit
-    const uint32_t quad = warp & 3, c4 = 4 * ((warp - 1) >> 2), u = rank * kTcUnits + lane, i0 = c4 + quad;
+    // reads gate `quad` of the columns 16 j + c8 .. + 7, finishes columns 16 j + c8 + quad and + 4; lane = unit
+    constexpr int kCells = 2 * NCH;
+    const uint32_t quad = warp & 3, c8 = 8 * (gw >> 2), u = rank * kTcUnits + lane, i0 = c8 + quad;
     const bool live_u = u < H;
     const uint32_t uc = min(u, H - 1);                  // (units that are not there read another's values and store nothing)
     const int wf = scale_field(wmax[32 * quad + lane]), t0 = wf + scale_field(word0) - 282, t1 = wf + scale_field(word1) - 282;
     const float hscale = live_u ? scale_of(word1) : 0.f;
-    const uint32_t tq = tmem + ((32 * quad) << 16) + c4;
+    const uint32_t tq = tmem + grp * 3 * NC + ((32 * quad) << 16) + c8;
     const float* mask = d.mask ? d.mask + uc : nullptr;
     float *pg = d.gates + uc, *pc = d.c + uc, *ph = d.h + uc, *phi = d.hn_hi ? d.hn_hi + uc : nullptr, *plo = phi ? d.hn_lo + uc : nullptr;
-    float pre[NCH][4], cst[NCH], mk[NCH];
-    uint32_t ho[NCH];                                    // where h of cell j goes in this CTA's block
+    float pre[kCells][4], cst[kCells], mk[kCells];
+    uint32_t ho[kCells];                                   // where h of cell j goes in this CTA's block
     auto fetch = [&](uint32_t c0, uint32_t nact) {
 #pragma unroll
-      for (int j = 0; j < NCH; ++j) {
-        const uint32_t i = 16 * j + i0, col = c0 + base + (i < nact ? i : 0);
+      for (int j = 0; j < kCells; ++j) {
+        const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), col = c0 + base + (i < nact ? i : 0);
 #pragma unroll
         for (int q = 0; q < 4; ++q) pre[j][q] = *at(pg + (size_t)q * H, col, 4 * H);
       }
     };
-    fetch(0, n);
+    if (n) fetch(0, n);          // (a group may have no column at all)
 #pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-      const uint32_t i = 16 * j + i0, sc = base + (i < ncol ? i : 0);
-      cst[j] = d.c0 ? __ldg(at(d.c0 + uc, sc, H)) : 0.f;
-      mk[j] = mask ? __ldg(at(mask, a.mask_full ? sc : 0, H)) : 1.f;
+    for (int j = 0; j < kCells; ++j) {
+      const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), sc = base + i;
+      cst[j] = d.c0 && i < ncol ? __ldg(at(d.c0 + uc, sc, H)) : 0.f;
+      mk[j] = mask && i < ncol ? __ldg(at(mask, a.mask_full ? sc : 0, H)) : 1.f;
       ho[j] = h_off(2 * NC, i, rank * kTcUnits + lane);
     }
     for (uint32_t t = 0; t < a.T && n > 0; ++t) {
@@ -288,26 +299,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       const float f0 = __int_as_float((th + 127) << 23), f1 = __int_as_float((ts - th + 127) << 23);
       ok = ok && mbar_wait(&acc_full, t & 1);
       tc_after();
-      {
-        float z[4 * NCH], z2[4 * NCH];
-#pragma unroll
-        for (int j = 0; j < NCH; ++j) {
-          tmem_ld4(tq + 16 * j, z + 4 * j);
-          tmem_ld4(tq + NC + 16 * j, z2 + 4 * j);
-        }
-        tmem_ld_wait();
-        tc_before();
-#pragma unroll
-        for (int j = 0; j < NCH; ++j)
-#pragma unroll
-          for (int x = 0; x < 4; ++x)
-            exch[((16 * j + c4 + x) * 4 + quad) * 32 + lane] = (fmaf(z2[4 * j + x], kLoScale, z[4 * j + x]) * f0) * f1;
-      }
-      bar_sync(2 + c4 / 4, 128);
-      float hv[NCH], hm[NCH], y[NCH][4];
 #pragma unroll
       for (int j = 0; j < NCH; ++j) {
-        const uint32_t i = 16 * j + i0;
+        float z[8], z2[8], z3[8];
+        tmem_ld8(tq + 16 * j, z);
+        tmem_ld8(tq + NC + 16 * j, z2);
+        tmem_ld8(tq + 2 * NC + 16 * j, z3);
+        tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < 8; ++x) exch[((16 * j + c8 + x) * 4 + quad) * 32 + lane] = (fmaf(z2[x] + z3[x], kLoScale, z[x]) * f0) * f1;
+      }
+      tc_before();
+      bar_sync(2 + 2 * grp + c8 / 8, 128);
+      float hv[kCells], hm[kCells], y[kCells][4];
+#pragma unroll
+      for (int j = 0; j < kCells; ++j) {
+        const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1);
 #pragma unroll
         for (int q = 0; q < 4; ++q) y[j][q] = exch[(i * 4 + q) * 32 + lane];
         if (i >= n) continue;                            // (the same for the whole warp)
@@ -329,8 +336,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(&h_ready);
 #pragma unroll
-      for (int j = 0; j < NCH; ++j) {
-        const uint32_t i = 16 * j + i0, sc = base + i;
+      for (int j = 0; j < kCells; ++j) {
+        const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), sc = base + i;
         if (!live_u || i >= n) continue;
 #pragma unroll
         for (int q = 0; q < 4; ++q) *at(pg + (size_t)q * H, col0 + sc, 4 * H) = y[j][q];
@@ -354,37 +361,44 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
   cluster_wait();
   if (warp == 0) {
     tc_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(2 * NC + 64 * KB)) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(kGroups * 3 * NC + 64 * KB)) : "memory");
   }
 }
 
-// grid (C, blocks x directions), cluster (C, 1, 1).  Dynamic shared memory (1024-byte aligned): dgates [2 blocks of 64 gate rows]
-// [NC hi rows, NC lo rows][128 bytes]; the partial sums [2][C ranks][NC columns][32 units].  TMEM: per row tile of 128 units the
-// accumulators (2 NC columns); then Wh^T hi and lo (64 columns each per row tile).  The slots of the sums that have just been read hold the outgoing ones: what comes into slot r next, rank r
+// grid (C, clusters x directions), cluster (C, 1, 1).  Dynamic shared memory (1024-byte aligned), for each group: dgates [2 blocks of 64
+// gate rows][NC hi rows, NC lo rows][128 bytes]; the partial sums [2][C ranks][NC columns][32 units].  TMEM: per group and row tile of 128
+// units the accumulators (2 NC columns); then Wh^T hi and lo (64 columns each per row tile).  The slots of the sums that have just been read hold the outgoing ones: what comes into slot r next, rank r
 // sends after it has what went out of that slot.  Gate row (unit ul, gate q) is element 4 ul + q of the reduction.
 template <int NCH>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_constant__ RecBwd a) {
   constexpr uint32_t NC = 16 * NCH, kSlot = NC * kTcUnits;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t got[2], acc_full;
+  __shared__ __align__(8) uint64_t got_[kGroups][2], acc_full_[kGroups];
   __shared__ uint32_t tmem_slot, wmax[256];
-  __shared__ float colscale[2][NC];
+  __shared__ float colscale_[kGroups][2][NC];
   const uint32_t ndir = a.ndir, dir = blockIdx.y % ndir, g = blockIdx.y / ndir;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t grp = warp < kGroups ? warp : (warp - kGroups) / kGroupWarps, gw = (warp - kGroups) % kGroupWarps;   // (gw: cell warps)
   const RecDirB d = dir ? a.d[1] : a.d[0];
   const uint32_t H = a.H, rank = blockIdx.x, C = gridDim.x, MT = (H + 127) / 128;
-  const uint32_t base = g * NC;
-  unsigned char* dgb = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* part = reinterpret_cast<float*>(dgb + 2 * 2 * NC * 128);
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t base = (g * kGroups + grp) * NC;
+  unsigned char* dgall = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* dgb = dgall + grp * 2 * 2 * NC * 128;
+  float* partall = reinterpret_cast<float*>(dgall + kGroups * 2 * 2 * NC * 128);
+  float* part = partall + grp * 2 * C * kSlot;
+  uint64_t *got = got_[grp], &acc_full = acc_full_[grp];
+  float (*colscale)[NC] = colscale_[grp];
   if (tid == 0) {
-    mbar_init(&got[0], 3);   // (the bytes of the others, and this CTA's own two warps)
-    mbar_init(&got[1], 3);
-    mbar_init(&acc_full, 1);
+    for (uint32_t k = 0; k < kGroups; ++k) {
+      mbar_init(&got_[k][0], 2);   // (the bytes of the others, and this CTA's own warp)
+      mbar_init(&got_[k][1], 2);
+      mbar_init(&acc_full_[k], 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (tid < 256) wmax[tid] = 0;
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols(MT * (2 * NC + 128))) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols(MT * (kGroups * 2 * NC + 128))) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   dyb_grid_dep_sync();
@@ -394,10 +408,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
   const uint32_t tmem = tmem_slot;
 
   // Lane = unit o of h_{t-1} (row o % 128 of its row tile), a warp has its weights in 16 of this CTA's units; scaled by the largest of all
-  if (warp > 0) {
+  if (warp >= kGroups) {
     float4 v[4][4];
     const bool quads = (H & 3) == 0 && aligned16(d.Wh);
-    const uint32_t q4 = warp & 3, p4 = (warp - 1) >> 2, mt = p4 >> 1, kh = p4 & 1, o = 128 * mt + 32 * q4 + lane;
+    const uint32_t q4 = warp & 3, p4 = (warp - kGroups) >> 2, mt = p4 >> 1, kh = p4 & 1, o = 128 * mt + 32 * q4 + lane;
     uint32_t m = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -422,7 +436,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     bar_sync(1, kCellThreads);
     if (mt < MT) {
       const float scale = scale_of(wmax[o]);
-      const uint32_t to = tmem + MT * 2 * NC + 64 * mt + 32 * kh + ((32 * q4) << 16);
+      const uint32_t to = tmem + MT * kGroups * 2 * NC + 64 * mt + 32 * kh + ((32 * q4) << 16);
 #pragma unroll
       for (int x = 0; x < 4; ++x) {   // (a column holds two gates of a unit)
         uint32_t hi[8], lo[8];
@@ -437,50 +451,52 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     }
     tc_before();
   }
-  for (uint32_t e = tid; e < 2 * 2 * NC * 128 / 16; e += kTcThreads) reinterpret_cast<uint4*>(dgb)[e] = make_uint4(0, 0, 0, 0);
+  for (uint32_t e = tid; e < kGroups * 2 * 2 * NC * 128 / 16; e += kTcThreads) reinterpret_cast<uint4*>(dgall)[e] = make_uint4(0, 0, 0, 0);
   fence_async();
   cluster_arrive();
   cluster_wait();
 
   // the last step that has a column of this block: widths never grow, so the steps before it have one too
-  uint32_t T = a.T;
+  uint32_t T = base < a.N ? a.T : 0;
   while (a.prefix && T > 0 && tc_active(a.prefix[T] - a.prefix[T - 1], base, NC) == 0) --T;
   auto start_of = [&](uint32_t t) { return a.prefix ? a.prefix[t] : t * a.N; };
   bool ok = true;
   float db[4] = {0.f, 0.f, 0.f, 0.f};
-  if (warp == 0) {
-    const uint32_t whi = tmem + MT * 2 * NC, wlo = whi + 64 * MT, dg = smem_u32(dgb);
+  if (warp < kGroups) {
+    const uint32_t acc = tmem + grp * MT * 2 * NC, whi = tmem + MT * kGroups * 2 * NC, wlo = whi + 64 * MT, dg = smem_u32(dgb);
     for (uint32_t t = T; t-- > 1;) {
-      bar_sync(2, kTcThreads);     // the step's gradients are in place
-      if (lane == 0) {
+      bar_sync(2 + grp, kGroupThreads + 32);     // the step's gradients are in place
+      if (elect_one()) {
         fence_async();
         tc_after();
-        for (uint32_t mt = 0; mt < MT; ++mt)
-          for (uint32_t kb = 0; kb < 2; ++kb) {
-            const uint64_t b = umma_desc(dg + kb * 2 * NC * 128);
-            tc_kblock<NC>(tmem + mt * 2 * NC, whi + mt * 64 + kb * 32, wlo + mt * 64 + kb * 32, b, b + 4, kb);
-          }
+#pragma unroll
+        for (uint32_t ks = 0; ks < 8; ++ks) {
+          const uint64_t bd = umma_desc(dg + (ks / 4) * 2 * NC * 128) + 2 * (ks % 4);
+          for (uint32_t mt = 0; mt < MT; ++mt)
+            tc_kstep<NC>(acc + mt * 2 * NC, acc + mt * 2 * NC + NC, whi + mt * 64 + 8 * ks, wlo + mt * 64 + 8 * ks, bd, ks, 1);
+        }
         umma_commit(&acc_full);
       }
       __syncwarp();
     }
   } else {
-    const uint32_t cw = warp - 1, quad = warp & 3, part4 = cw >> 2, u = rank * kTcUnits + lane;
+    constexpr int kCells = 2 * NCH;
+    const uint32_t u = rank * kTcUnits + lane;
     const bool live_u = u < H;
     const uint32_t uc = min(u, H - 1);                   // (units that are not there read another's values and store nothing)
-    // this warp's piece of the product: 32 rows (the units of rank `to`) x 8 NCH columns from `cols` on
-    const uint32_t to = 4 * (part4 >> 1) + quad, half = part4 & 1, cols = 8 * NCH * half;
+    // this warp's piece of the product: 32 rows (the units of rank `to`)
+    const uint32_t quad = warp & 3, mt = gw >> 2, to = 4 * mt + quad;
     const float wscale = __int_as_float((scale_field(wmax[32 * to + lane]) - 14) << 23);   // (undoes the scale of the row this lane reads)
-    const uint32_t tq = tmem + (part4 >> 1) * 2 * NC + cols + ((32 * quad) << 16);
+    const uint32_t tq = tmem + (grp * MT + mt) * 2 * NC + ((32 * quad) << 16);
     const float *pg = d.gates + uc, *pc = d.c + uc, *pc0 = d.c0 ? d.c0 + uc : nullptr;
     float *pdh = d.dh + uc, *pdc = d.dc ? d.dc + uc : nullptr, *phi = d.dn_hi + uc, *plo = d.dn_lo + uc;
     uint32_t phase[2] = {0, 0};
-    float gt[NCH][4], cv[NCH], cp[NCH], dhv[NCH], dcv[NCH], dcs[NCH], mk[NCH];
+    float gt[kCells][4], cv[kCells], cp[kCells], dhv[kCells], dcv[kCells], dcs[kCells], mk[kCells];
     // cell j: column 16 j + cw
     auto fetch = [&](bool first, uint32_t c0, uint32_t cm1, uint32_t nact) {
 #pragma unroll
-      for (int j = 0; j < NCH; ++j) {
-        const uint32_t i = 16 * j + cw, sc = base + (i < nact ? i : 0);
+      for (int j = 0; j < kCells; ++j) {
+        const uint32_t i = 8 * j + gw, sc = base + (i < nact ? i : 0);
 #pragma unroll
         for (int q = 0; q < 4; ++q) gt[j][q] = *at(pg + (size_t)q * H, c0 + sc, 4 * H);
         cv[j] = *at(pc, c0 + sc, H);
@@ -495,8 +511,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     uint32_t col = T ? start_of(T - 1) : 0, colm1 = T > 1 ? start_of(T - 2) : 0, colm2 = T > 2 ? start_of(T - 3) : 0;
     uint32_t n = T ? tc_active(start_of(T) - col, base, NC) : 0;
 #pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-      const uint32_t sc = base + 16 * j + cw;
+    for (int j = 0; j < kCells; ++j) {
+      const uint32_t sc = base + 8 * j + gw;
       dcs[j] = 0.f;
       mk[j] = d.mask && sc < a.N ? __ldg(at(d.mask + uc, a.mask_full ? sc : 0, H)) : 1.f;
     }
@@ -505,15 +521,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     for (uint32_t t = T; t-- > 0;) {
       const uint32_t pin = (t + 1) & 1, pout = t & 1, colm3 = t > 2 ? start_of(t - 3) : 0;
       float* in = part + (size_t)pin * C * kSlot;
-      if (t && tid == 32) msg_expect(&got[pout], n * (C - 1) * kTcUnits * 4);
+      if (t && gw == 0 && lane == 0) msg_expect(&got[pout], n * (C - 1) * kTcUnits * 4);
       if (n_later) {
         ok = ok && msg_wait(&got[pin], phase[pin]);
         phase[pin] ^= 1;
       }
-      float pr[NCH][4];
+      float pr[kCells][4];
 #pragma unroll
-      for (int j = 0; j < NCH; ++j) {
-        const uint32_t i = 16 * j + cw, sc = base + i;
+      for (int j = 0; j < kCells; ++j) {
+        const uint32_t i = 8 * j + gw, sc = base + i;
         pr[j][0] = pr[j][1] = pr[j][2] = pr[j][3] = 0.f;
         if (i < n) {                    // (the same for the whole warp)
           float dh = dhv[j], dcp = 0.f;
@@ -549,14 +565,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
       if (t) {
         fence_async();
         tc_before();
-        bar_sync(2, kTcThreads);
+        bar_sync(2 + grp, kGroupThreads + 32);
       }
       // while the product runs: the next step's values, the operand planes of the weight gradients
       const uint32_t nm1 = t ? tc_active(col - colm1, base, NC) : 0;
       if (t) fetch(t == 1, colm1, colm2, nm1);
 #pragma unroll
-      for (int j = 0; j < NCH; ++j) {
-        const uint32_t i = 16 * j + cw, sc = base + i;
+      for (int j = 0; j < kCells; ++j) {
+        const uint32_t i = 8 * j + gw, sc = base + i;
         if (!live_u || i >= n) continue;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -572,26 +588,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
       full ^= 1;
       tc_after();
       // (columns that are not there are neither written nor sent: their part of the slot may already be filling again)
-      const uint32_t out = n > cols ? min(n - cols, 8u * NCH) : 0;
-      if (to < C && out) {
-        float* slot = (to == rank ? part + (size_t)pout * C * kSlot : in) + to * kSlot + cols * kTcUnits;
-        const float* cs = colscale[t & 1] + cols;
+      if (to < C) {
+        float* slot = (to == rank ? part + (size_t)pout * C * kSlot : in) + to * kSlot;
+        const float* cs = colscale[t & 1];
 #pragma unroll
-        for (int x = 0; x < NCH; ++x) {
-          if (8u * x >= out) break;
+        for (int x = 0; x < 2 * NCH; ++x) {
+          if (8u * x >= n) break;
           float z[8], z2[8];
           tmem_ld8(tq + 8 * x, z);
           tmem_ld8(tq + NC + 8 * x, z2);
           tmem_ld_wait();
 #pragma unroll
           for (int y = 0; y < 8; ++y)
-            if (8u * x + y < out) slot[(8 * x + y) * kTcUnits + lane] = fmaf(z2[y], kLoScale, z[y]) * wscale * cs[8 * x + y];
+            if (8u * x + y < n) slot[(8 * x + y) * kTcUnits + lane] = fmaf(z2[y], kLoScale, z[y]) * wscale * cs[8 * x + y];
         }
         if (to != rank) {
           fence_async();
           __syncwarp();
           if (lane == 0)
-            send_bulk(map_rank(smem_u32(part + ((size_t)pout * C + rank) * kSlot + cols * kTcUnits), to), slot, out * kTcUnits * 4, map_rank(smem_u32(&got[pout]), to));
+            send_bulk(map_rank(smem_u32(part + ((size_t)pout * C + rank) * kSlot), to), slot, n * kTcUnits * 4, map_rank(smem_u32(&got[pout]), to));
         }
       }
       if (to == rank) {
@@ -609,58 +624,61 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
   cluster_wait();
   if (warp == 0) {
     tc_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(MT * (2 * NC + 128))) : "memory");
-  } else {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(MT * (kGroups * 2 * NC + 128))) : "memory");
+  }
+  if (warp >= kGroups) {
     // row sums of dgates: the sixteen threads of a unit, in ascending order (part is free: every CTA is through)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) part[((warp - 1) * 4 + q) * kTcUnits + lane] = db[q];
+    for (int q = 0; q < 4; ++q) partall[((warp - kGroups) * 4 + q) * kTcUnits + lane] = db[q];
   }
   __syncthreads();
   if (tid < 128) {
     const uint32_t q = tid / kTcUnits, ul = tid % kTcUnits, u = rank * kTcUnits + ul;
     if (u < H) {
       float r = 0.f;
-      for (uint32_t k = 0; k < 16; ++k) r += part[(k * 4 + q) * kTcUnits + ul];
+      for (uint32_t k = 0; k < 16; ++k) r += partall[(k * 4 + q) * kTcUnits + ul];
       d.dbpart[(size_t)g * 4 * H + q * H + u] = r;
     }
   }
 }
 
-constexpr uint32_t kTcMostCols = 64;   // columns per cluster: 165 KB of shared memory and, backward, all of the TMEM
-
+// nch: 16 columns per group
 uint32_t tc_smem(bool bwd, uint32_t H, uint32_t nch) {
   const uint32_t NC = 16 * nch, KB = (H + 63) / 64, C = (H + kTcUnits - 1) / kTcUnits;
-  // (the partial sums' room also holds the 16 x 128 row sums of dgates at the end)
-  const uint32_t part = 2 * C * NC * kTcUnits * 4;
-  return 1024 + (bwd ? 2 * 2 * NC * 128 + (part > 8192 ? part : 8192) : 2 * 2 * KB * 2 * NC * 64 + NC * 512);
+  // (the partial sums' room also holds the 16 x 128 row sums of dgates at the end: 8 KB at least)
+  return 1024 + kGroups * (bwd ? 2 * 2 * NC * 128 + 2 * C * NC * kTcUnits * 4 : 2 * 2 * KB * 2 * NC * 64 + NC * 512);
 }
 typedef void (*TcFwdKernel)(RecFwd);
 typedef void (*TcBwdKernel)(RecBwd);
-TcFwdKernel tc_fwd(uint32_t nch) { return nch == 1 ? k_rec_tc_fwd<1> : nch == 2 ? k_rec_tc_fwd<2> : nch == 3 ? k_rec_tc_fwd<3> : k_rec_tc_fwd<4>; }
-TcBwdKernel tc_bwd(uint32_t nch) { return nch == 1 ? k_rec_tc_bwd<1> : nch == 2 ? k_rec_tc_bwd<2> : nch == 3 ? k_rec_tc_bwd<3> : k_rec_tc_bwd<4>; }
+TcFwdKernel tc_fwd(uint32_t nch) { return nch == 1 ? k_rec_tc_fwd<1> : k_rec_tc_fwd<2>; }
+TcBwdKernel tc_bwd(uint32_t nch) { return nch == 1 ? k_rec_tc_bwd<1> : k_rec_tc_bwd<2>; }
 const void* tc_kernel(bool bwd, uint32_t nch) { return bwd ? (const void*)tc_bwd(nch) : (const void*)tc_fwd(nch); }
 
 }  // namespace
 
-// Room for columns in a cluster (16 per unit) and blocks of columns per direction: one round of clusters where that holds all columns, else
-// rounds of full blocks.
-bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int ndir, RecTcPlan* out) {
+// Columns per group / 16 (1 or 2) and clusters per direction.  A step of 2 x 32 columns takes about one and a half times as long as one of
+// 2 x 16; what counts is the rounds of clusters that each needs - in fractions for ragged batches, whose last round is short.
+bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int ndir, bool ragged, RecTcPlan* out) {
   if (H > 256 || N == 0) return false;
   const uint32_t C = (H + kTcUnits - 1) / kTcUnits;
   int16_t& fit = ctx->rec_tc_fit[bwd][C - 1];
   if (fit == 0) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    if (dyb200_rec_launch_cfg(ctx, tc_kernel(bwd, kTcMostCols / 16), &cfg, attr, dim3(C, 1, 1), kTcThreads, tc_smem(bwd, H, kTcMostCols / 16))) return false;
+    if (dyb200_rec_launch_cfg(ctx, tc_kernel(bwd, 2), &cfg, attr, dim3(C, 1, 1), kTcThreads, tc_smem(bwd, H, 2))) return false;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, tc_kernel(bwd, kTcMostCols / 16), &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
+    if (cudaOccupancyMaxActiveClusters(&n, tc_kernel(bwd, 2), &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
     fit = (int16_t)(n > 0 ? n : -1);
   }
   if (fit <= 0) return false;
   const uint32_t side = fit > ndir ? (uint32_t)(fit / ndir) : 1u;   // clusters per direction that run at the same time
-  const uint32_t each = (N + side - 1) / side;                      // columns per cluster in one round
-  out->nch = each > kTcMostCols ? kTcMostCols / 16 : (each + 15) / 16;
-  out->G = (N + 16 * out->nch - 1) / (16 * out->nch);
+  double rounds[2];
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t per = kGroups * 16 * (k + 1), c = (N + per - 1) / per;
+    rounds[k] = c <= side ? 1.0 : ragged ? (double)c / side : (double)((c + side - 1) / side);
+  }
+  out->nch = rounds[0] <= 1.5 * rounds[1] ? 1 : 2;
+  out->G = (N + kGroups * 16 * out->nch - 1) / (kGroups * 16 * out->nch);
   return true;
 }
 int dyb200_rec_tc_fwd(dyb200_ctx* ctx, const RecTcPlan& p, RecFwd* a, int ndir) {
