@@ -94,9 +94,12 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(e)::"memory");
   return e != 0;
 }
-// element `col * step` floats behind p
-__device__ __forceinline__ float* at(float* p, uint32_t col, uint32_t step) { return p + (uint64_t)col * step; }
-__device__ __forceinline__ const float* at(const float* p, uint32_t col, uint32_t step) { return p + (uint64_t)col * step; }
+// p + col * bytes: one multiply-add of 32 x 32 + 64 bits (indexing by floats adds a shift of 64 bits to every address; addresses were a
+// third of the cell passes' instructions)
+__device__ __forceinline__ float* at(float* p, uint32_t col, uint32_t bytes) { return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + (uint64_t)col * bytes); }
+__device__ __forceinline__ const float* at(const float* p, uint32_t col, uint32_t bytes) {
+  return reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + (uint64_t)col * bytes);
+}
 // columns of the block from `base` on that are active at a step of width B
 __device__ __forceinline__ uint32_t tc_active(uint32_t B, uint32_t base, uint32_t ncap) { return B > base ? min(B - base, ncap) : 0; }
 __device__ __forceinline__ uint32_t tmem_cols(uint32_t need) { return need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512; }
@@ -169,7 +172,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
 #pragma unroll
     for (int x = 0; x < 64; ++x) {
       const uint32_t k = 64 * kb + x;
-      v[x] = k < H && u < H ? __ldg(at(src, k, 4 * H)) : 0.f;
+      v[x] = k < H && u < H ? __ldg(at(src, k, 16 * H)) : 0.f;
     }
 #pragma unroll
     for (int x = 0; x < 64; ++x) m = max(m, finite_mag(v[x]));
@@ -281,15 +284,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       for (int j = 0; j < kCells; ++j) {
         const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), col = c0 + base + (i < nact ? i : 0);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pre[j][q] = *at(pg + (size_t)q * H, col, 4 * H);
+        for (int q = 0; q < 4; ++q) pre[j][q] = at(pg, col, 16 * H)[(size_t)q * H];
       }
     };
     if (n) fetch(0, n);          // (a group may have no column at all)
 #pragma unroll
     for (int j = 0; j < kCells; ++j) {
       const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), sc = base + i;
-      cst[j] = d.c0 && i < ncol ? __ldg(at(d.c0 + uc, sc, H)) : 0.f;
-      mk[j] = mask && i < ncol ? __ldg(at(mask, a.mask_full ? sc : 0, H)) : 1.f;
+      cst[j] = d.c0 && i < ncol ? __ldg(at(d.c0 + uc, sc, 4 * H)) : 0.f;
+      mk[j] = mask && i < ncol ? __ldg(at(mask, a.mask_full ? sc : 0, 4 * H)) : 1.f;
       ho[j] = h_off(2 * NC, i, rank * kTcUnits + lane);
     }
     for (uint32_t t = 0; t < a.T && n > 0; ++t) {
@@ -340,14 +343,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
         const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), sc = base + i;
         if (!live_u || i >= n) continue;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) *at(pg + (size_t)q * H, col0 + sc, 4 * H) = y[j][q];
-        *at(pc, col0 + sc, H) = cst[j];
-        *at(ph, col0 + sc, H) = hv[j];
+        for (int q = 0; q < 4; ++q) at(pg, col0 + sc, 16 * H)[(size_t)q * H] = y[j][q];
+        *at(pc, col0 + sc, 4 * H) = cst[j];
+        *at(ph, col0 + sc, 4 * H) = hv[j];
         if (phi && i < n1) {
           float hi, lo;
           split_tf32(hm[j], hi, lo);
-          *at(phi, col1 + sc, a.hn_pitch) = hi;
-          *at(plo, col1 + sc, a.hn_pitch) = lo;
+          *at(phi, col1 + sc, 4 * a.hn_pitch) = hi;
+          *at(plo, col1 + sc, 4 * a.hn_pitch) = lo;
         }
       }
       if (n1) fetch(col1, n1);
@@ -367,15 +370,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
 
 // grid (C, clusters x directions), cluster (C, 1, 1).  Dynamic shared memory (1024-byte aligned), for each group: dgates [2 blocks of 64
 // gate rows][NC hi rows, NC lo rows][128 bytes]; the partial sums [2][C ranks][NC columns][32 units].  TMEM: per group and row tile of 128
-// units the accumulators (2 NC columns); then Wh^T hi and lo (64 columns each per row tile).  The slots of the sums that have just been read hold the outgoing ones: what comes into slot r next, rank r
-// sends after it has what went out of that slot.  Gate row (unit ul, gate q) is element 4 ul + q of the reduction.
+// units the accumulators (2 NC columns); then Wh^T hi and lo (64 columns each per row tile).  The slots of the sums that have just been
+// read hold the outgoing ones: what comes into slot r next, rank r sends after it has what went out of that slot.  Gate row (unit ul,
+// gate q) is element 4 ul + q of the reduction.
 template <int NCH>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_constant__ RecBwd a) {
   constexpr uint32_t NC = 16 * NCH, kSlot = NC * kTcUnits;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t got_[kGroups][2], acc_full_[kGroups];
   __shared__ uint32_t tmem_slot, wmax[256];
-  __shared__ float colscale_[kGroups][2][NC];
+  __shared__ __align__(16) float colscale_[kGroups][2][NC];
   const uint32_t ndir = a.ndir, dir = blockIdx.y % ndir, g = blockIdx.y / ndir;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t grp = warp < kGroups ? warp : (warp - kGroups) / kGroupWarps, gw = (warp - kGroups) % kGroupWarps;   // (gw: cell warps)
@@ -418,7 +422,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         const uint32_t uu = rank * kTcUnits + 16 * kh + 4 * x;
-        const float* p = at(d.Wh + (size_t)q * H + uu, o, 4 * H);
+        const float* p = at(d.Wh + (size_t)q * H + uu, o, 16 * H);
         float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
         if (o < H && uu < H) {
           if (quads) w = __ldg(reinterpret_cast<const float4*>(p));
@@ -492,19 +496,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     float *pdh = d.dh + uc, *pdc = d.dc ? d.dc + uc : nullptr, *phi = d.dn_hi + uc, *plo = d.dn_lo + uc;
     uint32_t phase[2] = {0, 0};
     float gt[kCells][4], cv[kCells], cp[kCells], dhv[kCells], dcv[kCells], dcs[kCells], mk[kCells];
-    // cell j: column 16 j + cw
+    unsigned char* dgo = dgb + op_off(2 * NC, gw, 4 * lane);   // (eight columns on: 1024 bytes)
+    // cell j: column 8 j + gw
     auto fetch = [&](bool first, uint32_t c0, uint32_t cm1, uint32_t nact) {
 #pragma unroll
       for (int j = 0; j < kCells; ++j) {
         const uint32_t i = 8 * j + gw, sc = base + (i < nact ? i : 0);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) gt[j][q] = *at(pg + (size_t)q * H, c0 + sc, 4 * H);
-        cv[j] = *at(pc, c0 + sc, H);
-        dhv[j] = *at(pdh, c0 + sc, H);
+        for (int q = 0; q < 4; ++q) gt[j][q] = at(pg, c0 + sc, 16 * H)[(size_t)q * H];
+        cv[j] = *at(pc, c0 + sc, 4 * H);
+        dhv[j] = *at(pdh, c0 + sc, 4 * H);
         cp[j] = dcv[j] = 0.f;
         const float* before = first ? pc0 : pc;
-        if (before) cp[j] = *at(before, first ? sc : cm1 + sc, H);
-        if (pdc) dcv[j] = *at(pdc, c0 + sc, H);
+        if (before) cp[j] = *at(before, first ? sc : cm1 + sc, 4 * H);
+        if (pdc) dcv[j] = *at(pdc, c0 + sc, 4 * H);
       }
     };
     // first columns of the steps t, t - 1, t - 2, each read a step before it is needed; columns active at step t
@@ -514,7 +519,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     for (int j = 0; j < kCells; ++j) {
       const uint32_t sc = base + 8 * j + gw;
       dcs[j] = 0.f;
-      mk[j] = d.mask && sc < a.N ? __ldg(at(d.mask + uc, a.mask_full ? sc : 0, H)) : 1.f;
+      mk[j] = d.mask && sc < a.N ? __ldg(at(d.mask + uc, a.mask_full ? sc : 0, 4 * H)) : 1.f;
     }
     if (T) fetch(T == 1, col, colm1, n);
     uint32_t n_later = 0, full = 0;
@@ -542,8 +547,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
               if ((uint32_t)q < C) r += from[(size_t)q * kSlot];
             dh = fmaf(r, mk[j], dh);
             if (live_u) {
-              *at(pdh, col + sc, H) = dh;
-              if (pdc) *at(pdc, col + sc, H) = dci;
+              *at(pdh, col + sc, 4 * H) = dh;
+              if (pdc) *at(pdc, col + sc, 4 * H) = dci;
             }
           }
           lstm_cell_grad(gt[j][0], gt[j][1], gt[j][2], gt[j][3], cv[j], cp[j], dh, dci, true, dcp, pr[j][0], pr[j][1], pr[j][2], pr[j][3]);
@@ -558,8 +563,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
           __half hi[4], lo[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q) split_f16(pr[j][q] * scale, hi[q], lo[q]);
-          *reinterpret_cast<uint2*>(dgb + op_off(2 * NC, i, 4 * lane)) = *reinterpret_cast<uint2*>(hi);
-          *reinterpret_cast<uint2*>(dgb + op_off(2 * NC, NC + i, 4 * lane)) = *reinterpret_cast<uint2*>(lo);
+          *reinterpret_cast<uint2*>(dgo + j * 1024) = *reinterpret_cast<uint2*>(hi);
+          *reinterpret_cast<uint2*>(dgo + j * 1024 + NC * 128) = *reinterpret_cast<uint2*>(lo);
         }
       }
       if (t) {
@@ -579,15 +584,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
           db[q] += pr[j][q];
           float hi, lo;
           split_tf32(pr[j][q], hi, lo);
-          *at(phi + (size_t)q * H, col + sc, a.dn_pitch) = hi;
-          *at(plo + (size_t)q * H, col + sc, a.dn_pitch) = lo;
+          at(phi, col + sc, 4 * a.dn_pitch)[(size_t)q * H] = hi;
+          at(plo, col + sc, 4 * a.dn_pitch)[(size_t)q * H] = lo;
         }
       }
       if (t == 0) break;           // (no earlier state to hand dE/dh to)
       ok = ok && mbar_wait(&acc_full, full);
       full ^= 1;
       tc_after();
-      // (columns that are not there are neither written nor sent: their part of the slot may already be filling again)
+      // (columns that are not there are not sent: what the slot's owner sends later does not come before it has this)
       if (to < C) {
         float* slot = (to == rank ? part + (size_t)pout * C * kSlot : in) + to * kSlot;
         const float* cs = colscale[t & 1];
@@ -599,8 +604,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
           tmem_ld8(tq + NC + 8 * x, z2);
           tmem_ld_wait();
 #pragma unroll
-          for (int y = 0; y < 8; ++y)
-            if (8u * x + y < n) slot[(8 * x + y) * kTcUnits + lane] = fmaf(z2[y], kLoScale, z[y]) * wscale * cs[8 * x + y];
+          for (int y = 0; y < 8; y += 4) {
+            const float4 c = *reinterpret_cast<const float4*>(cs + 8 * x + y);
+            float* o = slot + (8 * x + y) * kTcUnits + lane;
+            o[0] = fmaf(z2[y], kLoScale, z[y]) * wscale * c.x;
+            o[kTcUnits] = fmaf(z2[y + 1], kLoScale, z[y + 1]) * wscale * c.y;
+            o[2 * kTcUnits] = fmaf(z2[y + 2], kLoScale, z[y + 2]) * wscale * c.z;
+            o[3 * kTcUnits] = fmaf(z2[y + 3], kLoScale, z[y + 3]) * wscale * c.w;
+          }
         }
         if (to != rank) {
           fence_async();
