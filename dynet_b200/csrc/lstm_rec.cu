@@ -558,7 +558,7 @@ bool deal_columns(uint32_t N, int fit, int ndir, size_t col_bytes, uint32_t* G, 
 
 }  // namespace
 
-bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, bool ragged, RecPlan* out) {
+bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan* out) {
   if (H == 0 || H > 384 || N == 0) return false;
   RecPlan p;
   // up to 256 units: 32 per CTA and at most 8 CTAs, the portable cluster size; beyond: 16 CTAs
@@ -569,9 +569,9 @@ bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, bool rag
   const int ff = clusters_that_fit(ctx, p, false, fwd_threads(p)), fb = clusters_that_fit(ctx, p, true, bwd_threads(p));
   const bool sf = ff > 0 && deal_columns(N, ff, ndir, fwd_col_bytes(p), &p.Gf, &p.ncapf), sb = fb > 0 && deal_columns(N, fb, ndir, bwd_col_bytes(p), &p.Gb, &p.ncapb);
   // More than four columns per cluster: the tensor pipe, where the width lets it (256 units, a step: 1.8 us here at 3 columns,
-  // 8.0 at 37; there KERNEL_STEP_US up to 48)
-  p.tcf = !(sf && (N + p.Gf - 1) / p.Gf <= 4) && dyb200_rec_tc_plan(ctx, false, H, N, ndir, ragged, &p.tf);
-  p.tcb = !(sb && (N + p.Gb - 1) / p.Gb <= 4) && dyb200_rec_tc_plan(ctx, true, H, N, ndir, ragged, &p.tb);
+  // 8.0 at 37; there 2.5 at any number)
+  p.tcf = !(sf && (N + p.Gf - 1) / p.Gf <= 4) && dyb200_rec_tc_plan(ctx, false, H, N, &p.tf);
+  p.tcb = !(sb && (N + p.Gb - 1) / p.Gb <= 4) && dyb200_rec_tc_plan(ctx, true, H, N, &p.tb);
   if (!(sf || p.tcf) || !(sb || p.tcb)) return false;
   *out = p;
   return true;
@@ -633,7 +633,7 @@ extern "C" {
 
 int dyb200i_rec_takes(dyb200_ctx* ctx, uint32_t H, uint32_t T, uint32_t N, int ndir) {
   RecPlan p;
-  return ctx->seq_kernels && T >= kRecMinSteps && dyb200_rec_plan(ctx, H, N, ndir, false, &p) ? 1 : 0;
+  return ctx->seq_kernels && T >= kRecMinSteps && dyb200_rec_plan(ctx, H, N, ndir, &p) ? 1 : 0;
 }
 
 int dyb200i_rec_inputs(dyb200_ctx* ctx, dyb200_wgrad* w, const float* Wx, const float* b, uint32_t I, uint32_t H, uint32_t columns, float* gates) {
@@ -653,7 +653,7 @@ int dyb200i_rec_inputs(dyb200_ctx* ctx, dyb200_wgrad* w, const float* Wx, const 
 int dyb200i_rec_fwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint32_t H, uint32_t T, uint32_t N, const uint32_t* prefix_dev,
                     int mask_full, float forget_bias) {
   RecPlan p;
-  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, N, ndir, prefix_dev != nullptr, &p), "lstm recurrence: %u units x %u columns are outside its range", H, N);
+  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, N, ndir, &p), "lstm recurrence: %u units x %u columns are outside its range", H, N);
   RecFwd a;
   memset(&a, 0, sizeof(a));
   for (int k = 0; k < ndir; ++k) {
@@ -677,7 +677,7 @@ int dyb200i_rec_bwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint
                     int mask_full, uint32_t columns) {
   { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
   RecPlan p;
-  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, N, ndir, prefix_dev != nullptr, &p), "lstm recurrence: %u units x %u columns are outside its range", H, N);
+  DYB_CHECK_ARG(ctx, (ndir == 1 || ndir == 2) && dyb200_rec_plan(ctx, H, N, ndir, &p), "lstm recurrence: %u units x %u columns are outside its range", H, N);
   RecBwd a;
   memset(&a, 0, sizeof(a));
   float* db[2] = {nullptr, nullptr};

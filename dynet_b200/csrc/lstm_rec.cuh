@@ -40,18 +40,18 @@ struct RecBwd {
   uint32_t* flags;
 };
 
-// lstm_rec_tc.cu: columns per group / 16, clusters per direction.
-struct RecTcPlan { uint32_t nch, G; };
+// lstm_rec_tc.cu: clusters per direction.
+struct RecTcPlan { uint32_t G; };
 // U hidden units per CTA, C CTAs per cluster, KD / KD2 = reduction elements per lane, G clusters per direction, room for ncap
 // columns per cluster (forward, backward).  tcf / tcb: the pass runs on the tensor pipe.
 struct RecPlan { uint32_t U, C, KD, KD2, Gf, Gb, ncapf, ncapb; bool tcf, tcb; RecTcPlan tf, tb; };
 // False when the width is outside what the registers of a cluster hold, or N columns are more than the clusters can carry.
-bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, bool ragged, RecPlan* out);
+bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan* out);
 // ndir directions (1 or 2) share T, N and prefix.  U, G, ncap and flags are filled in here.
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir);
 // db[dir] (4H) += row sums of dgates over all columns (partial sums in scratch memory).
 int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db);
 int dyb200_rec_launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, dim3 grid, uint32_t threads, size_t smem);
-bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int ndir, bool ragged, RecTcPlan* out);
+bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, RecTcPlan* out);
 int dyb200_rec_tc_fwd(dyb200_ctx* ctx, const RecTcPlan& p, RecFwd* a, int ndir);
 int dyb200_rec_tc_bwd(dyb200_ctx* ctx, const RecTcPlan& p, RecBwd* a, int ndir);

@@ -6,7 +6,7 @@
 // half of the TMEM for the whole sequence; TF32 pairs of the same precision would need all of it.  (From shared memory the 32 MMAs of
 // a step took 2400 cycles, each waiting for its 4 KB of Wh.)  A step is a chain of product, cell pass and one trip through the cluster.
 //
-// Columns: a cluster takes two groups of 16 NCH neighbours.  More clusters than fit run one after the other (no cluster waits for another):
+// Columns: a cluster takes kGroups groups of 16 neighbours.  More clusters than fit run one after the other (no cluster waits for another):
 // ragged batches come longest first, so every group ends with its own longest sentence.
 //
 // Cells: a warp's lanes are the CTA's 32 units of one column, so that every access to gates, states and operand planes is a full
@@ -29,11 +29,13 @@
 namespace {
 
 // Two groups of columns per CTA, each with its own loop, barriers and buffers (only Wh is shared): one's cell pass runs beside the other's
-// product and messages.  Warps 0 and 1 issue the groups' products and copies (the oldest warps of their schedulers go first), 2 .. 9
-// and 10 .. 17 are the groups' cell warps.
+// product and messages (one group of 32 or 64 columns: 302 and 450 us where two of 16 take 247 and 278, 256 sentences of up to 100
+// words; two of 32 spill registers, three of 16 too).  Warps 0 and 1 issue the groups' products and copies (the oldest warps of their
+// schedulers go first), 2 .. 9 and 10 .. 17 are the groups' cell warps.
 constexpr uint32_t kGroups = 2, kGroupWarps = 8, kGroupThreads = 32 * kGroupWarps;
 constexpr uint32_t kCellThreads = kGroups * kGroupThreads, kTcThreads = kCellThreads + 32 * kGroups;
 constexpr uint32_t kTcUnits = 32;      // hidden units per CTA
+constexpr uint32_t kTcCols = 16;       // columns per group
 
 // Positions of a column's K-major operand row: byte offset of element k (even or odd) of row r in a plane block of `rows` rows per 64 k.
 __device__ __forceinline__ uint32_t op_off(uint32_t rows, uint32_t r, uint32_t k) {
@@ -122,9 +124,8 @@ __device__ __forceinline__ void tc_kstep(uint32_t wide, uint32_t narrow, uint32_
 // h [2][2 KB blocks of 32 units][NC hi rows, NC lo rows][64 bytes]; gates on their way [NC][4][32]; KB = ceil(H / 64).
 // TMEM: each group's accumulators (3 NC columns: A_hi B_hi, A_hi B_lo, A_lo B_hi - the last apart, so that the chain of one waits on
 // the other's MMAs, not on its own), Wh_hi and Wh_lo (32 KB columns each).
-template <int NCH>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_constant__ RecFwd a) {
-  constexpr uint32_t NC = 16 * NCH, kBlock = 2 * NC * 64;   // bytes of a CTA's part of h
+  constexpr uint32_t NC = kTcCols, kBlock = 2 * NC * 64;   // bytes of a CTA's part of h
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t got_[kGroups][2], acc_full_[kGroups], h_ready_[kGroups];
   __shared__ uint32_t tmem_slot, hword_[kGroups][2], wmax[128];
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     }
   } else {
     // reads gate `quad` of the columns 16 j + c8 .. + 7, finishes columns 16 j + c8 + quad and + 4; lane = unit
-    constexpr int kCells = 2 * NCH;
+    constexpr int kCells = NC / 8;
     const uint32_t quad = warp & 3, c8 = 8 * (gw >> 2), u = rank * kTcUnits + lane, i0 = c8 + quad;
     const bool live_u = u < H;
     const uint32_t uc = min(u, H - 1);                  // (units that are not there read another's values and store nothing)
@@ -277,14 +278,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     const uint32_t tq = tmem + grp * 3 * NC + ((32 * quad) << 16) + c8;
     const float* mask = d.mask ? d.mask + uc : nullptr;
     float *pg = d.gates + uc, *pc = d.c + uc, *ph = d.h + uc, *phi = d.hn_hi ? d.hn_hi + uc : nullptr, *plo = phi ? d.hn_lo + uc : nullptr;
-    float pre[kCells][4], cst[kCells], mk[kCells];
+    float pre[kCells][4], ahead[kCells][4], cst[kCells], mk[kCells];   // (ahead: of the next step, requested a whole step before its use)
     uint32_t ho[kCells];                                   // where h of cell j goes in this CTA's block
     auto fetch = [&](uint32_t c0, uint32_t nact) {
 #pragma unroll
       for (int j = 0; j < kCells; ++j) {
         const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), col = c0 + base + (i < nact ? i : 0);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pre[j][q] = at(pg, col, 16 * H)[(size_t)q * H];
+        for (int q = 0; q < 4; ++q) ahead[j][q] = at(pg, col, 16 * H)[(size_t)q * H];
       }
     };
     if (n) fetch(0, n);          // (a group may have no column at all)
@@ -300,10 +301,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       unsigned char* hnext = hbuf + ((t & 1) ^ 1) * hbytes;
       const int ts = t ? t1 : t0, th = ts >> 1;
       const float f0 = __int_as_float((th + 127) << 23), f1 = __int_as_float((ts - th + 127) << 23);
+#pragma unroll
+      for (int j = 0; j < kCells; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) pre[j][q] = ahead[j][q];
+      if (n1) fetch(col1, n1);
       ok = ok && mbar_wait(&acc_full, t & 1);
       tc_after();
 #pragma unroll
-      for (int j = 0; j < NCH; ++j) {
+      for (int j = 0; j < (int)NC / 16; ++j) {
         float z[8], z2[8], z3[8];
         tmem_ld8(tq + 16 * j, z);
         tmem_ld8(tq + NC + 16 * j, z2);
@@ -353,7 +359,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
           *at(plo, col1 + sc, 4 * a.hn_pitch) = lo;
         }
       }
-      if (n1) fetch(col1, n1);
       col0 = col1; col1 = col2; col2 = col3; n = n1;
     }
   }
@@ -373,9 +378,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
 // units the accumulators (2 NC columns); then Wh^T hi and lo (64 columns each per row tile).  The slots of the sums that have just been
 // read hold the outgoing ones: what comes into slot r next, rank r sends after it has what went out of that slot.  Gate row (unit ul,
 // gate q) is element 4 ul + q of the reduction.
-template <int NCH>
+template <bool DC>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_constant__ RecBwd a) {
-  constexpr uint32_t NC = 16 * NCH, kSlot = NC * kTcUnits;
+  constexpr uint32_t NC = kTcCols, kSlot = NC * kTcUnits;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t got_[kGroups][2], acc_full_[kGroups];
   __shared__ uint32_t tmem_slot, wmax[256];
@@ -436,7 +441,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
         v[q][x] = w;
         m = max(m, max(max(finite_mag(w.x), finite_mag(w.y)), max(finite_mag(w.z), finite_mag(w.w))));
       }
-    atomicMax(&wmax[o], m);
+    if (mt < 2) atomicMax(&wmax[o], m);
     bar_sync(1, kCellThreads);
     if (mt < MT) {
       const float scale = scale_of(wmax[o]);
@@ -484,7 +489,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
       __syncwarp();
     }
   } else {
-    constexpr int kCells = 2 * NCH;
+    constexpr int kCells = NC / 8;
     const uint32_t u = rank * kTcUnits + lane;
     const bool live_u = u < H;
     const uint32_t uc = min(u, H - 1);                   // (units that are not there read another's values and store nothing)
@@ -493,9 +498,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     const float wscale = __int_as_float((scale_field(wmax[32 * to + lane]) - 14) << 23);   // (undoes the scale of the row this lane reads)
     const uint32_t tq = tmem + (grp * MT + mt) * 2 * NC + ((32 * quad) << 16);
     const float *pg = d.gates + uc, *pc = d.c + uc, *pc0 = d.c0 ? d.c0 + uc : nullptr;
-    float *pdh = d.dh + uc, *pdc = d.dc ? d.dc + uc : nullptr, *phi = d.dn_hi + uc, *plo = d.dn_lo + uc;
+    float *pdh = d.dh + uc, *pdc = DC ? d.dc + uc : nullptr, *phi = d.dn_hi + uc, *plo = d.dn_lo + uc;
     uint32_t phase[2] = {0, 0};
-    float gt[kCells][4], cv[kCells], cp[kCells], dhv[kCells], dcv[kCells], dcs[kCells], mk[kCells];
+    float gt[kCells][4], cv[kCells], cp[kCells], dhv[kCells], dcv[kCells], dcs[kCells];
     unsigned char* dgo = dgb + op_off(2 * NC, gw, 4 * lane);   // (eight columns on: 1024 bytes)
     // cell j: column 8 j + gw
     auto fetch = [&](bool first, uint32_t c0, uint32_t cm1, uint32_t nact) {
@@ -509,7 +514,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
         cp[j] = dcv[j] = 0.f;
         const float* before = first ? pc0 : pc;
         if (before) cp[j] = *at(before, first ? sc : cm1 + sc, 4 * H);
-        if (pdc) dcv[j] = *at(pdc, c0 + sc, 4 * H);
+        if (DC) dcv[j] = *at(pdc, c0 + sc, 4 * H);
       }
     };
     // first columns of the steps t, t - 1, t - 2, each read a step before it is needed; columns active at step t
@@ -517,9 +522,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     uint32_t n = T ? tc_active(start_of(T) - col, base, NC) : 0;
 #pragma unroll
     for (int j = 0; j < kCells; ++j) {
-      const uint32_t sc = base + 8 * j + gw;
       dcs[j] = 0.f;
-      mk[j] = d.mask && sc < a.N ? __ldg(at(d.mask + uc, a.mask_full ? sc : 0, 4 * H)) : 1.f;
     }
     if (T) fetch(T == 1, col, colm1, n);
     uint32_t n_later = 0, full = 0;
@@ -545,10 +548,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
 #pragma unroll
             for (int q = 0; q < 8; ++q)
               if ((uint32_t)q < C) r += from[(size_t)q * kSlot];
-            dh = fmaf(r, mk[j], dh);
+            dh = d.mask ? fmaf(r, __ldg(at(d.mask + uc, a.mask_full ? sc : 0, 4 * H)), dh) : dh + r;
             if (live_u) {
               *at(pdh, col + sc, 4 * H) = dh;
-              if (pdc) *at(pdc, col + sc, 4 * H) = dci;
+              if (DC) *at(pdc, col + sc, 4 * H) = dci;
             }
           }
           lstm_cell_grad(gt[j][0], gt[j][1], gt[j][2], gt[j][3], cv[j], cp[j], dh, dci, true, dcp, pr[j][0], pr[j][1], pr[j][2], pr[j][3]);
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
         float* slot = (to == rank ? part + (size_t)pout * C * kSlot : in) + to * kSlot;
         const float* cs = colscale[t & 1];
 #pragma unroll
-        for (int x = 0; x < 2 * NCH; ++x) {
+        for (int x = 0; x < (int)NC / 8; ++x) {
           if (8u * x >= n) break;
           float z[8], z2[8];
           tmem_ld8(tq + 8 * x, z);
@@ -638,7 +641,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(MT * (kGroups * 2 * NC + 128))) : "memory");
   }
   if (warp >= kGroups) {
-    // row sums of dgates: the sixteen threads of a unit, in ascending order (part is free: every CTA is through)
+    // row sums of dgates: the threads of a unit, in ascending order (part is free: every CTA is through)
 #pragma unroll
     for (int q = 0; q < 4; ++q) partall[((warp - kGroups) * 4 + q) * kTcUnits + lane] = db[q];
   }
@@ -647,68 +650,56 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     const uint32_t q = tid / kTcUnits, ul = tid % kTcUnits, u = rank * kTcUnits + ul;
     if (u < H) {
       float r = 0.f;
-      for (uint32_t k = 0; k < 16; ++k) r += partall[(k * 4 + q) * kTcUnits + ul];
+      for (uint32_t k = 0; k < kCellThreads / 32; ++k) r += partall[(k * 4 + q) * kTcUnits + ul];
       d.dbpart[(size_t)g * 4 * H + q * H + u] = r;
     }
   }
 }
 
-// nch: 16 columns per group
-uint32_t tc_smem(bool bwd, uint32_t H, uint32_t nch) {
-  const uint32_t NC = 16 * nch, KB = (H + 63) / 64, C = (H + kTcUnits - 1) / kTcUnits;
-  // (the partial sums' room also holds the 16 x 128 row sums of dgates at the end: 8 KB at least)
+uint32_t tc_smem(bool bwd, uint32_t H) {
+  const uint32_t NC = kTcCols, KB = (H + 63) / 64, C = (H + kTcUnits - 1) / kTcUnits;
+  // (the partial sums' room also holds the row sums of dgates at the end, 512 bytes per cell warp)
   return 1024 + kGroups * (bwd ? 2 * 2 * NC * 128 + 2 * C * NC * kTcUnits * 4 : 2 * 2 * KB * 2 * NC * 64 + NC * 512);
 }
-typedef void (*TcFwdKernel)(RecFwd);
-typedef void (*TcBwdKernel)(RecBwd);
-TcFwdKernel tc_fwd(uint32_t nch) { return nch == 1 ? k_rec_tc_fwd<1> : k_rec_tc_fwd<2>; }
-TcBwdKernel tc_bwd(uint32_t nch) { return nch == 1 ? k_rec_tc_bwd<1> : k_rec_tc_bwd<2>; }
-const void* tc_kernel(bool bwd, uint32_t nch) { return bwd ? (const void*)tc_bwd(nch) : (const void*)tc_fwd(nch); }
 
 }  // namespace
 
-// Columns per group / 16 (1 or 2) and clusters per direction.  A step of 2 x 32 columns takes about one and a half times as long as one of
-// 2 x 16; what counts is the rounds of clusters that each needs - in fractions for ragged batches, whose last round is short.
-bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int ndir, bool ragged, RecTcPlan* out) {
+// Clusters per direction (of kGroups x 16 columns each).
+bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, RecTcPlan* out) {
   if (H > 256 || N == 0) return false;
   const uint32_t C = (H + kTcUnits - 1) / kTcUnits;
   int16_t& fit = ctx->rec_tc_fit[bwd][C - 1];
-  if (fit == 0) {
+  if (fit == 0) {   // (asked once: whether a cluster fits this device at all)
+    const void* k = bwd ? (const void*)k_rec_tc_bwd<true> : (const void*)k_rec_tc_fwd;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    if (dyb200_rec_launch_cfg(ctx, tc_kernel(bwd, 2), &cfg, attr, dim3(C, 1, 1), kTcThreads, tc_smem(bwd, H, 2))) return false;
+    if (dyb200_rec_launch_cfg(ctx, k, &cfg, attr, dim3(C, 1, 1), kTcThreads, tc_smem(bwd, H))) return false;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, tc_kernel(bwd, 2), &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
     fit = (int16_t)(n > 0 ? n : -1);
   }
   if (fit <= 0) return false;
-  const uint32_t side = fit > ndir ? (uint32_t)(fit / ndir) : 1u;   // clusters per direction that run at the same time
-  double rounds[2];
-  for (int k = 0; k < 2; ++k) {
-    const uint32_t per = kGroups * 16 * (k + 1), c = (N + per - 1) / per;
-    rounds[k] = c <= side ? 1.0 : ragged ? (double)c / side : (double)((c + side - 1) / side);
-  }
-  out->nch = rounds[0] <= 1.5 * rounds[1] ? 1 : 2;
-  out->G = (N + kGroups * 16 * out->nch - 1) / (kGroups * 16 * out->nch);
+  out->G = (N + kGroups * kTcCols - 1) / (kGroups * kTcCols);
   return true;
 }
 int dyb200_rec_tc_fwd(dyb200_ctx* ctx, const RecTcPlan& p, RecFwd* a, int ndir) {
-  a->G = p.G; a->ncap = 16 * p.nch; a->ndir = (uint32_t)ndir; a->flags = ctx->dev_flags;
+  a->G = p.G; a->ndir = (uint32_t)ndir; a->flags = ctx->dev_flags;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  int rc = dyb200_rec_launch_cfg(ctx, tc_kernel(false, p.nch), &cfg, attr, dim3((a->H + kTcUnits - 1) / kTcUnits, p.G * ndir, 1), kTcThreads, tc_smem(false, a->H, p.nch));
+  int rc = dyb200_rec_launch_cfg(ctx, (const void*)k_rec_tc_fwd, &cfg, attr, dim3((a->H + kTcUnits - 1) / kTcUnits, p.G * ndir, 1), kTcThreads, tc_smem(false, a->H));
   if (rc) return rc;
-  cudaLaunchKernelEx(&cfg, tc_fwd(p.nch), *a);
+  cudaLaunchKernelEx(&cfg, k_rec_tc_fwd, *a);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
 int dyb200_rec_tc_bwd(dyb200_ctx* ctx, const RecTcPlan& p, RecBwd* a, int ndir) {
-  a->G = p.G; a->ncap = 16 * p.nch; a->ndir = (uint32_t)ndir; a->flags = ctx->dev_flags;
+  a->G = p.G; a->ndir = (uint32_t)ndir; a->flags = ctx->dev_flags;
+  void (*k)(RecBwd) = a->d[0].dc ? k_rec_tc_bwd<true> : k_rec_tc_bwd<false>;   // (both directions give dE/dc or neither)
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  int rc = dyb200_rec_launch_cfg(ctx, tc_kernel(true, p.nch), &cfg, attr, dim3((a->H + kTcUnits - 1) / kTcUnits, p.G * ndir, 1), kTcThreads, tc_smem(true, a->H, p.nch));
+  int rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3((a->H + kTcUnits - 1) / kTcUnits, p.G * ndir, 1), kTcThreads, tc_smem(true, a->H));
   if (rc) return rc;
-  cudaLaunchKernelEx(&cfg, tc_bwd(p.nch), *a);
+  cudaLaunchKernelEx(&cfg, k, *a);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
