@@ -137,7 +137,8 @@ def test_softmax_dim0(oracle, g, capi, rows, cols, bd):
     assert_close(g.host(d_), want, TOL_REDUCE, floor=ACC_FLOOR, what="softmax d0 bwd")
 
 
-@pytest.mark.parametrize("rows,cols,bd", [(1, 5, 1), (7, 3, 2), (33, 200, 2), (64, 4096, 1), (9, 4500, 1)])
+@pytest.mark.parametrize("rows,cols,bd", [(1, 5, 1), (7, 3, 2), (33, 200, 2), (64, 4096, 1), (9, 4500, 1),
+                                          (4, 1, 3), (20, 129, 2), (16, 256, 1), (36, 257, 2), (100, 1024, 1), (68, 1025, 1), (4096, 50, 1)])
 def test_softmax_dim1(oracle, g, capi, rows, cols, bd):
     r = rng(121)
     x = randn(r, bd, cols, rows, scale=2.0)
