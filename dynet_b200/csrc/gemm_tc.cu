@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t s = 0, ph = 0;
       for (uint32_t it = 0; it < total; ++it) {
         if (!mbar_wait(&empty_bar[s], ph ^ 1)) { atomicOr(flags, DYB200_FLAG_WAIT_TIMEOUT); break; }
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
       asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // This one thread issues every MMA of the tile, and the tensor pipe is only as busy as this loop is short:
       // descriptors of the three stages are built once, stage / phase / chunk counters are carried instead of divided,
       // and the 12 MMAs of a k-block go out in one block of PTX.
@@ -426,9 +426,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) persist_producer<BNT, F16>(&tm, ring, full_bar, empty_bar, tiles, tiles_m, (N + BNT - 1) / BNT, gm, kb0, kb1, S, flags);
+    if (elect_one()) persist_producer<BNT, F16>(&tm, ring, full_bar, empty_bar, tiles, tiles_m, (N + BNT - 1) / BNT, gm, kb0, kb1, S, flags);
   } else if (warp == 1) {
-    if (lane == 0) persist_issue<BNT, F16>(ring, full_bar, empty_bar, acc_full, acc_empty, tmem_base, tiles, kb0, kb1, S, tm.a_mn, tm.b_mn, flags);
+    if (elect_one()) persist_issue<BNT, F16>(ring, full_bar, empty_bar, acc_full, acc_empty, tmem_base, tiles, kb0, kb1, S, tm.a_mn, tm.b_mn, flags);
   } else {
     // epilogue warps 2..9: TMEM lanes 32 (warp % 4) .. +31; warps 2-5 hold columns 0-63 of the tile, warps 6-9 columns 64-127
     const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;

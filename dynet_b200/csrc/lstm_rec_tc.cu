@@ -90,12 +90,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
                "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// one lane of a converged warp, in a form that lets the compiler keep the MMAs' operands in uniform registers
-__device__ __forceinline__ bool elect_one() {
-  uint32_t e;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(e)::"memory");
-  return e != 0;
-}
 // p + col * bytes: one multiply-add of 32 x 32 + 64 bits (indexing by floats adds a shift of 64 bits to every address; addresses were a
 // third of the cell passes' instructions)
 __device__ __forceinline__ float* at(float* p, uint32_t col, uint32_t bytes) { return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + (uint64_t)col * bytes); }

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // TMA producer.  Step t reads Wx / Wh rows [m0, m0 + 128) and the operand planes of columns [t B + n0, + BNT).
       uint32_t s = 0, ph = 0;
       bool fail = false;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
       if (fail) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BNT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       uint64_t d_a_hi[kStages], d_a_lo[kStages], d_b_hi[kStages], d_b_lo[kStages];
 #pragma unroll

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_bwd(const __grid_const
   const uint32_t tmem_base = tmem_base_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // TMA producer.  Every product reads rows [m0, m0 + 128) of [Wx; Wh]^T and rows [t B + n0, + BNT) of the dgates planes.
       uint32_t s = 0, ph = 0;
       bool fail = false;
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_bwd(const __grid_const
       if (fail) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BNT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       uint64_t d_a_hi[kStages], d_a_lo[kStages], d_b_hi[kStages], d_b_lo[kStages];
 #pragma unroll

@@ -83,6 +83,36 @@ __global__ void __launch_bounds__(kBlock) k_weight_norm_dg(const float* __restri
   if (threadIdx.x == 0) dg[0] += dot / sqrtf(ss);
 }
 
+// The three of them for a tensor that one CTA reads in less time than a second launch takes: the sums and what follows from them in one
+// kernel.  MODE 0, 1 as above; 2: dg += dot / |w|, out = dg.
+constexpr size_t kWeightNormSmall = 16384;
+template <int MODE>
+__global__ void __launch_bounds__(1024) k_weight_norm_small(const float* __restrict__ w, const float* __restrict__ gptr, const float* __restrict__ y,
+                                                            const float* __restrict__ dy, float* __restrict__ out, uint32_t n) {
+  dyb_grid_dep_sync();
+  __shared__ float red[32];
+  float ss = 0.f, dot = 0.f;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < n; i += 1024) {
+    const float a = w[i];
+    ss += a * a;
+    if (MODE) dot += a * dy[i];
+  }
+  ss = block_sum(ss, red);
+  if (MODE) dot = block_sum(dot, red);
+  const float nrm = sqrtf(ss);
+  if (MODE == 2) {
+    if (threadIdx.x == 0) out[0] += dot / nrm;
+    return;
+  }
+  const float sc = gptr[0] / nrm, t2 = dot / ss;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < n; i += 1024) {
+    if (MODE == 0) out[i] = w[i] * sc;
+    else out[i] += dy[i] * sc - y[i] * t2;
+  }
+}
+
 // ---------------------------------------------------------------- moments
 // View of the input as (d0, d1, d2, bd) with a reduce mask per axis.
 struct Axes {
@@ -411,6 +441,39 @@ struct LnDg {
     return dy[(size_t)b * n + r] * ((x[(size_t)b * n + r] + (-mean)) / s2);
   }
 };
+// Gain gradient of a small layer norm in one launch: every CTA forms the statistics of all columns (a warp per column; at most 64 KB, from
+// L2) and sums its 128 rows over them.
+constexpr size_t kLnDgSmall = 16384;
+constexpr uint32_t kLnDgCols = 256;
+__global__ void __launch_bounds__(kBlock) k_layer_norm_dg_small(const float* __restrict__ x, const float* __restrict__ dy, uint32_t n, uint32_t ncols,
+                                                                float* __restrict__ dg) {
+  dyb_grid_dep_sync();
+  __shared__ float stats[2 * kLnDgCols];
+  __shared__ float half[128];
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t c = threadIdx.x >> 5; c < ncols; c += kBlock / 32) {
+    const float* xc = x + (size_t)c * n;
+    float s = 0.f, q = 0.f;
+#pragma unroll 4
+    for (uint32_t i = lane; i < n; i += 32) s += xc[i];
+    const float mean = warp_sum(s) / (float)n;
+#pragma unroll 4
+    for (uint32_t i = lane; i < n; i += 32) { const float d = xc[i] - mean; q += d * d; }
+    q = warp_sum(q);
+    if (lane == 0) { stats[2 * c] = mean; stats[2 * c + 1] = sqrtf(q / (float)n); }
+  }
+  __syncthreads();
+  const LnDg f{x, dy, stats, n};
+  const uint32_t r = blockIdx.x * 128 + (threadIdx.x & 127), h = threadIdx.x >> 7, mid = (ncols + 1) / 2;
+  float acc = 0.f;
+  if (r < n) {
+#pragma unroll 8
+    for (uint32_t b = h ? mid : 0; b < (h ? ncols : mid); ++b) acc += f(r, b);
+  }
+  if (h) half[threadIdx.x & 127] = acc;
+  __syncthreads();
+  if (!h && r < n) dg[r] += acc + half[threadIdx.x];
+}
 struct LnDb {
   const float* dy;
   size_t n;
@@ -463,6 +526,11 @@ int dyb200_weight_norm_fwd(DYB200_FWD_ARGS) {
   size_t n = t_size(&xs[0]);
   DYB_CHECK_ARG(ctx, t_size(fx) == n, "WeightNormalization: output size mismatch");
   if (n == 0) return DYB200_OK;
+  if (n <= kWeightNormSmall) {
+    dyb_launch(k_weight_norm_small<0>, 1, 1024, 0, ctx, xs[0].v, xs[1].v, nullptr, nullptr, fx->v, (uint32_t)n);
+    DYB_LAUNCHED(ctx);
+    return DYB200_OK;
+  }
   int np = ctx->sm_count * 4;
   void* partial;
   int rc = dyb200_scratch(ctx, 2 * np * sizeof(float), &partial);
@@ -481,6 +549,11 @@ int dyb200_weight_norm_bwd(DYB200_BWD_ARGS) {
   size_t n = t_size(&xs[0]);
   DYB_CHECK_ARG(ctx, t_size(dEdf) == n && t_size(fx) == n && t_size(dEdxi) == (i == 0 ? n : 1), "WeightNormalization::backward: size mismatch");
   if (n == 0) return DYB200_OK;
+  if (n <= kWeightNormSmall) {
+    dyb_launch(i == 0 ? k_weight_norm_small<1> : k_weight_norm_small<2>, 1, 1024, 0, ctx, xs[0].v, xs[1].v, fx->v, dEdf->v, dEdxi->v, (uint32_t)n);
+    DYB_LAUNCHED(ctx);
+    return DYB200_OK;
+  }
   int np = ctx->sm_count * 4;
   void* partial;
   int rc = dyb200_scratch(ctx, 2 * np * sizeof(float), &partial);
@@ -602,6 +675,11 @@ int dyb200_layer_norm_bwd(DYB200_BWD_ARGS) {
   if (i == 2) {
     LnDb f{dEdf->v, n};
     return batch_reduce_add(ctx, f, n, (uint32_t)ncols, dEdxi->v);
+  }
+  if (n * ncols <= kLnDgSmall && ncols <= kLnDgCols) {
+    dyb_launch(k_layer_norm_dg_small, (unsigned)((n + 127) / 128), kBlock, 0, ctx, xs[0].v, dEdf->v, (uint32_t)n, (uint32_t)ncols, dEdxi->v);
+    DYB_LAUNCHED(ctx);
+    return DYB200_OK;
   }
   // i == 1: per-column statistics first
   void* arena;

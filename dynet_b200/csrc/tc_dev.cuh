@@ -129,6 +129,13 @@ __device__ __forceinline__ uint64_t umma_desc_mn16(uint32_t smem_addr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
+// One lane of a converged warp, in a form that lets the compiler keep the operands of MMAs and TMA loads in uniform registers: from a
+// plain lane test each MMA of a chain took about 70 cycles to issue, more than a 128 x 64 one takes to run.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(e)::"memory");
+  return e != 0;
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

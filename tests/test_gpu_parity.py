@@ -347,7 +347,7 @@ def test_pickneglogsoftmax_errors(g, capi):
 
 
 # ------------------------------------------------------------------ norms
-@pytest.mark.parametrize("n", [9, 1000, 4096 * 3 + 1, 1024 * 4096])
+@pytest.mark.parametrize("n", [9, 1000, 4096 * 3 + 1, 1024 * 4096, 1, 16384, 16385])
 def test_weight_norm(oracle, g, n):
     r = rng(130)
     w = randn(r, n) + 0.1
@@ -417,7 +417,8 @@ def test_std_dim_value_golden(g, capi):
 
 
 @pytest.mark.parametrize("n,bd", [(3, 1), (10, 1), (130, 5), (4096, 16), (4100, 3), (9001, 2),
-                                  (128, 37), (256, 9), (640, 21), (1024, 300)])   # (the last four: a warp per column)
+                                  (128, 37), (256, 9), (640, 21), (1024, 300),      # (these four: a warp per column)
+                                  (60, 256), (60, 270), (129, 127)])
 def test_layer_norm(oracle, g, n, bd):
     r = rng(132)
     x = randn(r, bd, n)
