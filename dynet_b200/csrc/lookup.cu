@@ -247,6 +247,73 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_ids(const uint32_t* __res
   }
 }
 
+// The same for tables of fewer than 2^20 rows: the id and the position within the pass are one 32-bit key, four neighbouring keys per
+// thread.  Exchanges over less than 128 keys stay in a warp (registers and shuffles); the 15 longer ones of 4096 keys go through shared
+// memory, two buffers taken in turn, one barrier each.  4096 ids: 39 us with every one of the 78 exchanges of 64-bit keys in shared
+// memory, SORT32 here.
+constexpr uint32_t kSort32Vocab = (1u << 20) - 1;
+__global__ void __launch_bounds__(kSortThreads) k_sort_ids32(const uint32_t* __restrict__ ids, uint32_t n_total, uint32_t vocab,
+                                                            uint32_t* __restrict__ pos_sorted, uint32_t* __restrict__ id_at, uint32_t* flags) {
+  dyb_grid_dep_sync();
+  __shared__ uint4 buf[2][kSortThreads];
+  const uint32_t base = blockIdx.x * kSortMax, t = threadIdx.x;
+  const uint32_t n = min((uint32_t)kSortMax, n_total - base);
+  uint32_t npow = 128;
+  while (npow < n) npow <<= 1;
+  const bool active = 4 * t < npow;   // (whole warps)
+  uint32_t v[4];
+#pragma unroll
+  for (uint32_t r = 0; r < 4; ++r) {
+    const uint32_t k = 4 * t + r;
+    v[r] = 0xffffffffu;
+    if (k < n) {
+      uint32_t id = ids[base + k];
+      if (id >= vocab) { atomicOr(flags, DYB200_FLAG_BAD_INDEX); id = vocab - 1; }
+      v[r] = id << 12 | k;
+    }
+  }
+  uint32_t turn = 0;
+  for (uint32_t size = 2; size <= npow; size <<= 1) {
+    const bool up4 = (4 * t & size) == 0;             // direction of this thread's keys (sizes from 4 on)
+    for (uint32_t stride = size >> 1; stride >= 128; stride >>= 1) {
+      if (active) buf[turn][t] = make_uint4(v[0], v[1], v[2], v[3]);
+      __syncthreads();
+      if (active) {
+        const uint4 o = buf[turn][t ^ (stride >> 2)];
+        const bool least = ((4 * t & stride) == 0) == up4;
+        v[0] = least ? min(v[0], o.x) : max(v[0], o.x); v[1] = least ? min(v[1], o.y) : max(v[1], o.y);
+        v[2] = least ? min(v[2], o.z) : max(v[2], o.z); v[3] = least ? min(v[3], o.w) : max(v[3], o.w);
+      }
+      turn ^= 1;
+    }
+    if (!active) continue;
+    for (uint32_t stride = min(size >> 1, 64u); stride >= 4; stride >>= 1) {
+      const bool least = ((4 * t & stride) == 0) == up4;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], stride >> 2);
+        v[r] = least ? min(v[r], o) : max(v[r], o);
+      }
+    }
+    auto order = [&](uint32_t& a, uint32_t& b, bool up) {
+      const uint32_t lo = min(a, b), hi = max(a, b);
+      a = up ? lo : hi;
+      b = up ? hi : lo;
+    };
+    if (size > 2) { order(v[0], v[2], up4); order(v[1], v[3], up4); }
+    order(v[0], v[1], size == 2 ? true : up4);
+    order(v[2], v[3], size == 2 ? false : up4);
+  }
+#pragma unroll
+  for (uint32_t r = 0; r < 4; ++r) {
+    const uint32_t k = 4 * t + r;
+    if (k < n) {
+      pos_sorted[base + k] = base + (v[r] & 4095);
+      id_at[base + k] = v[r] >> 12;
+    }
+  }
+}
+
 // Merges the sorted runs of k_sort_ids (run p = positions [p kSortMax, ...), sorted by (id, position)) into one sorted list:
 // one thread per element, whose place is the number of smaller keys in every run.  Positions grow with the run number, so
 // among equal ids the earlier run comes first: runs before the element's own count their ids <= id, later runs their ids < id.
@@ -300,11 +367,16 @@ __global__ void __launch_bounds__(256) k_chunk_add(const float* __restrict__ g, 
     float* tslot = tail + ((size_t)c * slices + sl) * 128 + lane * 4;
     for (uint32_t j0 = 0; j0 < k1 - k0; j0 += 8) {
       // the gradient rows of the next 8 positions are requested together; the adds stay in order
-      float4 rows[8];
+      // and so are the table rows that runs start from (requested at each new id, one after the other, they made a chunk of 32
+      // rare words 14 us long)
+      float4 rows[8], start[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const uint32_t pos = __shfl_sync(0xffffffffu, my_pos, (j0 + u) & 31);
-        rows[u] = (live && j0 + u < k1 - k0) ? ld4_stream(g + (size_t)pos * E + col) : zero4;
+        const uint32_t pos = __shfl_sync(0xffffffffu, my_pos, (j0 + u) & 31), id = __shfl_sync(0xffffffffu, my_id, (j0 + u) & 31);
+        const uint32_t before = __shfl_sync(0xffffffffu, my_id, (j0 + u - 1) & 31);
+        const bool in = live && j0 + u < k1 - k0;
+        rows[u] = in ? ld4_stream(g + (size_t)pos * E + col) : zero4;
+        start[u] = in && j0 + u > 0 && id != before ? ld4(all_grads + (size_t)id * E + col) : zero4;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
@@ -317,7 +389,7 @@ __global__ void __launch_bounds__(256) k_chunk_add(const float* __restrict__ g, 
             }
             cur = id;
             started_before = false;
-            acc = live ? ld4(all_grads + (size_t)cur * E + col) : zero4;
+            acc = start[u];
           }
           add4(acc, rows[u]);
         }
@@ -396,7 +468,7 @@ static int scatter_run_chunked(dyb200_ctx* ctx, unsigned n, const unsigned* ids_
   float* head = (float*)(((uintptr_t)(id_all + (merged ? 3 : 1) * (size_t)n) + 255) & ~(uintptr_t)255);
   float* tail = head + (size_t)((np_max + kChunk - 1) / kChunk) * slices * 128;
   // every pass's ids are sorted in the same launch (one CTA each)
-  dyb_launch(k_sort_ids, npass, kSortThreads, 0, ctx, ids_dev, n, vocab, pos_all, id_all, ctx->dev_flags);
+  dyb_launch(vocab <= kSort32Vocab ? k_sort_ids32 : k_sort_ids, npass, kSortThreads, 0, ctx, ids_dev, n, vocab, pos_all, id_all, ctx->dev_flags);
   DYB_LAUNCHED(ctx);
   if (merged) {
     dyb_launch(k_merge_runs, (n + 255) / 256, 256, 0, ctx, (const uint32_t*)pos_all, (const uint32_t*)id_all, n, pos_m, id_m);

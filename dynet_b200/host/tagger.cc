@@ -84,8 +84,10 @@ struct Tagger {
   float *hf, *hr, *dhf, *dhr, *pre, *th, *dth, *dpre, *logits, *dlogits, *errs, *aux, *ones, *zeros, *scalars;
   // pointer / length tables of the four mover calls (device) and their pinned host staging
   float** tbl_dev; size_t* len_dev;
-  float** tbl_host;   // pinned: 8 N pointers, N lengths, then the ids (2 N words + N tags) and the first columns of the steps
-  size_t dact_off0, dact_off1;
+  float** tbl_host;   // pinned: 8 N pointers, N lengths; ids_host lies behind them
+  uint32_t* ids_dev;   // see ids_words
+  uint32_t* ids_host;
+  size_t dact_off0, dact_rec, dact_off1;
   char* ws;
   bool time_movers = false;
   cudaEvent_t ev[8];
@@ -97,18 +99,30 @@ struct Tagger {
   cudaStream_t stream2 = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   double host_schedule_ms = 0.0;
-  uint32_t* prefix_dev = nullptr;   // first column of every step, and their end
+  // The mover calls' tables (72 bytes a token) are not needed before the recurrence is through: they go over beside it.
+  cudaStream_t copy_stream = nullptr;
+  cudaEvent_t tables_ev = nullptr, pass_ev = nullptr;   // tables uploaded / the last pass has read them
+  bool pass_recorded = false;
   ~Tagger() {
+    if (copy_stream) { cudaStreamSynchronize(copy_stream); cudaStreamDestroy(copy_stream); }   // (before its source goes)
     for (int k = 0; k < 2; ++k) if (d[k].wg) dyb200_wgrad_destroy(d[k].wg);
     if (tbl_host) cudaFreeHost(tbl_host);
     for (auto& e : ev) if (e) cudaEventDestroy(e);
     if (upload_ev) cudaEventDestroy(upload_ev);
     if (fork_ev) cudaEventDestroy(fork_ev);
     if (join_ev) cudaEventDestroy(join_ev);
+    if (tables_ev) cudaEventDestroy(tables_ev);
+    if (pass_ev) cudaEventDestroy(pass_ev);
     if (dev2.ctx) dyb200_ctx_destroy(dev2.ctx);
     if (stream2) cudaStreamDestroy(stream2);
   }
 };
+
+// Words of one mini-batch on the device, uploaded in one piece: the ids of the two directions' columns (2 N), the tag layer's aux
+// memory (from the next multiple of four; 2 N floats of the node, then the N tags) and the first columns of the steps.
+size_t aux_at(size_t N) { return (2 * N + 3) / 4 * 4; }
+size_t prefix_at(size_t N) { return aux_at(N) + 3 * N; }
+size_t ids_words(size_t N, size_t steps) { return prefix_at(N) + steps + 1; }
 
 size_t plan(const dyb200h_tagger_config& c, uint32_t S, uint32_t N, Tagger* t, char* base) {
   Arena a{base, 0};
@@ -116,29 +130,31 @@ size_t plan(const dyb200h_tagger_config& c, uint32_t S, uint32_t N, Tagger* t, c
   Dir d[2];
   for (int k = 0; k < 2; ++k) {
     d[k].x = a.take<float>(E * N); d[k].gates = a.take<float>(G * N); d[k].c = a.take<float>(H * N); d[k].h = a.take<float>(H * N);
-    d[k].ids = a.take<uint32_t>(N);
+    d[k].ids = nullptr;
     d[k].wg = nullptr;
   }
   float* hf = a.take<float>(H * N); float* hr = a.take<float>(H * N);
   float* pre = a.take<float>((size_t)c.TH * N); float* th = a.take<float>((size_t)c.TH * N);
   float* logits = a.take<float>((size_t)c.NT * N);
-  float* errs = a.take<float>(N); float* aux = a.take<float>(3 * (size_t)N); float* ones = a.take<float>(N);
+  float* errs = a.take<float>(N); uint32_t* ids = a.take<uint32_t>(ids_words(N, N)); float* ones = a.take<float>(N);
   float* zeros = a.take<float>(H * S); float* scalars = a.take<float>(64);
   float** tbl = a.take<float*>(8 * (size_t)N); size_t* len = a.take<size_t>(N);
-  uint32_t* prefix_dev = a.take<uint32_t>((size_t)N + 1);   // (a batch has no more steps than tokens)
   // everything below is zeroed by one memset per pass
   a.off = (a.off + 255) & ~(size_t)255;
   const size_t z0 = a.off;
-  for (int k = 0; k < 2; ++k) { d[k].dh = a.take<float>(H * N); d[k].dc = a.take<float>(H * N); d[k].dx = a.take<float>(E * N); }
+  for (int k = 0; k < 2; ++k) d[k].dh = a.take<float>(H * N);
+  d[0].dx = d[1].dx = a.take<float>(2 * E * N);   // (the reverse direction's columns follow the forward direction's)
   float* dhf = a.take<float>(H * N); float* dhr = a.take<float>(H * N);
   float* dth = a.take<float>((size_t)c.TH * N); float* dpre = a.take<float>((size_t)c.TH * N);
   float* dlogits = a.take<float>((size_t)c.NT * N);
+  const size_t z_rec = a.off;                     // (the recurrence kernels take dE/dc as zero where none is given)
+  for (int k = 0; k < 2; ++k) d[k].dc = a.take<float>(H * N);
   const size_t z1 = a.off;
   if (t) {
     for (int k = 0; k < 2; ++k) { dyb200_wgrad* keep = t->d[k].wg; t->d[k] = d[k]; t->d[k].wg = keep; }
     t->hf = hf; t->hr = hr; t->dhf = dhf; t->dhr = dhr; t->pre = pre; t->th = th; t->dth = dth; t->dpre = dpre;
-    t->logits = logits; t->dlogits = dlogits; t->errs = errs; t->aux = aux; t->ones = ones; t->zeros = zeros; t->scalars = scalars;
-    t->prefix_dev = prefix_dev; t->tbl_dev = tbl; t->len_dev = len; t->dact_off0 = z0; t->dact_off1 = z1; t->ws = base;
+    t->logits = logits; t->dlogits = dlogits; t->errs = errs; t->ids_dev = ids; t->ones = ones; t->zeros = zeros; t->scalars = scalars;
+    t->tbl_dev = tbl; t->len_dev = len; t->dact_off0 = z0; t->dact_rec = z_rec; t->dact_off1 = z1; t->ws = base;
   }
   return a.off + 256;
 }
@@ -146,6 +162,9 @@ size_t plan(const dyb200h_tagger_config& c, uint32_t S, uint32_t N, Tagger* t, c
 }  // namespace
 
 namespace {
+
+// Tokens up to which both directions' columns are scattered together (eight sorted runs of 4096 of them: 13 000 tokens, 90 -> 47 us)
+constexpr uint32_t kFoldBoth = 32768;
 
 struct PassArgs { uint32_t S; const uint32_t* lens; const uint32_t* words; const uint32_t* tags; float* loss_dev; };
 
@@ -160,7 +179,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   if (S > m.max_sent) throw std::invalid_argument("tagger: more sentences than the workspace was planned for");
   // ---- host side: the batched executor's schedule for this mini-batch ----
   // (the pinned staging buffers are reused from pass to pass: the previous pass's uploads must have left them)
-  if (m.upload_pending) { CU(cudaEventSynchronize(m.upload_ev)); m.upload_pending = false; }
+  if (m.upload_pending) { CU(cudaEventSynchronize(m.upload_ev)); CU(cudaEventSynchronize(m.tables_ev)); m.upload_pending = false; }
   const auto t_host0 = std::chrono::steady_clock::now();
   const uint32_t Lmax = a.lens[0];
   if (Lmax == 0 || Lmax > m.max_len) throw std::invalid_argument("tagger: sentence length out of range");
@@ -183,8 +202,9 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   }
   float** tbl = m.tbl_host;
   size_t* lens_host = (size_t*)(m.tbl_host + 8 * (size_t)m.max_tok);
-  uint32_t* ids_host = (uint32_t*)(lens_host + m.max_tok);
-  uint32_t *ids_f = ids_host, *ids_r = ids_host + N, *tag_ids = ids_host + 2 * (size_t)N;
+  uint32_t *ids_f = m.ids_host, *ids_r = m.ids_host + N, *tag_ids = m.ids_host + aux_at(N) + 2 * (size_t)N;
+  m.d[0].ids = m.ids_dev; m.d[1].ids = m.ids_dev + N; m.aux = (float*)(m.ids_dev + aux_at(N));
+  m.d[1].dx = m.d[0].dx + (size_t)E * N;
   for (uint32_t s = 0; s < S; ++s) {
     const uint32_t len = a.lens[s];
     for (uint32_t t = 0; t < len; ++t) {
@@ -201,17 +221,14 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
     }
   }
   m.host_schedule_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_host0).count();
-  CU(cudaMemcpyAsync(m.tbl_dev, tbl, 8 * (size_t)N * sizeof(float*), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(m.len_dev, lens_host, (size_t)N * sizeof(size_t), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(m.d[0].ids, ids_f, (size_t)N * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(m.d[1].ids, ids_r, (size_t)N * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(m.aux + 2 * (size_t)N, tag_ids, (size_t)N * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   const bool rec = dyb200i_rec_takes(dev.ctx, H, Lmax, S, 2) != 0;   // the recurrence of both directions as one launch per pass
-  if (rec) {
-    uint32_t* prefix_host = ids_host + 3 * (size_t)m.max_tok;
-    std::memcpy(prefix_host, prefix.data(), (Lmax + 1) * sizeof(uint32_t));
-    CU(cudaMemcpyAsync(m.prefix_dev, prefix_host, (Lmax + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-  }
+  std::memcpy(m.ids_host + prefix_at(N), prefix.data(), (Lmax + 1) * sizeof(uint32_t));
+  const uint32_t* prefix_dev = m.ids_dev + prefix_at(N);
+  CU(cudaMemcpyAsync(m.ids_dev, m.ids_host, ids_words(N, Lmax) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  if (m.pass_recorded) CU(cudaStreamWaitEvent(m.copy_stream, m.pass_ev, 0));
+  CU(cudaMemcpyAsync(m.tbl_dev, tbl, 8 * (size_t)N * sizeof(float*), cudaMemcpyHostToDevice, m.copy_stream));
+  CU(cudaMemcpyAsync(m.len_dev, lens_host, (size_t)N * sizeof(size_t), cudaMemcpyHostToDevice, m.copy_stream));
+  CU(cudaEventRecord(m.tables_ev, m.copy_stream));
   CU(cudaEventRecord(m.upload_ev, st));
   m.upload_pending = true;
   dyb200i_rec_dir rdir[2];
@@ -256,8 +273,9 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   }
   CU(cudaEventRecord(m.join_ev, st2));
   CU(cudaStreamWaitEvent(st, m.join_ev, 0));
-  if (rec) throw_status(dev, dyb200i_rec_fwd(dev.ctx, 2, rdir, H, Lmax, S, m.prefix_dev, 0, at.forget_gate_bias));
+  if (rec) throw_status(dev, dyb200i_rec_fwd(dev.ctx, 2, rdir, H, Lmax, S, prefix_dev, 0, at.forget_gate_bias));
   // combine_tensors: the hidden states of all tokens, token-major
+  CU(cudaStreamWaitEvent(st, m.tables_ev, 0));
   for (int dr = 0; dr < 2; ++dr) {
     if (m.time_movers) CU(cudaEventRecord(m.ev[2 * dr], st));
     gpu::parallel_memcpy(dev, (int)N, (int)H, m.tbl_dev + 2 * (size_t)dr * N, m.tbl_dev + (2 * (size_t)dr + 1) * N, m.len_dev);
@@ -280,7 +298,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   throw_status(dev, dyb200_sum_all(m.errs, N, a.loss_dev, 0, dev.ctx));
 
   // ---------------- backward ----------------
-  CU(cudaMemsetAsync(m.ws + m.dact_off0, 0, m.dact_off1 - m.dact_off0, st));
+  CU(cudaMemsetAsync(m.ws + m.dact_off0, 0, (rec ? m.dact_rec : m.dact_off1) - m.dact_off0, st));
   Tensor tdlog(Dim({NT}, N), m.dlogits), tdth(Dim({TH}, N), m.dth), tdpre(Dim({TH}, N), m.dpre), tdhf(Dim({H}, N), m.dhf), tdhr(Dim({H}, N), m.dhr);
   Tensor gthb(Dim({TH}), m.g[P_THB]), gl2th(Dim({TH, H}), m.g[P_L2TH]), gr2th(Dim({TH, H}), m.g[P_R2TH]);
   Tensor gth2t(Dim({NT, TH}), m.g[P_TH2T]), gtbias(Dim({NT}), m.g[P_TB]);
@@ -300,8 +318,10 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
     gpu::parallel_accumulate(dev, (int)N, (int)H, m.tbl_dev + (4 + 2 * (size_t)dr) * N, m.tbl_dev + (5 + 2 * (size_t)dr) * N, m.len_dev);
     if (m.time_movers) CU(cudaEventRecord(m.ev[5 + 2 * dr], st));
   }
+  CU(cudaEventRecord(m.pass_ev, st));
+  m.pass_recorded = true;
   Tensor gEmb(Dim({E}, V), m.g[P_EMB]);
-  if (rec) throw_status(dev, dyb200i_rec_bwd(dev.ctx, 2, rdir, H, Lmax, S, m.prefix_dev, 0, N));
+  if (rec) throw_status(dev, dyb200i_rec_bwd(dev.ctx, 2, rdir, H, Lmax, S, prefix_dev, 0, N));
   CU(cudaEventRecord(m.fork_ev, st));
   CU(cudaStreamWaitEvent(st2, m.fork_ev, 0));
   for (int dr = 0; dr < 2; ++dr) {
@@ -331,13 +351,14 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   }
   CU(cudaEventRecord(m.join_ev, st2));
   CU(cudaStreamWaitEvent(st, m.join_ev, 0));
-  // the lookups' accumulate_grad calls, folded into one per direction over its columns (step order); both add into the one
-  // table gradient, so they run one after the other on the caller's stream
-  for (int dr = 0; dr < 2; ++dr) {
+  // the lookups' accumulate_grad calls, folded into one over the columns of both directions (the forward direction's in step order,
+  // then the reverse direction's).  Long lists are folded per direction: the merge of the sorted runs grows with their square.
+  const uint32_t folded = N <= kFoldBoth ? 2 : 1;
+  for (uint32_t dr = 0; dr < 2; dr += folded) {
     Dir& d = m.d[dr];
-    LookupNode look(tEmb, nullptr, N);
+    LookupNode look(tEmb, nullptr, folded * N);
     look.aux_mem = d.ids;
-    Tensor tdx(Dim({E}, N), d.dx);
+    Tensor tdx(Dim({E}, folded * N), d.dx);
     look.accumulate_grad(dev, tdx, gEmb);
   }
 }
@@ -395,9 +416,12 @@ int dyb200h_tagger_create(const dyb200h_tagger_config* c, float* params, float* 
   if (!rc && (cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
   for (int k = 0; k < 2 && !rc; ++k) rc = dyb200_wgrad_create(k ? m->dev2.ctx : ctx, 4 * c->H, c->E, c->H, max_tokens, &m->d[k].wg);
-  const size_t host_bytes = 8 * (size_t)max_tokens * sizeof(float*) + (size_t)max_tokens * sizeof(size_t) + 3 * (size_t)max_tokens * sizeof(uint32_t) +
-                            ((size_t)max_len + 1) * sizeof(uint32_t);
+  const size_t host_bytes = 8 * (size_t)max_tokens * sizeof(float*) + (size_t)max_tokens * sizeof(size_t) + ids_words(max_tokens, max_len) * sizeof(uint32_t);
   if (!rc && cudaMallocHost((void**)&m->tbl_host, host_bytes) != cudaSuccess) { cudaGetLastError(); rc = DYB200_ENOMEM; }
+  if (!rc) m->ids_host = (uint32_t*)((size_t*)(m->tbl_host + 8 * (size_t)max_tokens) + max_tokens);
+  if (!rc && cudaStreamCreateWithFlags(&m->copy_stream, cudaStreamNonBlocking) != cudaSuccess) rc = DYB200_ECUDA;
+  if (!rc && (cudaEventCreateWithFlags(&m->tables_ev, cudaEventDisableTiming) != cudaSuccess ||
+              cudaEventCreateWithFlags(&m->pass_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
   for (auto& e : m->ev) if (!rc && cudaEventCreate(&e) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc && cudaEventCreateWithFlags(&m->upload_ev, cudaEventDisableTiming) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc) rc = dyb200_fill(m->zeros, (size_t)c->H * max_sentences, 0.f, ctx);

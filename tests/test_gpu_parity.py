@@ -505,6 +505,7 @@ def test_lookup_errors(g, capi):
 
 
 @pytest.mark.parametrize("E,V,n", [(4, 9, 1), (4, 9, 5), (128, 1000, 512), (512, 5000, 4096), (6, 50, 77), (64, 300, 9000),
+                                   (4, (1 << 20) - 1, 300), (4, 1 << 20, 5000),   # (on both sides of the 32-bit sort keys)
                                    (128, 2000, 50000)])   # (the last: 13 sorted runs merged, the most frequent id spans ~150 chunks)
 def test_lookup_scatter_add(oracle, g, E, V, n):
     r = rng(141)
