@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_ids(const uint32_t* __res
 // The same for tables of fewer than 2^20 rows: the id and the position within the pass are one 32-bit key, four neighbouring keys per
 // thread.  Exchanges over less than 128 keys stay in a warp (registers and shuffles); the 15 longer ones of 4096 keys go through shared
 // memory, two buffers taken in turn, one barrier each.  4096 ids: 39 us with every one of the 78 exchanges of 64-bit keys in shared
-// memory, SORT32 here.
+// memory, 14 here.
 constexpr uint32_t kSort32Vocab = (1u << 20) - 1;
 __global__ void __launch_bounds__(kSortThreads) k_sort_ids32(const uint32_t* __restrict__ ids, uint32_t n_total, uint32_t vocab,
                                                             uint32_t* __restrict__ pos_sorted, uint32_t* __restrict__ id_at, uint32_t* flags) {

@@ -3,8 +3,8 @@
 // What bounds it.  With more than four columns per cluster the fp32 multiply-adds of lstm_rec.cu bound its steps (0.2 us per column
 // and step at 256 units: 8 us forward at 37 columns).  A step here is the same hand-over between CTAs around a product of 128 x
 // 2 NC x K on tcgen05: the operands are 2 x 11 bit fp16 pairs (gemm.cuh), of which a CTA's share of Wh is 128 KB, so that it stays in
-// half of the TMEM for the whole sequence; TF32 pairs of the same precision would need all of it.  (From shared memory the 32 MMAs of
-// a step took 2400 cycles, each waiting for its 4 KB of Wh.)  A step is a chain of product, cell pass and one trip through the cluster.
+// half of the TMEM for the whole sequence and leaves shared memory to the columns; TF32 pairs of the same precision would need all of
+// it.  A step is a chain of product, cell pass and one trip through the cluster.
 //
 // Columns: a cluster takes kGroups groups of 16 neighbours.  More clusters than fit run one after the other (no cluster waits for another):
 // ragged batches come longest first, so every group ends with its own longest sentence.
