@@ -19,6 +19,7 @@
 // kChunkKB k-blocks), the same K split (k_split) reduced in split order through distributed shared memory, the same epilogue.
 #include "seq_dev.cuh"
 #include "lstm_rec_api.h"
+#include "lstm_wide.cuh"
 
 namespace {
 
@@ -552,6 +553,20 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
       dyb200_tc_pack_begin(&batch);
       if ((rc = dyb200_wgrad_seq_h0(deferred, h0->v, mh, mh_full, ctx, &batch))) return rc;
       if ((rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
+    }
+    if (dyb200_wide_takes(ctx, H, B)) {   // all steps in one launch, Wh in the registers of the whole GPU (lstm_wide.cu)
+      WideFwd a;
+      memset(&a, 0, sizeof(a));
+      a.Wh = Wh->v; a.gates = gates_all->v; a.c = c_all->v; a.h = h_all->v; a.h0 = h0->v; a.c0 = c0->v; a.mask = mh; a.mask_full = mh_full;
+      a.H = H; a.B = B; a.T = T; a.fb = attrs->forget_gate_bias;
+      if (deferred) {
+        PackedOp X, Hs;
+        DYB_CHECK_ARG(ctx, dyb200_wgrad_column_planes(deferred, T * B, nullptr, &X, &Hs) && Hs.K == H, "lstm sequence: the accumulator does not hold the inputs of this layer");
+        a.hn_hi = Hs.hi; a.hn_lo = Hs.lo; a.hn_pitch = Hs.pitch;
+      }
+      if ((rc = dyb200_wide_fwd(ctx, a))) return rc;
+      if (deferred) dyb200_wgrad_seq_done(deferred);
+      return DYB200_OK;
     }
     for (uint32_t t = 0; t < T; ++t) {
       GemmPair p{Wh->v, G, 0, t ? h_all->v + (size_t)(t - 1) * HB : h0->v, H, 0, H, mh, H, mh_full, 1};
