@@ -80,15 +80,23 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_lstm_wide_fwd(const __grid_
       for (int p = 0; p < 4; ++p) pre[p] = g[(size_t)p * H];
     if (t) {
       const unsigned long long* x = a.xchg + (size_t)(t & 1) * B * H;
-      for (uint32_t e = tid; e < B * H; e += kWideThreads) {
-        unsigned long long v = 0;
-        for (uint32_t it = 0; ok; ++it) {
-          asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(x + e) : "memory");
-          if ((uint32_t)(v >> 32) == t) break;
-          if (it == kWidePolls) ok = false;
+      // (eight words at a time: one after the other, each cost its own trip to L2)
+      for (uint32_t e0 = tid; e0 < B * H; e0 += 8 * kWideThreads) {
+        unsigned long long v[8];
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r)
+          if (e0 + r * kWideThreads < B * H) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[r]) : "l"(x + e0 + r * kWideThreads) : "memory");
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) {
+          const uint32_t e = e0 + r * kWideThreads;
+          if (e >= B * H) break;
+          for (uint32_t it = 0; ok && (uint32_t)(v[r] >> 32) != t; ++it) {
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[r]) : "l"(x + e) : "memory");
+            if (it == kWidePolls) ok = false;
+          }
+          const uint32_t c = e / H;
+          hs[(size_t)c * HP + (e - c * H)] = __uint_as_float((uint32_t)v[r]);
         }
-        const uint32_t c = e / H;
-        hs[(size_t)c * HP + (e - c * H)] = __uint_as_float((uint32_t)v);
       }
     }
     __syncthreads();
@@ -158,7 +166,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_lstm_wide_fwd(const __grid_
 
 }  // namespace
 
-// Up to 8 columns (each costs a step 0.15 us of multiply-adds and polls) and as many units as the SMs hold, 8 each; narrower layers
+// Up to 8 columns (each costs a step 0.6 - 0.8 us of polls and multiply-adds; 1024 units: 2.1 us at 1, 5.3 at 4, 7.8 at 8 columns, launch by
+// launch 5.0, 7.3 and 10.4) and as many units as the SMs hold, 8 each; narrower layers
 // belong to the clusters of lstm_rec.cu.
 bool dyb200_wide_takes(const dyb200_ctx* ctx, uint32_t H, uint32_t B) { return H > 384 && H <= 1536 && H <= kWideUnits * (uint32_t)ctx->sm_count && B <= 8; }
 
