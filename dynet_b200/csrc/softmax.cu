@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kBlock) k_col_stream(ColArgs a) {
 constexpr uint32_t kColCluster = 8, kColVals = 16;   // up to 8 x 256 x 16 rows
 template <int MODE>
 __global__ void __launch_bounds__(kBlock) __cluster_dims__(8, 1, 1) k_col_cluster(ColArgs a) {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this CTA runs: its shared memory may be written to
   dyb_grid_dep_sync();
   __shared__ float red[32];
   __shared__ float2 part[kColCluster];
@@ -228,11 +229,13 @@ __global__ void __launch_bounds__(kBlock) __cluster_dims__(8, 1, 1) k_col_cluste
 #pragma unroll
   for (int k = 0; k < (int)kColVals; ++k) s += ex2_approx(fmaf(v[k], kLog2e, -ml));
   s = block_sum(s, red);
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // (all eight run; the loads and sums hid the wait)
   if (threadIdx.x < kColCluster) {
     uint32_t dst;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"((uint32_t)__cvta_generic_to_shared(&part[rank])), "r"(threadIdx.x));
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst), "f"(mx), "f"(s) : "memory");
   }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   float m = -INFINITY, tot = 0.f;
 #pragma unroll

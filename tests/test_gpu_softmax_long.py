@@ -29,3 +29,25 @@ def test_long_columns(oracle, rows, bd):
     assert_close(g.host(loss_), oracle.pnls_fwd(x, ids)[0], TOL_REDUCE, floor=1.0, what="pnls")
     assert g.ctx().device_errors() == 0
     g.release()
+
+
+def test_long_columns_beside_other_work():
+    """The CTAs of a cluster start unevenly on a GPU that is busy with another stream: the same bits as on a quiet one."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    rows, bd = 10000, 3
+    x_ = g.dev(randn(rng(3), bd, rows, scale=3.0))
+    y_ = torch.empty(200, bd, rows, device="cuda")
+    aux = torch.empty(2 * bd, device="cuda")
+    a, other = torch.randn(4096, 4096, device="cuda"), torch.cuda.Stream()
+    other.wait_stream(torch.cuda.current_stream())
+    for k in range(200):
+        if k % 5 == 1:
+            with torch.cuda.stream(other):
+                a = a * 1.0001 + 0.5
+        g.ctx().fwd("log_softmax", [g.T(x_, [rows], bd)], g.T(y_[k], [rows], bd), None, aux.data_ptr())
+    torch.cuda.synchronize()
+    assert all(torch.equal(y_[0], y_[k]) for k in range(200))
+    assert g.ctx().device_errors() == 0
+    g.release()
