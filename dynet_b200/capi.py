@@ -138,6 +138,11 @@ def lib_path():
     return os.environ.get("DYB200_LIB") or os.path.join(_HERE, "libdyb200.so")
 
 
+_TENSOR_P, _LSTM_P = C.POINTER(DyTensor), C.POINTER(LstmGatesAttrs)
+_FWD_TYPES = [_TENSOR_P, C.c_int, _TENSOR_P, C.c_void_p, C.c_void_p, C.c_void_p]
+_BWD_TYPES = [_TENSOR_P, C.c_int, _TENSOR_P, _TENSOR_P, C.c_uint, _TENSOR_P, C.c_void_p, C.c_void_p, C.c_void_p]
+
+
 def lib():
     """Loads libdyb200.so; raises (no fallback) if it has not been built."""
     global _LIB
@@ -147,15 +152,15 @@ def lib():
             raise ImportError("libdyb200.so is missing: run `python -m dynet_b200.build` (nvcc, sm_100a); "
                               "there is no CPU fallback")
         L = C.CDLL(p)
-        tp = C.POINTER(DyTensor)
+        tp = _TENSOR_P
         for n in NODES + FWD_ONLY:
             f = getattr(L, "dyb200_%s_fwd" % n)
             f.restype = C.c_int
-            f.argtypes = [tp, C.c_int, tp, C.c_void_p, C.c_void_p, C.c_void_p]
+            f.argtypes = _FWD_TYPES
         for n in NODES:
             f = getattr(L, "dyb200_%s_bwd" % n)
             f.restype = C.c_int
-            f.argtypes = [tp, C.c_int, tp, tp, C.c_uint, tp, C.c_void_p, C.c_void_p, C.c_void_p]
+            f.argtypes = _BWD_TYPES
         L.dyb200_ctx_create.restype = C.c_int
         L.dyb200_ctx_create.argtypes = [C.c_int, C.c_void_p, C.POINTER(C.c_void_p)]
         L.dyb200_ctx_destroy.argtypes = [C.c_void_p]
@@ -242,29 +247,41 @@ except ImportError:         # not built (no Python headers): every call goes thr
     def _native_call(*args):
         return NotImplemented
 
-_ADDRESS = {}
+_ENTRIES = {}
 
 
-def _address(name):
-    a = _ADDRESS.get(name)
-    if a is None:
-        a = _ADDRESS[name] = C.cast(getattr(lib(), name), C.c_void_p).value
-    return a
+def _entry(name):
+    """(address, one letter per parameter, structure types) of an entry point, as host/py/call.c takes them."""
+    e = _ENTRIES.get(name)
+    if e is None:
+        f = getattr(lib(), name)
+        if list(f.argtypes) == _FWD_TYPES:
+            kinds = b"xitavv"
+        elif list(f.argtypes) == _BWD_TYPES:
+            kinds = b"xittitavv"
+        else:
+            kinds = b"".join(b"T" if t is _TENSOR_P else b"v" if t is C.c_void_p else b"s" if t is _LSTM_P else b"n" if hasattr(t, "contents") else b"i"
+                             for t in f.argtypes)
+        e = _ENTRIES[name] = (C.cast(f, C.c_void_p).value, kinds, tuple(getattr(t, "_type_", None) for t in f.argtypes))
+    return e
 
 
 def _ctypes_call(name, args):
-    """The same call through ctypes, for argument kinds the extension does not take."""
+    """The same call through ctypes, for arguments the extension does not take: converted as the parameter's type asks, or refused."""
+    f, kinds = getattr(lib(), name), _entry(name)[1].decode()
+    if len(args) != len(kinds):
+        raise TypeError("%s takes %d arguments (%d given)" % (name, len(kinds), len(args)))
     out = []
-    for a in args:
-        if isinstance(a, C.Structure):
-            out.append(C.byref(a))
-        elif isinstance(a, (list, tuple)):
+    for k, a in zip(kinds, args):
+        if k == "x":
             out.append((DyTensor * len(a))(*a) if a else None)
+        elif k in "ts" or (k == "T" and a is not None):
+            out.append(C.byref(a))
+        elif k == "a" and a is not None:
+            out.append(C.cast(C.byref(a), C.c_void_p))
         else:
             out.append(a)
-    f = getattr(lib(), name)
-    # (node attributes are declared void *)
-    return f(*[C.cast(o, C.c_void_p) if t is C.c_void_p and isinstance(a, C.Structure) else o for o, a, t in zip(out, args, f.argtypes)])
+    return f(*out)
 
 
 class Context:
@@ -282,7 +299,7 @@ class Context:
         self._fwd, self._bwd = {}, {}
 
     def _run(self, name, *args):
-        rc = _native_call(_address(name), *args, self._hv)
+        rc = _native_call(_entry(name), *args, self._hv)
         if rc is NotImplemented:
             rc = _ctypes_call(name, args + (self._hv,))
         if rc:
@@ -332,20 +349,22 @@ class Context:
     def fwd(self, node, xs, fx, attrs=None, aux=None):
         f = self._fwd.get(node)
         if f is None:
-            f = self._fwd[node] = _address("dyb200_%s_fwd" % node)
-        rc = _native_call(f, xs, len(xs), fx, attrs, aux, self._hv)
+            f = self._fwd[node] = _entry("dyb200_%s_fwd" % node)
+        n = len(xs) if xs else 0
+        rc = _native_call(f, xs, n, fx, attrs, aux, self._hv)
         if rc is NotImplemented:
-            rc = _ctypes_call("dyb200_%s_fwd" % node, (xs, len(xs), fx, attrs, aux, self._hv))
+            rc = _ctypes_call("dyb200_%s_fwd" % node, (xs, n, fx, attrs, aux, self._hv))
         if rc:
             self.check(rc)
 
     def bwd(self, node, xs, fx, dEdf, i, dEdxi, attrs=None, aux=None):
         f = self._bwd.get(node)
         if f is None:
-            f = self._bwd[node] = _address("dyb200_%s_bwd" % node)
-        rc = _native_call(f, xs, len(xs), fx, dEdf, i, dEdxi, attrs, aux, self._hv)
+            f = self._bwd[node] = _entry("dyb200_%s_bwd" % node)
+        n = len(xs) if xs else 0
+        rc = _native_call(f, xs, n, fx, dEdf, i, dEdxi, attrs, aux, self._hv)
         if rc is NotImplemented:
-            rc = _ctypes_call("dyb200_%s_bwd" % node, (xs, len(xs), fx, dEdf, i, dEdxi, attrs, aux, self._hv))
+            rc = _ctypes_call("dyb200_%s_bwd" % node, (xs, n, fx, dEdf, i, dEdxi, attrs, aux, self._hv))
         if rc:
             self.check(rc)
 
