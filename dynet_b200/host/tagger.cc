@@ -101,8 +101,7 @@ struct Tagger {
   double host_schedule_ms = 0.0;
   // The mover calls' tables (72 bytes a token) are not needed before the recurrence is through: they go over beside it.
   cudaStream_t copy_stream = nullptr;
-  cudaEvent_t tables_ev = nullptr, pass_ev = nullptr;   // tables uploaded / the last pass has read them
-  bool pass_recorded = false;
+  cudaEvent_t tables_ev = nullptr, start_ev = nullptr;   // tables uploaded / the caller's stream has come to this pass
   ~Tagger() {
     if (copy_stream) { cudaStreamSynchronize(copy_stream); cudaStreamDestroy(copy_stream); }   // (before its source goes)
     for (int k = 0; k < 2; ++k) if (d[k].wg) dyb200_wgrad_destroy(d[k].wg);
@@ -112,7 +111,7 @@ struct Tagger {
     if (fork_ev) cudaEventDestroy(fork_ev);
     if (join_ev) cudaEventDestroy(join_ev);
     if (tables_ev) cudaEventDestroy(tables_ev);
-    if (pass_ev) cudaEventDestroy(pass_ev);
+    if (start_ev) cudaEventDestroy(start_ev);
     if (dev2.ctx) dyb200_ctx_destroy(dev2.ctx);
     if (stream2) cudaStreamDestroy(stream2);
   }
@@ -225,7 +224,10 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   std::memcpy(m.ids_host + prefix_at(N), prefix.data(), (Lmax + 1) * sizeof(uint32_t));
   const uint32_t* prefix_dev = m.ids_dev + prefix_at(N);
   CU(cudaMemcpyAsync(m.ids_dev, m.ids_host, ids_words(N, Lmax) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-  if (m.pass_recorded) CU(cudaStreamWaitEvent(m.copy_stream, m.pass_ev, 0));
+  // (behind everything that the caller's stream holds: the movers of the pass before, also of one that failed half-way, and whoever
+  // used the workspace's memory before it was handed to this driver)
+  CU(cudaEventRecord(m.start_ev, st));
+  CU(cudaStreamWaitEvent(m.copy_stream, m.start_ev, 0));
   CU(cudaMemcpyAsync(m.tbl_dev, tbl, 8 * (size_t)N * sizeof(float*), cudaMemcpyHostToDevice, m.copy_stream));
   CU(cudaMemcpyAsync(m.len_dev, lens_host, (size_t)N * sizeof(size_t), cudaMemcpyHostToDevice, m.copy_stream));
   CU(cudaEventRecord(m.tables_ev, m.copy_stream));
@@ -318,8 +320,6 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
     gpu::parallel_accumulate(dev, (int)N, (int)H, m.tbl_dev + (4 + 2 * (size_t)dr) * N, m.tbl_dev + (5 + 2 * (size_t)dr) * N, m.len_dev);
     if (m.time_movers) CU(cudaEventRecord(m.ev[5 + 2 * dr], st));
   }
-  CU(cudaEventRecord(m.pass_ev, st));
-  m.pass_recorded = true;
   Tensor gEmb(Dim({E}, V), m.g[P_EMB]);
   if (rec) throw_status(dev, dyb200i_rec_bwd(dev.ctx, 2, rdir, H, Lmax, S, prefix_dev, 0, N));
   CU(cudaEventRecord(m.fork_ev, st));
@@ -421,7 +421,7 @@ int dyb200h_tagger_create(const dyb200h_tagger_config* c, float* params, float* 
   if (!rc) m->ids_host = (uint32_t*)((size_t*)(m->tbl_host + 8 * (size_t)max_tokens) + max_tokens);
   if (!rc && cudaStreamCreateWithFlags(&m->copy_stream, cudaStreamNonBlocking) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc && (cudaEventCreateWithFlags(&m->tables_ev, cudaEventDisableTiming) != cudaSuccess ||
-              cudaEventCreateWithFlags(&m->pass_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
+              cudaEventCreateWithFlags(&m->start_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
   for (auto& e : m->ev) if (!rc && cudaEventCreate(&e) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc && cudaEventCreateWithFlags(&m->upload_ev, cudaEventDisableTiming) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc) rc = dyb200_fill(m->zeros, (size_t)c->H * max_sentences, 0.f, ctx);

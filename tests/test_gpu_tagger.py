@@ -285,3 +285,32 @@ def test_tagger_driver_rejects_bad_input():
     with pytest.raises(capi.InvalidArgument, match="tokens"):
         m.launch_forward_backward(np.array([8, 8, 8], np.uint32), np.zeros(24, np.uint32), np.zeros(24, np.uint32))
     m.close()
+
+
+def test_tagger_first_pass_behind_queued_work():
+    """The caller's stream still holds work on the memory that becomes the workspace (torch's allocator hands a freed block on within its
+    stream) when the first pass is issued: the tables that go over on a stream of their own must come after it."""
+    import torch
+    from dynet_b200 import tagger as tg
+    dims = (500, 32, 64, 16, 7)
+    lens, words, tags = tg.synthetic_corpus(24, 500, 7, seed=5, lo=8, hi=30)
+    size = dict(max_sentences=24, max_tokens=int(lens.sum()), max_len=30, seed=1)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        m = tg.Tagger(*dims, **size, stream=stream.cuda_stream)
+        want, n = m.forward_backward(lens, words, tags), m.workspace.numel()
+        grads = m.grads.clone()
+        m.close()
+        del m
+        torch.cuda.empty_cache()
+        held = torch.empty(n, dtype=torch.uint8, device="cuda")
+        at = held.data_ptr()
+        torch.cuda._sleep(1 << 29)                     # some 0.3 s
+        held.fill_(255)
+        del held
+        m = tg.Tagger(*dims, **size, stream=stream.cuda_stream)
+        assert m.workspace.data_ptr() == at
+        assert m.forward_backward(lens, words, tags) == want
+        assert torch.equal(m.grads, grads)
+        assert m.device_errors() == 0
+        m.close()
