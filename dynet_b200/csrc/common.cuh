@@ -118,6 +118,11 @@ static inline size_t t_size(const dyb200_tensor* t) { return t_batch_size(t) * t
 static inline uint32_t t_dim(const dyb200_tensor* t, uint32_t k) { return k < t->nd ? t->d[k] : 1u; }
 static inline uint32_t t_rows(const dyb200_tensor* t) { return t_dim(t, 0); }
 static inline uint32_t t_cols(const dyb200_tensor* t) { return t_dim(t, 1); }
+// Whether two arrays of floats share memory (null or empty: no).
+static inline bool t_overlap(const float* a, size_t na, const float* b, size_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x && y && na && nb && x < y + nb * sizeof(float) && y < x + na * sizeof(float);
+}
 __host__ __device__ static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Grid for a streaming kernel: enough CTAs to cover the work, capped at a

@@ -107,11 +107,25 @@ int dyb200_gemm_simt(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const 
   return DYB200_OK;
 }
 
+// Whether the result shares memory with an operand or its mask (by the address ranges they span).
+static bool on_operands(uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi) {
+  auto span = [](uint32_t rows, uint32_t cols, uint32_t ld) { return rows && cols ? (size_t)ld * (cols - 1) + rows : 0; };
+  const size_t c = span(M, N, epi.ldc);
+  for (int p = 0; p < npairs; ++p) {
+    const GemmPair& g = pairs[p];
+    const uint32_t br = g.transB ? N : g.K, bc = g.transB ? g.K : N;
+    if (t_overlap(epi.C, c, g.A, g.transA ? span(g.K, M, g.lda) : span(M, g.K, g.lda)) || t_overlap(epi.C, c, g.B, span(br, bc, g.ldb)) ||
+        t_overlap(epi.C, c, g.maskB, g.mask_full ? span(br, bc, g.mask_ld) : br)) return true;
+  }
+  return false;
+}
+
 int dyb200_gemm_fused(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const GemmPair* pairs, const GemmEpilogue& epi) {
   double flops = 0;
   for (int p = 0; p < npairs; ++p) flops += 2.0 * M * N * pairs[p].K;
-  if (M && N && dyb200_thin_takes(M, N, npairs, pairs, epi)) return dyb200_gemm_thin(ctx, M, N, npairs, pairs, epi);
-  if (M && N && dyb200_narrow_takes(M, N, npairs, pairs, epi)) return dyb200_gemm_narrow(ctx, M, N, pairs[0], epi);
+  // (both read their operands as they lie while they store the result: not for a result that lies on one of them)
+  if (M && N && dyb200_thin_takes(M, N, npairs, pairs, epi) && !on_operands(M, N, npairs, pairs, epi)) return dyb200_gemm_thin(ctx, M, N, npairs, pairs, epi);
+  if (M && N && dyb200_narrow_takes(M, N, npairs, pairs, epi) && !on_operands(M, N, npairs, pairs, epi)) return dyb200_gemm_narrow(ctx, M, N, pairs[0], epi);
   int handled = 0;
   int rc = dyb200_gemm_tc(ctx, M, N, npairs, pairs, epi, &handled);
   if (handled) return rc;

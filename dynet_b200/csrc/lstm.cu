@@ -530,15 +530,33 @@ int dyb200_vanilla_lstm_fwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
                            t_size(gates) == (size_t)G * B &&
                            (!attrs->dropout || ((mask_x->bd == B || mask_x->bd == 1) && (mask_h->bd == B || mask_h->bd == 1) &&
                                                 t_dim(mask_x, 0) == I && t_dim(mask_h, 0) == H));
-    if (shapes_ok && attrs->weightnoise_std == 0.f && I > 0 && H > 0 && B > 0 && dyb200_thin_columns(G, B, I + H)) {
+    // (its launch reads x, h_tm1 and the masks while it stores gates, c_t and h_t)
+    auto stored_on = [&](const dyb200_tensor* t) {
+      return t_overlap(gates->v, t_size(gates), t->v, t_size(t)) || t_overlap(c_t->v, total, t->v, t_size(t)) || t_overlap(h_t->v, total, t->v, t_size(t));
+    };
+    if (shapes_ok && attrs->weightnoise_std == 0.f && I > 0 && H > 0 && B > 0 && dyb200_thin_columns(G, B, I + H) &&
+        (!attrs->dropout || !(stored_on(mask_x) || stored_on(mask_h)))) {
       // few columns: one pass over the weights in fp32, c and h formed by the CTAs that hold the gates (gemm_thin.cu)
       const float* mx = attrs->dropout ? mask_x->v : nullptr;
       const float* mh = attrs->dropout ? mask_h->v : nullptr;
       const int mx_full = mx ? mask_x->bd == B : 0, mh_full = mh ? mask_h->bd == B : 0;
-      GemmPair pairs[2] = {{Wx->v, G, 0, x->v, I, 0, I, mx, I, mx_full, 1}, {Wh->v, G, 0, h_tm1->v, H, 0, H, mh, H, mh_full, 1}};
+      int rc;
+      // a state that is updated in place is read from a copy
+      const float *xv = x->v, *hv = h_tm1->v;
+      if (stored_on(x) || stored_on(h_tm1)) {
+        if ((rc = dyb200_scratch_begin(ctx))) return rc;
+        for (int q = 0; q < 2; ++q) {
+          const dyb200_tensor* t = q ? h_tm1 : x;
+          if (!stored_on(t)) continue;
+          void* copy;
+          if ((rc = dyb200_scratch(ctx, t_size(t) * sizeof(float), &copy))) return rc;
+          DYB_CUDA(ctx, cudaMemcpyAsync(copy, t->v, t_size(t) * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
+          (q ? hv : xv) = (const float*)copy;
+        }
+      }
+      GemmPair pairs[2] = {{Wx->v, G, 0, xv, I, 0, I, mx, I, mx_full, 1}, {Wh->v, G, 0, hv, H, 0, H, mh, H, mh_full, 1}};
       GemmEpilogue e{EPI_LSTM_CELL, gates->v, G, b->v, H, attrs->forget_gate_bias, nullptr, 0, 0};
       e.c_prev = c_tm1->v; e.c_out = c_t->v; e.h_out = h_t->v;
-      int rc;
       if (deferred) {
         DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_fwd_fused: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
         PackedOp px, ph;

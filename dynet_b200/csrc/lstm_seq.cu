@@ -554,10 +554,18 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
       if ((rc = dyb200_wgrad_seq_h0(deferred, h0->v, mh, mh_full, ctx, &batch))) return rc;
       if ((rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
     }
+    // (h0 on the first step's outputs is read from a copy: a step's launch reads h_{t-1} while it stores its own)
+    const float* h_first = h0->v;
+    if (t_overlap(h0->v, HB, h_all->v, HB) || t_overlap(h0->v, HB, c_all->v, HB)) {
+      void* copy;
+      if ((rc = dyb200_scratch(ctx, HB * sizeof(float), &copy))) return rc;
+      DYB_CUDA(ctx, cudaMemcpyAsync(copy, h0->v, HB * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
+      h_first = (const float*)copy;
+    }
     if (dyb200_wide_takes(ctx, H, B)) {   // all steps in one launch, Wh in the registers of the whole GPU (lstm_wide.cu)
       WideFwd a;
       memset(&a, 0, sizeof(a));
-      a.Wh = Wh->v; a.gates = gates_all->v; a.c = c_all->v; a.h = h_all->v; a.h0 = h0->v; a.c0 = c0->v; a.mask = mh; a.mask_full = mh_full;
+      a.Wh = Wh->v; a.gates = gates_all->v; a.c = c_all->v; a.h = h_all->v; a.h0 = h_first; a.c0 = c0->v; a.mask = mh; a.mask_full = mh_full;
       a.H = H; a.B = B; a.T = T; a.fb = attrs->forget_gate_bias;
       if (deferred) {
         PackedOp X, Hs;
@@ -569,7 +577,7 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
       return DYB200_OK;
     }
     for (uint32_t t = 0; t < T; ++t) {
-      GemmPair p{Wh->v, G, 0, t ? h_all->v + (size_t)(t - 1) * HB : h0->v, H, 0, H, mh, H, mh_full, 1};
+      GemmPair p{Wh->v, G, 0, t ? h_all->v + (size_t)(t - 1) * HB : h_first, H, 0, H, mh, H, mh_full, 1};
       GemmEpilogue e{EPI_LSTM_CELL, gates_all->v + (size_t)t * 4 * HB, G, nullptr, H, attrs->forget_gate_bias, nullptr, 0, 0};
       e.c_prev = t ? c_all->v + (size_t)(t - 1) * HB : c0->v;
       e.c_out = c_all->v + (size_t)t * HB; e.h_out = h_all->v + (size_t)t * HB;

@@ -55,3 +55,70 @@ def test_thin_lstm_step(oracle, g, I, H, B, mask):
     for name, got, ref in (("gates", og, gates), ("c", oc, c_t), ("h", oh, h_t)):
         assert_close(g.host(got), ref, TOL_REDUCE, floor=0.1, what=name)
     assert g.ctx().device_errors() == 0
+
+
+@pytest.mark.parametrize("H,B,mask", [(1024, 1, False), (40, 3, True), (301, 8, False), (512, 20, True)])
+def test_thin_lstm_step_in_place(g, H, B, mask):
+    """h_t on h_tm1 and c_t on c_tm1, and h_t on x (a layer over the one below): the values of separate buffers."""
+    import torch
+    from dynet_b200 import capi
+    gen = torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen) * 0.3   # noqa: E731
+    x, h, c, Wx, Wh, b = rnd(B, H), rnd(B, H), rnd(B, H), rnd(H, 4 * H) * 0.1, rnd(H, 4 * H) * 0.1, rnd(4 * H)
+    masks = [(torch.rand(B, H, device="cuda", generator=gen) < 0.8).float() for _ in range(2)]
+    mx, mh = (g.T(masks[0]), g.T(masks[1])) if mask else (None, None)
+    at, W = capi.LstmGatesAttrs(1 if mask else 0, 0.0, 1.0), (g.T(Wx, [4 * H, H], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1))
+
+    def steps(n, onto):
+        hs, cs, xs, gates = h.clone(), c.clone(), x.clone(), torch.empty(B, 4 * H, device="cuda")
+        for _ in range(n):
+            ho, co = (hs, cs) if onto == "state" else (xs, torch.empty_like(c)) if onto == "x" else (torch.empty_like(h), torch.empty_like(c))
+            g.ctx().lstm_fwd_fused(g.T(xs), g.T(hs), g.T(cs), *W, mx, mh, at, g.T(gates), g.T(co), g.T(ho))
+            hs, cs = ho.clone() if onto == "x" else ho, co
+            xs = x.clone()
+            torch.cuda.synchronize()
+        return hs, cs
+    want = steps(5, None)
+    for onto in ("state", "x"):
+        for got, ref in zip(steps(5, onto), want):
+            assert torch.equal(got, ref), onto
+    assert g.ctx().device_errors() == 0
+
+
+@pytest.mark.parametrize("H,B", [(512, 3), (1024, 16), (256, 5), (300, 200)])
+def test_sequence_from_a_state_on_its_own_outputs(g, H, B):
+    """h0 and c0 on the first step's h and c, or on the last step's (a text read piece by piece into the same buffers)."""
+    import torch
+    from dynet_b200 import capi
+    T, I = 9, 24
+    gen = torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen) * 0.3   # noqa: E731
+    x, h0, c0, Wx, Wh, b = rnd(T * B, I), rnd(B, H), rnd(B, H), rnd(I, 4 * H) * 0.1, rnd(H, 4 * H) * 0.1, rnd(4 * H)
+    at, W = capi.LstmGatesAttrs(0, 0.0, 1.0), (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1))
+    out = []
+    for at_step in (None, 0, T - 1):
+        gates, cs, hs = (torch.zeros(T * B, n, device="cuda") for n in (4 * H, H, H))
+        hi, ci = (h0, c0) if at_step is None else (hs[at_step * B:(at_step + 1) * B].copy_(h0), cs[at_step * B:(at_step + 1) * B].copy_(c0))
+        g.ctx().lstm_seq_fwd(g.T(x, [I], T * B), g.T(hi), g.T(ci), *W, None, None, at, g.T(gates, [4 * H], T * B), g.T(cs, [H], T * B),
+                             g.T(hs, [H], T * B), None, T)
+        torch.cuda.synchronize()
+        out.append((gates, cs, hs))
+    for o in out[1:]:
+        assert all(torch.equal(p, q) for p, q in zip(o, out[0]))
+    assert g.ctx().device_errors() == 0
+
+
+@pytest.mark.parametrize("n,cols", [(512, 17), (64, 2000)])
+def test_product_onto_its_own_operand(g, n, cols):
+    """C on B (both paths that read B as it lies give such a product back to the one that splits it first)."""
+    import torch
+    A, B = torch.randn(n, n, device="cuda"), torch.randn(cols, n, device="cuda")
+    want = B.double() @ A.double()
+    reps = []
+    for _ in range(3):
+        C = B.clone()
+        g.ctx().gemm(0, 0, n, cols, n, A.data_ptr(), n, C.data_ptr(), n, C.data_ptr(), n, 0)
+        torch.cuda.synchronize()
+        reps.append(C)
+    assert all(torch.equal(r, reps[0]) for r in reps)
+    assert float((reps[0].double() - want).abs().max()) <= TOL_REDUCE * n ** 0.5
