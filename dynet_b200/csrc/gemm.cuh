@@ -74,6 +74,11 @@ __device__ __forceinline__ int scale_field(uint32_t word) {   // E, kept where b
   const int e = (int)(word >> 23);
   return e < 27 ? 27 : e;
 }
+// |v| as the word that maxima are taken of: bit pattern, infinities and NaNs (which come through a split as they are) count as 0
+__device__ __forceinline__ uint32_t finite_mag(float v) {
+  const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
+  return u < 0x7f800000u ? u : 0u;
+}
 __device__ __forceinline__ float scale_of(uint32_t word) { return __int_as_float((268 - scale_field(word)) << 23); }
 // v 2^(Ea + Eb - 282): in two factors, so that nothing overflows on the way to a result that does not
 __device__ __forceinline__ float unscale(float v, int t) {

@@ -724,11 +724,7 @@ __global__ void __launch_bounds__(256) k_pack_multi(const PackJobs jobs) {
 // Both passes read the source once; a line of a wide operand is shared by several CTAs, maxima meet by atomicMax on the bit
 // patterns (the same from run to run).  Infinities and NaNs do not count: they come through the split as they are.
 constexpr uint32_t kMaxLines = 32;   // lines per unit of work where positions have their own scale
-__device__ __forceinline__ uint32_t mag(float v) {
-  const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
-  return u < 0x7f800000u ? u : 0u;
-}
-__device__ __forceinline__ uint32_t mag4(float4 v) { return max(max(mag(v.x), mag(v.y)), max(mag(v.z), mag(v.w))); }
+__device__ __forceinline__ uint32_t mag4(float4 v) { return max(max(finite_mag(v.x), finite_mag(v.y)), max(finite_mag(v.z), finite_mag(v.w))); }
 __global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
   dyb_grid_dep_sync();
   const F16Job& j = jobs.job[blockIdx.z];
@@ -744,10 +740,10 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
         const float* p = j.src + (size_t)j.ld * l + e;
         if (vec && e + 4 <= j.n) {
           const float4 v = ld4(p);
-          m[0] = max(m[0], mag(v.x)); m[1] = max(m[1], mag(v.y)); m[2] = max(m[2], mag(v.z)); m[3] = max(m[3], mag(v.w));
+          m[0] = max(m[0], finite_mag(v.x)); m[1] = max(m[1], finite_mag(v.y)); m[2] = max(m[2], finite_mag(v.z)); m[3] = max(m[3], finite_mag(v.w));
         } else {
 #pragma unroll
-          for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) m[i] = max(m[i], mag(p[i]));
+          for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) m[i] = max(m[i], finite_mag(p[i]));
         }
       }
 #pragma unroll
@@ -767,11 +763,11 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
 #pragma unroll 4
       for (uint32_t e = lo + 4 * threadIdx.x; e < hi; e += 1024) {
         if (e + 4 <= hi) m = max(m, mag4(ld4(p + e)));
-        else for (uint32_t i = e; i < hi; ++i) m = max(m, mag(p[i]));
+        else for (uint32_t i = e; i < hi; ++i) m = max(m, finite_mag(p[i]));
       }
     } else {
 #pragma unroll 4
-      for (uint32_t e = lo + threadIdx.x; e < hi; e += 256) m = max(m, mag(p[e]));
+      for (uint32_t e = lo + threadIdx.x; e < hi; e += 256) m = max(m, finite_mag(p[e]));
     }
     if (j.mode == F16_ALL) { all = max(all, m); continue; }
     m = __reduce_max_sync(0xffffffffu, m);

@@ -60,10 +60,6 @@ __device__ __forceinline__ void send_bulk(uint32_t dst, const void* src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(smem_u32(src)),
                "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ uint32_t finite_mag(float v) {
-  const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
-  return u < 0x7f800000u ? u : 0u;
-}
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);

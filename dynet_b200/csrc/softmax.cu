@@ -444,63 +444,109 @@ struct ChunkOfPart {   // f(r, b) = v[r + n * b]
   __device__ float operator()(size_t r, uint32_t b) const { return v[r + n * (size_t)b]; }
 };
 
-// F16: the planes are scaled fp16 pairs (half the bytes); |d| <= |dz|, so the scale word is that of the largest |dz|.
+// d of four rows from r on (v = x there; rows that do not exist: 0); vec: rows % 4 == 0, the arithmetic of k_expsub_bwd's vector path,
+// else of its scalar one
+__device__ __forceinline__ float4 pnls_grad4(float4 v, uint32_t r, uint32_t rows, uint32_t pick, float zc, float dc, int vec) {
+  float4 d;
+  if (vec) {
+    const float zl = zc * kLog2e;
+    d = make_float4(ex2_approx(fmaf(v.x, kLog2e, -zl)) * dc, ex2_approx(fmaf(v.y, kLog2e, -zl)) * dc,
+                    ex2_approx(fmaf(v.z, kLog2e, -zl)) * dc, ex2_approx(fmaf(v.w, kLog2e, -zl)) * dc);
+  } else {
+    d = make_float4(expf(v.x - zc) * dc, r + 1 < rows ? expf(v.y - zc) * dc : 0.f, r + 2 < rows ? expf(v.z - zc) * dc : 0.f,
+                    r + 3 < rows ? expf(v.w - zc) * dc : 0.f);
+  }
+  if (pick - r < 4u) {
+    const uint32_t k = pick - r;
+    if (k == 0) d.x -= dc; else if (k == 1) d.y -= dc; else if (k == 2) d.z -= dc; else d.w -= dc;
+  }
+  return d;
+}
+__device__ __forceinline__ float4 pnls_x4(const float* xc, uint32_t r, uint32_t rows, int vec) {
+  if (vec) return ld4_stream(xc + r);
+  return make_float4(xc[r], r + 1 < rows ? xc[r + 1] : 0.f, r + 2 < rows ? xc[r + 2] : 0.f, r + 3 < rows ? xc[r + 3] : 0.f);
+}
+
+// The largest |d| of every row and of every column, for fp16 planes.  Bound by reading x once more (819 MB: 50 000 x 4096).  A CTA
+// takes 1024 rows x kPnlsMaxCols columns, eight columns requested at a time; a row's maximum stays with its thread, a column's meets by
+// one reduction per warp; both meet the other CTAs' by atomicMax on bit patterns (the same from run to run).
+constexpr uint32_t kPnlsMaxCols = 64;
+__global__ void __launch_bounds__(256) k_softmax_bwd_max(const float* __restrict__ x, const float* __restrict__ z, const float* __restrict__ dz,
+                                                         const uint32_t* __restrict__ ids, uint32_t rows, uint32_t ncols,
+                                                         uint32_t* __restrict__ row_max, uint32_t* __restrict__ col_max, int vec) {
+  dyb_grid_dep_sync();
+  const uint32_t r = (blockIdx.x * 256 + threadIdx.x) * 4, c_end = min(ncols, (blockIdx.y + 1) * kPnlsMaxCols);
+  const bool live = r < rows;
+  uint32_t m[4] = {0, 0, 0, 0};
+  for (uint32_t c0 = blockIdx.y * kPnlsMaxCols; c0 < c_end; c0 += 8) {
+    float4 v[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q)
+      v[q] = live && c0 + q < c_end ? pnls_x4(x + (size_t)(c0 + q) * rows, r, rows, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      const uint32_t c = c0 + q;
+      if (c >= c_end) break;
+      uint32_t most = 0;
+      if (live) {
+        const float4 d = pnls_grad4(v[q], r, rows, ids ? ids[c] : 0xffffffffu, z[c], dz[c], vec);
+        const uint32_t w[4] = {finite_mag(d.x), finite_mag(d.y), finite_mag(d.z), finite_mag(d.w)};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { m[k] = max(m[k], w[k]); most = max(most, w[k]); }
+      }
+      most = __reduce_max_sync(0xffffffffu, most);
+      if (most && (threadIdx.x & 31) == 0) atomicMax(col_max + c, most);
+    }
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k)
+    if (r + k < rows) atomicMax(row_max + r + k, m[k]);
+}
+
+// F16: the planes are scaled fp16 pairs (half the bytes), of which there are two sets - the scale belongs to the operand's row, and that
+// is a column of d for dh (hb) and a row of d for dR (ha): with one scale for both, or for the whole matrix, a word whose
+// probability is tiny everywhere, or a column with a small dE/df, would keep only a few bits (dR rows of words with p near 1e-22 were
+// off by 7 %).  The maxima and the second set cost 0.36 of 3.06 ms (forward and backward of 512 -> 50 000 for 4096 columns; TF32
+// pairs, whose elements need no scale: 4.14).
+struct PnlsF16 { __half *hb, *lb, *ha, *la; const uint32_t *col_max, *row_max; };
 template <bool F16>
 __global__ void __launch_bounds__(256) k_softmax_bwd_split(const float* __restrict__ x, const float* __restrict__ z,
                                                            const float* __restrict__ dz, const uint32_t* __restrict__ ids,
                                                            uint32_t rows, uint32_t ncols, float* __restrict__ bh,
                                                            float* __restrict__ bl, uint32_t pitch_b,
-                                                           float* __restrict__ colsum_part, int vec_in, const uint32_t* __restrict__ scale_word) {
+                                                           float* __restrict__ colsum_part, int vec_in, const PnlsF16 f) {
   dyb_grid_dep_sync();
-  const float sc = F16 ? scale_of(__ldg(scale_word)) : 1.f;
-  __half* const hh = reinterpret_cast<__half*>(bh);
-  __half* const hl = reinterpret_cast<__half*>(bl);
   __shared__ float tile[64][65];   // [column][row]
   const uint32_t r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
   {
     const uint32_t rq = threadIdx.x & 15, cl = threadIdx.x >> 4;
     const uint32_t r = r0 + 4 * rq;
+    float rs[4] = {1.f, 1.f, 1.f, 1.f};
+    if (F16) {
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) rs[k] = scale_of(__ldg(f.row_max + min(r + k, rows - 1)));
+    }
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const uint32_t c = c0 + cl + 16 * p;
       float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < ncols && r < rows) {
-        const float zc = z[c], dc = dz[c];
-        const uint32_t pick = ids ? ids[c] : 0xffffffffu;
-        const float* xc = x + (size_t)c * rows;
-        if (vec_in) {   // rows % 4 == 0: the four rows exist; same arithmetic as the vector path of k_expsub_bwd
-          const float4 v = ld4_stream(xc + r);
-          const float zl = zc * kLog2e;
-          d = make_float4(ex2_approx(fmaf(v.x, kLog2e, -zl)) * dc, ex2_approx(fmaf(v.y, kLog2e, -zl)) * dc,
-                          ex2_approx(fmaf(v.z, kLog2e, -zl)) * dc, ex2_approx(fmaf(v.w, kLog2e, -zl)) * dc);
-          if (pick - r < 4u) {
-            const uint32_t k = pick - r;
-            if (k == 0) d.x -= dc; else if (k == 1) d.y -= dc; else if (k == 2) d.z -= dc; else d.w -= dc;
-          }
-          if (F16) {
-            __half h[4], l[4];
-            split_f16(d.x * sc, h[0], l[0]); split_f16(d.y * sc, h[1], l[1]); split_f16(d.z * sc, h[2], l[2]); split_f16(d.w * sc, h[3], l[3]);
-            *reinterpret_cast<uint2*>(hh + (size_t)c * pitch_b + r) = *reinterpret_cast<const uint2*>(h);
-            *reinterpret_cast<uint2*>(hl + (size_t)c * pitch_b + r) = *reinterpret_cast<const uint2*>(l);
-          } else {
-            float4 h, l;
-            split_tf32(d.x, h.x, l.x); split_tf32(d.y, h.y, l.y); split_tf32(d.z, h.z, l.z); split_tf32(d.w, h.w, l.w);
-            st4(bh + (size_t)c * pitch_b + r, h);
-            st4(bl + (size_t)c * pitch_b + r, l);
-          }
-        } else {        // same arithmetic as its scalar path
-          float e[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (r + k < rows) {
-              e[k] = expf(xc[r + k] - zc) * dc;
-              if (r + k == pick) e[k] -= dc;
-              const size_t o = (size_t)c * pitch_b + r + k;
-              if (F16) split_f16(e[k] * sc, hh[o], hl[o]);
-              else split_tf32(e[k], bh[o], bl[o]);
-            }
-          }
-          d = make_float4(e[0], e[1], e[2], e[3]);
+        d = pnls_grad4(pnls_x4(x + (size_t)c * rows, r, rows, vec_in), r, rows, ids ? ids[c] : 0xffffffffu, z[c], dz[c], vec_in);
+        const size_t o = (size_t)c * pitch_b + r;   // (the pitch is a multiple of 32: the padding of a last, partial quad stays in it)
+        if (F16) {
+          const float cs = scale_of(__ldg(f.col_max + c));
+          __half h[4], l[4];
+          split_f16(d.x * cs, h[0], l[0]); split_f16(d.y * cs, h[1], l[1]); split_f16(d.z * cs, h[2], l[2]); split_f16(d.w * cs, h[3], l[3]);
+          *reinterpret_cast<uint2*>(f.hb + o) = *reinterpret_cast<const uint2*>(h);
+          *reinterpret_cast<uint2*>(f.lb + o) = *reinterpret_cast<const uint2*>(l);
+          split_f16(d.x * rs[0], h[0], l[0]); split_f16(d.y * rs[1], h[1], l[1]); split_f16(d.z * rs[2], h[2], l[2]); split_f16(d.w * rs[3], h[3], l[3]);
+          *reinterpret_cast<uint2*>(f.ha + o) = *reinterpret_cast<const uint2*>(h);
+          *reinterpret_cast<uint2*>(f.la + o) = *reinterpret_cast<const uint2*>(l);
+        } else {
+          float4 h, l;
+          split_tf32(d.x, h.x, l.x); split_tf32(d.y, h.y, l.y); split_tf32(d.z, h.z, l.z); split_tf32(d.w, h.w, l.w);
+          st4(bh + o, h);
+          st4(bl + o, l);
         }
       }
       float* t = &tile[cl + 16 * p][4 * rq];
@@ -934,15 +980,19 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
   if ((rc = dyb200_scratch(ctx, (size_t)grid.y * V * sizeof(float), &part))) return rc;
   const int vec_in = V % 4 == 0 && aligned16(x->v);
   if (f16) {
+    // lines = columns of x, positions = vocabulary; the planes are filled by the kernels here
+    F16Job jb, ja;
+    if ((rc = dyb200_f16_planes(ctx, nullptr, V, n, V, F16_LINE, &jb)) || (rc = dyb200_f16_planes(ctx, nullptr, V, n, V, F16_ELEM, &ja))) return rc;
+    dB = dyb200_f16_op(jb, false);
+    dA = dyb200_f16_op(ja, true);
+    DYB_CUDA(ctx, cudaMemsetAsync(jb.scale, 0, n * sizeof(uint32_t), ctx->stream));
+    DYB_CUDA(ctx, cudaMemsetAsync(ja.scale, 0, V * sizeof(uint32_t), ctx->stream));
+    dyb_launch(k_softmax_bwd_max, dim3((V + 1023) / 1024, (n + kPnlsMaxCols - 1) / kPnlsMaxCols), 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, ja.scale,
+               jb.scale, vec_in);
+    DYB_LAUNCHED(ctx);
+    dyb_launch(k_softmax_bwd_split<true>, grid, 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, nullptr, nullptr, jb.pitch, (float*)part, vec_in,
+               PnlsF16{jb.hi, jb.lo, ja.hi, ja.lo, jb.scale, ja.scale});
     F16Jobs jobs;
-    jobs.n = 1;
-    F16Job& jd = jobs.job[0];
-    if ((rc = dyb200_f16_planes(ctx, dEdf->v, n, n, V, F16_ALL, &jd))) return rc;   // lines = columns of x, positions = vocabulary
-    dB = dyb200_f16_op(jd, false);
-    dA = dyb200_f16_op(jd, true);
-    jd.lines = 1; jd.n = n;                                                          // (the scale word: over dE/df)
-    if ((rc = dyb200_f16_absmax(ctx, jobs))) return rc;
-    dyb_launch(k_softmax_bwd_split<true>, grid, 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, dB.hi, dB.lo, dB.pitch, (float*)part, vec_in, dB.scale);
     // R as H lines of V values, h as n lines of H values
     F16Job jr, jh;
     jobs.n = 0;
@@ -956,7 +1006,7 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
   } else {
     if ((rc = dyb200_tc_planes(ctx, n, V, &dB))) return rc;   // rows = columns, reduction over the vocabulary
     dA = dB; dA.rows = V; dA.K = n; dA.mn_major = 1;           // the same planes read with the vocabulary as rows
-    dyb_launch(k_softmax_bwd_split<false>, grid, 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, dB.hi, dB.lo, dB.pitch, (float*)part, vec_in, nullptr);
+    dyb_launch(k_softmax_bwd_split<false>, grid, 256, 0, ctx, x->v, z, dEdf->v, ids_dev, V, n, dB.hi, dB.lo, dB.pitch, (float*)part, vec_in, PnlsF16{});
     // h split as it lies (row = column, H values), read MN-major
     if ((rc = dyb200_tc_pack(ctx, h->v, H, true, n, H, nullptr, 0, 0, &hT, nullptr))) return rc;
     hT.rows = H; hT.K = n; hT.mn_major = 1;

@@ -52,3 +52,44 @@ def test_infinities_stay_in_their_rows():
     assert not bool(torch.isfinite(C[:, 5]).any())
     keep = torch.arange(M, device="cuda") != 5
     assert float((C[:50].double() - want)[:, keep].abs().max()) < 4.5e-7 * K * 2
+
+
+@pytest.mark.parametrize("V,H,n,param", [(12000, 256, 4000, False), (12001, 250, 4003, True)])
+def test_output_gradient_at_every_row_and_columns_own_scale(V, H, n, param):
+    """softmax_output_bwd_fused on fp16 pairs: vocabulary rows whose probability is tiny everywhere, columns whose dE/df differs by 2^40.
+    Against float64, every element of dR and dh relative to its own |row| |column|.  Bar: exp of arguments down to -65 (log2: 94) from
+    fp32 operands: half an ulp of the argument (2^-18), the rounding of log2(e) (94 x 2^-25) and of z (2^-21), times ln 2, and the
+    products' 4.5e-7: below 8e-6.  And the same operands as the node-by-node calls: equal bit for bit."""
+    import torch
+    from dynet_b200 import capi
+    ctx = capi.Context(0, torch.cuda.current_stream().cuda_stream)
+    gen = torch.Generator("cuda").manual_seed(V)
+    T = lambda t, d, bd=1: capi.DyTensor.of(t.data_ptr(), d, bd)   # noqa: E731
+    x = torch.randn(n, V, device="cuda", generator=gen)
+    x[:, 1::7] -= 28.0
+    x[:, 2::7] -= 50.0
+    ids = torch.randint(0, (V - 1) // 7, (n,), device="cuda", generator=gen) * 7
+    dE = torch.randn(n, device="cuda", generator=gen) * torch.exp2(torch.randint(-20, 20, (n,), device="cuda", generator=gen).float())
+    dE[11] = 0.0
+    h, R = torch.randn(n, H, device="cuda", generator=gen), torch.randn(H, V, device="cuda", generator=gen)
+    loss, aux = torch.empty(n, device="cuda"), torch.zeros(3 * n, device="cuda")
+    aux[2 * n:].view(torch.int32).copy_(ids.int())
+    tx, th, tR, tdE, at = T(x, [V], n), T(h, [H], n), T(R, [V, H]), T(dE, [1], n), capi.PickAttrs(None, n)
+    ctx.fwd("pickneglogsoftmax", [tx], T(loss, [1], n), at, aux.data_ptr())
+    dR, db, dh = torch.zeros(H, V, device="cuda"), torch.zeros(V, device="cuda"), torch.zeros(n, H, device="cuda")
+    ctx.softmax_output_bwd_fused(tx, th, tR, tdE, aux.data_ptr(), T(dR, [V, H]), T(db, [V]), T(dh, [H], n), flags=1 if param else 0)
+    # node by node
+    dx, nR, nh, nb = torch.zeros(n, V, device="cuda"), torch.zeros_like(dR), torch.zeros_like(dh), torch.zeros(V, device="cuda")
+    ctx.bwd("pickneglogsoftmax", [tx], T(loss, [1], n), tdE, 0, T(dx, [V], n), at, aux.data_ptr())
+    xs, aff = [T(db, [V]), tR, th], capi.AffineAttrs(1 if param else 0)
+    for i, d in ((1, T(nR, [V, H])), (2, T(nh, [H], n))):
+        ctx.bwd("affine_transform", xs, tx, T(dx, [V], n), i, d, aff)
+    d = torch.softmax(x.double(), dim=1)
+    d[torch.arange(n, device="cuda"), ids] -= 1.0
+    d *= dE.double()[:, None]
+    for name, got, want, scale in (("dR", dR, h.double().t() @ d, h.double().norm(dim=0)[:, None] * d.norm(dim=0)[None, :]),
+                                   ("dh", dh, d @ R.double().t(), d.norm(dim=1)[:, None] * R.double().norm(dim=1)[None, :])):
+        err = (got.double() - want).abs()
+        assert bool((err <= 1e-5 * scale).all()), "%s: %.3g" % (name, float((err / scale.clamp_min(1e-300)).max()))
+    assert torch.equal(dR, nR) and torch.equal(dh, nh)
+    assert ctx.device_errors() == 0
