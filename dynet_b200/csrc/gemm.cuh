@@ -63,7 +63,7 @@ __device__ __forceinline__ void epi_emit_h(const GemmEpilogue& epi, uint32_t u, 
 #ifdef __CUDACC__
 // ---- 2 x 11 bits in fp16 ---------------------------------------------------------------------------------------------------
 // A TF32 hi / lo pair carries 2 x 11 significand bits.  fp16 has the same 11, at twice the rate of the tensor pipe and half the
-// bytes, with 5 bits of exponent.  So an operand row (or a whole parameter) is scaled by a power of two that brings its largest
+// bytes, with 5 bits of exponent.  So an operand row is scaled by a power of two that brings its largest
 // element to [2^14, 2^15), hi = fp16(x s), lo = fp16((x s - hi) 2^11): elements down to 2^-28 of the row's largest keep all
 // 2 x 11 bits, smaller ones an absolute error below 2^-51 of it.  Per k step: A_hi x [B_hi | B_lo] as ONE instruction of twice
 // the columns (B_lo lies right behind B_hi in shared memory), whose halves are the accumulators D1 (hi hi) and D2, then
@@ -124,31 +124,32 @@ int dyb200_gemm_fused(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const
 // plane[r * pitch + k].  MN-major (left operands of dyb200_tc_gemm_packed only): element (r, k) at plane[k * pitch + r] -
 // the K-major planes of the transposed matrix, used as they are.
 // f16: the planes hold scaled fp16 pairs instead (below; hi / lo then point at halves, K-blocks are 64 wide) and `scale` the
-// scale words of the rows (scale_step 1) or of the whole operand (scale_step 0).
+// scale words of the rows.
 struct PackedOp {
   float* hi; float* lo; uint32_t rows, K, pitch; uint32_t mn_major = 0;
-  uint32_t f16 = 0; const uint32_t* scale = nullptr; uint32_t scale_step = 0;
+  uint32_t f16 = 0; const uint32_t* scale = nullptr;
 };
 // ---- fp16 operand planes ----
-// One operand as `lines` lines of n contiguous values (line i at src + ld i), its planes laid out alike.  Scale words: one per line
-// (F16_LINE: lines are rows of a K-major operand), one per position in the line (F16_ELEM: positions are rows of an MN-major
-// operand) or one in all (F16_ALL: planes that serve both ways).
-enum F16Scale { F16_LINE = 0, F16_ELEM = 1, F16_ALL = 2 };
+// One operand as `lines` lines of n contiguous values (line i at src + ld i), its planes laid out alike.  Every ROW of the operand has
+// a scale of its own: one word per line (F16_LINE: lines are rows of a K-major operand) or per position in the line (F16_ELEM:
+// positions are rows of an MN-major operand).  A matrix that is read both ways needs both sets of planes: with one scale for all of
+// it, rows 2^28 below its largest value would lose their bits.
+enum F16Scale { F16_LINE = 0, F16_ELEM = 1 };
 struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; };
 struct F16Jobs { F16Job job[2]; int n; };
 // Planes and scale words for a job from the scratch arena; dyb200_f16_pack fills those of up to two jobs in one pass each.
 int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
 int dyb200_f16_absmax(dyb200_ctx* ctx, const F16Jobs& jobs);       // the scale words alone
-// The same for a parameter (one scale word, so that its planes can be read both ways), from the parameter cache when it is on.
-int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, F16Job* job);
+// The same for a parameter, from the parameter cache when it is on.
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
 // Products from here on (useful flops) use fp16 pairs.  Finding the scales adds a clear and a pass over the operands: 8.6 GFLOP
 // (512 x 4096 x 2048) took 86 us that way and 70 us with TF32 pairs, 46 GFLOP (10000 x 2240 x 1024) 205 against 255 us.
 constexpr double kF16Flops = 24.0e9;
 // A queue of packing work that one kernel launch executes (several small operands per launch).
 constexpr int kMaxPackJobs = 8;
-constexpr int kLayoutGates = 2, kLayoutF16 = 3;
+constexpr int kLayoutGates = 2, kLayoutF16 = 3;   // (kLayoutF16 + F16_LINE or F16_ELEM)
 struct PackJob {
   const float* src; const float* mask; float* hi; float* lo;
   uint32_t ld, rows, K, mask_ld, pitch, gx, perm_H;

@@ -39,18 +39,12 @@ __device__ __forceinline__ uint64_t tile_desc(uint32_t addr, bool f16, uint32_t 
 __device__ __forceinline__ uint64_t mma_step(bool f16, uint32_t mn) { return !mn ? 2 : f16 ? 128 : 64; }
 // F16: the sums of row m, columns [n0, n0 + 64), divided by the scales of the row and the columns
 __device__ __forceinline__ void unscale_tile(const TmapPack& tm, float (&sum)[64], uint32_t m, uint32_t M, uint32_t n0, uint32_t N) {
-  const int ea = scale_field(__ldg(tm.sa + (size_t)min(m, M - 1) * tm.sa_step)) - 282;
-  if (tm.sb_step == 0) {
-    const int t = ea + scale_field(__ldg(tm.sb));
+  // (a lane fetches the words of two columns and hands them round)
+  const int ea = scale_field(__ldg(tm.sa + min(m, M - 1))) - 282;
+  const uint32_t lane = threadIdx.x & 31;
+  const int f0 = scale_field(__ldg(tm.sb + min(n0 + lane, N - 1))), f1 = scale_field(__ldg(tm.sb + min(n0 + 32 + lane, N - 1)));
 #pragma unroll
-    for (int j = 0; j < 64; ++j) sum[j] = unscale(sum[j], t);
-  } else {
-    // (a lane fetches the words of two columns and hands them round)
-    const uint32_t lane = threadIdx.x & 31;
-    const int f0 = scale_field(__ldg(tm.sb + min(n0 + lane, N - 1))), f1 = scale_field(__ldg(tm.sb + min(n0 + 32 + lane, N - 1)));
-#pragma unroll
-    for (int j = 0; j < 64; ++j) sum[j] = unscale(sum[j], ea + __shfl_sync(0xffffffffu, j < 32 ? f0 : f1, j & 31));
-  }
+  for (int j = 0; j < 64; ++j) sum[j] = unscale(sum[j], ea + __shfl_sync(0xffffffffu, j < 32 ? f0 : f1, j & 31));
 }
 
 // BNT = columns of the output tile: 128, or 64 for products with N <= 64 (small per-GPU batches), where a 128-wide tile
@@ -752,7 +746,6 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
     return;
   }
   __shared__ uint32_t red[8];
-  uint32_t all = 0;
   const uint32_t piece = 4096, pieces = (j.n + piece - 1) / piece;
   const uint64_t units = (uint64_t)pieces * j.lines;
   for (uint64_t u = blockIdx.x; u < units; u += gridDim.x) {
@@ -769,7 +762,6 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
 #pragma unroll 4
       for (uint32_t e = lo + threadIdx.x; e < hi; e += 256) m = max(m, finite_mag(p[e]));
     }
-    if (j.mode == F16_ALL) { all = max(all, m); continue; }
     m = __reduce_max_sync(0xffffffffu, m);
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
@@ -778,16 +770,6 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
 #pragma unroll
       for (int w = 1; w < 8; ++w) m = max(m, red[w]);
       if (pieces == 1) j.scale[line] = m; else atomicMax(j.scale + line, m);
-    }
-  }
-  if (j.mode == F16_ALL) {
-    all = __reduce_max_sync(0xffffffffu, all);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = all;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int w = 1; w < 8; ++w) all = max(all, red[w]);
-      if (all) atomicMax(j.scale, all);
     }
   }
 }
@@ -816,7 +798,7 @@ __global__ void __launch_bounds__(256) k_f16_split(const F16Jobs jobs) {
 #pragma unroll
       for (uint32_t i = 0; i < 4; ++i) s[i] = scale_of(__ldg(j.scale + min(e + i, j.n - 1)));
     } else {
-      s[0] = s[1] = s[2] = s[3] = scale_of(__ldg(j.scale + (j.mode == F16_LINE ? line : 0u)));
+      s[0] = s[1] = s[2] = s[3] = scale_of(__ldg(j.scale + line));
     }
     uint2 hi, lo;
     split4_f16(make_float4(v[0], v[1], v[2], v[3]), make_float4(s[0], s[1], s[2], s[3]), hi, lo);
@@ -920,7 +902,7 @@ int pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int layout, uint32_t ro
 inline uint32_t round_up(uint32_t x, uint32_t m) { return (x + m - 1) / m * m; }
 
 // Returns the cached packed form of a parameter matrix, packing it first if it is new or stale.
-// (k_is_fast = kLayoutF16: fp16 planes of the matrix as it lies, its scale word behind the hi plane)
+// (k_is_fast = kLayoutF16 + F16_LINE or F16_ELEM: fp16 planes of the matrix as it lies, its scale words behind the hi plane)
 int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_fast, uint32_t rows, uint32_t K, uint32_t pitch,
                       float** hi, float** lo, const float* src2 = nullptr, uint32_t rows2 = 0) {
   const int cap = (int)(sizeof(ctx->param_pack) / sizeof(ctx->param_pack[0]));
@@ -933,7 +915,7 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     else if (victim->hi && e->last_use < victim->last_use) victim = e;
   }
   dyb200_ctx::ParamPack* e = hit ? hit : victim;
-  const size_t floats = k_is_fast == kLayoutF16 ? (size_t)rows * pitch / 2 + 64 : (size_t)(rows + rows2) * pitch;
+  const size_t floats = k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE ? rows : K) : (size_t)(rows + rows2) * pitch;
   if (!hit) {
     if (e->hi && e->floats < floats) {   // evicted entry is too small: its buffers may still be read by queued kernels
       DYB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -952,10 +934,10 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     e->src = src; e->src2 = src2; e->rows2 = rows2; e->ld = ld; e->rows = rows; e->K = K; e->pitch = pitch; e->k_is_fast = (int)k_is_fast;
     e->version = ~0ull;
   }
-  if (e->version != ctx->param_version && k_is_fast == kLayoutF16) {
+  if (e->version != ctx->param_version && k_is_fast >= kLayoutF16) {
     F16Jobs jobs;
     jobs.n = 1;
-    jobs.job[0] = F16Job{src, ld, rows, K, pitch, F16_ALL, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
+    jobs.job[0] = F16Job{src, ld, rows, K, pitch, k_is_fast - kLayoutF16, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
     int rc = dyb200_f16_pack(ctx, &jobs);
     if (rc) return rc;
     e->version = ctx->param_version;
@@ -1010,27 +992,27 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
-int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, F16Job* job) {
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job) {
   if (!ctx->param_cache_on) {
     F16Jobs jobs;
     jobs.n = 1;
-    int rc = dyb200_f16_planes(ctx, src, ld, lines, n, F16_ALL, &jobs.job[0]);
+    int rc = dyb200_f16_planes(ctx, src, ld, lines, n, mode, &jobs.job[0]);
     if (!rc) rc = dyb200_f16_pack(ctx, &jobs);
     *job = jobs.job[0];
     return rc;
   }
   const uint32_t pitch = round_up(n, 64);
   float *hi, *lo;
-  int rc = cached_param_pack(ctx, src, ld, kLayoutF16, lines, n, pitch, &hi, &lo);
+  int rc = cached_param_pack(ctx, src, ld, kLayoutF16 + mode, lines, n, pitch, &hi, &lo);
   if (rc) return rc;
-  *job = F16Job{src, ld, lines, n, pitch, F16_ALL, reinterpret_cast<uint32_t*>(hi + (size_t)lines * pitch / 2), (__half*)hi, (__half*)lo};
+  *job = F16Job{src, ld, lines, n, pitch, mode, reinterpret_cast<uint32_t*>(hi + (size_t)lines * pitch / 2), (__half*)hi, (__half*)lo};
   return DYB200_OK;
 }
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major) {
   PackedOp p;
   p.hi = (float*)j.hi; p.lo = (float*)j.lo; p.pitch = j.pitch; p.f16 = 1; p.mn_major = mn_major ? 1u : 0u;
   p.rows = mn_major ? j.n : j.lines; p.K = mn_major ? j.lines : j.n;
-  p.scale = j.scale; p.scale_step = j.mode == F16_ALL ? 0u : 1u;
+  p.scale = j.scale;
   return p;
 }
 
@@ -1192,7 +1174,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   DYB_CHECK_ARG(ctx, !f16 || (npairs == 1 && B[0].f16 && A[0].scale && B[0].scale && A[0].pitch % 64 == 0 && B[0].pitch % 64 == 0),
                 "tensor GEMM: fp16 operands come in one pair, both with scale words and a pitch that is a multiple of 64");
   DYB_CHECK_ARG(ctx, f16 || !B[0].f16, "tensor GEMM: operands of two kinds");
-  tm.sa = A[0].scale; tm.sb = B[0].scale; tm.sa_step = A[0].scale_step; tm.sb_step = B[0].scale_step;
+  tm.sa = A[0].scale; tm.sb = B[0].scale;
   // (an MN-major plane is read in groups of 32 rows: its pitch covers the rows rounded up to 32)
   DYB_CHECK_ARG(ctx, !a_mn || (npairs == 1 && A[0].pitch % 32 == 0 && A[0].pitch >= M && aligned16(A[0].hi) && aligned16(A[0].lo)),
                 "tensor GEMM: an MN-major left operand needs a single pair, a pitch that is a multiple of 32 and covers the rows, and 16-byte aligned planes");
@@ -1357,10 +1339,10 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       auto ahead = [&](float* q, size_t n) { return f16 ? (float*)((__half*)q + n) : q + n; };
       const size_t ao = a_mn ? (size_t)m_off : (size_t)m_off * A[p].pitch, bo = b_mn ? (size_t)n_off : (size_t)n_off * B[p].pitch;
       A2[p].hi = ahead(A[p].hi, ao); A2[p].lo = ahead(A[p].lo, ao);
-      if (f16) { A2[p].scale += (size_t)m_off * A[p].scale_step; }
+      if (f16) A2[p].scale += m_off;
       B2[p] = B[p]; B2[p].rows = N - n_off;
       B2[p].hi = ahead(B[p].hi, bo); B2[p].lo = ahead(B[p].lo, bo);
-      if (f16) { B2[p].scale += (size_t)n_off * B[p].scale_step; }
+      if (f16) B2[p].scale += n_off;
     }
     GemmEpilogue e2 = epi;
     e2.C += m_off + (size_t)epi.ldc * n_off;
@@ -1424,15 +1406,14 @@ int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const Ge
   *handled = 1;
   PackedOp A[2], B[2];
   if (npairs == 1 && !pairs[0].maskB && flops >= kF16Flops) {
-    // Both operands as they lie: lines are rows of a K-major operand (A transposed / B not), or k of an MN-major one.  Rows have
-    // their own scale; a parameter has one, so that one set of planes serves this product and the one that uses it transposed.
+    // Both operands as they lie: lines are rows of a K-major operand (A transposed / B not), or k of an MN-major one.
     const GemmPair& g = pairs[0];
     const bool a_mn = g.transA == 0, b_mn = g.transB != 0;
     F16Jobs jobs;
     F16Job ja, jb;
     int rc;
     jobs.n = 0;
-    if (g.a_is_param) rc = dyb200_f16_param(ctx, g.A, g.lda, a_mn ? g.K : M, a_mn ? M : g.K, &ja);
+    if (g.a_is_param) rc = dyb200_f16_param(ctx, g.A, g.lda, a_mn ? g.K : M, a_mn ? M : g.K, a_mn ? F16_ELEM : F16_LINE, &ja);
     else if (!(rc = dyb200_f16_planes(ctx, g.A, g.lda, a_mn ? g.K : M, a_mn ? M : g.K, a_mn ? F16_ELEM : F16_LINE, &ja))) jobs.job[jobs.n++] = ja;
     if (rc) return rc;
     if ((rc = dyb200_f16_planes(ctx, g.B, g.ldb, b_mn ? g.K : N, b_mn ? N : g.K, b_mn ? F16_ELEM : F16_LINE, &jb))) return rc;

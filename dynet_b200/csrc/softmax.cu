@@ -996,7 +996,7 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
     // R as H lines of V values, h as n lines of H values
     F16Job jr, jh;
     jobs.n = 0;
-    if (flags & DYB200_GEMM_A_IS_PARAM) rc = dyb200_f16_param(ctx, R->v, V, H, V, &jr);
+    if (flags & DYB200_GEMM_A_IS_PARAM) rc = dyb200_f16_param(ctx, R->v, V, H, V, F16_LINE, &jr);
     else if (!(rc = dyb200_f16_planes(ctx, R->v, V, H, V, F16_LINE, &jr))) jobs.job[jobs.n++] = jr;
     if (rc || (rc = dyb200_f16_planes(ctx, h->v, H, n, H, F16_ELEM, &jh))) return rc;
     jobs.job[jobs.n++] = jh;

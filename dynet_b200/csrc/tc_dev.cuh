@@ -30,8 +30,8 @@ constexpr uint32_t kEpiWarps = 8;
 // plane[k * pitch + m], the layout of a K x M row-major matrix - and t[0], t[1] are 3-D maps over (m within a group of 32,
 // k, group) with a box of 32 x 32 x 4; see load_a_tile / umma_desc_mn.  b_mn: the same for the B planes (t[2], t[3]; the
 // box holds as many groups as the tile has columns / 32).
-// F16 products (see "2 x 11 bits" in gemm.cuh): sa / sb are the operands' scale words, one per row (step 1) or one for all (step 0).
-struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; const uint32_t *sa, *sb; uint32_t sa_step, sb_step;
+// F16 products (see "2 x 11 bits" in gemm.cuh): sa / sb are the scale words of the operands' rows.
+struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; const uint32_t *sa, *sb;
   uint32_t store_map; };   // store_map: t[4] describes the output (persistent kernel, plain stores; one pair)
 
 // The k-blocks of K split z of S: [b0, b0 + n0) of pair 0, then [b1, b1 + n1) of pair 1 (each pair cut into S equal shares).

@@ -54,6 +54,36 @@ def test_infinities_stay_in_their_rows():
     assert float((C[:50].double() - want)[:, keep].abs().max()) < 4.5e-7 * K * 2
 
 
+@pytest.mark.parametrize("tA", [0, 1])
+@pytest.mark.parametrize("cache", [False, True])
+def test_parameter_rows_keep_their_own_scale(tA, cache):
+    """A parameter operand whose rows differ by 2^60: the same bar as any other product.  With the cache on the second product takes
+    the planes of the first, and the transposed product of the same matrix must not get them with the wrong scales."""
+    import torch
+    from dynet_b200 import capi
+    M, N, K = 4100, 2999, 1030
+    ctx = capi.Context(0, torch.cuda.current_stream().cuda_stream)
+    ctx.param_cache(cache)
+    gen = torch.Generator("cuda").manual_seed(7)
+    A = torch.randn(*((M, K) if tA else (K, M)), device="cuda", generator=gen)
+    A *= torch.exp2(torch.randint(-30, 30, (M,), device="cuda", generator=gen).float()).view((M, 1) if tA else (1, M))
+    B = torch.randn(N, K, device="cuda", generator=gen)
+    C = torch.empty(N, M, device="cuda")
+    for _ in range(2):
+        C.fill_(7.0)
+        ctx.gemm(tA, 0, M, N, K, A.data_ptr(), K if tA else M, B.data_ptr(), K, C.data_ptr(), M, 0, 1)   # 1: A_IS_PARAM
+        Ad = (A if tA else A.t()).double()
+        err = (C.double() - B.double() @ Ad.t()).abs() / (B.double().norm(dim=1)[:, None] * Ad.norm(dim=1)[None, :])
+        assert float(err.max()) <= 4.5e-7
+    # the transposed product: K rows, every one of them with elements of all magnitudes
+    D, E = torch.randn(N, M, device="cuda", generator=gen), torch.empty(N, K, device="cuda")
+    ctx.gemm(1 - tA, 0, K, N, M, A.data_ptr(), K if tA else M, D.data_ptr(), M, E.data_ptr(), K, 0, 1)   # 1: A_IS_PARAM
+    At = (A.t() if tA else A).double()
+    err = (E.double() - D.double() @ At.t()).abs() / (D.double().norm(dim=1)[:, None] * At.norm(dim=1)[None, :])
+    assert float(err.max()) <= 4.5e-7
+    assert ctx.device_errors() == 0
+
+
 @pytest.mark.parametrize("V,H,n,param", [(12000, 256, 4000, False), (12001, 250, 4003, True)])
 def test_output_gradient_at_every_row_and_columns_own_scale(V, H, n, param):
     """softmax_output_bwd_fused on fp16 pairs: vocabulary rows whose probability is tiny everywhere, columns whose dE/df differs by 2^40.
