@@ -3,6 +3,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "lstm_rec_api.h"
 
 int dyb200_fail(dyb200_ctx* ctx, int code, const char* fmt, ...) {
   if (ctx) {
@@ -107,9 +108,15 @@ int dyb200_ctx_destroy(dyb200_ctx* ctx) {
   return DYB200_OK;
 }
 
+int dyb200i_dependent_launch(dyb200_ctx* ctx, int set) {
+  const int was = ctx->pdl;
+  if (set >= 0 && !ctx->pdl_chosen) ctx->pdl = set;
+  return was;
+}
 int dyb200_ctx_dependent_launch(dyb200_ctx* ctx, int enable) {
   if (!ctx) return DYB200_EINVAL;
   ctx->pdl = enable ? 1 : 0;
+  ctx->pdl_chosen = 1;
   return DYB200_OK;
 }
 

@@ -1,4 +1,4 @@
-/* Internal interface between the kernel library and the C++ drivers (host/): the LSTM recurrence of one or two directions over
+/* Internal interface between the kernel library and the C++ drivers (host/).  The LSTM recurrence of one or two directions over
  * ragged batches in one launch per pass, with its products over all columns formed outside.  Not part of the public C ABI.
  *
  * Columns are laid out step after step: step t has the columns [prefix[t], prefix[t + 1]), and the widths never grow.  The
@@ -32,6 +32,17 @@ int dyb200i_rec_bwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint
 /* dx += Wx^T dgates (.* mask_x, which repeats every `period` columns when mask_full), dgates = the planes left in w by rec_bwd. */
 int dyb200i_rec_dx(dyb200_ctx* ctx, struct dyb200_wgrad* w, const float* Wx, uint32_t I, uint32_t H, uint32_t columns, const float* mask_x,
                    int mask_full, uint32_t period, float* dx);
+
+/* The dependent-launch setting in force.  set >= 0 changes it, unless the caller of the library has chosen one. */
+int dyb200i_dependent_launch(dyb200_ctx* ctx, int set);
 #ifdef __cplusplus
 }
+/* A driver's own launches are ordinary ones unless the caller has chosen otherwise; the context is left as it was found. */
+struct dyb200i_ordinary_launches {
+  dyb200_ctx* ctx;
+  int was;
+  explicit dyb200i_ordinary_launches(dyb200_ctx* c) : ctx(c), was(dyb200i_dependent_launch(c, 0)) {}
+  ~dyb200i_ordinary_launches() { dyb200i_dependent_launch(ctx, was); }
+  dyb200i_ordinary_launches(const dyb200i_ordinary_launches&) = delete;
+};
 #endif

@@ -20,6 +20,7 @@
 #include <string>
 #include <vector>
 
+#include "../csrc/lstm_rec_api.h"
 #include "dynet_shim.h"
 
 using namespace dynet_b200;
@@ -470,8 +471,8 @@ int dyb200h_lm_create(const dyb200h_lm_config* c, float* params, float* grads, v
   dyb200_ctx_param_cache(ctx, 1);
   // Inside a CUDA graph the launches follow one another closely as it is, and CTAs that are scheduled early and wait keep the SMs
   // from other streams: three models on three streams took 143 instead of 126 us per step (V 2000, H 256, batch 16), 3.30 instead
-  // of 3.16 ms (V 10000, H 1024, batch 64).
-  dyb200_ctx_dependent_launch(ctx, 0);
+  // of 3.16 ms (V 10000, H 1024, batch 64).  So this driver's own launches are ordinary ones, here and in every call below.
+  const dyb200i_ordinary_launches ordinary(ctx);
   int rc = DYB200_OK;
   if (c->fused) {
     for (uint32_t l = 0; l < c->L && !rc; ++l) {
@@ -493,6 +494,7 @@ void dyb200h_lm_destroy(void* h) { delete (Lm*)h; }
 const char* dyb200h_lm_error(void* h) { return h ? ((Lm*)h)->err.c_str() : "null handle"; }
 
 static int guarded(Lm* m, void (*fn)(Lm&, void*), void* arg) {
+  const dyb200i_ordinary_launches ordinary(m->dev.ctx);
   try {
     fn(*m, arg);
     return DYB200_OK;
@@ -555,6 +557,7 @@ int dyb200h_lm_forward_backward_phase(void* h, int phase, const uint32_t* tokens
 // Squared L2 norm of the local gradients into a device scalar (reduce it over ranks before update).
 int dyb200h_lm_grad_sumsq(void* h, float** scalar_dev_out) {
   Lm* m = (Lm*)h;
+  const dyb200i_ordinary_launches ordinary(m->dev.ctx);
   size_t n = param_sizes(m->c, nullptr);
   int rc = dyb200_squared_norm(m->grads, n, m->scalars, 0, m->dev.ctx);
   if (rc) { m->err = dyb200_last_error(m->dev.ctx); return rc; }
@@ -565,6 +568,7 @@ int dyb200h_lm_grad_sumsq(void* h, float** scalar_dev_out) {
 // SimpleSGD update with gradient clipping from the scalar computed by dyb200h_lm_grad_sumsq; zeroes the gradients.
 int dyb200h_lm_update(void* h) {
   Lm* m = (Lm*)h;
+  const dyb200i_ordinary_launches ordinary(m->dev.ctx);
   size_t n = param_sizes(m->c, nullptr);
   int rc = dyb200_sgd_update(m->params, m->grads, n, m->c.lr, m->c.clip, m->scalars, m->dev.ctx);
   if (rc) m->err = dyb200_last_error(m->dev.ctx);

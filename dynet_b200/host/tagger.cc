@@ -364,6 +364,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
 }
 
 int guarded(Tagger* m, const PassArgs& a) {
+  const dyb200i_ordinary_launches ordinary(m->dev.ctx);
   try {
     tagger_pass(*m, a);
     return DYB200_OK;
@@ -411,7 +412,7 @@ int dyb200h_tagger_create(const dyb200h_tagger_config* c, float* params, float* 
   if (!rc) rc = dyb200_ctx_create(device, m->stream2, &m->dev2.ctx);
   if (!rc) dyb200_ctx_param_cache(m->dev2.ctx, 1);
   // (two streams: a kernel scheduled early would hold SMs that the other direction's kernels could use)
-  dyb200_ctx_dependent_launch(ctx, 0);
+  const dyb200i_ordinary_launches ordinary(ctx);
   if (!rc) dyb200_ctx_dependent_launch(m->dev2.ctx, 0);
   if (!rc && (cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
@@ -445,6 +446,7 @@ int dyb200h_tagger_forward_backward(void* h, uint32_t n_sent, const uint32_t* le
 
 int dyb200h_tagger_grad_sumsq(void* h, float** scalar_dev_out) {
   Tagger* m = (Tagger*)h;
+  const dyb200i_ordinary_launches ordinary(m->dev.ctx);
   int rc = dyb200_squared_norm(m->grads, tagger_sizes(m->c, nullptr), m->scalars, 0, m->dev.ctx);
   if (rc) { m->err = dyb200_last_error(m->dev.ctx); return rc; }
   if (scalar_dev_out) *scalar_dev_out = m->scalars;
@@ -452,6 +454,7 @@ int dyb200h_tagger_grad_sumsq(void* h, float** scalar_dev_out) {
 }
 int dyb200h_tagger_update(void* h) {
   Tagger* m = (Tagger*)h;
+  const dyb200i_ordinary_launches ordinary(m->dev.ctx);
   int rc = dyb200_sgd_update(m->params, m->grads, tagger_sizes(m->c, nullptr), m->c.lr, m->c.clip, m->scalars, m->dev.ctx);
   if (rc) m->err = dyb200_last_error(m->dev.ctx);
   dyb200_ctx_params_changed(m->dev2.ctx);   // (the second direction's context keeps its own split weights)

@@ -224,3 +224,33 @@ def test_lm_training_with_other_trainers(oracle, rule):
         assert not model.grads_host()[0].any()
     assert model.ctx.device_errors() == 0
     model.close()
+
+
+@pytest.mark.parametrize("kind", ["lm", "tagger"])
+def test_drivers_leave_the_dependent_launch_setting_as_they_find_it(kind):
+    """On by default for a context's node calls; a driver's own launches are ordinary ones unless the caller has chosen, and neither its
+    calls nor one that fails change what the caller's own calls on the context do."""
+    import ctypes as C
+    from dynet_b200 import capi, lm, tagger
+    setting = capi.lib().dyb200i_dependent_launch
+    setting.argtypes, setting.restype = [C.c_void_p, C.c_int], C.c_int
+    if kind == "lm":
+        dims = dict(V=50, E=20, H=12, L=1, T=3, B=5)
+        m = lm.LstmLm(device=0, seed=1, dropout=False, **dims)
+        batch, _ = lm.synthetic_batch(dims, seed=2, dropout=0.0)
+        calls = [lambda: m.launch_forward_backward(batch, None), m.update]
+    else:
+        m = tagger.Tagger(50, 16, 8, 6, 5, max_sentences=4, max_tokens=40, max_len=10, seed=1)
+        batch = tagger.synthetic_corpus(4, 50, 5, seed=3, lo=2, hi=10)
+
+        def refused():
+            with pytest.raises(capi.InvalidArgument):
+                m.launch_forward_backward(batch[0], batch[1] + 50, batch[2])
+        calls = [lambda: m.launch_forward_backward(*batch), refused, m.update]
+    for chosen in (None, True, False):
+        if chosen is not None:
+            m.ctx.dependent_launch(chosen)
+        for call in calls:
+            call()
+            assert setting(m.ctx.h, -1) == (0 if chosen is False else 1)
+    m.close()
