@@ -46,6 +46,7 @@ struct dyb200_ctx {
   int16_t rec_tc_fit[2][8];     // the same for lstm_rec_tc.cu: [pass][CTAs per cluster - 1]
   int16_t rec_fit[2][6][17];    // clusters of the recurrence kernels (lstm_rec.cu) that fit at once: [pass][width class][CTAs per cluster]
   int seq_coop;                 // 0 = not tried, 1 = launched with the cooperative attribute, -1 = the driver refused it
+  int wide_refused;             // the driver refused lstm_wide.cu's gang launch: its sequences run launch by launch
   uint64_t param_version, param_tick;
   struct ParamPack {
     const float* src; const float* src2; uint32_t ld, rows, rows2, K, pitch; int k_is_fast;   // src2 / rows2: a second matrix stacked below the first

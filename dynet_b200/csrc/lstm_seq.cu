@@ -572,9 +572,12 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
         DYB_CHECK_ARG(ctx, dyb200_wgrad_column_planes(deferred, T * B, nullptr, &X, &Hs) && Hs.K == H, "lstm sequence: the accumulator does not hold the inputs of this layer");
         a.hn_hi = Hs.hi; a.hn_lo = Hs.lo; a.hn_pitch = Hs.pitch;
       }
-      if ((rc = dyb200_wide_fwd(ctx, a))) return rc;
-      if (deferred) dyb200_wgrad_seq_done(deferred);
-      return DYB200_OK;
+      bool launched;
+      if ((rc = dyb200_wide_fwd(ctx, a, &launched))) return rc;
+      if (launched) {
+        if (deferred) dyb200_wgrad_seq_done(deferred);
+        return DYB200_OK;
+      }
     }
     for (uint32_t t = 0; t < T; ++t) {
       GemmPair p{Wh->v, G, 0, t ? h_all->v + (size_t)(t - 1) * HB : h_first, H, 0, H, mh, H, mh_full, 1};

@@ -169,9 +169,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_lstm_wide_fwd(const __grid_
 // Up to 8 columns (each costs a step 0.6 - 0.8 us of polls and multiply-adds; 1024 units: 2.1 us at 1, 5.3 at 4, 7.8 at 8 columns, launch by
 // launch 5.0, 7.3 and 10.4) and as many units as the SMs hold, 8 each; narrower layers
 // belong to the clusters of lstm_rec.cu.
-bool dyb200_wide_takes(const dyb200_ctx* ctx, uint32_t H, uint32_t B) { return H > 384 && H <= 1536 && H <= kWideUnits * (uint32_t)ctx->sm_count && B <= 8; }
+bool dyb200_wide_takes(const dyb200_ctx* ctx, uint32_t H, uint32_t B) { return !ctx->wide_refused && H > 384 && H <= 1536 && H <= kWideUnits * (uint32_t)ctx->sm_count && B <= 8; }
 
-int dyb200_wide_fwd(dyb200_ctx* ctx, WideFwd a) {
+int dyb200_wide_fwd(dyb200_ctx* ctx, WideFwd a, bool* launched) {
+  *launched = true;
   void* x;
   const size_t bytes = (size_t)2 * a.B * a.H * sizeof(unsigned long long);
   int rc = dyb200_scratch(ctx, bytes, &x);
@@ -186,12 +187,23 @@ int dyb200_wide_fwd(dyb200_ctx* ctx, WideFwd a) {
   cfg.gridDim = dim3((a.H + kWideUnits - 1) / kWideUnits); cfg.blockDim = dim3(kWideThreads);
   cfg.dynamicSmemBytes = (size_t)a.B * (512 * kj + 128) * sizeof(float); cfg.stream = ctx->stream;
   if (cfg.dynamicSmemBytes > 48 * 1024) DYB_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
-  // (the CTAs wait on one another: launched as one gang, as the sequence kernels are)
+  // The CTAs wait on one another: launched as one gang.  A driver that refuses that gets the launches step by step; where the
+  // caller has asked for launches without the attribute (dyb200_ctx_sequence_kernels), or the sequence kernels found it refused, a plain one.
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = ctx->seq_coop >= 0 ? 1 : 0;
+  if (ctx->seq_coop >= 0) {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k, a) != cudaSuccess) {
+      (void)cudaGetLastError();
+      ctx->wide_refused = 1;
+      *launched = false;
+      return DYB200_OK;
+    }
+    ctx->launches++;
+    return DYB200_OK;
+  }
   cudaLaunchKernelEx(&cfg, k, a);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;

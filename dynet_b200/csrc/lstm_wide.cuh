@@ -15,4 +15,5 @@ struct WideFwd {
   uint32_t* flags;
 };
 bool dyb200_wide_takes(const dyb200_ctx* ctx, uint32_t H, uint32_t B);
-int dyb200_wide_fwd(dyb200_ctx* ctx, WideFwd a);
+// *launched = false: the driver refused the launch, nothing has run.
+int dyb200_wide_fwd(dyb200_ctx* ctx, WideFwd a, bool* launched);

@@ -67,3 +67,60 @@ def test_wide_recurrence_matches_oracle(oracle, g, I, H, B, T, mask):
         assert_close(g.host(got), ref, TOL_REDUCE, floor=0.1, what=name)
     for name, got, ref in zip(("dWx", "dWh"), (dWx, dWh), want[5:7]):
         assert_close(g.host(got), ref, TOL_REDUCE, floor=row_floor(ref, 0, rel=1e-2), what=name + " (per-row scale)")
+
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <cuda_runtime_api.h>
+#include <dlfcn.h>
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) {
+  static cudaError_t (*real)(const cudaLaunchConfig_t*, const void*, void**);
+  if (!real) real = (cudaError_t (*)(const cudaLaunchConfig_t*, const void*, void**))dlsym(RTLD_NEXT, "cudaLaunchKernelExC");
+  for (unsigned k = 0; k < c->numAttrs; ++k)
+    if (c->attrs[k].id == cudaLaunchAttributeCooperative) return cudaErrorNotSupported;
+  return real(c, f, a);
+}
+"""
+SEQUENCE = """
+import sys, torch
+from dynet_b200 import capi
+H, B, T, I = 520, 3, 9, 16
+gen = torch.Generator("cuda").manual_seed(1)
+rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen) * 0.2
+x, h0, c0, Wx, Wh, b = rnd(T * B, I), rnd(B, H), rnd(B, H), rnd(I, 4 * H), rnd(H, 4 * H) * 0.2, rnd(4 * H)
+gates, cs, hs = (torch.zeros(T * B, n, device="cuda") for n in (4 * H, H, H))
+t = lambda v, d, n=1: capi.DyTensor.of(v.data_ptr(), d, n)
+ctx = capi.Context(0, torch.cuda.current_stream().cuda_stream)
+w = ctx.wgrad_create(4 * H, I, H, T * B)
+n = []
+for _ in range(2):
+    l0 = ctx.launches()
+    ctx.lstm_seq_fwd(t(x, [I], T * B), t(h0, [H], B), t(c0, [H], B), t(Wx, [4 * H, I]), t(Wh, [4 * H, H]), t(b, [4 * H]), None, None,
+                     capi.LstmGatesAttrs(0, 0.0, 1.0), t(gates, [4 * H], T * B), t(cs, [H], T * B), t(hs, [H], T * B), w, T)
+    n.append(ctx.launches() - l0)
+torch.cuda.synchronize()
+assert ctx.device_errors() == 0
+torch.save((n, gates.cpu(), cs.cpu(), hs.cpu()), sys.argv[1])
+"""
+
+
+def test_a_refused_gang_launch_runs_step_by_step(tmp_path):
+    """A driver that does not take the cooperative attribute (a fake of the launch call that returns cudaErrorNotSupported for it): the same
+    sequence, launch by launch, to the rounding of its sums."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    import torch
+    (tmp_path / "shim.c").write_text(SHIM)
+    subprocess.check_call(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "shim.so"), str(tmp_path / "shim.c"), "-I/usr/local/cuda/include", "-ldl"])
+    out = []
+    for name, extra in (("taken", {}), ("refused", {"LD_PRELOAD": str(tmp_path / "shim.so")})):
+        p = subprocess.run([sys.executable, "-c", SEQUENCE, str(tmp_path / name)], cwd=Path(__file__).resolve().parent.parent, env=dict(os.environ, **extra),
+                           capture_output=True, text=True)
+        assert p.returncode == 0, p.stderr[-800:]
+        out.append(torch.load(str(tmp_path / name)))
+    (n0, *a), (n1, *b) = out
+    assert max(n0) < 8 and min(n1) > 9
+    for p, q in zip(a, b):
+        assert_close(q.numpy(), p.numpy(), TOL_REDUCE, floor=0.1, what="refused")
