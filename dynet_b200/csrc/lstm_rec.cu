@@ -570,8 +570,8 @@ bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan*
   const bool sf = ff > 0 && deal_columns(N, ff, ndir, fwd_col_bytes(p), &p.Gf, &p.ncapf), sb = fb > 0 && deal_columns(N, fb, ndir, bwd_col_bytes(p), &p.Gb, &p.ncapb);
   // More than four columns per cluster: the tensor pipe, where the width lets it (256 units, a step: 1.8 us here at 3 columns,
   // 8.0 at 37; there 2.5 at any number)
-  p.tcf = !(sf && (N + p.Gf - 1) / p.Gf <= 4) && dyb200_rec_tc_plan(ctx, false, H, N, &p.tf);
-  p.tcb = !(sb && (N + p.Gb - 1) / p.Gb <= 4) && dyb200_rec_tc_plan(ctx, true, H, N, &p.tb);
+  p.tcf = !(sf && (N + p.Gf - 1) / p.Gf <= 4) && dyb200_rec_tc_plan(ctx, false, H, N, ndir, &p.tf);
+  p.tcb = !(sb && (N + p.Gb - 1) / p.Gb <= 4) && dyb200_rec_tc_plan(ctx, true, H, N, ndir, &p.tb);
   if (!(sf || p.tcf) || !(sb || p.tcb)) return false;
   *out = p;
   return true;

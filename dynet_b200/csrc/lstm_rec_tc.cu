@@ -654,9 +654,10 @@ uint32_t tc_smem(bool bwd, uint32_t H) {
 
 }  // namespace
 
-// Clusters per direction (of kGroups x 16 columns each).
-bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, RecTcPlan* out) {
-  if (H > 256 || N == 0) return false;
+// Clusters per direction (of kGroups x 16 columns each); all of them are the grid's second dimension.
+bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int ndir, RecTcPlan* out) {
+  const uint64_t clusters = ((uint64_t)N + kGroups * kTcCols - 1) / (kGroups * kTcCols);
+  if (H > 256 || N == 0 || clusters * ndir > 65535u) return false;
   const uint32_t C = (H + kTcUnits - 1) / kTcUnits;
   int16_t& fit = ctx->rec_tc_fit[bwd][C - 1];
   if (fit == 0) {   // (asked once: whether a cluster fits this device at all)
@@ -669,7 +670,7 @@ bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, RecTc
     fit = (int16_t)(n > 0 ? n : -1);
   }
   if (fit <= 0) return false;
-  out->G = (N + kGroups * kTcCols - 1) / (kGroups * kTcCols);
+  out->G = (uint32_t)clusters;
   return true;
 }
 int dyb200_rec_tc_fwd(dyb200_ctx* ctx, const RecTcPlan& p, RecFwd* a, int ndir) {

@@ -139,3 +139,31 @@ def test_recurrence_is_the_same_every_time(g, I, H, B, T):
     finally:
         ctx.wgrad_destroy(w)
     assert ctx.device_errors() == 0
+
+
+def test_more_columns_than_a_grid_holds(g):
+    """Past 65 535 clusters the recurrence kernels hand the layer back to the per-step calls."""
+    import ctypes as C
+    import torch
+    from dynet_b200 import capi
+    ctx, most = g.ctx(), 65535 * 32
+    takes = capi.lib().dyb200i_rec_takes
+    takes.argtypes, takes.restype = [C.c_void_p, C.c_uint32, C.c_uint32, C.c_uint32, C.c_int], C.c_int
+    assert [takes(ctx.h, 4, 8, most, 1), takes(ctx.h, 4, 8, most + 1, 1), takes(ctx.h, 4, 8, 32767 * 32, 2), takes(ctx.h, 4, 8, 32768 * 32, 2)] == [1, 0, 1, 0]
+    I, H, T, B, few = 3, 4, 8, most + 1, 50
+    gen = torch.Generator("cuda").manual_seed(9)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen) * 0.5
+    x, h0, c0, Wx, Wh, b = rnd(T, B, I), rnd(B, H), rnd(B, H), rnd(I, 4 * H), rnd(H, 4 * H), rnd(4 * H)
+
+    def run(x, h0, c0):
+        n = h0.shape[0]
+        gates, cs, hs = (torch.empty(T * n, k, device="cuda") for k in (4 * H, H, H))
+        ctx.lstm_seq_fwd(g.T(x, [I], T * n), g.T(h0), g.T(c0), g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1), None, None,
+                         capi.LstmGatesAttrs(0, 0.0, 1.0), g.T(gates, [4 * H], T * n), g.T(cs, [H], T * n), g.T(hs, [H], T * n), None, T)
+        torch.cuda.synchronize()
+        return hs.view(T, n, H)
+    every = run(x, h0, c0)
+    for cols in (slice(0, few), slice(B - few, B)):
+        want = run(x[:, cols].contiguous(), h0[cols].contiguous(), c0[cols].contiguous())
+        assert_close(g.host(every[:, cols]), g.host(want), TOL_REDUCE, floor=0.1, what="h of %d columns" % B)
+    assert ctx.device_errors() == 0
