@@ -170,6 +170,13 @@ __device__ __forceinline__ void dyb_grid_dep_sync() {
     __builtin_unreachable();
   }
 }
+// Raises a kernel's limit on dynamic shared memory to `most`, one value per kernel whatever the launch takes of it: the limit belongs to the
+// function, and a value per launch would let one thread lower it between another thread's call and launch.
+template <class F>
+inline cudaError_t dyb_smem_limit(F kernel, size_t smem, size_t most) {
+  if (smem <= 48 * 1024) return cudaSuccess;
+  return smem > most ? cudaErrorInvalidValue : cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -14,6 +14,7 @@ namespace {
 constexpr int kThreadsN = 256;
 constexpr uint32_t kNarrow = 64;                 // what counts as narrow
 constexpr uint32_t kSmallMax = 16 * 1024;        // floats of op(A) kept in shared memory
+constexpr size_t kSmemNarrow = 200 * 1024;       // above what any shape takes: 64 KB of op(A) and three pieces of up to 35 KB; 96 KB
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(void* dst, const float* src, uint32_t bytes) {   // bytes < 16: the rest is zero
@@ -287,7 +288,7 @@ int launch_narrow(dyb200_ctx* ctx, Narrow a) {
   a.MP = per * 8 * ML;
   const uint32_t by = (blocks + per - 1) / per;
   const size_t smem = sizeof(float) * ((size_t)a.K * a.MP + (size_t)kStagesN * TN * a.pitch);
-  if (smem > 48 * 1024) DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_narrow<ML, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DYB_CUDA(ctx, dyb_smem_limit(k_gemm_narrow<ML, NJ>, smem, kSmemNarrow));
   const uint32_t per_sm = smem <= 72 * 1024 ? 3 : smem <= 110 * 1024 ? 2 : 1, cap = per_sm * (uint32_t)ctx->sm_count;
   dyb_launch(k_gemm_narrow<ML, NJ>, dim3(tiles < cap ? tiles : cap, by), kThreadsN, smem, ctx, a);
   DYB_LAUNCHED(ctx);
@@ -360,7 +361,7 @@ int dyb200_gemm_narrow(dyb200_ctx* ctx, uint32_t M, uint32_t N, const GemmPair& 
   a.part = (float*)part;
   const size_t ring = (size_t)kStagesN * a.KC * (a.MT + a.NT), sums = (size_t)a.groups * a.MT * a.NT;
   const size_t smem = sizeof(float) * (ring > sums ? ring : sums);
-  if (smem > 48 * 1024) DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_narrow_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DYB_CUDA(ctx, dyb_smem_limit(k_gemm_narrow_k, smem, kSmemNarrow));
   dyb_launch(k_gemm_narrow_k, dim3(gx, by), kThreadsN, smem, ctx, a);
   DYB_LAUNCHED(ctx);
   dyb_launch(k_narrow_reduce, (M * N + 31) / 32, 256, 0, ctx, (const float*)a.part, gx, M, N, epi.C, epi.ldc, epi.mode == EPI_ACCUM ? 1 : 0);

@@ -281,7 +281,7 @@ int thin_launch(dyb200_ctx* ctx, ThinArgs& a, bool gates, double flops) {
   const size_t smem = xs > red ? xs : red;
   void (*k)(ThinArgs) = gates ? (vec ? thin_kernel<true, true>(nb) : thin_kernel<true, false>(nb))
                               : (vec ? thin_kernel<false, true>(nb) : thin_kernel<false, false>(nb));
-  if (smem > 48 * 1024) DYB_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DYB_CUDA(ctx, dyb_smem_limit(k, smem, 160 * 1024));
   GemmProfScope scope(ctx, flops, 0, a.M, a.N, a.p[0].K + (a.npairs > 1 ? a.p[1].K : 0), (uint32_t)a.mode);
   dyb_launch(k, dim3(blocks, (a.N + nb - 1) / nb), threads, smem, ctx, a);
   DYB_LAUNCHED(ctx);

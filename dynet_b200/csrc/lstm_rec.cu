@@ -523,7 +523,7 @@ size_t fwd_smem(const RecPlan& p, uint32_t ncap) {
 }  // namespace
 
 int dyb200_rec_launch_cfg(dyb200_ctx* ctx, const void* kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, dim3 grid, uint32_t threads, size_t smem) {
-  DYB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DYB_CUDA(ctx, dyb_smem_limit(kernel, smem, kRecSmemMax));
   if (grid.x > 8) DYB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   memset(cfg, 0, sizeof(*cfg));
   cfg->gridDim = grid; cfg->blockDim = dim3(threads, 1, 1); cfg->dynamicSmemBytes = smem; cfg->stream = ctx->stream;

@@ -186,7 +186,7 @@ int dyb200_wide_fwd(dyb200_ctx* ctx, WideFwd a, bool* launched) {
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((a.H + kWideUnits - 1) / kWideUnits); cfg.blockDim = dim3(kWideThreads);
   cfg.dynamicSmemBytes = (size_t)a.B * (512 * kj + 128) * sizeof(float); cfg.stream = ctx->stream;
-  if (cfg.dynamicSmemBytes > 48 * 1024) DYB_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+  DYB_CUDA(ctx, dyb_smem_limit(k, cfg.dynamicSmemBytes, 8 * (512 * 3 + 128) * sizeof(float)));
   // The CTAs wait on one another: launched as one gang.  A driver that refuses that gets the launches step by step; where the
   // caller has asked for launches without the attribute (dyb200_ctx_sequence_kernels), or the sequence kernels found it refused, a plain one.
   cudaLaunchAttribute attr[1];
