@@ -174,14 +174,8 @@ class LstmLm:
             ptr, on_dev = tokens.data_ptr(), 1 if tokens.is_cuda else 0
         mp = None
         if masks_dev is not None:
-            mp = self._pointers(masks_dev)
+            mp = (C.c_void_p * len(masks_dev))(*[m.data_ptr() for m in masks_dev])
         self._check(self.H.dyb200h_lm_forward_backward(self.h, ptr, on_dev, mp, self.loss_dev.data_ptr()))
-
-    def _pointers(self, masks):
-        own = self._mask_views
-        if own is not None and len(own) == len(masks) and all(a is b for a, b in zip(own, masks)):
-            return self._mask_ptrs          # the driver's own buffers, as draw_masks hands them out
-        return (C.c_void_p * len(masks))(*[m.data_ptr() for m in masks])
 
     def _token_ptr(self, tokens):
         if isinstance(tokens, np.ndarray):
@@ -269,7 +263,6 @@ class LstmLm:
             off = ptrs[k] - base
             out.append(self.workspace[off:off + 4 * B * cols].view(self.torch.float32).view(B, cols))
         self._mask_views = out
-        self._mask_ptrs = (C.c_void_p * n)(*[m.data_ptr() for m in out])
         # the masks' part of a draw: (tensor, vectors of four random numbers before it)
         self._mask_plan, quads = [], 0
         for m in out:

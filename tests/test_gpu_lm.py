@@ -254,3 +254,23 @@ def test_drivers_leave_the_dependent_launch_setting_as_they_find_it(kind):
             call()
             assert setting(m.ctx.h, -1) == (0 if chosen is False else 1)
     m.close()
+
+
+def test_masks_are_read_where_they_are_at_the_call():
+    """A mask tensor that draw_masks has handed out and that the caller has since pointed at other memory: its present memory counts."""
+    import torch
+    from dynet_b200 import lm
+    dims = dict(V=50, E=16, H=12, L=1, T=3, B=5)
+    m = lm.LstmLm(device=0, seed=1, dropout=True, **dims)
+    tokens, _ = lm.synthetic_batch(dims, seed=2, dropout=0.0)
+
+    def loss(masks):
+        m.grads.zero_()
+        m.launch_forward_backward(tokens, masks)
+        return float(m.loss_dev.item())
+    bufs = m.draw_masks(0.5, 3, 0)
+    own, ones = loss(bufs), torch.ones_like(bufs[0])
+    want = loss([ones, bufs[1]])
+    bufs[0].data = ones
+    assert loss(bufs) == want != own
+    m.close()
