@@ -239,13 +239,19 @@ def lib():
     return _LIB
 
 
-try:
-    from . import _call
-    _call.setup(C.Structure, DyTensor, C.c_void_p, C.sizeof(DyTensor))
-    _native_call = _call.call
-except ImportError:         # not built (no Python headers): every call goes through ctypes
-    def _native_call(*args):
-        return NotImplemented
+def _native_call(*args):
+    """host/py/call.c's call(), loaded when the first entry point is called (whoever imports this module for its shapes alone maps nothing);
+    not built (no Python headers): every call goes through ctypes."""
+    global _native_call
+    try:
+        from . import _call
+        _call.setup(C.Structure, DyTensor, C.c_void_p, C.sizeof(DyTensor))
+        _native_call = _call.call
+    except ImportError:
+        def _native_call(*args):
+            return NotImplemented
+    return _native_call(*args)
+
 
 _ENTRIES = {}
 

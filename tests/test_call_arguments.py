@@ -97,3 +97,15 @@ except (TypeError, C.ArgumentError):
 """ % call
     p = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True)
     assert p.returncode == 0 and p.stdout.strip() == "refused", (p.returncode, p.stdout, p.stderr[-500:])
+
+
+def test_importing_the_bindings_maps_nothing():
+    """The reference arm of the benchmark imports them for the synthetic batch and the parameter shapes."""
+    code = """
+import bench
+from dynet_b200 import lm, tagger
+lm.synthetic_batch(dict(V=20, E=8, H=8, L=1, T=2, B=3), seed=1, dropout=0.0), lm.param_shapes(20, 8, 8, 1), tagger.param_shapes(20, 8, 8, 4, 3)
+print([l.split("/")[-1].strip() for l in open("/proc/self/maps") if "dynet_b200" in l])
+"""
+    p = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True)
+    assert p.returncode == 0 and p.stdout.strip() == "[]", (p.stdout, p.stderr[-500:])
