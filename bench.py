@@ -365,18 +365,22 @@ def run_gpu(args):
         which = "tensor" if prof["tensor"][1] >= prof["simt"][1] and prof["tensor"][1] > 0 else "simt"
         g_ms, g_n, g_fl = prof[which]
         achieved = g_fl / (g_ms * 1e-3) / 1e12 if g_ms > 0 else 0.0
-        peak = tf32 / 3.0
+        # ceiling: a product on TF32 pairs (path 1) costs three TF32 MMAs, one on fp16 pairs (path 2) three fp16 ones; together, the rate at
+        # which the step's mix of the two would run at both ceilings
+        f16 = peaks["bf16_tflops_sustained"]
+        fl_f16 = sum(r_[6] for r_ in per_launch if r_[4] == 2)
+        peak = 1.0 / ((1.0 - fl_f16 / g_fl) * 3.0 / tf32 + fl_f16 / g_fl * 3.0 / f16) if g_fl > 0 else tf32 / 3.0
         # per shape: launches per step, device time, useful TFLOP/s, and the bytes one launch has to move at least (the split
         # operand planes once, the result once; read-modify-write for the accumulating epilogues)
         shapes = {}
         for (M_, N_, K_, mode, path, t_ms, fl) in per_launch:
-            rec = shapes.setdefault((M_, N_, K_, mode), [0, 0.0, 0.0])
+            rec = shapes.setdefault((M_, N_, K_, mode, path), [0, 0.0, 0.0])
             rec[0] += 1; rec[1] += t_ms; rec[2] += fl
         by_shape = []
-        for (M_, N_, K_, mode), (cnt, t_ms, fl) in sorted(shapes.items(), key=lambda kv: -kv[1][1]):
-            operand = 8.0 * K_ * (M_ + N_)
+        for (M_, N_, K_, mode, path), (cnt, t_ms, fl) in sorted(shapes.items(), key=lambda kv: -kv[1][1]):
+            operand = (4.0 if path == 2 else 8.0) * K_ * (M_ + N_)
             result = 4.0 * M_ * N_ * (2 if mode in (1, 3) else 1) * (5.0 / 4.0 if mode == 5 else 1.0)   # LSTM epilogue: + c and h
-            by_shape.append({"M": M_, "N": N_, "K": K_, "epilogue": int(mode), "launches_per_step": cnt / args.steps,
+            by_shape.append({"M": M_, "N": N_, "K": K_, "epilogue": int(mode), "pairs": {1: "tf32", 2: "fp16"}.get(path), "launches_per_step": cnt / args.steps,
                              "us_per_launch": 1e3 * t_ms / cnt, "useful_tflops": fl / (t_ms * 1e-3) / 1e12 if t_ms > 0 else None,
                              "algorithmic_bytes_per_launch": operand + result})
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
@@ -388,13 +392,14 @@ def run_gpu(args):
                         "output_layer_M10000_N17920_K1024": 1.54e9,
                         "note": "dram__bytes_read.sum + dram__bytes_write.sum of one launch from the committed ncu summaries "
                                 "(0.82 GB read + 0.72 GB written; algorithmic 0.83 GB); tensor-bound kernels, DRAM at 15-19 % of peak"},
-                    "kernel": "gemm_3xtf32_tcgen05" if which == "tensor" else "gemm_fp32_cuda_core",
+                    "kernel": "tcgen05 products on TF32 and fp16 pairs" if which == "tensor" else "gemm_fp32_cuda_core",
+                    "share_of_flops_on_fp16_pairs": fl_f16 / g_fl if g_fl > 0 else None,
                     "launches": g_n, "share_of_step_time": g_ms / ms_prof if ms_prof else None,
                     "by_shape": by_shape[:12],
                     "measured_over": "the same %d steps issued launch by launch (%.2f ms/step) right after the timed region, "
                                      "which replays them as one CUDA graph" % (args.steps, ms_prof / args.steps),
-                    "peak_source": "cuBLAS TF32 8192^3 measured in this run (%.0f TFLOP/s) / 3; bf16 peak of %s: %s TFLOP/s"
-                                   % (tf32, peaks["source"], peaks["bf16_tflops"]),
+                    "peak_source": "cuBLAS TF32 8192^3 measured in this run (%.0f TFLOP/s) / 3 and the sustained bf16 rate of %s (%s TFLOP/s) / 3, weighted "
+                                   "by the step's operations on either kind of pairs" % (tf32, peaks["source"], f16),
                     "useful_tflop_per_step": flops_per_step(B) * world / 1e12}
         cpu_rec = None if args.no_cpu_baseline else cpu_baseline_record(32, 1)
         # the memory-bound kernels one by one (CUDA-graph timed, rotating buffers): the other half of the metric

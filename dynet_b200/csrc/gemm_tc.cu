@@ -1252,7 +1252,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       kb_per_split = (kb_total + Sc - 1) / Sc;
       cfg.gridDim = dim3(grid.x, grid.y, Sc);
       attr[0].val.clusterDim.z = Sc;
-      GemmProfScope scope(ctx, flops, 1, M, N, kb_total * el, (uint32_t)epi.mode);
+      GemmProfScope scope(ctx, flops, f16 ? 2 : 1, M, N, kb_total * el, (uint32_t)epi.mode);
       auto kern = f16 ? (bn == 64 ? k_gemm_tc<64, true, true> : k_gemm_tc<128, true, true>) : (bn == 64 ? k_gemm_tc<64, true> : k_gemm_tc<128, true>);
       cudaLaunchKernelEx(&cfg, kern, tm, M, N, kb0, kb1, kb_per_split, epi, ctx->dev_flags);
       DYB_LAUNCHED(ctx);
@@ -1321,7 +1321,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       tm.store_map = 1;
     }
     {
-      GemmProfScope scope(ctx, flops * ((double)tiles_run / (grid.x * grid.y)), 1, M, N, kb_total * el, (uint32_t)epi.mode);
+      GemmProfScope scope(ctx, flops * ((double)tiles_run / (grid.x * grid.y)), f16 ? 2 : 1, M, N, kb_total * el, (uint32_t)epi.mode);
       // grouped tile order when the A operand has many row blocks (unless the last round runs apart as part of the last
       // column of tiles, which relies on the row-block-fastest order)
       const uint32_t gm = (tail_form != 1 && rows_run > 16) ? 16u : 0u;
@@ -1351,7 +1351,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   }
   {
     // times the MMA kernel (and the split-K reduction); the packing launches show up in the step time
-    GemmProfScope scope(ctx, flops, 1, M, N, kb_total * el, (uint32_t)epi.mode);
+    GemmProfScope scope(ctx, flops, f16 ? 2 : 1, M, N, kb_total * el, (uint32_t)epi.mode);
     auto kern = f16 ? (bn == 64 ? k_gemm_tc<64, false, true> : k_gemm_tc<128, false, true>) : (bn == 64 ? k_gemm_tc<64, false> : k_gemm_tc<128, false>);
     dyb_launch(kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb0, kb1, kb_per_split, kepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);

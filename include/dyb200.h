@@ -74,15 +74,17 @@ uint64_t dyb200_ctx_launch_count(const dyb200_ctx* ctx);
 int dyb200_ctx_profile_begin(dyb200_ctx* ctx, int capacity);
 int dyb200_ctx_profile_end(dyb200_ctx* ctx, double ms_out[2], uint64_t launches_out[2], double flops_out[2]);
 /* Between begin and end: the number of GEMM launches recorded so far, and launch k of them: shape = {M, N, sum of K,
- * epilogue mode}, path = 1 for the tensor-pipe kernels, its device time (waits for that launch) and its useful FLOPs. */
+ * epilogue mode}, path = 0 for the CUDA-core kernels, 1 for the tensor pipe on TF32 pairs, 2 on fp16 pairs, its device time (waits for
+ * that launch) and its useful FLOPs. */
 int dyb200_ctx_profile_count(const dyb200_ctx* ctx);
 int dyb200_ctx_profile_launch(dyb200_ctx* ctx, int k, uint32_t shape_out[4], int* path_out, float* ms_out, double* flops_out);
 /* Parameter cache for the tensor-pipe GEMM (off by default).  The GEMM splits every operand into
- * TF32 hi/lo planes first; with the cache on, the planes of a PARAMETER matrix (the LSTM's Wx / Wh, or
+ * hi / lo planes first; with the cache on, the planes of a PARAMETER matrix (the LSTM's Wx / Wh, or
  * the A operand of dyb200_gemm called with DYB200_GEMM_A_IS_PARAM) are kept and reused until the
  * parameters change.  The caller must call dyb200_ctx_params_changed after every in-place update of
  * parameter values (dyb200_sgd_update does it itself); in a DyNet tree that is the end of
- * Trainer::update (dynet/training.cc:195-265).  Costs up to 2x the size of each cached matrix. */
+ * Trainer::update (dynet/training.cc:195-265).  Costs, for every way a matrix is read (as it lies, transposed, gate rows
+ * interleaved), twice its size on TF32 pairs and once on fp16 pairs. */
 int dyb200_ctx_param_cache(dyb200_ctx* ctx, int enable);
 /* Programmatic dependent launch (on by default).  When on, the kernels of this library are launched so that they may be
  * scheduled while their predecessor in the stream still runs; each kernel waits, before its first memory access, until that
@@ -163,7 +165,9 @@ int dyb200_pickneglogsoftmax_bwd(DYB200_BWD_ARGS); /* dynet/nodes-pickneglogsoft
  * dyb200_pickneglogsoftmax_bwd into a zeroed d(x) followed by dyb200_affine_transform_bwd for i = 0, 1, 2
  * (dynet/nodes-pickneglogsoftmax.cc:120-146, dynet/nodes-affinetransform.cc:120-157), but d(x) is never stored as a
  * tensor: one pass over x writes it as the split operands of the two products (dR += d h^T, dh += R^T d) and as
- * per-tile column sums for db.  x: Dim({V}, n) logits; h: Dim({H}, n); R: Dim({V, H}); dEdf: n loss gradients; aux_mem:
+ * per-tile column sums for db.  From 24 GFLOP on the operands are fp16 pairs (2 x 11 bits) with one scale per row of dR and one per
+ * column of dh: an error is relative to |row of d| |row of h| and |row of R^T| |column of d|, whatever the probabilities and dEdf of the
+ * other words and columns.  x: Dim({V}, n) logits; h: Dim({H}, n); R: Dim({V, H}); dEdf: n loss gradients; aux_mem:
  * the PickNegLogSoftmax node's aux_mem as left by its forward call; dR, db, dh are accumulated into.  dx_scratch
  * (Dim({V}, n), overwritten) is only used for shapes too small for the tensor-pipe products and may be NULL otherwise.
  * flags: DYB200_GEMM_A_IS_PARAM when R is a parameter and the parameter cache is on. */
@@ -309,21 +313,27 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
  * x_all = Dim({I}, steps * batch) holds the layer inputs of all steps side by side (batch columns each), gates_all / c_all /
  * h_all = Dim({4H} / {H} / {H}, steps * batch) receive every step's gates, c_t and h_t; h0 / c0 = Dim({H}, batch) are the state
  * before the first step; masks as in dyb200_vanilla_lstm_fwd_fused (the same mask for every step, dynet/lstm.cc:1010-1030).
- * Equivalent, bit for bit, to dyb200_wgrad_pack_inputs(deferred, x_all, mask_x, batch) followed by steps calls of
- * dyb200_vanilla_lstm_fwd_fused_at with deferred_col = t * batch, h_tm1 / c_tm1 = the previous step's outputs.  When the shape
- * allows (tensor-path sizes, whole tiles, every CTA resident at once) the steps run inside ONE kernel whose CTAs stay on the
- * GPU for the whole sequence and hand h_t over through device memory; otherwise the per-step calls are made.  Sequences of at
- * least 8 steps of layers up to 384 units, or with at most 32 columns, form Wx x of all steps at once and keep only Wh h in the
- * recurrence, in fp32: the same values to fp32 rounding (the sums associate differently), and the same bits from run to run.
- * dyb200_ctx_sequence_kernels(ctx, 0) forces the per-step form.  deferred may be NULL (nothing recorded for the weight
- * gradients). */
+ * Equivalent to dyb200_wgrad_pack_inputs(deferred, x_all, mask_x, batch) followed by steps calls of
+ * dyb200_vanilla_lstm_fwd_fused_at with deferred_col = t * batch, h_tm1 / c_tm1 = the previous step's outputs.
+ *   * When the shape allows (deferred given, tensor-path sizes, whole tiles, every CTA resident at once) the steps run inside ONE
+ *     kernel whose CTAs stay on the GPU for the whole sequence and hand h_t over through device memory: bit for bit the calls above.
+ *   * Other sequences of at least 8 steps of layers up to 384 units, or with at most 32 columns, form Wx x of all steps at once and
+ *     keep only Wh h in the recurrence: the same values to the rounding of their sums, which associate differently, and the same
+ *     bits from run to run.  Wh h is plain fp32 above 256 units, and below while there are at most four columns per cluster of
+ *     CTAs (60 columns at 256 units, more for narrower layers); with more columns it is a product of scaled fp16 pairs, 2 x 11 bits as
+ *     the TF32 pairs of the calls above have: Wh scaled by the largest value of each gate row, h by that of the initial state in
+ *     the first step and by the largest mask value (1 without) after it (16 columns share them).  What lies 2^28 below such a scale keeps
+ *     an absolute error of 2^-51 of it, the rounding of a pre-activation of 2^-27.
+ *   * Otherwise the calls above are made.  dyb200_ctx_sequence_kernels(ctx, 0) forces that.
+ * h0 / c0 may lie on a step's columns of h_all / c_all (a text read piece by piece into the same buffers).  deferred may be NULL
+ * (nothing recorded for the weight gradients). */
 int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0,
                                 const dyb200_tensor* Wx, const dyb200_tensor* Wh, const dyb200_tensor* b,
                                 const dyb200_tensor* mask_x, const dyb200_tensor* mask_h, const dyb200_lstm_gates_attrs* attrs,
                                 dyb200_tensor* gates_all, dyb200_tensor* c_all, dyb200_tensor* h_all, struct dyb200_wgrad* deferred,
                                 uint32_t steps, dyb200_ctx* ctx);
 /* The backward pass of the same layer over all time steps, in sweep order (dynet/exec.cc:96-140 visits the nodes of step
- * steps - 1 first): equivalent, bit for bit, to calling dyb200_vanilla_lstm_bwd_fused_at for t = steps - 1 .. 0 with
+ * steps - 1 first): equivalent to calling dyb200_vanilla_lstm_bwd_fused_at for t = steps - 1 .. 0 with
  * gates / c_t / dEdh / dEdc = the columns of step t of gates_all / c_all / dh_all / dc_all, dx = the columns of step t of
  * dx_all, dh_tm1 / dc_tm1 = the columns of step t - 1 of dh_all / dc_all (NULL at t = 0; h_tm1 / c_tm1 are h0 / c0 there) and
  * deferred_col = t * batch.  dh_all / dc_all hold dE/dh_t and dE/dc_t of every
@@ -333,8 +343,10 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
  * steps run inside ONE kernel whose CTAs stay on the GPU: the cell pass and the [Wx; Wh]^T dgates product of a step hand
  * over through counters in device memory, and every CTA alternates between two independent blocks of batch columns so that
  * one block's hand-overs hide behind the other's products (the per-step call uses the same K splits for such shapes, which
- * keeps the two forms bit-identical).  Sequences of at least 8 steps of layers up to 384 units keep only Wh^T dgates in the
- * recurrence, in fp32, and form dx of all steps at once: the same values to fp32 rounding.
+ * keeps the two forms bit-identical).  Other sequences of at least 8 steps of layers up to 384 units keep only Wh^T dgates in the
+ * recurrence and form dx of all steps at once: the same values to the rounding of their sums, the same bits from run to run.  Wh^T
+ * dgates is plain fp32 or a product of scaled fp16 pairs by the same rule as forward; Wh is scaled by the largest value of a unit's
+ * weights within a CTA's 32 units, dgates by the largest value of a column within them.
  * dyb200_ctx_sequence_kernels(ctx, 0) forces the per-step form. */
 int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0,
                                 const dyb200_tensor* Wx, const dyb200_tensor* Wh, const dyb200_tensor* mask_x,
@@ -387,8 +399,10 @@ int dyb200_trainer_update(int rule, float* params, float* grads, float* state0, 
                           const dyb200_trainer_hyper* hyper, const float* grad_sumsq, int zero_grads, dyb200_ctx* ctx);
 
 /* ---- GEMM used by the LSTM gates (dynet/matrix-multiply.h:16-37, :97-117, :162-180) ----
- * C[M x N] (+)= op(A) * op(B), column-major, fp32 in/out, 3xTF32 on the tensor pipe
- * when the shape allows (else an fp32 CUDA-core kernel).  transA/transB as in BLAS. */
+ * C[M x N] (+)= op(A) * op(B), column-major, fp32 in/out.  Up to 32 columns, and with a narrow side and a long one, on
+ * the CUDA cores in fp32; else on the tensor pipe as three products of TF32 pairs or, from 24 GFLOP on, of fp16 pairs whose rows
+ * of op(A) and columns of op(B) are scaled by their largest value (2 x 11 bits either way); shapes too small for that on the
+ * CUDA cores.  transA/transB as in BLAS. */
 #define DYB200_GEMM_A_IS_PARAM 1u /* flags: A is a parameter matrix (see dyb200_ctx_param_cache) */
 int dyb200_gemm(int transA, int transB, uint32_t M, uint32_t N, uint32_t K, const float* A,
                 uint32_t lda, const float* B, uint32_t ldb, float* C, uint32_t ldc, int accumulate,
