@@ -389,9 +389,9 @@ def run_gpu(args):
                     # traffic is therefore given per shape below, next to the bytes that shape has to move at least
                     "traffic": None,
                     "traffic_captured_per_launch": {
-                        "output_layer_M10000_N17920_K1024": 1.54e9,
-                        "note": "dram__bytes_read.sum + dram__bytes_write.sum of one launch from the committed ncu summaries "
-                                "(0.82 GB read + 0.72 GB written; algorithmic 0.83 GB); tensor-bound kernels, DRAM at 15-19 % of peak"},
+                        "output_layer_M10000_N17920_K1024": 1.08e9,
+                        "note": "dram__bytes_read.sum + dram__bytes_write.sum of one launch from the committed ncu summary "
+                                "(0.41 GB read + 0.67 GB written; algorithmic 0.83 GB); tensor-bound, DRAM at a fifth of its peak"},
                     "kernel": "tcgen05 products on TF32 and fp16 pairs" if which == "tensor" else "gemm_fp32_cuda_core",
                     "share_of_flops_on_fp16_pairs": fl_f16 / g_fl if g_fl > 0 else None,
                     "launches": g_n, "share_of_step_time": g_ms / ms_prof if ms_prof else None,

@@ -6,7 +6,7 @@
 // keeps the 32 gate rows of its 8 units for the whole sequence, and a step is one trip of h_t through L2: every value goes out
 // as one 8-byte store of the value and the number of its step, and whoever needs it polls that word - no fence, no counter, no second
 // round trip.  Two buffers: a CTA writes h_{t+1} only after it has read all of h_t, which every CTA wrote after reading h_{t-1}.
-// 2.0 us per step of 1024 units, one column.
+// 2.1 us per step of 1024 units, one column.
 //
 // Thread (q, s) of 4 x 128: gate q of the 8 units, k = 512 j + 4 s + 0..3.  Sums over s by a butterfly that leaves each group of four
 // lanes one unit, then over four warps through shared memory; thread (column, unit) of the first ones finishes the cell.

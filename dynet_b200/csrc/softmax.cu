@@ -437,7 +437,8 @@ int run_expsub_bwd(dyb200_ctx* ctx, const float* x, const float* z, const float*
 // but stored only as the hi / lo TF32 planes of the two products that consume it in the backward pass of
 // x = b + R h:  planes bh / bl [c][r] - K-major right operand of dh += R^T d (reduction index = r) and, as they are, the
 // MN-major left operand of dR += d h^T (reduction index = c) - plus the sums over the 64 columns of the tile for the bias
-// gradient (transposed through shared memory).  One 64 x 64 tile per CTA, 16-byte accesses along r.  x is read once;
+// gradient (transposed through shared memory).  One 64 x 64 tile per CTA, 16-byte accesses along r.  x is read once
+// (fp16 pairs: once more for their scales, and two sets of planes, see below);
 // nothing else of d reaches HBM (the fp32 tensor, its zero fill, two packing passes and a transposed copy of the planes go).
 struct ChunkOfPart {   // f(r, b) = v[r + n * b]
   const float* v; size_t n;
