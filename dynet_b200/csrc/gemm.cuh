@@ -227,4 +227,8 @@ bool dyb200_wgrad_column_planes(const dyb200_wgrad* w, uint32_t columns, PackedO
 void dyb200_wgrad_h_done(dyb200_wgrad* w);
 // A 2-D tensor map (CUtensorMap, 128 bytes at `map`) over a K-major plane: box = 32 floats of K x box_rows rows, 128-byte swizzle.
 int dyb200_tc_make_tmap(dyb200_ctx* ctx, void* map, float* plane, uint32_t rows, uint32_t K, uint32_t pitch, uint32_t box_rows);
+// A 3-D tensor map over S matrices side by side (M x N each, leading dimension ldc, 16-byte aligned): box = 128 rows x box_cols columns.
+int dyb200_tc_make_store_map(dyb200_ctx* ctx, void* map, float* C, uint32_t M, uint32_t N, uint32_t S, uint32_t ldc, uint32_t box_cols);
+// Products of fp16 pairs on pairs of SMs (gemm_pair.cu).
+bool dyb200_pair_takes(const dyb200_ctx* ctx, uint32_t M, uint32_t N, const GemmEpilogue& epi);
 uint32_t dyb200_tc_tile_cols(uint32_t N);   // width of the output tile the tensor path uses for N columns (64 or 128)

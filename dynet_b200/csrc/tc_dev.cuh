@@ -8,6 +8,15 @@
 
 #include "gemm.cuh"
 
+// pair p: t[4p] = A_hi, A_lo, B_hi, B_lo.  a_mn != 0 (one pair only): the A planes are MN-major - element (m, k) at
+// plane[k * pitch + m], the layout of a K x M row-major matrix - and t[0], t[1] are 3-D maps over (m within a group of 32,
+// k, group) with a box of 32 x 32 x 4; see load_a_tile / umma_desc_mn.  b_mn: the same for the B planes (t[2], t[3]; the
+// box holds as many groups as the tile has columns / 32).
+// F16 products (see "2 x 11 bits" in gemm.cuh): sa / sb are the scale words of the operands' rows.
+struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; const uint32_t *sa, *sb;
+  uint32_t store_map; };   // store_map: t[4] describes the output (persistent kernel, plain stores; one pair)
+int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint32_t kb, double flops, const GemmEpilogue& epi);
+
 namespace {
 
 
@@ -25,14 +34,6 @@ constexpr uint32_t kTmemCols = 256;       // two 128-column accumulators, used a
 constexpr uint32_t kChunkKB = 8;
 constexpr uint32_t kChunkF16 = 16;        // F16 products: k-blocks are 64 wide
 constexpr uint32_t kEpiWarps = 8;
-
-// pair p: t[4p] = A_hi, A_lo, B_hi, B_lo.  a_mn != 0 (one pair only): the A planes are MN-major - element (m, k) at
-// plane[k * pitch + m], the layout of a K x M row-major matrix - and t[0], t[1] are 3-D maps over (m within a group of 32,
-// k, group) with a box of 32 x 32 x 4; see load_a_tile / umma_desc_mn.  b_mn: the same for the B planes (t[2], t[3]; the
-// box holds as many groups as the tile has columns / 32).
-// F16 products (see "2 x 11 bits" in gemm.cuh): sa / sb are the scale words of the operands' rows.
-struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; const uint32_t *sa, *sb;
-  uint32_t store_map; };   // store_map: t[4] describes the output (persistent kernel, plain stores; one pair)
 
 // The k-blocks of K split z of S: [b0, b0 + n0) of pair 0, then [b1, b1 + n1) of pair 1 (each pair cut into S equal shares).
 struct KSplit { uint32_t b0, n0, b1, n1; };
