@@ -156,12 +156,12 @@ inline void dyb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   cfg.numAttrs = ctx->pdl && smem <= 96 * 1024 ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);   // a failure is picked up by DYB_LAUNCHED (cudaGetLastError)
 }
+// dyb_grid_dep_sync also lets the next kernel of the stream start now; after dyb_grid_dep_wait alone it starts when this one's CTAs end.
 // The branch behind the wait is never taken (no launch has that much shared memory).  It is what keeps the kernel's loads behind the
 // wait: a load through a const __restrict__ pointer, or __ldg, is free to move across an asm statement that does not name the
 // pointer, "memory" clobber or not, and did (a scale word was read before the kernel that computes it had written it); past a
 // branch that may end the thread a load whose address may not be valid stays where it is.
-__device__ __forceinline__ void dyb_grid_dep_sync() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__device__ __forceinline__ void dyb_grid_dep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t smem;
   asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(smem)::"memory");
@@ -169,6 +169,10 @@ __device__ __forceinline__ void dyb_grid_dep_sync() {
     asm volatile("exit;" ::: "memory");
     __builtin_unreachable();
   }
+}
+__device__ __forceinline__ void dyb_grid_dep_sync() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  dyb_grid_dep_wait();
 }
 // Raises a kernel's limit on dynamic shared memory to `most`, one value per kernel whatever the launch takes of it: the limit belongs to the
 // function, and a value per launch would let one thread lower it between another thread's call and launch.

@@ -7,7 +7,8 @@
 // 10000 x 1 x 1024 projection.  Here A is read once, as it lies, in fp32 with plain multiply-adds: a CTA owns 32 rows (the four
 // gates of 8 hidden units, or 32 consecutive rows), 8 lanes x 16 bytes cover them for one k, the other lanes and warps take
 // other k; two batches of eight 16-byte loads are in
-// flight per thread, the first of them before B is fetched.  B (all of its k, N columns) sits in shared memory as [k][column], so
+// flight per thread, the first of them before B is fetched.  Plain products of up to four columns share their rows out evenly over the SMs
+// instead (thin_launch).  B (all of its k, N columns) sits in shared memory as [k][column], so
 // that a thread gets the N factors of a k with 16-byte loads that the warp shares.  The partial sums of the k lanes meet by
 // shuffles, those of the warps in shared memory as a tree: the result does not depend on the run.
 // Up to 16 columns per CTA (64 sums per thread); beyond that a second column of CTAs reads A again (from L2).
@@ -26,7 +27,7 @@ struct ThinPair {
 struct ThinArgs {
   ThinPair p[2];
   int npairs, mode, pre_in_c;       // pre_in_c: (gates) C holds the rest of the pre-activation, bias included
-  uint32_t M, N;
+  uint32_t M, N, quads;             // quads: (up to kFlexColumns) groups of four rows per CTA
   float* C; uint32_t ldc;
   const float* bias; uint32_t H; float fb;
   const float* c_prev; float *c_out, *h_out;        // gates with the cell update (null: gates only)
@@ -107,23 +108,30 @@ __device__ __forceinline__ float4 thin_b(const ThinArgs& a, uint32_t kg, uint32_
   return make_float4(v[0] * m[0], v[1] * m[1], v[2] * m[2], v[3] * m[3]);
 }
 
+// Plain products of up to four columns: any number of row quads per CTA, so that one CTA per SM takes an equal share of the rows.
+constexpr uint32_t kFlexColumns = 4;
+
 // grid (row blocks, column blocks); 256 or 512 threads
 template <int NB, bool GATES, bool VEC>
 __global__ void __launch_bounds__(512, 1) k_gemm_thin(const __grid_constant__ ThinArgs a) {
   extern __shared__ __align__(16) float thin_smem[];
-  dyb_grid_dep_sync();
+  // No early launch of the dependent kernel: the CTAs of a following product would settle two and more on the SMs that this one leaves free
+  // and read their shares of the weights from there (a token of a 2-layer, 1024-unit generator: 40.4 us with it, 31.5 without).
+  dyb_grid_dep_wait();
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x / 32, n0 = blockIdx.y * NB;
   // row of the CTA's 32 that this thread's first value belongs to
-  const uint32_t r = VEC ? 4 * (tid & 7) : lane;
-  const uint32_t u = blockIdx.x * 8 + r % 8, m = GATES ? (r / 8) * a.H + u : blockIdx.x * kRows + r;
-  const bool row_live = GATES ? u < a.H : m < a.M;
+  constexpr bool FLEX = VEC && !GATES && NB <= kFlexColumns;
+  const uint32_t quads = FLEX ? a.quads : 8u, rows = FLEX ? 4 * quads : kRows;
+  const uint32_t r = VEC ? 4 * (FLEX ? tid % quads : tid & 7) : lane;
+  const uint32_t u = blockIdx.x * 8 + r % 8, m = GATES ? (r / 8) * a.H + u : blockIdx.x * rows + r;
   float acc[VEC ? 4 : 1][NB];
 #pragma unroll
   for (int i = 0; i < (VEC ? 4 : 1); ++i)
 #pragma unroll
     for (int c = 0; c < NB; ++c) acc[i][c] = 0.f;
   constexpr int IN = NB >= 16 && VEC ? 4 : 8;   // loads per batch; two batches are on their way at any time
-  const uint32_t sub = VEC ? tid / 8 : warp, step = VEC ? blockDim.x / 8 : warps;
+  const uint32_t sub = VEC ? tid / quads : warp, step = VEC ? blockDim.x / quads : warps;
+  const bool row_live = (GATES ? u < a.H : m < a.M) && sub < step;
   const uint32_t K0 = a.p[0].K, K = a.npairs > 1 ? K0 + a.p[1].K : K0;
   ThinCursor cur;
   auto pair_start = [&](int q) {
@@ -188,6 +196,40 @@ __global__ void __launch_bounds__(512, 1) k_gemm_thin(const __grid_constant__ Th
     next(w1, k1, e1);
   }
   if (k1 < e1) thin_fma<NB, IN, VEC>(w1, k1, e1, step, thin_smem, acc);
+  if (FLEX) {   // the k lanes of a warp by shuffles where its quads divide it, the rest in order, one thread per (column, row)
+    uint32_t parts = step, part = sub;
+    bool holds = sub < step;
+    if (32 % quads == 0) {
+      for (uint32_t d = quads; d < 32; d <<= 1)
+#pragma unroll
+        for (int i = 0; i < (VEC ? 4 : 1); ++i)
+#pragma unroll
+          for (int c = 0; c < NB; ++c) acc[i][c] += __shfl_xor_sync(0xffffffffu, acc[i][c], d);
+      parts = warps; part = warp; holds = lane < quads;
+    }
+    __syncthreads();
+    float* red = thin_smem;   // [column][row][parts, odd pitch]
+    const uint32_t rp = parts | 1;
+    if (holds) {
+#pragma unroll
+      for (int c = 0; c < NB; ++c)
+#pragma unroll
+        for (int i = 0; i < (VEC ? 4 : 1); ++i) red[(size_t)(c * rows + r + i) * rp + part] = acc[i][c];
+    }
+    __syncthreads();
+    for (uint32_t e = tid; e < rows * NB; e += blockDim.x) {
+      const uint32_t mm = blockIdx.x * rows + e % rows, n = n0 + e / rows;
+      if (mm >= a.M || n >= a.N) continue;
+      float v = 0.f;
+#pragma unroll 8
+      for (uint32_t k = 0; k < parts; ++k) v += red[(size_t)e * rp + k];
+      float* dst = a.C + mm + (size_t)a.ldc * n;
+      if (a.mode == EPI_BIAS) v += a.bias[mm];
+      else if (a.mode == EPI_ACCUM) v += *dst;
+      *dst = v;
+    }
+    return;
+  }
   // the k lanes of a warp (VEC: lanes 8 j + s hold rows 4 s .. 4 s + 3), then the warps in order
   if (VEC) {
 #pragma unroll
@@ -275,9 +317,26 @@ int thin_launch(dyb200_ctx* ctx, ThinArgs& a, bool gates, double flops) {
                  (!a.p[q].mask || (aligned16(a.p[q].mask) && (!a.p[q].mask_full || a.p[q].mask_ld % 4 == 0)));
     ktot += a.p[q].K;
   }
-  const uint32_t blocks = gates ? (a.H + 7) / 8 : (a.M + kRows - 1) / kRows;
-  const uint32_t threads = blocks <= (uint32_t)ctx->sm_count ? 512u : 256u;   // (one CTA per SM: more loads in flight from it)
-  const size_t xs = (size_t)(ktot + 3) / 4 * 4 * nb * 4, red = (size_t)(threads / 32 + 1) * nb * kRows * 4;
+  uint32_t blocks = gates ? (a.H + 7) / 8 : (a.M + kRows - 1) / kRows;
+  uint32_t threads = blocks <= (uint32_t)ctx->sm_count ? 512u : 256u;   // (one CTA per SM: more loads in flight from it)
+  size_t red = (size_t)(threads / 32 + 1) * nb * kRows * 4;
+  if (vec && !gates && nb <= kFlexColumns) {
+    // One CTA of 512 threads per SM with up to 32 quads of rows, at least 32 bytes of a column; more rows in whole rounds of two CTAs per
+    // SM.  (us for 1 / 4 columns, against CTAs of 32 rows whatever the number of rows: 10000 x 1024 10.2 / 12.1 against 12.3 / 17.3 in
+    // 313 CTAs, 50000 x 128 8.3 / 10.5 against 13.7 / 20.7, 1024 x 4096 6.4 / 9.9 against 10.2 / 15.5 in 32 CTAs.)
+    const uint32_t sms = (uint32_t)ctx->sm_count, all = a.M / 4;
+    a.quads = (all + sms - 1) / sms;
+    threads = 512;
+    if (a.quads <= 8) a.quads = a.quads <= 2 ? 2 : a.quads <= 4 ? 4 : 8;   // (so that shuffles add up a warp's k lanes)
+    if (a.quads > 32) {
+      threads = 256;
+      const uint32_t rounds = (all + 64 * sms - 1) / (64 * sms);
+      a.quads = (all + 2 * sms * rounds - 1) / (2 * sms * rounds);
+    }
+    blocks = (all + a.quads - 1) / a.quads;
+    red = (size_t)((threads / a.quads) | 1) * nb * 4 * a.quads * 4;
+  }
+  const size_t xs = (size_t)(ktot + 3) / 4 * 4 * nb * 4;
   const size_t smem = xs > red ? xs : red;
   void (*k)(ThinArgs) = gates ? (vec ? thin_kernel<true, true>(nb) : thin_kernel<true, false>(nb))
                               : (vec ? thin_kernel<false, true>(nb) : thin_kernel<false, false>(nb));

@@ -122,3 +122,22 @@ def test_product_onto_its_own_operand(g, n, cols):
         reps.append(C)
     assert all(torch.equal(r, reps[0]) for r in reps)
     assert float((reps[0].double() - want).abs().max()) <= TOL_REDUCE * n ** 0.5
+
+
+@pytest.mark.parametrize("M,K", [(4, 3), (1184, 257), (1188, 513), (4736, 65), (4740, 301), (18944, 41), (18948, 67), (49996, 33), (100000, 20)])
+@pytest.mark.parametrize("N", [1, 3, 4])
+def test_thin_row_shares(g, M, K, N):
+    """Plain products of up to four columns at the edges of the row shares (2, 4, 8, 9, 32 quads of rows per CTA on 148 SMs, then rounds of
+    smaller CTAs), reductions shorter than the k lanes."""
+    import torch
+    gen = torch.Generator("cuda").manual_seed(M + N)
+    A, B, C = torch.randn(K, M, device="cuda", generator=gen), torch.randn(N, K, device="cuda", generator=gen), torch.randn(N, M, device="cuda", generator=gen)
+    want = B.double() @ A.double()
+    for accumulate in (0, 1):
+        C0 = C.double() if accumulate else 0.0
+        got = C.clone()
+        g.ctx().gemm(0, 0, M, N, K, A.data_ptr(), M, B.data_ptr(), K, got.data_ptr(), M, accumulate)
+        # an fp32 sum of K products, each rounded at the size of the partial sum: below K 2^-24 of |row| |column|, and the last rounding
+        bar = (K + 2) * 2.0 ** -24 * (B.double().norm(dim=1)[:, None] * A.double().norm(dim=0)[None, :] + (C.double().abs() if accumulate else 0.0))
+        assert bool(((got.double() - want - C0).abs() <= bar).all())
+    assert g.ctx().device_errors() == 0
