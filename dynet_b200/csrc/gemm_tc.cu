@@ -1655,7 +1655,8 @@ int dyb200_wgrad_create(dyb200_ctx* ctx, uint32_t M, uint32_t N0, uint32_t N1, u
     for (int q = 0; q < 3 && ok; ++q) {
       if (!ps[q]->hi) continue;
       const size_t bytes = (size_t)ps[q]->pitch * w->Kcap * sizeof(float);
-      ok = cudaMemset(ps[q]->hi, 0, bytes) == cudaSuccess && cudaMemset(ps[q]->lo, 0, bytes) == cudaSuccess;
+      // (on the context's stream: the legacy default stream's clear could land on planes that a non-blocking stream had filled by then)
+      ok = cudaMemsetAsync(ps[q]->hi, 0, bytes, ctx->stream) == cudaSuccess && cudaMemsetAsync(ps[q]->lo, 0, bytes, ctx->stream) == cudaSuccess;
     }
     if (!ok) cudaGetLastError();
   }
