@@ -135,18 +135,21 @@ struct PackedOp {
 // positions are rows of an MN-major operand).  A matrix that is read both ways needs both sets of planes: with one scale for all of
 // it, rows 2^28 below its largest value would lose their bits.
 enum F16Scale { F16_LINE = 0, F16_ELEM = 1 };
-struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; };
-struct F16Jobs { F16Job job[2]; int n; };
-// Planes and scale words for a job from the scratch arena; dyb200_f16_pack fills those of up to two jobs in one pass each.
+// src_lo: the source is a pair of TF32 planes, src the hi one (null: plain fp32).
+constexpr int kF16MaxJobs = 3;
+struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; const float* src_lo = nullptr; };
+struct F16Jobs { F16Job job[kF16MaxJobs]; int n; uint32_t start[kF16MaxJobs + 1]; };   // start: units of work before each job (set for a launch)
+// Planes and scale words for a job from the scratch arena; dyb200_f16_pack fills those of up to three jobs in one pass each.
 int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
-int dyb200_f16_absmax(dyb200_ctx* ctx, const F16Jobs& jobs);       // the scale words alone
 // The same for a parameter, from the parameter cache when it is on.
 int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
-// Products from here on (useful flops) use fp16 pairs.  Finding the scales adds a clear and a pass over the operands: 8.6 GFLOP
-// (512 x 4096 x 2048) took 86 us that way and 70 us with TF32 pairs, 46 GFLOP (10000 x 2240 x 1024) 205 against 255 us.
-constexpr double kF16Flops = 24.0e9;
+// Products that use fp16 pairs, by useful flops.  Finding the scales adds a clear and a pass over the operands; us with TF32 / fp16 pairs,
+// splitting included: 1500^3 (6.8 GFLOP) 43 / 45, 1024 x 256 x 13000 (6.8) 77 / 75, 2000 x 2000 x 1000 (8.0) 50 / 39, 4096 x 512 x 2240 (9.4)
+// 74 / 68, 10000 x 512 x 1024 (10.5) 89 / 74, 2048^3 (17) 96 / 61, 10000 x 1024 x 1120 (23) 192 / 99.  A short reduction is bound by its result
+// either way (1024 x 107000 x 128, 28 GFLOP: 200 / 217); from 24 GFLOP on it takes the pairs for their smaller error.
+inline bool dyb200_f16_takes(double flops, uint32_t K) { return flops >= 24.0e9 || (flops >= 8.0e9 && K >= 256); }
 // A queue of packing work that one kernel launch executes (several small operands per launch).
 constexpr int kMaxPackJobs = 8;
 constexpr int kLayoutGates = 2, kLayoutF16 = 3;   // (kLayoutF16 + F16_LINE or F16_ELEM)

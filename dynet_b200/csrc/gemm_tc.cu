@@ -725,60 +725,137 @@ __global__ void __launch_bounds__(256) k_pack_multi(const PackJobs jobs) {
 // ---- fp16 operand planes: the largest |x| per line, per position or in all, then the split ---------------------------------
 // Both passes read the source once; a line of a wide operand is shared by several CTAs, maxima meet by atomicMax on the bit
 // patterns (the same from run to run).  Infinities and NaNs do not count: they come through the split as they are.
-constexpr uint32_t kMaxLines = 32;   // lines per unit of work where positions have their own scale
+// A unit of work is one CTA's; the 16-byte loads of a batch are requested together (behind a branch per load they went out one by one:
+// 219 instead of 122 us for the scales of 50000 x 4096, 433 instead of 282 us for its split).
+constexpr uint32_t kMaxLines = 64;      // F16_ELEM: lines of each thread
+constexpr uint32_t kWarpLine = 2048;    // F16_LINE: lines up to this length are a warp's, kWarpLines of them; longer ones go in pieces of kPiece
+constexpr uint32_t kWarpLines = 4, kPiece = 8192;
+struct F16Units { uint32_t groups, x, total; };   // F16_ELEM: groups of threads with lines of their own, units along the line
+__host__ __device__ __forceinline__ F16Units f16_max_units(const F16Job& j) {
+  F16Units u;
+  u.groups = 1; u.x = 1;
+  if (j.mode == F16_ELEM) {
+    const uint32_t q = (j.n + 3) / 4;
+    u.groups = q < 256 ? 256 / q : 1;
+    u.x = (q + 255) / 256;
+    u.total = u.x * ((j.lines + kMaxLines * u.groups - 1) / (kMaxLines * u.groups));
+  } else if (j.n <= kWarpLine) {
+    u.total = (j.lines + 8 * kWarpLines - 1) / (8 * kWarpLines);
+  } else {
+    u.x = (j.n + kPiece - 1) / kPiece;
+    u.total = u.x * j.lines;
+  }
+  return u;
+}
+__device__ __forceinline__ uint32_t f16_job_of(const F16Jobs& jobs) {
+  uint32_t z = 0;
+#pragma unroll
+  for (int q = 1; q < kF16MaxJobs; ++q) if (q < jobs.n && blockIdx.x >= jobs.start[q]) z = q;
+  return z;
+}
 __device__ __forceinline__ uint32_t mag4(float4 v) { return max(max(finite_mag(v.x), finite_mag(v.y)), max(finite_mag(v.z), finite_mag(v.w))); }
-__global__ void __launch_bounds__(256) k_f16_absmax(const F16Jobs jobs) {
+// elements [e, e + 4) of a line of n (zeros past its end)
+__device__ __forceinline__ float4 f16_load4(const float* line, uint32_t e, uint32_t n, bool vec) {
+  if (vec && e + 4 <= n) return ld4(line + e);
+  float v[4];
+#pragma unroll
+  for (uint32_t i = 0; i < 4; ++i) v[i] = e + i < n ? line[e + i] : 0.f;
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+__global__ void __launch_bounds__(256) k_f16_absmax(const __grid_constant__ F16Jobs jobs) {
   dyb_grid_dep_sync();
-  const F16Job& j = jobs.job[blockIdx.z];
+  const uint32_t z = f16_job_of(jobs), unit = blockIdx.x - jobs.start[z];
+  const F16Job& j = jobs.job[z];
   const bool vec = (j.ld & 3) == 0 && aligned16(j.src);
-  if (j.mode == F16_ELEM) {   // a unit is 1024 positions of kMaxLines lines, four positions per thread
-    const uint32_t xb = (j.n + 1023) / 1024, yb = (j.lines + kMaxLines - 1) / kMaxLines;
-    for (uint32_t u = blockIdx.x; u < xb * yb; u += gridDim.x) {
-      const uint32_t e = 4 * ((u % xb) * 256 + threadIdx.x), l0 = u / xb * kMaxLines;
-      if (e >= j.n) continue;
-      uint32_t m[4] = {0, 0, 0, 0};
-#pragma unroll 8
-      for (uint32_t l = l0; l < min(l0 + kMaxLines, j.lines); ++l) {
-        const float* p = j.src + (size_t)j.ld * l + e;
-        if (vec && e + 4 <= j.n) {
-          const float4 v = ld4(p);
-          m[0] = max(m[0], finite_mag(v.x)); m[1] = max(m[1], finite_mag(v.y)); m[2] = max(m[2], finite_mag(v.z)); m[3] = max(m[3], finite_mag(v.w));
+  const F16Units us = f16_max_units(j);
+  if (j.mode == F16_ELEM) {   // four positions per thread; short lines: groups of threads take every groups-th line and meet in shared memory
+    __shared__ uint32_t top[1024];
+    const uint32_t q = us.groups > 1 ? (j.n + 3) / 4 : 256u, grp = threadIdx.x / q, e = 4 * ((unit % us.x) * 256 + threadIdx.x % q);
+    const uint32_t l0 = unit / us.x * kMaxLines * us.groups + grp;
+    const bool live = grp < us.groups && e < j.n;
+    uint32_t m[4] = {0, 0, 0, 0};
+    if (live) {
+      for (uint32_t b = 0; b < kMaxLines && l0 + b * us.groups < j.lines; b += 8) {
+        float4 v[8];
+        const uint32_t l = l0 + b * us.groups;
+        const float* p = j.src + (size_t)j.ld * l;
+        const size_t next = (size_t)j.ld * us.groups;
+        if (vec && e + 4 <= j.n && l + 7 * us.groups < j.lines) {
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) v[k] = ld4(p + k * next + e);
         } else {
 #pragma unroll
-          for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) m[i] = max(m[i], finite_mag(p[i]));
+          for (uint32_t k = 0; k < 8; ++k) v[k] = l + k * us.groups < j.lines ? f16_load4(p + k * next, e, j.n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+          m[0] = max(m[0], finite_mag(v[k].x)); m[1] = max(m[1], finite_mag(v[k].y)); m[2] = max(m[2], finite_mag(v[k].z)); m[3] = max(m[3], finite_mag(v[k].w));
         }
       }
+    }
+    if (us.groups > 1) {
+      for (uint32_t i = threadIdx.x; i < 1024; i += 256) top[i] = 0;
+      __syncthreads();
+      if (live) {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) atomicMax(top + e + i, m[i]);
+      }
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < j.n; i += 256) atomicMax(j.scale + i, top[i]);
+    } else if (live) {
 #pragma unroll
       for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) atomicMax(j.scale + e + i, m[i]);
     }
     return;
   }
-  __shared__ uint32_t red[8];
-  const uint32_t piece = 4096, pieces = (j.n + piece - 1) / piece;
-  const uint64_t units = (uint64_t)pieces * j.lines;
-  for (uint64_t u = blockIdx.x; u < units; u += gridDim.x) {
-    const uint32_t line = (uint32_t)(u / pieces), lo = (uint32_t)(u % pieces) * piece, hi = min(j.n, lo + piece);
-    const float* p = j.src + (size_t)j.ld * line;
-    uint32_t m = 0;
-    if (vec) {
-#pragma unroll 4
-      for (uint32_t e = lo + 4 * threadIdx.x; e < hi; e += 1024) {
-        if (e + 4 <= hi) m = max(m, mag4(ld4(p + e)));
-        else for (uint32_t i = e; i < hi; ++i) m = max(m, finite_mag(p[i]));
-      }
-    } else {
-#pragma unroll 4
-      for (uint32_t e = lo + threadIdx.x; e < hi; e += 256) m = max(m, finite_mag(p[e]));
-    }
-    m = __reduce_max_sync(0xffffffffu, m);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+  if (j.n <= kWarpLine) {
+    const uint32_t lane = threadIdx.x & 31, l0 = (unit * 8 + (threadIdx.x >> 5)) * kWarpLines;
+    uint32_t m[kWarpLines] = {0, 0, 0, 0};
+    for (uint32_t e = 4 * lane; e < j.n; e += 256) {
+      float4 v[kWarpLines][2];
+      if (vec && e + 132 <= j.n && l0 + kWarpLines <= j.lines) {
 #pragma unroll
-      for (int w = 1; w < 8; ++w) m = max(m, red[w]);
-      if (pieces == 1) j.scale[line] = m; else atomicMax(j.scale + line, m);
+        for (uint32_t k = 0; k < kWarpLines; ++k)
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h) v[k][h] = ld4(j.src + (size_t)j.ld * (l0 + k) + e + 128 * h);
+      } else {
+#pragma unroll
+        for (uint32_t k = 0; k < kWarpLines; ++k)
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h)
+            v[k][h] = l0 + k < j.lines ? f16_load4(j.src + (size_t)j.ld * (l0 + k), e + 128 * h, j.n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kWarpLines; ++k) m[k] = max(m[k], max(mag4(v[k][0]), mag4(v[k][1])));
     }
+#pragma unroll
+    for (uint32_t k = 0; k < kWarpLines; ++k) {
+      m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+      if (lane == 0 && l0 + k < j.lines) j.scale[l0 + k] = m[k];
+    }
+    return;
+  }
+  __shared__ uint32_t red[8];
+  const uint32_t line = unit / us.x, e0 = unit % us.x * kPiece + 4 * threadIdx.x;
+  float4 v[8];
+  const float* p = j.src + (size_t)j.ld * line;
+  if (vec && e0 + 7 * 1024 + 4 <= j.n) {
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) v[k] = ld4(p + e0 + 1024 * k);
+  } else {
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) v[k] = f16_load4(p, e0 + 1024 * k, j.n, vec);
+  }
+  uint32_t m = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 8; ++k) m = max(m, mag4(v[k]));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) m = max(m, red[w]);
+    if (us.x == 1) j.scale[line] = m; else atomicMax(j.scale + line, m);
   }
 }
 __device__ __forceinline__ void split4_f16(float4 v, float4 s, uint2& hi, uint2& lo) {
@@ -787,32 +864,64 @@ __device__ __forceinline__ void split4_f16(float4 v, float4 s, uint2& hi, uint2&
   hi = *reinterpret_cast<const uint2*>(h);
   lo = *reinterpret_cast<const uint2*>(l);
 }
-__global__ void __launch_bounds__(256) k_f16_split(const F16Jobs jobs) {
+// A unit: kSplitItems items of four values, the lines end to end.  (A pair of planes is added up, hi + lo: the fp32 value that it stands for.)
+constexpr uint32_t kSplitItems = 1024;
+__global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jobs jobs) {
   dyb_grid_dep_sync();
-  const F16Job& j = jobs.job[blockIdx.z];
-  const bool vec = (j.ld & 3) == 0 && aligned16(j.src);
-  const uint32_t q = (j.n + 3) / 4;   // items of four values per line
-  const uint64_t items = (uint64_t)q * j.lines;
-  for (uint64_t it = (uint64_t)blockIdx.x * 256 + threadIdx.x; it < items; it += (uint64_t)gridDim.x * 256) {
-    const uint32_t line = (uint32_t)(it / q), e = 4 * (uint32_t)(it % q);
-    const float* p = j.src + (size_t)j.ld * line + e;
-    float v[4] = {0.f, 0.f, 0.f, 0.f}, s[4];
-    if (vec && e + 4 <= j.n) { const float4 x = ld4(p); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
-    else {
+  const uint32_t z = f16_job_of(jobs), unit = blockIdx.x - jobs.start[z];
+  const F16Job& j = jobs.job[z];
+  const bool vec = (j.ld & 3) == 0 && aligned16(j.src) && (!j.src_lo || aligned16(j.src_lo));
+  const uint32_t q = (j.n + 3) / 4;
+  const uint64_t first = (uint64_t)unit * kSplitItems;
+  const uint32_t line0 = (uint32_t)(first / q), rem = (uint32_t)(first - (uint64_t)line0 * q);
+  float4 v[4];
+  uint32_t line[4], e[4];
 #pragma unroll
-      for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) v[i] = p[i];
-    }
-    if (j.mode == F16_ELEM) {
+  for (uint32_t k = 0; k < 4; ++k) {
+    const uint32_t it = rem + 256 * k + threadIdx.x;
+    line[k] = line0 + it / q; e[k] = 4 * (it % q);
+  }
+  // (the last item is the furthest in the source; lines that are whole quads: one straight set of loads)
+  const bool plain = vec && (j.n & 3) == 0 && line[3] < j.lines;
+  if (plain) {
 #pragma unroll
-      for (uint32_t i = 0; i < 4; ++i) s[i] = scale_of(__ldg(j.scale + min(e + i, j.n - 1)));
+    for (uint32_t k = 0; k < 4; ++k) v[k] = ld4(j.src + (size_t)j.ld * line[k] + e[k]);
+  } else {
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) v[k] = line[k] < j.lines ? f16_load4(j.src + (size_t)j.ld * line[k], e[k], j.n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (j.src_lo) {
+    float4 w[4];
+    if (plain) {
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) w[k] = ld4(j.src_lo + (size_t)j.ld * line[k] + e[k]);
     } else {
-      s[0] = s[1] = s[2] = s[3] = scale_of(__ldg(j.scale + line));
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) w[k] = line[k] < j.lines ? f16_load4(j.src_lo + (size_t)j.ld * line[k], e[k], j.n, vec) : v[k];
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) v[k] = make_float4(v[k].x + w[k].x, v[k].y + w[k].y, v[k].z + w[k].z, v[k].w + w[k].w);
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) {
+    if (line[k] >= j.lines) break;
+    float4 s;
+    if (j.mode == F16_ELEM) {
+      const uint32_t top = j.n - 1;
+      if (e[k] + 4 <= j.n) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(j.scale + e[k]));
+        s = make_float4(scale_of(w.x), scale_of(w.y), scale_of(w.z), scale_of(w.w));
+      } else {
+        s = make_float4(scale_of(__ldg(j.scale + min(e[k], top))), scale_of(__ldg(j.scale + min(e[k] + 1, top))), scale_of(__ldg(j.scale + min(e[k] + 2, top))), 1.f);
+      }
+    } else {
+      s.x = s.y = s.z = s.w = scale_of(__ldg(j.scale + line[k]));
     }
     uint2 hi, lo;
-    split4_f16(make_float4(v[0], v[1], v[2], v[3]), make_float4(s[0], s[1], s[2], s[3]), hi, lo);
+    split4_f16(v[k], s, hi, lo);
     // (the pitch is a multiple of 64: the last item's padding stays inside the line's pitch)
-    *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line + e) = hi;
-    *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line + e) = lo;
+    *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line[k] + e[k]) = hi;
+    *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line[k] + e[k]) = lo;
   }
 }
 
@@ -975,28 +1084,25 @@ int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t l
   *job = F16Job{src, ld, lines, n, pitch, mode, (uint32_t*)sc, (__half*)h, (__half*)l};
   return DYB200_OK;
 }
-int dyb200_f16_absmax(dyb200_ctx* ctx, const F16Jobs& jobs) {
-  uint32_t gx = 1;
-  for (int k = 0; k < jobs.n; ++k) {
-    const F16Job& j = jobs.job[k];
-    const bool one_store = j.mode == F16_LINE && j.n <= 4096;   // (every word is written once, no maximum to start from)
-    const size_t words = j.mode == F16_LINE ? j.lines : j.mode == F16_ELEM ? j.n : 1;
-    if (!one_store) DYB_CUDA(ctx, cudaMemsetAsync(j.scale, 0, words * sizeof(uint32_t), ctx->stream));
-    uint64_t x = j.mode == F16_ELEM ? (uint64_t)((j.n + 1023) / 1024) * ((j.lines + kMaxLines - 1) / kMaxLines) : (uint64_t)((j.n + 4095) / 4096) * j.lines;
-    if (x > 8ull * ctx->sm_count) x = 8ull * ctx->sm_count;
-    if (x > gx) gx = (uint32_t)x;
-  }
-  dyb_launch(k_f16_absmax, dim3(gx, 1, jobs.n), 256, 0, ctx, jobs);
-  DYB_LAUNCHED(ctx);
-  return DYB200_OK;
-}
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
   if (jobs->n == 0) return DYB200_OK;
-  int rc = dyb200_f16_absmax(ctx, *jobs);
-  if (rc) return rc;
-  uint64_t most = 0;
-  for (int k = 0; k < jobs->n; ++k) { const uint64_t it = (uint64_t)((jobs->job[k].n + 3) / 4) * jobs->job[k].lines; if (it > most) most = it; }
-  dyb_launch(k_f16_split, dim3(stream_grid(ctx, most, 256, 16), 1, jobs->n), 256, 0, ctx, *jobs);
+  jobs->start[0] = 0;
+  for (int k = 0; k < jobs->n; ++k) {
+    const F16Job& j = jobs->job[k];
+    const bool one_store = j.mode == F16_LINE && j.n <= kPiece;   // (every word is written once, no maximum to start from)
+    if (!one_store) DYB_CUDA(ctx, cudaMemsetAsync(j.scale, 0, (j.mode == F16_LINE ? j.lines : j.n) * sizeof(uint32_t), ctx->stream));
+    const uint64_t end = (uint64_t)jobs->start[k] + f16_max_units(j).total;
+    DYB_CHECK_ARG(ctx, end < 0x7fffffffull, "fp16 planes: operand too large (%u x %u)", j.lines, j.n);
+    jobs->start[k + 1] = (uint32_t)end;
+  }
+  dyb_launch(k_f16_absmax, jobs->start[jobs->n], 256, 0, ctx, *jobs);
+  DYB_LAUNCHED(ctx);
+  for (int k = 0; k < jobs->n; ++k) {
+    const uint64_t end = jobs->start[k] + ((uint64_t)((jobs->job[k].n + 3) / 4) * jobs->job[k].lines + kSplitItems - 1) / kSplitItems;
+    DYB_CHECK_ARG(ctx, end < 0x7fffffffull, "fp16 planes: operand too large (%u x %u)", jobs->job[k].lines, jobs->job[k].n);
+    jobs->start[k + 1] = (uint32_t)end;
+  }
+  dyb_launch(k_f16_split, jobs->start[jobs->n], 256, 0, ctx, *jobs);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
@@ -1410,7 +1516,7 @@ int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const Ge
   for (int p = 0; p < npairs; ++p) if (pairs[p].K == 0) return DYB200_OK;
   *handled = 1;
   PackedOp A[2], B[2];
-  if (npairs == 1 && !pairs[0].maskB && flops >= kF16Flops) {
+  if (npairs == 1 && !pairs[0].maskB && dyb200_f16_takes(flops, pairs[0].K)) {
     // Both operands as they lie: lines are rows of a K-major operand (A transposed / B not), or k of an MN-major one.
     const GemmPair& g = pairs[0];
     const bool a_mn = g.transA == 0, b_mn = g.transB != 0;

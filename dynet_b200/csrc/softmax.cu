@@ -974,7 +974,7 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
   }
   int rc;
   PackedOp dA, dB, hT, RT;
-  const bool f16 = flops >= kF16Flops;   // fp16 pairs, as for the single products
+  const bool f16 = dyb200_f16_takes(flops, n < V ? n : V);   // fp16 pairs, as for the single products
   const dim3 grid((V + 63) / 64, (n + 63) / 64);
   DYB_CHECK_ARG(ctx, grid.y <= 65535u, "softmax_output_bwd_fused: too many columns (%u)", n);
   void* part;
