@@ -1588,6 +1588,15 @@ struct dyb200_wgrad {
   // of that sequence (0: varying).
   uint32_t x_cols, h_col, step;
 };
+// Whether the flush makes fp16 pairs of the TF32 planes first: 16 bytes moved per value (a pass for the scales over the hi planes, one
+// that reads both planes and writes the pairs) against products at 490 instead of 190 TFLOP/s, so it is the multiply-adds per
+// value, M N / (M + N), that decide.  us with TF32 / fp16 pairs: 4096 x (1024 + 1024), K = 17920 1285 / 887, K = 2240 243 / 144, K = 560
+// 112 / 71; 4096 x (512 + 1024) x 2240 185 / 134; 2048 x (512 + 512) (683 per value) x 4480 120 / 123; 1024 x (128 + 256) (279) x 107000
+// 536 / 664.  The error is no larger (max / rms of |row| |column|, 4096 x 1024 x 17920: 9.5e-8 / 1.4e-8 and 9.2e-8 / 1.1e-8).
+static bool wgrad_on_f16(const dyb200_wgrad* w) {
+  const double N = (double)w->N[0] + w->N[1];
+  return w->k >= 256 && w->M * N >= 800.0 * (w->M + N);
+}
 // natural pack of the k columns [col, col + k) of operand j (b is N[j] x k column-major; the mask is indexed like b)
 static int pack_b_rows(dyb200_ctx* ctx, dyb200_wgrad* w, int j, uint32_t col, uint32_t k, const float* b, uint32_t ldb, const float* mask,
                        int mask_full, PackJobs* batch) {
@@ -1824,12 +1833,24 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
   w->x_cols = 0; w->h_col = 0xffffffffu;
   if (w->k == 0) { w->kb = 0; return DYB200_OK; }
   DYB_CHECK_ARG(ctx, kb_seen >= w->k, "wgrad_flush: the B operands cover %u columns, the A operand %u", kb_seen, w->k);
-  PackedOp A = w->A;
-  A.K = w->k;
+  PackedOp ops[3] = {w->A, w->B[0], w->B[1]};   // (MN-major: one plane row per column)
+  for (PackedOp& o : ops) o.K = w->k;
+  if (wgrad_on_f16(w)) {
+    F16Jobs jobs;
+    jobs.n = w->N[1] ? 3 : 2;
+    for (int q = 0; q < jobs.n; ++q) {
+      int rc = dyb200_f16_planes(ctx, ops[q].hi, ops[q].pitch, w->k, ops[q].rows, F16_ELEM, &jobs.job[q]);
+      if (rc) return rc;
+      jobs.job[q].src_lo = ops[q].lo;
+    }
+    int rc = dyb200_f16_pack(ctx, &jobs);
+    if (rc) return rc;
+    for (int q = 0; q < jobs.n; ++q) ops[q] = dyb200_f16_op(jobs.job[q], true);
+  }
+  const PackedOp& A = ops[0];
   for (int j = 0; j < 2; ++j) {
     if (w->N[j] == 0) continue;
-    PackedOp B = w->B[j];   // (MN-major: rows = N[j], one plane row per column)
-    B.K = w->k;
+    const PackedOp& B = ops[1 + j];
     GemmEpilogue e{EPI_ACCUM, j == 0 ? C0 : C1, j == 0 ? ldc0 : ldc1, nullptr, 0, 0.f, nullptr, 0, 0};
     int rc = dyb200_tc_gemm_packed(ctx, w->M, w->N[j], 1, &A, &B, e);
     if (rc) return rc;
