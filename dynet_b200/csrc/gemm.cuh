@@ -80,6 +80,7 @@ __device__ __forceinline__ uint32_t finite_mag(float v) {
   return u < 0x7f800000u ? u : 0u;
 }
 __device__ __forceinline__ float scale_of(uint32_t word) { return __int_as_float((268 - scale_field(word)) << 23); }
+__device__ __forceinline__ float inv_scale_of(uint32_t word) { return __int_as_float((scale_field(word) - 14) << 23); }   // 2^(E - 141)
 // v 2^(Ea + Eb - 282): in two factors, so that nothing overflows on the way to a result that does not
 __device__ __forceinline__ float unscale(float v, int t) {
   const int h = t >> 1;
@@ -137,7 +138,8 @@ struct PackedOp {
 enum F16Scale { F16_LINE = 0, F16_ELEM = 1 };
 // src_lo: the source is a pair of TF32 planes, src the hi one (null: plain fp32).
 constexpr int kF16MaxJobs = 3;
-struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; const float* src_lo = nullptr; };
+struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; const float* src_lo = nullptr;
+  uint32_t perm_H = 0; };   // perm_H (F16_ELEM): positions are gate rows q perm_H + u, written interleaved as dyb200_tc_param_gates does
 struct F16Jobs { F16Job job[kF16MaxJobs]; int n; uint32_t start[kF16MaxJobs + 1]; };   // start: units of work before each job (set for a launch)
 // Planes and scale words for a job from the scratch arena; dyb200_f16_pack fills those of up to three jobs in one pass each.
 int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
@@ -145,6 +147,10 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
 // The same for a parameter, from the parameter cache when it is on.
 int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
+// The gate weights of a layer, Wx (4H x I) and Wh (4H x H), as MN-major planes with interleaved rows (lines = their columns, pitch 4H) and one
+// scale word per row of [Wx Wh] (not interleaved); from the parameter cache when it is on.
+struct F16Gates { __half *x_hi, *x_lo, *h_hi, *h_lo; const uint32_t* scale; };
+int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, F16Gates* out);
 // Products that use fp16 pairs, by useful flops.  Finding the scales adds a clear and a pass over the operands; us with TF32 / fp16 pairs,
 // splitting included: 1500^3 (6.8 GFLOP) 43 / 45, 1024 x 256 x 13000 (6.8) 77 / 75, 2000 x 2000 x 1000 (8.0) 50 / 39, 4096 x 512 x 2240 (9.4)
 // 74 / 68, 10000 x 512 x 1024 (10.5) 89 / 74, 2048^3 (17) 96 / 61, 10000 x 1024 x 1120 (23) 192 / 99.  A short reduction is bound by its result
@@ -152,7 +158,7 @@ PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
 inline bool dyb200_f16_takes(double flops, uint32_t K) { return flops >= 24.0e9 || (flops >= 8.0e9 && K >= 256); }
 // A queue of packing work that one kernel launch executes (several small operands per launch).
 constexpr int kMaxPackJobs = 8;
-constexpr int kLayoutGates = 2, kLayoutF16 = 3;   // (kLayoutF16 + F16_LINE or F16_ELEM)
+constexpr int kLayoutGates = 2, kLayoutF16 = 3, kLayoutGatesF16 = 5;   // (kLayoutF16 + F16_LINE or F16_ELEM)
 struct PackJob {
   const float* src; const float* mask; float* hi; float* lo;
   uint32_t ld, rows, K, mask_ld, pitch, gx, perm_H;
@@ -228,8 +234,23 @@ void dyb200_wgrad_seq_done(dyb200_wgrad* w);
 // False when X is asked for and the inputs of that many columns are not in place.  dyb200_wgrad_h_done: all Hs rows are written.
 bool dyb200_wgrad_column_planes(const dyb200_wgrad* w, uint32_t columns, PackedOp* D, PackedOp* X, PackedOp* Hs);
 void dyb200_wgrad_h_done(dyb200_wgrad* w);
+// The planes of columns [col, col + k) of both right operands, filled or to be filled.
+bool dyb200_wgrad_b_planes(const dyb200_wgrad* w, uint32_t col, uint32_t k, PackedOp* X, PackedOp* Hs);
+// The forward product of a layer on fp16 pairs (lstm_seq.cu): T steps of B columns, or a single one driven from outside - the same kernel, so
+// the same bits.  Whether a shape takes it, with its tile width and K splits; the call, whose inputs are planes of the accumulator.
+bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* bn, uint32_t* S);
+struct SeqF16Call {
+  uint32_t I, H, B, T;
+  const float *Wx, *Wh, *b, *h0, *c0, *mh; int mh_full; float forget_bias;
+  float *gates, *c, *h;
+  PackedOp X, Hs;          // TF32 planes of the columns' inputs; rows [0, B) of Hs are filled here unless h0_done, the later ones by the kernel
+  int h0_done, emit_last;  // emit_last: rows [T B, (T + 1) B) of Hs receive the last step's h
+};
+int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q);
 // A 2-D tensor map (CUtensorMap, 128 bytes at `map`) over a K-major plane: box = 32 floats of K x box_rows rows, 128-byte swizzle.
 int dyb200_tc_make_tmap(dyb200_ctx* ctx, void* map, float* plane, uint32_t rows, uint32_t K, uint32_t pitch, uint32_t box_rows);
+// The same over a plane of halves (64 of K), and over an MN-major one (K lines of `rows` halves).
+int dyb200_tc_make_tmap_f16(dyb200_ctx* ctx, void* map, __half* plane, uint32_t rows, uint32_t K, uint32_t pitch, uint32_t box_rows, bool mn_major);
 // A 3-D tensor map over S matrices side by side (M x N each, leading dimension ldc, 16-byte aligned): box = 128 rows x box_cols columns.
 int dyb200_tc_make_store_map(dyb200_ctx* ctx, void* map, float* C, uint32_t M, uint32_t N, uint32_t S, uint32_t ldc, uint32_t box_cols);
 // Products of fp16 pairs on pairs of SMs (gemm_pair.cu).

@@ -919,6 +919,7 @@ __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jo
     }
     uint2 hi, lo;
     split4_f16(v[k], s, hi, lo);
+    if (j.perm_H) { const uint32_t g = e[k] / j.perm_H, u = e[k] % j.perm_H; e[k] = 128 * (u / 32) + 32 * g + u % 32; }   // (four units stay together)
     // (the pitch is a multiple of 64: the last item's padding stays inside the line's pitch)
     *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line[k] + e[k]) = hi;
     *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line[k] + e[k]) = lo;
@@ -1018,6 +1019,18 @@ int pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int layout, uint32_t ro
 
 inline uint32_t round_up(uint32_t x, uint32_t m) { return (x + m - 1) / m * m; }
 
+// fp16 planes of the gate weights (F16Gates): I lines of Wx, then H lines of Wh, one set of scales.
+int gates_f16_pack(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, __half* hi, __half* lo, uint32_t* scale) {
+  F16Jobs jobs;
+  jobs.n = 2;
+  for (int q = 0; q < 2; ++q) {
+    const size_t at = q ? (size_t)I * 4 * H : 0;
+    jobs.job[q] = F16Job{q ? Wh : Wx, 4 * H, q ? H : I, 4 * H, 4 * H, F16_ELEM, scale, hi + at, lo + at};
+    jobs.job[q].perm_H = H;
+  }
+  return dyb200_f16_pack(ctx, &jobs);
+}
+
 // Returns the cached packed form of a parameter matrix, packing it first if it is new or stale.
 // (k_is_fast = kLayoutF16 + F16_LINE or F16_ELEM: fp16 planes of the matrix as it lies, its scale words behind the hi plane)
 int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_fast, uint32_t rows, uint32_t K, uint32_t pitch,
@@ -1032,7 +1045,7 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     else if (victim->hi && e->last_use < victim->last_use) victim = e;
   }
   dyb200_ctx::ParamPack* e = hit ? hit : victim;
-  const size_t floats = k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE ? rows : K) : (size_t)(rows + rows2) * pitch;
+  const size_t floats = k_is_fast == kLayoutGatesF16 ? (size_t)(K + rows2) * pitch / 2 + rows : k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE ? rows : K) : (size_t)(rows + rows2) * pitch;
   if (!hit) {
     if (e->hi && e->floats < floats) {   // evicted entry is too small: its buffers may still be read by queued kernels
       DYB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1051,7 +1064,11 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     e->src = src; e->src2 = src2; e->rows2 = rows2; e->ld = ld; e->rows = rows; e->K = K; e->pitch = pitch; e->k_is_fast = (int)k_is_fast;
     e->version = ~0ull;
   }
-  if (e->version != ctx->param_version && k_is_fast >= kLayoutF16) {
+  if (e->version != ctx->param_version && k_is_fast == kLayoutGatesF16) {   // (rows2 = columns of the second matrix)
+    int rc = gates_f16_pack(ctx, src, src2, K, rows2, (__half*)e->hi, (__half*)e->lo, reinterpret_cast<uint32_t*>(e->hi + (size_t)(K + rows2) * pitch / 2));
+    if (rc) return rc;
+    e->version = ctx->param_version;
+  } else if (e->version != ctx->param_version && k_is_fast >= kLayoutF16) {
     F16Jobs jobs;
     jobs.n = 1;
     jobs.job[0] = F16Job{src, ld, rows, K, pitch, k_is_fast - kLayoutF16, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
@@ -1120,6 +1137,25 @@ int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t li
   int rc = cached_param_pack(ctx, src, ld, kLayoutF16 + mode, lines, n, pitch, &hi, &lo);
   if (rc) return rc;
   *job = F16Job{src, ld, lines, n, pitch, mode, reinterpret_cast<uint32_t*>(hi + (size_t)lines * pitch / 2), (__half*)hi, (__half*)lo};
+  return DYB200_OK;
+}
+int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, F16Gates* out) {
+  const uint32_t G = 4 * H;
+  const size_t plane = (size_t)(I + H) * G;
+  float *hi, *lo;
+  uint32_t* scale;
+  int rc;
+  if (ctx->param_cache_on) {
+    if ((rc = cached_param_pack(ctx, Wx, G, kLayoutGatesF16, G, I, G, &hi, &lo, Wh, H))) return rc;
+    scale = reinterpret_cast<uint32_t*>(hi + plane / 2);
+  } else {
+    void *h, *l, *sc;
+    if ((rc = dyb200_scratch(ctx, plane * sizeof(__half), &h)) || (rc = dyb200_scratch(ctx, plane * sizeof(__half), &l)) || (rc = dyb200_scratch(ctx, G * sizeof(uint32_t), &sc))) return rc;
+    hi = (float*)h; lo = (float*)l; scale = (uint32_t*)sc;
+    if ((rc = gates_f16_pack(ctx, Wx, Wh, I, H, (__half*)hi, (__half*)lo, scale))) return rc;
+  }
+  const size_t at = (size_t)I * G;
+  *out = F16Gates{(__half*)hi, (__half*)lo, (__half*)hi + at, (__half*)lo + at, scale};
   return DYB200_OK;
 }
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major) {
@@ -1719,6 +1755,16 @@ bool dyb200_wgrad_column_planes(const dyb200_wgrad* w, uint32_t columns, PackedO
   if (Hs) { *Hs = w->B[1]; Hs->rows = columns; Hs->K = w->N[1]; Hs->mn_major = 0; }
   return true;
 }
+bool dyb200_wgrad_b_planes(const dyb200_wgrad* w, uint32_t col, uint32_t k, PackedOp* X, PackedOp* Hs) {
+  if (!w || w->N[1] == 0 || (uint64_t)col + k > w->Kcap) return false;
+  PackedOp* o[2] = {X, Hs};
+  for (int j = 0; j < 2; ++j) {
+    *o[j] = w->B[j];
+    o[j]->rows = k; o[j]->K = w->N[j]; o[j]->mn_major = 0;
+    o[j]->hi += (size_t)col * w->Np[j]; o[j]->lo += (size_t)col * w->Np[j];
+  }
+  return true;
+}
 void dyb200_wgrad_h_done(dyb200_wgrad* w) {
   w->h_col = 0xffffffffu;           // (no single step's planes are the latest)
   if (w->x_cols > w->kb) w->kb = w->x_cols;
@@ -1728,6 +1774,13 @@ int dyb200_tc_make_tmap(dyb200_ctx* ctx, void* map, float* plane, uint32_t rows,
   int rc = get_encoder(ctx, &enc);
   if (rc) return rc;
   return make_map(ctx, enc, (CUtensorMap*)map, plane, rows, K, pitch, box_rows);
+}
+int dyb200_tc_make_tmap_f16(dyb200_ctx* ctx, void* map, __half* plane, uint32_t rows, uint32_t K, uint32_t pitch, uint32_t box_rows, bool mn_major) {
+  EncodeTiledFn enc;
+  int rc = get_encoder(ctx, &enc);
+  if (rc) return rc;
+  return mn_major ? make_map_mn(ctx, enc, (CUtensorMap*)map, (float*)plane, rows, K, pitch, box_rows, true)
+                  : make_map(ctx, enc, (CUtensorMap*)map, (float*)plane, rows, K, pitch, box_rows, true);
 }
 int dyb200_tc_make_store_map(dyb200_ctx* ctx, void* map, float* C, uint32_t M, uint32_t N, uint32_t S, uint32_t ldc, uint32_t box_cols) {
   EncodeTiledFn enc;

@@ -3,7 +3,7 @@
 // (dynet/rnn.h:120) for a batch of equally long sequences, i.e. T times
 //     gates_t = VanillaLSTMGates(x_t, h_{t-1}, Wx, Wh, b [, masks]);  c_t = VanillaLSTMC(c_{t-1}, gates_t);
 //     h_t = VanillaLSTMH(c_t, gates_t).
-// The per-step form (dyb200_vanilla_lstm_fwd_fused_at) launches one 3xTF32 product per step.  Here the CTAs of that
+// The per-step form (dyb200_vanilla_lstm_fwd_fused_at) launches one 3xTF32 product per step (wide layers: this kernel with T = 1).  Here the CTAs of that
 // product stay resident for the whole sequence: CTA (mt, nt[, split]) owns the same 128 interleaved gate rows (32 hidden
 // units) x BNT batch columns in every step.  What that buys per step: no launch gap, no TMEM allocation / barrier set-up /
 // tensor-map fetch, and the Wx x_{t+1} share of a step's k-blocks (which does not depend on h_t) runs while the epilogue of
@@ -33,13 +33,37 @@ struct SeqFwd {
   // weight-gradient product reads the same planes MN-major)
   float *hn_hi, *hn_lo; uint32_t hn_pitch;
   const float* hmask; uint32_t hmask_ld; int hmask_full;
+  int emit_last;                    // the last step's h goes out as operand planes too (a single step of a sequence driven from outside)
+  // F16: scale words of the gate rows (row q H + u of [Wx Wh]), of the columns of x (sequence columns), of h_{-1} (batch columns) and of all
+  // later h (batch columns, or one for all; null: |h| < 1), and the planes of h .* mask_h as fp16 pairs: two slots of B rows, step t reads
+  // slot t % 2
+  const uint32_t *gate_scale, *x_scale, *h0_scale, *h_scale; int h_scale_full;
+  __half *h16_hi, *h16_lo; uint32_t h16_pitch;
   uint32_t* ready;                  // one arrival counter per column block, zero at launch
   uint32_t* flags;
 };
 
+__device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return a.h_scale ? __ldg(a.h_scale + (a.h_scale_full ? n : 0)) : 0x3f800000u; }
+__device__ __forceinline__ void tmem_ld16x2(uint32_t t1, uint32_t t2, float* v1, float* v2) {
+  uint32_t *r = reinterpret_cast<uint32_t*>(v1), *x = reinterpret_cast<uint32_t*>(v2);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
+                 "=r"(x[7]), "=r"(x[8]), "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
+               : "r"(t1), "r"(t2)
+               : "memory");
+}
+
+// F16: the products of wide layers on scaled fp16 pairs (gemm.cuh) in k-blocks of 64 - half the weight bytes from L2 per step and 0.61 us per 64 k
+// instead of 2 x 0.66.  The weights' planes are MN-major as they lie, their rows interleaved like the TF32 ones; [Wx Wh] has a scale per gate row.
+// A column of x has a scale of its own, h .* mask_h one that is known beforehand (|h| < 1: the largest mask value of the column), h_{-1} the
+// larger of that and its own; so accumulation chains end between Wx x and Wh h, and a chain is unscaled as it is drained.  (Elements of h below 2^-28 of
+// the mask's largest value keep an absolute error of 2^-51 of it.)
 // grid = (4H / 128, B / BNT, S); with S > 1 the S CTAs of a tile are one thread-block cluster (1 x 1 x S).  S (1, 2, 4 or 8) is
 // a template parameter so that the column exchange indexes registers statically.
-template <int BNT, uint32_t S>
+template <int BNT, uint32_t S, bool F16>
 __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_constant__ TmapPack tm, const SeqFwd a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // 64-column tiles need 48 KiB per stage, so the ring holds four of them: at 0.4 us per k-block three stages do not cover
@@ -59,6 +83,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
   const KSplit ks = k_split(a.kb0, a.kb1, rank, S);
   const uint32_t total = ks.n0 + ks.n1;          // k-blocks of this CTA per time step
   const uint32_t M = 4 * a.H, N = a.B;
+  constexpr uint32_t kAccCols = F16 ? 2 * BNT : BN, kBufs = F16 ? kSeqBufs * BN / kAccCols : kSeqBufs, kChunk = F16 ? kChunkF16 : kChunkKB;
+  constexpr int EL = F16 ? 64 : 32;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -89,7 +115,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
       bool fail = false;
       const uint32_t per_step = gridDim.x * S;   // arrivals per column block and step: every CTA that writes a piece of h_t
       for (uint32_t t = 0; t < a.T && !fail; ++t) {
-        const int brow = (int)(t * a.B + n0);
+        const int brow = (int)(t * a.B + n0), hrow = F16 ? (int)((t & 1) * a.B + n0) : brow;
         for (uint32_t it = 0; it < total;) {
           if (it == ks.n0 && t > 0) {
             // The Wh h share of this step needs the planes of h_{t-1}, complete for this column block.  The weight tiles
@@ -101,8 +127,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
               if (!mbar_wait(&empty_bar[s2], ph2 ^ 1)) { fail = true; break; }
               unsigned char* st = ring + (size_t)s2 * kStageBytes;
               mbar_expect_tx(&full_bar[s2], STAGE_TX);
-              tma_load_2d(st, &tm.t[4], &full_bar[s2], (int)((ks.b1 + j) * BK), (int)m0);
-              tma_load_2d(st + TILE_BYTES, &tm.t[5], &full_bar[s2], (int)((ks.b1 + j) * BK), (int)m0);
+              load_a_tile<EL>(st, &tm.t[4], &full_bar[s2], ks.b1 + j, m0, F16);
+              load_a_tile<EL>(st + TILE_BYTES, &tm.t[5], &full_bar[s2], ks.b1 + j, m0, F16);
               if (++s2 == kStages) { s2 = 0; ph2 ^= 1; }
             }
             if (fail) break;
@@ -110,8 +136,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
             asm volatile("fence.proxy.async.global;" ::: "memory");   // generic-proxy stores of other CTAs -> this CTA's TMA reads
             for (uint32_t j = 0; j < pre; ++j) {
               unsigned char* st = ring + (size_t)s * kStageBytes;
-              tma_load_2d(st + 2 * TILE_BYTES, &tm.t[6], &full_bar[s], (int)((ks.b1 + j) * BK), brow);
-              tma_load_2d(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[7], &full_bar[s], (int)((ks.b1 + j) * BK), brow);
+              tma_load_2d(st + 2 * TILE_BYTES, &tm.t[6], &full_bar[s], (int)((ks.b1 + j) * EL), hrow);
+              tma_load_2d(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[7], &full_bar[s], (int)((ks.b1 + j) * EL), hrow);
               if (++s == kStages) { s = 0; ph ^= 1; }
             }
             it += pre;
@@ -121,10 +147,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
           const uint32_t pair = it < ks.n0 ? 0 : 1, kblk = pair ? ks.b1 + (it - ks.n0) : ks.b0 + it;
           unsigned char* st = ring + (size_t)s * kStageBytes;
           mbar_expect_tx(&full_bar[s], STAGE_TX);
-          tma_load_2d(st, &tm.t[4 * pair + 0], &full_bar[s], (int)(kblk * BK), (int)m0);
-          tma_load_2d(st + TILE_BYTES, &tm.t[4 * pair + 1], &full_bar[s], (int)(kblk * BK), (int)m0);
-          tma_load_2d(st + 2 * TILE_BYTES, &tm.t[4 * pair + 2], &full_bar[s], (int)(kblk * BK), brow);
-          tma_load_2d(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[4 * pair + 3], &full_bar[s], (int)(kblk * BK), brow);
+          load_a_tile<EL>(st, &tm.t[4 * pair + 0], &full_bar[s], kblk, m0, F16);
+          load_a_tile<EL>(st + TILE_BYTES, &tm.t[4 * pair + 1], &full_bar[s], kblk, m0, F16);
+          tma_load_2d(st + 2 * TILE_BYTES, &tm.t[4 * pair + 2], &full_bar[s], (int)(kblk * EL), pair ? hrow : brow);
+          tma_load_2d(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[4 * pair + 3], &full_bar[s], (int)(kblk * EL), pair ? hrow : brow);
           if (++s == kStages) { s = 0; ph ^= 1; }
           ++it;
         }
@@ -133,12 +159,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BNT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint32_t idesc = (1u << 4) | (F16 ? 1u << 15 : (2u << 7) | (2u << 10)) | ((uint32_t)(BNT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint32_t idesc_wide = idesc + ((uint32_t)(BNT >> 3) << 17);
       uint64_t d_a_hi[kStages], d_a_lo[kStages], d_b_hi[kStages], d_b_lo[kStages];
 #pragma unroll
       for (int q = 0; q < kStages; ++q) {
         const uint32_t base = smem_u32(ring + (size_t)q * kStageBytes);
-        d_a_hi[q] = umma_desc(base); d_a_lo[q] = umma_desc(base + TILE_BYTES);
+        d_a_hi[q] = F16 ? umma_desc_mn16(base) : umma_desc(base); d_a_lo[q] = F16 ? umma_desc_mn16(base + TILE_BYTES) : umma_desc(base + TILE_BYTES);
         d_b_hi[q] = umma_desc(base + 2 * TILE_BYTES); d_b_lo[q] = umma_desc(base + 2 * TILE_BYTES + TILE_B_BYTES);
       }
       // stage, phase and chunk counters run on across time steps; an accumulation chain never crosses a step
@@ -147,8 +174,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
       for (uint32_t t = 0; t < a.T && !fail; ++t) {
         uint32_t in_chunk = 0;
         for (uint32_t it = 0; it < total; ++it) {
-          if (in_chunk == 0 && chunk >= kSeqBufs) {
-            if (!mbar_wait(&acc_empty[buf], ((chunk / kSeqBufs) - 1) & 1)) { fail = true; break; }
+          if (in_chunk == 0 && chunk >= kBufs) {
+            if (!mbar_wait(&acc_empty[buf], ((chunk / kBufs) - 1) & 1)) { fail = true; break; }
           }
           if (!mbar_wait(&full_bar[s], ph)) { fail = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -157,10 +184,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
           else if (s == 1) { a_hi = d_a_hi[1]; a_lo = d_a_lo[1]; b_hi = d_b_hi[1]; b_lo = d_b_lo[1]; }
           else if (s == 2 || kStages == 3) { a_hi = d_a_hi[2]; a_lo = d_a_lo[2]; b_hi = d_b_hi[2]; b_lo = d_b_lo[2]; }
           else { a_hi = d_a_hi[kStages - 1]; a_lo = d_a_lo[kStages - 1]; b_hi = d_b_hi[kStages - 1]; b_lo = d_b_lo[kStages - 1]; }
-          issue_kblock(tmem_base + buf * BN, a_hi, a_lo, b_hi, b_lo, idesc, in_chunk);
+          if (F16) issue_kblock_f16(tmem_base + buf * kAccCols, tmem_base + buf * kAccCols + BNT, a_hi, a_lo, b_hi, idesc_wide, idesc, in_chunk, 128, 2);
+          else issue_kblock(tmem_base + buf * kAccCols, a_hi, a_lo, b_hi, b_lo, idesc, in_chunk);
           umma_commit(&empty_bar[s]);
-          const bool chunk_ends = in_chunk == kChunkKB - 1 || it == total - 1;
-          if (chunk_ends) { umma_commit(&acc_full[buf]); in_chunk = 0; ++chunk; buf = chunk % kSeqBufs; }
+          const bool chunk_ends = in_chunk == kChunk - 1 || it == total - 1 || (F16 && it + 1 == ks.n0);
+          if (chunk_ends) { umma_commit(&acc_full[buf]); in_chunk = 0; ++chunk; buf = chunk % kBufs; }
           else ++in_chunk;
           if (++s == kStages) { s = 0; ph ^= 1; }
         }
@@ -172,7 +200,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
     const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
     const uint32_t te = threadIdx.x - 64;
     const bool has_cols = 64 * half < BNT;
-    const uint32_t nchunks = (total + kChunkKB - 1) / kChunkKB;
+    const uint32_t x_chunks = (ks.n0 + kChunk - 1) / kChunk;   // (F16: those of Wx x)
+    const uint32_t nchunks = F16 ? x_chunks + (ks.n1 + kChunk - 1) / kChunk : (total + kChunk - 1) / kChunk;
+    // F16: 2^-s of this thread's gate row; of the columns lane and lane + 32 of its half (h after the first step); and 2^s of the columns it finishes
+    float row_f = 1.f, h_f[2] = {1.f, 1.f}, h_s[BNT / 64][2];
+    const uint32_t hn0 = n0 + 64 * half + lane;
+    if (F16) {
+      row_f = inv_scale_of(__ldg(a.gate_scale + (size_t)quarter * a.H + 32 * blockIdx.x + lane));
+      if (has_cols) { h_f[0] = inv_scale_of(h_word(a, hn0)); h_f[1] = inv_scale_of(h_word(a, hn0 + 32)); }
+#pragma unroll
+      for (int hh = 0; hh < BNT / 64; ++hh)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) h_s[hh][k] = scale_of(h_word(a, n0 + 64 * hh + (te >> 3) + 32 * k));
+    }
     // In the cooperative pass over a finished 64-column half this thread owns hidden units [u, u + 4) (rows 32 q + l of the
     // tile are gate q of unit 32 mt + l) for the columns te / 8 and te / 8 + 32 of that half.
     const uint32_t l = 4 * (te & 7), u = blockIdx.x * 32 + l;
@@ -203,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
       const float* const c_prev = t ? a.cs + (size_t)(t - 1) * HB : a.c0;
       float* const c_out = a.cs + (size_t)t * HB;
       float* const h_out = a.hs + (size_t)t * HB;
-      const bool emit = t + 1 < a.T;   // h_t is the next step's input
+      const bool emit = t + 1 < a.T || a.emit_last;   // h_t is the next step's input
       // h_t .* mask_h as operand planes of step t + 1: rows (t + 1) B .. of the planes
       float* const hn_hi = a.hn_hi + (size_t)(t + 1) * a.B * a.hn_pitch;
       float* const hn_lo = a.hn_lo + (size_t)(t + 1) * a.B * a.hn_pitch;
@@ -219,18 +259,34 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
           cp[hh][k] = mine ? ld4(c_prev + u + (size_t)a.H * n) : make_float4(0.f, 0.f, 0.f, 0.f);
           hm[hh][k] = (mine && a.hmask) ? ld4(a.hmask + u + (a.hmask_full ? (size_t)a.hmask_ld * n : 0)) : make_float4(1.f, 1.f, 1.f, 1.f);
         }
+      float f[2] = {1.f, 1.f};   // F16: 2^-s of the columns lane and lane + 32 in the coming chains
+      if (F16 && has_cols) { f[0] = inv_scale_of(__ldg(a.x_scale + (size_t)t * a.B + hn0)); f[1] = inv_scale_of(__ldg(a.x_scale + (size_t)t * a.B + hn0 + 32)); }
       float sum[64];
 #pragma unroll
       for (int q = 0; q < 64; ++q) sum[q] = 0.f;
 #pragma unroll 1
       for (uint32_t c = 0; c < nchunks; ++c, ++cg) {
-        const uint32_t buf = cg % kSeqBufs;
+        const uint32_t buf = cg % kBufs;
+        if (F16 && c == x_chunks) {
+          f[0] = h_f[0]; f[1] = h_f[1];
+          if (t == 0 && has_cols) { f[0] = inv_scale_of(__ldg(a.h0_scale + hn0)); f[1] = inv_scale_of(__ldg(a.h0_scale + hn0 + 32)); }
+        }
         if (!ok) continue;
-        if (!mbar_wait(&acc_full[buf], (cg / kSeqBufs) & 1)) { ok = false; continue; }
+        if (!mbar_wait(&acc_full[buf], (cg / kBufs) & 1)) { ok = false; continue; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (has_cols) {
+        if (F16 && has_cols) {
+          const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + 2 * half * 32;
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {   // (16 columns of both accumulators at a time)
+            float v1[16], v2[16];
+            tmem_ld16x2(taddr + 16 * p, taddr + BNT + 16 * p, v1, v2);
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              sum[16 * p + q] = fmaf(fmaf(v2[q], kLoScale, v1[q]) * row_f, __shfl_sync(0xffffffffu, f[p / 2], 16 * (p % 2) + q), sum[16 * p + q]);
+          }
+        } else if (has_cols) {
           float v[32];
-          const uint32_t taddr = tmem_base + buf * BN + ((quarter * 32) << 16) + 2 * half * 32;
+          const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + 2 * half * 32;
           tmem_ld32(taddr, v);
 #pragma unroll
           for (int q = 0; q < 32; ++q) sum[q] += v[q];
@@ -305,6 +361,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
             split_tf32(hmk.z, phi[k].z, plo[k].z); split_tf32(hmk.w, phi[k].w, plo[k].w);
             st4(hn_hi + (size_t)n * a.hn_pitch + u, phi[k]);
             st4(hn_lo + (size_t)n * a.hn_pitch + u, plo[k]);
+            if (F16 && t + 1 < a.T) {
+              // (of the value that the TF32 pair stands for, as a single step's call makes it of those planes)
+              const float hs = h_s[hh][k];
+              __half ph[4], pl[4];
+              split_f16((phi[k].x + plo[k].x) * hs, ph[0], pl[0]); split_f16((phi[k].y + plo[k].y) * hs, ph[1], pl[1]);
+              split_f16((phi[k].z + plo[k].z) * hs, ph[2], pl[2]); split_f16((phi[k].w + plo[k].w) * hs, ph[3], pl[3]);
+              const size_t o = (size_t)(((t + 1) & 1) * a.B + n) * a.h16_pitch + u;
+              *reinterpret_cast<uint2*>(a.h16_hi + o) = *reinterpret_cast<const uint2*>(ph);
+              *reinterpret_cast<uint2*>(a.h16_lo + o) = *reinterpret_cast<const uint2*>(pl);
+            }
           }
         }
         // all reads of the exchange buffer are done (the next pass may overwrite it) and, in the last pass, every thread has
@@ -346,9 +412,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
 namespace {
 
 // How many clusters of S CTAs of the sequence kernel fit on the GPU at once (remembered per context = per device).
-template <int BNT, uint32_t S>
+template <int BNT, uint32_t S, bool F16>
 int seq_clusters_that_fit(dyb200_ctx* ctx) {
-  int& mc = ctx->seq_max_clusters[BNT == 64 ? 0 : 1][S];
+  int& mc = ctx->seq_max_clusters[(BNT == 64 ? 0 : 1) + (F16 ? 2 : 0)][S];
   if (mc == 0) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -358,13 +424,13 @@ int seq_clusters_that_fit(dyb200_ctx* ctx) {
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = S;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_lstm_seq_fwd<BNT, S>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
+    if (cudaOccupancyMaxActiveClusters(&n, k_lstm_seq_fwd<BNT, S, F16>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
     mc = n > 0 ? n : -1;
   }
   return mc;
 }
 
-template <int BNT, uint32_t S>
+template <int BNT, uint32_t S, bool F16>
 int launch_seq_fwd(dyb200_ctx* ctx, const TmapPack& tm, const SeqFwd& a, dim3 grid, double flops, uint32_t K) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -379,56 +445,117 @@ int launch_seq_fwd(dyb200_ctx* ctx, const TmapPack& tm, const SeqFwd& a, dim3 gr
   // All CTAs wait on one another, so they have to be resident together.  The grid never exceeds what the GPU holds at
   // once (checked by the caller); the cooperative attribute additionally makes the driver schedule them as one gang.  A
   // driver that refuses the attribute for this launch shape gets a plain launch (the waits are bounded either way).
-  if (ctx->seq_coop >= 0) {
+  if (ctx->seq_coop >= 0 && a.T > 1) {   // (a single step's CTAs wait for nobody but their cluster)
     attr[na].id = cudaLaunchAttributeCooperative;
     attr[na].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = na + 1;
-    GemmProfScope scope(ctx, flops, 1, 4 * a.H, a.B * a.T, K, EPI_LSTM_CELL);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S>, tm, a);
+    GemmProfScope scope(ctx, flops, F16 ? 2 : 1, 4 * a.H, a.B * a.T, K, EPI_LSTM_CELL);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S, F16>, tm, a);
     if (e == cudaSuccess) { ctx->seq_coop = 1; ctx->launches++; return DYB200_OK; }
     (void)cudaGetLastError();
     if (ctx->seq_coop == 1) return dyb200_fail(ctx, DYB200_ECUDA, "sequence kernel launch failed: %s", cudaGetErrorString(e));
     ctx->seq_coop = -1;
   }
   cfg.attrs = attr; cfg.numAttrs = na;
-  GemmProfScope scope(ctx, flops, 1, 4 * a.H, a.B * a.T, K, EPI_LSTM_CELL);
-  cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S>, tm, a);
+  GemmProfScope scope(ctx, flops, F16 ? 2 : 1, 4 * a.H, a.B * a.T, K, EPI_LSTM_CELL);
+  cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S, F16>, tm, a);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
 
 // the (tile width, K splits) instantiations behind one switch
 enum SeqOp { SEQ_SET_SMEM, SEQ_FIT, SEQ_LAUNCH };
-template <int BNT, uint32_t S>
+template <int BNT, uint32_t S, bool F16>
 int seq_fwd_do(SeqOp op, dyb200_ctx* ctx, const TmapPack* tm, const SeqFwd* a, dim3 grid, double flops, uint32_t K) {
   if (op == SEQ_SET_SMEM) {
     // (the shared-memory limit of the kernel has to be raised before its occupancy is asked for)
-    const uint32_t bit = (BNT == 64 ? 16u : 256u) << (S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : 3);
+    const uint32_t log_s = S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : 3, bit = (F16 ? (BNT == 64 ? 1u << 12 : 1u << 16) : BNT == 64 ? 16u : 256u) << log_s;
     if (!(ctx->func_attr_done & bit)) {
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_lstm_seq_fwd<BNT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SEQ_BYTES));
+      DYB_CUDA(ctx, cudaFuncSetAttribute(k_lstm_seq_fwd<BNT, S, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SEQ_BYTES));
       ctx->func_attr_done |= bit;
     }
     return DYB200_OK;
   }
-  if (op == SEQ_FIT) return seq_clusters_that_fit<BNT, S>(ctx);
-  return launch_seq_fwd<BNT, S>(ctx, *tm, *a, grid, flops, K);
+  if (op == SEQ_FIT) return seq_clusters_that_fit<BNT, S, F16>(ctx);
+  return launch_seq_fwd<BNT, S, F16>(ctx, *tm, *a, grid, flops, K);
 }
+template <bool F16>
 int seq_fwd_dispatch(SeqOp op, uint32_t bn, uint32_t S, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const SeqFwd* a = nullptr,
                      dim3 grid = dim3(), double flops = 0, uint32_t K = 0) {
   if (bn == 64) {
     switch (S) {
-      case 1: return seq_fwd_do<64, 1>(op, ctx, tm, a, grid, flops, K);
-      case 2: return seq_fwd_do<64, 2>(op, ctx, tm, a, grid, flops, K);
-      case 4: return seq_fwd_do<64, 4>(op, ctx, tm, a, grid, flops, K);
-      default: return seq_fwd_do<64, 8>(op, ctx, tm, a, grid, flops, K);
+      case 1: return seq_fwd_do<64, 1, F16>(op, ctx, tm, a, grid, flops, K);
+      case 2: return seq_fwd_do<64, 2, F16>(op, ctx, tm, a, grid, flops, K);
+      case 4: return seq_fwd_do<64, 4, F16>(op, ctx, tm, a, grid, flops, K);
+      default: return seq_fwd_do<64, 8, F16>(op, ctx, tm, a, grid, flops, K);
     }
   }
   switch (S) {
-    case 1: return seq_fwd_do<128, 1>(op, ctx, tm, a, grid, flops, K);
-    case 2: return seq_fwd_do<128, 2>(op, ctx, tm, a, grid, flops, K);
-    case 4: return seq_fwd_do<128, 4>(op, ctx, tm, a, grid, flops, K);
-    default: return seq_fwd_do<128, 8>(op, ctx, tm, a, grid, flops, K);
+    case 1: return seq_fwd_do<128, 1, F16>(op, ctx, tm, a, grid, flops, K);
+    case 2: return seq_fwd_do<128, 2, F16>(op, ctx, tm, a, grid, flops, K);
+    case 4: return seq_fwd_do<128, 4, F16>(op, ctx, tm, a, grid, flops, K);
+    default: return seq_fwd_do<128, F16 ? 4 : 8, F16>(op, ctx, tm, a, grid, flops, K);
   }
+}
+
+// ---- the inputs of the F16 form, one launch: a warp per line ----
+// x: planes of the columns' inputs (hi + lo) -> fp16 pairs, a word per line.  h_{-1}: h0 .* mask -> TF32 planes (unless they are in place) and
+// fp16 pairs of what those stand for, a word per line: the largest of its values and the mask's.  mask: the words alone.
+struct SeqPrep {
+  const float *x_hi, *x_lo; uint32_t x_ld, I, x_lines; __half *x16_hi, *x16_lo; uint32_t x16_pitch; uint32_t* x_scale;
+  const float *h0, *mask; uint32_t H, B; int mask_full, h0_done; float *hn_hi, *hn_lo; uint32_t hn_pitch; __half *h16_hi, *h16_lo; uint32_t h16_pitch; uint32_t* h0_scale;
+  uint32_t mask_lines; uint32_t* h_scale;
+};
+__global__ void __launch_bounds__(256) k_seq_prep(const __grid_constant__ SeqPrep a) {
+  dyb_grid_dep_sync();
+  uint32_t line = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const uint32_t lane = threadIdx.x & 31;
+  const int kind = line < a.x_lines ? 0 : line < a.x_lines + a.B ? 1 : 2;
+  line -= kind == 0 ? 0 : kind == 1 ? a.x_lines : a.x_lines + a.B;
+  if (kind == 2 && line >= a.mask_lines) return;
+  const uint32_t n = kind == 0 ? a.I : a.H;
+  const float *p = kind == 0 ? a.x_hi + (size_t)line * a.x_ld : kind == 1 ? a.h0 + (size_t)line * a.H : a.mask + (size_t)line * a.H;
+  const float *p2 = kind == 0 ? a.x_lo + (size_t)line * a.x_ld : kind == 1 && a.mask ? a.mask + (a.mask_full ? (size_t)line * a.H : 0) : nullptr;
+  const bool vec = aligned16(p) && (!p2 || aligned16(p2));
+  auto mag = [](float4 v) { return max(max(finite_mag(v.x), finite_mag(v.y)), max(finite_mag(v.z), finite_mag(v.w))); };
+  uint32_t m = kind == 1 && !p2 ? 0x3f800000u : 0;   // (h_{-1}: no smaller than the scale of later h, which an h_{-1} from a call for the step before is)
+  auto value = [&](uint32_t e) {   // elements [e, e + 4), n is a multiple of 4
+    float4 v = vec ? ld4(p + e) : make_float4(p[e], p[e + 1], p[e + 2], p[e + 3]);
+    if (p2) {
+      const float4 w = vec ? ld4(p2 + e) : make_float4(p2[e], p2[e + 1], p2[e + 2], p2[e + 3]);
+      if (kind == 0) v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+      else {
+        v = make_float4(v.x * w.x, v.y * w.y, v.z * w.z, v.w * w.w);
+        m = max(m, mag(w));
+      }
+    }
+    if (kind == 1) {
+      float4 hi, lo;
+      split_tf32(v.x, hi.x, lo.x); split_tf32(v.y, hi.y, lo.y); split_tf32(v.z, hi.z, lo.z); split_tf32(v.w, hi.w, lo.w);
+      if (!a.h0_done) { st4(a.hn_hi + (size_t)line * a.hn_pitch + e, hi); st4(a.hn_lo + (size_t)line * a.hn_pitch + e, lo); }
+      v = make_float4(hi.x + lo.x, hi.y + lo.y, hi.z + lo.z, hi.w + lo.w);
+    }
+    return v;
+  };
+  float4 keep[8];   // lines of up to 1024 values stay in registers between the scale and the split
+#pragma unroll
+  for (uint32_t k = 0; k < 8; ++k) if (4 * lane + 128 * k < n) { keep[k] = value(4 * lane + 128 * k); m = max(m, mag(keep[k])); }
+  for (uint32_t e = 1024 + 4 * lane; e < n; e += 128) m = max(m, mag(value(e)));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (lane == 0) (kind == 0 ? a.x_scale : kind == 1 ? a.h0_scale : a.h_scale)[line] = m;
+  if (kind == 2) return;
+  const float s = scale_of(m);
+  __half* const dh = kind == 0 ? a.x16_hi + (size_t)line * a.x16_pitch : a.h16_hi + (size_t)line * a.h16_pitch;
+  __half* const dl = kind == 0 ? a.x16_lo + (size_t)line * a.x16_pitch : a.h16_lo + (size_t)line * a.h16_pitch;
+  auto split = [&](uint32_t e, float4 v) {
+    __half hi[4], lo[4];
+    split_f16(v.x * s, hi[0], lo[0]); split_f16(v.y * s, hi[1], lo[1]); split_f16(v.z * s, hi[2], lo[2]); split_f16(v.w * s, hi[3], lo[3]);
+    *reinterpret_cast<uint2*>(dh + e) = *reinterpret_cast<const uint2*>(hi);
+    *reinterpret_cast<uint2*>(dl + e) = *reinterpret_cast<const uint2*>(lo);
+  };
+#pragma unroll
+  for (uint32_t k = 0; k < 8; ++k) if (4 * lane + 128 * k < n) split(4 * lane + 128 * k, keep[k]);
+  for (uint32_t e = 1024 + 4 * lane; e < n; e += 128) split(e, value(e));
 }
 
 // gates = Wx x + b over all columns: from the accumulator's input planes, or from x itself without one (no mask then)
@@ -442,6 +569,70 @@ int layer_inputs(dyb200_ctx* ctx, dyb200_wgrad* deferred, const float* Wx, const
 }
 
 }  // namespace
+
+// Layers from 512 units on whose batch is in whole 64-column tiles and whose tiles are all resident (one CTA per SM: 225 KB of shared memory); the
+// TF32 form serves narrower ones.  64-column tiles where there are SMs for them (us per step, I = H = 1024, TF32 / this form with 128 / with 64
+// columns: batch 128 16.5 / 14.3 / 10.5, 256 23.3 / 17.4 / 14.8; batch 512 has 128 columns only, 40.8 / 25.4; batch 64 11.1 / - / 9.0), then as
+// many K splits as there are SMs for, four k-blocks each and more.
+bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* bn, uint32_t* S) {
+  if (H < 512 || H % 32 != 0 || I == 0 || I % 4 != 0 || B == 0 || B % 64 != 0) return false;
+  const uint32_t sms = (uint32_t)ctx->sm_count, tiles_m = 4 * H / BM, kb = (I + 63) / 64 + (H + 63) / 64;
+  *bn = tiles_m * (B / 64) <= sms ? 64 : 128;
+  const uint32_t tiles = tiles_m * (B / *bn);
+  if (B % *bn != 0 || B / *bn > 32) return false;   // (one hand-over counter per column block)
+  for (uint32_t s = *bn == 64 ? 8 : 4; s >= 1; s /= 2) {
+    if (tiles * s > sms || (s > 1 && (kb / s < 4 || !ctx->cluster_splitk))) continue;
+    if (seq_fwd_dispatch<true>(SEQ_SET_SMEM, *bn, s, ctx) != DYB200_OK) return false;
+    if (s > 1) {
+      const int fit = seq_fwd_dispatch<true>(SEQ_FIT, *bn, s, ctx);
+      if (fit <= 0 || tiles > (uint32_t)fit) continue;
+    }
+    *S = s;
+    return true;
+  }
+  return false;
+}
+
+int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q) {
+  const uint32_t I = q.I, H = q.H, B = q.B, T = q.T, G = 4 * H;
+  uint32_t bn, S;
+  DYB_CHECK_ARG(ctx, dyb200_seq_f16_plan(ctx, I, H, B, &bn, &S), "lstm_seq_fwd: shape %u, %u x %u", I, H, B);
+  F16Gates W;
+  int rc;
+  if ((rc = dyb200_f16_gates(ctx, q.Wx, q.Wh, I, H, &W))) return rc;
+  const uint32_t xp = (I + 63) / 64 * 64, hp = (H + 63) / 64 * 64, slots = T > 1 ? 2 : 1;
+  const size_t xn = (size_t)T * B * xp, hn = (size_t)slots * B * hp;
+  void *p16, *words;
+  if ((rc = dyb200_scratch(ctx, 2 * (xn + hn) * sizeof(__half), &p16)) || (rc = dyb200_scratch(ctx, ((size_t)T * B + 2 * (size_t)B) * sizeof(uint32_t), &words))) return rc;
+  SeqPrep p;
+  memset(&p, 0, sizeof(p));
+  p.x_hi = q.X.hi; p.x_lo = q.X.lo; p.x_ld = q.X.pitch; p.I = I; p.x_lines = T * B;
+  p.x16_hi = (__half*)p16; p.x16_lo = p.x16_hi + xn; p.x16_pitch = xp; p.x_scale = (uint32_t*)words;
+  p.h0 = q.h0; p.mask = q.mh; p.H = H; p.B = B; p.mask_full = q.mh_full; p.h0_done = q.h0_done; p.hn_hi = q.Hs.hi; p.hn_lo = q.Hs.lo; p.hn_pitch = q.Hs.pitch;
+  p.h16_hi = p.x16_lo + xn; p.h16_lo = p.h16_hi + hn; p.h16_pitch = hp; p.h0_scale = p.x_scale + (size_t)T * B;
+  p.mask_lines = q.mh ? (q.mh_full ? B : 1) : 0; p.h_scale = p.h0_scale + B;
+  dyb_launch(k_seq_prep, (unsigned)(((size_t)T * B + B + p.mask_lines + 7) / 8), 256, 0, ctx, p);
+  DYB_LAUNCHED(ctx);
+  TmapPack tm;
+  memset(&tm, 0, sizeof(tm));
+  struct { __half* plane; uint32_t rows, K, pitch, box; bool mn; } maps[8] = {
+      {W.x_hi, G, I, G, BM, true}, {W.x_lo, G, I, G, BM, true}, {p.x16_hi, T * B, I, xp, bn, false}, {p.x16_lo, T * B, I, xp, bn, false},
+      {W.h_hi, G, H, G, BM, true}, {W.h_lo, G, H, G, BM, true}, {p.h16_hi, slots * B, H, hp, bn, false}, {p.h16_lo, slots * B, H, hp, bn, false}};
+  for (int k = 0; k < 8; ++k)
+    if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[k], maps[k].plane, maps[k].rows, maps[k].K, maps[k].pitch, maps[k].box, maps[k].mn))) return rc;
+  SeqFwd a;
+  memset(&a, 0, sizeof(a));
+  a.T = T; a.B = B; a.H = H; a.kb0 = xp / 64; a.kb1 = hp / 64;
+  a.gates = q.gates; a.cs = q.c; a.hs = q.h; a.c0 = q.c0; a.bias = q.b; a.forget_bias = q.forget_bias;
+  a.hn_hi = q.Hs.hi; a.hn_lo = q.Hs.lo; a.hn_pitch = q.Hs.pitch;
+  a.hmask = q.mh; a.hmask_ld = H; a.hmask_full = q.mh_full; a.emit_last = q.emit_last;
+  a.gate_scale = W.scale; a.x_scale = p.x_scale; a.h0_scale = p.h0_scale; a.h_scale = q.mh ? p.h_scale : nullptr; a.h_scale_full = q.mh_full;
+  a.h16_hi = p.h16_hi; a.h16_lo = p.h16_lo; a.h16_pitch = hp;
+  a.ready = ctx->dev_flags + DYB200_DEV_SEQ0;
+  a.flags = ctx->dev_flags;
+  DYB_CUDA(ctx, cudaMemsetAsync(a.ready, 0, 32 * sizeof(uint32_t), ctx->stream));
+  return seq_fwd_dispatch<true>(SEQ_LAUNCH, bn, S, ctx, &tm, &a, dim3(G / BM, B / bn, S), 2.0 * G * (double)B * (I + H) * T, I + H);
+}
 
 extern "C" {
 
@@ -472,13 +663,22 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
   // 763 / 1228 / 2070 against 535 / 930 / 1738.)
   const uint32_t bn = dyb200_tc_tile_cols(B);
   const uint32_t kb0 = (I + 31) / 32, kb1 = (H + 31) / 32, kb_total = kb0 + kb1;
-  bool persistent = ctx->seq_kernels && deferred && T >= 2 && attrs->weightnoise_std == 0.f && H % 32 == 0 && I % 4 == 0 && B % bn == 0 &&
+  const bool resident = ctx->seq_kernels && deferred && T >= 2 && attrs->weightnoise_std == 0.f && H % 32 == 0 && I % 4 == 0 &&
                     dyb200_tc_eligible(G, B, 2.0 * G * B * (I + H)) && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 &&
                     Wh->d[0] == G && Wh->d[1] == H && t_size(b) == G && aligned16(gates_all->v) && aligned16(b->v) && aligned16(c0->v) &&
                     aligned16(c_all->v) && aligned16(h_all->v) && (!mh || aligned16(mh)) &&
                     (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H));
-  uint32_t S = 1;
+  uint32_t S = 1, f16_bn;
   SeqPlanes pl;
+  if (resident && dyb200_seq_f16_plan(ctx, I, H, B, &f16_bn, &S) && dyb200_wgrad_seq_planes(deferred, T, B, &pl)) {   // (wide layers)
+    { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
+    DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_seq_fwd: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
+    SeqF16Call q{I, H, B, T, Wx->v, Wh->v, b->v, h0->v, c0->v, mh, mh_full, attrs->forget_gate_bias, gates_all->v, c_all->v, h_all->v, pl.X, pl.Hs, 0, 0};
+    if ((rc = dyb200_seq_f16(ctx, q))) return rc;
+    dyb200_wgrad_seq_done(deferred);
+    return DYB200_OK;
+  }
+  bool persistent = resident && B % bn == 0;
   if (persistent) {
     S = dyb200_tc_splits(ctx, G, B, kb_total);
     const uint32_t per = (kb_total + S - 1) / S;
@@ -486,9 +686,9 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
     const uint32_t tiles = (G / BM) * (B / bn);
     if (S > 8 || (S & (S - 1)) != 0 || (S > 1 && !ctx->cluster_splitk)) persistent = false;   // (the column exchange wants a power of two)
     else {
-      if ((rc = seq_fwd_dispatch(SEQ_SET_SMEM, bn, S, ctx))) return rc;
+      if ((rc = seq_fwd_dispatch<false>(SEQ_SET_SMEM, bn, S, ctx))) return rc;
       if (S > 1) {
-        const int fit = seq_fwd_dispatch(SEQ_FIT, bn, S, ctx);
+        const int fit = seq_fwd_dispatch<false>(SEQ_FIT, bn, S, ctx);
         persistent = fit > 0 && tiles <= (uint32_t)fit;
       } else {
         persistent = tiles <= (uint32_t)ctx->sm_count;   // one CTA per SM (225 KB of shared memory each)
@@ -528,7 +728,7 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
     DYB_CUDA(ctx, cudaMemsetAsync(a.ready, 0, 32 * sizeof(uint32_t), ctx->stream));
     const dim3 grid(G / BM, B / bn, S);
     const double flops = 2.0 * G * (double)B * (I + H) * T;
-    rc = seq_fwd_dispatch(SEQ_LAUNCH, bn, S, ctx, &tm, &a, grid, flops, I + H);
+    rc = seq_fwd_dispatch<false>(SEQ_LAUNCH, bn, S, ctx, &tm, &a, grid, flops, I + H);
     if (rc) return rc;
     dyb200_wgrad_seq_done(deferred);
     return DYB200_OK;

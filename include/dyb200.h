@@ -317,13 +317,15 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
  * dyb200_vanilla_lstm_fwd_fused_at with deferred_col = t * batch, h_tm1 / c_tm1 = the previous step's outputs.
  *   * When the shape allows (deferred given, tensor-path sizes, whole tiles, every CTA resident at once) the steps run inside ONE
  *     kernel whose CTAs stay on the GPU for the whole sequence and hand h_t over through device memory: bit for bit the calls above.
+ *     From 512 units on the products of both (calls with an accumulator, batches in whole 64-column tiles) are of scaled fp16 pairs: a scale
+ *     per gate row and per column of x, and for a column of h the largest of its mask's values (1 without) and, in the first step, of h0.
  *   * Other sequences of at least 8 steps of layers up to 384 units, or with at most 32 columns, form Wx x of all steps at once and
  *     keep only Wh h in the recurrence: the same values to the rounding of their sums, which associate differently, and the same
  *     bits from run to run.  Wh h is plain fp32 above 256 units, and below while there are at most four columns per cluster of
  *     CTAs (60 columns at 256 units, more for narrower layers); with more columns it is a product of scaled fp16 pairs, 2 x 11 bits as
  *     the TF32 pairs of the calls above have: Wh scaled by the largest value of each gate row, h by that of the initial state in
- *     the first step and by the largest mask value (1 without) after it (16 columns share them).  What lies 2^28 below such a scale keeps
- *     an absolute error of 2^-51 of it, the rounding of a pre-activation of 2^-27.
+ *     the first step and by the largest mask value (1 without) after it (16 columns share them).
+ *     What lies 2^28 below such a scale keeps an absolute error of 2^-51 of it, the rounding of a pre-activation of 2^-27.
  *   * Otherwise the calls above are made.  dyb200_ctx_sequence_kernels(ctx, 0) forces that.
  * h0 / c0 may lie on a step's columns of h_all / c_all (a text read piece by piece into the same buffers).  deferred may be NULL
  * (nothing recorded for the weight gradients). */

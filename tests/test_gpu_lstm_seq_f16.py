@@ -1,0 +1,62 @@
+"""The forward recurrence of wide layers on fp16 pairs (csrc/lstm_seq.cu, F16): reductions that are no multiple of a k-block or longer than a
+chain, one to eight K splits, 64- and 128-column tiles, masks per column and for all, an initial state far above 1, columns of x that differ
+by 2^60 and a column of zeros, the slots of h in turn.  Step by step against float64 from the device's own h_{t-1} and c_{t-1}.  Bar of a
+pre-activation: 4.5e-7 of |row of Wx| |x| + |row of Wh| |h .* mask|, that of every product on fp16 pairs; of a gate: that (its slope is at
+most 1) and 3e-6 for the approximate exponential and reciprocal.  The single-step calls must give the same bits, also where
+saturated gates leave elements of h far below 2^-28."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("I,H,B,T,mask", [
+    (300, 544, 64, 4, "full"),       # tails in both reductions, eight splits
+    (1100, 1056, 64, 3, None),       # chains cut within both products, lines longer than a warp holds
+    (4, 512, 192, 3, "one"),         # the shortest x, three column blocks
+    (512, 1024, 256, 2, "full"),     # one split, 64 columns
+    (36, 1024, 512, 3, "one"),       # 128 columns
+    (1024, 2048, 128, 2, None),      # a reduction of 48 k-blocks
+])
+def test_sequence_of_a_wide_layer(I, H, B, T, mask):
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    gen = torch.Generator("cuda").manual_seed(H + B)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    x, h0, c0, b = rnd(T * B, I), rnd(B, H) * 30.0, rnd(B, H), rnd(4 * H) * 0.1
+    x *= torch.exp2(torch.randint(-60, 3, (T * B, 1), device="cuda", generator=gen).float())
+    x[5] = 0.0
+    Wx, Wh = rnd(I, 4 * H) / I ** 0.5, rnd(H, 4 * H) / H ** 0.5
+    mB = B if mask == "full" else 1
+    mx, mh = [((torch.rand(mB, n, device="cuda", generator=gen) < 0.8) / 0.8).float() if mask else torch.ones(1, n, device="cuda") for n in (I, H)]
+    at, tm = capi.LstmGatesAttrs(1 if mask else 0, 0.0, 1.0), (g.T(mx), g.T(mh)) if mask else (None, None)
+    W = (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1))
+    out = []
+    for single in (False, True):
+        w = ctx.wgrad_create(4 * H, I, H, T * B)
+        gates, cs, hs = (torch.full((T * B, n), 7.0, device="cuda") for n in (4 * H, H, H))
+        if single:
+            for t in range(T):
+                sl, pr = slice(t * B, (t + 1) * B), slice((t - 1) * B, t * B)
+                ctx.lstm_fwd_fused_at(g.T(x[sl]), g.T(hs[pr] if t else h0), g.T(cs[pr] if t else c0), *W, *tm, at, g.T(gates[sl]), g.T(cs[sl]), g.T(hs[sl]), w, t * B)
+        else:
+            ctx.lstm_seq_fwd(g.T(x, [I], T * B), g.T(h0), g.T(c0), *W, *tm, at, g.T(gates, [4 * H], T * B), g.T(cs, [H], T * B), g.T(hs, [H], T * B), w, T)
+        torch.cuda.synchronize()
+        ctx.wgrad_destroy(w)
+        out.append((gates, cs, hs))
+    for p, q in zip(*out):
+        assert torch.equal(p, q)
+    gates, cs, hs = (o.double().view(T, B, -1) for o in out[0])
+    for t in range(T):
+        xt, hp, cp = x.double().view(T, B, I)[t] * mx.double(), (hs[t - 1] if t else h0.double()) * mh.double(), cs[t - 1] if t else c0.double()
+        pre = xt @ Wx.double() + hp @ Wh.double() + b.double()
+        bar = 4.5e-7 * (xt.norm(dim=1)[:, None] * Wx.double().norm(dim=0) + hp.norm(dim=1)[:, None] * Wh.double().norm(dim=0)) + 3e-6
+        pre[:, H:2 * H] += 1.0
+        want = torch.cat([torch.sigmoid(pre[:, :3 * H]), torch.tanh(pre[:, 3 * H:])], dim=1)
+        assert bool(((gates[t] - want).abs() <= bar).all()), "step %d: %.3g" % (t, float(((gates[t] - want).abs() / bar).max()))
+        i, f, o, gg = gates[t].split(H, dim=1)
+        c = i * gg + f * cp
+        assert bool(((cs[t] - c).abs() <= 2e-7 * ((i * gg).abs() + (f * cp).abs())).all())
+        assert bool(((hs[t] - o * torch.tanh(cs[t])).abs() <= 5e-7).all())
+    assert ctx.device_errors() == 0
