@@ -95,18 +95,20 @@ __global__ void __launch_bounds__(kBlock) k_col_warp(ColArgs a) {
   }
 }
 
-// ---- CTA per column, rows <= 4096, 16-byte aligned columns --------------------
-template <int MODE>
+// ---- CTA per column, the column in registers (VEC 16-byte loads per thread, all in flight together), 16-byte aligned columns ----
+// Up to 4096 rows with 4 loads per thread, 8192 with 8, 12288 with 12 (10 000 rows, 17 920 columns: 161 us streamed, 145 in registers).
+__device__ __forceinline__ float shift_log2(float m) { return m == -INFINITY ? 0.f : m * kLog2e; }
+template <int MODE, int VEC>
 __global__ void __launch_bounds__(kBlock) k_col_block_vec(ColArgs a) {
   dyb_grid_dep_sync();
   __shared__ float red[32];
   const uint32_t rows4 = a.rows / 4;
   for (size_t c = blockIdx.x; c < a.ncols; c += gridDim.x) {
     const float* xc = a.x + c * a.rows;
-    float4 v[kBlockVec];
+    float4 v[VEC];
     float mx = -INFINITY;
 #pragma unroll
-    for (int k = 0; k < kBlockVec; ++k) {
+    for (int k = 0; k < VEC; ++k) {
       uint32_t i = threadIdx.x + kBlock * k;
       if (i < rows4) {
         v[k] = ld4_stream(xc + 4 * i);
@@ -116,10 +118,10 @@ __global__ void __launch_bounds__(kBlock) k_col_block_vec(ColArgs a) {
     mx = block_max(mx, red);
     float s = 0.f;
 #pragma unroll
-    for (int k = 0; k < kBlockVec; ++k) {
+    for (int k = 0; k < VEC; ++k) {
       uint32_t i = threadIdx.x + kBlock * k;
       if (i < rows4) {
-        const float ml = mx * kLog2e;
+        const float ml = VEC > kBlockVec ? shift_log2(mx) : mx * kLog2e;   // (columns of -inf: as the streaming form has it for their length)
         float4 e = make_float4(ex2_approx(fmaf(v[k].x, kLog2e, -ml)), ex2_approx(fmaf(v[k].y, kLog2e, -ml)),
                                ex2_approx(fmaf(v[k].z, kLog2e, -ml)), ex2_approx(fmaf(v[k].w, kLog2e, -ml)));
         s += (e.x + e.y) + (e.z + e.w);
@@ -133,7 +135,7 @@ __global__ void __launch_bounds__(kBlock) k_col_block_vec(ColArgs a) {
       const float inv = 1.f / s;   // one division per column
       float* yc = a.y + c * a.rows;
 #pragma unroll
-      for (int k = 0; k < kBlockVec; ++k) {
+      for (int k = 0; k < VEC; ++k) {
         uint32_t i = threadIdx.x + kBlock * k;
         if (i < rows4) {
           float4 r = MODE == M_SOFTMAX ? make_float4(v[k].x * inv, v[k].y * inv, v[k].z * inv, v[k].w * inv)
@@ -154,7 +156,6 @@ __device__ __forceinline__ void online_add(float& m, float& s, float v) {
   if (v > m) { s = s * ex2_approx((m - v) * kLog2e) + 1.f; m = v; }
   else if (v != -INFINITY) s += ex2_approx((v - m) * kLog2e);
 }
-__device__ __forceinline__ float shift_log2(float m) { return m == -INFINITY ? 0.f : m * kLog2e; }
 __device__ __forceinline__ float max4(float4 v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
 __device__ __forceinline__ float sumexp4(float4 v, float ml) {
   return (ex2_approx(fmaf(v.x, kLog2e, -ml)) + ex2_approx(fmaf(v.y, kLog2e, -ml))) +
@@ -261,9 +262,12 @@ int run_columns(dyb200_ctx* ctx, ColArgs a) {
   if (a.rows <= kWarpRowsMax) {
     dyb_launch(k_col_warp<MODE>, stream_grid(ctx, a.ncols, kBlock / 32), kBlock, 0, ctx, a);
   } else if (a.rows <= kBlockRowsMax && a.rows % 4 == 0 && aligned16(a.x) && (a.y == nullptr || aligned16(a.y))) {
-    dyb_launch(k_col_block_vec<MODE>, stream_grid(ctx, a.ncols, 1), kBlock, 0, ctx, a);
+    dyb_launch(k_col_block_vec<MODE, kBlockVec>, stream_grid(ctx, a.ncols, 1), kBlock, 0, ctx, a);
   } else if (a.rows > 2048 && a.rows <= kColCluster * kBlock * kColVals && a.ncols * kColCluster <= (size_t)ctx->sm_count) {
     dyb_launch(k_col_cluster<MODE>, dim3(kColCluster, (unsigned)a.ncols), kBlock, 0, ctx, a);
+  } else if (a.rows <= 3 * kBlockRowsMax && a.rows % 4 == 0 && aligned16(a.x) && (a.y == nullptr || aligned16(a.y))) {
+    if (a.rows <= 2 * kBlockRowsMax) dyb_launch(k_col_block_vec<MODE, 2 * kBlockVec>, stream_grid(ctx, a.ncols, 1, 4), kBlock, 0, ctx, a);
+    else dyb_launch(k_col_block_vec<MODE, 3 * kBlockVec>, stream_grid(ctx, a.ncols, 1, 3), kBlock, 0, ctx, a);
   } else {
     dyb_launch(k_col_stream<MODE>, stream_grid(ctx, a.ncols, 1), kBlock, 0, ctx, a);
   }
@@ -470,38 +474,52 @@ __device__ __forceinline__ float4 pnls_x4(const float* xc, uint32_t r, uint32_t 
 
 // The largest |d| of every row and of every column, for fp16 planes.  Bound by reading x once more (819 MB: 50 000 x 4096).  A CTA
 // takes 1024 rows x kPnlsMaxCols columns, eight columns requested at a time; a row's maximum stays with its thread, a column's meets by
-// one reduction per warp; both meet the other CTAs' by atomicMax on bit patterns (the same from run to run).
+// one reduction per warp and the CTA's in shared memory; both meet the other CTAs' by atomicMax on bit patterns (the same from run to run).
 constexpr uint32_t kPnlsMaxCols = 64;
 __global__ void __launch_bounds__(256) k_softmax_bwd_max(const float* __restrict__ x, const float* __restrict__ z, const float* __restrict__ dz,
                                                          const uint32_t* __restrict__ ids, uint32_t rows, uint32_t ncols,
                                                          uint32_t* __restrict__ row_max, uint32_t* __restrict__ col_max, int vec) {
   dyb_grid_dep_sync();
-  const uint32_t r = (blockIdx.x * 256 + threadIdx.x) * 4, c_end = min(ncols, (blockIdx.y + 1) * kPnlsMaxCols);
+  __shared__ float col_z[kPnlsMaxCols], col_dz[kPnlsMaxCols];
+  __shared__ uint32_t col_id[kPnlsMaxCols], col_top[kPnlsMaxCols];
+  const uint32_t r = (blockIdx.x * 256 + threadIdx.x) * 4, c_begin = blockIdx.y * kPnlsMaxCols, cols = min(ncols - c_begin, kPnlsMaxCols);
   const bool live = r < rows;
+  if (threadIdx.x < cols) {
+    const uint32_t c = c_begin + threadIdx.x;
+    col_z[threadIdx.x] = z[c]; col_dz[threadIdx.x] = dz[c]; col_id[threadIdx.x] = ids ? ids[c] : 0xffffffffu; col_top[threadIdx.x] = 0;
+  }
+  __syncthreads();
   uint32_t m[4] = {0, 0, 0, 0};
-  for (uint32_t c0 = blockIdx.y * kPnlsMaxCols; c0 < c_end; c0 += 8) {
+  const float* p = x + (size_t)c_begin * rows;
+  for (uint32_t c0 = 0; c0 < cols; c0 += 8, p += 8 * (size_t)rows) {
     float4 v[8];
+    if (vec && c0 + 8 <= cols) {   // (straight loads; behind a branch per load they went out one by one: 239 us for 50 000 x 4096, 150 now)
 #pragma unroll
-    for (uint32_t q = 0; q < 8; ++q)
-      v[q] = live && c0 + q < c_end ? pnls_x4(x + (size_t)(c0 + q) * rows, r, rows, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (uint32_t q = 0; q < 8; ++q) v[q] = ld4_stream(p + (size_t)q * rows + (live ? r : 0));
+    } else {
+#pragma unroll
+      for (uint32_t q = 0; q < 8; ++q) v[q] = live && c0 + q < cols ? pnls_x4(p + (size_t)q * rows, r, rows, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 #pragma unroll
     for (uint32_t q = 0; q < 8; ++q) {
       const uint32_t c = c0 + q;
-      if (c >= c_end) break;
+      if (c >= cols) break;
       uint32_t most = 0;
       if (live) {
-        const float4 d = pnls_grad4(v[q], r, rows, ids ? ids[c] : 0xffffffffu, z[c], dz[c], vec);
+        const float4 d = pnls_grad4(v[q], r, rows, col_id[c], col_z[c], col_dz[c], vec);
         const uint32_t w[4] = {finite_mag(d.x), finite_mag(d.y), finite_mag(d.z), finite_mag(d.w)};
 #pragma unroll
         for (int k = 0; k < 4; ++k) { m[k] = max(m[k], w[k]); most = max(most, w[k]); }
       }
       most = __reduce_max_sync(0xffffffffu, most);
-      if (most && (threadIdx.x & 31) == 0) atomicMax(col_max + c, most);
+      if (most && (threadIdx.x & 31) == 0) atomicMax(col_top + c, most);
     }
   }
 #pragma unroll
   for (uint32_t k = 0; k < 4; ++k)
     if (r + k < rows) atomicMax(row_max + r + k, m[k]);
+  __syncthreads();
+  if (threadIdx.x < cols && col_top[threadIdx.x]) atomicMax(col_max + c_begin + threadIdx.x, col_top[threadIdx.x]);
 }
 
 // F16: the planes are scaled fp16 pairs (half the bytes), of which there are two sets - the scale belongs to the operand's row, and that

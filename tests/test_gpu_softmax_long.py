@@ -51,3 +51,31 @@ def test_long_columns_beside_other_work():
     assert all(torch.equal(y_[0], y_[k]) for k in range(200))
     assert g.ctx().device_errors() == 0
     g.release()
+
+
+@pytest.mark.parametrize("rows", [4100, 8192, 8196, 12288, 12292])
+def test_columns_in_registers(rows):
+    """Many columns at the lengths where a thread's share of a column changes, with entries of -inf, against float64.  Bar: log-probabilities
+    down to -30 from fp32 exponents, an ulp of 30 and of the sum; probabilities to 1e-5 of themselves."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    bd = 150
+    gen = torch.Generator("cuda").manual_seed(rows)
+    x = torch.randn(bd, rows, device="cuda", generator=gen) * 3.0
+    x[:, 7::11] = -float("inf")
+    x[3] -= 80.0
+    y, ly, loss = torch.empty_like(x), torch.empty_like(x), torch.empty(bd, device="cuda")
+    aux, paux = torch.empty(2 * bd, device="cuda"), torch.zeros(3 * bd, device="cuda")
+    ids = torch.randint(0, rows // 11, (bd,), device="cuda", generator=gen) * 11
+    paux[2 * bd:].view(torch.int32).copy_(ids.int())
+    g.ctx().fwd("softmax", [g.T(x, [rows], bd)], g.T(y, [rows], bd), capi.DimAttrs(0))
+    g.ctx().fwd("log_softmax", [g.T(x, [rows], bd)], g.T(ly, [rows], bd), None, aux.data_ptr())
+    g.ctx().fwd("pickneglogsoftmax", [g.T(x, [rows], bd)], g.T(loss, [1], bd), capi.PickAttrs(None, bd), paux.data_ptr())
+    want = torch.log_softmax(x.double(), dim=1)
+    live = torch.isfinite(want)
+    assert bool(((y.double() - want.exp()).abs() <= 1e-5 * want.exp()).all())
+    assert bool((ly[live] - want[live]).abs().max() <= 1.6e-5) and bool((ly[~live] == -float("inf")).all())
+    assert bool((loss.double() + want[torch.arange(bd), ids]).abs().max() <= 1.6e-5)
+    assert g.ctx().device_errors() == 0
+    g.release()
