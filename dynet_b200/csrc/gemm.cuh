@@ -46,7 +46,17 @@ struct GemmEpilogue {
   // weight-gradient product.  16-byte aligned, H % 4 == 0.
   float* hn_hi = nullptr; float* hn_lo = nullptr; uint32_t hn_pitch = 0;
   const float* hmask = nullptr; uint32_t hmask_ld = 0; int hmask_full = 0;
+  // Two right operands side by side (TmapPack::n_split): columns [0, n_live) belong to C, those from n_split on to Cn, the ones between do not exist.
+  uint32_t n_split = 0, n_live = 0; float* Cn = nullptr; uint32_t ldcn = 0;
 };
+#ifdef __CUDACC__
+// The destination of a tile whose first column is n0 (a tile lies on one side): C, n0 and the end of its columns N.
+__device__ __forceinline__ void epi_side(GemmEpilogue& e, uint32_t& n0, uint32_t& N) {
+  if (!e.n_split) return;
+  if (n0 >= e.n_split) { e.C = e.Cn; e.ldc = e.ldcn; n0 -= e.n_split; N -= e.n_split; }
+  else N = e.n_live;
+}
+#endif
 #ifdef __CUDACC__
 // h .* mask of four hidden units [u, u + 4) of batch column n, written as operand planes (see GemmEpilogue::hn_hi).
 __device__ __forceinline__ void epi_emit_h(const GemmEpilogue& epi, uint32_t u, uint32_t n, float4 h) {
@@ -186,7 +196,9 @@ int dyb200_tc_param2(dyb200_ctx* ctx, const float* src, uint32_t rows, const flo
 // force_splits > 0: that many K splits (normalised so that no split is empty) instead of the cost model's choice.
 int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const PackedOp* A, const PackedOp* B,
                           const GemmEpilogue& epi, uint32_t force_splits = 0);
-int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi);
+int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi, size_t split_stride = 0);
+// C0 += A B0^T and C1 += A B1^T in one launch (TF32 planes, all MN-major; dWx and dWh of a layer).
+int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const PackedOp* B, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1);
 // Tiling of the backward recurrence of an LSTM layer (dx_t, dh_{t-1} += [Wx; Wh]^T dgates_t), shared by the per-step call
 // and the sequence kernel so that both add the same partial sums: tile width, batch-column blocks per CTA of the sequence
 // kernel (1 or 2) and K splits.  False when the shape does not suit the sequence kernel (the per-step call then lets the

@@ -103,6 +103,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
   if (warp == 0) {
     if (elect_one()) {
       uint32_t s = 0, ph = 0;
+      const bool second = tm.n_split && n0 >= tm.n_split;
+      const uint32_t nb0 = second ? n0 - tm.n_split : n0;
       for (uint32_t it = 0; it < total; ++it) {
         if (!mbar_wait(&empty_bar[s], ph ^ 1)) { atomicOr(flags, DYB200_FLAG_WAIT_TIMEOUT); break; }
         const uint32_t pair = it < ks.n0 ? 0 : 1, kblk = pair ? ks.b1 + (it - ks.n0) : ks.b0 + it;
@@ -110,8 +112,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
         mbar_expect_tx(&full_bar[s], STAGE_TX);
         load_a_tile<EL>(st, &tm.t[4 * pair + 0], &full_bar[s], kblk, m0, tm.a_mn);
         load_a_tile<EL>(st + TILE_BYTES, &tm.t[4 * pair + 1], &full_bar[s], kblk, m0, tm.a_mn);
-        load_b_tile<EL>(st + 2 * TILE_BYTES, &tm.t[4 * pair + 2], &full_bar[s], kblk, n0, tm.b_mn);
-        load_b_tile<EL>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[4 * pair + 3], &full_bar[s], kblk, n0, tm.b_mn);
+        load_b_tile<EL>(st + 2 * TILE_BYTES, &tm.t[second ? 6 : 4 * pair + 2], &full_bar[s], kblk, nb0, tm.b_mn);
+        load_b_tile<EL>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[second ? 7 : 4 * pair + 3], &full_bar[s], kblk, nb0, tm.b_mn);
         if (++s == STAGES) { s = 0; ph ^= 1; }
       }
     }
@@ -229,11 +231,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
 #pragma unroll
       for (int j = 0; j < 64; ++j) col[(size_t)j * BM] = sum[j];
     }
+    uint32_t ne0 = n0, Ne = N;
+    epi_side(epi, ne0, Ne);
     uint32_t all_ok;
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, 1, 256, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(all_ok) : "r"((uint32_t)ok) : "memory");
     if (!CLUSTER) {
-      if (all_ok) epilogue_pass<BNT, 256>(epi, tile, te, blockIdx.x, m0, n0, M, N, cprev);
+      if (all_ok) epilogue_pass<BNT, 256>(epi, tile, te, blockIdx.x, m0, ne0, M, Ne, cprev);
     } else {
       // every thread of every CTA of the cluster takes part in the two cluster barriers below (the TMA and MMA warps
       // reach them further down); between them rank 0 reads the other CTAs' tiles
@@ -269,7 +273,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
             t4[f] = acc;
           }
           asm volatile("barrier.cta.sync 1, 256;" ::: "memory");   // the pass below reads other threads' pieces
-          epilogue_pass<BNT, 256>(epi, tile, te, blockIdx.x, m0, n0, M, N, cprev, c_lo, c_hi);
+          epilogue_pass<BNT, 256>(epi, tile, te, blockIdx.x, m0, ne0, M, Ne, cprev, c_lo, c_hi);
         } else if (te == 0 && rank == 0) {
           atomicOr(flags, DYB200_FLAG_WAIT_TIMEOUT);
         }
@@ -328,6 +332,8 @@ __device__ __noinline__ void persist_producer(const TmapPack* tm, unsigned char*
     uint32_t mt, nt;
     persist_tile_coords(tile, tiles_m, tiles_n, gm, mt, nt);
     const uint32_t m0 = mt * BM, n0 = nt * BNT;
+    const bool second = tm->n_split && n0 >= tm->n_split;
+    const uint32_t nb0 = second ? n0 - tm->n_split : n0;
     for (uint32_t g = 0; g < ks.n0 + ks.n1; ++g) {
       if (!mbar_wait(&empty_bar[s], ph ^ 1)) { fail = true; break; }
       const uint32_t pair = g < ks.n0 ? 0 : 1, kblk = pair ? ks.b1 + (g - ks.n0) : ks.b0 + g;
@@ -335,8 +341,8 @@ __device__ __noinline__ void persist_producer(const TmapPack* tm, unsigned char*
       mbar_expect_tx(&full_bar[s], STAGE_TX);
       load_a_tile<F16 ? 64 : 32>(st, &tm->t[4 * pair + 0], &full_bar[s], kblk, m0, tm->a_mn);
       load_a_tile<F16 ? 64 : 32>(st + TILE_BYTES, &tm->t[4 * pair + 1], &full_bar[s], kblk, m0, tm->a_mn);
-      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES, &tm->t[4 * pair + 2], &full_bar[s], kblk, n0, tm->b_mn);
-      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm->t[4 * pair + 3], &full_bar[s], kblk, n0, tm->b_mn);
+      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES, &tm->t[second ? 6 : 4 * pair + 2], &full_bar[s], kblk, nb0, tm->b_mn);
+      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm->t[second ? 7 : 4 * pair + 3], &full_bar[s], kblk, nb0, tm->b_mn);
       if (++s == STAGES) { s = 0; ph ^= 1; }
     }
   }
@@ -519,7 +525,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
       uint32_t all_ok;
       asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, %2, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                    : "=r"(all_ok) : "r"((uint32_t)ok), "r"(1u + 2u * half) : "memory");
-      if (all_ok) epilogue_pass<64, 128>(epi, stage, th, mt, m0, n0 + n_shift, M, N + n_shift, cprev);
+      GemmEpilogue e = epi;
+      uint32_t ne0 = n0, Ne = N;
+      epi_side(e, ne0, Ne);
+      if (all_ok) epilogue_pass<64, 128>(e, stage, th, mt, m0, ne0 + n_shift, M, Ne + n_shift, cprev);
       if (BNT == 128) {
         if (half == 0) bar_arrive(2, 256);
         else if (w + gridDim.x < tiles * S) bar_arrive(4, 256);
@@ -537,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
 
 // ---- split-K second stage: C = epilogue(sum_s part[s]) in ascending split order ----------------
 __global__ void __launch_bounds__(256) k_splitk_reduce(const float* __restrict__ part, uint32_t S, uint32_t M, uint32_t N,
-                                                      GemmEpilogue epi, int vec) {
+                                                      GemmEpilogue epi, int vec, size_t stride) {
   dyb_grid_dep_sync();
   const size_t MN = (size_t)M * N;
   if (vec) {   // M % 4 == 0 and 16-byte aligned C / mask: four rows of one column per thread
@@ -550,7 +559,7 @@ __global__ void __launch_bounds__(256) k_splitk_reduce(const float* __restrict__
       for (uint32_t s0 = 0; s0 < S; s0 += 8) {
         float4 v[8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) if (s0 + k < S) v[k] = ld4_stream(part + (size_t)(s0 + k) * MN + e);
+        for (uint32_t k = 0; k < 8; ++k) if (s0 + k < S) v[k] = ld4_stream(part + (size_t)(s0 + k) * stride + e);
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k) {
           if (s0 + k >= S) break;
@@ -577,7 +586,7 @@ __global__ void __launch_bounds__(256) k_splitk_reduce(const float* __restrict__
   for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < MN; e += (size_t)gridDim.x * 256) {
     const uint32_t m = (uint32_t)(e % M), n = (uint32_t)(e / M);
     float acc = 0.f;
-    for (uint32_t s2 = 0; s2 < S; ++s2) acc += part[(size_t)s2 * MN + e];
+    for (uint32_t s2 = 0; s2 < S; ++s2) acc += part[(size_t)s2 * stride + e];
     const EpiRow row = epi_row(epi, m);
     float* dst = row.c + (size_t)row.ldc * n;
     if (epi.mode == EPI_STORE) *dst = acc;
@@ -1302,19 +1311,50 @@ int dyb200_tc_param2(dyb200_ctx* ctx, const float* src, uint32_t rows, const flo
   return rc;
 }
 
+// The kernels' limits on dynamic shared memory (function attributes are per device: the context remembers what it has set on its own).
+static int gemm_tc_limits(dyb200_ctx* ctx) {
+  if (ctx->func_attr_done & 1u) return DYB200_OK;
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
+  ctx->func_attr_done |= 1u;
+  return DYB200_OK;
+}
+// Whether `clusters` clusters of S one-tile CTAs are resident at once (asked for once per device, tile width and size).
+static bool cluster_fits(dyb200_ctx* ctx, uint32_t bn, uint32_t S, uint32_t clusters) {
+  int& mc = ctx->max_clusters[bn == 64 ? 0 : 1][S];
+  if (mc == 0) {
+    if (gemm_tc_limits(ctx)) return false;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(1, 1, S); cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = S;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    const cudaError_t e = bn == 64 ? cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<64, true>, &cfg) : cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<128, true>, &cfg);
+    if (e != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
+    mc = n > 0 ? n : -1;
+  }
+  return mc > 0 && clusters <= (uint32_t)mc;
+}
+
 int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const PackedOp* A, const PackedOp* B,
                           const GemmEpilogue& epi, uint32_t force_splits) {
   EncodeTiledFn enc;
   int rc = get_encoder(ctx, &enc);
   if (rc) return rc;
-  // (function attributes are per device: the context remembers what it has set on its own device)
-  if (!(ctx->func_attr_done & 1u)) {
-    DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    ctx->func_attr_done |= 1u;
-  }
+  if ((rc = gemm_tc_limits(ctx))) return rc;
   const uint32_t bn = tile_cols(N);
   TmapPack tm;
   memset(&tm, 0, sizeof(tm));
@@ -1368,13 +1408,6 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   // K splits as one thread-block cluster per tile (partial tiles meet in distributed shared memory) when every cluster
   // of the launch can be resident at once; dyb200_ctx_cluster_splitk(ctx, 0) keeps the workspace + second-kernel form.
   if (S > 1 && ctx->cluster_splitk) {
-    if (!(ctx->func_attr_done & 2u)) {
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-      ctx->func_attr_done |= 2u;
-    }
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = ctx->stream;
@@ -1383,22 +1416,9 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    auto fits = [&](uint32_t Sc) -> bool {
-      int& mc = ctx->max_clusters[bn == 64 ? 0 : 1][Sc];   // [tile width][cluster size], 0 = not asked yet on this device
-      if (mc == 0) {
-        cfg.gridDim = dim3(grid.x, grid.y, Sc);
-        attr[0].val.clusterDim.z = Sc;
-        int n = 0;
-        cudaError_t e = bn == 64 ? cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<64, true>, &cfg)
-                                 : cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<128, true>, &cfg);
-        if (e != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
-        mc = n > 0 ? n : -1;
-      }
-      return mc > 0 && grid.x * grid.y <= (uint32_t)mc;
-    };
     // (a smaller cluster size that fits was tried when the model's count does not - batch 64, 16 tiles: 7 instead of 8 -
     // and measured slower than the workspace form of the model's count: 4.73 vs 4.60 ms per step)
-    const uint32_t Sc = (S <= 8 && fits(S)) ? S : 0;
+    const uint32_t Sc = (S <= 8 && cluster_fits(ctx, bn, S, grid.x * grid.y)) ? S : 0;
     if (Sc) {
       kb_per_split = (kb_total + Sc - 1) / Sc;
       cfg.gridDim = dim3(grid.x, grid.y, Sc);
@@ -1431,13 +1451,6 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     if (tail_apart) tiles_run -= tail;
     // row blocks the persistent launch covers (all of them, unless the last ones run apart in every column of tiles)
     const uint32_t rows_run = tail_form == 2 ? grid.x - tail / grid.y : grid.x;
-    if (!(ctx->func_attr_done & 4u)) {
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-      ctx->func_attr_done |= 4u;
-    }
     // A long reduction whose tiles fill the last round badly (the deferred weight gradients: 256 tiles of 560 k-blocks on
     // 148 SMs = two rounds, the second 73 % full) is cut into Sp K splits as further work items of the same persistent
     // launch: 1024 items of 140 k-blocks make seven nearly full rounds.  The partial products go to a workspace and
@@ -1512,7 +1525,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       if (epi.split_m)
         vec = vec && epi.split_m % 4 == 0 && epi.ldc2 % 4 == 0 && aligned16(epi.C2) &&
               (epi.mode != EPI_ACCUM_MASK || (aligned16(epi.maskC2) && (!epi.maskc2_full || epi.maskc2_ld % 4 == 0)));
-      dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec);
+      dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec, (size_t)M * N);
       DYB_LAUNCHED(ctx);
     }
   }
@@ -1521,15 +1534,96 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
 
 // Second stage of a K split for callers outside this file: C = epilogue(sum over s of part[s]), the S partial products
 // (M x N each, leading dimension M) added in ascending order.
-int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi) {
-  int vec = M % 4 == 0 && epi.ldc % 4 == 0 && aligned16(epi.C) && epi.mode != EPI_GATES && (epi.mode != EPI_BIAS || aligned16(epi.bias)) &&
+int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi, size_t split_stride) {
+  int vec = M % 4 == 0 && split_stride % 4 == 0 && aligned16(part) && epi.ldc % 4 == 0 && aligned16(epi.C) && epi.mode != EPI_GATES && (epi.mode != EPI_BIAS || aligned16(epi.bias)) &&
             (epi.mode != EPI_ACCUM_MASK || (aligned16(epi.maskC) && (!epi.maskc_full || epi.maskc_ld % 4 == 0)));
   if (epi.split_m)
     vec = vec && epi.split_m % 4 == 0 && epi.ldc2 % 4 == 0 && aligned16(epi.C2) &&
           (epi.mode != EPI_ACCUM_MASK || (aligned16(epi.maskC2) && (!epi.maskc2_full || epi.maskc2_ld % 4 == 0)));
-  dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec);
+  dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec, split_stride ? split_stride : (size_t)M * N);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
+}
+
+// Two products with one left operand, C0 += A B0^T and C1 += A B1^T, as one over the columns of both (each side's columns rounded up to whole
+// tiles): a short product of its own is mostly pipeline fill and epilogue, and the few tiles of one leave SMs idle.  K splits as clusters
+// where they fit, or as work items of the persistent kernel with a second stage, by the estimates of dyb200_tc_splits.
+// us for both, as two launches / in one: 1024 x (128 + 256), K = 1600 38 / 22, 13000 99 / 69, 107000 538 / 378; 1200 x (200 + 300) x 1050 36 / 26;
+// 2048 x (512 + 512) x 4480 120 / 103.
+int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const PackedOp* B, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1) {
+  EncodeTiledFn enc;
+  int rc = get_encoder(ctx, &enc);
+  if (rc) return rc;
+  const uint32_t N0 = B[0].rows, N1 = B[1].rows, bn = N0 <= 64 && N1 <= 64 ? 64 : BN, split = round_up(N0, bn), N = split + N1;
+  const uint32_t tiles_m = (M + BM - 1) / BM, tiles = tiles_m * ((N + bn - 1) / bn), kb = round_up(A.K, 32) / 32;
+  TmapPack tm;
+  memset(&tm, 0, sizeof(tm));
+  tm.a_mn = tm.b_mn = 1;
+  tm.n_split = split;
+  DYB_CHECK_ARG(ctx, A.mn_major && B[0].mn_major && B[1].mn_major && !A.f16 && A.K == B[0].K && A.K == B[1].K && A.rows == M, "tensor GEMM: operands of a grouped product");
+  if ((rc = make_map_mn(ctx, enc, &tm.t[0], A.hi, M, A.K, A.pitch, BM)) || (rc = make_map_mn(ctx, enc, &tm.t[1], A.lo, M, A.K, A.pitch, BM))) return rc;
+  for (int q = 0; q < 2; ++q)
+    if ((rc = make_map_mn(ctx, enc, &tm.t[q ? 6 : 2], B[q].hi, B[q].rows, B[q].K, B[q].pitch, bn)) ||
+        (rc = make_map_mn(ctx, enc, &tm.t[q ? 7 : 3], B[q].lo, B[q].rows, B[q].K, B[q].pitch, bn))) return rc;
+  tm.t[4] = tm.t[0]; tm.t[5] = tm.t[1];
+  GemmEpilogue epi{EPI_ACCUM, C0, ldc0, nullptr, 0, 0.f, nullptr, 0, 0};
+  epi.n_split = split; epi.n_live = N0; epi.Cn = C1; epi.ldcn = ldc1;
+  const double flops = 2.0 * M * (double)(N0 + N1) * A.K, sms = (double)ctx->sm_count, t_kb = bn == 64 ? 0.40 : 0.66;
+  // clusters of S splits that are all resident, at least eight k-blocks each (shorter splits end sooner on an idle GPU, but hold several
+  // times the SMs: three language models of 256 units on three streams took 133 us a step with two k-blocks per split, 119 with eight)
+  uint32_t Sc = 0;
+  double cost = 1e30;
+  for (uint32_t S = 1; S <= 8 && (S == 1 || (kb / S >= 8 && ctx->cluster_splitk)); ++S) {
+    if (S == 1 ? tiles > (uint32_t)ctx->sm_count : (kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S || !cluster_fits(ctx, bn, S, tiles)) continue;
+    const double t = ((kb + S - 1) / S) * t_kb + 9.0;
+    if (t < cost) { cost = t; Sc = S; }
+  }
+  // work items of the persistent kernel
+  uint32_t Sp = 0;
+  for (uint32_t S = 1; S <= 64 && (S == 1 || kb / S >= 16); ++S) {
+    if ((kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S) continue;   // (no empty split)
+    const double t = ceil((double)tiles * S / sms) * (((kb + S - 1) / S) * t_kb + 3.0) + 6.0 + (S > 1 ? (S + 2) * 4.0e-6 * M * N / 5.0 + 5.0 : 0.0);
+    if (t < 0.97 * cost) { cost = t; Sp = S; }
+  }
+  if ((rc = gemm_tc_limits(ctx))) return rc;
+  const dim3 grid(tiles_m, (N + bn - 1) / bn, 1);
+  if (Sp == 0) {
+    GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
+    if (Sc == 1) {
+      dyb_launch(bn == 64 ? k_gemm_tc<64, false> : k_gemm_tc<128, false>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
+    } else {
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof(cfg));
+      cfg.gridDim = dim3(grid.x, grid.y, Sc); cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = ctx->stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = Sc;
+      cfg.attrs = attr; cfg.numAttrs = 1;
+      cudaLaunchKernelEx(&cfg, bn == 64 ? k_gemm_tc<64, true> : k_gemm_tc<128, true>, tm, M, N, kb, 0u, (kb + Sc - 1) / Sc, epi, ctx->dev_flags);
+    }
+    DYB_LAUNCHED(ctx);
+    return DYB200_OK;
+  }
+  GemmEpilogue pepi = epi;
+  float* part = nullptr;
+  if (Sp > 1) {   // partial products over the columns of both sides
+    void* pw;
+    if ((rc = dyb200_scratch(ctx, (size_t)Sp * M * N * sizeof(float), &pw))) return rc;
+    part = (float*)pw;
+    pepi = GemmEpilogue{EPI_STORE, part, M, nullptr, 0, 0.f, nullptr, 0, 0};
+    tm.store_map = M % 4 == 0;
+    if (tm.store_map && (rc = dyb200_tc_make_store_map(ctx, &tm.t[4], part, M, N, Sp, M, 64))) return rc;
+  }
+  {
+    GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
+    dyb_launch(bn == 64 ? k_gemm_persist<64> : k_gemm_persist<128>, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb, 0u, tiles_m, tiles, tiles_m > 16 ? 16u : 0u,
+               Sp, pepi, ctx->dev_flags);
+    DYB_LAUNCHED(ctx);
+  }
+  if (Sp == 1) return DYB200_OK;
+  const GemmEpilogue e0{EPI_ACCUM, C0, ldc0, nullptr, 0, 0.f, nullptr, 0, 0}, e1{EPI_ACCUM, C1, ldc1, nullptr, 0, 0.f, nullptr, 0, 0};
+  if ((rc = dyb200_splitk_reduce(ctx, part, Sp, M, N0, e0, (size_t)M * N))) return rc;
+  return dyb200_splitk_reduce(ctx, part + (size_t)M * split, Sp, M, N1, e1, (size_t)M * N);
 }
 
 bool dyb200_tc_eligible(uint32_t M, uint32_t N, double flops) {
@@ -1901,6 +1995,13 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
     for (int q = 0; q < jobs.n; ++q) ops[q] = dyb200_f16_op(jobs.job[q], true);
   }
   const PackedOp& A = ops[0];
+  if (!A.f16 && w->N[1]) {
+    int rc = dyb200_tc_gemm_packed2(ctx, w->M, A, ops + 1, C0, ldc0, C1, ldc1);
+    if (rc) return rc;
+    w->k = 0;
+    w->kb = 0;
+    return DYB200_OK;
+  }
   for (int j = 0; j < 2; ++j) {
     if (w->N[j] == 0) continue;
     const PackedOp& B = ops[1 + j];
