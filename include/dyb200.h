@@ -165,7 +165,7 @@ int dyb200_pickneglogsoftmax_bwd(DYB200_BWD_ARGS); /* dynet/nodes-pickneglogsoft
  * dyb200_pickneglogsoftmax_bwd into a zeroed d(x) followed by dyb200_affine_transform_bwd for i = 0, 1, 2
  * (dynet/nodes-pickneglogsoftmax.cc:120-146, dynet/nodes-affinetransform.cc:120-157), but d(x) is never stored as a
  * tensor: one pass over x writes it as the split operands of the two products (dR += d h^T, dh += R^T d) and as
- * per-tile column sums for db.  From 24 GFLOP on the operands are fp16 pairs (2 x 11 bits) with one scale per row of dR and one per
+ * per-tile column sums for db.  Large products (dyb200_gemm) have operands of fp16 pairs (2 x 11 bits) with one scale per row of dR and one per
  * column of dh: an error is relative to |row of d| |row of h| and |row of R^T| |column of d|, whatever the probabilities and dEdf of the
  * other words and columns.  x: Dim({V}, n) logits; h: Dim({H}, n); R: Dim({V, H}); dEdf: n loss gradients; aux_mem:
  * the PickNegLogSoftmax node's aux_mem as left by its forward call; dR, db, dh are accumulated into.  dx_scratch
@@ -402,8 +402,8 @@ int dyb200_trainer_update(int rule, float* params, float* grads, float* state0, 
 
 /* ---- GEMM used by the LSTM gates (dynet/matrix-multiply.h:16-37, :97-117, :162-180) ----
  * C[M x N] (+)= op(A) * op(B), column-major, fp32 in/out.  Up to 32 columns, and with a narrow side and a long one, on
- * the CUDA cores in fp32; else on the tensor pipe as three products of TF32 pairs or, from 24 GFLOP on, of fp16 pairs whose rows
- * of op(A) and columns of op(B) are scaled by their largest value (2 x 11 bits either way); shapes too small for that on the
+ * the CUDA cores in fp32; else on the tensor pipe as three products of TF32 pairs or, from 24 GFLOP on (8 with K >= 256), of fp16
+ * pairs whose rows of op(A) and columns of op(B) are scaled by their largest value (2 x 11 bits either way); shapes too small for that on the
  * CUDA cores.  transA/transB as in BLAS. */
 #define DYB200_GEMM_A_IS_PARAM 1u /* flags: A is a parameter matrix (see dyb200_ctx_param_cache) */
 int dyb200_gemm(int transA, int transB, uint32_t M, uint32_t N, uint32_t K, const float* A,
