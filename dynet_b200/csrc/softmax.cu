@@ -750,6 +750,11 @@ __global__ void __launch_bounds__(kRQ * kRLanes) k_row_quads(const float* __rest
       v[k] = in ? ld4(p + k * step) : zero;
       d[k] = in ? ld4(q + k * step) : zero;
     }
+    if (live && threadIdx.x % kRQ == 0) {   // (the lines that are added to are on their way into L2 while the row sums are formed)
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (cj + kRLanes * k < cols) asm volatile("prefetch.global.L2 [%0];" ::"l"(o + k * step));
+    }
 #pragma unroll
     for (int k = 0; k < NV; ++k) z = make_float4(fmaf(v[k].x, d[k].x, z.x), fmaf(v[k].y, d[k].y, z.y), fmaf(v[k].z, d[k].z, z.z), fmaf(v[k].w, d[k].w, z.w));
     z = quad_reduce(z, sm[0], false);
