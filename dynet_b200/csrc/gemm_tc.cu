@@ -53,7 +53,10 @@ __device__ __forceinline__ void unscale_tile(const TmapPack& tm, float (&sum)[64
 // its own shared memory, and CTA r adds all partial tiles of its 1 / S of the columns through distributed shared memory, in
 // split order, and runs the epilogue on that slice - no workspace round trip and no second kernel.
 // F16: the operands are fp16 pairs (tc_dev.cuh) in k-blocks of 64; an accumulator is D1 | D2, 2 BNT columns of TMEM.
-template <int BNT, bool CLUSTER, bool F16 = false>
+// TWO: two right operands side by side, each with its own destination (TmapPack::n_split).  A variant of its own, since the choice of the
+// destination costs the epilogue registers; the persistent kernel leaves it to k_splitk_reduce: with it in its epilogue, its three
+// products in a step of a language model of 128 units (vocabulary 1901, 10560 tokens) took 60 us each instead of 38.
+template <int BNT, bool CLUSTER, bool F16 = false, bool TWO = false>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__ TmapPack tm, uint32_t M, uint32_t N,
                                                          uint32_t kb0, uint32_t kb1, uint32_t kb_per_split,
                                                          GemmEpilogue epi, uint32_t* flags) {
@@ -103,8 +106,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
   if (warp == 0) {
     if (elect_one()) {
       uint32_t s = 0, ph = 0;
-      const bool second = tm.n_split && n0 >= tm.n_split;
-      const uint32_t nb0 = second ? n0 - tm.n_split : n0;
+      const bool second = TWO && n0 >= tm.n_split;
+      const uint32_t nb0 = second ? n0 - tm.n_split : n0, tb = second ? 6u : 2u;
       for (uint32_t it = 0; it < total; ++it) {
         if (!mbar_wait(&empty_bar[s], ph ^ 1)) { atomicOr(flags, DYB200_FLAG_WAIT_TIMEOUT); break; }
         const uint32_t pair = it < ks.n0 ? 0 : 1, kblk = pair ? ks.b1 + (it - ks.n0) : ks.b0 + it;
@@ -112,8 +115,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
         mbar_expect_tx(&full_bar[s], STAGE_TX);
         load_a_tile<EL>(st, &tm.t[4 * pair + 0], &full_bar[s], kblk, m0, tm.a_mn);
         load_a_tile<EL>(st + TILE_BYTES, &tm.t[4 * pair + 1], &full_bar[s], kblk, m0, tm.a_mn);
-        load_b_tile<EL>(st + 2 * TILE_BYTES, &tm.t[second ? 6 : 4 * pair + 2], &full_bar[s], kblk, nb0, tm.b_mn);
-        load_b_tile<EL>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[second ? 7 : 4 * pair + 3], &full_bar[s], kblk, nb0, tm.b_mn);
+        load_b_tile<EL>(st + 2 * TILE_BYTES, &tm.t[4 * pair + tb], &full_bar[s], kblk, nb0, tm.b_mn);
+        load_b_tile<EL>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[4 * pair + tb + 1], &full_bar[s], kblk, nb0, tm.b_mn);
         if (++s == STAGES) { s = 0; ph ^= 1; }
       }
     }
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
       for (int j = 0; j < 64; ++j) col[(size_t)j * BM] = sum[j];
     }
     uint32_t ne0 = n0, Ne = N;
-    epi_side(epi, ne0, Ne);
+    if (TWO) epi_side(epi, ne0, Ne);
     uint32_t all_ok;
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, 1, 256, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(all_ok) : "r"((uint32_t)ok) : "memory");
@@ -333,7 +336,7 @@ __device__ __noinline__ void persist_producer(const TmapPack* tm, unsigned char*
     persist_tile_coords(tile, tiles_m, tiles_n, gm, mt, nt);
     const uint32_t m0 = mt * BM, n0 = nt * BNT;
     const bool second = tm->n_split && n0 >= tm->n_split;
-    const uint32_t nb0 = second ? n0 - tm->n_split : n0;
+    const uint32_t nb0 = second ? n0 - tm->n_split : n0, tb = second ? 6u : 2u;
     for (uint32_t g = 0; g < ks.n0 + ks.n1; ++g) {
       if (!mbar_wait(&empty_bar[s], ph ^ 1)) { fail = true; break; }
       const uint32_t pair = g < ks.n0 ? 0 : 1, kblk = pair ? ks.b1 + (g - ks.n0) : ks.b0 + g;
@@ -341,8 +344,8 @@ __device__ __noinline__ void persist_producer(const TmapPack* tm, unsigned char*
       mbar_expect_tx(&full_bar[s], STAGE_TX);
       load_a_tile<F16 ? 64 : 32>(st, &tm->t[4 * pair + 0], &full_bar[s], kblk, m0, tm->a_mn);
       load_a_tile<F16 ? 64 : 32>(st + TILE_BYTES, &tm->t[4 * pair + 1], &full_bar[s], kblk, m0, tm->a_mn);
-      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES, &tm->t[second ? 6 : 4 * pair + 2], &full_bar[s], kblk, nb0, tm->b_mn);
-      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm->t[second ? 7 : 4 * pair + 3], &full_bar[s], kblk, nb0, tm->b_mn);
+      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES, &tm->t[4 * pair + tb], &full_bar[s], kblk, nb0, tm->b_mn);
+      load_b_tile<F16 ? 64 : 32>(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm->t[4 * pair + tb + 1], &full_bar[s], kblk, nb0, tm->b_mn);
       if (++s == STAGES) { s = 0; ph ^= 1; }
     }
   }
@@ -525,10 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
       uint32_t all_ok;
       asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, %2, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                    : "=r"(all_ok) : "r"((uint32_t)ok), "r"(1u + 2u * half) : "memory");
-      GemmEpilogue e = epi;
-      uint32_t ne0 = n0, Ne = N;
-      epi_side(e, ne0, Ne);
-      if (all_ok) epilogue_pass<64, 128>(e, stage, th, mt, m0, ne0 + n_shift, M, Ne + n_shift, cprev);
+      if (all_ok) epilogue_pass<64, 128>(epi, stage, th, mt, m0, n0 + n_shift, M, N + n_shift, cprev);
       if (BNT == 128) {
         if (half == 0) bar_arrive(2, 256);
         else if (w + gridDim.x < tiles * S) bar_arrive(4, 256);
@@ -1322,6 +1322,10 @@ static int gemm_tc_limits(dyb200_ctx* ctx) {
   DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
   DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
   DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
@@ -1569,20 +1573,22 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   GemmEpilogue epi{EPI_ACCUM, C0, ldc0, nullptr, 0, 0.f, nullptr, 0, 0};
   epi.n_split = split; epi.n_live = N0; epi.Cn = C1; epi.ldcn = ldc1;
   const double flops = 2.0 * M * (double)(N0 + N1) * A.K, sms = (double)ctx->sm_count, t_kb = bn == 64 ? 0.40 : 0.66;
-  // clusters of S splits that are all resident, at least eight k-blocks each (shorter splits end sooner on an idle GPU, but hold several
-  // times the SMs: three language models of 256 units on three streams took 133 us a step with two k-blocks per split, 119 with eight)
+  // one tile per CTA (in waves: 2816 x (704 + 704) over 35 columns 22 us, 29 as work items of the persistent kernel), or clusters of S splits
+  // that are all resident, at least eight k-blocks each (shorter splits end sooner on an idle GPU, but hold several times the SMs: three
+  // language models of 256 units on three streams took 133 us a step with two k-blocks per split, 119 with eight)
   uint32_t Sc = 0;
   double cost = 1e30;
   for (uint32_t S = 1; S <= 8 && (S == 1 || (kb / S >= 8 && ctx->cluster_splitk)); ++S) {
-    if (S == 1 ? tiles > (uint32_t)ctx->sm_count : (kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S || !cluster_fits(ctx, bn, S, tiles)) continue;
-    const double t = ((kb + S - 1) / S) * t_kb + 9.0;
+    if (S > 1 && ((kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S || !cluster_fits(ctx, bn, S, tiles))) continue;
+    const double t = (S == 1 ? ceil(tiles / sms) : 1.0) * (((kb + S - 1) / S) * t_kb + 9.0);
     if (t < cost) { cost = t; Sc = S; }
   }
-  // work items of the persistent kernel
+  // work items of the persistent kernel, as partial products and one sum per side (512 x (32 + 128) over 10560 columns: 19 us and 2 x 4, two
+  // launches 29 and 35; 1024 x (128 + 256) over 107000: 369 us and 2 x 3, two launches 537)
   uint32_t Sp = 0;
-  for (uint32_t S = 1; S <= 64 && (S == 1 || kb / S >= 16); ++S) {
+  for (uint32_t S = 2; S <= 64 && kb / S >= 16; ++S) {
     if ((kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S) continue;   // (no empty split)
-    const double t = ceil((double)tiles * S / sms) * (((kb + S - 1) / S) * t_kb + 3.0) + 6.0 + (S > 1 ? (S + 2) * 4.0e-6 * M * N / 5.0 + 5.0 : 0.0);
+    const double t = ceil((double)tiles * S / sms) * (((kb + S - 1) / S) * t_kb + 3.0) + 6.0 + (S + 2) * 4.0e-6 * M * N / 5.0 + 5.0;
     if (t < 0.97 * cost) { cost = t; Sp = S; }
   }
   if ((rc = gemm_tc_limits(ctx))) return rc;
@@ -1590,7 +1596,7 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   if (Sp == 0) {
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
     if (Sc == 1) {
-      dyb_launch(bn == 64 ? k_gemm_tc<64, false> : k_gemm_tc<128, false>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
+      dyb_launch(bn == 64 ? k_gemm_tc<64, false, false, true> : k_gemm_tc<128, false, false, true>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
     } else {
       cudaLaunchConfig_t cfg;
       memset(&cfg, 0, sizeof(cfg));
@@ -1599,28 +1605,24 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = Sc;
       cfg.attrs = attr; cfg.numAttrs = 1;
-      cudaLaunchKernelEx(&cfg, bn == 64 ? k_gemm_tc<64, true> : k_gemm_tc<128, true>, tm, M, N, kb, 0u, (kb + Sc - 1) / Sc, epi, ctx->dev_flags);
+      cudaLaunchKernelEx(&cfg, bn == 64 ? k_gemm_tc<64, true, false, true> : k_gemm_tc<128, true, false, true>, tm, M, N, kb, 0u, (kb + Sc - 1) / Sc, epi, ctx->dev_flags);
     }
     DYB_LAUNCHED(ctx);
     return DYB200_OK;
   }
-  GemmEpilogue pepi = epi;
-  float* part = nullptr;
-  if (Sp > 1) {   // partial products over the columns of both sides
-    void* pw;
-    if ((rc = dyb200_scratch(ctx, (size_t)Sp * M * N * sizeof(float), &pw))) return rc;
-    part = (float*)pw;
-    pepi = GemmEpilogue{EPI_STORE, part, M, nullptr, 0, 0.f, nullptr, 0, 0};
-    tm.store_map = M % 4 == 0;
-    if (tm.store_map && (rc = dyb200_tc_make_store_map(ctx, &tm.t[4], part, M, N, Sp, M, 64))) return rc;
-  }
+  // partial products over the columns of both sides
+  void* pw;
+  if ((rc = dyb200_scratch(ctx, (size_t)Sp * M * N * sizeof(float), &pw))) return rc;
+  float* const part = (float*)pw;
+  const GemmEpilogue pepi{EPI_STORE, part, M, nullptr, 0, 0.f, nullptr, 0, 0};
+  tm.store_map = M % 4 == 0;
+  if (tm.store_map && (rc = dyb200_tc_make_store_map(ctx, &tm.t[4], part, M, N, Sp, M, 64))) return rc;
   {
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
     dyb_launch(bn == 64 ? k_gemm_persist<64> : k_gemm_persist<128>, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb, 0u, tiles_m, tiles, tiles_m > 16 ? 16u : 0u,
                Sp, pepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);
   }
-  if (Sp == 1) return DYB200_OK;
   const GemmEpilogue e0{EPI_ACCUM, C0, ldc0, nullptr, 0, 0.f, nullptr, 0, 0}, e1{EPI_ACCUM, C1, ldc1, nullptr, 0, 0.f, nullptr, 0, 0};
   if ((rc = dyb200_splitk_reduce(ctx, part, Sp, M, N0, e0, (size_t)M * N))) return rc;
   return dyb200_splitk_reduce(ctx, part + (size_t)M * split, Sp, M, N1, e1, (size_t)M * N);
