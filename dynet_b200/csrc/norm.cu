@@ -442,12 +442,14 @@ struct LnDg {
   }
 };
 // Gain gradient of long columns that fit a CTA's registers: statistics and terms from one read of x and dy (statistics, then the terms as a batch
-// reduction that reads x again, took 17 us for 1024 columns of 4096, this 10), the CTA's columns summed in ascending order and left as
-// one partial sum per CTA.
-constexpr uint32_t kLnDgRows = 1024;
-__global__ void __launch_bounds__(kBlock) k_layer_norm_dg(const float* __restrict__ x, const float* __restrict__ dy, uint32_t n, size_t ncols, float* __restrict__ partial) {
+// reduction that reads x again, took 17 us for 1024 columns of 4096, this 10), the CTA's columns summed in ascending order, the eight
+// CTAs of a cluster through their shared memory (an eighth of the rows each, in rank order) and left as one partial sum per cluster: 0.7 MB of
+// workspace at 4096 rows.  With one per CTA, 5.6 MB, a context's first sweep of the normalisations waited 0.6 ms for the allocation.
+constexpr uint32_t kLnDgRows = 1024, kLnDgCluster = 8;
+__global__ void __launch_bounds__(kBlock) __cluster_dims__(kLnDgCluster, 1, 1) k_layer_norm_dg(const float* __restrict__ x, const float* __restrict__ dy, uint32_t n, size_t ncols, float* __restrict__ partial) {
   dyb_grid_dep_sync();
   __shared__ float red[32];
+  __shared__ float4 sums[kBlock * kVec];
   const uint32_t n4 = n / 4;
   float4 acc[kVec];
 #pragma unroll
@@ -474,9 +476,23 @@ __global__ void __launch_bounds__(kBlock) k_layer_norm_dg(const float* __restric
   }
 #pragma unroll
   for (int k = 0; k < kVec; ++k) {
-    const uint32_t i = threadIdx.x + kBlock * k;
-    if (i < n4) st4(partial + (size_t)blockIdx.x * n + 4 * i, acc[k]);
+    sums[threadIdx.x + kBlock * k] = acc[k];
   }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const uint32_t per = (n4 + kLnDgCluster - 1) / kLnDgCluster, i0 = (blockIdx.x % kLnDgCluster) * per, i1 = min(i0 + per, n4);
+  for (uint32_t i = i0 + threadIdx.x; i < i1; i += kBlock) {
+    float4 v[kLnDgCluster];
+#pragma unroll
+    for (uint32_t r = 0; r < kLnDgCluster; ++r) {
+      uint32_t src;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(src) : "r"((uint32_t)__cvta_generic_to_shared(&sums[i])), "r"(r));
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[r].x), "=f"(v[r].y), "=f"(v[r].z), "=f"(v[r].w) : "r"(src) : "memory");
+    }
+#pragma unroll
+    for (uint32_t r = 1; r < kLnDgCluster; ++r) { v[0].x += v[r].x; v[0].y += v[r].y; v[0].z += v[r].z; v[0].w += v[r].w; }
+    st4(partial + (size_t)(blockIdx.x / kLnDgCluster) * n + 4 * i, v[0]);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // (nobody leaves while its sums are read)
 }
 // Gain gradient of a small layer norm in one launch: every CTA forms the statistics of all columns (a warp per column; at most 64 KB, from
 // L2) and sums its 128 rows over them.
@@ -719,12 +735,12 @@ int dyb200_layer_norm_bwd(DYB200_BWD_ARGS) {
     return DYB200_OK;
   }
   if (cached && n >= kLnDgRows && aligned16(dEdf->v)) {
-    const size_t per = (ncols + 3 * ctx->sm_count - 1) / (3 * ctx->sm_count), grid = (ncols + per - 1) / per;   // (three CTAs per SM)
+    const size_t per = (ncols + 3 * ctx->sm_count - 1) / (3 * ctx->sm_count), clusters = ((ncols + per - 1) / per + kLnDgCluster - 1) / kLnDgCluster;   // (three CTAs per SM)
     void* part;
-    if ((rc = dyb200_scratch(ctx, grid * n * sizeof(float), &part))) return rc;
-    dyb_launch(k_layer_norm_dg, (unsigned)grid, kBlock, 0, ctx, xs[0].v, dEdf->v, (uint32_t)n, ncols, (float*)part);
+    if ((rc = dyb200_scratch(ctx, clusters * n * sizeof(float), &part))) return rc;
+    dyb_launch(k_layer_norm_dg, (unsigned)(clusters * kLnDgCluster), kBlock, 0, ctx, xs[0].v, dEdf->v, (uint32_t)n, ncols, (float*)part);
     DYB_LAUNCHED(ctx);
-    dyb_launch(k_batch_reduce_final, (unsigned)((n + 31) / 32), 256, 0, ctx, (const float*)part, (uint32_t)grid, n, dEdxi->v);
+    dyb_launch(k_batch_reduce_final, (unsigned)((n + 31) / 32), 256, 0, ctx, (const float*)part, (uint32_t)clusters, n, dEdxi->v);
     DYB_LAUNCHED(ctx);
     return DYB200_OK;
   }
