@@ -44,6 +44,13 @@ int dyb200_scratch_begin(dyb200_ctx* ctx) {
 int dyb200_scratch(dyb200_ctx* ctx, size_t bytes, void** out) {
   size_t off = (ctx->scratch_off + 255) & ~(size_t)255;
   if (bytes == 0) bytes = 256;
+  if (!ctx->scratch && ctx->n_overflow == 0) {
+    // A context's first block is the arena itself, with the room that dyb200_scratch_begin would add at the next call: a block of the exact size
+    // cost that call a synchronisation, a free and a second allocation (first pass of a normalisation sweep 0.3 - 0.5 ms of them).
+    const size_t want = bytes + (bytes >> 2) + (1u << 20);
+    if (cudaMalloc(&ctx->scratch, want) == cudaSuccess) ctx->scratch_bytes = want;
+    else { cudaGetLastError(); ctx->scratch = nullptr; }   // (the exact size below may still fit)
+  }
   if (off + bytes <= ctx->scratch_bytes) {
     *out = (char*)ctx->scratch + off;
   } else {
