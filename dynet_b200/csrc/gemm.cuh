@@ -48,6 +48,7 @@ struct GemmEpilogue {
   const float* hmask = nullptr; uint32_t hmask_ld = 0; int hmask_full = 0;
   // Two right operands side by side (TmapPack::n_split): columns [0, n_live) belong to C, those from n_split on to Cn, the ones between do not exist.
   uint32_t n_split = 0, n_live = 0; float* Cn = nullptr; uint32_t ldcn = 0;
+  const uint32_t* only_if = nullptr;   // (dyb200_tc_gemm_packed2) a device word: the kernel runs where it is not zero
 };
 #ifdef __CUDACC__
 // The destination of a tile whose first column is n0 (a tile lies on one side): C, n0 and the end of its columns N.
@@ -149,8 +150,14 @@ enum F16Scale { F16_LINE = 0, F16_ELEM = 1 };
 // src_lo: the source is a pair of TF32 planes, src the hi one (null: plain fp32).
 constexpr int kF16MaxJobs = 3;
 struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; const float* src_lo = nullptr;
-  uint32_t perm_H = 0; };   // perm_H (F16_ELEM): positions are gate rows q perm_H + u, written interleaved as dyb200_tc_param_gates does
-struct F16Jobs { F16Job job[kF16MaxJobs]; int n; uint32_t start[kF16MaxJobs + 1]; };   // start: units of work before each job (set for a launch)
+  uint32_t perm_H = 0;        // (F16_ELEM) positions are gate rows q perm_H + u, written interleaved as dyb200_tc_param_gates does
+  uint32_t* low = nullptr; };   // (F16_ELEM) a word per position, see F16Jobs::wide
+// wide: becomes 1 where the values of a position span more than a pair holds: of its blocks of eight lines that are not all zero, one's largest
+// value lies more than 2^kF16Span below the position's (jobs with `low` words).  words: scale and low words and the flag of all
+// jobs, cleared at once (null: each job's scale words by themselves).
+constexpr int kF16Span = 24;
+struct F16Jobs { F16Job job[kF16MaxJobs]; int n; uint32_t start[kF16MaxJobs + 1];   // start: units of work before each job (set for a launch)
+  uint32_t* wide = nullptr; uint32_t* words = nullptr; size_t n_words = 0; };
 // Planes and scale words for a job from the scratch arena; dyb200_f16_pack fills those of up to three jobs in one pass each.
 int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
@@ -194,11 +201,15 @@ uint32_t dyb200_tc_splits(const dyb200_ctx* ctx, uint32_t M, uint32_t N, uint32_
 int dyb200_tc_param2(dyb200_ctx* ctx, const float* src, uint32_t rows, const float* src2, uint32_t rows2, uint32_t ld,
                      bool k_is_fast, uint32_t K, PackedOp* out);
 // force_splits > 0: that many K splits (normalised so that no split is empty) instead of the cost model's choice.
+// unless (products of the pair kernel): a device word; where it is not zero the product is left out.
 int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const PackedOp* A, const PackedOp* B,
-                          const GemmEpilogue& epi, uint32_t force_splits = 0);
-int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi, size_t split_stride = 0);
-// C0 += A B0^T and C1 += A B1^T in one launch (TF32 planes, all MN-major; dWx and dWh of a layer).
-int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const PackedOp* B, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1);
+                          const GemmEpilogue& epi, uint32_t force_splits = 0, const uint32_t* unless = nullptr);
+int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi, size_t split_stride = 0,
+                         const uint32_t* unless = nullptr);
+// C0 += A B0^T and C1 += A B1^T in one launch (TF32 planes, all MN-major; dWx and dWh of a layer).  only_if: a device word; where it is zero
+// the launch does nothing (then B[1].rows may be 0, and the launch is one tile per CTA).
+int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const PackedOp* B, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1,
+                           const uint32_t* only_if = nullptr);
 // Tiling of the backward recurrence of an LSTM layer (dx_t, dh_{t-1} += [Wx; Wh]^T dgates_t), shared by the per-step call
 // and the sequence kernel so that both add the same partial sums: tile width, batch-column blocks per CTA of the sequence
 // kernel (1 or 2) and K splits.  False when the shape does not suit the sequence kernel (the per-step call then lets the

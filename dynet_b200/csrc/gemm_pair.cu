@@ -41,6 +41,7 @@ struct PairArgs {
   uint32_t M, N, kb, tiles_m, tiles_n, gm, S;
   float* C; uint32_t ldc; const float* bias; int accumulate;   // (splits: C = the partial products, split z at columns z N)
   uint32_t* flags;
+  const uint32_t* unless;   // a device word: where it is not zero there is nothing to do (null: always run)
 };
 
 // This CTA's tile, its bytes reported to the barrier of the leader (both CTAs' loads complete one phase of it).
@@ -154,6 +155,10 @@ __device__ __forceinline__ void pair_issue(const TmapPack* tm, const PairArgs* a
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_constant__ TmapPack tm, const __grid_constant__ PairArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (a.unless) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (*(const volatile uint32_t*)a.unless) return;   // (the same in every CTA)
+  }
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];   // acc: 0 = D1, 1 = D2
   __shared__ uint32_t tmem_base_slot;
@@ -310,7 +315,7 @@ bool dyb200_pair_takes(const dyb200_ctx* ctx, uint32_t M, uint32_t N, const Gemm
 }
 
 // tm: the operand maps and scale words of dyb200_tc_gemm_packed (boxes of 128 rows x 64 k); K in k-blocks of 64.
-int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint32_t kb, double flops, const GemmEpilogue& epi) {
+int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint32_t kb, double flops, const GemmEpilogue& epi, const uint32_t* unless) {
   if (!(ctx->func_attr_done & (1u << 24))) {
     DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PAIR_BYTES));
     ctx->func_attr_done |= 1u << 24;
@@ -318,7 +323,7 @@ int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint
   const uint32_t pairs = (uint32_t)ctx->sm_count / 2;
   PairArgs a;
   memset(&a, 0, sizeof(a));
-  a.M = M; a.N = N; a.kb = kb; a.flags = ctx->dev_flags;
+  a.M = M; a.N = N; a.kb = kb; a.flags = ctx->dev_flags; a.unless = unless;
   a.tiles_m = (M + kPairTile - 1) / kPairTile; a.tiles_n = (N + kPairTile - 1) / kPairTile; a.gm = 8;
   const uint32_t tiles = a.tiles_m * a.tiles_n;
   // K splits: rounds of the pairs x (k-blocks x 1.05 us + 2 us between items), and for more than one split the second stage, (S + 2) M N
@@ -349,5 +354,5 @@ int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint
   GemmProfScope scope(ctx, flops, 2, M, N, kb * 64, (uint32_t)epi.mode);
   dyb_launch(k_gemm_pair, dim3(2 * pairs), kPairThreads, SMEM_PAIR_BYTES, ctx, *tm, a);
   DYB_LAUNCHED(ctx);
-  return a.S > 1 ? dyb200_splitk_reduce(ctx, e.C, a.S, M, N, epi) : DYB200_OK;
+  return a.S > 1 ? dyb200_splitk_reduce(ctx, e.C, a.S, M, N, epi, 0, unless) : DYB200_OK;
 }

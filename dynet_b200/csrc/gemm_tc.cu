@@ -61,6 +61,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
                                                          uint32_t kb0, uint32_t kb1, uint32_t kb_per_split,
                                                          GemmEpilogue epi, uint32_t* flags) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (the wait comes after the prologue, below)
+  if (TWO && !CLUSTER && epi.only_if) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!*(const volatile uint32_t*)epi.only_if) return;   // (the same in every CTA)
+  }
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
@@ -546,8 +550,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_const
 
 // ---- split-K second stage: C = epilogue(sum_s part[s]) in ascending split order ----------------
 __global__ void __launch_bounds__(256) k_splitk_reduce(const float* __restrict__ part, uint32_t S, uint32_t M, uint32_t N,
-                                                      GemmEpilogue epi, int vec, size_t stride) {
+                                                      GemmEpilogue epi, int vec, size_t stride, const uint32_t* unless) {
   dyb_grid_dep_sync();
+  if (unless && *(const volatile uint32_t*)unless) return;
   const size_t MN = (size_t)M * N;
   if (vec) {   // M % 4 == 0 and 16-byte aligned C / mask: four rows of one column per thread
     const size_t MN4 = MN / 4;
@@ -777,43 +782,46 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const __grid_constant__ F16J
   const F16Job& j = jobs.job[z];
   const bool vec = (j.ld & 3) == 0 && aligned16(j.src);
   const F16Units us = f16_max_units(j);
-  if (j.mode == F16_ELEM) {   // four positions per thread; short lines: groups of threads take every groups-th line and meet in shared memory
-    __shared__ uint32_t top[1024];
+  if (j.mode == F16_ELEM) {   // four positions per thread; short lines: groups of threads with lines of their own meet in shared memory
+    __shared__ uint32_t top[1024], bot[1024];
     const uint32_t q = us.groups > 1 ? (j.n + 3) / 4 : 256u, grp = threadIdx.x / q, e = 4 * ((unit % us.x) * 256 + threadIdx.x % q);
-    const uint32_t l0 = unit / us.x * kMaxLines * us.groups + grp;
+    const uint32_t l0 = (unit / us.x * us.groups + grp) * kMaxLines;
     const bool live = grp < us.groups && e < j.n;
-    uint32_t m[4] = {0, 0, 0, 0};
+    uint32_t m[4] = {0, 0, 0, 0}, low[4] = {0, 0, 0, 0};   // low: ~(the smallest of the blocks' maxima that are not zero)
     if (live) {
-      for (uint32_t b = 0; b < kMaxLines && l0 + b * us.groups < j.lines; b += 8) {
+      for (uint32_t b = 0; b < kMaxLines && l0 + b < j.lines; b += 8) {
         float4 v[8];
-        const uint32_t l = l0 + b * us.groups;
+        const uint32_t l = l0 + b;
         const float* p = j.src + (size_t)j.ld * l;
-        const size_t next = (size_t)j.ld * us.groups;
-        if (vec && e + 4 <= j.n && l + 7 * us.groups < j.lines) {
+        if (vec && e + 4 <= j.n && l + 7 < j.lines) {
 #pragma unroll
-          for (uint32_t k = 0; k < 8; ++k) v[k] = ld4(p + k * next + e);
+          for (uint32_t k = 0; k < 8; ++k) v[k] = ld4(p + (size_t)j.ld * k + e);
         } else {
 #pragma unroll
-          for (uint32_t k = 0; k < 8; ++k) v[k] = l + k * us.groups < j.lines ? f16_load4(p + k * next, e, j.n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (uint32_t k = 0; k < 8; ++k) v[k] = l + k < j.lines ? f16_load4(p + (size_t)j.ld * k, e, j.n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k) {
-          m[0] = max(m[0], finite_mag(v[k].x)); m[1] = max(m[1], finite_mag(v[k].y)); m[2] = max(m[2], finite_mag(v[k].z)); m[3] = max(m[3], finite_mag(v[k].w));
+          w[0] = max(w[0], finite_mag(v[k].x)); w[1] = max(w[1], finite_mag(v[k].y)); w[2] = max(w[2], finite_mag(v[k].z)); w[3] = max(w[3], finite_mag(v[k].w));
         }
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) { m[i] = max(m[i], w[i]); if (w[i]) low[i] = max(low[i], ~w[i]); }
       }
     }
     if (us.groups > 1) {
-      for (uint32_t i = threadIdx.x; i < 1024; i += 256) top[i] = 0;
+      for (uint32_t i = threadIdx.x; i < 1024; i += 256) top[i] = bot[i] = 0;
       __syncthreads();
       if (live) {
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) atomicMax(top + e + i, m[i]);
+        for (uint32_t i = 0; i < 4; ++i) { atomicMax(top + e + i, m[i]); if (j.low) atomicMax(bot + e + i, low[i]); }
       }
       __syncthreads();
-      for (uint32_t i = threadIdx.x; i < j.n; i += 256) atomicMax(j.scale + i, top[i]);
+      for (uint32_t i = threadIdx.x; i < j.n; i += 256) { atomicMax(j.scale + i, top[i]); if (j.low) atomicMax(j.low + i, bot[i]); }
     } else if (live) {
 #pragma unroll
-      for (uint32_t i = 0; i < 4; ++i) if (e + i < j.n) atomicMax(j.scale + e + i, m[i]);
+      for (uint32_t i = 0; i < 4; ++i)
+        if (e + i < j.n) { atomicMax(j.scale + e + i, m[i]); if (j.low) atomicMax(j.low + e + i, low[i]); }
     }
     return;
   }
@@ -915,6 +923,13 @@ __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jo
   for (uint32_t k = 0; k < 4; ++k) {
     if (line[k] >= j.lines) break;
     float4 s;
+    if (j.low && line[k] == 0) {   // (a position's words are looked at where its first line is split)
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t p = min(e[k] + i, j.n - 1), low = j.low[p];
+        if (low && (j.scale[p] >> 23) > ((~low) >> 23) + kF16Span) *jobs.wide = 1;
+      }
+    }
     if (j.mode == F16_ELEM) {
       const uint32_t top = j.n - 1;
       if (e[k] + 4 <= j.n) {
@@ -1113,10 +1128,11 @@ int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t l
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
   if (jobs->n == 0) return DYB200_OK;
   jobs->start[0] = 0;
+  if (jobs->words) DYB_CUDA(ctx, cudaMemsetAsync(jobs->words, 0, jobs->n_words * sizeof(uint32_t), ctx->stream));
   for (int k = 0; k < jobs->n; ++k) {
     const F16Job& j = jobs->job[k];
     const bool one_store = j.mode == F16_LINE && j.n <= kPiece;   // (every word is written once, no maximum to start from)
-    if (!one_store) DYB_CUDA(ctx, cudaMemsetAsync(j.scale, 0, (j.mode == F16_LINE ? j.lines : j.n) * sizeof(uint32_t), ctx->stream));
+    if (!one_store && !jobs->words) DYB_CUDA(ctx, cudaMemsetAsync(j.scale, 0, (j.mode == F16_LINE ? j.lines : j.n) * sizeof(uint32_t), ctx->stream));
     const uint64_t end = (uint64_t)jobs->start[k] + f16_max_units(j).total;
     DYB_CHECK_ARG(ctx, end < 0x7fffffffull, "fp16 planes: operand too large (%u x %u)", j.lines, j.n);
     jobs->start[k + 1] = (uint32_t)end;
@@ -1354,7 +1370,7 @@ static bool cluster_fits(dyb200_ctx* ctx, uint32_t bn, uint32_t S, uint32_t clus
 }
 
 int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const PackedOp* A, const PackedOp* B,
-                          const GemmEpilogue& epi, uint32_t force_splits) {
+                          const GemmEpilogue& epi, uint32_t force_splits, const uint32_t* unless) {
   EncodeTiledFn enc;
   int rc = get_encoder(ctx, &enc);
   if (rc) return rc;
@@ -1398,7 +1414,8 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   if (npairs == 1) for (int k = 0; k < 4; ++k) tm.t[4 + k] = tm.t[k];
   uint32_t kb0 = round_up(A[0].K, el) / el, kb1 = npairs > 1 ? round_up(A[1].K, el) / el : 0;
   const uint32_t kb_total = kb0 + kb1;
-  if (f16 && !force_splits && dyb200_pair_takes(ctx, M, N, epi)) return dyb200_gemm_pair(ctx, &tm, M, N, kb_total, flops, epi);
+  if (f16 && !force_splits && dyb200_pair_takes(ctx, M, N, epi)) return dyb200_gemm_pair(ctx, &tm, M, N, kb_total, flops, epi, unless);
+  DYB_CHECK_ARG(ctx, !unless, "tensor GEMM: a conditional product of a shape that the pair kernel does not take");
   dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, 1);
   DYB_CHECK_ARG(ctx, epi.mode != EPI_LSTM_CELL || (M % BM == 0 && epi.H * 4 == M && epi.ldc % 4 == 0 && aligned16(epi.C) &&
                                                       aligned16(epi.bias) && aligned16(epi.c_prev) && aligned16(epi.c_out) && aligned16(epi.h_out)),
@@ -1529,7 +1546,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       if (epi.split_m)
         vec = vec && epi.split_m % 4 == 0 && epi.ldc2 % 4 == 0 && aligned16(epi.C2) &&
               (epi.mode != EPI_ACCUM_MASK || (aligned16(epi.maskC2) && (!epi.maskc2_full || epi.maskc2_ld % 4 == 0)));
-      dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec, (size_t)M * N);
+      dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec, (size_t)M * N, nullptr);
       DYB_LAUNCHED(ctx);
     }
   }
@@ -1538,13 +1555,14 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
 
 // Second stage of a K split for callers outside this file: C = epilogue(sum over s of part[s]), the S partial products
 // (M x N each, leading dimension M) added in ascending order.
-int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi, size_t split_stride) {
+int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_t M, uint32_t N, const GemmEpilogue& epi, size_t split_stride,
+                         const uint32_t* unless) {
   int vec = M % 4 == 0 && split_stride % 4 == 0 && aligned16(part) && epi.ldc % 4 == 0 && aligned16(epi.C) && epi.mode != EPI_GATES && (epi.mode != EPI_BIAS || aligned16(epi.bias)) &&
             (epi.mode != EPI_ACCUM_MASK || (aligned16(epi.maskC) && (!epi.maskc_full || epi.maskc_ld % 4 == 0)));
   if (epi.split_m)
     vec = vec && epi.split_m % 4 == 0 && epi.ldc2 % 4 == 0 && aligned16(epi.C2) &&
           (epi.mode != EPI_ACCUM_MASK || (aligned16(epi.maskC2) && (!epi.maskc2_full || epi.maskc2_ld % 4 == 0)));
-  dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec, split_stride ? split_stride : (size_t)M * N);
+  dyb_launch(k_splitk_reduce, stream_grid(ctx, (size_t)M * N / 4 + 1, 256), 256, 0, ctx, part, S, M, N, epi, vec, split_stride ? split_stride : (size_t)M * N, unless);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
@@ -1554,31 +1572,34 @@ int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_
 // where they fit, or as work items of the persistent kernel with a second stage, by the estimates of dyb200_tc_splits.
 // us for both, as two launches / in one: 1024 x (128 + 256), K = 1600 38 / 22, 13000 99 / 69, 107000 538 / 378; 1200 x (200 + 300) x 1050 36 / 26;
 // 2048 x (512 + 512) x 4480 120 / 103.
-int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const PackedOp* B, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1) {
+int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const PackedOp* B, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1,
+                           const uint32_t* only_if) {
   EncodeTiledFn enc;
   int rc = get_encoder(ctx, &enc);
   if (rc) return rc;
-  const uint32_t N0 = B[0].rows, N1 = B[1].rows, bn = N0 <= 64 && N1 <= 64 ? 64 : BN, split = round_up(N0, bn), N = split + N1;
+  const uint32_t N0 = B[0].rows, N1 = B[1].rows, bn = N0 <= 64 && N1 <= 64 ? 64 : BN, split = N1 ? round_up(N0, bn) : 0, N = N1 ? split + N1 : N0;
   const uint32_t tiles_m = (M + BM - 1) / BM, tiles = tiles_m * ((N + bn - 1) / bn), kb = round_up(A.K, 32) / 32;
   TmapPack tm;
   memset(&tm, 0, sizeof(tm));
   tm.a_mn = tm.b_mn = 1;
   tm.n_split = split;
-  DYB_CHECK_ARG(ctx, A.mn_major && B[0].mn_major && B[1].mn_major && !A.f16 && A.K == B[0].K && A.K == B[1].K && A.rows == M, "tensor GEMM: operands of a grouped product");
+  DYB_CHECK_ARG(ctx, A.mn_major && B[0].mn_major && !A.f16 && A.K == B[0].K && A.rows == M && (N1 ? B[1].mn_major && A.K == B[1].K : only_if != nullptr),
+                "tensor GEMM: operands of a grouped product");
   if ((rc = make_map_mn(ctx, enc, &tm.t[0], A.hi, M, A.K, A.pitch, BM)) || (rc = make_map_mn(ctx, enc, &tm.t[1], A.lo, M, A.K, A.pitch, BM))) return rc;
-  for (int q = 0; q < 2; ++q)
+  for (int q = 0; q < (N1 ? 2 : 1); ++q)
     if ((rc = make_map_mn(ctx, enc, &tm.t[q ? 6 : 2], B[q].hi, B[q].rows, B[q].K, B[q].pitch, bn)) ||
         (rc = make_map_mn(ctx, enc, &tm.t[q ? 7 : 3], B[q].lo, B[q].rows, B[q].K, B[q].pitch, bn))) return rc;
+  if (!N1) { tm.t[6] = tm.t[2]; tm.t[7] = tm.t[3]; }   // (n_split = 0: every tile is of the second side)
   tm.t[4] = tm.t[0]; tm.t[5] = tm.t[1];
   GemmEpilogue epi{EPI_ACCUM, C0, ldc0, nullptr, 0, 0.f, nullptr, 0, 0};
-  epi.n_split = split; epi.n_live = N0; epi.Cn = C1; epi.ldcn = ldc1;
+  epi.n_split = split; epi.n_live = N0; epi.Cn = C1; epi.ldcn = ldc1; epi.only_if = only_if;
   const double flops = 2.0 * M * (double)(N0 + N1) * A.K, sms = (double)ctx->sm_count, t_kb = bn == 64 ? 0.40 : 0.66;
   // one tile per CTA (in waves: 2816 x (704 + 704) over 35 columns 22 us, 29 as work items of the persistent kernel), or clusters of S splits
   // that are all resident, at least eight k-blocks each (shorter splits end sooner on an idle GPU, but hold several times the SMs: three
   // language models of 256 units on three streams took 133 us a step with two k-blocks per split, 119 with eight)
   uint32_t Sc = 0;
   double cost = 1e30;
-  for (uint32_t S = 1; S <= 8 && (S == 1 || (kb / S >= 8 && ctx->cluster_splitk)); ++S) {
+  for (uint32_t S = 1; S <= (only_if ? 1u : 8u) && (S == 1 || (kb / S >= 8 && ctx->cluster_splitk)); ++S) {
     if (S > 1 && ((kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S || !cluster_fits(ctx, bn, S, tiles))) continue;
     const double t = (S == 1 ? ceil(tiles / sms) : 1.0) * (((kb + S - 1) / S) * t_kb + 9.0);
     if (t < cost) { cost = t; Sc = S; }
@@ -1586,7 +1607,7 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   // work items of the persistent kernel, as partial products and one sum per side (512 x (32 + 128) over 10560 columns: 19 us and 2 x 4, two
   // launches 29 and 35; 1024 x (128 + 256) over 107000: 369 us and 2 x 3, two launches 537)
   uint32_t Sp = 0;
-  for (uint32_t S = 2; S <= 64 && kb / S >= 16; ++S) {
+  for (uint32_t S = 2; S <= 64 && kb / S >= 16 && !only_if; ++S) {
     if ((kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S) continue;   // (no empty split)
     const double t = ceil((double)tiles * S / sms) * (((kb + S - 1) / S) * t_kb + 3.0) + 6.0 + (S + 2) * 4.0e-6 * M * N / 5.0 + 5.0;
     if (t < 0.97 * cost) { cost = t; Sp = S; }
@@ -1728,6 +1749,40 @@ struct dyb200_wgrad {
 static bool wgrad_on_f16(const dyb200_wgrad* w) {
   const double N = (double)w->N[0] + w->N[1];
   return w->k >= 256 && w->M * N >= 800.0 * (w->M + N);
+}
+// A pair of halves has the 22 bits of a TF32 pair within 2^28 of its scale, the largest value of a row over ALL columns.  Gradients that fade over
+// the steps leave that range, and dWx of a feature that is there in the first steps only would be made of what is left of them.  So the
+// passes that make the pairs also look at each row's blocks of eight columns: where one that is not all zero lies more than 2^kF16Span below
+// the row's largest value, a device word sends the flush back to the TF32 planes - the products of pairs end at once, and the grouped
+// product, which otherwise ends at once, adds its result.  So no element is further off than 2^-27 of the largest of its block.
+// The words and the empty launch cost 4 us of 66 (4096 x (1024 + 1024), K = 560) or 888 (K = 17920).
+static int wgrad_f16_planes(dyb200_ctx* ctx, const dyb200_wgrad* w, const PackedOp* ops, const bool* side, PackedOp* pairs, const uint32_t** wide) {
+  F16Jobs jobs;
+  jobs.n = 0;
+  size_t halves = 0, words = 0;
+  for (int q = 0; q < 3; ++q) {
+    if (q && !side[q - 1]) continue;
+    halves += 2 * (size_t)w->k * round_up(ops[q].rows, 64);
+    words += 2 * (size_t)round_up(ops[q].rows, 4);
+  }
+  void *hp, *wp;
+  int rc;
+  if ((rc = dyb200_scratch(ctx, halves * sizeof(__half), &hp)) || (rc = dyb200_scratch(ctx, (words + 1) * sizeof(uint32_t), &wp))) return rc;
+  __half* h = (__half*)hp;
+  uint32_t* s = (uint32_t*)wp;
+  jobs.words = s; jobs.n_words = words + 1; jobs.wide = s + words;
+  for (int q = 0; q < 3; ++q) {
+    if (q && !side[q - 1]) continue;
+    const uint32_t n = ops[q].rows, pitch = round_up(n, 64), wn = round_up(n, 4);
+    F16Job& j = jobs.job[jobs.n++];
+    j = F16Job{ops[q].hi, ops[q].pitch, w->k, n, pitch, F16_ELEM, s, h, h + (size_t)w->k * pitch};
+    j.src_lo = ops[q].lo;
+    j.low = s + wn;
+    h += 2 * (size_t)w->k * pitch; s += 2 * (size_t)wn;
+    pairs[q] = dyb200_f16_op(j, true);
+  }
+  *wide = jobs.wide;
+  return dyb200_f16_pack(ctx, &jobs);
 }
 // natural pack of the k columns [col, col + k) of operand j (b is N[j] x k column-major; the mask is indexed like b)
 static int pack_b_rows(dyb200_ctx* ctx, dyb200_wgrad* w, int j, uint32_t col, uint32_t k, const float* b, uint32_t ldb, const float* mask,
@@ -1984,32 +2039,33 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
   DYB_CHECK_ARG(ctx, kb_seen >= w->k, "wgrad_flush: the B operands cover %u columns, the A operand %u", kb_seen, w->k);
   PackedOp ops[3] = {w->A, w->B[0], w->B[1]};   // (MN-major: one plane row per column)
   for (PackedOp& o : ops) o.K = w->k;
+  float* const C[2] = {C0, C1};
+  const uint32_t ldc[2] = {ldc0, ldc1};
+  int rc;
+  bool done[2] = {false, w->N[1] == 0};
   if (wgrad_on_f16(w)) {
-    F16Jobs jobs;
-    jobs.n = w->N[1] ? 3 : 2;
-    for (int q = 0; q < jobs.n; ++q) {
-      int rc = dyb200_f16_planes(ctx, ops[q].hi, ops[q].pitch, w->k, ops[q].rows, F16_ELEM, &jobs.job[q]);
-      if (rc) return rc;
-      jobs.job[q].src_lo = ops[q].lo;
+    // (a side of one tile is no product of the pair kernel and stays on the TF32 planes; by the rule at least one side is wider)
+    PackedOp pairs[3], sides[2];
+    const uint32_t* wide;
+    int n = 0, at[2] = {0, 0};
+    for (int j = 0; j < 2; ++j)
+      if (w->N[j] > (uint32_t)BN) { done[j] = true; at[n] = j; sides[n++] = ops[1 + j]; }
+    const bool side[2] = {w->N[0] > (uint32_t)BN, w->N[1] > (uint32_t)BN};
+    if ((rc = wgrad_f16_planes(ctx, w, ops, side, pairs, &wide))) return rc;
+    for (int q = 0; q < n; ++q) {
+      const GemmEpilogue e{EPI_ACCUM, C[at[q]], ldc[at[q]], nullptr, 0, 0.f, nullptr, 0, 0};
+      if ((rc = dyb200_tc_gemm_packed(ctx, w->M, sides[q].rows, 1, &pairs[0], &pairs[1 + at[q]], e, 0, wide))) return rc;
     }
-    int rc = dyb200_f16_pack(ctx, &jobs);
-    if (rc) return rc;
-    for (int q = 0; q < jobs.n; ++q) ops[q] = dyb200_f16_op(jobs.job[q], true);
-  }
-  const PackedOp& A = ops[0];
-  if (!A.f16 && w->N[1]) {
-    int rc = dyb200_tc_gemm_packed2(ctx, w->M, A, ops + 1, C0, ldc0, C1, ldc1);
-    if (rc) return rc;
-    w->k = 0;
-    w->kb = 0;
-    return DYB200_OK;
+    if (n == 1) sides[1].rows = 0;
+    if ((rc = dyb200_tc_gemm_packed2(ctx, w->M, ops[0], sides, C[at[0]], ldc[at[0]], C[at[1]], ldc[at[1]], wide))) return rc;
+  } else if (w->N[1]) {
+    if ((rc = dyb200_tc_gemm_packed2(ctx, w->M, ops[0], ops + 1, C0, ldc0, C1, ldc1))) return rc;
+    done[0] = done[1] = true;
   }
   for (int j = 0; j < 2; ++j) {
-    if (w->N[j] == 0) continue;
-    const PackedOp& B = ops[1 + j];
-    GemmEpilogue e{EPI_ACCUM, j == 0 ? C0 : C1, j == 0 ? ldc0 : ldc1, nullptr, 0, 0.f, nullptr, 0, 0};
-    int rc = dyb200_tc_gemm_packed(ctx, w->M, w->N[j], 1, &A, &B, e);
-    if (rc) return rc;
+    if (done[j]) continue;
+    const GemmEpilogue e{EPI_ACCUM, C[j], ldc[j], nullptr, 0, 0.f, nullptr, 0, 0};
+    if ((rc = dyb200_tc_gemm_packed(ctx, w->M, w->N[j], 1, &ops[0], &ops[1 + j], e))) return rc;
   }
   w->k = 0;
   w->kb = 0;

@@ -16,7 +16,7 @@
 struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; const uint32_t *sa, *sb;
   uint32_t store_map;      // t[4] describes the output (persistent kernel, plain stores; one pair)
   uint32_t n_split; };     // columns from here on are those of a second right operand, t[6] and t[7] (0: none; one pair, a multiple of the tile)
-int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint32_t kb, double flops, const GemmEpilogue& epi);
+int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint32_t kb, double flops, const GemmEpilogue& epi, const uint32_t* unless);
 
 namespace {
 
