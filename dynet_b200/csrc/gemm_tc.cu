@@ -2029,6 +2029,16 @@ int dyb200_wgrad_pack_inputs(dyb200_wgrad* w, const dyb200_tensor* x_all, const 
   return DYB200_OK;
 }
 
+// Whether the two results share an element (M x N0 and M x N1, column-major): one weight read at both places, say.  Rows of one matrix side by
+// side (the same leading dimension, row ranges that do not meet) do not.
+static bool wgrad_results_meet(const dyb200_wgrad* w, const float* C0, uint32_t ldc0, const float* C1, uint32_t ldc1) {
+  const uintptr_t a = (uintptr_t)C0, b = (uintptr_t)C1;
+  const size_t na = 4 * ((size_t)ldc0 * (w->N[0] - 1) + w->M), nb = 4 * ((size_t)ldc1 * (w->N[1] - 1) + w->M);
+  if (a + na <= b || b + nb <= a) return false;
+  if (ldc0 != ldc1 || ldc0 < w->M || (a - b) % 4 != 0) return true;
+  const uint32_t gap = (uint32_t)((a > b ? a - b : b - a) / 4 % ldc0);
+  return gap < w->M || ldc0 - gap < w->M;
+}
 int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1, dyb200_ctx* ctx) {
   { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
   DYB_CHECK_ARG(ctx, w && C0 && (w->N[1] == 0 || C1), "wgrad_flush: null argument");
@@ -2043,6 +2053,8 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
   const uint32_t ldc[2] = {ldc0, ldc1};
   int rc;
   bool done[2] = {false, w->N[1] == 0};
+  // (results that meet are added to by one product after the other, not by the tiles of one launch)
+  const bool apart = w->N[1] && wgrad_results_meet(w, C0, ldc0, C1, ldc1);
   if (wgrad_on_f16(w)) {
     // (a side of one tile is no product of the pair kernel and stays on the TF32 planes; by the rule at least one side is wider)
     PackedOp pairs[3], sides[2];
@@ -2056,9 +2068,12 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
       const GemmEpilogue e{EPI_ACCUM, C[at[q]], ldc[at[q]], nullptr, 0, 0.f, nullptr, 0, 0};
       if ((rc = dyb200_tc_gemm_packed(ctx, w->M, sides[q].rows, 1, &pairs[0], &pairs[1 + at[q]], e, 0, wide))) return rc;
     }
-    if (n == 1) sides[1].rows = 0;
-    if ((rc = dyb200_tc_gemm_packed2(ctx, w->M, ops[0], sides, C[at[0]], ldc[at[0]], C[at[1]], ldc[at[1]], wide))) return rc;
-  } else if (w->N[1]) {
+    for (int q = 0; q < n; q += apart ? 1 : 2) {
+      PackedOp two[2] = {sides[q], sides[1]};
+      if (n == 1 || apart) two[1].rows = 0;
+      if ((rc = dyb200_tc_gemm_packed2(ctx, w->M, ops[0], two, C[at[q]], ldc[at[q]], C[at[1]], ldc[at[1]], wide))) return rc;
+    }
+  } else if (w->N[1] && !apart) {
     if ((rc = dyb200_tc_gemm_packed2(ctx, w->M, ops[0], ops + 1, C0, ldc0, C1, ldc1))) return rc;
     done[0] = done[1] = true;
   }

@@ -33,3 +33,34 @@ def test_grouped_products(M, N0, N1, k):
     finally:
         ctx.wgrad_destroy(w)
     assert ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("M,N,k", [(1024, 128, 320), (256, 100, 31), (1024, 128, 40000), (1700, 1600, 400)])
+@pytest.mark.parametrize("layout", ["same", "columns", "rows"])
+def test_results_in_one_matrix(M, N, k, layout):
+    """One weight read at both places: both products are added to the same matrix, or to one that starts some columns into it; and the two results
+    as row blocks of one matrix, which do not meet."""
+    import torch
+    import gpu_util as g
+    ctx = g.ctx()
+    gen = torch.Generator("cuda").manual_seed(M + N)
+    w = ctx.wgrad_create(M, N, N, k)
+    try:
+        a, b0, b1 = (torch.randn(k, n, device="cuda", generator=gen) for n in (M, N, N))
+        ld = 2 * M if layout == "rows" else M
+        C = torch.randn(2 * N, ld, device="cuda", generator=gen)
+        want, off = C.double(), dict(same=0, columns=7 * M, rows=M)[layout]
+        p0, p1 = b0.double().t() @ a.double(), b1.double().t() @ a.double()
+        want[:N, :M] += p0
+        if layout == "rows":
+            want[:N, M:] += p1
+        else:
+            want[off // M:off // M + N] += p1
+        ctx.wgrad_push(w, k, a.data_ptr(), M, b0.data_ptr(), N, None, 0, b1.data_ptr(), N, None, 0)
+        ctx.wgrad_flush(w, C.data_ptr(), ld, C.data_ptr() + 4 * off, ld)
+        # (two results of 5.7e-6 of |row| |column| each, and their last roundings)
+        bar = 2 * 5.7e-6 * float(a.double().norm(dim=0).max()) * float(torch.cat([b0, b1], 1).double().norm(dim=0).max()) + 2.4e-7 * want.abs().max()
+        assert float((C.double() - want).abs().max()) <= float(bar)
+    finally:
+        ctx.wgrad_destroy(w)
+    assert ctx.device_errors() == 0
