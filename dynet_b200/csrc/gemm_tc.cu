@@ -1599,7 +1599,7 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   // language models of 256 units on three streams took 133 us a step with two k-blocks per split, 119 with eight)
   uint32_t Sc = 0;
   double cost = 1e30;
-  for (uint32_t S = 1; S <= (only_if ? 1u : 8u) && (S == 1 || (kb / S >= 8 && ctx->cluster_splitk)); ++S) {
+  for (uint32_t S = 1; S <= (only_if ? 1u : 8u) && (S == 1 || kb / S >= 8); ++S) {
     if (S > 1 && ((kb + (kb + S - 1) / S - 1) / ((kb + S - 1) / S) != S || !cluster_fits(ctx, bn, S, tiles))) continue;
     const double t = (S == 1 ? ceil(tiles / sms) : 1.0) * (((kb + S - 1) / S) * t_kb + 9.0);
     if (t < cost) { cost = t; Sc = S; }
@@ -1614,7 +1614,8 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   }
   if ((rc = gemm_tc_limits(ctx))) return rc;
   const dim3 grid(tiles_m, (N + bn - 1) / bn, 1);
-  if (Sp == 0) {
+  const bool through_memory = Sp == 0 && Sc > 1 && !ctx->cluster_splitk;   // (dyb200_ctx_cluster_splitk: the clusters' splits, the same partial tiles)
+  if (Sp == 0 && !through_memory) {
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
     if (Sc == 1) {
       dyb_launch(bn == 64 ? k_gemm_tc<64, false, false, true> : k_gemm_tc<128, false, false, true>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
@@ -1632,13 +1633,19 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
     return DYB200_OK;
   }
   // partial products over the columns of both sides
+  if (through_memory) Sp = Sc;
   void* pw;
   if ((rc = dyb200_scratch(ctx, (size_t)Sp * M * N * sizeof(float), &pw))) return rc;
   float* const part = (float*)pw;
   const GemmEpilogue pepi{EPI_STORE, part, M, nullptr, 0, 0.f, nullptr, 0, 0};
-  tm.store_map = M % 4 == 0;
-  if (tm.store_map && (rc = dyb200_tc_make_store_map(ctx, &tm.t[4], part, M, N, Sp, M, 64))) return rc;
-  {
+  if (through_memory) {
+    GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
+    dyb_launch(bn == 64 ? k_gemm_tc<64, false, false, true> : k_gemm_tc<128, false, false, true>, dim3(grid.x, grid.y, Sp), kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u,
+               (kb + Sp - 1) / Sp, pepi, ctx->dev_flags);
+    DYB_LAUNCHED(ctx);
+  } else {
+    tm.store_map = M % 4 == 0;
+    if (tm.store_map && (rc = dyb200_tc_make_store_map(ctx, &tm.t[4], part, M, N, Sp, M, 64))) return rc;
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
     dyb_launch(bn == 64 ? k_gemm_persist<64> : k_gemm_persist<128>, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb, 0u, tiles_m, tiles, tiles_m > 16 ? 16u : 0u,
                Sp, pepi, ctx->dev_flags);

@@ -573,7 +573,8 @@ int layer_inputs(dyb200_ctx* ctx, dyb200_wgrad* deferred, const float* Wx, const
 // Layers from 512 units on whose batch is in whole 64-column tiles and whose tiles are all resident (one CTA per SM: 225 KB of shared memory); the
 // TF32 form serves narrower ones.  64-column tiles where there are SMs for them (us per step, I = H = 1024, TF32 / this form with 128 / with 64
 // columns: batch 128 16.5 / 14.3 / 10.5, 256 23.3 / 17.4 / 14.8; batch 512 has 128 columns only, 40.8 / 25.4; batch 64 11.1 / - / 9.0), then as
-// many K splits as there are SMs for, four k-blocks each and more.
+// many K splits as there are SMs for, four k-blocks each and more (as clusters whatever dyb200_ctx_cluster_splitk says: there is no other form, and
+// another number of splits would give other bits).
 bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* bn, uint32_t* S) {
   if (H < 512 || H % 32 != 0 || I == 0 || I % 4 != 0 || B == 0 || B % 64 != 0) return false;
   const uint32_t sms = (uint32_t)ctx->sm_count, tiles_m = 4 * H / BM, kb = (I + 63) / 64 + (H + 63) / 64;
@@ -581,7 +582,7 @@ bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, ui
   const uint32_t tiles = tiles_m * (B / *bn);
   if (B % *bn != 0 || B / *bn > 32) return false;   // (one hand-over counter per column block)
   for (uint32_t s = *bn == 64 ? 8 : 4; s >= 1; s /= 2) {
-    if (tiles * s > sms || (s > 1 && (kb / s < 4 || !ctx->cluster_splitk))) continue;
+    if (tiles * s > sms || (s > 1 && kb / s < 4)) continue;
     if (seq_fwd_dispatch<true>(SEQ_SET_SMEM, *bn, s, ctx) != DYB200_OK) return false;
     if (s > 1) {
       const int fit = seq_fwd_dispatch<true>(SEQ_FIT, *bn, s, ctx);

@@ -93,7 +93,8 @@ int dyb200_ctx_param_cache(dyb200_ctx* ctx, int enable);
 int dyb200_ctx_dependent_launch(dyb200_ctx* ctx, int enable);
 /* K splits of a tensor-pipe product as one thread-block cluster per output tile, reduced through distributed shared memory
  * (on by default).  Off: the splits
- * go through a workspace and a second kernel.  Results are bitwise the same either way. */
+ * go through a workspace and a second kernel.  Results are bitwise the same either way.  The recurrence kernels of LSTM sequences that exist
+ * as clusters only (layers up to 384 units; wide layers on fp16 pairs) stay clusters. */
 int dyb200_ctx_cluster_splitk(dyb200_ctx* ctx, int enable);
 int dyb200_ctx_params_changed(dyb200_ctx* ctx);
 /* Library build string ("dyb200 <n> sm_100a"). */
