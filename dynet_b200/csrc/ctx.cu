@@ -28,13 +28,13 @@ int dyb200_scratch_begin(dyb200_ctx* ctx) {
       if (ctx->scratch) DYB_CUDA(ctx, cudaFree(ctx->scratch));
       ctx->scratch = nullptr;
       ctx->scratch_bytes = 0;
-      size_t want = ctx->scratch_peak + (ctx->scratch_peak >> 2) + (1u << 20);
-      cudaError_t e = cudaMalloc(&ctx->scratch, want);
-      if (e != cudaSuccess) {
+      // (little memory left: without the room on top, or no arena for now - what a call asks for may still fit)
+      for (const size_t want : {ctx->scratch_peak + (ctx->scratch_peak >> 2) + (1u << 20), ctx->scratch_peak}) {
+        if (cudaMalloc(&ctx->scratch, want) == cudaSuccess) { ctx->scratch_bytes = want; break; }
         cudaGetLastError();
-        return dyb200_fail(ctx, DYB200_ENOMEM, "scratch arena: cudaMalloc(%zu) failed: %s", want, cudaGetErrorString(e));
+        ctx->scratch = nullptr;
       }
-      ctx->scratch_bytes = want;
+      if (!ctx->scratch) ctx->scratch_peak = 0;
     }
   }
   ctx->scratch_off = 0;

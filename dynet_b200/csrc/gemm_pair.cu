@@ -341,9 +341,8 @@ int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint
   GemmEpilogue e = epi;
   if (a.S > 1) {
     void* part;
-    int rc = dyb200_scratch(ctx, (size_t)a.S * M * N * sizeof(float), &part);
-    if (rc) return rc;
-    e = GemmEpilogue{EPI_STORE, (float*)part, M, nullptr, 0, 0.f, nullptr, 0, 0};
+    if (dyb200_scratch(ctx, (size_t)a.S * M * N * sizeof(float), &part) == DYB200_OK) e = GemmEpilogue{EPI_STORE, (float*)part, M, nullptr, 0, 0.f, nullptr, 0, 0};
+    else a.S = 1;   // (no room for partial products)
   }
   a.C = e.C; a.ldc = e.ldc; a.bias = e.mode == EPI_BIAS ? e.bias : nullptr; a.accumulate = e.mode == EPI_ACCUM;
   tm->store_map = e.ldc % 4 == 0 && aligned16(e.C);

@@ -1615,7 +1615,13 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   if ((rc = gemm_tc_limits(ctx))) return rc;
   const dim3 grid(tiles_m, (N + bn - 1) / bn, 1);
   const bool through_memory = Sp == 0 && Sc > 1 && !ctx->cluster_splitk;   // (dyb200_ctx_cluster_splitk: the clusters' splits, the same partial tiles)
-  if (Sp == 0 && !through_memory) {
+  if (through_memory) Sp = Sc;
+  void* pw = nullptr;
+  if (Sp && dyb200_scratch(ctx, (size_t)Sp * M * N * sizeof(float), &pw) != DYB200_OK) {   // (no room for partial products)
+    Sp = 0;
+    if (!ctx->cluster_splitk) Sc = 1;
+  }
+  if (Sp == 0) {
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
     if (Sc == 1) {
       dyb_launch(bn == 64 ? k_gemm_tc<64, false, false, true> : k_gemm_tc<128, false, false, true>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
@@ -1633,9 +1639,6 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
     return DYB200_OK;
   }
   // partial products over the columns of both sides
-  if (through_memory) Sp = Sc;
-  void* pw;
-  if ((rc = dyb200_scratch(ctx, (size_t)Sp * M * N * sizeof(float), &pw))) return rc;
   float* const part = (float*)pw;
   const GemmEpilogue pepi{EPI_STORE, part, M, nullptr, 0, 0.f, nullptr, 0, 0};
   if (through_memory) {
@@ -1772,11 +1775,11 @@ static int wgrad_f16_planes(dyb200_ctx* ctx, const dyb200_wgrad* w, const Packed
     halves += 2 * (size_t)w->k * round_up(ops[q].rows, 64);
     words += 2 * (size_t)round_up(ops[q].rows, 4);
   }
-  void *hp, *wp;
+  void* p;   // (one block: there is room for all or nothing is taken; the planes are whole 128-byte lines)
   int rc;
-  if ((rc = dyb200_scratch(ctx, halves * sizeof(__half), &hp)) || (rc = dyb200_scratch(ctx, (words + 1) * sizeof(uint32_t), &wp))) return rc;
-  __half* h = (__half*)hp;
-  uint32_t* s = (uint32_t*)wp;
+  if ((rc = dyb200_scratch(ctx, halves * sizeof(__half) + (words + 1) * sizeof(uint32_t), &p))) return rc;
+  __half* h = (__half*)p;
+  uint32_t* s = (uint32_t*)(h + halves);
   jobs.words = s; jobs.n_words = words + 1; jobs.wide = s + words;
   for (int q = 0; q < 3; ++q) {
     if (q && !side[q - 1]) continue;
@@ -2059,18 +2062,23 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
   float* const C[2] = {C0, C1};
   const uint32_t ldc[2] = {ldc0, ldc1};
   int rc;
-  bool done[2] = {false, w->N[1] == 0};
+  bool done[2] = {false, w->N[1] == 0}, pairs_fit = false;
   // (results that meet are added to by one product after the other, not by the tiles of one launch)
   const bool apart = w->N[1] && wgrad_results_meet(w, C0, ldc0, C1, ldc1);
+  PackedOp pairs[3];
+  const uint32_t* wide;
+  const bool side[2] = {w->N[0] > (uint32_t)BN, w->N[1] > (uint32_t)BN};
   if (wgrad_on_f16(w)) {
+    rc = wgrad_f16_planes(ctx, w, ops, side, pairs, &wide);
+    if (rc && rc != DYB200_ENOMEM) return rc;
+    pairs_fit = rc == DYB200_OK;   // (without room for them the planes in hand serve)
+  }
+  if (pairs_fit) {
     // (a side of one tile is no product of the pair kernel and stays on the TF32 planes; by the rule at least one side is wider)
-    PackedOp pairs[3], sides[2];
-    const uint32_t* wide;
+    PackedOp sides[2];
     int n = 0, at[2] = {0, 0};
     for (int j = 0; j < 2; ++j)
-      if (w->N[j] > (uint32_t)BN) { done[j] = true; at[n] = j; sides[n++] = ops[1 + j]; }
-    const bool side[2] = {w->N[0] > (uint32_t)BN, w->N[1] > (uint32_t)BN};
-    if ((rc = wgrad_f16_planes(ctx, w, ops, side, pairs, &wide))) return rc;
+      if (side[j]) { done[j] = true; at[n] = j; sides[n++] = ops[1 + j]; }
     for (int q = 0; q < n; ++q) {
       const GemmEpilogue e{EPI_ACCUM, C[at[q]], ldc[at[q]], nullptr, 0, 0.f, nullptr, 0, 0};
       if ((rc = dyb200_tc_gemm_packed(ctx, w->M, sides[q].rows, 1, &pairs[0], &pairs[1 + at[q]], e, 0, wide))) return rc;

@@ -670,16 +670,20 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
                     aligned16(c_all->v) && aligned16(h_all->v) && (!mh || aligned16(mh)) &&
                     (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H));
   uint32_t S = 1, f16_bn;
+  bool wide_fits = true;
   SeqPlanes pl;
   if (resident && dyb200_seq_f16_plan(ctx, I, H, B, &f16_bn, &S) && dyb200_wgrad_seq_planes(deferred, T, B, &pl)) {   // (wide layers)
     { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
     DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_seq_fwd: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
     SeqF16Call q{I, H, B, T, Wx->v, Wh->v, b->v, h0->v, c0->v, mh, mh_full, attrs->forget_gate_bias, gates_all->v, c_all->v, h_all->v, pl.X, pl.Hs, 0, 0};
-    if ((rc = dyb200_seq_f16(ctx, q))) return rc;
-    dyb200_wgrad_seq_done(deferred);
-    return DYB200_OK;
+    rc = dyb200_seq_f16(ctx, q);
+    if (rc != DYB200_ENOMEM) {
+      if (!rc) dyb200_wgrad_seq_done(deferred);
+      return rc;
+    }
+    wide_fits = false;   // (no room for the pairs of all steps: the single-step calls, with those of one)
   }
-  bool persistent = resident && B % bn == 0;
+  bool persistent = resident && wide_fits && B % bn == 0;
   if (persistent) {
     S = dyb200_tc_splits(ctx, G, B, kb_total);
     const uint32_t per = (kb_total + S - 1) / S;
