@@ -165,7 +165,7 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
 int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
 // The gate weights of a layer, Wx (4H x I) and Wh (4H x H), as MN-major planes with interleaved rows (lines = their columns, pitch 4H) and one
-// scale word per row of [Wx Wh] (not interleaved); from the parameter cache when it is on.
+// scale word per row of Wx and one per row of Wh (4H words each, not interleaved); from the parameter cache when it is on.
 struct F16Gates { __half *x_hi, *x_lo, *h_hi, *h_lo; const uint32_t* scale; };
 int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, F16Gates* out);
 // Products that use fp16 pairs, by useful flops.  Finding the scales adds a clear and a pass over the operands; us with TF32 / fp16 pairs,

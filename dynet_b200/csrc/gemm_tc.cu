@@ -1043,13 +1043,13 @@ int pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int layout, uint32_t ro
 
 inline uint32_t round_up(uint32_t x, uint32_t m) { return (x + m - 1) / m * m; }
 
-// fp16 planes of the gate weights (F16Gates): I lines of Wx, then H lines of Wh, one set of scales.
+// fp16 planes of the gate weights (F16Gates): I lines of Wx, then H lines of Wh, the scale words in the same order.
 int gates_f16_pack(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, __half* hi, __half* lo, uint32_t* scale) {
   F16Jobs jobs;
   jobs.n = 2;
   for (int q = 0; q < 2; ++q) {
     const size_t at = q ? (size_t)I * 4 * H : 0;
-    jobs.job[q] = F16Job{q ? Wh : Wx, 4 * H, q ? H : I, 4 * H, 4 * H, F16_ELEM, scale, hi + at, lo + at};
+    jobs.job[q] = F16Job{q ? Wh : Wx, 4 * H, q ? H : I, 4 * H, 4 * H, F16_ELEM, scale + q * 4 * H, hi + at, lo + at};
     jobs.job[q].perm_H = H;
   }
   return dyb200_f16_pack(ctx, &jobs);
@@ -1069,7 +1069,7 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     else if (victim->hi && e->last_use < victim->last_use) victim = e;
   }
   dyb200_ctx::ParamPack* e = hit ? hit : victim;
-  const size_t floats = k_is_fast == kLayoutGatesF16 ? (size_t)(K + rows2) * pitch / 2 + rows : k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE ? rows : K) : (size_t)(rows + rows2) * pitch;
+  const size_t floats = k_is_fast == kLayoutGatesF16 ? (size_t)(K + rows2) * pitch / 2 + 2 * rows : k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE ? rows : K) : (size_t)(rows + rows2) * pitch;
   if (!hit) {
     if (e->hi && e->floats < floats) {   // evicted entry is too small: its buffers may still be read by queued kernels
       DYB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1175,7 +1175,7 @@ int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t
     scale = reinterpret_cast<uint32_t*>(hi + plane / 2);
   } else {
     void *h, *l, *sc;
-    if ((rc = dyb200_scratch(ctx, plane * sizeof(__half), &h)) || (rc = dyb200_scratch(ctx, plane * sizeof(__half), &l)) || (rc = dyb200_scratch(ctx, G * sizeof(uint32_t), &sc))) return rc;
+    if ((rc = dyb200_scratch(ctx, plane * sizeof(__half), &h)) || (rc = dyb200_scratch(ctx, plane * sizeof(__half), &l)) || (rc = dyb200_scratch(ctx, 2 * G * sizeof(uint32_t), &sc))) return rc;
     hi = (float*)h; lo = (float*)l; scale = (uint32_t*)sc;
     if ((rc = gates_f16_pack(ctx, Wx, Wh, I, H, (__half*)hi, (__half*)lo, scale))) return rc;
   }

@@ -34,7 +34,7 @@ struct SeqFwd {
   float *hn_hi, *hn_lo; uint32_t hn_pitch;
   const float* hmask; uint32_t hmask_ld; int hmask_full;
   int emit_last;                    // the last step's h goes out as operand planes too (a single step of a sequence driven from outside)
-  // F16: scale words of the gate rows (row q H + u of [Wx Wh]), of the columns of x (sequence columns), of h_{-1} (batch columns) and of all
+  // F16: scale words of the gate rows (row q H + u of Wx, 4H further on of Wh), of the columns of x (sequence columns), of h_{-1} (batch columns) and of all
   // later h (batch columns, or one for all; null: |h| < 1), and the planes of h .* mask_h as fp16 pairs: two slots of B rows, step t reads
   // slot t % 2
   const uint32_t *gate_scale, *x_scale, *h0_scale, *h_scale; int h_scale_full;
@@ -57,7 +57,7 @@ __device__ __forceinline__ void tmem_ld16x2(uint32_t t1, uint32_t t2, float* v1,
 }
 
 // F16: the products of wide layers on scaled fp16 pairs (gemm.cuh) in k-blocks of 64 - half the weight bytes from L2 per step and 0.61 us per 64 k
-// instead of 2 x 0.66.  The weights' planes are MN-major as they lie, their rows interleaved like the TF32 ones; [Wx Wh] has a scale per gate row.
+// instead of 2 x 0.66.  The weights' planes are MN-major as they lie, their rows interleaved like the TF32 ones; a scale per gate row of Wx and of Wh.
 // A column of x has a scale of its own, h .* mask_h one that is known beforehand (|h| < 1: the largest mask value of the column), h_{-1} the
 // larger of that and its own; so accumulation chains end between Wx x and Wh h, and a chain is unscaled as it is drained.  (Elements of h below 2^-28 of
 // the mask's largest value keep an absolute error of 2^-51 of it.)
@@ -202,11 +202,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
     const bool has_cols = 64 * half < BNT;
     const uint32_t x_chunks = (ks.n0 + kChunk - 1) / kChunk;   // (F16: those of Wx x)
     const uint32_t nchunks = F16 ? x_chunks + (ks.n1 + kChunk - 1) / kChunk : (total + kChunk - 1) / kChunk;
-    // F16: 2^-s of this thread's gate row; of the columns lane and lane + 32 of its half (h after the first step); and 2^s of the columns it finishes
-    float row_f = 1.f, h_f[2] = {1.f, 1.f}, h_s[BNT / 64][2];
+    // F16: 2^-s of this thread's gate row in Wx and in Wh; of the columns lane and lane + 32 of its half (h after the first step); and 2^s of the columns it finishes
+    float row_x = 1.f, row_h = 1.f, h_f[2] = {1.f, 1.f}, h_s[BNT / 64][2];
     const uint32_t hn0 = n0 + 64 * half + lane;
     if (F16) {
-      row_f = inv_scale_of(__ldg(a.gate_scale + (size_t)quarter * a.H + 32 * blockIdx.x + lane));
+      row_x = inv_scale_of(__ldg(a.gate_scale + (size_t)quarter * a.H + 32 * blockIdx.x + lane));
+      row_h = inv_scale_of(__ldg(a.gate_scale + (size_t)(4 + quarter) * a.H + 32 * blockIdx.x + lane));
       if (has_cols) { h_f[0] = inv_scale_of(h_word(a, hn0)); h_f[1] = inv_scale_of(h_word(a, hn0 + 32)); }
 #pragma unroll
       for (int hh = 0; hh < BNT / 64; ++hh)
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
           cp[hh][k] = mine ? ld4(c_prev + u + (size_t)a.H * n) : make_float4(0.f, 0.f, 0.f, 0.f);
           hm[hh][k] = (mine && a.hmask) ? ld4(a.hmask + u + (a.hmask_full ? (size_t)a.hmask_ld * n : 0)) : make_float4(1.f, 1.f, 1.f, 1.f);
         }
-      float f[2] = {1.f, 1.f};   // F16: 2^-s of the columns lane and lane + 32 in the coming chains
+      float f[2] = {1.f, 1.f}, row_f = row_x;   // F16: 2^-s of the columns lane and lane + 32 in the coming chains, and of the row
       if (F16 && has_cols) { f[0] = inv_scale_of(__ldg(a.x_scale + (size_t)t * a.B + hn0)); f[1] = inv_scale_of(__ldg(a.x_scale + (size_t)t * a.B + hn0 + 32)); }
       float sum[64];
 #pragma unroll
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
       for (uint32_t c = 0; c < nchunks; ++c, ++cg) {
         const uint32_t buf = cg % kBufs;
         if (F16 && c == x_chunks) {
-          f[0] = h_f[0]; f[1] = h_f[1];
+          f[0] = h_f[0]; f[1] = h_f[1]; row_f = row_h;
           if (t == 0 && has_cols) { f[0] = inv_scale_of(__ldg(a.h0_scale + hn0)); f[1] = inv_scale_of(__ldg(a.h0_scale + hn0 + 32)); }
         }
         if (!ok) continue;
@@ -282,7 +283,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
             tmem_ld16x2(taddr + 16 * p, taddr + BNT + 16 * p, v1, v2);
 #pragma unroll
             for (int q = 0; q < 16; ++q)
-              sum[16 * p + q] = fmaf(fmaf(v2[q], kLoScale, v1[q]) * row_f, __shfl_sync(0xffffffffu, f[p / 2], 16 * (p % 2) + q), sum[16 * p + q]);
+              // (both factors at once: the sum times one of them may leave fp32's range where the product does not)
+              sum[16 * p + q] = fmaf(fmaf(v2[q], kLoScale, v1[q]), row_f * __shfl_sync(0xffffffffu, f[p / 2], 16 * (p % 2) + q), sum[16 * p + q]);
           }
         } else if (has_cols) {
           float v[32];

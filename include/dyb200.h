@@ -321,7 +321,7 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
  *   * When the shape allows (deferred given, tensor-path sizes, whole tiles, every CTA resident at once) the steps run inside ONE
  *     kernel whose CTAs stay on the GPU for the whole sequence and hand h_t over through device memory: bit for bit the calls above.
  *     From 512 units on the products of both (calls with an accumulator, batches in whole 64-column tiles) are of scaled fp16 pairs: a scale
- *     per gate row and per column of x, and for a column of h the largest of its mask's values (1 without) and, in the first step, of h0.
+ *     per gate row of Wx and of Wh and per column of x, and for a column of h the largest of its mask's values (1 without) and, in the first step, of h0.
  *   * Other sequences of at least 8 steps of layers up to 384 units, or with at most 32 columns, form Wx x of all steps at once and
  *     keep only Wh h in the recurrence: the same values to the rounding of their sums, which associate differently, and the same
  *     bits from run to run.  Wh h is plain fp32 above 256 units, and below while there are at most four columns per cluster of

@@ -60,3 +60,34 @@ def test_sequence_of_a_wide_layer(I, H, B, T, mask):
         assert bool(((cs[t] - c).abs() <= 2e-7 * ((i * gg).abs() + (f * cp).abs())).all())
         assert bool(((hs[t] - o * torch.tanh(cs[t])).abs() <= 5e-7).all())
     assert ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("e", [20, 45, 112, -112])
+@pytest.mark.parametrize("single", [False, True])
+def test_weights_and_inputs_of_other_magnitudes(e, single):
+    """Wx 2^e times larger and x as much smaller: Wh and h keep their bits beside them, and no factor leaves fp32's range on the way.  Bar as above."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    I, H, B = 512, 512, 64
+    gen = torch.Generator("cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    x, h0, c0, b = rnd(2 * B, I) * 2.0 ** -e, rnd(B, H) * 0.3, rnd(B, H), rnd(4 * H) * 0.1
+    Wx, Wh = rnd(I, 4 * H) / I ** 0.5 * 2.0 ** e, rnd(H, 4 * H) / H ** 0.5
+    W, at = (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1)), capi.LstmGatesAttrs(0, 0.0, 1.0)
+    gates, cs, hs = (torch.empty(2 * B, n, device="cuda") for n in (4 * H, H, H))
+    w = ctx.wgrad_create(4 * H, I, H, 2 * B)
+    if single:
+        ctx.lstm_fwd_fused_at(g.T(x[:B]), g.T(h0), g.T(c0), *W, None, None, at, g.T(gates[:B]), g.T(cs[:B]), g.T(hs[:B]), w, 0)
+    else:
+        ctx.lstm_seq_fwd(g.T(x, [I], 2 * B), g.T(h0), g.T(c0), *W, None, None, at, g.T(gates, [4 * H], 2 * B), g.T(cs, [H], 2 * B), g.T(hs, [H], 2 * B), w, 2)
+    torch.cuda.synchronize()
+    ctx.wgrad_destroy(w)
+    xd, hd = x[:B].double(), h0.double()
+    pre = xd @ Wx.double() + hd @ Wh.double() + b.double()
+    bar = 4.5e-7 * (xd.norm(dim=1)[:, None] * Wx.double().norm(dim=0) + hd.norm(dim=1)[:, None] * Wh.double().norm(dim=0)) + 3e-6
+    pre[:, H:2 * H] += 1.0
+    want = torch.cat([torch.sigmoid(pre[:, :3 * H]), torch.tanh(pre[:, 3 * H:])], dim=1)
+    assert bool(((gates[:B].double() - want).abs() <= bar).all())
+    assert ctx.device_errors() == 0
