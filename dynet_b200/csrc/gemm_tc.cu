@@ -1052,6 +1052,7 @@ int gates_f16_pack(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I
     jobs.job[q] = F16Job{q ? Wh : Wx, 4 * H, q ? H : I, 4 * H, 4 * H, F16_ELEM, scale + q * 4 * H, hi + at, lo + at};
     jobs.job[q].perm_H = H;
   }
+  jobs.words = scale; jobs.n_words = 8 * (size_t)H;
   return dyb200_f16_pack(ctx, &jobs);
 }
 

@@ -575,8 +575,9 @@ int layer_inputs(dyb200_ctx* ctx, dyb200_wgrad* deferred, const float* Wx, const
 // Layers from 512 units on whose batch is in whole 64-column tiles and whose tiles are all resident (one CTA per SM: 225 KB of shared memory); the
 // TF32 form serves narrower ones.  64-column tiles where there are SMs for them (us per step, I = H = 1024, TF32 / this form with 128 / with 64
 // columns: batch 128 16.5 / 14.3 / 10.5, 256 23.3 / 17.4 / 14.8; batch 512 has 128 columns only, 40.8 / 25.4; batch 64 11.1 / - / 9.0), then as
-// many K splits as there are SMs for, four k-blocks each and more (as clusters whatever dyb200_ctx_cluster_splitk says: there is no other form, and
-// another number of splits would give other bits).
+// many K splits as there are SMs for, four k-blocks each on average and more (Wx and Wh are cut separately, so the last share may be short or
+// empty: 9 + 9 k-blocks make 6, 6, 6, 0, the longest still shorter than the 10 of two splits).  They are clusters whatever dyb200_ctx_cluster_splitk
+// says: there is no other form, and another number of splits would give other bits.
 bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* bn, uint32_t* S) {
   if (H < 512 || H % 32 != 0 || I == 0 || I % 4 != 0 || B == 0 || B % 64 != 0) return false;
   const uint32_t sms = (uint32_t)ctx->sm_count, tiles_m = 4 * H / BM, kb = (I + 63) / 64 + (H + 63) / 64;
@@ -633,7 +634,7 @@ int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q) {
   a.h16_hi = p.h16_hi; a.h16_lo = p.h16_lo; a.h16_pitch = hp;
   a.ready = ctx->dev_flags + DYB200_DEV_SEQ0;
   a.flags = ctx->dev_flags;
-  DYB_CUDA(ctx, cudaMemsetAsync(a.ready, 0, 32 * sizeof(uint32_t), ctx->stream));
+  if (T > 1) DYB_CUDA(ctx, cudaMemsetAsync(a.ready, 0, 32 * sizeof(uint32_t), ctx->stream));   // (a single step's CTAs count, but nobody waits)
   return seq_fwd_dispatch<true>(SEQ_LAUNCH, bn, S, ctx, &tm, &a, dim3(G / BM, B / bn, S), 2.0 * G * (double)B * (I + H) * T, I + H);
 }
 
