@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_base_slot;
   if (S > 1) cluster_sync_all();   // every CTA's barriers exist before anyone arrives on them remotely
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  dyb_grid_dep_wait();
 
   if (warp == 0) {
     if (elect_one()) {
@@ -457,6 +457,11 @@ int launch_seq_fwd(dyb200_ctx* ctx, const TmapPack& tm, const SeqFwd& a, dim3 gr
     (void)cudaGetLastError();
     if (ctx->seq_coop == 1) return dyb200_fail(ctx, DYB200_ECUDA, "sequence kernel launch failed: %s", cudaGetErrorString(e));
     ctx->seq_coop = -1;
+  }
+  if (F16 && a.T == 1 && ctx->pdl) {   // (a single step's prologue runs beside the short kernel that makes its pairs)
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
   }
   cfg.attrs = attr; cfg.numAttrs = na;
   GemmProfScope scope(ctx, flops, F16 ? 2 : 1, 4 * a.H, a.B * a.T, K, EPI_LSTM_CELL);
