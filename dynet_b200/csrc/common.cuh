@@ -38,7 +38,7 @@ struct dyb200_ctx {
   int param_cache_on;
   // per-device facts this context has established on its device: kernels whose dynamic shared-memory limit is raised
   // (bit per kernel family) and how many thread-block clusters of each size fit on the GPU at once
-  uint32_t func_attr_done;
+  uint32_t func_attr_done, gemm_attr_done;   // (the second one: gemm_tc.cu's kernels)
   int max_clusters[2][9];
   // sequence-persistent LSTM kernels (one launch per layer instead of one per time step): on by default
   int seq_kernels;

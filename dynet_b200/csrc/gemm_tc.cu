@@ -1328,33 +1328,38 @@ int dyb200_tc_param2(dyb200_ctx* ctx, const float* src, uint32_t rows, const flo
   return rc;
 }
 
-// The kernels' limits on dynamic shared memory (function attributes are per device: the context remembers what it has set on its own).
-static int gemm_tc_limits(dyb200_ctx* ctx) {
-  if (ctx->func_attr_done & 1u) return DYB200_OK;
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<128, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<64, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-  DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_persist<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PERSIST_BYTES));
-  ctx->func_attr_done |= 1u;
+// The kernels by tile width and form.  Their limit on dynamic shared memory is raised when one is first asked for (function attributes are per
+// device, so the context remembers what it has set on its own; a limit loads its kernel, and a program needs a few of them).
+using TcKernel = void (*)(TmapPack, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, GemmEpilogue, uint32_t*);
+using PersistKernel = void (*)(TmapPack, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, GemmEpilogue, uint32_t*);
+enum TcKind { TC_TF32, TC_F16, TC_TWO };
+template <class K>
+static int tc_limit(dyb200_ctx* ctx, uint32_t index, K kernel, int bytes) {
+  if (ctx->gemm_attr_done & (1u << index)) return DYB200_OK;
+  DYB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  ctx->gemm_attr_done |= 1u << index;
   return DYB200_OK;
+}
+static int tc_kernel(dyb200_ctx* ctx, uint32_t bn, bool cluster, TcKind kind, TcKernel* k) {
+  static const TcKernel table[3][2][2] = {{{k_gemm_tc<64, false>, k_gemm_tc<128, false>}, {k_gemm_tc<64, true>, k_gemm_tc<128, true>}},
+                                          {{k_gemm_tc<64, false, true>, k_gemm_tc<128, false, true>}, {k_gemm_tc<64, true, true>, k_gemm_tc<128, true, true>}},
+                                          {{k_gemm_tc<64, false, false, true>, k_gemm_tc<128, false, false, true>}, {k_gemm_tc<64, true, false, true>, k_gemm_tc<128, true, false, true>}}};
+  const uint32_t w = bn == 64 ? 0 : 1, c = cluster ? 1 : 0;
+  *k = table[kind][c][w];
+  return tc_limit(ctx, 4 * kind + 2 * c + w, *k, SMEM_BYTES);
+}
+static int persist_kernel(dyb200_ctx* ctx, uint32_t bn, bool f16, PersistKernel* k) {
+  static const PersistKernel table[2][2] = {{k_gemm_persist<64>, k_gemm_persist<128>}, {k_gemm_persist<64, true>, k_gemm_persist<128, true>}};
+  const uint32_t w = bn == 64 ? 0 : 1, f = f16 ? 1 : 0;
+  *k = table[f][w];
+  return tc_limit(ctx, 12 + 2 * f + w, *k, SMEM_PERSIST_BYTES);
 }
 // Whether `clusters` clusters of S one-tile CTAs are resident at once (asked for once per device, tile width and size).
 static bool cluster_fits(dyb200_ctx* ctx, uint32_t bn, uint32_t S, uint32_t clusters) {
   int& mc = ctx->max_clusters[bn == 64 ? 0 : 1][S];
   if (mc == 0) {
-    if (gemm_tc_limits(ctx)) return false;
+    TcKernel k;
+    if (tc_kernel(ctx, bn, true, TC_TF32, &k)) return false;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(1, 1, S); cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = ctx->stream;
@@ -1363,7 +1368,7 @@ static bool cluster_fits(dyb200_ctx* ctx, uint32_t bn, uint32_t S, uint32_t clus
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = S;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    const cudaError_t e = bn == 64 ? cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<64, true>, &cfg) : cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<128, true>, &cfg);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k, &cfg);
     if (e != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
     mc = n > 0 ? n : -1;
   }
@@ -1375,7 +1380,6 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   EncodeTiledFn enc;
   int rc = get_encoder(ctx, &enc);
   if (rc) return rc;
-  if ((rc = gemm_tc_limits(ctx))) return rc;
   const uint32_t bn = tile_cols(N);
   TmapPack tm;
   memset(&tm, 0, sizeof(tm));
@@ -1446,7 +1450,8 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       cfg.gridDim = dim3(grid.x, grid.y, Sc);
       attr[0].val.clusterDim.z = Sc;
       GemmProfScope scope(ctx, flops, f16 ? 2 : 1, M, N, kb_total * el, (uint32_t)epi.mode);
-      auto kern = f16 ? (bn == 64 ? k_gemm_tc<64, true, true> : k_gemm_tc<128, true, true>) : (bn == 64 ? k_gemm_tc<64, true> : k_gemm_tc<128, true>);
+      TcKernel kern;
+      if ((rc = tc_kernel(ctx, bn, true, f16 ? TC_F16 : TC_TF32, &kern))) return rc;
       cudaLaunchKernelEx(&cfg, kern, tm, M, N, kb0, kb1, kb_per_split, epi, ctx->dev_flags);
       DYB_LAUNCHED(ctx);
       return DYB200_OK;
@@ -1507,7 +1512,8 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
       // grouped tile order when the A operand has many row blocks (unless the last round runs apart as part of the last
       // column of tiles, which relies on the row-block-fastest order)
       const uint32_t gm = (tail_form != 1 && rows_run > 16) ? 16u : 0u;
-      auto kern = f16 ? (bn == 64 ? k_gemm_persist<64, true> : k_gemm_persist<128, true>) : (bn == 64 ? k_gemm_persist<64> : k_gemm_persist<128>);
+      PersistKernel kern;
+      if ((rc = persist_kernel(ctx, bn, f16, &kern))) return rc;
       dyb_launch(kern, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb0, kb1, rows_run, tiles_run, gm, Sp, pepi, ctx->dev_flags);
       DYB_LAUNCHED(ctx);
       if (Sp > 1 && (rc = dyb200_splitk_reduce(ctx, ppart, Sp, M, N, epi))) return rc;
@@ -1534,7 +1540,8 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   {
     // times the MMA kernel (and the split-K reduction); the packing launches show up in the step time
     GemmProfScope scope(ctx, flops, f16 ? 2 : 1, M, N, kb_total * el, (uint32_t)epi.mode);
-    auto kern = f16 ? (bn == 64 ? k_gemm_tc<64, false, true> : k_gemm_tc<128, false, true>) : (bn == 64 ? k_gemm_tc<64, false> : k_gemm_tc<128, false>);
+    TcKernel kern;
+    if ((rc = tc_kernel(ctx, bn, false, f16 ? TC_F16 : TC_TF32, &kern))) return rc;
     dyb_launch(kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb0, kb1, kb_per_split, kepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);
     if (S > 1 && epi.mode == EPI_LSTM_CELL) {
@@ -1613,7 +1620,6 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
     const double t = ceil((double)tiles * S / sms) * (((kb + S - 1) / S) * t_kb + 3.0) + 6.0 + (S + 2) * 4.0e-6 * M * N / 5.0 + 5.0;
     if (t < 0.97 * cost) { cost = t; Sp = S; }
   }
-  if ((rc = gemm_tc_limits(ctx))) return rc;
   const dim3 grid(tiles_m, (N + bn - 1) / bn, 1);
   const bool through_memory = Sp == 0 && Sc > 1 && !ctx->cluster_splitk;   // (dyb200_ctx_cluster_splitk: the clusters' splits, the same partial tiles)
   if (through_memory) Sp = Sc;
@@ -1622,10 +1628,12 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
     Sp = 0;
     if (!ctx->cluster_splitk) Sc = 1;
   }
+  TcKernel kern;
   if (Sp == 0) {
+    if ((rc = tc_kernel(ctx, bn, Sc > 1, TC_TWO, &kern))) return rc;
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
     if (Sc == 1) {
-      dyb_launch(bn == 64 ? k_gemm_tc<64, false, false, true> : k_gemm_tc<128, false, false, true>, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
+      dyb_launch(kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
     } else {
       cudaLaunchConfig_t cfg;
       memset(&cfg, 0, sizeof(cfg));
@@ -1634,7 +1642,7 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = Sc;
       cfg.attrs = attr; cfg.numAttrs = 1;
-      cudaLaunchKernelEx(&cfg, bn == 64 ? k_gemm_tc<64, true, false, true> : k_gemm_tc<128, true, false, true>, tm, M, N, kb, 0u, (kb + Sc - 1) / Sc, epi, ctx->dev_flags);
+      cudaLaunchKernelEx(&cfg, kern, tm, M, N, kb, 0u, (kb + Sc - 1) / Sc, epi, ctx->dev_flags);
     }
     DYB_LAUNCHED(ctx);
     return DYB200_OK;
@@ -1643,15 +1651,18 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   float* const part = (float*)pw;
   const GemmEpilogue pepi{EPI_STORE, part, M, nullptr, 0, 0.f, nullptr, 0, 0};
   if (through_memory) {
+    if ((rc = tc_kernel(ctx, bn, false, TC_TWO, &kern))) return rc;
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
-    dyb_launch(bn == 64 ? k_gemm_tc<64, false, false, true> : k_gemm_tc<128, false, false, true>, dim3(grid.x, grid.y, Sp), kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u,
+    dyb_launch(kern, dim3(grid.x, grid.y, Sp), kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u,
                (kb + Sp - 1) / Sp, pepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);
   } else {
     tm.store_map = M % 4 == 0;
     if (tm.store_map && (rc = dyb200_tc_make_store_map(ctx, &tm.t[4], part, M, N, Sp, M, 64))) return rc;
+    PersistKernel persist;
+    if ((rc = persist_kernel(ctx, bn, false, &persist))) return rc;
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
-    dyb_launch(bn == 64 ? k_gemm_persist<64> : k_gemm_persist<128>, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb, 0u, tiles_m, tiles, tiles_m > 16 ? 16u : 0u,
+    dyb_launch(persist, dim3(ctx->sm_count), kThreads, SMEM_PERSIST_BYTES, ctx, tm, M, N, kb, 0u, tiles_m, tiles, tiles_m > 16 ? 16u : 0u,
                Sp, pepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);
   }
