@@ -645,6 +645,11 @@ int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q) {
 
 extern "C" {
 
+// Whether the forward products of such a layer run on fp16 pairs (1 or 0), and their column tile and K splits.
+int dyb200i_seq_f16_tiling(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* tile, uint32_t* splits) {
+  return dyb200_seq_f16_plan(ctx, I, H, B, tile, splits) ? 1 : 0;
+}
+
 int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0,
                                 const dyb200_tensor* Wx, const dyb200_tensor* Wh, const dyb200_tensor* b,
                                 const dyb200_tensor* mask_x, const dyb200_tensor* mask_h, const dyb200_lstm_gates_attrs* attrs,

@@ -14,11 +14,19 @@ pytestmark = pytest.mark.gpu
     (1, 1, 1500, 4103, 2111, False),     # K-major A, MN-major B
     (0, 0, 20000, 1500, 520, False),     # many tiles, less than one accumulation chain
     (1, 0, 130, 1200, 80000, False),     # a long reduction over few tiles: K splits
+    # a side of at most 128: one SM per tile (those above are products of the pair kernel)
+    (0, 1, 50000, 128, 4096, True),      # persistent, 128 columns
+    (0, 0, 20000, 64, 4000, False),      # persistent, 64 columns
+    (0, 0, 19999, 63, 4004, True),       # ... and edges
+    (1, 0, 100, 12000, 12000, True),     # one row of tiles
+    (0, 1, 128, 1200, 90000, True),      # K splits
+    (1, 0, 128, 300, 120000, False),
+    (0, 1, 1030, 128, 100000, False),
 ])
 def test_large_product(tA, tB, M, N, K, accumulate):
     import torch
     import gpu_util as g
-    assert 2.0 * M * N * K > 24e9 or K == 80000
+    assert 2.0 * M * N * K > 8e9
     gen = torch.Generator("cuda").manual_seed(M + N)
     A = torch.randn(*((M, K) if tA else (K, M)), device="cuda", generator=gen)
     B = torch.randn(*((N, K) if tB == 0 else (K, N)), device="cuda", generator=gen)
@@ -84,7 +92,7 @@ def test_parameter_rows_keep_their_own_scale(tA, cache):
     assert ctx.device_errors() == 0
 
 
-@pytest.mark.parametrize("V,H,n,param", [(12000, 256, 4000, False), (12001, 250, 4003, True)])
+@pytest.mark.parametrize("V,H,n,param", [(12000, 256, 4000, False), (12001, 250, 4003, True), (12000, 128, 8100, False), (12001, 64, 5600, True)])
 def test_output_gradient_at_every_row_and_columns_own_scale(V, H, n, param):
     """softmax_output_bwd_fused on fp16 pairs: vocabulary rows whose probability is tiny everywhere, columns whose dE/df differs by 2^40.
     Against float64, every element of dR and dh relative to its own |row| |column|.  Bar: exp of arguments down to -65 (log2: 94) from

@@ -41,3 +41,23 @@ def test_pair_product(tA, tB, M, N, K, accumulate):
         g.ctx().gemm(tA, tB, M, N, K, A.data_ptr(), K if tA else M, B.data_ptr(), K if tB == 0 else N, again.data_ptr(), M, 0)
         assert torch.equal(C, again)
     assert g.ctx().device_errors() == 0
+
+
+def test_subnormal_results_are_kept():
+    """An accumulated product leaves as TMA adds: results and summands below 2^-126 stay what plain adds make of them."""
+    import torch
+    import gpu_util as g
+    M, N, K = 8000, 3000, 512
+    gen = torch.Generator("cuda").manual_seed(1)
+    A, B = torch.randn(K, M, device="cuda", generator=gen) * 1e-20, torch.rand(N, K, device="cuda", generator=gen) * 1e-21
+    A[:, ::2] = 0.0
+    C = torch.rand(N, M, device="cuda", generator=gen) * 2e-38 - 1e-38
+    C[:, ::4] = 1e-40
+    before = C.double()
+    g.ctx().gemm(0, 0, M, N, K, A.data_ptr(), M, B.data_ptr(), K, C.data_ptr(), M, 1)
+    assert torch.equal(C.double()[:, ::2], before[:, ::2])
+    # (the bar above, and the roundings of the product and of the sum to multiples of 2^-149)
+    want = B.double() @ A.double() + before
+    bar = 4.5e-7 * B.double().norm(dim=1)[:, None] * A.double().norm(dim=0)[None, :] + 2.0 ** -149
+    assert bool(((C.double() - want).abs() <= bar).all())
+    assert g.ctx().device_errors() == 0

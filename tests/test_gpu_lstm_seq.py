@@ -2,9 +2,9 @@
 they replace: gates, cell and hidden states of every step, dE/dx, dE/dh and dE/dc of every step, the bias gradient and the
 weight gradients that the recorded operand planes produce must agree BIT FOR BIT, and the forward values must match the CPU
 oracle (the backward values of the per-step calls are checked against it in test_gpu_parity.py / test_gpu_lm.py).
-Shapes: one tile per CTA (batch 512 and 384), K splits reduced inside a thread-block cluster with 128-column tiles (batch 256:
-2 splits, batch 128: 4) and with 64-column tiles (batch 64), batch-1 masks, a layer whose input is narrower than its state,
-and shapes the kernels decline (per-step calls inside)."""
+Shapes: from 512 units on, where the forward products are of fp16 pairs, one tile per CTA (batch 512, 384 and 256) and K splits reduced inside a
+thread-block cluster (batch 128: 2, batch 64: 4); below, on TF32 pairs, 64- and 128-column tiles with K splits; batch-1 masks, a layer whose
+input is narrower than its state, and shapes the kernels decline (per-step calls inside)."""
 import numpy as np
 import pytest
 
@@ -98,10 +98,15 @@ def _same(seq, per):
     (512, 1024, 512, 4, True, True, True, True),      # benchmark layer 1 on one GPU: one tile per CTA, 128 CTAs
     (1024, 1024, 64, 6, True, True, True, True),      # benchmark layer 2 on 8 GPUs: 64-column tiles, 4 K splits per cluster
     (512, 1024, 64, 5, True, False, True, True),      # layer 1 on 8 GPUs, batch-1 masks
-    (1024, 1024, 128, 3, True, True, True, True),     # 4 GPUs: 128-column tiles, 4 K splits per cluster
-    (512, 1024, 256, 3, False, True, True, True),     # 2 GPUs: 2 K splits per cluster, no dropout
+    (1024, 1024, 128, 3, True, True, True, True),     # 4 GPUs: 64-column tiles, 2 K splits per cluster
+    (512, 1024, 256, 3, False, True, True, True),     # 2 GPUs: 64-column tiles, no split, no dropout
     (256, 1024, 384, 3, True, True, True, True),      # three column blocks, one tile per CTA
-    (256, 512, 384, 3, True, True, False, True),      # 3 K splits: 48 clusters of 3 do not fit on the GPU at once -> per-step calls
+    (256, 512, 384, 3, True, True, True, True),       # six 64-column blocks
+    (128, 256, 64, 4, True, True, True, True),        # TF32 pairs: 64 columns
+    (128, 256, 64, 3, False, True, True, True),
+    (256, 256, 128, 4, True, False, True, True),      # 128 columns, batch-1 masks
+    (256, 256, 256, 3, True, True, True, True),       # two blocks of them
+    (300, 416, 128, 3, False, True, True, False),     # the last k-blocks partly filled
     (128, 256, 96, 3, True, True, False, False),       # 96 columns are not whole tiles: per-step calls inside
     (32, 64, 8, 3, True, True, False, False),          # far below the tensor path
 ])

@@ -1,27 +1,37 @@
 """The forward recurrence of wide layers on fp16 pairs (csrc/lstm_seq.cu, F16): reductions that are no multiple of a k-block or longer than a
-chain, one to eight K splits, 64- and 128-column tiles, masks per column and for all, an initial state far above 1, columns of x that differ
+chain, K splits with even, short and empty last shares, 64- and 128-column tiles, masks per column and for all, an initial state far above 1, columns of x that differ
 by 2^60 and a column of zeros, the slots of h in turn.  Step by step against float64 from the device's own h_{t-1} and c_{t-1}.  Bar of a
 pre-activation: 4.5e-7 of |row of Wx| |x| + |row of Wh| |h .* mask|, that of every product on fp16 pairs; of a gate: that (its slope is at
 most 1) and 3e-6 for the approximate exponential and reciprocal.  The single-step calls must give the same bits, also where
 saturated gates leave elements of h far below 2^-28."""
+import ctypes as C
+
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("I,H,B,T,mask", [
-    (300, 544, 64, 4, "full"),       # tails in both reductions, eight splits
-    (1100, 1056, 64, 3, None),       # chains cut within both products, lines longer than a warp holds
-    (4, 512, 192, 3, "one"),         # the shortest x, three column blocks
-    (512, 1024, 256, 2, "full"),     # one split, 64 columns
-    (36, 1024, 512, 3, "one"),       # 128 columns
-    (1024, 2048, 128, 2, None),      # a reduction of 48 k-blocks
+# splits: of the rule on 148 SMs, and where the number of clusters that fit differs between GPUs both
+@pytest.mark.parametrize("I,H,B,T,mask,tile,splits", [
+    (300, 544, 64, 4, "full", 64, (2,)),       # tails in both reductions
+    (1100, 1056, 64, 3, None, 64, (4,)),       # chains cut within both products, lines longer than a warp holds
+    (4, 512, 192, 3, "one", 64, (2,)),         # the shortest x, three column blocks
+    (512, 1024, 256, 2, "full", 64, (1,)),
+    (36, 1024, 512, 3, "one", 128, (1,)),
+    (1024, 2048, 128, 2, None, 64, (1,)),      # a reduction of 48 k-blocks
+    (1536, 512, 64, 3, "full", 64, (8, 4)),
+    (576, 576, 64, 3, None, 64, (4,)),         # 9 + 9 k-blocks: the last share is empty
+    (576, 576, 128, 3, "one", 64, (2, 4)),     # (thirty-six clusters of four are more than most GPUs hold)
+    (640, 576, 64, 2, "full", 64, (4,)),       # ... or has one
 ])
-def test_sequence_of_a_wide_layer(I, H, B, T, mask):
+def test_sequence_of_a_wide_layer(I, H, B, T, mask, tile, splits):
     import torch
     import gpu_util as g
     from dynet_b200 import capi
     ctx = g.ctx()
+    bn, S = C.c_uint32(), C.c_uint32()
+    assert ctx.L.dyb200i_seq_f16_tiling(ctx.h, I, H, B, C.byref(bn), C.byref(S)) == 1
+    assert bn.value == tile and S.value in splits, (bn.value, S.value)
     gen = torch.Generator("cuda").manual_seed(H + B)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
     x, h0, c0, b = rnd(T * B, I), rnd(B, H) * 30.0, rnd(B, H), rnd(4 * H) * 0.1

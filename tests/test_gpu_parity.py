@@ -730,7 +730,7 @@ def test_gemm(g, tA, tB, M, N, K):
         assert_close(g.host(C_), want, TOL_REDUCE, floor=0.1 * K ** 0.5 + 1.0, what="gemm %d%d acc=%d" % (tA, tB, acc))
 
 
-@pytest.mark.parametrize("M,N,K,acc", [(2048, 512, 4096, 1), (1536, 512, 4096, 1), (4096, 64, 2048, 0), (1024, 200, 1100, 1), (512, 96, 3000, 0)])
+@pytest.mark.parametrize("M,N,K,acc", [(2048, 512, 3800, 1), (1536, 512, 4096, 1), (4096, 64, 2048, 0), (1024, 200, 1100, 1), (512, 96, 3000, 0)])
 def test_gemm_cluster_split_equals_workspace_split(g, M, N, K, acc):
     """Products whose K is split: the cluster form (partial tiles reduced through distributed shared memory) and the
     workspace form (second kernel) add the partial tiles in the same order, so they agree bit for bit."""
