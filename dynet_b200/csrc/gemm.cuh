@@ -48,7 +48,6 @@ struct GemmEpilogue {
   const float* hmask = nullptr; uint32_t hmask_ld = 0; int hmask_full = 0;
   // Two right operands side by side (TmapPack::n_split): columns [0, n_live) belong to C, those from n_split on to Cn, the ones between do not exist.
   uint32_t n_split = 0, n_live = 0; float* Cn = nullptr; uint32_t ldcn = 0;
-  const uint32_t* only_if = nullptr;   // (dyb200_tc_gemm_packed2) a device word: the kernel runs where it is not zero
 };
 #ifdef __CUDACC__
 // The destination of a tile whose first column is n0 (a tile lies on one side): C, n0 and the end of its columns N.

@@ -61,9 +61,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
                                                          uint32_t kb0, uint32_t kb1, uint32_t kb_per_split,
                                                          GemmEpilogue epi, uint32_t* flags) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (the wait comes after the prologue, below)
-  if (TWO && !CLUSTER && epi.only_if) {
+  if (TWO && !CLUSTER && tm.sa) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!*(const volatile uint32_t*)epi.only_if) return;   // (the same in every CTA)
+    if (!*(const volatile uint32_t*)tm.sa) return;   // (the same in every CTA)
   }
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -776,6 +776,8 @@ __device__ __forceinline__ float4 f16_load4(const float* line, uint32_t e, uint3
   for (uint32_t i = 0; i < 4; ++i) v[i] = e + i < n ? line[e + i] : 0.f;
   return make_float4(v[0], v[1], v[2], v[3]);
 }
+// LOW: jobs with `low` words (F16Jobs::wide).
+template <bool LOW>
 __global__ void __launch_bounds__(256) k_f16_absmax(const __grid_constant__ F16Jobs jobs) {
   dyb_grid_dep_sync();
   const uint32_t z = f16_job_of(jobs), unit = blockIdx.x - jobs.start[z];
@@ -783,7 +785,7 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const __grid_constant__ F16J
   const bool vec = (j.ld & 3) == 0 && aligned16(j.src);
   const F16Units us = f16_max_units(j);
   if (j.mode == F16_ELEM) {   // four positions per thread; short lines: groups of threads with lines of their own meet in shared memory
-    __shared__ uint32_t top[1024], bot[1024];
+    __shared__ uint32_t top[1024], bot[LOW ? 1024 : 1];
     const uint32_t q = us.groups > 1 ? (j.n + 3) / 4 : 256u, grp = threadIdx.x / q, e = 4 * ((unit % us.x) * 256 + threadIdx.x % q);
     const uint32_t l0 = (unit / us.x * us.groups + grp) * kMaxLines;
     const bool live = grp < us.groups && e < j.n;
@@ -806,22 +808,22 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const __grid_constant__ F16J
           w[0] = max(w[0], finite_mag(v[k].x)); w[1] = max(w[1], finite_mag(v[k].y)); w[2] = max(w[2], finite_mag(v[k].z)); w[3] = max(w[3], finite_mag(v[k].w));
         }
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) { m[i] = max(m[i], w[i]); if (w[i]) low[i] = max(low[i], ~w[i]); }
+        for (uint32_t i = 0; i < 4; ++i) { m[i] = max(m[i], w[i]); if (LOW && w[i]) low[i] = max(low[i], ~w[i]); }
       }
     }
     if (us.groups > 1) {
-      for (uint32_t i = threadIdx.x; i < 1024; i += 256) top[i] = bot[i] = 0;
+      for (uint32_t i = threadIdx.x; i < 1024; i += 256) { top[i] = 0; if (LOW) bot[i] = 0; }
       __syncthreads();
       if (live) {
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) { atomicMax(top + e + i, m[i]); if (j.low) atomicMax(bot + e + i, low[i]); }
+        for (uint32_t i = 0; i < 4; ++i) { atomicMax(top + e + i, m[i]); if (LOW) atomicMax(bot + e + i, low[i]); }
       }
       __syncthreads();
-      for (uint32_t i = threadIdx.x; i < j.n; i += 256) { atomicMax(j.scale + i, top[i]); if (j.low) atomicMax(j.low + i, bot[i]); }
+      for (uint32_t i = threadIdx.x; i < j.n; i += 256) { atomicMax(j.scale + i, top[i]); if (LOW) atomicMax(j.low + i, bot[i]); }
     } else if (live) {
 #pragma unroll
       for (uint32_t i = 0; i < 4; ++i)
-        if (e + i < j.n) { atomicMax(j.scale + e + i, m[i]); if (j.low) atomicMax(j.low + e + i, low[i]); }
+        if (e + i < j.n) { atomicMax(j.scale + e + i, m[i]); if (LOW) atomicMax(j.low + e + i, low[i]); }
     }
     return;
   }
@@ -1138,7 +1140,7 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
     DYB_CHECK_ARG(ctx, end < 0x7fffffffull, "fp16 planes: operand too large (%u x %u)", j.lines, j.n);
     jobs->start[k + 1] = (uint32_t)end;
   }
-  dyb_launch(k_f16_absmax, jobs->start[jobs->n], 256, 0, ctx, *jobs);
+  dyb_launch(jobs->wide ? k_f16_absmax<true> : k_f16_absmax<false>, jobs->start[jobs->n], 256, 0, ctx, *jobs);
   DYB_LAUNCHED(ctx);
   for (int k = 0; k < jobs->n; ++k) {
     const uint64_t end = jobs->start[k] + ((uint64_t)((jobs->job[k].n + 3) / 4) * jobs->job[k].lines + kSplitItems - 1) / kSplitItems;
@@ -1600,7 +1602,8 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   if (!N1) { tm.t[6] = tm.t[2]; tm.t[7] = tm.t[3]; }   // (n_split = 0: every tile is of the second side)
   tm.t[4] = tm.t[0]; tm.t[5] = tm.t[1];
   GemmEpilogue epi{EPI_ACCUM, C0, ldc0, nullptr, 0, 0.f, nullptr, 0, 0};
-  epi.n_split = split; epi.n_live = N0; epi.Cn = C1; epi.ldcn = ldc1; epi.only_if = only_if;
+  epi.n_split = split; epi.n_live = N0; epi.Cn = C1; epi.ldcn = ldc1;
+  tm.sa = only_if;
   const double flops = 2.0 * M * (double)(N0 + N1) * A.K, sms = (double)ctx->sm_count, t_kb = bn == 64 ? 0.40 : 0.66;
   // one tile per CTA (in waves: 2816 x (704 + 704) over 35 columns 22 us, 29 as work items of the persistent kernel), or clusters of S splits
   // that are all resident, at least eight k-blocks each (shorter splits end sooner on an idle GPU, but hold several times the SMs: three

@@ -12,7 +12,8 @@
 // plane[k * pitch + m], the layout of a K x M row-major matrix - and t[0], t[1] are 3-D maps over (m within a group of 32,
 // k, group) with a box of 32 x 32 x 4; see load_a_tile / umma_desc_mn.  b_mn: the same for the B planes (t[2], t[3]; the
 // box holds as many groups as the tile has columns / 32).
-// F16 products (see "2 x 11 bits" in gemm.cuh): sa / sb are the scale words of the operands' rows.
+// F16 products (see "2 x 11 bits" in gemm.cuh): sa / sb are the scale words of the operands' rows.  TF32 products of two right operands: sa is a
+// device word or null, and where the word is zero the kernel does nothing (a field of its own in GemmEpilogue cost every product 0.15 us).
 struct TmapPack { CUtensorMap t[8]; uint32_t a_mn, b_mn; const uint32_t *sa, *sb;
   uint32_t store_map;      // t[4] describes the output (persistent kernel, plain stores; one pair)
   uint32_t n_split; };     // columns from here on are those of a second right operand, t[6] and t[7] (0: none; one pair, a multiple of the tile)
