@@ -1580,8 +1580,8 @@ int dyb200_splitk_reduce(dyb200_ctx* ctx, const float* part, uint32_t S, uint32_
 // Two products with one left operand, C0 += A B0^T and C1 += A B1^T, as one over the columns of both (each side's columns rounded up to whole
 // tiles): a short product of its own is mostly pipeline fill and epilogue, and the few tiles of one leave SMs idle.  K splits as clusters
 // where they fit, or as work items of the persistent kernel with a second stage, by the estimates of dyb200_tc_splits.
-// us for both, as two launches / in one: 1024 x (128 + 256), K = 1600 38 / 22, 13000 99 / 69, 107000 538 / 378; 1200 x (200 + 300) x 1050 36 / 26;
-// 2048 x (512 + 512) x 4480 120 / 103.
+// us for a flush (events), as two launches / in one: 1024 x (128 + 256), K = 300 36 / 22, 520 44 / 21, 1600 38 / 21, 13000 99 / 68, 107000 538 / 378;
+// 1200 x (200 + 300) x 1050 36 / 27; 512 x (32 + 128) x 10560 71 / 34; 2816 x (704 + 704) x 35 28 / 27; 2048 x (512 + 512) x 4480 120 / 103.
 int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const PackedOp* B, float* C0, uint32_t ldc0, float* C1, uint32_t ldc1,
                            const uint32_t* only_if) {
   EncodeTiledFn enc;
@@ -1606,8 +1606,9 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   tm.sa = only_if;
   const double flops = 2.0 * M * (double)(N0 + N1) * A.K, sms = (double)ctx->sm_count, t_kb = bn == 64 ? 0.40 : 0.66;
   // one tile per CTA (in waves: 2816 x (704 + 704) over 35 columns 22 us, 29 as work items of the persistent kernel), or clusters of S splits
-  // that are all resident, at least eight k-blocks each (shorter splits end sooner on an idle GPU, but hold several times the SMs: three
-  // language models of 256 units on three streams took 133 us a step with two k-blocks per split, 119 with eight)
+  // that are all resident, at least eight k-blocks each.  Two k-blocks end hardly sooner on an idle GPU and hold several times the SMs; us with
+  // two / with eight: a flush of 1024 x (128 + 256) over 300 columns 20.5 / 22.2, 800 20.9 / 20.5, 1600 21.2 / 20.8; a step of a language model of
+  // 256 units alone 222 / 226, three on three streams 134 / 119; a tagger of 16 sentences alone 532 / 524, three 256 / 237.
   uint32_t Sc = 0;
   double cost = 1e30;
   for (uint32_t S = 1; S <= (only_if ? 1u : 8u) && (S == 1 || kb / S >= 8); ++S) {
