@@ -406,8 +406,8 @@ int dyb200_trainer_update(int rule, float* params, float* grads, float* state0, 
 /* ---- GEMM used by the LSTM gates (dynet/matrix-multiply.h:16-37, :97-117, :162-180) ----
  * C[M x N] (+)= op(A) * op(B), column-major, fp32 in/out.  Up to 32 columns, and with a narrow side and a long one, on
  * the CUDA cores in fp32; else on the tensor pipe as three products of TF32 pairs or, from 24 GFLOP on (8 with K >= 256), of fp16
- * pairs whose rows of op(A) and columns of op(B) are scaled by their largest value (2 x 11 bits either way); shapes too small for that on the
- * CUDA cores.  transA/transB as in BLAS. */
+ * pairs whose rows of op(A) and columns of op(B) are scaled by their largest value (2 x 11 bits either way; an element more than 2^28 below that
+ * value keeps an absolute error of 2^-51 of it, so an error is bounded by |row| |column|); shapes too small for that on the CUDA cores.  transA/transB as in BLAS. */
 #define DYB200_GEMM_A_IS_PARAM 1u /* flags: A is a parameter matrix (see dyb200_ctx_param_cache) */
 int dyb200_gemm(int transA, int transB, uint32_t M, uint32_t N, uint32_t K, const float* A,
                 uint32_t lda, const float* B, uint32_t ldb, float* C, uint32_t ldc, int accumulate,
