@@ -318,6 +318,11 @@ bool dyb200_pair_takes(const dyb200_ctx* ctx, uint32_t M, uint32_t N, const Gemm
 int dyb200_gemm_pair(dyb200_ctx* ctx, TmapPack* tm, uint32_t M, uint32_t N, uint32_t kb, double flops, const GemmEpilogue& epi, const uint32_t* unless) {
   if (!(ctx->func_attr_done & (1u << 24))) {
     DYB_CUDA(ctx, cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PAIR_BYTES));
+    // (the epilogue warps' share comes out of what the block is launched with; a build with fewer registers would wait for it without end)
+    cudaFuncAttributes fa;
+    DYB_CUDA(ctx, cudaFuncGetAttributes(&fa, k_gemm_pair));
+    DYB_CHECK_ARG(ctx, 3 * fa.numRegs >= kPairRegsLow + 2 * kPairRegsHigh, "pair kernel built with %d registers per thread, its split needs %d", fa.numRegs,
+                  (kPairRegsLow + 2 * kPairRegsHigh) / 3);
     ctx->func_attr_done |= 1u << 24;
   }
   const uint32_t pairs = (uint32_t)ctx->sm_count / 2;
