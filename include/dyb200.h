@@ -289,7 +289,8 @@ int dyb200_vanilla_lstm_bwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
  * (N1 > 0): dWx and dWh of a layer share the gate gradient.  The operands are TF32 pairs; wide ones (M N / (M + N) >= 800 with N = N0 + N1, 256
  * columns and more) become fp16 pairs, 2 x 11 bits with a scale per row, where each row's blocks of eight columns that are not all zero have
  * their largest value within 2^24 of the row's (looked up on the device at each flush).  push: a is M x k, b0 / b1 are N0 x k / N1 x k, all
- * column-major; mask0 / mask1 multiply b0 / b1 elementwise (batch size 1 when *_full is 0). */
+ * column-major; mask0 / mask1 multiply b0 / b1 elementwise (batch size 1 when *_full is 0).  create clears the planes on its context's stream: a
+ * first use on another stream has to be ordered after it. */
 typedef struct dyb200_wgrad dyb200_wgrad;
 int dyb200_wgrad_create(dyb200_ctx* ctx, uint32_t M, uint32_t N0, uint32_t N1, uint32_t Kcap, dyb200_wgrad** out);
 int dyb200_wgrad_destroy(dyb200_wgrad* w);
