@@ -45,6 +45,7 @@ struct dyb200_ctx {
   int seq_max_clusters[4][9];   // thread-block clusters of each size that fit at once, per tile width and kind of operand pairs (0 = not asked yet)
   int16_t rec_tc_fit[2][8];     // the same for lstm_rec_tc.cu: [pass][CTAs per cluster - 1]
   int16_t rec_fit[2][6][17];    // clusters of the recurrence kernels (lstm_rec.cu) that fit at once: [pass][width class][CTAs per cluster]
+  int16_t bwd_wide_fit[7];      // the same for lstm_bwd_wide.cu, by instantiation
   int seq_coop;                 // 0 = not tried, 1 = launched with the cooperative attribute, -1 = the driver refused it
   int wide_refused;             // the driver refused lstm_wide.cu's gang launch: its sequences run launch by launch
   uint64_t param_version, param_tick;
@@ -79,6 +80,8 @@ struct GemmProfScope {
 
 #define DYB200_DEV_WORDS 2048
 #define DYB200_DEV_SEQ0 16      // 32 words: hand-over counters of the sequence kernels (zeroed before each launch)
+#define DYB200_DEV_BWD0 48      // hand-over counters of lstm_bwd_wide.cu (zero between launches: the launch behind each of its kernels clears them)
+#define DYB200_DEV_BWD_WORDS 16
 #define DYB200_DEV_COUNTER0 64
 #define DYB200_DEV_COUNTERS (DYB200_DEV_WORDS - DYB200_DEV_COUNTER0)
 // Device error bits written into ctx->dev_flags.

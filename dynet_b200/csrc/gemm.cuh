@@ -269,6 +269,22 @@ struct SeqF16Call {
   int h0_done, emit_last;  // emit_last: rows [T B, (T + 1) B) of Hs receive the last step's h
 };
 int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q);
+// The backward pass of a wide layer on fp16 pairs (lstm_bwd_wide.cu): T steps of B columns, or a single one driven from outside - the same kernels, so
+// the same bits.  Whether a layer takes it, with the column blocks per CTA and K splits of its recurrence; the call.
+bool dyb200_bwd_wide_plan(dyb200_ctx* ctx, uint32_t H, uint32_t B, uint32_t* ncb, uint32_t* S);
+struct BwdWideCall {
+  uint32_t I, H, B, T;
+  const float *Wx, *Wh, *gates, *c, *c0;
+  float *dh, *dc;                // of all steps; a single step without dE/dc has none
+  float *dh_prev, *dc_prev;      // of the step before the first, or null
+  float* dx; const float* mx; int mx_full; const float* mh; int mh_full;   // (dx null: not wanted)
+  float* db;
+  float *dn_hi, *dn_lo; uint32_t dn_pitch;   // TF32 planes of the columns' dgates, to be filled
+};
+int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q);
+// db += row sums of dgates, part = [step][tile][G], tiles in order and then the steps (at most kDbMaxSteps); clears the counters at `done`, if any
+constexpr uint32_t kDbMaxSteps = 256;
+int dyb200_seq_db(dyb200_ctx* ctx, const float* part, uint32_t steps, uint32_t tiles, uint32_t G, float* db, uint32_t* done);
 // A 2-D tensor map (CUtensorMap, 128 bytes at `map`) over a K-major plane: box = 32 floats of K x box_rows rows, 128-byte swizzle.
 int dyb200_tc_make_tmap(dyb200_ctx* ctx, void* map, float* plane, uint32_t rows, uint32_t K, uint32_t pitch, uint32_t box_rows);
 // The same over a plane of halves (64 of K), and over an MN-major one (K lines of `rows` halves).

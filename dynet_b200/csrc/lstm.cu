@@ -692,6 +692,18 @@ int dyb200_vanilla_lstm_bwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
   const bool tiled = tensor_path && H % kCT_J == 0 && H / kCT_J <= DYB200_DEV_COUNTERS && aligned16(c_t->v) &&
                      aligned16(c_tm1->v) && aligned16(gates->v) && aligned16(dEdh->v) && (!dEdc || aligned16(dEdc->v)) &&
                      (!dc_tm1 || aligned16(dc_tm1->v));
+  uint32_t wide_ncb, wide_S;
+  if (deferred && I > 0 && (!mh || aligned16(mh)) && aligned16(gates->v) && aligned16(c_t->v) && aligned16(c_tm1->v) && aligned16(dEdh->v) &&
+      (!dEdc || aligned16(dEdc->v)) && (!dc_tm1 || aligned16(dc_tm1->v)) && (!dh_tm1 || aligned16(dh_tm1->v)) && dyb200_bwd_wide_plan(ctx, H, B, &wide_ncb, &wide_S)) {
+    // wide layers with an accumulator: the sequence's kernels, for one step (lstm_bwd_wide.cu)
+    DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_bwd_fused: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
+    BwdWideCall q{I, H, B, 1, Wx->v, Wh->v, gates->v, c_t->v, c_tm1->v, dEdh->v, dEdc ? dEdc->v : nullptr, dh_tm1 ? dh_tm1->v : nullptr, dc_tm1 ? dc_tm1->v : nullptr,
+                  dx ? dx->v : nullptr, mx, mx_full, mh, mh_full, db->v, nullptr, nullptr, 0};
+    if (at_col) rc = dyb200_wgrad_reserve_a_at(deferred, deferred_col, B, &q.dn_hi, &q.dn_lo, &q.dn_pitch, ctx);
+    else rc = dyb200_wgrad_reserve(deferred, B, &q.dn_hi, &q.dn_lo, &q.dn_pitch, x->v, I, mx, mx_full, h_tm1->v, H, mh, mh_full, ctx, &batch);
+    if (rc || (rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
+    return dyb200_bwd_wide(ctx, q);
+  }
   float* dpre = nullptr;
   if (tiled) {
     // The planes of the gate gradient (row = batch column, K = 4H) are the right operand of the dx / dh product below and,

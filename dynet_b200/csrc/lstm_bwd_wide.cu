@@ -1,0 +1,612 @@
+// The backward recurrence of wide LSTM layers (more than 384 units) on fp16 pairs: what T calls of VanillaLSTMH, VanillaLSTMC and VanillaLSTMGates
+// backward (dynet/nodes-lstm.cc:262-330, 415-470, 530-580) do in the order of the executor's backward sweep (dynet/exec.cc:96-140), with the products
+// that need no step's predecessor - dx of all columns - taken out of the chain:
+//     dh_{t-1} += mask_h .* (Wh^T dgates_t),  then the cell pass of step t - 1, which makes dgates_{t-1}      (k_bwd_wide<.., true>, resident)
+//     dx += mask_x .* (Wx^T dgates)                                            all columns, one launch        (k_bwd_wide<.., false>)
+// A CTA owns 128 units x BNT batch columns of Wh^T dgates and the share `rank` of its reduction; the S CTAs of a tile are one cluster and send each
+// other partial sums through distributed shared memory, so that CTA r finishes 1/S of the tile's columns - dE/dh and, from the same registers, the
+// cell pass of the step before.  The only hand-over through global memory is that of dgates: a counter per column block, which the next
+// product's TMA thread polls (bounded, then DYB200_FLAG_WAIT_TIMEOUT, as every wait here).
+//
+// dgates as fp16 pairs (gemm.cuh): a column's values fade by many powers of two over the steps and their largest is not known before the cell pass is
+// through everywhere, so a pair's scale belongs to (column, block of 128 units, all four gates) - what one warp of the cell pass holds.  The
+// reduction is ordered by these blocks (4 gates x 128 units = 8 k-blocks of 64), each one accumulation chain that is unscaled as it is drained.
+//
+// Measured (us per step of 35, all of a layer's backward call, I = H = 1024; TF32 pairs with dx inside the recurrence / this form): batch 512 48.2 / 30.5,
+// 256 35.8 / 17.9, 128 21.8 / 15.2, 64 16.6 / 9.9; batch 100 (a launch and more per step before) 31 / 14; 600 units, batch 30: 21 / 8.  dx is 10 of
+// the 30.5, at 430 TFLOP/s useful.  What bounds the recurrence: at batch 512, two column blocks per CTA in turn (one block of 128 columns had nothing
+// to overlap its exchange and cell pass with: 25 us a step against 20), 196 MB of operands per step from L2 at 11 - 14 TB/s; at batch 64 the chain
+// itself: 0.5 until the first pairs of dgates are there, 2.8 for 8 k-blocks, 0.5 to drain the last, 1.2 exchange, 1.0 cell pass, 0.8 until the stores are
+// out and counted, 0.5 until the count is seen.
+#include "lstm_cell.cuh"
+#include "seq_dev.cuh"
+
+namespace {
+
+struct BwdWide {
+  uint32_t T, B, H, Hp;             // steps, columns per step, units (rows of the product; dx: I), units rounded up to 64
+  uint32_t kbs;                     // k-blocks of the product
+  uint32_t P;                       // products of a column block: T - 1, and one more when dh_prev is given; dx: tiles
+  uint32_t ncb, tiles_n;            // column blocks that a CTA serves in turn, of how many (dx: 1)
+  uint32_t M, tiles_m;              // rows of the product and its tiles of 128
+  const float *gates, *cs, *c0;     // step t at + t * 4 H B / + t * H B
+  float *dh, *dc;                   // dE/dh, dE/dc of the steps (accumulated; dc may be null: none from outside, T = 1)
+  float *dh_prev, *dc_prev;         // those of the step before the first (null: not wanted)
+  float *dn_hi, *dn_lo; uint32_t dn_pitch;       // TF32 planes of dgates for the weight gradients: row = column of the sequence
+  __half *d16_hi, *d16_lo;          // fp16 pairs, row = column of the sequence, gate q's unit u at q Hp + u (zeros from H on)
+  uint32_t* dsc; uint32_t dsc_ld;   // scale words [block of 128 units][column of the sequence]
+  const uint32_t* wscale;           // of the rows of Wh^T (dx: Wx^T)
+  float* part;                      // row sums of dgates: [step in sweep order][column block, rank][4H]
+  const float* mask; int mask_full; // of the result's rows; full: one column per batch column
+  float* dx; uint32_t columns;      // dx only
+  uint32_t* done;                   // a counter per column block, zero at launch (cleared by the launch that sums up db)
+  uint32_t* flags;
+};
+
+// k-block i of the reduction: block of 128 units (i / 8), gate, half.  The last block has 64 units or fewer when H % 128 is in 1 .. 64.
+struct KBlock { int xa, xb; };
+__device__ __forceinline__ KBlock k_block(uint32_t i, uint32_t H, uint32_t Hp) {
+  const uint32_t full = H / BM, blk = i >> 3;
+  uint32_t q = (i >> 1) & 3, h = i & 1;
+  if (blk >= full && H % BM <= 64) { q = i - 8 * full; h = 0; }
+  const uint32_t u = BM * min(blk, full) + 64 * h;
+  return KBlock{(int)(q * H + u), (int)(q * Hp + u)};
+}
+
+constexpr int kMaxBlocks = 4;   // column blocks per CTA
+
+struct CellIn { float4 gi, gf, go, gg, c, cp, dci, dcp; };
+
+// REC: the recurrence, grid = (tiles_m, column blocks, S).  Otherwise dx: grid = (clusters, 1, S), the clusters walk the tiles.
+template <int BNT, uint32_t S, bool REC>
+__global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant__ TmapPack tm, const __grid_constant__ BwdWide a) {
+  constexpr int kStages = BNT == 64 ? 4 : 3;
+  constexpr int TILE_B_BYTES = BNT * BK * 4, kStageBytes = 2 * TILE_BYTES + 2 * TILE_B_BYTES;
+  constexpr uint32_t kAccCols = 2 * BNT, kBufs = kSeqBufs * BN / kAccCols, kHalf = BNT / 2, kParkBytes = 64 * BM * 4;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages], acc_full[kBufs], acc_empty[kBufs], park_full, park_free, go[kMaxBlocks];
+  __shared__ uint32_t tmem_base_slot;
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  float* park = reinterpret_cast<float*>(ring + (size_t)kStages * kStageBytes);   // 64 columns x BM rows
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = blockIdx.z;
+  // this CTA's k-blocks: an equal share, or (dx with splits) one block of units, so that the sums are those of the unsplit form
+  const uint32_t per = REC || S == 1 ? (a.kbs + S - 1) / S : 8, k0 = min(rank * per, a.kbs), total = min(k0 + per, a.kbs) - k0;
+  const uint32_t slots = REC ? S : min(S, (a.kbs + 7) / 8);
+  const uint32_t item0 = REC ? 0 : blockIdx.x, item_step = REC ? 1 : gridDim.x;
+  const uint32_t block0 = REC ? blockIdx.y * a.ncb : 0, nblocks = REC ? min(a.ncb, a.tiles_n - block0) : 1;   // this CTA's column blocks
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (uint32_t q = 0; q < kBufs; ++q) { mbar_init(&acc_full[q], 1); mbar_init(&acc_empty[q], kEpiWarps); }
+    mbar_init(&park_full, 1); mbar_init(&park_free, S);   // the bytes of a pass, 64 columns, whoever sends them / an arrival per CTA
+    for (int q = 0; q < kMaxBlocks; ++q) mbar_init(&go[q], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (S > 1) mbar_expect_tx(&park_full, kParkBytes);
+  }
+  if (threadIdx.x == 32 * 2) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm.t[q]) : "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kSeqBufs * BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = tmem_base_slot;
+  if (S > 1) cluster_sync_all();   // every CTA's barriers exist before anyone arrives on them remotely
+  dyb_grid_dep_wait();
+
+  if (warp == 0) {
+    if (elect_one()) {
+      // TMA producer: rows [m0, + 128) of the weights, rows [col0, + BNT) of the pairs of dgates
+      uint32_t s = 0, ph = 0;
+      bool fail = false;
+      const uint32_t per_step = gridDim.x * S;   // REC: arrivals per column block and step
+      for (uint32_t it = item0; it < a.P && !fail; it += item_step)
+      for (uint32_t cb = 0; cb < nblocks && !fail; ++cb) {
+        const int m0 = (int)(REC ? blockIdx.x * BM : it % a.tiles_m * BM);
+        const int col0 = (int)(REC ? (a.T - 1 - it) * a.B + (block0 + cb) * BNT : it / a.tiles_m * BNT);
+        uint32_t i = 0;
+        if (REC) {
+          // The weights of the first k-blocks do not depend on the cell pass and are requested as their stages become free; the pairs of dgates follow
+          // as soon as the counter says so, with more column blocks than one before all of those stages are free.
+          const uint32_t pre = min((uint32_t)kStages, total), want = (it + 1) * per_step;
+          uint32_t sa = s, pa = ph, na = 0;   // next stage for weights, its phase, weights requested so far
+          bool ready = false;
+          for (uint32_t poll = 0; !fail && (!ready || i < pre); ++poll) {
+            if (poll == kPollLimit) fail = true;
+            if (!ready && peek_counter(a.done + block0 + cb) >= want) {
+              ready = true;
+              mbar_arrive(&go[cb]);                                       // (the scale words may be read)
+              asm volatile("fence.proxy.async.global;" ::: "memory");     // generic-proxy stores of other CTAs -> this CTA's TMA reads
+            }
+            if (na < pre && mbar_test(&empty_bar[sa], pa ^ 1)) {
+              unsigned char* st = ring + (size_t)sa * kStageBytes;
+              const KBlock kb = k_block(k0 + na, a.H, a.Hp);
+              mbar_expect_tx(&full_bar[sa], kStageBytes);
+              tma_load_2d(st, &tm.t[0], &full_bar[sa], kb.xa, m0);
+              tma_load_2d(st + TILE_BYTES, &tm.t[1], &full_bar[sa], kb.xa, m0);
+              if (++sa == kStages) { sa = 0; pa ^= 1; }
+              ++na;
+            }
+            if (ready && i < na) {
+              unsigned char* st = ring + (size_t)s * kStageBytes;
+              const KBlock kb = k_block(k0 + i, a.H, a.Hp);
+              tma_load_2d(st + 2 * TILE_BYTES, &tm.t[2], &full_bar[s], kb.xb, col0);
+              tma_load_2d(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[3], &full_bar[s], kb.xb, col0);
+              if (++s == kStages) { s = 0; ph ^= 1; }
+              ++i;
+            }
+          }
+          if (fail) break;
+        }
+        for (; i < total; ++i) {
+          if (!mbar_wait(&empty_bar[s], ph ^ 1)) { fail = true; break; }
+          unsigned char* st = ring + (size_t)s * kStageBytes;
+          const KBlock kb = k_block(k0 + i, a.H, a.Hp);
+          mbar_expect_tx(&full_bar[s], kStageBytes);
+          tma_load_2d(st, &tm.t[0], &full_bar[s], kb.xa, m0);
+          tma_load_2d(st + TILE_BYTES, &tm.t[1], &full_bar[s], kb.xa, m0);
+          tma_load_2d(st + 2 * TILE_BYTES, &tm.t[2], &full_bar[s], kb.xb, col0);
+          tma_load_2d(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[3], &full_bar[s], kb.xb, col0);
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+      }
+      if (fail) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(BNT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint32_t idesc_wide = idesc + ((uint32_t)(BNT >> 3) << 17);
+      uint64_t d_a_hi[kStages], d_a_lo[kStages], d_b[kStages];
+#pragma unroll
+      for (int q = 0; q < kStages; ++q) {
+        const uint32_t base = smem_u32(ring + (size_t)q * kStageBytes);
+        d_a_hi[q] = umma_desc(base); d_a_lo[q] = umma_desc(base + TILE_BYTES); d_b[q] = umma_desc(base + 2 * TILE_BYTES);
+      }
+      // stage, phase and chain counters run on across products; a chain ends with its block of units, or with this CTA's share
+      uint32_t s = 0, ph = 0, chain = 0, buf = 0;
+      bool fail = false;
+      for (uint32_t it = item0; it < a.P && !fail; it += item_step)
+      for (uint32_t cb = 0; cb < nblocks && !fail; ++cb) {
+        uint32_t in_chain = 0;
+        for (uint32_t i = 0; i < total; ++i) {
+          if (in_chain == 0 && chain >= kBufs) {
+            if (!mbar_wait(&acc_empty[buf], ((chain / kBufs) - 1) & 1)) { fail = true; break; }
+          }
+          if (!mbar_wait(&full_bar[s], ph)) { fail = true; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          uint64_t a_hi, a_lo, b;   // select without dynamic register indexing
+          if (s == 0) { a_hi = d_a_hi[0]; a_lo = d_a_lo[0]; b = d_b[0]; }
+          else if (s == 1) { a_hi = d_a_hi[1]; a_lo = d_a_lo[1]; b = d_b[1]; }
+          else if (s == 2 || kStages == 3) { a_hi = d_a_hi[2]; a_lo = d_a_lo[2]; b = d_b[2]; }
+          else { a_hi = d_a_hi[kStages - 1]; a_lo = d_a_lo[kStages - 1]; b = d_b[kStages - 1]; }
+          issue_kblock_f16(tmem_base + buf * kAccCols, tmem_base + buf * kAccCols + BNT, a_hi, a_lo, b, idesc_wide, idesc, in_chain, 2, 2);
+          umma_commit(&empty_bar[s]);
+          if (((k0 + i) & 7) == 7 || i == total - 1) { umma_commit(&acc_full[buf]); in_chain = 0; ++chain; buf = chain % kBufs; }
+          else ++in_chain;
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+      }
+      if (fail) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
+    }
+  } else {
+    // epilogue warps 2..9: TMEM lanes 32 (warp % 4) .. + 31; warps 2 - 5 drain the tile's first BNT / 2 columns, warps 6 - 9 the others
+    const uint32_t quarter = warp & 3, half = (warp - 2) >> 2, row = quarter * 32 + lane;
+    const uint32_t te = threadIdx.x - 64, ew = te >> 5;
+    const uint32_t nchains = total ? ((k0 + total - 1) >> 3) - (k0 >> 3) + 1 : 0;
+    // The exchange goes in passes of 64 columns: pass hh takes columns [32 hh, + 32) of either half, position p of a pass being column p % 32 of the
+    // half p / 32.  Rank r finishes the positions [r w, + w); sender s's partial sums of them lie in slot s of r's buffer.
+    constexpr uint32_t w = 64 / S, KC = w / 8, GB = KC < 2 ? KC : 2;   // a warp holds one column: 8 columns of a slice at a time, GB of them in flight
+    const uint32_t uq = 4 * (te & 31);                                  // this thread's four rows of the tile
+    uint32_t cg = 0, pf_phase = 0, pr_phase = 0;
+    bool ok = true;   // the same for all 256 threads after every bar_and below
+    const size_t HB = (size_t)a.H * a.B;
+    const uint32_t u = blockIdx.x * BM + uq;                            // REC: units [u, u + 4)
+    const bool own_u = u < a.H;
+    float4 rs[4];   // REC: row sums of dgates over this thread's columns of a step
+
+    auto column = [&](int hh, uint32_t k) { const uint32_t p = rank * w + ew + 8 * k; return (p >> 5) * kHalf + 32 * hh + (p & 31); };
+    auto cell_load = [&](CellIn& in, uint32_t t, uint32_t n) {
+      const size_t e = (size_t)n * a.H + u;
+      const float* g = a.gates + (size_t)t * 4 * HB + (size_t)n * 4 * a.H + u;
+      in.gi = ld4(g); in.gf = ld4(g + a.H); in.go = ld4(g + 2 * a.H); in.gg = ld4(g + 3 * a.H);
+      in.c = ld4(a.cs + (size_t)t * HB + e);
+      in.cp = ld4((t ? a.cs + (size_t)(t - 1) * HB : a.c0) + e);
+      const float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
+      in.dci = a.dc ? __ldcg(reinterpret_cast<const float4*>(a.dc + (size_t)t * HB + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      in.dcp = dcp ? __ldcg(reinterpret_cast<const float4*>(dcp + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    // The cell pass of units [u, + 4), column n of step t from dE/dh: dE/dc of the step before, and dgates as fp16 pairs with the word of the warp's
+    // (column, block).  The four gates' gradients come back in p.  (All lanes of a warp take part; those past the last unit with zeros.)
+    auto cell = [&](CellIn& in, float4 dh, uint32_t t, uint32_t n, float4 (&p)[4]) {
+      uint32_t m = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) p[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (own_u) {
+        const float* f[8] = {&in.gi.x, &in.gf.x, &in.go.x, &in.gg.x, &in.c.x, &in.cp.x, &dh.x, &in.dci.x};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          lstm_cell_grad(f[0][q], f[1][q], f[2][q], f[3][q], f[4][q], f[5][q], f[6][q], f[7][q], a.dc != nullptr, (&in.dcp.x)[q], (&p[0].x)[q], (&p[1].x)[q],
+                         (&p[2].x)[q], (&p[3].x)[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          m = max(m, max(max(finite_mag(p[q].x), finite_mag(p[q].y)), max(finite_mag(p[q].z), finite_mag(p[q].w))));
+          rs[q].x += p[q].x; rs[q].y += p[q].y; rs[q].z += p[q].z; rs[q].w += p[q].w;
+        }
+      }
+      m = __reduce_max_sync(0xffffffffu, m);
+      const size_t r = (size_t)t * a.B + n;
+      if (lane == 0) a.dsc[(size_t)blockIdx.x * a.dsc_ld + r] = m;
+      const float s = scale_of(m);
+      if (u < a.Hp) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          __half hi[4], lo[4];
+          split_f16(p[q].x * s, hi[0], lo[0]); split_f16(p[q].y * s, hi[1], lo[1]); split_f16(p[q].z * s, hi[2], lo[2]); split_f16(p[q].w * s, hi[3], lo[3]);
+          const size_t o = (r * 4 + q) * a.Hp + u;
+          *reinterpret_cast<uint2*>(a.d16_hi + o) = *reinterpret_cast<const uint2*>(hi);
+          *reinterpret_cast<uint2*>(a.d16_lo + o) = *reinterpret_cast<const uint2*>(lo);
+        }
+      }
+    };
+    auto cell_rest = [&](const CellIn& in, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dE/dc of the step before, dgates for the weight gradients
+      if (!own_u) return;
+      float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
+      if (dcp) st4(dcp + (size_t)n * a.H + u, in.dcp);
+      const size_t o = ((size_t)t * a.B + n) * a.dn_pitch + u;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float4 hi, lo;
+        split_tf32(p[q].x, hi.x, lo.x); split_tf32(p[q].y, hi.y, lo.y); split_tf32(p[q].z, hi.z, lo.z); split_tf32(p[q].w, hi.w, lo.w);
+        st4(a.dn_hi + o + (size_t)q * a.H, hi); st4(a.dn_lo + o + (size_t)q * a.H, lo);
+      }
+    };
+    auto publish = [&](uint32_t cb) {   // (behind a barrier: one thread's release orders all the stores it has observed, for both proxies)
+      if (te == 0) {
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        signal_counter(a.done + block0 + cb);
+      }
+    };
+    // The row sums of this CTA's columns in step `step` of the sweep, through the exchange buffer: the eight warps' columns in order.
+    auto row_sums = [&](uint32_t step, uint32_t cb) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) st4(park + (ew * 4 + q) * BM + uq, rs[q]);
+      bar_sync(1, 256);
+      float* part = a.part + (((size_t)step * a.tiles_n + block0 + cb) * S + rank) * 4 * a.H;
+#pragma unroll
+      for (uint32_t k = 0; k < 2; ++k) {
+        const uint32_t r = te + 256 * k, q = r / BM, j = r % BM;
+        float v[8];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) v[x] = park[(x * 4 + q) * BM + j];
+#pragma unroll
+        for (int x = 1; x < 8; ++x) v[0] += v[x];
+        if (ok && blockIdx.x * BM + j < a.H) part[(size_t)q * a.H + blockIdx.x * BM + j] = v[0];
+      }
+      bar_sync(1, 256);
+    };
+    auto clear_sums = [&]() {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) rs[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+
+    for (uint32_t cb = 0; REC && cb < nblocks; ++cb) {   // the cell pass of the last step
+      const uint32_t t = a.T - 1, n0 = (block0 + cb) * BNT;
+      clear_sums();
+#pragma unroll 1
+      for (int hh = 0; hh < BNT / 64; ++hh)
+#pragma unroll 1
+        for (uint32_t k = 0; k < KC; ++k) {
+          const uint32_t n = n0 + column(hh, k);
+          if (n >= a.B) continue;
+          CellIn in = {};
+          float4 dh = make_float4(0.f, 0.f, 0.f, 0.f), p[4];
+          if (own_u) { cell_load(in, t, n); dh = ld4(a.dh + (size_t)t * HB + (size_t)n * a.H + u); }
+          cell(in, dh, t, n, p);
+          cell_rest(in, p, t, n);
+        }
+      row_sums(0, cb);
+    }
+    if (REC)   // (all blocks at the end: the exchange buffer belongs to the others from the first one on)
+      for (uint32_t cb = 0; cb < nblocks; ++cb) publish(cb);
+
+    float row_f = REC ? inv_scale_of(blockIdx.x * BM + row < a.M ? __ldg(a.wscale + blockIdx.x * BM + row) : 0x3f800000u) : 1.f;
+#pragma unroll 1
+    for (uint32_t it = item0; it < a.P; it += item_step)
+#pragma unroll 1
+    for (uint32_t cb = 0; cb < nblocks; ++cb) {
+      const uint32_t n0 = REC ? (block0 + cb) * BNT : 0;
+      const uint32_t m0 = REC ? blockIdx.x * BM : it % a.tiles_m * BM;
+      const uint32_t t = REC ? a.T - 1 - it : 0;                           // REC: dgates of step t -> dE/dh of step t - 1
+      const uint32_t col0 = REC ? n0 : it / a.tiles_m * BNT, cols = REC ? a.B : a.columns;   // first column of the tile and their end
+      const uint32_t seq0 = REC ? t * a.B : 0;                             // ... as columns of the sequence
+      float* const dst = REC ? (t ? a.dh + (size_t)(t - 1) * HB : a.dh_prev) : a.dx;
+      const uint32_t m = m0 + uq;
+      const bool own = m < a.M, vec = REC || ((a.M & 3) == 0 && aligned16(a.dx) && aligned16(a.mask));
+      if (!REC) row_f = inv_scale_of(m0 + row < a.M ? __ldg(a.wscale + m0 + row) : 0x3f800000u);
+      if (REC && t) {   // what the cell pass will read from HBM is asked for now (a request per 128-byte line)
+        if (own_u && (te & 7) == 0) {
+#pragma unroll
+          for (int hh = 0; hh < BNT / 64; ++hh)
+#pragma unroll
+            for (uint32_t k = 0; k < KC; ++k) {
+              const uint32_t n = n0 + column(hh, k);
+              if (n >= a.B) continue;
+              const size_t e = (size_t)n * a.H + u;
+              const float* g = a.gates + (size_t)(t - 1) * 4 * HB + (size_t)n * 4 * a.H + u;
+              const float* ps[7] = {g, g + a.H, g + 2 * a.H, g + 3 * a.H, (t > 1 ? a.cs + (size_t)(t - 2) * HB : a.c0) + e, dst + e, t > 1 ? a.dc + (size_t)(t - 2) * HB + e : dst + e};
+#pragma unroll
+              for (int q = 0; q < 7; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(ps[q]));
+            }
+        }
+      }
+      // ---- drain the chains of this product ----
+      float sum[kHalf];
+#pragma unroll
+      for (uint32_t q = 0; q < kHalf; ++q) sum[q] = 0.f;
+      if (REC && nchains && ok && !mbar_wait(&go[cb], it & 1)) ok = false;
+#pragma unroll 1
+      for (uint32_t c = 0; c < nchains; ++c, ++cg) {
+        const uint32_t buf = cg % kBufs;
+        if (!ok) continue;
+        float f[BNT / 64];   // 2^-s of the columns lane (and lane + 32) of this warp's half, and of its row
+#pragma unroll
+        for (int k = 0; k < BNT / 64; ++k) {
+          const uint32_t n = col0 + half * kHalf + 32 * k + lane;
+          f[k] = inv_scale_of(n < cols ? __ldcg(a.dsc + (size_t)((k0 >> 3) + c) * a.dsc_ld + seq0 + n) : 0x3f800000u);
+        }
+        if (!mbar_wait(&acc_full[buf], (cg / kBufs) & 1)) { ok = false; continue; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + half * kHalf;
+#pragma unroll
+        for (uint32_t p = 0; p < kHalf / 16; ++p) {   // (16 columns of both accumulators at a time)
+          float v1[16], v2[16];
+          tmem_ld16x2(taddr + 16 * p, taddr + BNT + 16 * p, v1, v2);
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            // (both factors at once: the sum times one of them may leave fp32's range where the product does not; rounded before it is added, as where
+            // another CTA adds it)
+            sum[16 * p + q] = __fadd_rn(sum[16 * p + q], __fmul_rn(__fmaf_rn(v2[q], kLoScale, v1[q]), row_f * __shfl_sync(0xffffffffu, f[p / 2], 16 * (p % 2) + q)));
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      }
+      if (REC) clear_sums();
+#pragma unroll
+      for (int hh = 0; hh < BNT / 64; ++hh) {
+        // ---- partial sums to the ranks that finish them ----
+        if (S > 1 && ok && !mbar_wait_cluster(&park_free, pr_phase ^ 1)) ok = false;
+        if (S > 1) {
+#pragma unroll
+          for (uint32_t rr = 0; rr < S / 2; ++rr) {
+            const uint32_t to = mapa_u32(smem_u32(park), half * (S / 2) + rr) + 4u * (rank * w * BM), bar = mapa_u32(smem_u32(&park_full), half * (S / 2) + rr);
+#pragma unroll
+            for (uint32_t q = 0; q < w; q += 4)   // column q + lane % 4, rows of the lane's quad
+              send4(to + 4u * park_at(q + (lane & 3), row >> 2), transpose4(sum + (32 * hh + rr * w + q) % kHalf, lane), bar);
+          }
+        } else {
+#pragma unroll
+          for (uint32_t q = 0; q < 32; ++q) park[park_at(32 * half + q, row >> 2) + (row & 3)] = sum[32 * hh + q];
+        }
+        const bool last_pass = hh == BNT / 64 - 1;
+#pragma unroll 1
+        for (uint32_t kb = 0; kb < KC; kb += GB) {
+          CellIn in[GB];
+          float4 old[GB], mk[GB], p[GB][4];
+          uint32_t n[GB];
+#pragma unroll
+          for (uint32_t g = 0; g < GB; ++g) {   // everything that comes from memory, before the wait
+            n[g] = col0 + column(hh, kb + g);
+            in[g] = CellIn{};
+            mk[g] = make_float4(1.f, 1.f, 1.f, 1.f);
+            old[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!own || n[g] >= cols || !vec) continue;
+            old[g] = __ldcg(reinterpret_cast<const float4*>(dst + (size_t)n[g] * a.M + m));
+            if (a.mask) mk[g] = ld4(a.mask + m + (a.mask_full ? (size_t)(REC ? n[g] : n[g] % a.B) * a.M : 0));
+            if (REC && t) cell_load(in[g], t - 1, n[g]);
+          }
+          if (kb == 0) {
+            const bool got = S > 1 ? mbar_wait_cluster(&park_full, pf_phase) : true;
+            ok = bar_and(1, 256, ok && got) != 0;
+            pf_phase ^= 1; pr_phase ^= 1;
+            if (S > 1 && te == 0) mbar_expect_tx(&park_full, kParkBytes);   // (the next pass; it begins when this CTA has arrived on the others' park_free)
+          }
+#pragma unroll
+          for (uint32_t g = 0; g < GB; ++g) {
+            if (n[g] >= cols) continue;   // (the same for a whole warp)
+            const float* col = park + park_at(ew + 8 * (kb + g), te & 31);
+            float4 v = ld4(col);
+#pragma unroll
+            for (uint32_t r = 1; r < S; ++r)
+              if (REC || r < slots) { const float4 x = ld4(col + (size_t)r * w * BM); v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w; }
+            if (vec) {
+              if (a.mask) v = make_float4(__fmaf_rn(v.x, mk[g].x, old[g].x), __fmaf_rn(v.y, mk[g].y, old[g].y), __fmaf_rn(v.z, mk[g].z, old[g].z), __fmaf_rn(v.w, mk[g].w, old[g].w));
+              else v = make_float4(v.x + old[g].x, v.y + old[g].y, v.z + old[g].z, v.w + old[g].w);
+            }
+            old[g] = v;
+            if (REC && t && ok) cell(in[g], v, t - 1, n[g], p[g]);
+            if (vec || !own || !ok) continue;
+            for (uint32_t q = 0; q < 4 && m + q < a.M; ++q) {
+              float* d = dst + (size_t)n[g] * a.M + m + q;
+              *d = __fmaf_rn((&v.x)[q], a.mask ? a.mask[m + q + (a.mask_full ? (size_t)(n[g] % a.B) * a.M : 0)] : 1.f, *d);
+            }
+          }
+          if (REC && t && last_pass && kb + GB >= KC) {
+            bar_sync(1, 256);   // all stores of the pairs and their words are issued; what nobody waits for goes out behind them
+            publish(cb);
+          }
+          if (!ok) continue;
+#pragma unroll
+          for (uint32_t g = 0; g < GB; ++g) {
+            if (n[g] >= cols) continue;
+            if (own && vec) st4(dst + (size_t)n[g] * a.M + m, old[g]);
+            if (REC && t) cell_rest(in[g], p[g], t - 1, n[g]);
+          }
+        }
+        if (REC && t && last_pass) row_sums(it + 1, cb);
+        else bar_sync(1, 256);    // every read of the exchange buffer is done
+        if (S > 1 && te < S) mbar_arrive_remote(&park_free, te);
+      }
+    }
+    if (!ok && lane == 0) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (S > 1) cluster_sync_all();   // no CTA leaves while another may still arrive on its barriers
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kSeqBufs * BN) : "memory");
+  }
+}
+
+// ---- host side ---------------------------------------------------------------------------------------------------------
+enum WideOp { WIDE_FIT, WIDE_LAUNCH };
+
+template <int BNT, uint32_t S, bool REC>
+int wide_do(WideOp op, dyb200_ctx* ctx, int slot, const TmapPack* tm, const BwdWide* a, dim3 grid, double flops) {
+  const auto kernel = k_bwd_wide<BNT, S, REC>;
+  int16_t& fit = ctx->bwd_wide_fit[slot];
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = op == WIDE_FIT ? dim3(1, 1, S) : grid; cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_SEQ_BYTES; cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (S > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 1; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = S;
+    ++na;
+  }
+  cfg.attrs = attr; cfg.numAttrs = na;
+  if (op == WIDE_FIT) {   // clusters (S = 1: CTAs) that fit on the GPU at once; the kernel's shared-memory limit is raised with the first question
+    if (fit == 0) {
+      int n = ctx->sm_count;   // (225 KB of shared memory: one CTA per SM)
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SEQ_BYTES) != cudaSuccess ||
+          (S > 1 && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess)) { (void)cudaGetLastError(); n = -1; }
+      fit = (int16_t)(n > 0 ? n : -1);
+    }
+    return fit;
+  }
+  GemmProfScope scope(ctx, flops, 2, a->M, REC ? a->B * a->T : a->columns, 4 * a->H, EPI_ACCUM_MASK);
+  if (REC && ctx->seq_coop >= 0) {
+    // all CTAs wait on one another: as many as fit at once (the plan), scheduled as one gang where the driver takes the attribute
+    attr[na].id = cudaLaunchAttributeCooperative;
+    attr[na].val.cooperative = 1;
+    cfg.numAttrs = na + 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, *tm, *a);
+    if (e == cudaSuccess) { ctx->seq_coop = 1; ctx->launches++; return DYB200_OK; }
+    (void)cudaGetLastError();
+    if (ctx->seq_coop == 1) return dyb200_fail(ctx, DYB200_ECUDA, "backward recurrence: launch failed: %s", cudaGetErrorString(e));
+    ctx->seq_coop = -1;
+    cfg.numAttrs = na;
+  }
+  cudaLaunchKernelEx(&cfg, kernel, *tm, *a);
+  DYB_LAUNCHED(ctx);
+  return DYB200_OK;
+}
+constexpr uint32_t kRecCols = 64;
+int wide_rec(WideOp op, uint32_t S, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const BwdWide* a = nullptr, dim3 grid = dim3(), double flops = 0) {
+  if (S == 8) return wide_do<kRecCols, 8, true>(op, ctx, 0, tm, a, grid, flops);
+  if (S == 4) return wide_do<kRecCols, 4, true>(op, ctx, 1, tm, a, grid, flops);
+  if (S == 2) return wide_do<kRecCols, 2, true>(op, ctx, 2, tm, a, grid, flops);
+  return wide_do<kRecCols, 1, true>(op, ctx, 3, tm, a, grid, flops);
+}
+enum DxForm { DX_128, DX_64, DX_SPLIT };   // tiles of 128 or 64 columns, a CTA each; tiles of 64 columns, a CTA of eight for each block of 128 units
+int wide_dx(WideOp op, DxForm f, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const BwdWide* a = nullptr, dim3 grid = dim3(), double flops = 0) {
+  if (f == DX_128) return wide_do<128, 1, false>(op, ctx, 4, tm, a, grid, flops);
+  if (f == DX_64) return wide_do<64, 1, false>(op, ctx, 5, tm, a, grid, flops);
+  return wide_do<64, 8, false>(op, ctx, 6, tm, a, grid, flops);
+}
+uint32_t k_blocks(uint32_t H) { return 8 * (H / BM) + (H % BM == 0 ? 0 : H % BM <= 64 ? 4 : 8); }
+
+}  // namespace
+
+// Column blocks per CTA and K splits: the fastest by what a product was measured to take - 0.36 us per k-block on the tensor pipe and 6 us from its last
+// MMA to the next step's first, which another block's MMAs overlap.
+bool dyb200_bwd_wide_plan(dyb200_ctx* ctx, uint32_t H, uint32_t B, uint32_t* ncb, uint32_t* S) {
+  if (H <= 384 || H % 8 != 0 || B <= 8) return false;
+  const uint32_t tiles_m = (H + BM - 1) / BM, tiles_n = (B + kRecCols - 1) / kRecCols, kbs = k_blocks(H);
+  if (tiles_n > DYB200_DEV_BWD_WORDS) return false;   // (a hand-over counter per column block)
+  struct { double t; uint32_t n, s; } c[12];
+  int nc = 0;
+  for (uint32_t n = 1; n <= kMaxBlocks && n <= tiles_n; n *= 2)
+    for (uint32_t s = 8; s >= 1; s /= 2) {
+      if (tiles_m * ((tiles_n + n - 1) / n) * s > (uint32_t)ctx->sm_count) continue;
+      const double mma = (kbs + s - 1) / s * 0.36;
+      c[nc].t = n == 1 ? mma + 6.0 : n * (mma > 6.0 ? mma : 6.0) + 1.5; c[nc].n = n; c[nc].s = s;
+      ++nc;
+    }
+  while (nc > 0) {   // (the best one first: asking how many clusters fit loads the kernel, a few ms each)
+    int k = 0;
+    for (int q = 1; q < nc; ++q) if (c[q].t < c[k].t) k = q;
+    const int fit = wide_rec(WIDE_FIT, c[k].s, ctx);
+    if (fit > 0 && tiles_m * ((tiles_n + c[k].n - 1) / c[k].n) <= (uint32_t)fit) { *ncb = c[k].n; *S = c[k].s; return true; }
+    c[k] = c[--nc];
+  }
+  return false;
+}
+
+int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
+  const uint32_t H = q.H, I = q.I, B = q.B, T = q.T, G = 4 * H, Hp = (H + 63) / 64 * 64, tiles_m = (H + BM - 1) / BM, columns = T * B;
+  uint32_t ncb, S;
+  DYB_CHECK_ARG(ctx, dyb200_bwd_wide_plan(ctx, H, B, &ncb, &S), "lstm_seq_bwd: shape %u, %u x %u", I, H, B);
+  const uint32_t tiles_n = (B + kRecCols - 1) / kRecCols;
+  F16Job wh, wx;
+  int rc;
+  void *p16, *words, *part;
+  const size_t plane = (size_t)columns * 4 * Hp;
+  if ((rc = dyb200_scratch(ctx, 2 * plane * sizeof(__half), &p16)) || (rc = dyb200_scratch(ctx, (size_t)tiles_m * columns * sizeof(uint32_t), &words)) ||
+      (rc = dyb200_scratch(ctx, (size_t)T * tiles_n * S * G * sizeof(float), &part))) return rc;
+  if ((rc = dyb200_f16_param(ctx, q.Wh, G, H, G, F16_LINE, &wh))) return rc;
+  if (q.dx && (rc = dyb200_f16_param(ctx, q.Wx, G, I, G, F16_LINE, &wx))) return rc;
+  BwdWide a;
+  memset(&a, 0, sizeof(a));
+  a.T = T; a.B = B; a.H = H; a.Hp = Hp; a.kbs = k_blocks(H); a.P = T - 1 + (q.dh_prev ? 1 : 0); a.M = H; a.tiles_m = tiles_m;
+  a.ncb = ncb; a.tiles_n = tiles_n;
+  a.gates = q.gates; a.cs = q.c; a.c0 = q.c0; a.dh = q.dh; a.dc = q.dc; a.dh_prev = q.dh_prev; a.dc_prev = q.dc_prev;
+  a.dn_hi = q.dn_hi; a.dn_lo = q.dn_lo; a.dn_pitch = q.dn_pitch;
+  a.d16_hi = (__half*)p16; a.d16_lo = a.d16_hi + plane;
+  a.dsc = (uint32_t*)words; a.dsc_ld = columns; a.wscale = wh.scale; a.part = (float*)part;
+  a.mask = q.mh; a.mask_full = q.mh_full;
+  a.done = ctx->dev_flags + DYB200_DEV_BWD0; a.flags = ctx->dev_flags;
+  TmapPack tm;
+  memset(&tm, 0, sizeof(tm));
+  if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[0], wh.hi, H, G, wh.pitch, BM, false)) || (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[1], wh.lo, H, G, wh.pitch, BM, false)) ||
+      (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[2], a.d16_hi, columns, 4 * Hp, 4 * Hp, kRecCols, false)) ||
+      (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[3], a.d16_lo, columns, 4 * Hp, 4 * Hp, kRecCols, false))) return rc;
+  if ((rc = wide_rec(WIDE_LAUNCH, S, ctx, &tm, &a, dim3(tiles_m, (tiles_n + ncb - 1) / ncb, S), 2.0 * G * (double)H * B * a.P))) return rc;
+  if ((rc = dyb200_seq_db(ctx, a.part, T, tiles_n * S, G, q.db, a.done)) || !q.dx) return rc;
+  // dx of all columns
+  a.M = I; a.tiles_m = (I + BM - 1) / BM; a.columns = columns; a.dx = q.dx; a.mask = q.mx; a.mask_full = q.mx_full; a.wscale = wx.scale;
+  // The form by what a round of tiles was measured to take.  All give the same bits, whatever the number of columns: chains are added in the order of
+  // the blocks of units.  (1024 x 64 of a single step: 17 us with two CTAs per tile, 9 with
+  // eight; 1024 x 17 920: 350 on 128-column tiles.)
+  DxForm form = DX_128;
+  double best = 0;
+  for (const DxForm f : {DX_128, DX_64, DX_SPLIT}) {
+    if (f == DX_SPLIT && a.kbs > 64) continue;
+    const uint32_t n = f == DX_128 ? 128 : 64, tiles = a.tiles_m * ((columns + n - 1) / n), room = f == DX_SPLIT ? (uint32_t)ctx->sm_count / 10 + 1 : (uint32_t)ctx->sm_count;
+    const double t = (tiles + room - 1) / room * (f == DX_128 ? a.kbs * 0.55 + 6.0 : f == DX_64 ? a.kbs * 0.36 + 4.0 : 8 * 0.36 + 4.5);
+    if (best == 0 || t < best) { best = t; form = f; }
+  }
+  int fit = wide_dx(WIDE_FIT, form, ctx);
+  if (fit <= 0 && form == DX_SPLIT) fit = wide_dx(WIDE_FIT, form = DX_64, ctx);
+  if (fit <= 0) return dyb200_fail(ctx, DYB200_ECUDA, "lstm_seq_bwd: no launch of the dx product fits");
+  const uint32_t dn = form == DX_128 ? 128 : 64;
+  a.P = a.tiles_m * ((columns + dn - 1) / dn);
+  if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[0], wx.hi, I, G, wx.pitch, BM, false)) || (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[1], wx.lo, I, G, wx.pitch, BM, false)) ||
+      (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[2], a.d16_hi, columns, 4 * Hp, 4 * Hp, dn, false)) ||
+      (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[3], a.d16_lo, columns, 4 * Hp, 4 * Hp, dn, false))) return rc;
+  return wide_dx(WIDE_LAUNCH, form, ctx, &tm, &a, dim3(a.P < (uint32_t)fit ? a.P : (uint32_t)fit, 1, form == DX_SPLIT ? 8 : 1), 2.0 * G * (double)I * columns);
+}
+
+// Whether the backward pass of such a layer takes this form (1 or 0), and its column blocks per CTA and K splits.
+extern "C" int dyb200i_bwd_wide_tiling(dyb200_ctx* ctx, uint32_t H, uint32_t B, uint32_t* blocks, uint32_t* splits) {
+  return dyb200_bwd_wide_plan(ctx, H, B, blocks, splits) ? 1 : 0;
+}

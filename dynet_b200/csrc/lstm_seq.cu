@@ -44,17 +44,6 @@ struct SeqFwd {
 };
 
 __device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return a.h_scale ? __ldg(a.h_scale + (a.h_scale_full ? n : 0)) : 0x3f800000u; }
-__device__ __forceinline__ void tmem_ld16x2(uint32_t t1, uint32_t t2, float* v1, float* v2) {
-  uint32_t *r = reinterpret_cast<uint32_t*>(v1), *x = reinterpret_cast<uint32_t*>(v2);
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
-               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
-               "tcgen05.wait::ld.sync.aligned;"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
-                 "=r"(x[7]), "=r"(x[8]), "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
-               : "r"(t1), "r"(t2)
-               : "memory");
-}
 
 // F16: the products of wide layers on scaled fp16 pairs (gemm.cuh) in k-blocks of 64 - half the weight bytes from L2 per step and 0.61 us per 64 k
 // instead of 2 x 0.66.  The weights' planes are MN-major as they lie, their rows interleaved like the TF32 ones; a scale per gate row of Wx and of Wh.

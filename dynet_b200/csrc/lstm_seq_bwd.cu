@@ -515,10 +515,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_bwd(const __grid_const
 // db += the row sums of dgates of all steps: per step the batch tiles in ascending order, then the steps in sweep order (a
 // fixed order, so the result is the same from run to run).  A CTA owns 32 gate rows; its 8 warps take the steps s, s + 8, ...
 // in parallel (lane = row, all tiles of a step in flight), leave the per-step sums in shared memory, and warp 0 adds them up.
-constexpr uint32_t kDbMaxSteps = 256;
 __global__ void __launch_bounds__(256) k_seq_db_reduce(const float* __restrict__ part, uint32_t steps, uint32_t tiles, uint32_t G,
-                                                       float* __restrict__ db) {
+                                                       float* __restrict__ db, uint32_t* __restrict__ done) {
   dyb_grid_dep_sync();
+  if (done && blockIdx.x == 0 && threadIdx.x < DYB200_DEV_BWD_WORDS) done[threadIdx.x] = 0;
   __shared__ float per_step[kDbMaxSteps][32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t row = blockIdx.x * 32 + lane;
@@ -585,6 +585,12 @@ int launch_seq_bwd(dyb200_ctx* ctx, const TmapPack& tm, const SeqBwd& a, dim3 gr
 
 }  // namespace
 
+int dyb200_seq_db(dyb200_ctx* ctx, const float* part, uint32_t steps, uint32_t tiles, uint32_t G, float* db, uint32_t* done) {
+  dyb_launch(k_seq_db_reduce, (G + 31) / 32, 256, 0, ctx, part, steps, tiles, G, db, done);
+  DYB_LAUNCHED(ctx);
+  return DYB200_OK;
+}
+
 extern "C" {
 
 int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0,
@@ -608,12 +614,29 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
   const float* mh = attrs->dropout ? mask_h->v : nullptr;
   const int mx_full = mx ? mask_x->bd == B : 0, mh_full = mh ? mask_h->bd == B : 0;
 
-  // ---- all steps in one kernel, when its CTAs can all be resident ----
+  // ---- wide layers: the recurrence on fp16 pairs, then dx of all steps as one product (lstm_bwd_wide.cu) ----
   uint32_t first = T;   // steps [0, first) run as per-step calls below
+  uint32_t wide_ncb, wide_S;
+  const bool weights_ok = Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 && Wh->d[0] == G && Wh->d[1] == H && t_size(db) == G;
+  const bool masks_ok = !mx || ((mask_x->bd == B || mask_x->bd == 1) && (mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_x, 0) == I && t_dim(mask_h, 0) == H);
+  bool wide_fits = true;
+  if (ctx->seq_kernels && deferred && T >= 2 && T <= kDbMaxSteps && attrs->weightnoise_std == 0.f && I > 0 && weights_ok && masks_ok && dyb200_wgrad_rows(deferred) == G &&
+      aligned16(gates_all->v) && aligned16(c_all->v) && aligned16(c0->v) && aligned16(dh_all->v) && aligned16(dc_all->v) && (!mh || aligned16(mh)) &&
+      dyb200_bwd_wide_plan(ctx, H, B, &wide_ncb, &wide_S)) {
+    { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
+    BwdWideCall q{I, H, B, T, Wx->v, Wh->v, gates_all->v, c_all->v, c0->v, dh_all->v, dc_all->v, nullptr, nullptr, dx_all ? dx_all->v : nullptr,
+                  mx, mx_full, mh, mh_full, db->v, nullptr, nullptr, 0};
+    if ((rc = dyb200_wgrad_reserve_a_at(deferred, 0, T * B, &q.dn_hi, &q.dn_lo, &q.dn_pitch, ctx))) return rc;
+    rc = dyb200_bwd_wide(ctx, q);
+    if (rc != DYB200_ENOMEM) return rc;
+    wide_fits = false;   // (no room for the pairs of all steps: the single-step calls, with those of one)
+  }
+
+  // ---- all steps in one kernel, when its CTAs can all be resident ----
   LstmBwdTiling tl{64, 1, 1};
   const uint32_t Imin = I < H ? I : H;
   const double flops_small = 2.0 * Imin * (double)B * G;
-  const bool persistent = ctx->seq_kernels && deferred && dx_all && T >= 2 && T <= kDbMaxSteps && attrs->weightnoise_std == 0.f &&
+  const bool persistent = wide_fits && ctx->seq_kernels && deferred && dx_all && T >= 2 && T <= kDbMaxSteps && attrs->weightnoise_std == 0.f &&
                           dyb200_lstm_bwd_tiling(ctx, I, H, B, &tl) && dyb200_tc_eligible(Imin, B, flops_small) &&
                           dyb200_tc_eligible(G, Imin, flops_small) && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 &&
                           Wh->d[0] == G && Wh->d[1] == H && t_size(db) == G && aligned16(gates_all->v) && aligned16(c_all->v) &&
@@ -657,8 +680,7 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
     if (S > 1) rc = bn == 64 ? launch_seq_bwd<64, true>(ctx, tm, a, grid, flops) : launch_seq_bwd<128, true>(ctx, tm, a, grid, flops);
     else rc = bn == 64 ? launch_seq_bwd<64, false>(ctx, tm, a, grid, flops) : launch_seq_bwd<128, false>(ctx, tm, a, grid, flops);
     if (rc) return rc;
-    dyb_launch(k_seq_db_reduce, (G + 31) / 32, 256, 0, ctx, (const float*)pp, T, btiles, G, db->v);
-    DYB_LAUNCHED(ctx);
+    if ((rc = dyb200_seq_db(ctx, (const float*)pp, T, btiles, G, db->v, nullptr))) return rc;
     first = 0;
   }
 

@@ -1,4 +1,4 @@
-// Device helpers of the sequence-persistent LSTM kernels (lstm_seq.cu, lstm_seq_bwd.cu): bounded polling of hand-over
+// Device helpers of the sequence-persistent LSTM kernels (lstm_seq.cu, lstm_seq_bwd.cu, lstm_bwd_wide.cu): bounded polling of hand-over
 // counters in global memory, cluster-scope mbarrier operations, named-barrier reductions.
 #pragma once
 #include "tc_dev.cuh"
@@ -53,8 +53,43 @@ __device__ __forceinline__ uint32_t bar_and(uint32_t id, uint32_t count, bool pr
                : "=r"(r) : "r"((uint32_t)pred), "r"(id), "r"(count) : "memory");
   return r;
 }
+// 16 columns of two accumulators
+__device__ __forceinline__ void tmem_ld16x2(uint32_t t1, uint32_t t2, float* v1, float* v2) {
+  uint32_t *r = reinterpret_cast<uint32_t*>(v1), *x = reinterpret_cast<uint32_t*>(v2);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
+                 "=r"(x[7]), "=r"(x[8]), "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
+               : "r"(t1), "r"(t2)
+               : "memory");
+}
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The exchange buffer: columns of BM rows, quads of rows moved about so that the 16-byte stores of four neighbouring columns meet no bank twice.
+__device__ __forceinline__ uint32_t park_at(uint32_t col, uint32_t quad) { return col * BM + 4 * (quad ^ (2 * (col & 3))); }
+// v: four columns of this lane's row -> rows 4 (lane / 4) .. + 3 of column lane % 4.  (One 16-byte message to another CTA instead of four.)
+__device__ __forceinline__ float4 transpose4(const float* v, uint32_t lane) {
+  const bool o = lane & 1, h = lane & 2;
+  float x = __shfl_xor_sync(0xffffffffu, o ? v[0] : v[1], 1), y = __shfl_xor_sync(0xffffffffu, o ? v[2] : v[3], 1);
+  const float a0 = o ? x : v[0], a1 = o ? v[1] : x, b0 = o ? y : v[2], b1 = o ? v[3] : y;   // columns lane % 2 and 2 + lane % 2, two rows each
+  x = __shfl_xor_sync(0xffffffffu, h ? a0 : b0, 2);
+  y = __shfl_xor_sync(0xffffffffu, h ? a1 : b1, 2);
+  return h ? make_float4(x, y, b0, b1) : make_float4(a0, a1, x, y);
+}
+// Messages to the shared memory of a CTA of the cluster that count towards an mbarrier beside their destination.  (Plain remote stores and an arrival
+// that releases them took a round trip: the 32 KB of partial sums of a 128 x 64 tile were with their ranks 2.0 us after the last chain, this way 1.2.)
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void send4(uint32_t to, float4 v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+               : "memory");
 }
 
 }  // namespace

@@ -1,0 +1,115 @@
+"""The backward pass of wide layers on fp16 pairs (csrc/lstm_bwd_wide.cu): units that are no multiple of a k-block or of a tile, batches that are no
+multiple of a column tile, one to four column blocks per CTA, K splits with even, short and empty last shares, an input of one row, masks per column and for
+all, columns whose gradients differ by 2^60, a column of zeros.  Step by step against float64 from the device's own dE/dh_t and dE/dc_t.  Bar of a
+product: 4.5e-7 of |row| |dgates column|, that of every product on fp16 pairs; dgates themselves are a handful of fp32 operations and a tanhf:
+1e-6 of their column, which the product passes on as that much of |row| |column|.  The single-step calls must give the same bits."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# blocks: column blocks of 64 per CTA; both of the rule on 148 SMs, where 15 clusters of eight fit, 33 of four, 74 of two
+@pytest.mark.parametrize("I,H,B,T,mask,blocks,splits", [
+    (512, 1024, 64, 4, "full", 1, 8),
+    (1024, 1024, 512, 3, "full", 2, 4),
+    (96, 1024, 128, 3, None, 1, 4),
+    (256, 1024, 256, 3, "one", 1, 4),
+    (512, 512, 64, 3, None, 1, 8),
+    (1, 392, 9, 4, "one", 1, 8),           # 28 k-blocks: the last share is empty; the last block of units has eight
+    (33, 448, 100, 3, "full", 1, 8),       # ... 64
+    (300, 744, 33, 3, "full", 1, 8),       # ... 104: its second half is partly filled
+    (130, 904, 300, 3, None, 2, 4),        # five column blocks: the last CTAs have one
+    (200, 576, 500, 2, "full", 1, 2),
+    (64, 2048, 500, 2, "one", 2, 2),
+    (40, 2048, 1000, 2, None, 2, 1),
+    (8, 3072, 1000, 2, None, 4, 1),
+])
+def test_backward_of_a_wide_layer(I, H, B, T, mask, blocks, splits):
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    ncb, S = C.c_uint32(), C.c_uint32()
+    assert ctx.L.dyb200i_bwd_wide_tiling(ctx.h, H, B, C.byref(ncb), C.byref(S)) == 1
+    assert (ncb.value, S.value) == (blocks, splits)
+    gen = torch.Generator("cuda").manual_seed(H + B)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    Wx, Wh = rnd(I, 4 * H) / H ** 0.5, rnd(H, 4 * H) / H ** 0.5
+    gates = torch.cat([torch.sigmoid(rnd(T * B, 3 * H)), torch.tanh(rnd(T * B, H))], dim=1)
+    cs, c0, x, h0 = rnd(T * B, H), rnd(B, H), rnd(T * B, I), rnd(B, H)
+    dh_in, dc_in, dx_in, db_in = rnd(T * B, H), rnd(T * B, H), rnd(T * B, I), rnd(4 * H)
+    mag = torch.exp2(torch.randint(-60, 3, (B, 1), device="cuda", generator=gen).float()).repeat(T, 1)
+    mag[5::B] = 0.0
+    dh_in, dc_in, dx_in = dh_in * mag, dc_in * mag, dx_in * mag
+    mB = B if mask == "full" else 1
+    mx, mh = [((torch.rand(mB, n, device="cuda", generator=gen) < 0.8) / 0.8).float() if mask else torch.ones(1, n, device="cuda") for n in (I, H)]
+    at, tm = capi.LstmGatesAttrs(1 if mask else 0, 0.0, 1.0), (g.T(mx), g.T(mh)) if mask else (None, None)
+    W = (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1))
+    outs = []
+    for single in (False, True):
+        w = ctx.wgrad_create(4 * H, I, H, T * B)
+        dh, dc, dx, db = dh_in.clone(), dc_in.clone(), dx_in.clone(), db_in.clone()
+        ctx.wgrad_pack_inputs(w, g.T(x, [I], T * B), tm[0], B)
+        if single:
+            for t in range(T - 1, -1, -1):
+                sl, pr = slice(t * B, (t + 1) * B), slice((t - 1) * B, t * B)
+                ctx.lstm_bwd_fused_at(g.T(x[sl]), g.T(h0), g.T(cs[pr] if t else c0), *W, *tm, g.T(gates[sl]), g.T(cs[sl]), g.T(dh[sl]), g.T(dc[sl]), g.T(dx[sl]),
+                                      g.T(dh[pr]) if t else None, g.T(dc[pr]) if t else None, None, None, g.T(db, [4 * H], 1), at, w, t * B)
+        else:
+            ctx.lstm_seq_bwd(g.T(x, [I], T * B), g.T(h0), g.T(c0), *W, *tm, at, g.T(gates, [4 * H], T * B), g.T(cs, [H], T * B), g.T(cs, [H], T * B),
+                             g.T(dh, [H], T * B), g.T(dc, [H], T * B), g.T(dx, [I], T * B), None, None, g.T(db, [4 * H], 1), w, T)
+        torch.cuda.synchronize()
+        ctx.wgrad_destroy(w)
+        outs.append((dh, dc, dx, db))
+    assert ctx.device_errors() == 0
+    for p, q in zip(*outs):
+        assert torch.equal(p, q)
+    dh, dc, dx, db = (o.double() for o in outs[0])
+    db_want, db_bar = db_in.double(), torch.zeros(4 * H, device="cuda", dtype=torch.float64)
+    for t in range(T - 1, -1, -1):
+        sl, pr = slice(t * B, (t + 1) * B), slice((t - 1) * B, t * B)
+        i, f, o, gg = gates[sl].double().split(H, dim=1)
+        c, cp = cs[sl].double(), (cs[pr] if t else c0).double()
+        tc = torch.tanh(c)
+        d = dh[sl] * o * (1 - tc * tc) + dc[sl]
+        dg = torch.cat([d * gg * i * (1 - i), d * cp * f * (1 - f), dh[sl] * tc * o * (1 - o), d * i * (1 - gg * gg)], dim=1)
+        db_want += dg.sum(dim=0)
+        db_bar += 2e-6 * dg.norm(dim=0) * B ** 0.5 + 1e-6 * db_want.abs()
+        col = dg.norm(dim=1)[:, None]
+        want = dx_in[sl].double() + mx.double() * (dg @ Wx.double().t())
+        bar = 1.45e-6 * 1.25 * col * Wx.double().norm(dim=1)[None, :] + 1.3e-7 * want.abs() + 1e-44
+        assert bool(((dx[sl] - want).abs() <= bar).all()), "dx %d: %.3g" % (t, float(((dx[sl] - want).abs() / bar).max()))
+        if t:
+            want = dh_in[pr].double() + mh.double() * (dg @ Wh.double().t())
+            bar = 1.45e-6 * 1.25 * col * Wh.double().norm(dim=1)[None, :] + 1.3e-7 * want.abs() + 1e-44
+            assert bool(((dh[pr] - want).abs() <= bar).all()), "dh %d: %.3g" % (t - 1, float(((dh[pr] - want).abs() / bar).max()))
+            want = dc_in[pr].double() + d * f
+            assert bool(((dc[pr] - want).abs() <= 1e-6 * (dc_in[pr].double().abs() + (d * f).abs() + (dh[sl] * o * f).abs()) + 1e-44).all()), "dc %d" % (t - 1)
+    assert bool(((db - db_want).abs() <= db_bar).all()), float(((db - db_want).abs() / db_bar).max())
+
+
+def test_sequence_without_room_for_its_pairs():
+    """Little device memory: the pairs of all steps (134 MB) do not fit, those of one (2 MB) do - the single-step calls run, with the same bits."""
+    import contextlib
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    from test_gpu_scratch_limits import room_for
+    I, H, B, T = 64, 512, 256, 64
+    rnd = lambda *s: torch.randn(*s, device="cuda")   # noqa: E731
+    x, c0, cs, gates = rnd(T * B, I), rnd(B, H), rnd(T * B, H), torch.sigmoid(rnd(T * B, 4 * H))
+    Wx, Wh, dh_in = rnd(I, 4 * H) / H ** 0.5, rnd(H, 4 * H) / H ** 0.5, rnd(T * B, H)
+    w = g.ctx().wgrad_create(4 * H, I, H, T * B)
+    outs = [[dh_in.clone(), torch.zeros(T * B, H, device="cuda"), torch.zeros(T * B, I, device="cuda"), torch.zeros(4 * H, device="cuda")] for _ in range(2)]
+    try:
+        for c, (dh, dc, dx, db) in zip((g.ctx(), None), outs):
+            with contextlib.nullcontext(c) if c else room_for(48) as ctx:
+                ctx.lstm_seq_bwd(g.T(x, [I], T * B), g.T(c0), g.T(c0), g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), None, None, capi.LstmGatesAttrs(0, 0.0, 1.0),
+                                 g.T(gates, [4 * H], T * B), g.T(cs, [H], T * B), g.T(cs, [H], T * B), g.T(dh, [H], T * B), g.T(dc, [H], T * B), g.T(dx, [I], T * B),
+                                 None, None, g.T(db, [4 * H], 1), w, T)
+        torch.cuda.synchronize()
+        assert all(torch.equal(p, q) for p, q in zip(*outs))
+    finally:
+        g.ctx().wgrad_destroy(w)
