@@ -163,7 +163,7 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
 // The same for a parameter, from the parameter cache when it is on.
 int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
-// The gate weights of a layer, Wx (4H x I) and Wh (4H x H), as MN-major planes with interleaved rows (lines = their columns, pitch 4H) and one
+// The gate weights of a layer, Wx (4H x I) and Wh (4H x H), as MN-major planes with interleaved rows (lines = their columns, 128 rows per 32 units) and one
 // scale word per row of Wx and one per row of Wh (4H words each, not interleaved); from the parameter cache when it is on.
 struct F16Gates { __half *x_hi, *x_lo, *h_hi, *h_lo; const uint32_t* scale; };
 int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, F16Gates* out);
@@ -265,7 +265,8 @@ struct SeqF16Call {
   uint32_t I, H, B, T;
   const float *Wx, *Wh, *b, *h0, *c0, *mh; int mh_full; float forget_bias;
   float *gates, *c, *h;
-  PackedOp X, Hs;          // TF32 planes of the columns' inputs; rows [0, B) of Hs are filled here unless h0_done, the later ones by the kernel
+  PackedOp X, Hs;          // TF32 planes of the columns' inputs (X without lo: the inputs themselves); rows [0, B) of Hs are filled here unless h0_done, the later
+                           // ones by the kernel (without hi: not wanted)
   int h0_done, emit_last;  // emit_last: rows [T B, (T + 1) B) of Hs receive the last step's h
 };
 int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q);

@@ -1045,13 +1045,14 @@ int pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int layout, uint32_t ro
 
 inline uint32_t round_up(uint32_t x, uint32_t m) { return (x + m - 1) / m * m; }
 
-// fp16 planes of the gate weights (F16Gates): I lines of Wx, then H lines of Wh, the scale words in the same order.
+// fp16 planes of the gate weights (F16Gates): I lines of Wx, then H lines of Wh, the scale words in the same order.  A line is tiles of 32 units, 128 rows.
+inline uint32_t gates_f16_pitch(uint32_t H) { return 128 * ((H + 31) / 32); }
 int gates_f16_pack(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, __half* hi, __half* lo, uint32_t* scale) {
   F16Jobs jobs;
   jobs.n = 2;
   for (int q = 0; q < 2; ++q) {
-    const size_t at = q ? (size_t)I * 4 * H : 0;
-    jobs.job[q] = F16Job{q ? Wh : Wx, 4 * H, q ? H : I, 4 * H, 4 * H, F16_ELEM, scale + q * 4 * H, hi + at, lo + at};
+    const size_t at = q ? (size_t)I * gates_f16_pitch(H) : 0;
+    jobs.job[q] = F16Job{q ? Wh : Wx, 4 * H, q ? H : I, 4 * H, gates_f16_pitch(H), F16_ELEM, scale + q * 4 * H, hi + at, lo + at};
     jobs.job[q].perm_H = H;
   }
   jobs.words = scale; jobs.n_words = 8 * (size_t)H;
@@ -1168,13 +1169,13 @@ int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t li
   return DYB200_OK;
 }
 int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I, uint32_t H, F16Gates* out) {
-  const uint32_t G = 4 * H;
-  const size_t plane = (size_t)(I + H) * G;
+  const uint32_t G = 4 * H, pitch = gates_f16_pitch(H);
+  const size_t plane = (size_t)(I + H) * pitch;
   float *hi, *lo;
   uint32_t* scale;
   int rc;
   if (ctx->param_cache_on) {
-    if ((rc = cached_param_pack(ctx, Wx, G, kLayoutGatesF16, G, I, G, &hi, &lo, Wh, H))) return rc;
+    if ((rc = cached_param_pack(ctx, Wx, G, kLayoutGatesF16, G, I, pitch, &hi, &lo, Wh, H))) return rc;
     scale = reinterpret_cast<uint32_t*>(hi + plane / 2);
   } else {
     void *h, *l, *sc;
@@ -1182,7 +1183,7 @@ int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t
     hi = (float*)h; lo = (float*)l; scale = (uint32_t*)sc;
     if ((rc = gates_f16_pack(ctx, Wx, Wh, I, H, (__half*)hi, (__half*)lo, scale))) return rc;
   }
-  const size_t at = (size_t)I * G;
+  const size_t at = (size_t)I * pitch;
   *out = F16Gates{(__half*)hi, (__half*)lo, (__half*)hi + at, (__half*)lo + at, scale};
   return DYB200_OK;
 }

@@ -571,31 +571,35 @@ int dyb200_vanilla_lstm_fwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
       }
       return dyb200_lstm_thin(ctx, H, B, 2, pairs, 0, e);
     }
+    uint32_t bn, S;
+    if (shapes_ok && deferred && attrs->weightnoise_std == 0.f && I > 0 && B > 0 && aligned16(gates->v) && aligned16(b->v) && aligned16(c_tm1->v) && aligned16(c_t->v) &&
+        aligned16(h_t->v) && (!attrs->dropout || aligned16(mask_h->v)) && dyb200_seq_f16_plan(ctx, I, H, B, &bn, &S)) {
+      { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
+      PackedOp Bp[2];
+      int rc;
+      // wide layers with an accumulator: the sequence kernel's product on fp16 pairs, for one step
+      const float* mx = attrs->dropout ? mask_x->v : nullptr;
+      const float* mh = attrs->dropout ? mask_h->v : nullptr;
+      const int mx_full = mx ? mask_x->bd == B : 0, mh_full = mh ? mask_h->bd == B : 0;
+      DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_fwd_fused: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
+      const bool x_pre = dyb200_wgrad_x_planes(deferred, deferred_col, B, &Bp[0]), h_pre = x_pre && dyb200_wgrad_h_planes(deferred, deferred_col, B, &Bp[1]);
+      if (!(x_pre && h_pre)) {
+        PackJobs batch;
+        dyb200_tc_pack_begin(&batch);
+        if ((rc = dyb200_wgrad_push_b_at(deferred, deferred_col, B, x_pre ? nullptr : x->v, I, mx, mx_full, h_tm1->v, H, mh, mh_full, ctx, &batch))) return rc;
+        if ((rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
+      }
+      GemmEpilogue next;
+      SeqF16Call q{I, H, B, 1, Wx->v, Wh->v, b->v, h_tm1->v, c_tm1->v, mh, mh_full, attrs->forget_gate_bias, gates->v, c_t->v, h_t->v, PackedOp(), PackedOp(), 1,
+                   x_pre && dyb200_wgrad_next_h(deferred, deferred_col, B, &next)};
+      DYB_CHECK_ARG(ctx, dyb200_wgrad_b_planes(deferred, deferred_col, B, &q.X, &q.Hs), "lstm_fwd_fused: columns [%u, %u) exceed the accumulator", deferred_col, deferred_col + B);
+      return dyb200_seq_f16(ctx, q);
+    }
     if (shapes_ok && attrs->weightnoise_std == 0.f && H % 32 == 0 && I > 0 && B > 0 && dyb200_tc_eligible(G, B, 2.0 * G * B * (I + H)) &&
         aligned16(gates->v) && aligned16(b->v) && aligned16(c_tm1->v) && aligned16(c_t->v) && aligned16(h_t->v)) {
       { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
       PackedOp A[2], Bp[2];
       int rc;
-      uint32_t bn, S;
-      if (deferred && (!attrs->dropout || aligned16(mask_h->v)) && dyb200_seq_f16_plan(ctx, I, H, B, &bn, &S)) {
-        // wide layers with an accumulator: the sequence kernel's product on fp16 pairs, for one step
-        const float* mx = attrs->dropout ? mask_x->v : nullptr;
-        const float* mh = attrs->dropout ? mask_h->v : nullptr;
-        const int mx_full = mx ? mask_x->bd == B : 0, mh_full = mh ? mask_h->bd == B : 0;
-        DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_fwd_fused: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
-        const bool x_pre = dyb200_wgrad_x_planes(deferred, deferred_col, B, &Bp[0]), h_pre = x_pre && dyb200_wgrad_h_planes(deferred, deferred_col, B, &Bp[1]);
-        if (!(x_pre && h_pre)) {
-          PackJobs batch;
-          dyb200_tc_pack_begin(&batch);
-          if ((rc = dyb200_wgrad_push_b_at(deferred, deferred_col, B, x_pre ? nullptr : x->v, I, mx, mx_full, h_tm1->v, H, mh, mh_full, ctx, &batch))) return rc;
-          if ((rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
-        }
-        GemmEpilogue next;
-        SeqF16Call q{I, H, B, 1, Wx->v, Wh->v, b->v, h_tm1->v, c_tm1->v, mh, mh_full, attrs->forget_gate_bias, gates->v, c_t->v, h_t->v, PackedOp(), PackedOp(), 1,
-                     x_pre && dyb200_wgrad_next_h(deferred, deferred_col, B, &next)};
-        DYB_CHECK_ARG(ctx, dyb200_wgrad_b_planes(deferred, deferred_col, B, &q.X, &q.Hs), "lstm_fwd_fused: columns [%u, %u) exceed the accumulator", deferred_col, deferred_col + B);
-        return dyb200_seq_f16(ctx, q);
-      }
       if ((rc = dyb200_tc_param_gates(ctx, Wx->v, G, G, I, &A[0]))) return rc;
       if ((rc = dyb200_tc_param_gates(ctx, Wh->v, G, G, H, &A[1]))) return rc;
       PackJobs batch;

@@ -43,7 +43,7 @@ struct SeqFwd {
   uint32_t* flags;
 };
 
-__device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return a.h_scale ? __ldg(a.h_scale + (a.h_scale_full ? n : 0)) : 0x3f800000u; }
+__device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return a.h_scale && n < a.B ? __ldg(a.h_scale + (a.h_scale_full ? n : 0)) : 0x3f800000u; }
 
 // F16: the products of wide layers on scaled fp16 pairs (gemm.cuh) in k-blocks of 64 - half the weight bytes from L2 per step and 0.61 us per 64 k
 // instead of 2 x 0.66.  The weights' planes are MN-major as they lie, their rows interleaved like the TF32 ones; a scale per gate row of Wx and of Wh.
@@ -74,13 +74,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
   const uint32_t M = 4 * a.H, N = a.B;
   constexpr uint32_t kAccCols = F16 ? 2 * BNT : BN, kBufs = F16 ? kSeqBufs * BN / kAccCols : kSeqBufs, kChunk = F16 ? kChunkF16 : kChunkKB;
   constexpr int EL = F16 ? 64 : 32;
+  constexpr uint32_t kHalf = BNT / 2, kParkBytes = 64 * BM * 4;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (uint32_t q = 0; q < kSeqBufs; ++q) { mbar_init(&acc_full[q], 1); mbar_init(&acc_empty[q], kEpiWarps); }
-    mbar_init(&park_full, 4 * S); mbar_init(&park_free, S);   // arrivals: the 4 sending warps of every CTA / one per CTA
+    mbar_init(&park_full, 1); mbar_init(&park_free, S);   // the bytes of a pass, 64 columns, whoever sends them / an arrival per CTA
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (S > 1) mbar_expect_tx(&park_full, kParkBytes);
   }
   if (threadIdx.x == 32 * 2) {
 #pragma unroll
@@ -185,43 +187,41 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
       if (fail) atomicOr(a.flags, DYB200_FLAG_WAIT_TIMEOUT);
     }
   } else {
-    // epilogue warps 2..9: TMEM lanes 32 (warp % 4) .. +31; warps 2-5 hold columns 0-63 of the tile, warps 6-9 columns 64-127
-    const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
+    // epilogue warps 2..9: TMEM lanes 32 (warp % 4) .. +31; warps 2-5 drain the tile's first BNT / 2 columns, warps 6-9 the others
+    const uint32_t quarter = warp & 3, half = (warp - 2) >> 2, row = quarter * 32 + lane;
     const uint32_t te = threadIdx.x - 64;
-    const bool has_cols = 64 * half < BNT;
     const uint32_t x_chunks = (ks.n0 + kChunk - 1) / kChunk;   // (F16: those of Wx x)
     const uint32_t nchunks = F16 ? x_chunks + (ks.n1 + kChunk - 1) / kChunk : (total + kChunk - 1) / kChunk;
-    // F16: 2^-s of this thread's gate row in Wx and in Wh; of the columns lane and lane + 32 of its half (h after the first step); and 2^s of the columns it finishes
-    float row_x = 1.f, row_h = 1.f, h_f[2] = {1.f, 1.f}, h_s[BNT / 64][2];
-    const uint32_t hn0 = n0 + 64 * half + lane;
+    // The tile is finished in passes of 64 columns: pass hh takes columns [32 hh, + 32) of either half, position p of a pass being column p % 32 of the
+    // half p / 32.  In the cooperative pass this thread owns hidden units [u, u + 4) (rows 32 q + l of the tile are gate q of unit 32 mt + l) at the
+    // positions te / 8 and te / 8 + 32.
+    const uint32_t l = 4 * (te & 7), u = blockIdx.x * 32 + l;
+    const bool own_u = u < a.H;
+    auto column = [&](int hh, uint32_t p) { return (p >> 5) * kHalf + 32 * hh + (p & 31); };
+    // F16: 2^-s of this thread's gate row in Wx and in Wh; of the columns lane (and lane + 32) of its half (h after the first step); and 2^s of the columns it finishes
+    float row_x = 1.f, row_h = 1.f, h_f[kHalf / 32], h_s[BNT / 64][2];
+    const uint32_t hn0 = n0 + half * kHalf + lane;
     if (F16) {
-      row_x = inv_scale_of(__ldg(a.gate_scale + (size_t)quarter * a.H + 32 * blockIdx.x + lane));
-      row_h = inv_scale_of(__ldg(a.gate_scale + (size_t)(4 + quarter) * a.H + 32 * blockIdx.x + lane));
-      if (has_cols) { h_f[0] = inv_scale_of(h_word(a, hn0)); h_f[1] = inv_scale_of(h_word(a, hn0 + 32)); }
+      if (32 * blockIdx.x + lane < a.H) {
+        row_x = inv_scale_of(__ldg(a.gate_scale + (size_t)quarter * a.H + 32 * blockIdx.x + lane));
+        row_h = inv_scale_of(__ldg(a.gate_scale + (size_t)(4 + quarter) * a.H + 32 * blockIdx.x + lane));
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kHalf / 32; ++k) h_f[k] = inv_scale_of(h_word(a, hn0 + 32 * k));
 #pragma unroll
       for (int hh = 0; hh < BNT / 64; ++hh)
 #pragma unroll
-        for (int k = 0; k < 2; ++k) h_s[hh][k] = scale_of(h_word(a, n0 + 64 * hh + (te >> 3) + 32 * k));
+        for (int k = 0; k < 2; ++k) h_s[hh][k] = scale_of(h_word(a, n0 + column(hh, (te >> 3) + 32 * k)));
     }
-    // In the cooperative pass over a finished 64-column half this thread owns hidden units [u, u + 4) (rows 32 q + l of the
-    // tile are gate q of unit 32 mt + l) for the columns te / 8 and te / 8 + 32 of that half.
-    const uint32_t l = 4 * (te & 7), u = blockIdx.x * 32 + l;
-    // The 64 columns of a half are finished by the S CTAs of the cluster, w columns each (S is a power of two here): rank r
-    // takes columns [r w, r w + w).  Every CTA sends its partial sums of those columns straight into rank r's exchange
-    // buffer (slot = sender's rank), so the owner adds S slots from its own shared memory - no remote loads, whose round
-    // trips would sit on the step's critical path.  Without a K split (S = 1) the buffer is simply the parked half tile.
+    // The positions of a pass are finished by the S CTAs of the cluster, w each: rank r takes [r w, + w).  Every CTA sends its partial sums of those
+    // columns straight into rank r's exchange buffer (slot = sender's rank), so the owner adds S slots from its own shared memory - no remote loads, whose
+    // round trips would sit on the step's critical path.  Without a K split (S = 1) the buffer is simply the parked pass.
     constexpr uint32_t w = 64 / S;
     const uint32_t c_lo = rank * w, c_hi = c_lo + w;
-    uint32_t peer[8];   // this CTA's exchange buffer as seen ... and the peers': shared::cluster addresses
-#pragma unroll
-    for (uint32_t r = 0; r < 8; ++r) {
-      peer[r] = smem_u32(park);
-      if (S > 1 && r < S) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer[r]) : "r"(smem_u32(park)), "r"(r));
-    }
     float4 bias[4];   // the same for every step
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      bias[q] = ld4(a.bias + (size_t)q * a.H + u);
+      bias[q] = own_u ? ld4(a.bias + (size_t)q * a.H + u) : make_float4(0.f, 0.f, 0.f, 0.f);
       if (q == 1) { bias[q].x += a.forget_bias; bias[q].y += a.forget_bias; bias[q].z += a.forget_bias; bias[q].w += a.forget_bias; }
     }
     uint32_t cg = 0, pf_phase = 0, pr_phase = 0;
@@ -244,30 +244,32 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
       for (int hh = 0; hh < BNT / 64; ++hh)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          const uint32_t c = (te >> 3) + 32 * k, n = n0 + 64 * hh + c;
-          const bool mine = n < N && c >= c_lo && c < c_hi;
+          const uint32_t c = (te >> 3) + 32 * k, n = n0 + column(hh, c);
+          const bool mine = own_u && n < N && c >= c_lo && c < c_hi;
           cp[hh][k] = mine ? ld4(c_prev + u + (size_t)a.H * n) : make_float4(0.f, 0.f, 0.f, 0.f);
           hm[hh][k] = (mine && a.hmask) ? ld4(a.hmask + u + (a.hmask_full ? (size_t)a.hmask_ld * n : 0)) : make_float4(1.f, 1.f, 1.f, 1.f);
         }
-      float f[2] = {1.f, 1.f}, row_f = row_x;   // F16: 2^-s of the columns lane and lane + 32 in the coming chains, and of the row
-      if (F16 && has_cols) { f[0] = inv_scale_of(__ldg(a.x_scale + (size_t)t * a.B + hn0)); f[1] = inv_scale_of(__ldg(a.x_scale + (size_t)t * a.B + hn0 + 32)); }
-      float sum[64];
+      float f[kHalf / 32], row_f = row_x;   // F16: 2^-s of the columns lane (and lane + 32) in the coming chains, and of the row
 #pragma unroll
-      for (int q = 0; q < 64; ++q) sum[q] = 0.f;
+      for (uint32_t k = 0; k < kHalf / 32; ++k) f[k] = F16 && hn0 + 32 * k < N ? inv_scale_of(__ldg(a.x_scale + (size_t)t * a.B + hn0 + 32 * k)) : 1.f;
+      float sum[kHalf];
+#pragma unroll
+      for (uint32_t q = 0; q < kHalf; ++q) sum[q] = 0.f;
 #pragma unroll 1
       for (uint32_t c = 0; c < nchunks; ++c, ++cg) {
         const uint32_t buf = cg % kBufs;
         if (F16 && c == x_chunks) {
-          f[0] = h_f[0]; f[1] = h_f[1]; row_f = row_h;
-          if (t == 0 && has_cols) { f[0] = inv_scale_of(__ldg(a.h0_scale + hn0)); f[1] = inv_scale_of(__ldg(a.h0_scale + hn0 + 32)); }
+          row_f = row_h;
+#pragma unroll
+          for (uint32_t k = 0; k < kHalf / 32; ++k) f[k] = t || hn0 + 32 * k >= N ? h_f[k] : inv_scale_of(__ldg(a.h0_scale + hn0 + 32 * k));
         }
         if (!ok) continue;
         if (!mbar_wait(&acc_full[buf], (cg / kBufs) & 1)) { ok = false; continue; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (F16 && has_cols) {
-          const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + 2 * half * 32;
+        const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + half * kHalf;
+        if (F16) {
 #pragma unroll
-          for (int p = 0; p < 4; ++p) {   // (16 columns of both accumulators at a time)
+          for (uint32_t p = 0; p < kHalf / 16; ++p) {   // (16 columns of both accumulators at a time)
             float v1[16], v2[16];
             tmem_ld16x2(taddr + 16 * p, taddr + BNT + 16 * p, v1, v2);
 #pragma unroll
@@ -275,15 +277,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
               // (both factors at once: the sum times one of them may leave fp32's range where the product does not)
               sum[16 * p + q] = fmaf(fmaf(v2[q], kLoScale, v1[q]), row_f * __shfl_sync(0xffffffffu, f[p / 2], 16 * (p % 2) + q), sum[16 * p + q]);
           }
-        } else if (has_cols) {
-          float v[32];
-          const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + 2 * half * 32;
-          tmem_ld32(taddr, v);
+        } else {
 #pragma unroll
-          for (int q = 0; q < 32; ++q) sum[q] += v[q];
-          tmem_ld32(taddr + 32, v);
+          for (uint32_t p = 0; p < kHalf / 32; ++p) {
+            float v[32];
+            tmem_ld32(taddr + 32 * p, v);
 #pragma unroll
-          for (int q = 0; q < 32; ++q) sum[32 + q] += v[q];
+            for (int q = 0; q < 32; ++q) sum[32 * p + q] += v[q];
+          }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -294,48 +295,40 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
         // Every CTA's exchange buffer is free once its owner has read the previous pass: the owners say so on park_free
         // (S > 1), or this CTA's own threads have left the previous pass (the barrier at its end).
         if (S > 1 && ok && !mbar_wait_cluster(&park_free, pr_phase ^ 1)) ok = false;
-        if (half == (uint32_t)hh) {
-          // column q of this half goes to rank q / w, slot = this rank, as column q % w; 32 consecutive rows per warp store
-          const uint32_t row = quarter * 32 + lane;
-#pragma unroll
-          for (int q = 0; q < 64; ++q) {
-            const uint32_t dst = peer[(uint32_t)q / w] + 4u * (((rank * w + (uint32_t)q % w) * BM) + row);
-            if (S > 1) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(sum[q]) : "memory");
-            else park[(size_t)q * BM + row] = sum[q];
-          }
-        }
         if (S > 1) {
-          // each sending warp reports on its own: its lanes' stores are ordered before the arrivals by the warp barrier,
-          // so a receiver can start as soon as the 4 S sending warps of the cluster are through
-          if (half == (uint32_t)hh) {
-            __syncwarp();
-            if (lane < S) mbar_arrive_remote(&park_full, lane);   // (release at cluster scope)
+#pragma unroll
+          for (uint32_t rr = 0; rr < S / 2; ++rr) {
+            const uint32_t to = mapa_u32(smem_u32(park), half * (S / 2) + rr) + 4u * (rank * w * BM), bar = mapa_u32(smem_u32(&park_full), half * (S / 2) + rr);
+#pragma unroll
+            for (uint32_t q = 0; q < w; q += 4)   // position q + lane % 4 of the rank's, rows of the lane's quad
+              send4(to + 4u * park_at(q + (lane & 3), row >> 2), transpose4(sum + (32 * hh + rr * w + q) % kHalf, lane), bar);
           }
           const bool got = mbar_wait_cluster(&park_full, pf_phase);
           ok = bar_and(1, 256, ok && got) != 0;
           pf_phase ^= 1; pr_phase ^= 1;
+          if (te == 0) mbar_expect_tx(&park_full, kParkBytes);   // (the next pass; it begins when this CTA has arrived on the others' park_free)
         } else {
+#pragma unroll
+          for (uint32_t q = 0; q < 32; ++q) park[park_at(32 * half + q, row >> 2) + (row & 3)] = sum[32 * hh + q];
           ok = bar_and(1, 256, ok) != 0;
         }
         // ---- the LSTM epilogue on this CTA's columns of the half: the arithmetic of epilogue_pass (EPI_LSTM_CELL), the S
         // partial sums added in split order, c / h / the operand planes of h.  The planes of h, which the next step waits for,
         // go out first and are published before the other stores are issued.
-        const uint32_t nh = n0 + 64 * hh;
         const bool last_pass = hh == BNT / 64 - 1;
         float4 g[2][4], cn[2], hv[2], phi[2], plo[2];
         bool live[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          const uint32_t c = (te >> 3) + 32 * k, n = nh + c;
-          live[k] = ok && n < N && c >= c_lo && c < c_hi;
+          const uint32_t c = (te >> 3) + 32 * k, n = n0 + column(hh, c);
+          live[k] = ok && own_u && n < N && c >= c_lo && c < c_hi;
           if (!live[k]) continue;
-          const float* col = park + (size_t)(c - c_lo) * BM + l;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            float4 acc = ld4(col + 32 * q);
+            const float* col = park + park_at(c - c_lo, 8 * q + (te & 7));
+            float4 acc = ld4(col);
 #pragma unroll
-            for (uint32_t r = 1; r < 8; ++r)
-              if (r < S) { const float4 pv = ld4(col + (size_t)r * w * BM + 32 * q); acc.x += pv.x; acc.y += pv.y; acc.z += pv.z; acc.w += pv.w; }
+            for (uint32_t r = 1; r < S; ++r) { const float4 pv = ld4(col + (size_t)r * w * BM); acc.x += pv.x; acc.y += pv.y; acc.z += pv.z; acc.w += pv.w; }
             const float4 x = make_float4(acc.x + bias[q].x, acc.y + bias[q].y, acc.z + bias[q].z, acc.w + bias[q].w);
             g[k][q] = q == 3 ? make_float4(gate_tanh(x.x), gate_tanh(x.y), gate_tanh(x.z), gate_tanh(x.w))
                              : make_float4(gate_sigmoid(x.x), gate_sigmoid(x.y), gate_sigmoid(x.z), gate_sigmoid(x.w));
@@ -350,8 +343,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
             const float4 hmk = a.hmask ? make_float4(hv[k].x * mk.x, hv[k].y * mk.y, hv[k].z * mk.z, hv[k].w * mk.w) : hv[k];
             split_tf32(hmk.x, phi[k].x, plo[k].x); split_tf32(hmk.y, phi[k].y, plo[k].y);
             split_tf32(hmk.z, phi[k].z, plo[k].z); split_tf32(hmk.w, phi[k].w, plo[k].w);
-            st4(hn_hi + (size_t)n * a.hn_pitch + u, phi[k]);
-            st4(hn_lo + (size_t)n * a.hn_pitch + u, plo[k]);
+            if (a.hn_hi) {
+              st4(hn_hi + (size_t)n * a.hn_pitch + u, phi[k]);
+              st4(hn_lo + (size_t)n * a.hn_pitch + u, plo[k]);
+            }
             if (F16 && t + 1 < a.T) {
               // (of the value that the TF32 pair stands for, as a single step's call makes it of those planes)
               const float hs = h_s[hh][k];
@@ -377,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           if (!live[k]) continue;
-          const uint32_t n = nh + (te >> 3) + 32 * k;
+          const uint32_t n = n0 + column(hh, (te >> 3) + 32 * k);
 #pragma unroll
           for (int q = 0; q < 4; ++q) st4(gates_t + (size_t)q * a.H + u + (size_t)M * n, g[k][q]);
           const size_t ei = u + (size_t)a.H * n;
@@ -495,7 +490,7 @@ int seq_fwd_dispatch(SeqOp op, uint32_t bn, uint32_t S, dyb200_ctx* ctx, const T
 }
 
 // ---- the inputs of the F16 form, one launch: a warp per line ----
-// x: planes of the columns' inputs (hi + lo) -> fp16 pairs, a word per line.  h_{-1}: h0 .* mask -> TF32 planes (unless they are in place) and
+// x: planes of the columns' inputs (hi + lo, or the values themselves without lo planes) -> fp16 pairs, a word per line.  h_{-1}: h0 .* mask -> TF32 planes (unless they are in place) and
 // fp16 pairs of what those stand for, a word per line: the largest of its values and the mask's.  mask: the words alone.
 struct SeqPrep {
   const float *x_hi, *x_lo; uint32_t x_ld, I, x_lines; __half *x16_hi, *x16_lo; uint32_t x16_pitch; uint32_t* x_scale;
@@ -511,11 +506,11 @@ __global__ void __launch_bounds__(256) k_seq_prep(const __grid_constant__ SeqPre
   if (kind == 2 && line >= a.mask_lines) return;
   const uint32_t n = kind == 0 ? a.I : a.H;
   const float *p = kind == 0 ? a.x_hi + (size_t)line * a.x_ld : kind == 1 ? a.h0 + (size_t)line * a.H : a.mask + (size_t)line * a.H;
-  const float *p2 = kind == 0 ? a.x_lo + (size_t)line * a.x_ld : kind == 1 && a.mask ? a.mask + (a.mask_full ? (size_t)line * a.H : 0) : nullptr;
+  const float *p2 = kind == 0 ? (a.x_lo ? a.x_lo + (size_t)line * a.x_ld : nullptr) : kind == 1 && a.mask ? a.mask + (a.mask_full ? (size_t)line * a.H : 0) : nullptr;
   const bool vec = aligned16(p) && (!p2 || aligned16(p2));
   auto mag = [](float4 v) { return max(max(finite_mag(v.x), finite_mag(v.y)), max(finite_mag(v.z), finite_mag(v.w))); };
   uint32_t m = kind == 1 && !p2 ? 0x3f800000u : 0;   // (h_{-1}: no smaller than the scale of later h, which an h_{-1} from a call for the step before is)
-  auto value = [&](uint32_t e) {   // elements [e, e + 4), n is a multiple of 4
+  auto value = [&](uint32_t e) {   // elements [e, e + 4): n is a multiple of 4, or the line goes on with zeros (planes)
     float4 v = vec ? ld4(p + e) : make_float4(p[e], p[e + 1], p[e + 2], p[e + 3]);
     if (p2) {
       const float4 w = vec ? ld4(p2 + e) : make_float4(p2[e], p2[e + 1], p2[e + 2], p2[e + 3]);
@@ -528,7 +523,7 @@ __global__ void __launch_bounds__(256) k_seq_prep(const __grid_constant__ SeqPre
     if (kind == 1) {
       float4 hi, lo;
       split_tf32(v.x, hi.x, lo.x); split_tf32(v.y, hi.y, lo.y); split_tf32(v.z, hi.z, lo.z); split_tf32(v.w, hi.w, lo.w);
-      if (!a.h0_done) { st4(a.hn_hi + (size_t)line * a.hn_pitch + e, hi); st4(a.hn_lo + (size_t)line * a.hn_pitch + e, lo); }
+      if (!a.h0_done && a.hn_hi) { st4(a.hn_hi + (size_t)line * a.hn_pitch + e, hi); st4(a.hn_lo + (size_t)line * a.hn_pitch + e, lo); }
       v = make_float4(hi.x + lo.x, hi.y + lo.y, hi.z + lo.z, hi.w + lo.w);
     }
     return v;
@@ -566,18 +561,20 @@ int layer_inputs(dyb200_ctx* ctx, dyb200_wgrad* deferred, const float* Wx, const
 
 }  // namespace
 
-// Layers from 512 units on whose batch is in whole 64-column tiles and whose tiles are all resident (one CTA per SM: 225 KB of shared memory); the
-// TF32 form serves narrower ones.  64-column tiles where there are SMs for them (us per step, I = H = 1024, TF32 / this form with 128 / with 64
-// columns: batch 128 16.5 / 14.3 / 10.5, 256 23.3 / 17.4 / 14.8; batch 512 has 128 columns only, 40.8 / 25.4; batch 64 11.1 / - / 9.0), then as
-// many K splits as there are SMs for, four k-blocks each on average and more (Wx and Wh are cut separately, so the last share may be short or
+// Layers of more than 384 units (narrower ones: lstm_rec.cu and the TF32 form) and batches of more than eight columns (fewer: lstm_wide.cu) whose tiles are
+// all resident (one CTA per SM: 225 KB of shared memory).  64-column tiles where there are SMs for them (us per step, I = H = 1024, TF32 / this form
+// with 128 / with 64 columns: batch 128 16.5 / 14.3 / 10.5, 256 23.3 / 17.4 / 14.8; batch 512 has 128 columns only, 40.8 / 25.4; batch 64 11.1 / - / 8.4),
+// then as many K splits as there are SMs for, four k-blocks each on average and more (Wx and Wh are cut separately, so the last share may be short or
 // empty: 9 + 9 k-blocks make 6, 6, 6, 0, the longest still shorter than the 10 of two splits).  They are clusters whatever dyb200_ctx_cluster_splitk
-// says: there is no other form, and another number of splits would give other bits.
+// says: there is no other form, and another number of splits would give other bits.  Columns and units past the end of a tile are computed and
+// dropped: a launch and more per step, which such layers took before, was 19 us at (512, 1024, 100 columns), 25 at (300, 600, 30), 24 at (512, 768, 300),
+// 31 at (512, 1000, 100) and 18 at (256, 1024, 16); here it is 8.9, 7.1, 10.8, 8.9 and 7.1.
 bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* bn, uint32_t* S) {
-  if (H < 512 || H % 32 != 0 || I == 0 || I % 4 != 0 || B == 0 || B % 64 != 0) return false;
-  const uint32_t sms = (uint32_t)ctx->sm_count, tiles_m = 4 * H / BM, kb = (I + 63) / 64 + (H + 63) / 64;
-  *bn = tiles_m * (B / 64) <= sms ? 64 : 128;
-  const uint32_t tiles = tiles_m * (B / *bn);
-  if (B % *bn != 0 || B / *bn > 32) return false;   // (one hand-over counter per column block)
+  if (H <= 384 || H % 4 != 0 || I == 0 || B <= 8) return false;
+  const uint32_t sms = (uint32_t)ctx->sm_count, tiles_m = (H + 31) / 32, kb = (I + 63) / 64 + (H + 63) / 64;
+  *bn = tiles_m * ((B + 63) / 64) <= sms ? 64 : 128;
+  const uint32_t tiles_n = (B + *bn - 1) / *bn, tiles = tiles_m * tiles_n;
+  if (tiles_n > 32) return false;   // (one hand-over counter per column block)
   for (uint32_t s = *bn == 64 ? 8 : 4; s >= 1; s /= 2) {
     if (tiles * s > sms || (s > 1 && kb / s < 4)) continue;
     if (seq_fwd_dispatch<true>(SEQ_SET_SMEM, *bn, s, ctx) != DYB200_OK) return false;
@@ -592,7 +589,7 @@ bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, ui
 }
 
 int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q) {
-  const uint32_t I = q.I, H = q.H, B = q.B, T = q.T, G = 4 * H;
+  const uint32_t I = q.I, H = q.H, B = q.B, T = q.T, G = 4 * H, tiles_m = (H + 31) / 32, rows = tiles_m * BM;
   uint32_t bn, S;
   DYB_CHECK_ARG(ctx, dyb200_seq_f16_plan(ctx, I, H, B, &bn, &S), "lstm_seq_fwd: shape %u, %u x %u", I, H, B);
   F16Gates W;
@@ -613,11 +610,11 @@ int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q) {
   DYB_LAUNCHED(ctx);
   TmapPack tm;
   memset(&tm, 0, sizeof(tm));
-  struct { __half* plane; uint32_t rows, K, pitch, box; bool mn; } maps[8] = {
-      {W.x_hi, G, I, G, BM, true}, {W.x_lo, G, I, G, BM, true}, {p.x16_hi, T * B, I, xp, bn, false}, {p.x16_lo, T * B, I, xp, bn, false},
-      {W.h_hi, G, H, G, BM, true}, {W.h_lo, G, H, G, BM, true}, {p.h16_hi, slots * B, H, hp, bn, false}, {p.h16_lo, slots * B, H, hp, bn, false}};
+  struct { __half* plane; uint32_t n, K, pitch, box; bool mn; } maps[8] = {
+      {W.x_hi, rows, I, rows, BM, true}, {W.x_lo, rows, I, rows, BM, true}, {p.x16_hi, T * B, I, xp, bn, false}, {p.x16_lo, T * B, I, xp, bn, false},
+      {W.h_hi, rows, H, rows, BM, true}, {W.h_lo, rows, H, rows, BM, true}, {p.h16_hi, slots * B, H, hp, bn, false}, {p.h16_lo, slots * B, H, hp, bn, false}};
   for (int k = 0; k < 8; ++k)
-    if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[k], maps[k].plane, maps[k].rows, maps[k].K, maps[k].pitch, maps[k].box, maps[k].mn))) return rc;
+    if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[k], maps[k].plane, maps[k].n, maps[k].K, maps[k].pitch, maps[k].box, maps[k].mn))) return rc;
   SeqFwd a;
   memset(&a, 0, sizeof(a));
   a.T = T; a.B = B; a.H = H; a.kb0 = xp / 64; a.kb1 = hp / 64;
@@ -629,7 +626,7 @@ int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q) {
   a.ready = ctx->dev_flags + DYB200_DEV_SEQ0;
   a.flags = ctx->dev_flags;
   if (T > 1) DYB_CUDA(ctx, cudaMemsetAsync(a.ready, 0, 32 * sizeof(uint32_t), ctx->stream));   // (a single step's CTAs count, but nobody waits)
-  return seq_fwd_dispatch<true>(SEQ_LAUNCH, bn, S, ctx, &tm, &a, dim3(G / BM, B / bn, S), 2.0 * G * (double)B * (I + H) * T, I + H);
+  return seq_fwd_dispatch<true>(SEQ_LAUNCH, bn, S, ctx, &tm, &a, dim3(tiles_m, (B + bn - 1) / bn, S), 2.0 * G * (double)B * (I + H) * T, I + H);
 }
 
 extern "C" {
@@ -666,21 +663,24 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
   // 763 / 1228 / 2070 against 535 / 930 / 1738.)
   const uint32_t bn = dyb200_tc_tile_cols(B);
   const uint32_t kb0 = (I + 31) / 32, kb1 = (H + 31) / 32, kb_total = kb0 + kb1;
-  const bool resident = ctx->seq_kernels && deferred && T >= 2 && attrs->weightnoise_std == 0.f && H % 32 == 0 && I % 4 == 0 &&
-                    dyb200_tc_eligible(G, B, 2.0 * G * B * (I + H)) && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 &&
+  const bool sequence = ctx->seq_kernels && T >= 2 && attrs->weightnoise_std == 0.f && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 &&
                     Wh->d[0] == G && Wh->d[1] == H && t_size(b) == G && aligned16(gates_all->v) && aligned16(b->v) && aligned16(c0->v) &&
                     aligned16(c_all->v) && aligned16(h_all->v) && (!mh || aligned16(mh)) &&
                     (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H));
+  const bool resident = sequence && deferred && H % 32 == 0 && I % 4 == 0 && dyb200_tc_eligible(G, B, 2.0 * G * B * (I + H));
   uint32_t S = 1, f16_bn;
   bool wide_fits = true;
   SeqPlanes pl;
-  if (resident && dyb200_seq_f16_plan(ctx, I, H, B, &f16_bn, &S) && dyb200_wgrad_seq_planes(deferred, T, B, &pl)) {   // (wide layers)
+  // (wide layers.  Without an accumulator the inputs are x itself, and a sequence has to be worth making the weights' pairs for)
+  if (sequence && (deferred || (!attrs->dropout && T >= kRecMinSteps && I % 4 == 0)) && dyb200_seq_f16_plan(ctx, I, H, B, &f16_bn, &S) &&
+      (!deferred || dyb200_wgrad_seq_planes(deferred, T, B, &pl))) {
     { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
-    DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_seq_fwd: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
+    if (deferred) DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_seq_fwd: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
+    else { pl.X.hi = x_all->v; pl.X.lo = nullptr; pl.X.pitch = I; pl.Hs.hi = pl.Hs.lo = nullptr; pl.Hs.pitch = 0; }
     SeqF16Call q{I, H, B, T, Wx->v, Wh->v, b->v, h0->v, c0->v, mh, mh_full, attrs->forget_gate_bias, gates_all->v, c_all->v, h_all->v, pl.X, pl.Hs, 0, 0};
     rc = dyb200_seq_f16(ctx, q);
     if (rc != DYB200_ENOMEM) {
-      if (!rc) dyb200_wgrad_seq_done(deferred);
+      if (!rc && deferred) dyb200_wgrad_seq_done(deferred);
       return rc;
     }
     wide_fits = false;   // (no room for the pairs of all steps: the single-step calls, with those of one)

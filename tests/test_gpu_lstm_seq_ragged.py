@@ -1,0 +1,70 @@
+"""The forward recurrence of wide layers (csrc/lstm_seq.cu, F16) where units and columns do not fill its tiles: batches below and beside whole 64 columns on
+64- and 128-column tiles, units that are no multiple of 32 (the last tile of 32 units partly there), inputs of any number of rows, K splits, masks, and calls
+without an accumulator, whose inputs are split from x itself.  Step by step against float64 from the device's own h_{t-1} and c_{t-1}; bars as in
+test_gpu_lstm_seq_f16.py.  Where the single-step call takes this form too (from 33 columns on, with an accumulator) it must give the same bits."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("I,H,B,T,mask,acc", [
+    (300, 600, 30, 8, "full", True),        # 19 tiles of units, the last of 24; one block, 30 columns
+    (512, 1000, 100, 8, "one", True),       # the last block has 36 columns
+    (7, 388, 9, 9, None, True),             # the smallest of its range; a tile of four units
+    (130, 516, 500, 3, "full", True),       # 128-column tiles, the last of 116
+    (512, 768, 300, 3, None, True),
+    (33, 1020, 65, 3, "full", True),        # a block of one column
+    (512, 1024, 64, 8, None, False),
+    (128, 412, 17, 8, None, False),
+])
+def test_sequence_that_does_not_fill_its_tiles(I, H, B, T, mask, acc):
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    bn, S = C.c_uint32(), C.c_uint32()
+    assert ctx.L.dyb200i_seq_f16_tiling(ctx.h, I, H, B, C.byref(bn), C.byref(S)) == 1
+    gen = torch.Generator("cuda").manual_seed(H + B)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    x, h0, c0, b = rnd(T * B, I), rnd(B, H) * 3.0, rnd(B, H), rnd(4 * H) * 0.1
+    x *= torch.exp2(torch.randint(-40, 3, (T * B, 1), device="cuda", generator=gen).float())
+    Wx, Wh = rnd(I, 4 * H) / I ** 0.5, rnd(H, 4 * H) / H ** 0.5
+    mB = B if mask == "full" else 1
+    mx, mh = [((torch.rand(mB, n, device="cuda", generator=gen) < 0.8) / 0.8).float() if mask else torch.ones(1, n, device="cuda") for n in (I, H)]
+    at, tm = capi.LstmGatesAttrs(1 if mask else 0, 0.0, 1.0), (g.T(mx), g.T(mh)) if mask else (None, None)
+    W = (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1))
+    out, launches = [], []
+    for single in (False, True) if acc and B > 32 else (False,):
+        w = ctx.wgrad_create(4 * H, I, H, T * B) if acc else None
+        gates, cs, hs = (torch.full((T * B + 1, n), 7.0, device="cuda") for n in (4 * H, H, H))     # (a column past the end)
+        at0 = ctx.launches()
+        if single:
+            for t in range(T):
+                sl, pr = slice(t * B, (t + 1) * B), slice((t - 1) * B, t * B)
+                ctx.lstm_fwd_fused_at(g.T(x[sl]), g.T(hs[pr] if t else h0), g.T(cs[pr] if t else c0), *W, *tm, at, g.T(gates[sl]), g.T(cs[sl]), g.T(hs[sl]), w, t * B)
+        else:
+            ctx.lstm_seq_fwd(g.T(x, [I], T * B), g.T(h0), g.T(c0), *W, *tm, at, g.T(gates[:T * B], [4 * H], T * B), g.T(cs[:T * B], [H], T * B), g.T(hs[:T * B], [H], T * B), w, T)
+        launches.append(ctx.launches() - at0)
+        torch.cuda.synchronize()
+        if acc:
+            ctx.wgrad_destroy(w)
+        for o in (gates, cs, hs):
+            assert bool((o[T * B] == 7.0).all())
+        out.append((gates[:T * B], cs[:T * B], hs[:T * B]))
+    assert launches[0] <= 5, launches                        # inputs, weights (two launches), pairs, the recurrence
+    for p, q in zip(out[0], out[-1]):
+        assert torch.equal(p, q)
+    gates, cs, hs = (o.double().view(T, B, -1) for o in out[0])
+    for t in range(T):
+        xt, hp, cp = x.double().view(T, B, I)[t] * mx.double(), (hs[t - 1] if t else h0.double()) * mh.double(), cs[t - 1] if t else c0.double()
+        pre = xt @ Wx.double() + hp @ Wh.double() + b.double()
+        bar = 4.5e-7 * (xt.norm(dim=1)[:, None] * Wx.double().norm(dim=0) + hp.norm(dim=1)[:, None] * Wh.double().norm(dim=0)) + 3e-6
+        pre[:, H:2 * H] += 1.0
+        want = torch.cat([torch.sigmoid(pre[:, :3 * H]), torch.tanh(pre[:, 3 * H:])], dim=1)
+        assert bool(((gates[t] - want).abs() <= bar).all()), "step %d: %.3g" % (t, float(((gates[t] - want).abs() / bar).max()))
+        i, f, o, gg = gates[t].split(H, dim=1)
+        assert bool(((cs[t] - (i * gg + f * cp)).abs() <= 2e-7 * ((i * gg).abs() + (f * cp).abs())).all())
+        assert bool(((hs[t] - o * torch.tanh(cs[t])).abs() <= 5e-7).all())
+    assert ctx.device_errors() == 0
