@@ -952,6 +952,112 @@ __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jo
   }
 }
 
+// ---- both in one pass, for operands whose rows fit into registers between the scale and the split ----
+// (The passes above read an operand twice and are two launches and a clear.  us, those / one pass: gate weights of 1024 + 1024 columns x 4096 (34 MB) 28 / 17, 1024 lines of
+// 10 000 positions (41 MB) 27 / 22, 1024 lines of 4096 11 / 7, of 10 000 24 / 17.  Strips of 32 positions store 64-byte pieces: from memory, not L2, that is the
+// slower form, 512 lines of 50 000 positions 60 / 94.)
+// Positions: a CTA takes strips of 32 positions, 128 bytes of every line; thread -> positions [p, p + 4) of the lines t / 8, t / 8 + 32, ...
+template <int R>
+__global__ void __launch_bounds__(256) k_f16_strip(const __grid_constant__ F16Jobs jobs) {
+  dyb_grid_dep_sync();
+  __shared__ uint32_t top[8][32];
+  const uint32_t z = f16_job_of(jobs), unit = blockIdx.x - jobs.start[z];
+  const F16Job& j = jobs.job[z];
+  const bool vec = (j.ld & 3) == 0 && aligned16(j.src);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = 4 * (threadIdx.x & 7), e = 32 * unit + q, l0 = threadIdx.x >> 3;
+  float4 v[R];
+  if (vec && e + 4 <= j.n && j.lines >= 32 * R) {
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] = ld4(j.src + (size_t)j.ld * (l0 + 32 * k) + e);
+  } else {
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] = l0 + 32 * k < j.lines && e < j.n ? f16_load4(j.src + (size_t)j.ld * (l0 + 32 * k), e, j.n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  uint32_t m[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    m[0] = max(m[0], finite_mag(v[k].x)); m[1] = max(m[1], finite_mag(v[k].y)); m[2] = max(m[2], finite_mag(v[k].z)); m[3] = max(m[3], finite_mag(v[k].w));
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = max(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
+    m[i] = max(m[i], __shfl_xor_sync(0xffffffffu, m[i], 16));
+    if (lane < 8) top[warp][q + i] = m[i];
+  }
+  __syncthreads();
+  float s[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m[i] = max(m[i], top[w][q + i]);
+    s[i] = scale_of(m[i]);
+    if (threadIdx.x < 8 && e + i < j.n) j.scale[e + i] = m[i];
+  }
+  if (e >= j.n) return;
+  uint32_t to = e;
+  if (j.perm_H) { const uint32_t g = e / j.perm_H, u = e % j.perm_H; to = 128 * (u / 32) + 32 * g + u % 32; }   // (four units stay together)
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const uint32_t line = l0 + 32 * k;
+    if (line >= j.lines) break;
+    uint2 hi, lo;
+    split4_f16(v[k], make_float4(s[0], s[1], s[2], s[3]), hi, lo);
+    *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line + to) = hi;
+    *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line + to) = lo;
+  }
+}
+// Lines: a warp per line of up to 1024 values, a CTA per longer one.
+constexpr uint32_t kOneLine = 16384, kOneStrip = 1024;   // longest line, most lines of a strip
+template <uint32_t R>
+__device__ __forceinline__ void line_pairs(const F16Job& j, uint32_t line, uint32_t e0, uint32_t step, uint32_t* red) {
+  const float* p = j.src + (size_t)j.ld * line;
+  const bool vec = aligned16(p);
+  float4 v[R];
+  if (vec && e0 + (R - 1) * step + 4 <= j.n) {
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k) v[k] = ld4(p + e0 + step * k);
+  } else {
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k) v[k] = e0 + step * k < j.n ? f16_load4(p, e0 + step * k, j.n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  uint32_t m = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < R; ++k) m = max(m, mag4(v[k]));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (red) {
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = max(m, red[w]);
+  }
+  if (e0 == 0) j.scale[line] = m;
+  const float s = scale_of(m);
+#pragma unroll
+  for (uint32_t k = 0; k < R; ++k) {
+    const uint32_t e = e0 + step * k;
+    if (e >= j.n) break;
+    uint2 hi, lo;
+    split4_f16(v[k], make_float4(s, s, s, s), hi, lo);
+    *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line + e) = hi;
+    *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line + e) = lo;
+  }
+}
+template <uint32_t R>   // (16: lines of more than 8192)
+__global__ void __launch_bounds__(256) k_f16_line(const __grid_constant__ F16Jobs jobs) {
+  dyb_grid_dep_sync();
+  __shared__ uint32_t red[8];
+  const uint32_t z = f16_job_of(jobs), unit = blockIdx.x - jobs.start[z];
+  const F16Job& j = jobs.job[z];
+  if (j.n > 1024) {
+    line_pairs<R>(j, unit, 4 * threadIdx.x, 1024, red);
+  } else {
+    const uint32_t line = 8 * unit + (threadIdx.x >> 5);
+    if (line < j.lines) line_pairs<8>(j, line, 4 * (threadIdx.x & 31), 128, nullptr);
+  }
+}
+constexpr uint64_t kOneValues = 12u << 20;   // (48 MB and as much again of pairs: L2 still holds most of both)
+bool f16_one_pass(const F16Job& j) { return !j.src_lo && !j.low && (j.mode == F16_ELEM ? j.lines <= kOneStrip && (uint64_t)j.lines * j.n <= kOneValues : j.n <= kOneLine); }
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1130,6 +1236,29 @@ int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t l
   return DYB200_OK;
 }
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
+  if (jobs->n == 0) return DYB200_OK;
+  F16Jobs rest = *jobs;
+  rest.n = 0;
+  for (const int mode : {F16_ELEM, F16_LINE}) {   // (a launch per kind)
+    F16Jobs part;
+    part.n = 0; part.start[0] = 0;
+    uint32_t lines = 0, longest = 0;
+    for (int k = 0; k < jobs->n; ++k) {
+      const F16Job& j = jobs->job[k];
+      if (j.mode != mode) continue;
+      if (!f16_one_pass(j)) { rest.job[rest.n++] = j; continue; }
+      if (j.lines > lines) lines = j.lines;
+      if (j.n > longest) longest = j.n;
+      part.job[part.n] = j;
+      part.start[part.n + 1] = part.start[part.n] + (mode == F16_ELEM ? (j.n + 31) / 32 : j.n > 1024 ? j.lines : (j.lines + 7) / 8);
+      ++part.n;
+    }
+    if (part.n == 0 || part.start[part.n] == 0) continue;
+    dyb_launch(mode == F16_LINE ? (longest <= 8192 ? k_f16_line<8> : k_f16_line<16>) : lines <= 256 ? k_f16_strip<8> : lines <= 512 ? k_f16_strip<16> : k_f16_strip<32>,
+               part.start[part.n], 256, 0, ctx, part);
+    DYB_LAUNCHED(ctx);
+  }
+  jobs = &rest;
   if (jobs->n == 0) return DYB200_OK;
   jobs->start[0] = 0;
   if (jobs->words) DYB_CUDA(ctx, cudaMemsetAsync(jobs->words, 0, jobs->n_words * sizeof(uint32_t), ctx->stream));

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
     const uint32_t nchains = total ? ((k0 + total - 1) >> 3) - (k0 >> 3) + 1 : 0;
     // The exchange goes in passes of 64 columns: pass hh takes columns [32 hh, + 32) of either half, position p of a pass being column p % 32 of the
     // half p / 32.  Rank r finishes the positions [r w, + w); sender s's partial sums of them lie in slot s of r's buffer.
-    constexpr uint32_t w = 64 / S, KC = w / 8, GB = KC < 2 ? KC : 2;   // a warp holds one column: 8 columns of a slice at a time, GB of them in flight
+    constexpr uint32_t w = 64 / S, KC = w / 8, GB = KC < 2 ? KC : REC ? 2 : KC < 4 ? KC : 4;   // a warp holds one column: 8 columns of a slice at a time, GB of them in flight
     const uint32_t uq = 4 * (te & 31);                                  // this thread's four rows of the tile
     uint32_t cg = 0, pf_phase = 0, pr_phase = 0;
     bool ok = true;   // the same for all 256 threads after every bar_and below
@@ -346,6 +346,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             }
         }
       }
+      if (!REC && own && (te & 7) == 0)   // (the values that this tile adds to)
+#pragma unroll
+        for (int hh = 0; hh < BNT / 64; ++hh)
+#pragma unroll
+          for (uint32_t k = 0; k < KC; ++k) {
+            const uint32_t n = col0 + column(hh, k);
+            if (n < cols) asm volatile("prefetch.global.L2 [%0];" ::"l"(dst + (size_t)n * a.M + m));
+          }
       // ---- drain the chains of this product ----
       float sum[kHalf];
 #pragma unroll
