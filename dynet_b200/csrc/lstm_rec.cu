@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
 // grid (C, G, directions), cluster (C, 1, 1); block = C U threads rounded up to warps.  KD = gate rows per slice: 8 KD >= 4 U.
 // Dynamic shared memory: part[2][C][ncap][U], dg[2][ncap][8 KD], dcs[ncap][U].  (dg in two: a step's gradients are written as soon
 // as the sums of the step before have arrived, which some warps of this CTA may still be forming for other CTAs.)
-template <int KD, int NB, int NF = NB>
-__global__ void __launch_bounds__(KD == 16 ? 256 : 384, 1) k_lstm_rec_bwd(const __grid_constant__ RecBwd a) {
+template <int KD, int NB, int NF = NB, int MT = KD == 16 ? 256 : 384>   // MT: most threads of a CTA
+__global__ void __launch_bounds__(MT, 1) k_lstm_rec_bwd(const __grid_constant__ RecBwd a) {
   constexpr int KP = 8 * KD;
   extern __shared__ __align__(16) float rec_smem[];
   __shared__ __align__(8) uint64_t got[2];
@@ -505,9 +505,11 @@ FwdKernel fwd_kernel(uint32_t kd, uint32_t n) {
 #undef REC_F
 #undef REC_F4
 }
-// (16 gate rows per lane: at most 256 units and threads, 255 registers each; fewer: up to 384 threads of 168 registers)
-BwdKernel bwd_kernel(uint32_t kd, uint32_t n) {
+// (16 gate rows per lane: 255 registers at up to 256 units and threads, 168 at up to 320; fewer rows: up to 384 threads of 168)
+BwdKernel bwd_kernel(uint32_t kd, uint32_t n, uint32_t threads) {
 #define REC_B(K) (n == 1 ? k_lstm_rec_bwd<K, 1> : n == 2 ? k_lstm_rec_bwd<K, 2> : n == 3 ? k_lstm_rec_bwd<K, 4, 3> : k_lstm_rec_bwd<K, 4>)
+  if (kd == 16 && threads > 256)
+    return n == 1 ? k_lstm_rec_bwd<16, 1, 1, 320> : n == 2 ? k_lstm_rec_bwd<16, 2, 2, 320> : n == 3 ? k_lstm_rec_bwd<16, 4, 3, 320> : k_lstm_rec_bwd<16, 4, 4, 320>;
   switch (kd) {
     case 8: return REC_B(8);
     case 12: return REC_B(12);
@@ -515,13 +517,13 @@ BwdKernel bwd_kernel(uint32_t kd, uint32_t n) {
   }
 #undef REC_B
 }
-uint32_t fwd_threads(const RecPlan& p) { return 8 * p.Uf; }
+uint32_t fwd_threads(const RecPlan& p) { return 8 * p.U; }
 uint32_t bwd_threads(const RecPlan& p) { return (p.C * p.U + 31) / 32 * 32; }
 // shared memory: per column carried, and for Wh on its way into registers (forward)
-size_t fwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * 16 * p.KD + p.Uf); }
+size_t fwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * 16 * p.KD + p.U); }
 size_t bwd_col_bytes(const RecPlan& p) { return sizeof(float) * (2 * p.C * p.U + 2 * 8 * p.KD2 + p.U); }
 size_t fwd_smem(const RecPlan& p, uint32_t ncap) {
-  const size_t cols = ncap * fwd_col_bytes(p), weights = sizeof(float) * (16 * p.KD * (4 * p.Uf + 32) + 32);
+  const size_t cols = ncap * fwd_col_bytes(p), weights = sizeof(float) * (16 * p.KD * (4 * p.U + 32) + 32);
   return cols > weights ? cols : weights;
 }
 
@@ -541,10 +543,10 @@ namespace {
 
 // How many clusters run side by side (remembered per context and width class): the columns are dealt out over that many.
 int clusters_that_fit(dyb200_ctx* ctx, const RecPlan& p, bool bwd, uint32_t threads) {
-  const uint32_t C = bwd ? p.C : p.Cf;
+  const uint32_t C = p.C;
   int16_t& fit = ctx->rec_fit[bwd][p.KD / 4 - 1][C];
   if (fit == 0) {
-    const void* k = bwd ? (const void*)bwd_kernel(p.KD2, 4) : (const void*)fwd_kernel(p.KD, 4);
+    const void* k = bwd ? (const void*)bwd_kernel(p.KD2, 4, threads) : (const void*)fwd_kernel(p.KD, 4);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     if (dyb200_rec_launch_cfg(ctx, k, &cfg, attr, dim3(C, 1, 1), threads, kRecSmemMax)) return -1;
@@ -569,12 +571,11 @@ bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan*
   RecPlan p;
   // up to 256 units: 32 per CTA and at most 8 CTAs, the portable cluster size; beyond: 16 CTAs
   p.U = H <= 256 ? (H < 32 ? (H + 3) / 4 * 4 : 32u) : ((H + 15) / 16 + 3) / 4 * 4;
+  // From 8 columns on: 32 per CTA also up to 320 units (beyond, a CTA's weights do not pass through its shared memory), since more clusters
+  // of 10 CTAs than of 16 run side by side: 300 units, 35 steps, forward: 30 columns 149 -> 94 us, 130 317 -> 222, 300 656 -> 466; backward, 30 columns
+  // 115 -> 86 us.  Below, every column has a cluster of its own either way, and the smaller CTAs are through sooner: 4 columns 70 against 75 us.
+  if (H > 256 && H <= 320 && N >= 8) p.U = 32;
   p.C = (H + p.U - 1) / p.U;
-  // Forward from 8 columns on: 32 per CTA also up to 320 units (beyond, a CTA's weights do not pass through its shared memory), since more clusters
-  // of 10 CTAs than of 16 run side by side: 300 units, 35 steps, 30 columns 149 -> 94 us, 130 317 -> 222, 300 656 -> 466.  Below, every column has
-  // a cluster of its own either way, and the smaller CTAs are through sooner: 4 columns 70 against 75 us.
-  p.Uf = H > 256 && H <= 320 && N >= 8 ? 32u : p.U;
-  p.Cf = (H + p.Uf - 1) / p.Uf;
   p.KD = (H + 63) / 64 * 4;
   p.KD2 = p.U <= 16 ? 8 : p.U <= 24 ? 12 : 16;
   const int ff = clusters_that_fit(ctx, p, false, fwd_threads(p)), fb = clusters_that_fit(ctx, p, true, bwd_threads(p));
@@ -590,11 +591,11 @@ bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan*
 
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
   if (p.tcf) return dyb200_rec_tc_fwd(ctx, p.tf, a, ndir);
-  a->U = p.Uf; a->G = p.Gf; a->ncap = p.ncapf; a->flags = ctx->dev_flags;
+  a->U = p.U; a->G = p.Gf; a->ncap = p.ncapf; a->flags = ctx->dev_flags;
   FwdKernel k = fwd_kernel(p.KD, (a->N + p.Gf - 1) / p.Gf);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  int rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.Cf, p.Gf, ndir), fwd_threads(p), fwd_smem(p, p.ncapf));
+  int rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gf, ndir), fwd_threads(p), fwd_smem(p, p.ncapf));
   if (rc) return rc;
   cudaLaunchKernelEx(&cfg, k, *a);
   DYB_LAUNCHED(ctx);
@@ -611,7 +612,7 @@ int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float
   if (p.tcb) {
     if ((rc = dyb200_rec_tc_bwd(ctx, p.tb, a, ndir))) return rc;
   } else {
-    BwdKernel k = bwd_kernel(p.KD2, (a->N + p.Gb - 1) / p.Gb);
+    BwdKernel k = bwd_kernel(p.KD2, (a->N + p.Gb - 1) / p.Gb, bwd_threads(p));
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3(p.C, p.Gb, ndir), bwd_threads(p), p.ncapb * bwd_col_bytes(p));

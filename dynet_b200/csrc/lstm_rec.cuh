@@ -42,9 +42,9 @@ struct RecBwd {
 
 // lstm_rec_tc.cu: clusters per direction.
 struct RecTcPlan { uint32_t G; };
-// U hidden units per CTA, C CTAs per cluster (Uf, Cf: forward), KD / KD2 = reduction elements per lane, G clusters per direction, room for ncap
+// U hidden units per CTA, C CTAs per cluster, KD / KD2 = reduction elements per lane, G clusters per direction, room for ncap
 // columns per cluster (forward, backward).  tcf / tcb: the pass runs on the tensor pipe.
-struct RecPlan { uint32_t U, C, Uf, Cf, KD, KD2, Gf, Gb, ncapf, ncapb; bool tcf, tcb; RecTcPlan tf, tb; };
+struct RecPlan { uint32_t U, C, KD, KD2, Gf, Gb, ncapf, ncapb; bool tcf, tcb; RecTcPlan tf, tb; };
 // False when the width is outside what the registers of a cluster hold, or N columns are more than the clusters can carry.
 bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan* out);
 // ndir directions (1 or 2) share T, N and prefix.  U, G, ncap and flags are filled in here.
