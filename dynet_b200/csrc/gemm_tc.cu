@@ -1239,6 +1239,10 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
   if (jobs->n == 0) return DYB200_OK;
   F16Jobs rest = *jobs;
   rest.n = 0;
+  // (the words of all jobs at once, those that a pass below writes among them: before it)
+  bool two_pass = false;
+  for (int k = 0; k < jobs->n; ++k) two_pass = two_pass || !f16_one_pass(jobs->job[k]);
+  if (jobs->words && two_pass) DYB_CUDA(ctx, cudaMemsetAsync(jobs->words, 0, jobs->n_words * sizeof(uint32_t), ctx->stream));
   for (const int mode : {F16_ELEM, F16_LINE}) {   // (a launch per kind)
     F16Jobs part;
     part.n = 0; part.start[0] = 0;
@@ -1261,7 +1265,6 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
   jobs = &rest;
   if (jobs->n == 0) return DYB200_OK;
   jobs->start[0] = 0;
-  if (jobs->words) DYB_CUDA(ctx, cudaMemsetAsync(jobs->words, 0, jobs->n_words * sizeof(uint32_t), ctx->stream));
   for (int k = 0; k < jobs->n; ++k) {
     const F16Job& j = jobs->job[k];
     const bool one_store = j.mode == F16_LINE && j.n <= kPiece;   // (every word is written once, no maximum to start from)
