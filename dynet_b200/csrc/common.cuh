@@ -42,10 +42,11 @@ struct dyb200_ctx {
   int max_clusters[2][9];
   // sequence-persistent LSTM kernels (one launch per layer instead of one per time step): on by default
   int seq_kernels;
-  int seq_max_clusters[4][9];   // thread-block clusters of each size that fit at once, per tile width and kind of operand pairs (0 = not asked yet)
+  uint32_t seq_odd_attr_done;   // (lstm_seq.cu's kernels for units that are no multiple of four)
+  int seq_max_clusters[6][9];   // thread-block clusters of each size that fit at once, per tile width and kind of operand pairs (0 = not asked yet)
   int16_t rec_tc_fit[2][8];     // the same for lstm_rec_tc.cu: [pass][CTAs per cluster - 1]
   int16_t rec_fit[2][6][17];    // clusters of the recurrence kernels (lstm_rec.cu) that fit at once: [pass][width class][CTAs per cluster]
-  int16_t bwd_wide_fit[7];      // the same for lstm_bwd_wide.cu, by instantiation
+  int16_t bwd_wide_fit[11];     // the same for lstm_bwd_wide.cu, by instantiation
   int seq_coop;                 // 0 = not tried, 1 = launched with the cooperative attribute, -1 = the driver refused it
   int wide_refused;             // the driver refused lstm_wide.cu's gang launch: its sequences run launch by launch
   uint64_t param_version, param_tick;

@@ -148,8 +148,10 @@ struct PackedOp {
 enum F16Scale { F16_LINE = 0, F16_ELEM = 1 };
 // src_lo: the source is a pair of TF32 planes, src the hi one (null: plain fp32).
 constexpr int kF16MaxJobs = 3;
+constexpr uint32_t kF16PadMax = 16384;
 struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; const float* src_lo = nullptr;
   uint32_t perm_H = 0;        // (F16_ELEM) positions are gate rows q perm_H + u, written interleaved as dyb200_tc_param_gates does
+  uint32_t pad_H = 0;         // (F16_LINE, lines of at most kF16PadMax values) values are gate units q pad_H + u, written at q (pad_H rounded up to 64) + u, zeros between
   uint32_t* low = nullptr; };   // (F16_ELEM) a word per position, see F16Jobs::wide
 // wide: becomes 1 where the values of a position span more than a pair holds: of its blocks of eight lines that are not all zero, one's largest
 // value lies more than 2^kF16Span below the position's (jobs with `low` words).  words: scale and low words and the flag of all
@@ -158,10 +160,10 @@ constexpr int kF16Span = 24;
 struct F16Jobs { F16Job job[kF16MaxJobs]; int n; uint32_t start[kF16MaxJobs + 1];   // start: units of work before each job (set for a launch)
   uint32_t* wide = nullptr; uint32_t* words = nullptr; size_t n_words = 0; };
 // Planes and scale words for a job from the scratch arena; dyb200_f16_pack fills those of up to three jobs in one pass each.
-int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
+int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H = 0);
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
 // The same for a parameter, from the parameter cache when it is on.
-int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job);
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H = 0);
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
 // The gate weights of a layer, Wx (4H x I) and Wh (4H x H), as MN-major planes with interleaved rows (lines = their columns, 128 rows per 32 units) and one
 // scale word per row of Wx and one per row of Wh (4H words each, not interleaved); from the parameter cache when it is on.
@@ -174,7 +176,7 @@ int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t
 inline bool dyb200_f16_takes(double flops, uint32_t K) { return flops >= 24.0e9 || (flops >= 8.0e9 && K >= 256); }
 // A queue of packing work that one kernel launch executes (several small operands per launch).
 constexpr int kMaxPackJobs = 8;
-constexpr int kLayoutGates = 2, kLayoutF16 = 3, kLayoutGatesF16 = 5;   // (kLayoutF16 + F16_LINE or F16_ELEM)
+constexpr int kLayoutGates = 2, kLayoutF16 = 3, kLayoutGatesF16 = 5, kLayoutPadF16 = 6;   // (kLayoutF16 + F16_LINE or F16_ELEM; kLayoutPadF16: F16Job::pad_H)
 struct PackJob {
   const float* src; const float* mask; float* hi; float* lo;
   uint32_t ld, rows, K, mask_ld, pitch, gx, perm_H;

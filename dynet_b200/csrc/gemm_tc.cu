@@ -883,6 +883,22 @@ __device__ __forceinline__ void split4_f16(float4 v, float4 s, uint2& hi, uint2&
   hi = *reinterpret_cast<const uint2*>(h);
   lo = *reinterpret_cast<const uint2*>(l);
 }
+// Positions [e, + 4) of a line to the planes: as they lie, or those of gate rows where they go (F16Job::perm_H; four units of a gate stay together
+// where the units come in fours).  The pitch is a multiple of 64: the last item's padding stays inside the line's pitch.
+__device__ __forceinline__ void store_pairs(const F16Job& j, uint32_t line, uint32_t e, uint2 hi, uint2 lo) {
+  __half *ph = j.hi + (size_t)j.pitch * line, *pl = j.lo + (size_t)j.pitch * line;
+  auto perm = [&](uint32_t x) { const uint32_t g = x / j.perm_H, u = x % j.perm_H; return 128 * (u / 32) + 32 * g + u % 32; };
+  if (j.perm_H && (j.perm_H & 3)) {
+    const __half *h = reinterpret_cast<const __half*>(&hi), *l = reinterpret_cast<const __half*>(&lo);
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+      if (e + i < j.n) { const uint32_t to = perm(e + i); ph[to] = h[i]; pl[to] = l[i]; }
+    return;
+  }
+  if (j.perm_H) e = perm(e);
+  *reinterpret_cast<uint2*>(ph + e) = hi;
+  *reinterpret_cast<uint2*>(pl + e) = lo;
+}
 // A unit: kSplitItems items of four values, the lines end to end.  (A pair of planes is added up, hi + lo: the fp32 value that it stands for.)
 constexpr uint32_t kSplitItems = 1024;
 __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jobs jobs) {
@@ -945,10 +961,7 @@ __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jo
     }
     uint2 hi, lo;
     split4_f16(v[k], s, hi, lo);
-    if (j.perm_H) { const uint32_t g = e[k] / j.perm_H, u = e[k] % j.perm_H; e[k] = 128 * (u / 32) + 32 * g + u % 32; }   // (four units stay together)
-    // (the pitch is a multiple of 64: the last item's padding stays inside the line's pitch)
-    *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line[k] + e[k]) = hi;
-    *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line[k] + e[k]) = lo;
+    store_pairs(j, line[k], e[k], hi, lo);
   }
 }
 
@@ -957,7 +970,7 @@ __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jo
 // 10 000 positions (41 MB) 27 / 22, 1024 lines of 4096 11 / 7, of 10 000 24 / 17.  Strips of 32 positions store 64-byte pieces: from memory, not L2, that is the
 // slower form, 512 lines of 50 000 positions 60 / 94.)
 // Positions: a CTA takes strips of 32 positions, 128 bytes of every line; thread -> positions [p, p + 4) of the lines t / 8, t / 8 + 32, ...
-template <int R>
+template <int R, bool ODD = false>   // (ODD: gate rows whose units do not come in fours.  As a branch of the same kernel it cost the others 10 - 20 of 15 - 22 us)
 __global__ void __launch_bounds__(256) k_f16_strip(const __grid_constant__ F16Jobs jobs) {
   dyb_grid_dep_sync();
   __shared__ uint32_t top[8][32];
@@ -995,20 +1008,21 @@ __global__ void __launch_bounds__(256) k_f16_strip(const __grid_constant__ F16Jo
   }
   if (e >= j.n) return;
   uint32_t to = e;
-  if (j.perm_H) { const uint32_t g = e / j.perm_H, u = e % j.perm_H; to = 128 * (u / 32) + 32 * g + u % 32; }   // (four units stay together)
+  if (j.perm_H && !ODD) { const uint32_t g = e / j.perm_H, u = e % j.perm_H; to = 128 * (u / 32) + 32 * g + u % 32; }   // (once, not line by line)
 #pragma unroll
   for (int k = 0; k < R; ++k) {
     const uint32_t line = l0 + 32 * k;
     if (line >= j.lines) break;
     uint2 hi, lo;
     split4_f16(v[k], make_float4(s[0], s[1], s[2], s[3]), hi, lo);
+    if (ODD) { store_pairs(j, line, e, hi, lo); continue; }
     *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line + to) = hi;
     *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line + to) = lo;
   }
 }
 // Lines: a warp per line of up to 1024 values, a CTA per longer one.
-constexpr uint32_t kOneLine = 16384, kOneStrip = 1024;   // longest line, most lines of a strip
-template <uint32_t R>
+constexpr uint32_t kOneLine = kF16PadMax, kOneStrip = 1024;   // longest line, most lines of a strip
+template <uint32_t R, bool PAD>
 __device__ __forceinline__ void line_pairs(const F16Job& j, uint32_t line, uint32_t e0, uint32_t step, uint32_t* red) {
   const float* p = j.src + (size_t)j.ld * line;
   const bool vec = aligned16(p);
@@ -1038,21 +1052,37 @@ __device__ __forceinline__ void line_pairs(const F16Job& j, uint32_t line, uint3
     if (e >= j.n) break;
     uint2 hi, lo;
     split4_f16(v[k], make_float4(s, s, s, s), hi, lo);
-    *reinterpret_cast<uint2*>(j.hi + (size_t)j.pitch * line + e) = hi;
-    *reinterpret_cast<uint2*>(j.lo + (size_t)j.pitch * line + e) = lo;
+    __half *ph = j.hi + (size_t)j.pitch * line, *pl = j.lo + (size_t)j.pitch * line;
+    if (PAD && j.pad_H) {
+      const __half *h = reinterpret_cast<const __half*>(&hi), *l = reinterpret_cast<const __half*>(&lo);
+      const uint32_t gap = (j.pad_H + 63) / 64 * 64 - j.pad_H;
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i)
+        if (e + i < j.n) { const uint32_t to = e + i + (e + i) / j.pad_H * gap; ph[to] = h[i]; pl[to] = l[i]; }
+    } else {
+      *reinterpret_cast<uint2*>(ph + e) = hi;
+      *reinterpret_cast<uint2*>(pl + e) = lo;
+    }
+  }
+  if (PAD && j.pad_H) {   // (the product meets zeros of the other operand here: any finite value would do)
+    const uint32_t Hp = (j.pad_H + 63) / 64 * 64, gap = Hp - j.pad_H;
+    for (uint32_t x = e0 / 4; x < 4 * gap; x += step / 4) {
+      const size_t to = (size_t)j.pitch * line + x / gap * Hp + j.pad_H + x % gap;
+      j.hi[to] = j.lo[to] = __float2half_rn(0.f);
+    }
   }
 }
-template <uint32_t R>   // (16: lines of more than 8192)
+template <uint32_t R, bool PAD>   // (R 16: lines of more than 8192; PAD: jobs with pad_H)
 __global__ void __launch_bounds__(256) k_f16_line(const __grid_constant__ F16Jobs jobs) {
   dyb_grid_dep_sync();
   __shared__ uint32_t red[8];
   const uint32_t z = f16_job_of(jobs), unit = blockIdx.x - jobs.start[z];
   const F16Job& j = jobs.job[z];
   if (j.n > 1024) {
-    line_pairs<R>(j, unit, 4 * threadIdx.x, 1024, red);
+    line_pairs<R, PAD>(j, unit, 4 * threadIdx.x, 1024, red);
   } else {
     const uint32_t line = 8 * unit + (threadIdx.x >> 5);
-    if (line < j.lines) line_pairs<8>(j, line, 4 * (threadIdx.x & 31), 128, nullptr);
+    if (line < j.lines) line_pairs<8, PAD>(j, line, 4 * (threadIdx.x & 31), 128, nullptr);
   }
 }
 constexpr uint64_t kOneValues = 12u << 20;   // (48 MB and as much again of pairs: L2 still holds most of both)
@@ -1179,7 +1209,7 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     else if (victim->hi && e->last_use < victim->last_use) victim = e;
   }
   dyb200_ctx::ParamPack* e = hit ? hit : victim;
-  const size_t floats = k_is_fast == kLayoutGatesF16 ? (size_t)(K + rows2) * pitch / 2 + 2 * rows : k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE ? rows : K) : (size_t)(rows + rows2) * pitch;
+  const size_t floats = k_is_fast == kLayoutGatesF16 ? (size_t)(K + rows2) * pitch / 2 + 2 * rows : k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE || k_is_fast == kLayoutPadF16 ? rows : K) : (size_t)(rows + rows2) * pitch;
   if (!hit) {
     if (e->hi && e->floats < floats) {   // evicted entry is too small: its buffers may still be read by queued kernels
       DYB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1205,7 +1235,9 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
   } else if (e->version != ctx->param_version && k_is_fast >= kLayoutF16) {
     F16Jobs jobs;
     jobs.n = 1;
-    jobs.job[0] = F16Job{src, ld, rows, K, pitch, k_is_fast - kLayoutF16, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
+    const bool pad = k_is_fast == kLayoutPadF16;
+    jobs.job[0] = F16Job{src, ld, rows, K, pitch, pad ? (int)F16_LINE : k_is_fast - kLayoutF16, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
+    if (pad) jobs.job[0].pad_H = K / 4;
     int rc = dyb200_f16_pack(ctx, &jobs);
     if (rc) return rc;
     e->version = ctx->param_version;
@@ -1226,13 +1258,14 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
 }  // namespace
 
 // ---- fp16 operand planes ----
-int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job) {
-  const uint32_t pitch = round_up(n, 64);
+int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H) {
+  const uint32_t pitch = pad_H ? 4 * round_up(pad_H, 64) : round_up(n, 64);
   const size_t plane = (size_t)lines * pitch * sizeof(__half), words = mode == F16_LINE ? lines : mode == F16_ELEM ? n : 1;
   void *h, *l, *sc;
   int rc;
   if ((rc = dyb200_scratch(ctx, plane, &h)) || (rc = dyb200_scratch(ctx, plane, &l)) || (rc = dyb200_scratch(ctx, words * sizeof(uint32_t), &sc))) return rc;
   *job = F16Job{src, ld, lines, n, pitch, mode, (uint32_t*)sc, (__half*)h, (__half*)l};
+  job->pad_H = pad_H;
   return DYB200_OK;
 }
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
@@ -1247,19 +1280,24 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
     F16Jobs part;
     part.n = 0; part.start[0] = 0;
     uint32_t lines = 0, longest = 0;
+    bool odd = false, pad = false;
     for (int k = 0; k < jobs->n; ++k) {
       const F16Job& j = jobs->job[k];
       if (j.mode != mode) continue;
       if (!f16_one_pass(j)) { rest.job[rest.n++] = j; continue; }
       if (j.lines > lines) lines = j.lines;
       if (j.n > longest) longest = j.n;
+      odd = odd || j.perm_H % 4 != 0; pad = pad || j.pad_H;
       part.job[part.n] = j;
       part.start[part.n + 1] = part.start[part.n] + (mode == F16_ELEM ? (j.n + 31) / 32 : j.n > 1024 ? j.lines : (j.lines + 7) / 8);
       ++part.n;
     }
     if (part.n == 0 || part.start[part.n] == 0) continue;
-    dyb_launch(mode == F16_LINE ? (longest <= 8192 ? k_f16_line<8> : k_f16_line<16>) : lines <= 256 ? k_f16_strip<8> : lines <= 512 ? k_f16_strip<16> : k_f16_strip<32>,
-               part.start[part.n], 256, 0, ctx, part);
+    void (*k)(F16Jobs);
+    if (mode == F16_LINE) k = longest <= 8192 ? (pad ? k_f16_line<8, true> : k_f16_line<8, false>) : pad ? k_f16_line<16, true> : k_f16_line<16, false>;
+    else if (odd) k = lines <= 512 ? k_f16_strip<16, true> : k_f16_strip<32, true>;
+    else k = lines <= 256 ? k_f16_strip<8> : lines <= 512 ? k_f16_strip<16> : k_f16_strip<32>;
+    dyb_launch(k, part.start[part.n], 256, 0, ctx, part);
     DYB_LAUNCHED(ctx);
   }
   jobs = &rest;
@@ -1284,18 +1322,18 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
-int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job) {
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H) {
   if (!ctx->param_cache_on) {
     F16Jobs jobs;
     jobs.n = 1;
-    int rc = dyb200_f16_planes(ctx, src, ld, lines, n, mode, &jobs.job[0]);
+    int rc = dyb200_f16_planes(ctx, src, ld, lines, n, mode, &jobs.job[0], pad_H);
     if (!rc) rc = dyb200_f16_pack(ctx, &jobs);
     *job = jobs.job[0];
     return rc;
   }
-  const uint32_t pitch = round_up(n, 64);
+  const uint32_t pitch = pad_H ? 4 * round_up(pad_H, 64) : round_up(n, 64);
   float *hi, *lo;
-  int rc = cached_param_pack(ctx, src, ld, kLayoutF16 + mode, lines, n, pitch, &hi, &lo);
+  int rc = cached_param_pack(ctx, src, ld, pad_H ? kLayoutPadF16 : kLayoutF16 + mode, lines, n, pitch, &hi, &lo);
   if (rc) return rc;
   *job = F16Job{src, ld, lines, n, pitch, mode, reinterpret_cast<uint32_t*>(hi + (size_t)lines * pitch / 2), (__half*)hi, (__half*)lo};
   return DYB200_OK;

@@ -13,7 +13,8 @@
 // reduction is ordered by these blocks (4 gates x 128 units = 8 k-blocks of 64), each one accumulation chain that is unscaled as it is drained.
 //
 // Measured (us per step of 35, all of a layer's backward call, I = H = 1024; TF32 pairs with dx inside the recurrence / this form): batch 512 48.2 / 30.5,
-// 256 35.8 / 17.9, 128 21.8 / 15.2, 64 16.6 / 9.9; batch 100 (a launch and more per step before) 31 / 14; 600 units, batch 30: 21 / 8.  dx is 10 of
+// 256 35.8 / 17.9, 128 21.8 / 15.2, 64 16.6 / 9.9; batch 100 (a launch and more per step before) 31 / 14; 600 units, batch 30: 21 / 8; 777 units, batch 100
+// (a value at a time, the weights' gates moved apart so that a k-block's copy starts on 16 bytes): 37 / 10.5.  dx is 10 of
 // the 30.5, at 430 TFLOP/s useful.  What bounds the recurrence: at batch 512, two column blocks per CTA in turn (one block of 128 columns had nothing
 // to overlap its exchange and cell pass with: 25 us a step against 20), 196 MB of operands per step from L2 at 11 - 14 TB/s; at batch 64 the chain
 // itself: 0.5 until the first pairs of dgates are there, 2.8 for 8 k-blocks, 0.5 to drain the last, 1.2 exchange, 1.0 cell pass, 0.8 until the stores are
@@ -24,7 +25,7 @@
 namespace {
 
 struct BwdWide {
-  uint32_t T, B, H, Hp;             // steps, columns per step, units (rows of the product; dx: I), units rounded up to 64
+  uint32_t T, B, H, Hp, Ha;         // steps, columns per step, units, units rounded up to 64, distance of the gates in a row of the weights' pairs
   uint32_t kbs;                     // k-blocks of the product
   uint32_t P;                       // products of a column block: T - 1, and one more when dh_prev is given; dx: tiles
   uint32_t ncb, tiles_n;            // column blocks that a CTA serves in turn, of how many (dx: 1)
@@ -45,12 +46,12 @@ struct BwdWide {
 
 // k-block i of the reduction: block of 128 units (i / 8), gate, half.  The last block has 64 units or fewer when H % 128 is in 1 .. 64.
 struct KBlock { int xa, xb; };
-__device__ __forceinline__ KBlock k_block(uint32_t i, uint32_t H, uint32_t Hp) {
+__device__ __forceinline__ KBlock k_block(uint32_t i, uint32_t H, uint32_t Ha, uint32_t Hp) {
   const uint32_t full = H / BM, blk = i >> 3;
   uint32_t q = (i >> 1) & 3, h = i & 1;
   if (blk >= full && H % BM <= 64) { q = i - 8 * full; h = 0; }
   const uint32_t u = BM * min(blk, full) + 64 * h;
-  return KBlock{(int)(q * H + u), (int)(q * Hp + u)};
+  return KBlock{(int)(q * Ha + u), (int)(q * Hp + u)};
 }
 
 constexpr int kMaxBlocks = 4;   // column blocks per CTA
@@ -58,7 +59,8 @@ constexpr int kMaxBlocks = 4;   // column blocks per CTA
 struct CellIn { float4 gi, gf, go, gg, c, cp, dci, dcp; };
 
 // REC: the recurrence, grid = (tiles_m, column blocks, S).  Otherwise dx: grid = (clusters, 1, S), the clusters walk the tiles.
-template <int BNT, uint32_t S, bool REC>
+// VEC: units in fours, on 16 bytes (dx has a rule of its own for its rows).
+template <int BNT, uint32_t S, bool REC, bool VEC>
 __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant__ TmapPack tm, const __grid_constant__ BwdWide a) {
   constexpr int kStages = BNT == 64 ? 4 : 3;
   constexpr int TILE_B_BYTES = BNT * BK * 4, kStageBytes = 2 * TILE_BYTES + 2 * TILE_B_BYTES;
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             }
             if (na < pre && mbar_test(&empty_bar[sa], pa ^ 1)) {
               unsigned char* st = ring + (size_t)sa * kStageBytes;
-              const KBlock kb = k_block(k0 + na, a.H, a.Hp);
+              const KBlock kb = k_block(k0 + na, a.H, a.Ha, a.Hp);
               mbar_expect_tx(&full_bar[sa], kStageBytes);
               tma_load_2d(st, &tm.t[0], &full_bar[sa], kb.xa, m0);
               tma_load_2d(st + TILE_BYTES, &tm.t[1], &full_bar[sa], kb.xa, m0);
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             }
             if (ready && i < na) {
               unsigned char* st = ring + (size_t)s * kStageBytes;
-              const KBlock kb = k_block(k0 + i, a.H, a.Hp);
+              const KBlock kb = k_block(k0 + i, a.H, a.Ha, a.Hp);
               tma_load_2d(st + 2 * TILE_BYTES, &tm.t[2], &full_bar[s], kb.xb, col0);
               tma_load_2d(st + 2 * TILE_BYTES + TILE_B_BYTES, &tm.t[3], &full_bar[s], kb.xb, col0);
               if (++s == kStages) { s = 0; ph ^= 1; }
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
         for (; i < total; ++i) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1)) { fail = true; break; }
           unsigned char* st = ring + (size_t)s * kStageBytes;
-          const KBlock kb = k_block(k0 + i, a.H, a.Hp);
+          const KBlock kb = k_block(k0 + i, a.H, a.Ha, a.Hp);
           mbar_expect_tx(&full_bar[s], kStageBytes);
           tma_load_2d(st, &tm.t[0], &full_bar[s], kb.xa, m0);
           tma_load_2d(st + TILE_BYTES, &tm.t[1], &full_bar[s], kb.xa, m0);
@@ -208,18 +210,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
     const size_t HB = (size_t)a.H * a.B;
     const uint32_t u = blockIdx.x * BM + uq;                            // REC: units [u, u + 4)
     const bool own_u = u < a.H;
+    const uint32_t left = a.H - u;                                      // (own_u) units from u on
     float4 rs[4];   // REC: row sums of dgates over this thread's columns of a step
 
     auto column = [&](int hh, uint32_t k) { const uint32_t p = rank * w + ew + 8 * k; return (p >> 5) * kHalf + 32 * hh + (p & 31); };
     auto cell_load = [&](CellIn& in, uint32_t t, uint32_t n) {
       const size_t e = (size_t)n * a.H + u;
       const float* g = a.gates + (size_t)t * 4 * HB + (size_t)n * 4 * a.H + u;
-      in.gi = ld4(g); in.gf = ld4(g + a.H); in.go = ld4(g + 2 * a.H); in.gg = ld4(g + 3 * a.H);
-      in.c = ld4(a.cs + (size_t)t * HB + e);
-      in.cp = ld4((t ? a.cs + (size_t)(t - 1) * HB : a.c0) + e);
+      in.gi = ldu<VEC>(g, left); in.gf = ldu<VEC>(g + a.H, left); in.go = ldu<VEC>(g + 2 * a.H, left); in.gg = ldu<VEC>(g + 3 * a.H, left);
+      in.c = ldu<VEC>(a.cs + (size_t)t * HB + e, left);
+      in.cp = ldu<VEC>((t ? a.cs + (size_t)(t - 1) * HB : a.c0) + e, left);
       const float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
-      in.dci = a.dc ? __ldcg(reinterpret_cast<const float4*>(a.dc + (size_t)t * HB + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      in.dcp = dcp ? __ldcg(reinterpret_cast<const float4*>(dcp + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      in.dci = a.dc ? ldu_cg<VEC>(a.dc + (size_t)t * HB + e, left) : make_float4(0.f, 0.f, 0.f, 0.f);
+      in.dcp = dcp ? ldu_cg<VEC>(dcp + e, left) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     // The cell pass of units [u, + 4), column n of step t from dE/dh: dE/dc of the step before, and dgates as fp16 pairs with the word of the warp's
     // (column, block).  The four gates' gradients come back in p.  (All lanes of a warp take part; those past the last unit with zeros.)
@@ -258,13 +261,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
     auto cell_rest = [&](const CellIn& in, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dE/dc of the step before, dgates for the weight gradients
       if (!own_u) return;
       float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
-      if (dcp) st4(dcp + (size_t)n * a.H + u, in.dcp);
+      if (dcp) stu<VEC>(dcp + (size_t)n * a.H + u, in.dcp, left);
       const size_t o = ((size_t)t * a.B + n) * a.dn_pitch + u;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float4 hi, lo;
         split_tf32(p[q].x, hi.x, lo.x); split_tf32(p[q].y, hi.y, lo.y); split_tf32(p[q].z, hi.z, lo.z); split_tf32(p[q].w, hi.w, lo.w);
-        st4(a.dn_hi + o + (size_t)q * a.H, hi); st4(a.dn_lo + o + (size_t)q * a.H, lo);
+        stu<VEC>(a.dn_hi + o + (size_t)q * a.H, hi, left); stu<VEC>(a.dn_lo + o + (size_t)q * a.H, lo, left);
       }
     };
     auto publish = [&](uint32_t cb) {   // (behind a barrier: one thread's release orders all the stores it has observed, for both proxies)
@@ -307,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
           if (n >= a.B) continue;
           CellIn in = {};
           float4 dh = make_float4(0.f, 0.f, 0.f, 0.f), p[4];
-          if (own_u) { cell_load(in, t, n); dh = ld4(a.dh + (size_t)t * HB + (size_t)n * a.H + u); }
+          if (own_u) { cell_load(in, t, n); dh = ldu<VEC>(a.dh + (size_t)t * HB + (size_t)n * a.H + u, left); }
           cell(in, dh, t, n, p);
           cell_rest(in, p, t, n);
         }
@@ -416,8 +419,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             mk[g] = make_float4(1.f, 1.f, 1.f, 1.f);
             old[g] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (!own || n[g] >= cols || !vec) continue;
-            old[g] = __ldcg(reinterpret_cast<const float4*>(dst + (size_t)n[g] * a.M + m));
-            if (a.mask) mk[g] = ld4(a.mask + m + (a.mask_full ? (size_t)(REC ? n[g] : n[g] % a.B) * a.M : 0));
+            old[g] = REC ? ldu_cg<VEC>(dst + (size_t)n[g] * a.M + m, left) : __ldcg(reinterpret_cast<const float4*>(dst + (size_t)n[g] * a.M + m));
+            if (a.mask) {
+              const float* mp = a.mask + m + (a.mask_full ? (size_t)(REC ? n[g] : n[g] % a.B) * a.M : 0);
+              mk[g] = REC ? ldu<VEC>(mp, left) : ld4(mp);
+            }
             if (REC && t) cell_load(in[g], t - 1, n[g]);
           }
           if (kb == 0) {
@@ -454,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
 #pragma unroll
           for (uint32_t g = 0; g < GB; ++g) {
             if (n[g] >= cols) continue;
-            if (own && vec) st4(dst + (size_t)n[g] * a.M + m, old[g]);
+            if (own && vec) { if (REC) stu<VEC>(dst + (size_t)n[g] * a.M + m, old[g], left); else st4(dst + (size_t)n[g] * a.M + m, old[g]); }
             if (REC && t) cell_rest(in[g], p[g], t - 1, n[g]);
           }
         }
@@ -477,9 +483,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
 // ---- host side ---------------------------------------------------------------------------------------------------------
 enum WideOp { WIDE_FIT, WIDE_LAUNCH };
 
-template <int BNT, uint32_t S, bool REC>
+template <int BNT, uint32_t S, bool REC, bool VEC = true>
 int wide_do(WideOp op, dyb200_ctx* ctx, int slot, const TmapPack* tm, const BwdWide* a, dim3 grid, double flops) {
-  const auto kernel = k_bwd_wide<BNT, S, REC>;
+  const auto kernel = k_bwd_wide<BNT, S, REC, VEC>;
   int16_t& fit = ctx->bwd_wide_fit[slot];
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -519,11 +525,16 @@ int wide_do(WideOp op, dyb200_ctx* ctx, int slot, const TmapPack* tm, const BwdW
   return DYB200_OK;
 }
 constexpr uint32_t kRecCols = 64;
-int wide_rec(WideOp op, uint32_t S, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const BwdWide* a = nullptr, dim3 grid = dim3(), double flops = 0) {
-  if (S == 8) return wide_do<kRecCols, 8, true>(op, ctx, 0, tm, a, grid, flops);
-  if (S == 4) return wide_do<kRecCols, 4, true>(op, ctx, 1, tm, a, grid, flops);
-  if (S == 2) return wide_do<kRecCols, 2, true>(op, ctx, 2, tm, a, grid, flops);
-  return wide_do<kRecCols, 1, true>(op, ctx, 3, tm, a, grid, flops);
+template <bool VEC>
+int wide_rec_of(WideOp op, uint32_t S, dyb200_ctx* ctx, const TmapPack* tm, const BwdWide* a, dim3 grid, double flops) {
+  constexpr int slot = VEC ? 0 : 7;
+  if (S == 8) return wide_do<kRecCols, 8, true, VEC>(op, ctx, slot, tm, a, grid, flops);
+  if (S == 4) return wide_do<kRecCols, 4, true, VEC>(op, ctx, slot + 1, tm, a, grid, flops);
+  if (S == 2) return wide_do<kRecCols, 2, true, VEC>(op, ctx, slot + 2, tm, a, grid, flops);
+  return wide_do<kRecCols, 1, true, VEC>(op, ctx, slot + 3, tm, a, grid, flops);
+}
+int wide_rec(WideOp op, uint32_t H, uint32_t S, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const BwdWide* a = nullptr, dim3 grid = dim3(), double flops = 0) {
+  return H % 4 == 0 ? wide_rec_of<true>(op, S, ctx, tm, a, grid, flops) : wide_rec_of<false>(op, S, ctx, tm, a, grid, flops);
 }
 enum DxForm { DX_128, DX_64, DX_SPLIT };   // tiles of 128 or 64 columns, a CTA each; tiles of 64 columns, a CTA of eight for each block of 128 units
 int wide_dx(WideOp op, DxForm f, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const BwdWide* a = nullptr, dim3 grid = dim3(), double flops = 0) {
@@ -538,7 +549,7 @@ uint32_t k_blocks(uint32_t H) { return 8 * (H / BM) + (H % BM == 0 ? 0 : H % BM 
 // Column blocks per CTA and K splits: the fastest by what a product was measured to take - 0.36 us per k-block on the tensor pipe and 6 us from its last
 // MMA to the next step's first, which another block's MMAs overlap.
 bool dyb200_bwd_wide_plan(dyb200_ctx* ctx, uint32_t H, uint32_t B, uint32_t* ncb, uint32_t* S) {
-  if (H <= 384 || H % 8 != 0 || B <= 8) return false;
+  if (H <= 384 || B <= 8 || (H % 8 != 0 && 4 * H > kF16PadMax)) return false;
   const uint32_t tiles_m = (H + BM - 1) / BM, tiles_n = (B + kRecCols - 1) / kRecCols, kbs = k_blocks(H);
   if (tiles_n > DYB200_DEV_BWD_WORDS) return false;   // (a hand-over counter per column block)
   struct { double t; uint32_t n, s; } c[12];
@@ -553,7 +564,7 @@ bool dyb200_bwd_wide_plan(dyb200_ctx* ctx, uint32_t H, uint32_t B, uint32_t* ncb
   while (nc > 0) {   // (the best one first: asking how many clusters fit loads the kernel, a few ms each)
     int k = 0;
     for (int q = 1; q < nc; ++q) if (c[q].t < c[k].t) k = q;
-    const int fit = wide_rec(WIDE_FIT, c[k].s, ctx);
+    const int fit = wide_rec(WIDE_FIT, H, c[k].s, ctx);
     if (fit > 0 && tiles_m * ((tiles_n + c[k].n - 1) / c[k].n) <= (uint32_t)fit) { *ncb = c[k].n; *S = c[k].s; return true; }
     c[k] = c[--nc];
   }
@@ -571,11 +582,13 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
   const size_t plane = (size_t)columns * 4 * Hp;
   if ((rc = dyb200_scratch(ctx, 2 * plane * sizeof(__half), &p16)) || (rc = dyb200_scratch(ctx, (size_t)tiles_m * columns * sizeof(uint32_t), &words)) ||
       (rc = dyb200_scratch(ctx, (size_t)T * tiles_n * S * G * sizeof(float), &part))) return rc;
-  if ((rc = dyb200_f16_param(ctx, q.Wh, G, H, G, F16_LINE, &wh))) return rc;
-  if (q.dx && (rc = dyb200_f16_param(ctx, q.Wx, G, I, G, F16_LINE, &wx))) return rc;
+  // (a k-block's copy starts at a gate's units: on 16 bytes as the weights lie, or with the gates moved apart)
+  const uint32_t pad = H % 8 == 0 ? 0 : H, K = pad ? 4 * Hp : G;
+  if ((rc = dyb200_f16_param(ctx, q.Wh, G, H, G, F16_LINE, &wh, pad))) return rc;
+  if (q.dx && (rc = dyb200_f16_param(ctx, q.Wx, G, I, G, F16_LINE, &wx, pad))) return rc;
   BwdWide a;
   memset(&a, 0, sizeof(a));
-  a.T = T; a.B = B; a.H = H; a.Hp = Hp; a.kbs = k_blocks(H); a.P = T - 1 + (q.dh_prev ? 1 : 0); a.M = H; a.tiles_m = tiles_m;
+  a.T = T; a.B = B; a.H = H; a.Hp = Hp; a.Ha = pad ? Hp : H; a.kbs = k_blocks(H); a.P = T - 1 + (q.dh_prev ? 1 : 0); a.M = H; a.tiles_m = tiles_m;
   a.ncb = ncb; a.tiles_n = tiles_n;
   a.gates = q.gates; a.cs = q.c; a.c0 = q.c0; a.dh = q.dh; a.dc = q.dc; a.dh_prev = q.dh_prev; a.dc_prev = q.dc_prev;
   a.dn_hi = q.dn_hi; a.dn_lo = q.dn_lo; a.dn_pitch = q.dn_pitch;
@@ -585,10 +598,10 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
   a.done = ctx->dev_flags + DYB200_DEV_BWD0; a.flags = ctx->dev_flags;
   TmapPack tm;
   memset(&tm, 0, sizeof(tm));
-  if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[0], wh.hi, H, G, wh.pitch, BM, false)) || (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[1], wh.lo, H, G, wh.pitch, BM, false)) ||
+  if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[0], wh.hi, H, K, wh.pitch, BM, false)) || (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[1], wh.lo, H, K, wh.pitch, BM, false)) ||
       (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[2], a.d16_hi, columns, 4 * Hp, 4 * Hp, kRecCols, false)) ||
       (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[3], a.d16_lo, columns, 4 * Hp, 4 * Hp, kRecCols, false))) return rc;
-  if ((rc = wide_rec(WIDE_LAUNCH, S, ctx, &tm, &a, dim3(tiles_m, (tiles_n + ncb - 1) / ncb, S), 2.0 * G * (double)H * B * a.P))) return rc;
+  if ((rc = wide_rec(WIDE_LAUNCH, H, S, ctx, &tm, &a, dim3(tiles_m, (tiles_n + ncb - 1) / ncb, S), 2.0 * G * (double)H * B * a.P))) return rc;
   if ((rc = dyb200_seq_db(ctx, a.part, T, tiles_n * S, G, q.db, a.done)) || !q.dx) return rc;
   // dx of all columns
   a.M = I; a.tiles_m = (I + BM - 1) / BM; a.columns = columns; a.dx = q.dx; a.mask = q.mx; a.mask_full = q.mx_full; a.wscale = wx.scale;
@@ -608,7 +621,7 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
   if (fit <= 0) return dyb200_fail(ctx, DYB200_ECUDA, "lstm_seq_bwd: no launch of the dx product fits");
   const uint32_t dn = form == DX_128 ? 128 : 64;
   a.P = a.tiles_m * ((columns + dn - 1) / dn);
-  if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[0], wx.hi, I, G, wx.pitch, BM, false)) || (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[1], wx.lo, I, G, wx.pitch, BM, false)) ||
+  if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[0], wx.hi, I, K, wx.pitch, BM, false)) || (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[1], wx.lo, I, K, wx.pitch, BM, false)) ||
       (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[2], a.d16_hi, columns, 4 * Hp, 4 * Hp, dn, false)) ||
       (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[3], a.d16_lo, columns, 4 * Hp, 4 * Hp, dn, false))) return rc;
   return wide_dx(WIDE_LAUNCH, form, ctx, &tm, &a, dim3(a.P < (uint32_t)fit ? a.P : (uint32_t)fit, 1, form == DX_SPLIT ? 8 : 1), 2.0 * G * (double)I * columns);

@@ -52,7 +52,8 @@ __device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return
 // the mask's largest value keep an absolute error of 2^-51 of it.)
 // grid = (4H / 128, B / BNT, S); with S > 1 the S CTAs of a tile are one thread-block cluster (1 x 1 x S).  S (1, 2, 4 or 8) is
 // a template parameter so that the column exchange indexes registers statically.
-template <int BNT, uint32_t S, bool F16>
+// VEC: units in fours, on 16 bytes (otherwise, F16 and 64-column tiles only, a value at a time).
+template <int BNT, uint32_t S, bool F16, bool VEC = true>
 __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_constant__ TmapPack tm, const SeqFwd a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // 64-column tiles need 48 KiB per stage, so the ring holds four of them: at 0.4 us per k-block three stages do not cover
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
     // positions te / 8 and te / 8 + 32.
     const uint32_t l = 4 * (te & 7), u = blockIdx.x * 32 + l;
     const bool own_u = u < a.H;
+    const uint32_t left = a.H - u;   // (own_u) units from u on
     auto column = [&](int hh, uint32_t p) { return (p >> 5) * kHalf + 32 * hh + (p & 31); };
     // F16: 2^-s of this thread's gate row in Wx and in Wh; of the columns lane (and lane + 32) of its half (h after the first step); and 2^s of the columns it finishes
     float row_x = 1.f, row_h = 1.f, h_f[kHalf / 32], h_s[BNT / 64][2];
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
     float4 bias[4];   // the same for every step
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      bias[q] = own_u ? ld4(a.bias + (size_t)q * a.H + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+      bias[q] = own_u ? ldu<VEC>(a.bias + (size_t)q * a.H + u, left) : make_float4(0.f, 0.f, 0.f, 0.f);
       if (q == 1) { bias[q].x += a.forget_bias; bias[q].y += a.forget_bias; bias[q].z += a.forget_bias; bias[q].w += a.forget_bias; }
     }
     uint32_t cg = 0, pf_phase = 0, pr_phase = 0;
@@ -246,8 +248,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
         for (int k = 0; k < 2; ++k) {
           const uint32_t c = (te >> 3) + 32 * k, n = n0 + column(hh, c);
           const bool mine = own_u && n < N && c >= c_lo && c < c_hi;
-          cp[hh][k] = mine ? ld4(c_prev + u + (size_t)a.H * n) : make_float4(0.f, 0.f, 0.f, 0.f);
-          hm[hh][k] = (mine && a.hmask) ? ld4(a.hmask + u + (a.hmask_full ? (size_t)a.hmask_ld * n : 0)) : make_float4(1.f, 1.f, 1.f, 1.f);
+          cp[hh][k] = mine ? ldu<VEC>(c_prev + u + (size_t)a.H * n, left) : make_float4(0.f, 0.f, 0.f, 0.f);
+          hm[hh][k] = (mine && a.hmask) ? ldu<VEC>(a.hmask + u + (a.hmask_full ? (size_t)a.hmask_ld * n : 0), left) : make_float4(1.f, 1.f, 1.f, 1.f);
         }
       float f[kHalf / 32], row_f = row_x;   // F16: 2^-s of the columns lane (and lane + 32) in the coming chains, and of the row
 #pragma unroll
@@ -337,6 +339,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
           cn[k] = make_float4(lstm_cell_c(g[k][0].x, g[k][3].x, g[k][1].x, cv.x), lstm_cell_c(g[k][0].y, g[k][3].y, g[k][1].y, cv.y),
                               lstm_cell_c(g[k][0].z, g[k][3].z, g[k][1].z, cv.z), lstm_cell_c(g[k][0].w, g[k][3].w, g[k][1].w, cv.w));
           hv[k] = make_float4(lstm_cell_h(g[k][2].x, cn[k].x), lstm_cell_h(g[k][2].y, cn[k].y), lstm_cell_h(g[k][2].z, cn[k].z), lstm_cell_h(g[k][2].w, cn[k].w));
+          if (!VEC) { if (left < 2) hv[k].y = 0.f; if (left < 3) hv[k].z = 0.f; if (left < 4) hv[k].w = 0.f; }   // (the planes' padding stays zero)
           if (emit) {
             // h .* mask_h as the next step's operand planes (the values of epi_emit_h)
             const float4 mk = hm[hh][k];
@@ -374,10 +377,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
           if (!live[k]) continue;
           const uint32_t n = n0 + column(hh, (te >> 3) + 32 * k);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) st4(gates_t + (size_t)q * a.H + u + (size_t)M * n, g[k][q]);
+          for (int q = 0; q < 4; ++q) stu<VEC>(gates_t + (size_t)q * a.H + u + (size_t)M * n, g[k][q], left);
           const size_t ei = u + (size_t)a.H * n;
-          st4(c_out + ei, cn[k]);
-          st4(h_out + ei, hv[k]);
+          stu<VEC>(c_out + ei, cn[k], left);
+          stu<VEC>(h_out + ei, hv[k], left);
         }
       }
     }
@@ -398,9 +401,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_const
 namespace {
 
 // How many clusters of S CTAs of the sequence kernel fit on the GPU at once (remembered per context = per device).
-template <int BNT, uint32_t S, bool F16>
+template <int BNT, uint32_t S, bool F16, bool VEC>
 int seq_clusters_that_fit(dyb200_ctx* ctx) {
-  int& mc = ctx->seq_max_clusters[(BNT == 64 ? 0 : 1) + (F16 ? 2 : 0)][S];
+  int& mc = ctx->seq_max_clusters[(BNT == 64 ? 0 : 1) + (F16 ? VEC ? 2 : 4 : 0)][S];
   if (mc == 0) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -410,13 +413,13 @@ int seq_clusters_that_fit(dyb200_ctx* ctx) {
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = S;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_lstm_seq_fwd<BNT, S, F16>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
+    if (cudaOccupancyMaxActiveClusters(&n, k_lstm_seq_fwd<BNT, S, F16, VEC>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = -1; }
     mc = n > 0 ? n : -1;
   }
   return mc;
 }
 
-template <int BNT, uint32_t S, bool F16>
+template <int BNT, uint32_t S, bool F16, bool VEC>
 int launch_seq_fwd(dyb200_ctx* ctx, const TmapPack& tm, const SeqFwd& a, dim3 grid, double flops, uint32_t K) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -436,7 +439,7 @@ int launch_seq_fwd(dyb200_ctx* ctx, const TmapPack& tm, const SeqFwd& a, dim3 gr
     attr[na].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = na + 1;
     GemmProfScope scope(ctx, flops, F16 ? 2 : 1, 4 * a.H, a.B * a.T, K, EPI_LSTM_CELL);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S, F16>, tm, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S, F16, VEC>, tm, a);
     if (e == cudaSuccess) { ctx->seq_coop = 1; ctx->launches++; return DYB200_OK; }
     (void)cudaGetLastError();
     if (ctx->seq_coop == 1) return dyb200_fail(ctx, DYB200_ECUDA, "sequence kernel launch failed: %s", cudaGetErrorString(e));
@@ -449,44 +452,51 @@ int launch_seq_fwd(dyb200_ctx* ctx, const TmapPack& tm, const SeqFwd& a, dim3 gr
   }
   cfg.attrs = attr; cfg.numAttrs = na;
   GemmProfScope scope(ctx, flops, F16 ? 2 : 1, 4 * a.H, a.B * a.T, K, EPI_LSTM_CELL);
-  cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S, F16>, tm, a);
+  cudaLaunchKernelEx(&cfg, k_lstm_seq_fwd<BNT, S, F16, VEC>, tm, a);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
 
 // the (tile width, K splits) instantiations behind one switch
 enum SeqOp { SEQ_SET_SMEM, SEQ_FIT, SEQ_LAUNCH };
-template <int BNT, uint32_t S, bool F16>
+template <int BNT, uint32_t S, bool F16, bool VEC>
 int seq_fwd_do(SeqOp op, dyb200_ctx* ctx, const TmapPack* tm, const SeqFwd* a, dim3 grid, double flops, uint32_t K) {
   if (op == SEQ_SET_SMEM) {
     // (the shared-memory limit of the kernel has to be raised before its occupancy is asked for)
     const uint32_t log_s = S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : 3, bit = (F16 ? (BNT == 64 ? 1u << 12 : 1u << 16) : BNT == 64 ? 16u : 256u) << log_s;
-    if (!(ctx->func_attr_done & bit)) {
-      DYB_CUDA(ctx, cudaFuncSetAttribute(k_lstm_seq_fwd<BNT, S, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SEQ_BYTES));
-      ctx->func_attr_done |= bit;
+    uint32_t& done = VEC ? ctx->func_attr_done : ctx->seq_odd_attr_done;
+    if (!(done & bit)) {
+      DYB_CUDA(ctx, cudaFuncSetAttribute(k_lstm_seq_fwd<BNT, S, F16, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SEQ_BYTES));
+      done |= bit;
     }
     return DYB200_OK;
   }
-  if (op == SEQ_FIT) return seq_clusters_that_fit<BNT, S, F16>(ctx);
-  return launch_seq_fwd<BNT, S, F16>(ctx, *tm, *a, grid, flops, K);
+  if (op == SEQ_FIT) return seq_clusters_that_fit<BNT, S, F16, VEC>(ctx);
+  return launch_seq_fwd<BNT, S, F16, VEC>(ctx, *tm, *a, grid, flops, K);
 }
-template <bool F16>
+template <bool F16, bool VEC = true>
 int seq_fwd_dispatch(SeqOp op, uint32_t bn, uint32_t S, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const SeqFwd* a = nullptr,
                      dim3 grid = dim3(), double flops = 0, uint32_t K = 0) {
   if (bn == 64) {
     switch (S) {
-      case 1: return seq_fwd_do<64, 1, F16>(op, ctx, tm, a, grid, flops, K);
-      case 2: return seq_fwd_do<64, 2, F16>(op, ctx, tm, a, grid, flops, K);
-      case 4: return seq_fwd_do<64, 4, F16>(op, ctx, tm, a, grid, flops, K);
-      default: return seq_fwd_do<64, 8, F16>(op, ctx, tm, a, grid, flops, K);
+      case 1: return seq_fwd_do<64, 1, F16, VEC>(op, ctx, tm, a, grid, flops, K);
+      case 2: return seq_fwd_do<64, 2, F16, VEC>(op, ctx, tm, a, grid, flops, K);
+      case 4: return seq_fwd_do<64, 4, F16, VEC>(op, ctx, tm, a, grid, flops, K);
+      default: return seq_fwd_do<64, 8, F16, VEC>(op, ctx, tm, a, grid, flops, K);
     }
   }
   switch (S) {
-    case 1: return seq_fwd_do<128, 1, F16>(op, ctx, tm, a, grid, flops, K);
-    case 2: return seq_fwd_do<128, 2, F16>(op, ctx, tm, a, grid, flops, K);
-    case 4: return seq_fwd_do<128, 4, F16>(op, ctx, tm, a, grid, flops, K);
-    default: return seq_fwd_do<128, F16 ? 4 : 8, F16>(op, ctx, tm, a, grid, flops, K);
+    case 1: return seq_fwd_do<128, 1, F16, VEC>(op, ctx, tm, a, grid, flops, K);
+    case 2: return seq_fwd_do<128, 2, F16, VEC>(op, ctx, tm, a, grid, flops, K);
+    case 4: return seq_fwd_do<128, 4, F16, VEC>(op, ctx, tm, a, grid, flops, K);
+    default: return seq_fwd_do<128, F16 ? 4 : 8, F16, VEC>(op, ctx, tm, a, grid, flops, K);
   }
+}
+
+// the F16 form for units in fours and for others
+int seq_f16_dispatch(SeqOp op, bool vec, uint32_t bn, uint32_t S, dyb200_ctx* ctx, const TmapPack* tm = nullptr, const SeqFwd* a = nullptr, dim3 grid = dim3(), double flops = 0,
+                     uint32_t K = 0) {
+  return vec ? seq_fwd_dispatch<true, true>(op, bn, S, ctx, tm, a, grid, flops, K) : seq_fwd_dispatch<true, false>(op, bn, S, ctx, tm, a, grid, flops, K);
 }
 
 // ---- the inputs of the F16 form, one launch: a warp per line ----
@@ -510,10 +520,14 @@ __global__ void __launch_bounds__(256) k_seq_prep(const __grid_constant__ SeqPre
   const bool vec = aligned16(p) && (!p2 || aligned16(p2));
   auto mag = [](float4 v) { return max(max(finite_mag(v.x), finite_mag(v.y)), max(finite_mag(v.z), finite_mag(v.w))); };
   uint32_t m = kind == 1 && !p2 ? 0x3f800000u : 0;   // (h_{-1}: no smaller than the scale of later h, which an h_{-1} from a call for the step before is)
-  auto value = [&](uint32_t e) {   // elements [e, e + 4): n is a multiple of 4, or the line goes on with zeros (planes)
-    float4 v = vec ? ld4(p + e) : make_float4(p[e], p[e + 1], p[e + 2], p[e + 3]);
+  auto four = [&](const float* q, uint32_t e) {   // (zeros past the line's end)
+    if (vec && e + 4 <= n) return ld4(q + e);
+    return make_float4(q[e], e + 1 < n ? q[e + 1] : 0.f, e + 2 < n ? q[e + 2] : 0.f, e + 3 < n ? q[e + 3] : 0.f);
+  };
+  auto value = [&](uint32_t e) {   // elements [e, e + 4)
+    float4 v = four(p, e);
     if (p2) {
-      const float4 w = vec ? ld4(p2 + e) : make_float4(p2[e], p2[e + 1], p2[e + 2], p2[e + 3]);
+      const float4 w = four(p2, e);
       if (kind == 0) v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
       else {
         v = make_float4(v.x * w.x, v.y * w.y, v.z * w.z, v.w * w.w);
@@ -568,18 +582,19 @@ int layer_inputs(dyb200_ctx* ctx, dyb200_wgrad* deferred, const float* Wx, const
 // empty: 9 + 9 k-blocks make 6, 6, 6, 0, the longest still shorter than the 10 of two splits).  They are clusters whatever dyb200_ctx_cluster_splitk
 // says: there is no other form, and another number of splits would give other bits.  Columns and units past the end of a tile are computed and
 // dropped: a launch and more per step, which such layers took before, was 19 us at (512, 1024, 100 columns), 25 at (300, 600, 30), 24 at (512, 768, 300),
-// 31 at (512, 1000, 100) and 18 at (256, 1024, 16); here it is 8.9, 7.1, 10.8, 8.9 and 7.1.
+// 31 at (512, 1000, 100) and 18 at (256, 1024, 16); here it is 8.9, 7.1, 10.8, 8.9 and 7.1.  Units that do not come in fours have instantiations that
+// read and write a value at a time: 28 -> 10.1 at (512, 777, 100), 26 -> 8.0 at (300, 601, 30).
 bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* bn, uint32_t* S) {
-  if (H <= 384 || H % 4 != 0 || I == 0 || B <= 8) return false;
+  if (H <= 384 || I == 0 || B <= 8) return false;
   const uint32_t sms = (uint32_t)ctx->sm_count, tiles_m = (H + 31) / 32, kb = (I + 63) / 64 + (H + 63) / 64;
   *bn = tiles_m * ((B + 63) / 64) <= sms ? 64 : 128;
   const uint32_t tiles_n = (B + *bn - 1) / *bn, tiles = tiles_m * tiles_n;
   if (tiles_n > 32) return false;   // (one hand-over counter per column block)
   for (uint32_t s = *bn == 64 ? 8 : 4; s >= 1; s /= 2) {
     if (tiles * s > sms || (s > 1 && kb / s < 4)) continue;
-    if (seq_fwd_dispatch<true>(SEQ_SET_SMEM, *bn, s, ctx) != DYB200_OK) return false;
+    if (seq_f16_dispatch(SEQ_SET_SMEM, H % 4 == 0, *bn, s, ctx) != DYB200_OK) return false;
     if (s > 1) {
-      const int fit = seq_fwd_dispatch<true>(SEQ_FIT, *bn, s, ctx);
+      const int fit = seq_f16_dispatch(SEQ_FIT, H % 4 == 0, *bn, s, ctx);
       if (fit <= 0 || tiles > (uint32_t)fit) continue;
     }
     *S = s;
@@ -626,7 +641,7 @@ int dyb200_seq_f16(dyb200_ctx* ctx, const SeqF16Call& q) {
   a.ready = ctx->dev_flags + DYB200_DEV_SEQ0;
   a.flags = ctx->dev_flags;
   if (T > 1) DYB_CUDA(ctx, cudaMemsetAsync(a.ready, 0, 32 * sizeof(uint32_t), ctx->stream));   // (a single step's CTAs count, but nobody waits)
-  return seq_fwd_dispatch<true>(SEQ_LAUNCH, bn, S, ctx, &tm, &a, dim3(tiles_m, (B + bn - 1) / bn, S), 2.0 * G * (double)B * (I + H) * T, I + H);
+  return seq_f16_dispatch(SEQ_LAUNCH, H % 4 == 0, bn, S, ctx, &tm, &a, dim3(tiles_m, (B + bn - 1) / bn, S), 2.0 * G * (double)B * (I + H) * T, I + H);
 }
 
 extern "C" {

@@ -69,6 +69,25 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// Four neighbouring values of a row of units, `left` of which are there (VEC: all, on 16 bytes)
+template <bool VEC>
+__device__ __forceinline__ float4 ldu(const float* p, uint32_t left) {
+  if (VEC) return ld4(p);
+  return make_float4(p[0], left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
+}
+template <bool VEC>
+__device__ __forceinline__ float4 ldu_cg(const float* p, uint32_t left) {   // (from L2)
+  if (VEC) return __ldcg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldcg(p), left > 1 ? __ldcg(p + 1) : 0.f, left > 2 ? __ldcg(p + 2) : 0.f, left > 3 ? __ldcg(p + 3) : 0.f);
+}
+template <bool VEC>
+__device__ __forceinline__ void stu(float* p, float4 v, uint32_t left) {
+  if (VEC) { st4(p, v); return; }
+  p[0] = v.x;
+  if (left > 1) p[1] = v.y;
+  if (left > 2) p[2] = v.z;
+  if (left > 3) p[3] = v.w;
+}
 // The exchange buffer: columns of BM rows, quads of rows moved about so that the 16-byte stores of four neighbouring columns meet no bank twice.
 __device__ __forceinline__ uint32_t park_at(uint32_t col, uint32_t quad) { return col * BM + 4 * (quad ^ (2 * (col & 3))); }
 // v: four columns of this lane's row -> rows 4 (lane / 4) .. + 3 of column lane % 4.  (One 16-byte message to another CTA instead of four.)

@@ -25,6 +25,12 @@ pytestmark = pytest.mark.gpu
     (64, 2048, 500, 2, "one", 2, 2),
     (40, 2048, 1000, 2, None, 2, 1),
     (8, 3072, 1000, 2, None, 4, 1),
+    (388, 388, 70, 3, "one", 1, 8),        # units in fours, not in eights: the gates of the weights' pairs moved apart
+    (512, 777, 100, 3, "full", 1, 8),      # in neither: a value at a time
+    (30, 514, 64, 3, None, 1, 8),
+    (64, 1022, 500, 2, "one", 2, 4),
+    (9, 2049, 500, 2, None, 2, 2),
+    (9, 2047, 1000, 2, "full", 2, 1),
 ])
 def test_backward_of_a_wide_layer(I, H, B, T, mask, blocks, splits):
     import torch
