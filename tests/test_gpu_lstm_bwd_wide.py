@@ -21,6 +21,7 @@ pytestmark = pytest.mark.gpu
     (33, 448, 100, 3, "full", 1, 8),       # ... 64
     (300, 744, 33, 3, "full", 1, 8),       # ... 104: its second half is partly filled
     (130, 904, 300, 3, None, 2, 4),        # five column blocks: the last CTAs have one
+    (130, 904, 300, 34, None, 2, 4),       # more steps than the sums of the bias gradient take side by side, 20 tiles each
     (200, 576, 500, 2, "full", 1, 2),
     (64, 2048, 500, 2, "one", 2, 2),
     (40, 2048, 1000, 2, None, 2, 1),
