@@ -206,6 +206,17 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   r = warp_sum(r);
   return r;
 }
+// two sums behind the same barriers (red must hold 64 floats); each is what block_sum gives
+__device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  a = warp_sum(a);
+  b = warp_sum(b);
+  __syncthreads();
+  if (lane == 0) { red[w] = a; red[32 + w] = b; }
+  __syncthreads();
+  a = warp_sum(lane < nw ? red[lane] : 0.f);
+  b = warp_sum(lane < nw ? red[32 + lane] : 0.f);
+}
 __device__ __forceinline__ float block_max(float v, float* red) {
   int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   v = warp_max(v);

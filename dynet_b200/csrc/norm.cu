@@ -16,15 +16,27 @@ constexpr int kColMax = kBlock * 4 * kVec;
 __global__ void __launch_bounds__(kBlock) k_sumsq_dot_partial(const float* __restrict__ w, const float* __restrict__ d,
                                                              size_t n, float* __restrict__ partial) {
   dyb_grid_dep_sync();
-  __shared__ float red[32];
+  __shared__ float red[64];
   float ss = 0.f, dot = 0.f;
   const bool vec = aligned16(w) && (d == nullptr || aligned16(d));
   if (vec) {
-    size_t n4 = n / 4;
-    for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n4; i += (size_t)gridDim.x * kBlock) {
-      float4 a = ld4(w + 4 * i);
-      ss += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
-      if (d) { float4 b = ld4_stream(d + 4 * i); dot += (a.x * b.x + a.y * b.y) + (a.z * b.z + a.w * b.w); }
+    // (four vectors of either tensor requested at a time: one by one a thread's seven trips to memory followed one another.  Forward and both backward calls at
+    // 4096 x 1024, with the first vectors of the second pass requested ahead of the partial sums: 47 us -> 38)
+    const size_t n4 = n / 4, step = (size_t)gridDim.x * kBlock;
+    for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n4; i += 4 * step) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool there = i + k * step < n4;
+        a[k] = there ? ld4(w + 4 * (i + k * step)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        b[k] = there && d ? ld4_stream(d + 4 * (i + k * step)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (i + k * step >= n4) break;
+        ss += (a[k].x * a[k].x + a[k].y * a[k].y) + (a[k].z * a[k].z + a[k].w * a[k].w);
+        if (d) dot += (a[k].x * b[k].x + a[k].y * b[k].y) + (a[k].z * b[k].z + a[k].w * b[k].w);
+      }
     }
     if (blockIdx.x == 0) {
       size_t i = 4 * n4 + threadIdx.x;
@@ -36,16 +48,17 @@ __global__ void __launch_bounds__(kBlock) k_sumsq_dot_partial(const float* __res
       if (d) dot += w[i] * d[i];
     }
   }
-  ss = block_sum(ss, red);
-  dot = block_sum(dot, red);
+  block_sum2(ss, dot, red);
   if (threadIdx.x == 0) { partial[2 * blockIdx.x] = ss; partial[2 * blockIdx.x + 1] = dot; }
 }
 // Every CTA reduces the same partial list in the same order.
 __device__ __forceinline__ void reduce_partials(const float* partial, int np, float* red, float& ss, float& dot) {
   float a = 0.f, b = 0.f;
+#pragma unroll 4
   for (int k = threadIdx.x; k < np; k += kBlock) { a += partial[2 * k]; b += partial[2 * k + 1]; }
-  ss = block_sum(a, red);
-  dot = block_sum(b, red);
+  block_sum2(a, b, red);
+  ss = a;
+  dot = b;
 }
 // MODE 0: y = (w / nrm) * g          MODE 1: dw += (dy / nrm) * g - y * (dot / ss)
 template <int MODE>
@@ -54,20 +67,33 @@ __global__ void __launch_bounds__(kBlock) k_weight_norm_apply(const float* __res
                                                              float* __restrict__ out, size_t n,
                                                              const float* __restrict__ partial, int np) {
   dyb_grid_dep_sync();
-  __shared__ float red[32];
+  __shared__ float red[64];
+  const bool vec = aligned16(w) && aligned16(out) && (MODE == 0 || (aligned16(y) && aligned16(dy)));
+  const size_t n4 = vec ? n / 4 : 0, step = (size_t)gridDim.x * kBlock;
+  constexpr int U = MODE == 0 ? 4 : 2;   // vectors of each tensor on their way, the first of them while the partial sums are added up
+  float4 a[U], yy[U], o[U];
+  size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x;
+  auto load = [&]() {
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const size_t e = 4 * (i + k * step);
+      if (i + k * step >= n4) break;
+      if (MODE == 0) a[k] = ld4(w + e);
+      else { a[k] = ld4_stream(dy + e); yy[k] = ld4_stream(y + e); o[k] = ld4_stream(out + e); }
+    }
+  };
+  load();
   float ss, dot;
   reduce_partials(partial, np, red, ss, dot);
   const float nrm = sqrtf(ss), g = gptr[0], t2 = dot / ss, sc = g / nrm;
-  const bool vec = aligned16(w) && aligned16(out) && (MODE == 0 || (aligned16(y) && aligned16(dy)));
-  const size_t n4 = vec ? n / 4 : 0;
-  for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n4; i += (size_t)gridDim.x * kBlock) {
-    if (MODE == 0) {
-      float4 a = ld4(w + 4 * i);
-      st4_stream(out + 4 * i, make_float4(a.x * sc, a.y * sc, a.z * sc, a.w * sc));
-    } else {
-      float4 d = ld4_stream(dy + 4 * i), yy = ld4_stream(y + 4 * i), o = ld4_stream(out + 4 * i);
-      st4_stream(out + 4 * i, make_float4(o.x + (d.x * sc - yy.x * t2), o.y + (d.y * sc - yy.y * t2),
-                                          o.z + (d.z * sc - yy.z * t2), o.w + (d.w * sc - yy.w * t2)));
+  for (; i < n4; i += U * step, load()) {
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const size_t e = 4 * (i + k * step);
+      if (i + k * step >= n4) break;
+      if (MODE == 0) st4_stream(out + e, make_float4(a[k].x * sc, a[k].y * sc, a[k].z * sc, a[k].w * sc));
+      else st4_stream(out + e, make_float4(o[k].x + (a[k].x * sc - yy[k].x * t2), o[k].y + (a[k].y * sc - yy[k].y * t2),
+                                           o[k].z + (a[k].z * sc - yy[k].z * t2), o[k].w + (a[k].w * sc - yy[k].w * t2)));
     }
   }
   for (size_t i = 4 * n4 + (size_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (size_t)gridDim.x * kBlock) {
@@ -77,7 +103,7 @@ __global__ void __launch_bounds__(kBlock) k_weight_norm_apply(const float* __res
 }
 __global__ void __launch_bounds__(kBlock) k_weight_norm_dg(const float* __restrict__ partial, int np, float* __restrict__ dg) {
   dyb_grid_dep_sync();
-  __shared__ float red[32];
+  __shared__ float red[64];
   float ss, dot;
   reduce_partials(partial, np, red, ss, dot);
   if (threadIdx.x == 0) dg[0] += dot / sqrtf(ss);
@@ -263,7 +289,7 @@ __global__ void __launch_bounds__(kBlock) k_layer_norm_bwd_x(const float* __rest
                                                             const float* __restrict__ dy, float* __restrict__ dx,
                                                             uint32_t n, size_t ncols, int cached) {
   dyb_grid_dep_sync();
-  __shared__ float red[32];
+  __shared__ float red[64];
   const float fn = (float)n;
   for (size_t c = blockIdx.x; c < ncols; c += gridDim.x) {
     LnLoad L;
@@ -294,8 +320,9 @@ __global__ void __launch_bounds__(kBlock) k_layer_norm_bwd_x(const float* __rest
         Bs += q;
       }
     }
-    A = block_sum(A, red) * inv * inv;
-    Bs = block_sum(Bs, red) * inv;
+    block_sum2(A, Bs, red);
+    A = A * inv * inv;
+    Bs = Bs * inv;
     const float sb = (-A) / (2.f * sigma), dmu_n = (-Bs) / fn, two_n = 2.f / fn;
     if (cached) {
       const uint32_t n4 = n / 4;
