@@ -1806,7 +1806,7 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   TcKernel kern;
   if (Sp == 0) {
     if ((rc = tc_kernel(ctx, bn, Sc > 1, TC_TWO, &kern))) return rc;
-    GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
+    GemmProfScope scope(ctx, only_if ? 0.0 : flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);   // (under a condition: the products on pairs have been counted)
     if (Sc == 1) {
       dyb_launch(kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
     } else {
