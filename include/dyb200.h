@@ -321,8 +321,9 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
  * dyb200_vanilla_lstm_fwd_fused_at with deferred_col = t * batch, h_tm1 / c_tm1 = the previous step's outputs.
  *   * When the shape allows (deferred given, tensor-path sizes, whole tiles, every CTA resident at once) the steps run inside ONE
  *     kernel whose CTAs stay on the GPU for the whole sequence and hand h_t over through device memory: bit for bit the calls above.
- *     From 512 units on the products of both (calls with an accumulator, batches in whole 64-column tiles) are of scaled fp16 pairs: a scale
- *     per gate row of Wx and of Wh and per column of x, and for a column of h the largest of its mask's values (1 without) and, in the first step, of h0.
+ *     Above 384 units and eight columns (any number of either; deferred given, or at least 8 steps without masks) the products are of scaled fp16 pairs, as
+ *     those of the single-step calls with an accumulator above 32 columns: a scale per gate row of Wx and of Wh and per column of x, and for a column of h
+ *     the largest of its mask's values (1 without) and, in the first step, of h0.
  *   * Other sequences of at least 8 steps of layers up to 384 units, or with at most 32 columns, form Wx x of all steps at once and
  *     keep only Wh h in the recurrence: the same values to the rounding of their sums, which associate differently, and the same
  *     bits from run to run.  Wh h is plain fp32 above 256 units, and below while there are at most four columns per cluster of
@@ -345,7 +346,10 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
  * deferred_col = t * batch.  dh_all / dc_all hold dE/dh_t and dE/dc_t of every
  * step as left by the layers above (the recurrent parts are accumulated into them on the way); dx_all accumulates.  With deferred the columns of the accumulator must hold the
  * layer inputs placed by dyb200_vanilla_lstm_seq_fwd / _fwd_fused_at, and dWx / dWh may be NULL; without it every step adds
- * its weight gradients to dWx / dWh at once.  When the shape allows (as for the forward call; deferred and dx_all given), the
+ * its weight gradients to dWx / dWh at once.  Above 384 units and eight columns (any number of either, deferred given, at most 256 steps) Wh^T dgates alone
+ * stays in the recurrence, one kernel for all steps, and dx of all columns is one product after it; the single-step calls run the same kernels for one step
+ * and give the same bits.  Both are products of scaled fp16 pairs: a scale per row of Wh^T and Wx^T, and one per column of dgates and block of 128 units (all
+ * four gates).  Narrower layers: when the shape allows (as for the forward call; deferred and dx_all given), the
  * steps run inside ONE kernel whose CTAs stay on the GPU: the cell pass and the [Wx; Wh]^T dgates product of a step hand
  * over through counters in device memory, and every CTA alternates between two independent blocks of batch columns so that
  * one block's hand-overs hide behind the other's products (the per-step call uses the same K splits for such shapes, which
