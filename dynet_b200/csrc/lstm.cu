@@ -572,8 +572,10 @@ int dyb200_vanilla_lstm_fwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
       return dyb200_lstm_thin(ctx, H, B, 2, pairs, 0, e);
     }
     uint32_t bn, S;
-    if (shapes_ok && deferred && attrs->weightnoise_std == 0.f && I > 0 && B > 0 && aligned16(gates->v) && aligned16(b->v) && aligned16(c_tm1->v) && aligned16(c_t->v) &&
-        aligned16(h_t->v) && (!attrs->dropout || aligned16(mask_h->v)) && dyb200_seq_f16_plan(ctx, I, H, B, &bn, &S)) {
+    // (units that do not come in fours are moved a value at a time: a step of stacked states may start anywhere)
+    const bool on16 = H % 4 != 0 || (aligned16(gates->v) && aligned16(b->v) && aligned16(c_tm1->v) && aligned16(c_t->v) && aligned16(h_t->v) &&
+                                     (!attrs->dropout || aligned16(mask_h->v)));
+    if (shapes_ok && deferred && attrs->weightnoise_std == 0.f && I > 0 && B > 0 && on16 && dyb200_seq_f16_plan(ctx, I, H, B, &bn, &S)) {
       { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
       PackedOp Bp[2];
       int rc;
@@ -697,8 +699,10 @@ int dyb200_vanilla_lstm_bwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
                      aligned16(c_tm1->v) && aligned16(gates->v) && aligned16(dEdh->v) && (!dEdc || aligned16(dEdc->v)) &&
                      (!dc_tm1 || aligned16(dc_tm1->v));
   uint32_t wide_ncb, wide_S;
-  if (deferred && I > 0 && (!mh || aligned16(mh)) && aligned16(gates->v) && aligned16(c_t->v) && aligned16(c_tm1->v) && aligned16(dEdh->v) &&
-      (!dEdc || aligned16(dEdc->v)) && (!dc_tm1 || aligned16(dc_tm1->v)) && (!dh_tm1 || aligned16(dh_tm1->v)) && dyb200_bwd_wide_plan(ctx, H, B, &wide_ncb, &wide_S)) {
+  // (units that do not come in fours are moved a value at a time: a step of stacked states may start anywhere)
+  const bool on16 = H % 4 != 0 || ((!mh || aligned16(mh)) && aligned16(gates->v) && aligned16(c_t->v) && aligned16(c_tm1->v) && aligned16(dEdh->v) &&
+                                   (!dEdc || aligned16(dEdc->v)) && (!dc_tm1 || aligned16(dc_tm1->v)) && (!dh_tm1 || aligned16(dh_tm1->v)));
+  if (deferred && I > 0 && on16 && dyb200_bwd_wide_plan(ctx, H, B, &wide_ncb, &wide_S)) {
     // wide layers with an accumulator: the sequence's kernels, for one step (lstm_bwd_wide.cu)
     DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_bwd_fused: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);
     BwdWideCall q{I, H, B, 1, Wx->v, Wh->v, gates->v, c_t->v, c_tm1->v, dEdh->v, dEdc ? dEdc->v : nullptr, dh_tm1 ? dh_tm1->v : nullptr, dc_tm1 ? dc_tm1->v : nullptr,

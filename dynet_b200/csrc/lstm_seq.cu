@@ -679,8 +679,8 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
   const uint32_t bn = dyb200_tc_tile_cols(B);
   const uint32_t kb0 = (I + 31) / 32, kb1 = (H + 31) / 32, kb_total = kb0 + kb1;
   const bool sequence = ctx->seq_kernels && T >= 2 && attrs->weightnoise_std == 0.f && Wx->nd == 2 && Wx->d[0] == G && Wx->d[1] == I && Wh->nd == 2 &&
-                    Wh->d[0] == G && Wh->d[1] == H && t_size(b) == G && aligned16(gates_all->v) && aligned16(b->v) && aligned16(c0->v) &&
-                    aligned16(c_all->v) && aligned16(h_all->v) && (!mh || aligned16(mh)) &&
+                    Wh->d[0] == G && Wh->d[1] == H && t_size(b) == G &&
+                    (H % 4 != 0 || (aligned16(gates_all->v) && aligned16(b->v) && aligned16(c0->v) && aligned16(c_all->v) && aligned16(h_all->v) && (!mh || aligned16(mh)))) &&
                     (!attrs->dropout || ((mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_h, 0) == H));
   const bool resident = sequence && deferred && H % 32 == 0 && I % 4 == 0 && dyb200_tc_eligible(G, B, 2.0 * G * B * (I + H));
   uint32_t S = 1, f16_bn;

@@ -629,7 +629,7 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
   const bool masks_ok = !mx || ((mask_x->bd == B || mask_x->bd == 1) && (mask_h->bd == B || mask_h->bd == 1) && t_dim(mask_x, 0) == I && t_dim(mask_h, 0) == H);
   bool wide_fits = true;
   if (ctx->seq_kernels && deferred && T >= 2 && T <= kDbMaxSteps && attrs->weightnoise_std == 0.f && I > 0 && weights_ok && masks_ok && dyb200_wgrad_rows(deferred) == G &&
-      aligned16(gates_all->v) && aligned16(c_all->v) && aligned16(c0->v) && aligned16(dh_all->v) && aligned16(dc_all->v) && (!mh || aligned16(mh)) &&
+      (H % 4 != 0 || (aligned16(gates_all->v) && aligned16(c_all->v) && aligned16(c0->v) && aligned16(dh_all->v) && aligned16(dc_all->v) && (!mh || aligned16(mh)))) &&
       dyb200_bwd_wide_plan(ctx, H, B, &wide_ncb, &wide_S)) {
     { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
     BwdWideCall q{I, H, B, T, Wx->v, Wh->v, gates_all->v, c_all->v, c0->v, dh_all->v, dc_all->v, nullptr, nullptr, dx_all ? dx_all->v : nullptr,

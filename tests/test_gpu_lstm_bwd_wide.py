@@ -32,6 +32,9 @@ pytestmark = pytest.mark.gpu
     (64, 1022, 500, 2, "one", 2, 4),
     (9, 2049, 500, 2, None, 2, 2),
     (9, 2047, 1000, 2, "full", 2, 1),
+    (512, 777, 33, 4, "full", 1, 8),       # ... and steps of the stacked states start on any four bytes
+    (9, 385, 37, 5, "one", 1, 8),
+    (64, 1022, 131, 3, None, 1, 4),        # (on eight)
 ])
 def test_backward_of_a_wide_layer(I, H, B, T, mask, blocks, splits):
     import torch
@@ -97,14 +100,15 @@ def test_backward_of_a_wide_layer(I, H, B, T, mask, blocks, splits):
     assert bool(((db - db_want).abs() <= db_bar).all()), float(((db - db_want).abs() / db_bar).max())
 
 
-def test_sequence_without_room_for_its_pairs():
-    """Little device memory: the pairs of all steps (134 MB) do not fit, those of one (2 MB) do - the single-step calls run, with the same bits."""
+@pytest.mark.parametrize("H,B", [(512, 256), (513, 255)])
+def test_sequence_without_room_for_its_pairs(H, B):
+    """Little device memory: the pairs of all steps (134 MB and more) do not fit, those of one (2 MB) do - the single-step calls run, with the same bits."""
     import contextlib
     import torch
     import gpu_util as g
     from dynet_b200 import capi
     from test_gpu_scratch_limits import room_for
-    I, H, B, T = 64, 512, 256, 64
+    I, T = 64, 64
     rnd = lambda *s: torch.randn(*s, device="cuda")   # noqa: E731
     x, c0, cs, gates = rnd(T * B, I), rnd(B, H), rnd(T * B, H), torch.sigmoid(rnd(T * B, 4 * H))
     Wx, Wh, dh_in = rnd(I, 4 * H) / H ** 0.5, rnd(H, 4 * H) / H ** 0.5, rnd(T * B, H)

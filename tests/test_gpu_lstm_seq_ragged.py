@@ -23,6 +23,9 @@ pytestmark = pytest.mark.gpu
     (64, 1023, 500, 3, None, True),         # ... on 128-column tiles
     (128, 433, 40, 8, None, False),
     (1100, 641, 64, 8, "full", True),       # weights in two passes (more lines than a strip holds)
+    (300, 777, 33, 8, "full", True),        # steps of the stacked states start on any four bytes
+    (31, 385, 37, 5, "one", True),
+    (64, 1022, 131, 3, None, True),         # (on eight)
 ])
 def test_sequence_that_does_not_fill_its_tiles(I, H, B, T, mask, acc):
     import torch
