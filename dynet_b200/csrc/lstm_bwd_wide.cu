@@ -57,6 +57,113 @@ __device__ __forceinline__ KBlock k_block(uint32_t i, uint32_t H, uint32_t Ha, u
 constexpr int kMaxBlocks = 4;   // column blocks per CTA
 
 struct CellIn { float4 gi, gf, go, gg, c, cp, dci, dcp; };
+// What a thread of the eight warps that share a CTA's columns does of the cell pass: units [u, + 4) of block `blk`, `left` of them there (own: any)
+struct CellUnits { uint32_t blk, u, left; bool own; };
+
+template <bool VEC>
+__device__ __forceinline__ void cell_load(const BwdWide& a, const CellUnits& q, CellIn& in, uint32_t t, uint32_t n) {
+  const size_t HB = (size_t)a.H * a.B, e = (size_t)n * a.H + q.u;
+  const float* g = a.gates + (size_t)t * 4 * HB + (size_t)n * 4 * a.H + q.u;
+  in.gi = ldu<VEC>(g, q.left); in.gf = ldu<VEC>(g + a.H, q.left); in.go = ldu<VEC>(g + 2 * a.H, q.left); in.gg = ldu<VEC>(g + 3 * a.H, q.left);
+  in.c = ldu<VEC>(a.cs + (size_t)t * HB + e, q.left);
+  in.cp = ldu<VEC>((t ? a.cs + (size_t)(t - 1) * HB : a.c0) + e, q.left);
+  const float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
+  in.dci = a.dc ? ldu_cg<VEC>(a.dc + (size_t)t * HB + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
+  in.dcp = dcp ? ldu_cg<VEC>(dcp + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// The cell pass of units [u, + 4), column n of step t from dE/dh: dE/dc of the step before, and dgates as fp16 pairs with the word of the warp's
+// (column, block).  The four gates' gradients come back in p and are added to rs.  (All lanes of a warp take part; those past the last unit with zeros.)
+__device__ __forceinline__ void cell(const BwdWide& a, const CellUnits& q, CellIn& in, float4 dh, uint32_t t, uint32_t n, float4 (&p)[4], float4 (&rs)[4]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) p[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (q.own) {
+    const float* f[8] = {&in.gi.x, &in.gf.x, &in.go.x, &in.gg.x, &in.c.x, &in.cp.x, &dh.x, &in.dci.x};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      lstm_cell_grad(f[0][k], f[1][k], f[2][k], f[3][k], f[4][k], f[5][k], f[6][k], f[7][k], a.dc != nullptr, (&in.dcp.x)[k], (&p[0].x)[k], (&p[1].x)[k],
+                     (&p[2].x)[k], (&p[3].x)[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      m = max(m, max(max(finite_mag(p[k].x), finite_mag(p[k].y)), max(finite_mag(p[k].z), finite_mag(p[k].w))));
+      rs[k].x += p[k].x; rs[k].y += p[k].y; rs[k].z += p[k].z; rs[k].w += p[k].w;
+    }
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  const size_t r = (size_t)t * a.B + n;
+  if ((threadIdx.x & 31) == 0) a.dsc[(size_t)q.blk * a.dsc_ld + r] = m;
+  const float s = scale_of(m);
+  if (q.u < a.Hp) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      __half hi[4], lo[4];
+      split_f16(p[k].x * s, hi[0], lo[0]); split_f16(p[k].y * s, hi[1], lo[1]); split_f16(p[k].z * s, hi[2], lo[2]); split_f16(p[k].w * s, hi[3], lo[3]);
+      const size_t o = (r * 4 + k) * a.Hp + q.u;
+      *reinterpret_cast<uint2*>(a.d16_hi + o) = *reinterpret_cast<const uint2*>(hi);
+      *reinterpret_cast<uint2*>(a.d16_lo + o) = *reinterpret_cast<const uint2*>(lo);
+    }
+  }
+}
+template <bool VEC>
+__device__ __forceinline__ void cell_rest(const BwdWide& a, const CellUnits& q, const CellIn& in, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dE/dc of the step before, dgates for the weight gradients
+  if (!q.own) return;
+  float* dcp = t ? a.dc + (size_t)(t - 1) * a.H * a.B : a.dc_prev;
+  if (dcp) stu<VEC>(dcp + (size_t)n * a.H + q.u, in.dcp, q.left);
+  const size_t o = ((size_t)t * a.B + n) * a.dn_pitch + q.u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float4 hi, lo;
+    split_tf32(p[k].x, hi.x, lo.x); split_tf32(p[k].y, hi.y, lo.y); split_tf32(p[k].z, hi.z, lo.z); split_tf32(p[k].w, hi.w, lo.w);
+    stu<VEC>(a.dn_hi + o + (size_t)k * a.H, hi, q.left); stu<VEC>(a.dn_lo + o + (size_t)k * a.H, lo, q.left);
+  }
+}
+// The row sums of a CTA's columns in a step (part: those of its column block and rank), through 4096 floats of shared memory: the eight warps' columns
+// in order.  te: thread of the 256.
+__device__ __forceinline__ void row_sums(const BwdWide& a, const float4 (&rs)[4], float* park, float* part, uint32_t blk, uint32_t te, uint32_t ew, uint32_t uq, bool ok) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) st4(park + (ew * 4 + q) * BM + uq, rs[q]);
+  bar_sync(1, 256);
+#pragma unroll
+  for (uint32_t k = 0; k < 2; ++k) {
+    const uint32_t r = te + 256 * k, q = r / BM, j = r % BM;
+    float v[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) v[x] = park[(x * 4 + q) * BM + j];
+#pragma unroll
+    for (int x = 1; x < 8; ++x) v[0] += v[x];
+    if (ok && blk * BM + j < a.H) part[(size_t)q * a.H + blk * BM + j] = v[0];
+  }
+  bar_sync(1, 256);
+}
+__device__ __forceinline__ float* part_of(const BwdWide& a, uint32_t step, uint32_t block, uint32_t splits, uint32_t rank) {
+  return a.part + (((size_t)step * a.tiles_n + block) * splits + rank) * 4 * a.H;
+}
+
+// The cell pass of a single step on its own: what a CTA of the recurrence does before its first product, its columns and their order included - the row sums
+// of dgates are the sequence's bit for bit.  Bound by its few loads' latency (a column per warp at eight splits); no cluster, no TMEM, 16 KB.
+// grid = (tiles_m, tiles_n, splits)
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_bwd_cells(const __grid_constant__ BwdWide a) {
+  dyb_grid_dep_sync();
+  __shared__ __align__(16) float park[32 * BM];
+  const uint32_t ew = threadIdx.x >> 5, u = blockIdx.x * BM + 4 * (threadIdx.x & 31), w = 64 / gridDim.z;
+  const CellUnits un{blockIdx.x, u, a.H - u, u < a.H};
+  float4 rs[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) rs[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (uint32_t c = ew; c < w; c += 8) {
+    const uint32_t n = 64 * blockIdx.y + blockIdx.z * w + c;
+    if (n >= a.B) break;
+    CellIn in = {};
+    float4 dh = make_float4(0.f, 0.f, 0.f, 0.f), p[4];
+    if (un.own) { cell_load<VEC>(a, un, in, 0, n); dh = ldu<VEC>(a.dh + (size_t)n * a.H + u, un.left); }
+    cell(a, un, in, dh, 0, n, p, rs);
+    cell_rest<VEC>(a, un, in, p, 0, n);
+  }
+  row_sums(a, rs, park, part_of(a, 0, blockIdx.y, gridDim.z, blockIdx.z), blockIdx.x, threadIdx.x, ew, 4 * (threadIdx.x & 31), true);
+}
 
 // REC: the recurrence, grid = (tiles_m, column blocks, S).  Otherwise dx: grid = (clusters, 1, S), the clusters walk the tiles.
 // VEC: units in fours, on 16 bytes (dx has a rule of its own for its rows).
@@ -72,6 +179,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
   float* park = reinterpret_cast<float*>(ring + (size_t)kStages * kStageBytes);   // 64 columns x BM rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = blockIdx.z;
+  if (a.T == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // this CTA's k-blocks: an equal share, or (dx with splits) one block of units, so that the sums are those of the unsplit form
   const uint32_t per = REC || S == 1 ? (a.kbs + S - 1) / S : 8, k0 = min(rank * per, a.kbs), total = min(k0 + per, a.kbs) - k0;
   const uint32_t slots = REC ? S : min(S, (a.kbs + 7) / 8);
@@ -116,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
         if (REC) {
           // The weights of the first k-blocks do not depend on the cell pass and are requested as their stages become free; the pairs of dgates follow
           // as soon as the counter says so, with more column blocks than one before all of those stages are free.
-          const uint32_t pre = min((uint32_t)kStages, total), want = (it + 1) * per_step;
+          const uint32_t pre = min((uint32_t)kStages, total), want = a.T > 1 ? (it + 1) * per_step : 0;
           uint32_t sa = s, pa = ph, na = 0;   // next stage for weights, its phase, weights requested so far
           bool ready = false;
           for (uint32_t poll = 0; !fail && (!ready || i < pre); ++poll) {
@@ -211,95 +319,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
     const uint32_t u = blockIdx.x * BM + uq;                            // REC: units [u, u + 4)
     const bool own_u = u < a.H;
     const uint32_t left = a.H - u;                                      // (own_u) units from u on
+    const CellUnits un{blockIdx.x, u, left, own_u};
     float4 rs[4];   // REC: row sums of dgates over this thread's columns of a step
 
     auto column = [&](int hh, uint32_t k) { const uint32_t p = rank * w + ew + 8 * k; return (p >> 5) * kHalf + 32 * hh + (p & 31); };
-    auto cell_load = [&](CellIn& in, uint32_t t, uint32_t n) {
-      const size_t e = (size_t)n * a.H + u;
-      const float* g = a.gates + (size_t)t * 4 * HB + (size_t)n * 4 * a.H + u;
-      in.gi = ldu<VEC>(g, left); in.gf = ldu<VEC>(g + a.H, left); in.go = ldu<VEC>(g + 2 * a.H, left); in.gg = ldu<VEC>(g + 3 * a.H, left);
-      in.c = ldu<VEC>(a.cs + (size_t)t * HB + e, left);
-      in.cp = ldu<VEC>((t ? a.cs + (size_t)(t - 1) * HB : a.c0) + e, left);
-      const float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
-      in.dci = a.dc ? ldu_cg<VEC>(a.dc + (size_t)t * HB + e, left) : make_float4(0.f, 0.f, 0.f, 0.f);
-      in.dcp = dcp ? ldu_cg<VEC>(dcp + e, left) : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    // The cell pass of units [u, + 4), column n of step t from dE/dh: dE/dc of the step before, and dgates as fp16 pairs with the word of the warp's
-    // (column, block).  The four gates' gradients come back in p.  (All lanes of a warp take part; those past the last unit with zeros.)
-    auto cell = [&](CellIn& in, float4 dh, uint32_t t, uint32_t n, float4 (&p)[4]) {
-      uint32_t m = 0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) p[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (own_u) {
-        const float* f[8] = {&in.gi.x, &in.gf.x, &in.go.x, &in.gg.x, &in.c.x, &in.cp.x, &dh.x, &in.dci.x};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          lstm_cell_grad(f[0][q], f[1][q], f[2][q], f[3][q], f[4][q], f[5][q], f[6][q], f[7][q], a.dc != nullptr, (&in.dcp.x)[q], (&p[0].x)[q], (&p[1].x)[q],
-                         (&p[2].x)[q], (&p[3].x)[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          m = max(m, max(max(finite_mag(p[q].x), finite_mag(p[q].y)), max(finite_mag(p[q].z), finite_mag(p[q].w))));
-          rs[q].x += p[q].x; rs[q].y += p[q].y; rs[q].z += p[q].z; rs[q].w += p[q].w;
-        }
-      }
-      m = __reduce_max_sync(0xffffffffu, m);
-      const size_t r = (size_t)t * a.B + n;
-      if (lane == 0) a.dsc[(size_t)blockIdx.x * a.dsc_ld + r] = m;
-      const float s = scale_of(m);
-      if (u < a.Hp) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          __half hi[4], lo[4];
-          split_f16(p[q].x * s, hi[0], lo[0]); split_f16(p[q].y * s, hi[1], lo[1]); split_f16(p[q].z * s, hi[2], lo[2]); split_f16(p[q].w * s, hi[3], lo[3]);
-          const size_t o = (r * 4 + q) * a.Hp + u;
-          *reinterpret_cast<uint2*>(a.d16_hi + o) = *reinterpret_cast<const uint2*>(hi);
-          *reinterpret_cast<uint2*>(a.d16_lo + o) = *reinterpret_cast<const uint2*>(lo);
-        }
-      }
-    };
-    auto cell_rest = [&](const CellIn& in, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dE/dc of the step before, dgates for the weight gradients
-      if (!own_u) return;
-      float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
-      if (dcp) stu<VEC>(dcp + (size_t)n * a.H + u, in.dcp, left);
-      const size_t o = ((size_t)t * a.B + n) * a.dn_pitch + u;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float4 hi, lo;
-        split_tf32(p[q].x, hi.x, lo.x); split_tf32(p[q].y, hi.y, lo.y); split_tf32(p[q].z, hi.z, lo.z); split_tf32(p[q].w, hi.w, lo.w);
-        stu<VEC>(a.dn_hi + o + (size_t)q * a.H, hi, left); stu<VEC>(a.dn_lo + o + (size_t)q * a.H, lo, left);
-      }
-    };
     auto publish = [&](uint32_t cb) {   // (behind a barrier: one thread's release orders all the stores it has observed, for both proxies)
       if (te == 0) {
         asm volatile("fence.proxy.async.global;" ::: "memory");
         signal_counter(a.done + block0 + cb);
       }
     };
-    // The row sums of this CTA's columns in step `step` of the sweep, through the exchange buffer: the eight warps' columns in order.
-    auto row_sums = [&](uint32_t step, uint32_t cb) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) st4(park + (ew * 4 + q) * BM + uq, rs[q]);
-      bar_sync(1, 256);
-      float* part = a.part + (((size_t)step * a.tiles_n + block0 + cb) * S + rank) * 4 * a.H;
-#pragma unroll
-      for (uint32_t k = 0; k < 2; ++k) {
-        const uint32_t r = te + 256 * k, q = r / BM, j = r % BM;
-        float v[8];
-#pragma unroll
-        for (int x = 0; x < 8; ++x) v[x] = park[(x * 4 + q) * BM + j];
-#pragma unroll
-        for (int x = 1; x < 8; ++x) v[0] += v[x];
-        if (ok && blockIdx.x * BM + j < a.H) part[(size_t)q * a.H + blockIdx.x * BM + j] = v[0];
-      }
-      bar_sync(1, 256);
-    };
     auto clear_sums = [&]() {
 #pragma unroll
       for (int q = 0; q < 4; ++q) rs[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     };
 
-    for (uint32_t cb = 0; REC && cb < nblocks; ++cb) {   // the cell pass of the last step
+    for (uint32_t cb = 0; REC && a.T > 1 && cb < nblocks; ++cb) {   // the cell pass of the last step (of a single one: k_bwd_cells)
       const uint32_t t = a.T - 1, n0 = (block0 + cb) * BNT;
       clear_sums();
 #pragma unroll 1
@@ -310,13 +345,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
           if (n >= a.B) continue;
           CellIn in = {};
           float4 dh = make_float4(0.f, 0.f, 0.f, 0.f), p[4];
-          if (own_u) { cell_load(in, t, n); dh = ldu<VEC>(a.dh + (size_t)t * HB + (size_t)n * a.H + u, left); }
-          cell(in, dh, t, n, p);
-          cell_rest(in, p, t, n);
+          if (own_u) { cell_load<VEC>(a, un, in, t, n); dh = ldu<VEC>(a.dh + (size_t)t * HB + (size_t)n * a.H + u, left); }
+          cell(a, un, in, dh, t, n, p, rs);
+          cell_rest<VEC>(a, un, in, p, t, n);
         }
-      row_sums(0, cb);
+      row_sums(a, rs, park, part_of(a, 0, block0 + cb, S, rank), blockIdx.x, te, ew, uq, ok);
     }
-    if (REC)   // (all blocks at the end: the exchange buffer belongs to the others from the first one on)
+    if (REC && a.T > 1)   // (all blocks at the end: the exchange buffer belongs to the others from the first one on)
       for (uint32_t cb = 0; cb < nblocks; ++cb) publish(cb);
 
     float row_f = REC ? inv_scale_of(blockIdx.x * BM + row < a.M ? __ldg(a.wscale + blockIdx.x * BM + row) : 0x3f800000u) : 1.f;
@@ -424,7 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
               const float* mp = a.mask + m + (a.mask_full ? (size_t)(REC ? n[g] : n[g] % a.B) * a.M : 0);
               mk[g] = REC ? ldu<VEC>(mp, left) : ld4(mp);
             }
-            if (REC && t) cell_load(in[g], t - 1, n[g]);
+            if (REC && t) cell_load<VEC>(a, un, in[g], t - 1, n[g]);
           }
           if (kb == 0) {
             const bool got = S > 1 ? mbar_wait_cluster(&park_full, pf_phase) : true;
@@ -445,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
               else v = make_float4(v.x + old[g].x, v.y + old[g].y, v.z + old[g].z, v.w + old[g].w);
             }
             old[g] = v;
-            if (REC && t && ok) cell(in[g], v, t - 1, n[g], p[g]);
+            if (REC && t && ok) cell(a, un, in[g], v, t - 1, n[g], p[g], rs);
             if (vec || !own || !ok) continue;
             for (uint32_t q = 0; q < 4 && m + q < a.M; ++q) {
               float* d = dst + (size_t)n[g] * a.M + m + q;
@@ -461,10 +496,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
           for (uint32_t g = 0; g < GB; ++g) {
             if (n[g] >= cols) continue;
             if (own && vec) { if (REC) stu<VEC>(dst + (size_t)n[g] * a.M + m, old[g], left); else st4(dst + (size_t)n[g] * a.M + m, old[g]); }
-            if (REC && t) cell_rest(in[g], p[g], t - 1, n[g]);
+            if (REC && t) cell_rest<VEC>(a, un, in[g], p[g], t - 1, n[g]);
           }
         }
-        if (REC && t && last_pass) row_sums(it + 1, cb);
+        if (REC && t && last_pass) row_sums(a, rs, park, part_of(a, it + 1, block0 + cb, S, rank), blockIdx.x, te, ew, uq, ok);
         else bar_sync(1, 256);    // every read of the exchange buffer is done
         if (S > 1 && te < S) mbar_arrive_remote(&park_free, te);
       }
@@ -508,8 +543,8 @@ int wide_do(WideOp op, dyb200_ctx* ctx, int slot, const TmapPack* tm, const BwdW
     return fit;
   }
   GemmProfScope scope(ctx, flops, 2, a->M, REC ? a->B * a->T : a->columns, 4 * a->H, EPI_ACCUM_MASK);
-  if (REC && ctx->seq_coop >= 0) {
-    // all CTAs wait on one another: as many as fit at once (the plan), scheduled as one gang where the driver takes the attribute
+  if (REC && a->T > 1 && ctx->seq_coop >= 0) {
+    // all CTAs wait on one another (a single step's for none beside those of their cluster): as many as fit at once (the plan), scheduled as one gang where the driver takes the attribute
     attr[na].id = cudaLaunchAttributeCooperative;
     attr[na].val.cooperative = 1;
     cfg.numAttrs = na + 1;
@@ -519,6 +554,11 @@ int wide_do(WideOp op, dyb200_ctx* ctx, int slot, const TmapPack* tm, const BwdW
     if (ctx->seq_coop == 1) return dyb200_fail(ctx, DYB200_ECUDA, "backward recurrence: launch failed: %s", cudaGetErrorString(e));
     ctx->seq_coop = -1;
     cfg.numAttrs = na;
+  }
+  if (a->T == 1 && ctx->pdl) {   // (a single step's kernels are short: each one's prologue runs beside the one before)
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = na + 1;
   }
   cudaLaunchKernelEx(&cfg, kernel, *tm, *a);
   DYB_LAUNCHED(ctx);
@@ -601,8 +641,19 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
   if ((rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[0], wh.hi, H, K, wh.pitch, BM, false)) || (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[1], wh.lo, H, K, wh.pitch, BM, false)) ||
       (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[2], a.d16_hi, columns, 4 * Hp, 4 * Hp, kRecCols, false)) ||
       (rc = dyb200_tc_make_tmap_f16(ctx, &tm.t[3], a.d16_lo, columns, 4 * Hp, 4 * Hp, kRecCols, false))) return rc;
-  if ((rc = wide_rec(WIDE_LAUNCH, H, S, ctx, &tm, &a, dim3(tiles_m, (tiles_n + ncb - 1) / ncb, S), 2.0 * G * (double)H * B * a.P))) return rc;
-  if ((rc = dyb200_seq_db(ctx, a.part, T, tiles_n * S, G, q.db, a.done)) || !q.dx) return rc;
+  const dim3 grid(tiles_m, (tiles_n + ncb - 1) / ncb, S);
+  // A single step's cell pass is a launch of its own, and the product behind it polls no counter: a step's call depends on no CTA beside those of its
+  // cluster being on the GPU with it.  The bits are those of the sequence.  (us, a gang that does both and hands over through counters / so, each kernel's
+  // prologue beside the one before: 512 x 1024 x 64 columns 26.5 / 24.3, 512 x 512 x 64 24.5 / 19.7, 1024 x 1024 x 512 66.5 / 66.3.  As two launches of the
+  // recurrence kernel one after the other: 30.4, 29.5, 72.9.)
+  if (T == 1) {
+    dyb_launch(H % 4 == 0 ? k_bwd_cells<true> : k_bwd_cells<false>, dim3(tiles_m, tiles_n, S), 256, 0, ctx, a);
+    DYB_LAUNCHED(ctx);
+    if ((rc = dyb200_seq_db(ctx, a.part, 1, tiles_n * S, G, q.db, nullptr))) return rc;
+  }
+  if (a.P && (rc = wide_rec(WIDE_LAUNCH, H, S, ctx, &tm, &a, grid, 2.0 * G * (double)H * B * a.P))) return rc;
+  if (T > 1 && (rc = dyb200_seq_db(ctx, a.part, T, tiles_n * S, G, q.db, a.done))) return rc;
+  if (!q.dx) return DYB200_OK;
   // dx of all columns
   a.M = I; a.tiles_m = (I + BM - 1) / BM; a.columns = columns; a.dx = q.dx; a.mask = q.mx; a.mask_full = q.mx_full; a.wscale = wx.scale;
   // The form by what a round of tiles was measured to take.  All give the same bits, whatever the number of columns: chains are added in the order of

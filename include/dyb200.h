@@ -365,7 +365,8 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
                                 dyb200_tensor* dx_all, dyb200_tensor* dWx, dyb200_tensor* dWh, dyb200_tensor* db,
                                 struct dyb200_wgrad* deferred, uint32_t steps, dyb200_ctx* ctx);
 /* Sequence-persistent kernels (1, the default): 0 makes dyb200_vanilla_lstm_seq_* issue one call per time step; 2 keeps the
- * kernels but launches them without the cooperative-launch attribute (profilers that cannot replay cooperative launches). */
+ * kernels but launches them without the cooperative-launch attribute (profilers that cannot replay cooperative launches).
+ * The single-step calls are the same in all three: no CTA of theirs waits for one beside those of its own cluster. */
 int dyb200_ctx_sequence_kernels(dyb200_ctx* ctx, int enable);
 
 /* ---- A14 autobatch ragged movers (same argument meaning as dynet/gpu-ops.h:14-15;

@@ -124,3 +124,46 @@ def test_sequence_without_room_for_its_pairs(H, B):
         assert all(torch.equal(p, q) for p, q in zip(*outs))
     finally:
         g.ctx().wgrad_destroy(w)
+
+
+@pytest.mark.parametrize("I,H,B", [(96, 1024, 64), (33, 448, 100), (9, 777, 500)])
+def test_single_step_waits_for_no_other_cluster(I, H, B):
+    """A single step's cell pass and the product behind it are launches of their own - one more than where the product is not wanted - so that no CTA waits for
+    one beside those of its cluster; the switch for the sequence kernels changes neither that nor the bits."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    gen = torch.Generator("cuda").manual_seed(H + B)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    x, c0, cs, gates = rnd(B, I), rnd(B, H), rnd(B, H), torch.sigmoid(rnd(B, 4 * H))
+    Wx, Wh, dh, dc, db0 = rnd(I, 4 * H) / H ** 0.5, rnd(H, 4 * H) / H ** 0.5, rnd(B, H), rnd(B, H), rnd(4 * H)
+    W, at = (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1)), capi.LstmGatesAttrs(0, 0.0, 1.0)
+    outs = []
+
+    def step(prev):
+        w = ctx.wgrad_create(4 * H, I, H, B)
+        ctx.wgrad_pack_inputs(w, g.T(x), None, B)
+        out = [torch.ones(B, n, device="cuda") for n in (I, H, H)] + [db0.clone()]
+        at0 = ctx.launches()
+        ctx.lstm_bwd_fused_at(g.T(x), g.T(c0), g.T(c0), *W, None, None, g.T(gates), g.T(cs), g.T(dh), g.T(dc), g.T(out[0]), g.T(out[1]) if prev else None, g.T(out[2]),
+                              None, None, g.T(out[3], [4 * H], 1), at, w, 0)
+        n = ctx.launches() - at0
+        torch.cuda.synchronize()
+        ctx.wgrad_destroy(w)
+        return n, out
+
+    ctx.param_cache(True)
+    try:
+        step(True)
+        for mode in (1, 2, 0):
+            ctx.sequence_kernels(mode)
+            with_product, out = step(True)
+            outs.append(out)
+            assert with_product == step(False)[0] + 1
+    finally:
+        ctx.sequence_kernels(1)
+        ctx.param_cache(False)
+    for out in outs[1:]:
+        assert all(torch.equal(p, q) for p, q in zip(outs[0], out))
+    assert ctx.device_errors() == 0
