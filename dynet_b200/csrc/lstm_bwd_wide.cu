@@ -396,7 +396,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
       float sum[kHalf];
 #pragma unroll
       for (uint32_t q = 0; q < kHalf; ++q) sum[q] = 0.f;
-      if (REC && nchains && ok && !mbar_wait(&go[cb], it & 1)) ok = false;
+      // (a share without k-blocks waits too: once the counter is up, the others are done with their exchange buffers as scratch for row sums)
+      if (REC && ok && !mbar_wait(&go[cb], it & 1)) ok = false;
 #pragma unroll 1
       for (uint32_t c = 0; c < nchains; ++c, ++cg) {
         const uint32_t buf = cg % kBufs;

@@ -34,3 +34,12 @@ def test_finds_the_kernels_that_talk_across_a_cluster():
 def test_waits_for_the_cluster_before_the_first_remote_access(where, name, body):
     wait = WAIT.search(body)
     assert wait and wait.start() < REMOTE.search(body).start()
+
+
+def test_wide_backward_sends_only_behind_the_counter():
+    """The exchange buffer of another CTA of the cluster is that CTA's scratch for row sums until it has published them, so every rank - one whose share of the
+    reduction is empty included - waits for its column block's counter (go[cb]) before the partial sums of a product go out."""
+    (body,) = [b for _, n, b in FOUND if n == "k_bwd_wide"]
+    send = body.index("send4(")
+    conditions = re.findall(r"if \(([^;{}]*mbar_wait\(&go\[cb\], it & 1\))\)", body[:send])
+    assert conditions == ["REC && ok && !mbar_wait(&go[cb], it & 1)"]
