@@ -2028,6 +2028,7 @@ int dyb200_wgrad_reserve(dyb200_wgrad* w, uint32_t k, float** a_hi, float** a_lo
   w->kb = w->k;
   return DYB200_OK;
 }
+void dyb200_wgrad_unreserve(dyb200_wgrad* w, uint32_t k) { w->k -= k; w->kb = w->k; }
 // Explicit column positions, for callers that fill the B operands (the layer inputs) during the forward pass and the A
 // operand (the gate gradient) during the backward pass: step t of a sequence uses columns [t * k, (t + 1) * k) both times.
 int dyb200_wgrad_push_b_at(dyb200_wgrad* w, uint32_t col, uint32_t k, const float* b0, uint32_t ldb0, const float* mask0, int mask0_full,

@@ -710,7 +710,12 @@ int dyb200_vanilla_lstm_bwd_fused_at(const dyb200_tensor* x, const dyb200_tensor
     if (at_col) rc = dyb200_wgrad_reserve_a_at(deferred, deferred_col, B, &q.dn_hi, &q.dn_lo, &q.dn_pitch, ctx);
     else rc = dyb200_wgrad_reserve(deferred, B, &q.dn_hi, &q.dn_lo, &q.dn_pitch, x->v, I, mx, mx_full, h_tm1->v, H, mh, mh_full, ctx, &batch);
     if (rc || (rc = dyb200_tc_pack_flush(ctx, &batch))) return rc;
-    return dyb200_bwd_wide(ctx, q);
+    rc = dyb200_bwd_wide(ctx, q);
+    if (rc != DYB200_ENOMEM) return rc;
+    // no room for the pairs, nothing has been launched: the form below, whose scratch is smaller where the batch is larger than I + H
+    if (!at_col) dyb200_wgrad_unreserve(deferred, B);
+    dyb200_tc_pack_begin(&batch);
+    if ((rc = dyb200_scratch_begin(ctx))) return rc;
   }
   float* dpre = nullptr;
   if (tiled) {

@@ -167,3 +167,43 @@ def test_single_step_waits_for_no_other_cluster(I, H, B):
     for out in outs[1:]:
         assert all(torch.equal(p, q) for p, q in zip(outs[0], out))
     assert ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("append", [False, True])
+def test_single_step_without_room_for_its_pairs(append):
+    """Little device memory: a step's pairs (11 MB: 1000 columns of dgates, the weights) do not fit, the planes of the weights that the generic form needs (7 MB)
+    do - it runs, with the same values to the rounding of either form (2 x 11 bits, sums of 1792: 2e-6 each of a result's norm), and the accumulator holds the
+    step once."""
+    import contextlib
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    from test_gpu_scratch_limits import room_for
+    I, H, B = 32, 448, 1000
+    gen = torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    x, c0, cs, gates = rnd(B, I), rnd(B, H), rnd(B, H), torch.sigmoid(rnd(B, 4 * H))
+    Wx, Wh, dh, dc = rnd(I, 4 * H) / H ** 0.5, rnd(H, 4 * H) / H ** 0.5, rnd(B, H), rnd(B, H)
+    outs = []
+    spare = [torch.zeros(n, device="cuda") for n in (I * B, H * B, H * B, 4 * H * I, 4 * H * H, 4 * H)]   # (the generic form once with all the memory: its kernels are loaded)
+    g.ctx().lstm_bwd_fused(g.T(x), g.T(c0), g.T(c0), g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), None, None, g.T(gates), g.T(cs), g.T(dh), g.T(dc),
+                           *(g.T(t, [n], B) for t, n in zip(spare, (I, H, H))), g.T(spare[3], [4 * H, I], 1), g.T(spare[4], [4 * H, H], 1), g.T(spare[5], [4 * H], 1),
+                           capi.LstmGatesAttrs(0, 0.0, 1.0))
+    for c in (g.ctx(), None):
+        out = [torch.ones(B, n, device="cuda") for n in (I, H, H)] + [torch.zeros(n, 4 * H, device="cuda") for n in (1, I, H)]
+        w = g.ctx().wgrad_create(4 * H, I, H, B)
+        if not append:
+            g.ctx().wgrad_pack_inputs(w, g.T(x), None, B)
+        with contextlib.nullcontext(c) if c else room_for(11) as ctx:
+            ctx.lstm_bwd_fused_at(g.T(x), g.T(c0), g.T(c0), g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), None, None, g.T(gates), g.T(cs), g.T(dh), g.T(dc),
+                                  g.T(out[0]), g.T(out[1]), g.T(out[2]), None, None, g.T(out[3], [4 * H], 1), capi.LstmGatesAttrs(0, 0.0, 1.0), w,
+                                  ctx.WGRAD_APPEND if append else 0)
+        torch.cuda.synchronize()
+        if append:
+            g.ctx().wgrad_flush(w, out[4].data_ptr(), 4 * H, out[5].data_ptr(), 4 * H)
+        torch.cuda.synchronize()
+        g.ctx().wgrad_destroy(w)
+        outs.append(out)
+    for p, q in zip(*outs):
+        assert bool((p - q).double().norm() <= 4e-6 * p.double().norm())
+    assert not append or float(outs[0][5].abs().max()) > 1.0
