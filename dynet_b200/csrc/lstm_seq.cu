@@ -686,8 +686,10 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
   uint32_t S = 1, f16_bn;
   bool wide_fits = true;
   SeqPlanes pl;
-  // (wide layers.  Without an accumulator the inputs are x itself, and a sequence has to be worth making the weights' pairs for)
-  if (sequence && (deferred || (!attrs->dropout && T >= kRecMinSteps && I % 4 == 0)) && dyb200_seq_f16_plan(ctx, I, H, B, &f16_bn, &S) &&
+  // (wide layers.  Without an accumulator the inputs are x itself, and a sequence has to be worth making the weights' pairs for.  A short sequence of few
+  // columns keeps the step calls' own sums, plain fp32 there: gemm_thin.cu)
+  const bool short_thin = T < kRecMinSteps && dyb200_thin_columns(G, B, I + H);
+  if (sequence && !short_thin && (deferred || (!attrs->dropout && T >= kRecMinSteps && I % 4 == 0)) && dyb200_seq_f16_plan(ctx, I, H, B, &f16_bn, &S) &&
       (!deferred || dyb200_wgrad_seq_planes(deferred, T, B, &pl))) {
     { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
     if (deferred) DYB_CHECK_ARG(ctx, dyb200_wgrad_rows(deferred) == G, "lstm_seq_fwd: the deferred accumulator has %u rows, the layer %u", dyb200_wgrad_rows(deferred), G);

@@ -76,3 +76,35 @@ def test_sequence_that_does_not_fill_its_tiles(I, H, B, T, mask, acc):
         assert bool(((cs[t] - (i * gg + f * cp)).abs() <= 2e-7 * ((i * gg).abs() + (f * cp).abs())).all())
         assert bool(((hs[t] - o * torch.tanh(cs[t])).abs() <= 5e-7).all())
     assert ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("I,H,B,T,mask", [(64, 400, 9, 7, None), (300, 600, 30, 5, "full"), (31, 777, 12, 2, "one"), (512, 1024, 24, 5, None)])
+def test_short_sequence_of_few_columns(I, H, B, T, mask):
+    """Fewer than eight steps of up to 32 columns: bit for bit the step calls - plain fp32 where those are (up to 64 M multiply-adds), the wide form in the last row."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    gen = torch.Generator("cuda").manual_seed(H + B)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    x, h0, c0, b = rnd(T * B, I), rnd(B, H), rnd(B, H), rnd(4 * H) * 0.1
+    Wx, Wh = rnd(I, 4 * H) / I ** 0.5, rnd(H, 4 * H) / H ** 0.5
+    mB = B if mask == "full" else 1
+    mx, mh = [((torch.rand(mB, n, device="cuda", generator=gen) < 0.8) / 0.8).float() for n in (I, H)]
+    at, tm = capi.LstmGatesAttrs(1 if mask else 0, 0.0, 1.0), (g.T(mx), g.T(mh)) if mask else (None, None)
+    W, out = (g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1)), []
+    for single in (False, True):
+        w = ctx.wgrad_create(4 * H, I, H, T * B)
+        gates, cs, hs = (torch.empty(T * B, n, device="cuda") for n in (4 * H, H, H))
+        if single:
+            ctx.wgrad_pack_inputs(w, g.T(x, [I], T * B), tm[0], B)
+            for t in range(T):
+                sl, pr = slice(t * B, (t + 1) * B), slice((t - 1) * B, t * B)
+                ctx.lstm_fwd_fused_at(g.T(x[sl]), g.T(hs[pr] if t else h0), g.T(cs[pr] if t else c0), *W, *tm, at, g.T(gates[sl]), g.T(cs[sl]), g.T(hs[sl]), w, t * B)
+        else:
+            ctx.lstm_seq_fwd(g.T(x, [I], T * B), g.T(h0), g.T(c0), *W, *tm, at, g.T(gates, [4 * H], T * B), g.T(cs, [H], T * B), g.T(hs, [H], T * B), w, T)
+        torch.cuda.synchronize()
+        ctx.wgrad_destroy(w)
+        out.append((gates, cs, hs))
+    assert all(torch.equal(p, q) for p, q in zip(*out))
+    assert ctx.device_errors() == 0
