@@ -37,3 +37,26 @@ def test_products_of_pairs_made_in_one_pass(M, N, K, tA, tB, off):
     bar = 4.5e-7 * B.norm(dim=1)[:, None] * A.norm(dim=1)[None, :] + 1e-44
     assert bool(((Cm.double() - want).abs() <= bar).all())
     assert g.ctx().device_errors() == 0
+
+
+@pytest.mark.parametrize("M,N,K,tA,tB", [(1500, 3001, 1000, 1, 0), (600, 900, 8193, 1, 0), (4001, 4099, 257, 0, 1), (2001, 2003, 1024, 0, 1)])
+def test_infinities_and_nans_stay_in_their_row(M, N, K, tA, tB):
+    import torch
+    import gpu_util as g
+    gen = torch.Generator("cuda").manual_seed(M)
+    A, B = [torch.randn(r, K, device="cuda", generator=gen) for r in (M, N)]
+
+    def product(A, B):
+        a, b, C = A if tA else A.t().contiguous(), B if not tB else B.t().contiguous(), torch.empty(N, M, device="cuda")
+        g.ctx().gemm(tA, tB, M, N, K, a.data_ptr(), K if tA else M, b.data_ptr(), N if tB else K, C.data_ptr(), M, 0)
+        torch.cuda.synchronize()
+        return C
+
+    clean = product(A, B)
+    A2, B2 = A.clone(), B.clone()
+    A2[M - 1, 0], A2[130, K - 1], B2[N - 1, 3] = float("inf"), float("nan"), float("-inf")
+    got = product(A2, B2)
+    rows, cols = [r for r in range(M) if r not in (130, M - 1)], [n for n in range(N - 1)]
+    assert torch.equal(got[cols][:, rows], clean[cols][:, rows])
+    assert not bool(torch.isfinite(got[:, [130, M - 1]]).any()) and not bool(torch.isfinite(got[N - 1]).any())
+    assert g.ctx().device_errors() == 0

@@ -207,3 +207,109 @@ def test_single_step_without_room_for_its_pairs(append):
     for p, q in zip(*outs):
         assert bool((p - q).double().norm() <= 4e-6 * p.double().norm())
     assert not append or float(outs[0][5].abs().max()) > 1.0
+
+
+def _sweep(I, H, B, T, Wx, Wh, gates, cs, c0, dh_in, dc_in):
+    """The sequence call on copies of its gradients: dh, dc of all steps, dx, db."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    w = ctx.wgrad_create(4 * H, I, H, T * B)
+    dh, dc, dx, db = dh_in.clone(), dc_in.clone(), torch.zeros(T * B, I, device="cuda"), torch.zeros(4 * H, device="cuda")
+    x = torch.ones(T * B, I, device="cuda")
+    ctx.wgrad_pack_inputs(w, g.T(x, [I], T * B), None, B)
+    ctx.lstm_seq_bwd(g.T(x, [I], T * B), g.T(c0), g.T(c0), g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), None, None, capi.LstmGatesAttrs(0, 0.0, 1.0),
+                     g.T(gates, [4 * H], T * B), g.T(cs, [H], T * B), g.T(cs, [H], T * B), g.T(dh, [H], T * B), g.T(dc, [H], T * B), g.T(dx, [I], T * B),
+                     None, None, g.T(db, [4 * H], 1), w, T)
+    torch.cuda.synchronize()
+    ctx.wgrad_destroy(w)
+    assert ctx.device_errors() == 0
+    return dh, dc, dx, db
+
+
+def _dgates(gates, c, cp, dh, dc, H):
+    import torch
+    i, f, o, gg = gates.double().split(H, dim=1)
+    tc = torch.tanh(c.double())
+    d = dh.double() * o * (1 - tc * tc) + dc.double()
+    return torch.cat([d * gg * i * (1 - i), d * cp.double() * f * (1 - f), dh.double() * tc * o * (1 - o), d * i * (1 - gg * gg)], dim=1)
+
+
+# A pair's scale belongs to a column and 128 units of all gates (dgates) or to a row (weights).  Odd units have gradients 2^-e below the even ones; every third
+# row of the weights is zero at the even units, every third 2^-e smaller there than at the odd ones.  Bar of a result: 1.45e-6 * 1.25 (as above) of the sum of its
+# products' magnitudes - never more than |row| |column|, and all that a product or a truncated sum can be off by in proportion - and 2^-49 of a scale's
+# largest value times the other factor's sum: what lies 2^28 below a scale keeps an absolute error of 2^-50 of it, and its lo part meets no lo part, half of that again.
+@pytest.mark.parametrize("I,H,B", [(96, 512, 64), (100, 777, 33)])
+@pytest.mark.parametrize("e", [10, 20, 28, 30, 40, 50])
+def test_values_that_differ_within_a_scale(I, H, B, e):
+    import torch
+    T = 2
+    gen = torch.Generator("cuda").manual_seed(H + e)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    odd = torch.arange(H, device="cuda") % 2 == 1
+    weight = [torch.ones(H, device="cuda"), odd.float(), torch.where(odd, 1.0, 2.0 ** -e)]
+    Wx, Wh = [torch.stack([weight[j % 3] for j in range(n)]).repeat(1, 4) * rnd(n, 4 * H) / H ** 0.5 for n in (I, H)]
+    gates = torch.cat([torch.sigmoid(rnd(T * B, 3 * H)), torch.tanh(rnd(T * B, H))], dim=1)
+    cs, c0, small = rnd(T * B, H), rnd(B, H), torch.where(odd, 2.0 ** -e, 1.0)
+    dh_in, dc_in = rnd(T * B, H) * small, rnd(T * B, H) * small
+    dh, dc, dx, _ = _sweep(I, H, B, T, Wx, Wh, gates, cs, c0, dh_in, dc_in)
+    sl, pr = slice(B, 2 * B), slice(0, B)
+    dg = _dgates(gates[sl], cs[sl], cs[pr], dh[sl], dc[sl], H)
+    block = dg.abs().view(B, 4, H)
+    top = torch.cat([block[:, :, u:u + 128].amax(dim=(1, 2), keepdim=True).expand(-1, 4, min(128, H - u)) for u in range(0, H, 128)], dim=2).reshape(B, 4 * H)
+    for W, got, old in ((Wx, dx[sl], None), (Wh, dh[pr], dh_in[pr])):
+        W = W.double()
+        want = dg @ W.t() + (0 if old is None else old.double())
+        bar = 1.45e-6 * 1.25 * (dg.abs() @ W.abs().t()) + 2.0 ** -49 * (top @ W.abs().t() + dg.abs().sum(dim=1)[:, None] * W.abs().amax(dim=1)[None, :]) + 1.3e-7 * want.abs()
+        assert bool(((got - want).abs() <= bar).all()), float(((got - want).abs() / bar).max())
+
+
+@pytest.mark.parametrize("I,H,B", [(96, 512, 64), (100, 777, 33)])
+def test_gradients_that_fade_over_the_steps(I, H, B):
+    """2^-20 smaller with every step towards the first, 2^-80 in all; the bar is that of a single magnitude."""
+    import torch
+    T = 5
+    gen = torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    Wx, Wh = rnd(I, 4 * H) / H ** 0.5, rnd(H, 4 * H) / H ** 0.5 * 2.0 ** -20
+    gates = torch.cat([torch.sigmoid(rnd(T * B, 3 * H)), torch.tanh(rnd(T * B, H))], dim=1)
+    gates[:, H:2 * H] *= 2.0 ** -20
+    cs, c0, dh_in, dc_in = rnd(T * B, H), rnd(B, H), rnd(T * B, H), rnd(T * B, H)
+    dh_in[:-B] = 0.0
+    dc_in[:-B] = 0.0
+    dh, dc, dx, _ = _sweep(I, H, B, T, Wx, Wh, gates, cs, c0, dh_in, dc_in)
+    for t in range(T - 1, -1, -1):
+        sl, pr = slice(t * B, (t + 1) * B), slice((t - 1) * B, t * B)
+        dg = _dgates(gates[sl], cs[sl], cs[pr] if t else c0, dh[sl], dc[sl], H)
+        assert float(dh[sl].abs().max()) < 2.0 ** (5 - 18 * (T - 1 - t))
+        for W, got in ((Wx, dx[sl]), (Wh, dh[pr]))[:2 if t else 1]:
+            W = W.double()
+            assert bool(((got - dg @ W.t()).abs() <= 1.45e-6 * 1.25 * dg.norm(dim=1)[:, None] * W.norm(dim=1)[None, :]).all()), t
+
+
+@pytest.mark.parametrize("I,H,B", [(96, 512, 100), (2000, 777, 33)])
+def test_infinities_and_nans_stay_in_their_column_and_row(I, H, B):
+    import torch
+    T = 3
+    gen = torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    Wx, Wh = rnd(I, 4 * H) / H ** 0.5, rnd(H, 4 * H) / H ** 0.5
+    gates = torch.cat([torch.sigmoid(rnd(T * B, 3 * H)), torch.tanh(rnd(T * B, H))], dim=1)
+    cs, c0, dh_in, dc_in = rnd(T * B, H), rnd(B, H), rnd(T * B, H), rnd(T * B, H)
+    clean = _sweep(I, H, B, T, Wx, Wh, gates, cs, c0, dh_in, dc_in)
+    bad_h, bad_c = dh_in.clone(), dc_in.clone()
+    bad_h[2 * B + 5, 130], bad_h[2 * B + 31, 0], bad_c[B + 32, H - 1] = float("inf"), float("nan"), float("-inf")
+    dh, dc, dx, _ = _sweep(I, H, B, T, Wx, Wh, gates, cs, c0, bad_h, bad_c)
+    hit = torch.zeros(T, B, dtype=torch.bool, device="cuda")
+    hit[:, 5] = hit[:, 31] = hit[:2, 32] = True
+    for got, ref in zip((dh, dc, dx), clean):
+        assert torch.equal(got[~hit.view(-1)], ref[~hit.view(-1)])
+    assert not bool(torch.isfinite(dx[hit.view(-1)]).any())
+    Wx2, Wh2 = Wx.clone(), Wh.clone()
+    Wx2[7, 3 * H], Wx2[I - 1, 4 * H - 1], Wh2[200, 5] = float("inf"), float("nan"), float("-inf")   # rows 7 and I - 1 of dx; unit 200's dh, from step 1 down all of it
+    dh, dc, dx, _ = _sweep(I, H, B, T, Wx2, Wh2, gates, cs, c0, dh_in, dc_in)
+    rest = [r for r in range(I) if r not in (7, I - 1)]
+    assert torch.equal(dx[2 * B:, rest], clean[2][2 * B:, rest]) and not bool(torch.isfinite(dx[2 * B:, [7, I - 1]]).any())
+    units = [r for r in range(H) if r != 200]
+    assert torch.equal(dh[B:2 * B, units], clean[0][B:2 * B, units]) and not bool(torch.isfinite(dh[B:2 * B, 200]).any())

@@ -108,3 +108,41 @@ def test_short_sequence_of_few_columns(I, H, B, T, mask):
         out.append((gates, cs, hs))
     assert all(torch.equal(p, q) for p, q in zip(*out))
     assert ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("I,H,B,acc", [(96, 512, 100, True), (1100, 777, 40, True), (128, 512, 64, False)])
+def test_infinities_and_nans_stay_in_their_column_and_gate(I, H, B, acc):
+    """In a column of x and of h0, and in a gate row of Wx and of Wh (made into pairs in one pass, or in two above 1024 inputs)."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx, T = g.ctx(), 8
+    gen = torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    x, h0, c0, b, Wx, Wh = rnd(T * B, I), rnd(B, H), rnd(B, H), rnd(4 * H) * 0.1, rnd(I, 4 * H) / I ** 0.5, rnd(H, 4 * H) / H ** 0.5
+
+    def run(x, h0, Wx, Wh):
+        w = ctx.wgrad_create(4 * H, I, H, T * B) if acc else None
+        out = [torch.empty(T * B, n, device="cuda") for n in (4 * H, H, H)]
+        ctx.lstm_seq_fwd(g.T(x, [I], T * B), g.T(h0), g.T(c0), g.T(Wx, [4 * H, I], 1), g.T(Wh, [4 * H, H], 1), g.T(b, [4 * H], 1), None, None, capi.LstmGatesAttrs(0, 0.0, 1.0),
+                         g.T(out[0], [4 * H], T * B), g.T(out[1], [H], T * B), g.T(out[2], [H], T * B), w, T)
+        torch.cuda.synchronize()
+        if acc:
+            ctx.wgrad_destroy(w)
+        assert ctx.device_errors() == 0
+        return [o.view(T, B, -1) for o in out]
+
+    clean = run(x, h0, Wx, Wh)
+    x2, h2 = x.clone(), h0.clone()
+    x2[2 * B + 3, I - 1], h2[39, 0] = float("inf"), float("nan")
+    got = run(x2, h2, Wx, Wh)
+    hit = torch.zeros(T, B, dtype=torch.bool, device="cuda")
+    hit[2:, 3] = hit[:, 39] = True
+    for p, q in zip(got, clean):
+        assert torch.equal(p[~hit], q[~hit])
+    assert bool(torch.isnan(got[0][hit]).all())
+    Wx2, Wh2 = Wx.clone(), Wh.clone()
+    Wx2[5, H + 7], Wh2[H - 1, 4 * H - 1] = float("nan"), float("inf")    # a forget gate, the last unit's candidate
+    got = run(x, h0, Wx2, Wh2)
+    rest = [r for r in range(4 * H) if r not in (H + 7, 4 * H - 1)]
+    assert torch.equal(got[0][0][:, rest], clean[0][0][:, rest]) and bool(torch.isnan(got[0][0][:, H + 7]).all()) and not bool(torch.equal(got[0][0][:, -1], clean[0][0][:, -1]))
