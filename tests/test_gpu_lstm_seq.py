@@ -107,6 +107,8 @@ def _same(seq, per):
     (256, 256, 128, 4, True, False, True, True),      # 128 columns, batch-1 masks
     (256, 256, 256, 3, True, True, True, True),       # two blocks of them
     (300, 416, 128, 3, False, True, True, False),     # the last k-blocks partly filled
+    (64, 448, 1152, 2, True, True, True, True),       # more columns than the wide backward form takes: TF32 pairs above 384 units, four K splits
+    (640, 448, 1152, 2, False, True, True, True),     # ... and none
     (128, 256, 96, 3, True, True, False, False),       # 96 columns are not whole tiles: per-step calls inside
     (32, 64, 8, 3, True, True, False, False),          # far below the tensor path
 ])
