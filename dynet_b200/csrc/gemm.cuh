@@ -75,7 +75,7 @@ __device__ __forceinline__ void epi_emit_h(const GemmEpilogue& epi, uint32_t u, 
 // A TF32 hi / lo pair carries 2 x 11 significand bits.  fp16 has the same 11, at twice the rate of the tensor pipe and half the
 // bytes, with 5 bits of exponent.  So an operand row is scaled by a power of two that brings its largest
 // element to [2^14, 2^15), hi = fp16(x s), lo = fp16((x s - hi) 2^11): elements down to 2^-28 of the row's largest keep all
-// 2 x 11 bits, smaller ones an absolute error below 2^-51 of it.  Per k step: A_hi x [B_hi | B_lo] as ONE instruction of twice
+// 2 x 11 bits, smaller ones an absolute error below 2^-50 of it.  Per k step: A_hi x [B_hi | B_lo] as ONE instruction of twice
 // the columns (B_lo lies right behind B_hi in shared memory), whose halves are the accumulators D1 (hi hi) and D2, then
 // A_lo x B_hi into D2; the result is (D1 + 2^-11 D2) / (s_a s_b).  A chain of D1 is one third of the accumulations of the TF32
 // chain for the same K (the tensor core truncates at each), so chains are cut every 1024 of K here.

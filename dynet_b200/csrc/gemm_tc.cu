@@ -1951,7 +1951,7 @@ static bool wgrad_on_f16(const dyb200_wgrad* w) {
 // the steps leave that range, and dWx of a feature that is there in the first steps only would be made of what is left of them.  So the
 // passes that make the pairs also look at each row's blocks of eight columns: where one that is not all zero lies more than 2^kF16Span below
 // the row's largest value, a device word sends the flush back to the TF32 planes - the products of pairs end at once, and the grouped
-// product, which otherwise ends at once, adds its result.  So no element is further off than 2^-27 of the largest of its block.
+// product, which otherwise ends at once, adds its result.  So no element is further off than 2^-26 of the largest of its block.
 // The words and the empty launch cost 4 us of 66 (4096 x (1024 + 1024), K = 560) or 888 (K = 17920).
 static int wgrad_f16_planes(dyb200_ctx* ctx, const dyb200_wgrad* w, const PackedOp* ops, const bool* side, PackedOp* pairs, const uint32_t** wide) {
   F16Jobs jobs;

@@ -12,10 +12,16 @@
 // through everywhere, so a pair's scale belongs to (column, block of 128 units, all four gates) - what one warp of the cell pass holds.  The
 // reduction is ordered by these blocks (4 gates x 128 units = 8 k-blocks of 64), each one accumulation chain that is unscaled as it is drained.
 //
-// Measured (us per step of 35, all of a layer's backward call, I = H = 1024; TF32 pairs with dx inside the recurrence / this form): batch 512 48.2 / 30.5,
-// 256 35.8 / 17.9, 128 21.8 / 15.2, 64 16.6 / 9.9; batch 100 (a launch and more per step before) 31 / 14; 600 units, batch 30: 21 / 8; 777 units, batch 100
-// (a value at a time, the weights' gates moved apart so that a k-block's copy starts on 16 bytes): 37 / 10.5.  dx is 10 of
-// the 30.5, at 430 TFLOP/s useful.  What bounds the recurrence: at batch 512, two column blocks per CTA in turn (one block of 128 columns had nothing
+// What that costs a value: pairs have 2 x 11 bits down to 2^-28 of their scale's largest value and an absolute error of 2^-50 of it below; the TF32 pairs of the
+// form before had an exponent each.  A sum that only such small values reach loses bits (units 2^-40 of others of their block, the others' weights zero: 3e-4
+// instead of 2e-7).  Everywhere else the sums are the better ones - a third of the truncated accumulations: error of whole sequences against float64 (2-norm, before / here)
+// dh 3.1 - 4.1e-7 / 0.5 - 1.2e-7, dx 0.5 - 2.1e-6 / 2.5 - 5.9e-7, db 0.5 - 1.4e-6 / 1.2 - 4.8e-7, dWx and dWh 0.4 - 0.9 of before (1 - 1024 inputs, 385 - 1024 units,
+// 9 - 512 columns, weights as initialised).
+//
+// Measured (us per step of 35, all of a layer's backward call, I = H = 1024; TF32 pairs with dx inside the recurrence / this form): batch 512 48.2 / 29.5,
+// 256 35.8 / 17.3, 128 21.8 / 14.3, 64 16.6 / 9.2; batch 100 (a launch and more per step before) 31 / 14; 600 units, batch 30: 21 / 7.5; 777 units, batch 100
+// (a value at a time, the weights' gates moved apart so that a k-block's copy starts on 16 bytes): 37 / 10.2.  dx is 10 of
+// the 29.5, at 430 TFLOP/s useful.  What bounds the recurrence: at batch 512, two column blocks per CTA in turn (one block of 128 columns had nothing
 // to overlap its exchange and cell pass with: 25 us a step against 20), 196 MB of operands per step from L2 at 11 - 14 TB/s; at batch 64 the chain
 // itself: 0.5 until the first pairs of dgates are there, 2.8 for 8 k-blocks, 0.5 to drain the last, 1.2 exchange, 1.0 cell pass, 0.8 until the stores are
 // out and counted, 0.5 until the count is seen.
@@ -588,7 +594,9 @@ uint32_t k_blocks(uint32_t H) { return 8 * (H / BM) + (H % BM == 0 ? 0 : H % BM 
 }  // namespace
 
 // Column blocks per CTA and K splits: the fastest by what a product was measured to take - 0.36 us per k-block on the tensor pipe and 6 us from its last
-// MMA to the next step's first, which another block's MMAs overlap.
+// MMA to the next step's first, which another block's MMAs overlap (both from 1024 units).  The rule's edges, us per step, the forms before / this one: (64, 385, 9)
+// 37.8 / 8.2, (512, 385, 9) 20.3 / 8.2, (512, 416, 64) 21.2 / 7.4, (512, 448, 512) 26.6 / 13.1, (512, 777, 500) 81.5 / 31.7, (64, 1024, 1024) 58.5 / 49.9, (64, 2048, 1000) 164 / 127,
+// (64, 4096, 64) 107 / 78, (64, 4096, 500) 272 / 216; two steps with the weights' pairs made for them: (512, 512, 64) 24.4 / 23.7, (512, 385, 40) 33.0 / 27.1.
 bool dyb200_bwd_wide_plan(dyb200_ctx* ctx, uint32_t H, uint32_t B, uint32_t* ncb, uint32_t* S) {
   if (H <= 384 || B <= 8 || (H % 8 != 0 && 4 * H > kF16PadMax)) return false;
   const uint32_t tiles_m = (H + BM - 1) / BM, tiles_n = (B + kRecCols - 1) / kRecCols, kbs = k_blocks(H);

@@ -505,7 +505,8 @@ FwdKernel fwd_kernel(uint32_t kd, uint32_t n) {
 #undef REC_F
 #undef REC_F4
 }
-// (16 gate rows per lane: 255 registers at up to 256 units and threads, 168 at up to 320; fewer rows: up to 384 threads of 168)
+// (16 gate rows per lane: 255 registers at up to 256 units and threads, 168 at up to 320, where the instances of two and of three columns spill 48 and 28
+// bytes; fewer rows: up to 384 threads of 168)
 BwdKernel bwd_kernel(uint32_t kd, uint32_t n, uint32_t threads) {
 #define REC_B(K) (n == 1 ? k_lstm_rec_bwd<K, 1> : n == 2 ? k_lstm_rec_bwd<K, 2> : n == 3 ? k_lstm_rec_bwd<K, 4, 3> : k_lstm_rec_bwd<K, 4>)
   if (kd == 16 && threads > 256)

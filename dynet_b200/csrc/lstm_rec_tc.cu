@@ -17,8 +17,8 @@
 // warps that read the four gates of a group of columns exchange them through shared memory.  h_t goes to every CTA of the cluster as
 // fp16 pairs in the layout of the MMA's right operand, one bulk copy per CTA (messages of 16 bytes, st.async, moved 10 bytes per cycle:
 // 5000 cycles for 48 columns).  |h| < 1 and the largest dropout factor give one scale for the whole launch; an initial state has its own.
-// (Elements of h down to 2^-28 keep all their bits; smaller ones an absolute error below 2^-51, which is what rounding adds to any
-// pre-activation from 2^-27 up.)
+// (Elements of h down to 2^-28 keep all their bits; smaller ones an absolute error below 2^-50, which is what rounding adds to any
+// pre-activation from 2^-26 up.)
 // Backward: D (unit of h_{t-1} x column) = Wh_r^T dgates_r over the CTA's own 128 gate rows, partial sums to the unit's owner.  dgates
 // have no bound known in advance: a column's scale is the largest value of its 128 rows, found in the cell pass.
 #include "lstm_rec.cuh"

@@ -49,10 +49,11 @@ __device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return
 // instead of 2 x 0.66.  The weights' planes are MN-major as they lie, their rows interleaved like the TF32 ones; a scale per gate row of Wx and of Wh.
 // A column of x has a scale of its own, h .* mask_h one that is known beforehand (|h| < 1: the largest mask value of the column), h_{-1} the
 // larger of that and its own; so accumulation chains end between Wx x and Wh h, and a chain is unscaled as it is drained.  (Elements of h below 2^-28 of
-// the mask's largest value keep an absolute error of 2^-51 of it.)
+// the mask's largest value keep an absolute error of 2^-50 of it.)
 // grid = (4H / 128, B / BNT, S); with S > 1 the S CTAs of a tile are one thread-block cluster (1 x 1 x S).  S (1, 2, 4 or 8) is
 // a template parameter so that the column exchange indexes registers statically.
-// VEC: units in fours, on 16 bytes (otherwise, F16 and 64-column tiles only, a value at a time).
+// VEC: units in fours, on 16 bytes (otherwise, F16 only, a value at a time; those on 128-column tiles spill 464 - 592 bytes: 512 x 777 x 500 columns 23 us a
+// step, launch by launch 53).
 template <int BNT, uint32_t S, bool F16, bool VEC = true>
 __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_constant__ TmapPack tm, const SeqFwd a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -583,7 +584,12 @@ int layer_inputs(dyb200_ctx* ctx, dyb200_wgrad* deferred, const float* Wx, const
 // says: there is no other form, and another number of splits would give other bits.  Columns and units past the end of a tile are computed and
 // dropped: a launch and more per step, which such layers took before, was 19 us at (512, 1024, 100 columns), 25 at (300, 600, 30), 24 at (512, 768, 300),
 // 31 at (512, 1000, 100) and 18 at (256, 1024, 16); here it is 8.9, 7.1, 10.8, 8.9 and 7.1.  Units that do not come in fours have instantiations that
-// read and write a value at a time: 28 -> 10.1 at (512, 777, 100), 26 -> 8.0 at (300, 601, 30).
+// read and write a value at a time: 28 -> 10.1 at (512, 777, 100), 26 -> 8.0 at (300, 601, 30).  At the rule's edges, the forms before / here: (64, 385, 9) 12.0 / 8.8,
+// (512, 385, 40) 21.7 / 8.4, (512, 416, 64) 15.4 / 7.5 and (512, 448, 512) 15.3 / 10.0 (TF32 pairs in whole tiles there), (512, 2048, 256) 45.4 / 44.1,
+// (512, 4096, 64) 67.3 / 64.9, (64, 4736, 128) 91.1 / 90.3, (512, 1023, 500) 58.7 / 25.7; two steps with the weights' pairs made for them: (512, 512, 64) 28.0 / 21.7,
+// (512, 385, 40) 38.5 / 27.6, (64, 400, 9) 20.9 / 18.4.
+// Error of whole sequences against float64 (2-norm, forms before / here): gates 0.13 - 0.97 of what it was at 32 - 1024 inputs, 385 - 1024 units, 9 - 512 columns; with 1 - 16
+// inputs and at most 32 columns, all plain fp32 before, 1.00 - 1.03 (6.8e-8).
 bool dyb200_seq_f16_plan(dyb200_ctx* ctx, uint32_t I, uint32_t H, uint32_t B, uint32_t* bn, uint32_t* S) {
   if (H <= 384 || I == 0 || B <= 8) return false;
   const uint32_t sms = (uint32_t)ctx->sm_count, tiles_m = (H + 31) / 32, kb = (I + 63) / 64 + (H + 63) / 64;

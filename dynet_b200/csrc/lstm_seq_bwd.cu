@@ -21,6 +21,8 @@
 // sums of dgates added per step in tile order and the steps in sweep order (k_seq_db_reduce), the same k-blocks in the same
 // accumulation chains (cut every kChunkKB k-blocks), the same K splits (dyb200_lstm_bwd_tiling, which the per-step call
 // also asks) added in split order, the epilogue of the product kernels (epilogue_pass).
+//
+// Layers up to 384 units, and wider ones with more than 1024 columns (fewer: lstm_bwd_wide.cu), in whole 64 columns.
 #include "lstm_cell.cuh"
 #include "seq_dev.cuh"
 #include "lstm_rec_api.h"

@@ -321,16 +321,18 @@ int dyb200_wgrad_flush(dyb200_wgrad* w, float* C0, uint32_t ldc0, float* C1, uin
  * dyb200_vanilla_lstm_fwd_fused_at with deferred_col = t * batch, h_tm1 / c_tm1 = the previous step's outputs.
  *   * When the shape allows (deferred given, tensor-path sizes, whole tiles, every CTA resident at once) the steps run inside ONE
  *     kernel whose CTAs stay on the GPU for the whole sequence and hand h_t over through device memory: bit for bit the calls above.
- *     Above 384 units and eight columns (any number of either; deferred given, or at least 8 steps without masks) the products are of scaled fp16 pairs, as
- *     those of the single-step calls with an accumulator above 32 columns: a scale per gate row of Wx and of Wh and per column of x, and for a column of h
- *     the largest of its mask's values (1 without) and, in the first step, of h0.
+ *     Above 384 units and eight columns (units / 32 times columns / 128, each rounded up, at most the number of SMs - 512 columns at 1024 units, 256 at 2048;
+ *     deferred given, or at least 8 steps without masks) the products are of scaled fp16 pairs: a scale per gate row of Wx and of Wh and per column of x, and
+ *     for a column of h the largest of its mask's values (1 without) and, in the first step, of h0.  The single-step calls with an accumulator are the same
+ *     kernel and give the same bits, except with at most 32 columns and 64 M multiply-adds, where they are plain fp32: sequences of fewer than 8 steps make
+ *     those calls, longer ones agree with them to rounding.  What lies 2^28 below its scale keeps an absolute error of 2^-50 of it.
  *   * Other sequences of at least 8 steps of layers up to 384 units, or with at most 32 columns, form Wx x of all steps at once and
  *     keep only Wh h in the recurrence: the same values to the rounding of their sums, which associate differently, and the same
  *     bits from run to run.  Wh h is plain fp32 above 256 units, and below while there are at most four columns per cluster of
  *     CTAs (60 columns at 256 units, more for narrower layers); with more columns it is a product of scaled fp16 pairs, 2 x 11 bits as
  *     the TF32 pairs of the calls above have: Wh scaled by the largest value of each gate row, h by that of the initial state in
  *     the first step and by the largest mask value (1 without) after it (16 columns share them).
- *     What lies 2^28 below such a scale keeps an absolute error of 2^-51 of it, the rounding of a pre-activation of 2^-27.
+ *     What lies 2^28 below such a scale keeps an absolute error of 2^-50 of it, the rounding of a pre-activation of 2^-26.
  *   * Otherwise the calls above are made.  dyb200_ctx_sequence_kernels(ctx, 0) forces that.
  * h0 / c0 may lie on a step's columns of h_all / c_all (a text read piece by piece into the same buffers).  deferred may be NULL
  * (nothing recorded for the weight gradients). */
@@ -346,10 +348,12 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
  * deferred_col = t * batch.  dh_all / dc_all hold dE/dh_t and dE/dc_t of every
  * step as left by the layers above (the recurrent parts are accumulated into them on the way); dx_all accumulates.  With deferred the columns of the accumulator must hold the
  * layer inputs placed by dyb200_vanilla_lstm_seq_fwd / _fwd_fused_at, and dWx / dWh may be NULL; without it every step adds
- * its weight gradients to dWx / dWh at once.  Above 384 units and eight columns (any number of either, deferred given, at most 256 steps) Wh^T dgates alone
- * stays in the recurrence, one kernel for all steps, and dx of all columns is one product after it; the single-step calls run the same kernels for one step
+ * its weight gradients to dWx / dWh at once.  Above 384 units, with 9 to 1024 columns (deferred given, at most 256 steps, every CTA resident at once; up to
+ * 4096 units where they do not come in eights) Wh^T dgates alone
+ * stays in the recurrence, one kernel for all steps, and dx of all columns is one product after it; the single-step calls form the same products for one step
  * and give the same bits.  Both are products of scaled fp16 pairs: a scale per row of Wh^T and Wx^T, and one per column of dgates and block of 128 units (all
- * four gates).  Narrower layers: when the shape allows (as for the forward call; deferred and dx_all given), the
+ * four gates).  What lies 2^28 below its scale keeps an absolute error of 2^-50 of it: a sum that only such values reach - units 2^28 below others of their
+ * block, the others' weights zero - loses bits that pairs with an exponent per value have.  Narrower layers and larger batches: when the shape allows (as for the forward call; deferred and dx_all given), the
  * steps run inside ONE kernel whose CTAs stay on the GPU: the cell pass and the [Wx; Wh]^T dgates product of a step hand
  * over through counters in device memory, and every CTA alternates between two independent blocks of batch columns so that
  * one block's hand-overs hide behind the other's products (the per-step call uses the same K splits for such shapes, which
@@ -413,7 +417,7 @@ int dyb200_trainer_update(int rule, float* params, float* grads, float* state0, 
  * C[M x N] (+)= op(A) * op(B), column-major, fp32 in/out.  Up to 32 columns, and with a narrow side and a long one, on
  * the CUDA cores in fp32; else on the tensor pipe as three products of TF32 pairs or, from 24 GFLOP on (8 with K >= 256), of fp16
  * pairs whose rows of op(A) and columns of op(B) are scaled by their largest value (2 x 11 bits either way; an element more than 2^28 below that
- * value keeps an absolute error of 2^-51 of it, so an error is bounded by |row| |column|); shapes too small for that on the CUDA cores.  transA/transB as in BLAS. */
+ * value keeps an absolute error of 2^-50 of it, so an error is bounded by |row| |column|); shapes too small for that on the CUDA cores.  transA/transB as in BLAS. */
 #define DYB200_GEMM_A_IS_PARAM 1u /* flags: A is a parameter matrix (see dyb200_ctx_param_cache) */
 int dyb200_gemm(int transA, int transB, uint32_t M, uint32_t N, uint32_t K, const float* A,
                 uint32_t lda, const float* B, uint32_t ldb, float* C, uint32_t ldc, int accumulate,
