@@ -89,6 +89,8 @@ __device__ __forceinline__ uint32_t finite_mag(float v) {
   const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
   return u < 0x7f800000u ? u : 0u;
 }
+// Whether a magnitude loses bits to the scale of its row: it is not zero and lies 2^28 below the largest one.
+__device__ __forceinline__ bool pair_loses(uint32_t mag, uint32_t word) { return mag && (int)(mag >> 23) + 28 <= scale_field(word); }
 __device__ __forceinline__ float scale_of(uint32_t word) { return __int_as_float((268 - scale_field(word)) << 23); }
 __device__ __forceinline__ float inv_scale_of(uint32_t word) { return __int_as_float((scale_field(word) - 14) << 23); }   // 2^(E - 141)
 // v 2^(Ea + Eb - 282): in two factors, so that nothing overflows on the way to a result that does not
@@ -151,6 +153,7 @@ constexpr int kF16MaxJobs = 3;
 constexpr uint32_t kF16PadMax = 16384;
 struct F16Job { const float* src; uint32_t ld, lines, n, pitch; int mode; uint32_t* scale; __half* hi; __half* lo; const float* src_lo = nullptr;
   uint32_t perm_H = 0;        // (F16_ELEM) positions are gate rows q perm_H + u, written interleaved as dyb200_tc_param_gates does
+  uint32_t mark = 0;          // (F16_LINE) 1: four values side by side that all lose bits to their line's scale (pair_loses) become zeros, bit 0 of its word says so
   uint32_t pad_H = 0;         // (F16_LINE, lines of at most kF16PadMax values) values are gate units q pad_H + u, written at q (pad_H rounded up to 64) + u, zeros between
   uint32_t* low = nullptr; };   // (F16_ELEM) a word per position, see F16Jobs::wide
 // wide: becomes 1 where the values of a position span more than a pair holds: of its blocks of eight lines that are not all zero, one's largest
@@ -163,7 +166,7 @@ struct F16Jobs { F16Job job[kF16MaxJobs]; int n; uint32_t start[kF16MaxJobs + 1]
 int dyb200_f16_planes(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H = 0);
 int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs);
 // The same for a parameter, from the parameter cache when it is on.
-int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H = 0);
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H = 0, uint32_t mark = 0);
 PackedOp dyb200_f16_op(const F16Job& j, bool mn_major);
 // The gate weights of a layer, Wx (4H x I) and Wh (4H x H), as MN-major planes with interleaved rows (lines = their columns, 128 rows per 32 units) and one
 // scale word per row of Wx and one per row of Wh (4H words each, not interleaved); from the parameter cache when it is on.
@@ -176,7 +179,7 @@ int dyb200_f16_gates(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t
 inline bool dyb200_f16_takes(double flops, uint32_t K) { return flops >= 24.0e9 || (flops >= 8.0e9 && K >= 256); }
 // A queue of packing work that one kernel launch executes (several small operands per launch).
 constexpr int kMaxPackJobs = 8;
-constexpr int kLayoutGates = 2, kLayoutF16 = 3, kLayoutGatesF16 = 5, kLayoutPadF16 = 6;   // (kLayoutF16 + F16_LINE or F16_ELEM; kLayoutPadF16: F16Job::pad_H)
+constexpr int kLayoutGates = 2, kLayoutF16 = 3, kLayoutGatesF16 = 5, kLayoutPadF16 = 6, kLayoutMarkF16 = 7;   // (kLayoutF16 + F16_LINE or F16_ELEM; the last two: F16Job::pad_H, mark)
 struct PackJob {
   const float* src; const float* mask; float* hi; float* lo;
   uint32_t ld, rows, K, mask_ld, pitch, gx, perm_H;

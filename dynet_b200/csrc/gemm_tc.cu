@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const __grid_constant__ F16J
 #pragma unroll
     for (uint32_t k = 0; k < kWarpLines; ++k) {
       m[k] = __reduce_max_sync(0xffffffffu, m[k]);
-      if (lane == 0 && l0 + k < j.lines) j.scale[l0 + k] = m[k];
+      if (lane == 0 && l0 + k < j.lines) j.scale[l0 + k] = m[k] & ~j.mark;
     }
     return;
   }
@@ -874,6 +874,7 @@ __global__ void __launch_bounds__(256) k_f16_absmax(const __grid_constant__ F16J
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int w = 1; w < 8; ++w) m = max(m, red[w]);
+    m &= ~j.mark;
     if (us.x == 1) j.scale[line] = m; else atomicMax(j.scale + line, m);
   }
 }
@@ -957,7 +958,9 @@ __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jo
         s = make_float4(scale_of(__ldg(j.scale + min(e[k], top))), scale_of(__ldg(j.scale + min(e[k] + 1, top))), scale_of(__ldg(j.scale + min(e[k] + 2, top))), 1.f);
       }
     } else {
-      s.x = s.y = s.z = s.w = scale_of(__ldg(j.scale + line[k]));
+      const uint32_t word = __ldcg(j.scale + line[k]);   // (bit 0 may be set meanwhile)
+      s.x = s.y = s.z = s.w = scale_of(word);
+      if (j.mark && pair_loses(mag4(v[k]), word)) { v[k] = make_float4(0.f, 0.f, 0.f, 0.f); atomicOr(j.scale + line[k], 1u); }
     }
     uint2 hi, lo;
     split4_f16(v[k], s, hi, lo);
@@ -1043,6 +1046,14 @@ __device__ __forceinline__ void line_pairs(const F16Job& j, uint32_t line, uint3
     __syncthreads();
 #pragma unroll
     for (int w = 0; w < 8; ++w) m = max(m, red[w]);
+  }
+  if (j.mark) {
+    bool loses = false;
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k)
+      if (pair_loses(mag4(v[k]), m)) { v[k] = make_float4(0.f, 0.f, 0.f, 0.f); loses = true; }
+    loses = red ? __syncthreads_or(loses) : __any_sync(0xffffffffu, loses);
+    m = (m & ~1u) | loses;
   }
   if (e0 == 0) j.scale[line] = m;
   const float s = scale_of(m);
@@ -1209,7 +1220,7 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     else if (victim->hi && e->last_use < victim->last_use) victim = e;
   }
   dyb200_ctx::ParamPack* e = hit ? hit : victim;
-  const size_t floats = k_is_fast == kLayoutGatesF16 ? (size_t)(K + rows2) * pitch / 2 + 2 * rows : k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE || k_is_fast == kLayoutPadF16 ? rows : K) : (size_t)(rows + rows2) * pitch;
+  const size_t floats = k_is_fast == kLayoutGatesF16 ? (size_t)(K + rows2) * pitch / 2 + 2 * rows : k_is_fast >= kLayoutF16 ? (size_t)rows * pitch / 2 + (k_is_fast == kLayoutF16 + F16_LINE || k_is_fast >= kLayoutPadF16 ? rows : K) : (size_t)(rows + rows2) * pitch;
   if (!hit) {
     if (e->hi && e->floats < floats) {   // evicted entry is too small: its buffers may still be read by queued kernels
       DYB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1235,9 +1246,10 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
   } else if (e->version != ctx->param_version && k_is_fast >= kLayoutF16) {
     F16Jobs jobs;
     jobs.n = 1;
-    const bool pad = k_is_fast == kLayoutPadF16;
-    jobs.job[0] = F16Job{src, ld, rows, K, pitch, pad ? (int)F16_LINE : k_is_fast - kLayoutF16, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
+    const bool pad = k_is_fast == kLayoutPadF16, mark = k_is_fast >= kLayoutPadF16;
+    jobs.job[0] = F16Job{src, ld, rows, K, pitch, mark ? (int)F16_LINE : k_is_fast - kLayoutF16, reinterpret_cast<uint32_t*>(e->hi + (size_t)rows * pitch / 2), (__half*)e->hi, (__half*)e->lo};
     if (pad) jobs.job[0].pad_H = K / 4;
+    jobs.job[0].mark = mark;
     int rc = dyb200_f16_pack(ctx, &jobs);
     if (rc) return rc;
     e->version = ctx->param_version;
@@ -1322,18 +1334,19 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
-int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H) {
+int dyb200_f16_param(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t lines, uint32_t n, int mode, F16Job* job, uint32_t pad_H, uint32_t mark) {
   if (!ctx->param_cache_on) {
     F16Jobs jobs;
     jobs.n = 1;
     int rc = dyb200_f16_planes(ctx, src, ld, lines, n, mode, &jobs.job[0], pad_H);
+    jobs.job[0].mark = mark;
     if (!rc) rc = dyb200_f16_pack(ctx, &jobs);
     *job = jobs.job[0];
     return rc;
   }
   const uint32_t pitch = pad_H ? 4 * round_up(pad_H, 64) : round_up(n, 64);
   float *hi, *lo;
-  int rc = cached_param_pack(ctx, src, ld, pad_H ? kLayoutPadF16 : kLayoutF16 + mode, lines, n, pitch, &hi, &lo);
+  int rc = cached_param_pack(ctx, src, ld, pad_H ? kLayoutPadF16 : mark ? kLayoutMarkF16 : kLayoutF16 + mode, lines, n, pitch, &hi, &lo);
   if (rc) return rc;
   *job = F16Job{src, ld, lines, n, pitch, mode, reinterpret_cast<uint32_t*>(hi + (size_t)lines * pitch / 2), (__half*)hi, (__half*)lo};
   return DYB200_OK;

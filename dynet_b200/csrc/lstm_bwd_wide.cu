@@ -12,16 +12,17 @@
 // through everywhere, so a pair's scale belongs to (column, block of 128 units, all four gates) - what one warp of the cell pass holds.  The
 // reduction is ordered by these blocks (4 gates x 128 units = 8 k-blocks of 64), each one accumulation chain that is unscaled as it is drained.
 //
-// What that costs a value: pairs have 2 x 11 bits down to 2^-28 of their scale's largest value and an absolute error of 2^-50 of it below; the TF32 pairs of the
-// form before had an exponent each.  A sum that only such small values reach loses bits (units 2^-40 of others of their block, the others' weights zero: 3e-4
-// instead of 2e-7).  Everywhere else the sums are the better ones - a third of the truncated accumulations: error of whole sequences against float64 (2-norm, before / here)
+// A pair has 2 x 11 bits down to 2^-28 of its scale's largest value and an absolute error of 2^-50 of it below, where the TF32 pairs of the form before had an
+// exponent each.  Quads of values that lie that low are added in fp32 ("small quads" below): without them a sum that only such values reach - units 2^-40 of
+// others of their block, the others' weights zero - was off by 3e-4 of itself; looking for them costs 0.1 - 0.5 us a step.  Everywhere else the sums are better than
+// those of TF32 pairs, a third of the truncated accumulations: error of whole sequences against float64 (2-norm, before / here)
 // dh 3.1 - 4.1e-7 / 0.5 - 1.2e-7, dx 0.5 - 2.1e-6 / 2.5 - 5.9e-7, db 0.5 - 1.4e-6 / 1.2 - 4.8e-7, dWx and dWh 0.4 - 0.9 of before (1 - 1024 inputs, 385 - 1024 units,
 // 9 - 512 columns, weights as initialised).
 //
-// Measured (us per step of 35, all of a layer's backward call, I = H = 1024; TF32 pairs with dx inside the recurrence / this form): batch 512 48.2 / 29.5,
-// 256 35.8 / 17.3, 128 21.8 / 14.3, 64 16.6 / 9.2; batch 100 (a launch and more per step before) 31 / 14; 600 units, batch 30: 21 / 7.5; 777 units, batch 100
-// (a value at a time, the weights' gates moved apart so that a k-block's copy starts on 16 bytes): 37 / 10.2.  dx is 10 of
-// the 29.5, at 430 TFLOP/s useful.  What bounds the recurrence: at batch 512, two column blocks per CTA in turn (one block of 128 columns had nothing
+// Measured (us per step of 35, all of a layer's backward call, I = H = 1024; TF32 pairs with dx inside the recurrence / this form): batch 512 48.2 / 29.8,
+// 256 35.8 / 17.8, 128 21.8 / 14.6, 64 16.6 / 9.5; batch 100 (a launch and more per step before) 31 / 14; 600 units, batch 30: 21 / 7.6; 777 units, batch 100
+// (a value at a time, the weights' gates moved apart so that a k-block's copy starts on 16 bytes): 37 / 10.4.  dx is 10 of
+// the 29.8, at 430 TFLOP/s useful.  What bounds the recurrence: at batch 512, two column blocks per CTA in turn (one block of 128 columns had nothing
 // to overlap its exchange and cell pass with: 25 us a step against 20), 196 MB of operands per step from L2 at 11 - 14 TB/s; at batch 64 the chain
 // itself: 0.5 until the first pairs of dgates are there, 2.8 for 8 k-blocks, 0.5 to drain the last, 1.2 exchange, 1.0 cell pass, 0.8 until the stores are
 // out and counted, 0.5 until the count is seen.
@@ -41,8 +42,9 @@ struct BwdWide {
   float *dh_prev, *dc_prev;         // those of the step before the first (null: not wanted)
   float *dn_hi, *dn_lo; uint32_t dn_pitch;       // TF32 planes of dgates for the weight gradients: row = column of the sequence
   __half *d16_hi, *d16_lo;          // fp16 pairs, row = column of the sequence, gate q's unit u at q Hp + u (zeros from H on)
-  uint32_t* dsc; uint32_t dsc_ld;   // scale words [block of 128 units][column of the sequence]
-  const uint32_t* wscale;           // of the rows of Wh^T (dx: Wx^T)
+  uint32_t* dsc; uint32_t dsc_ld;   // scale words [block of 128 units][column of the sequence]; bit 0: small quads
+  const float* W;                   // Wh (dx: Wx)
+  const uint32_t* wscale;           // of the rows of W^T; bit 0: small quads
   float* part;                      // row sums of dgates: [step in sweep order][column block, rank][4H]
   const float* mask; int mask_full; // of the result's rows; full: one column per batch column
   float* dx; uint32_t columns;      // dx only
@@ -77,10 +79,94 @@ __device__ __forceinline__ void cell_load(const BwdWide& a, const CellUnits& q, 
   in.dci = a.dc ? ldu_cg<VEC>(a.dc + (size_t)t * HB + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
   in.dcp = dcp ? ldu_cg<VEC>(dcp + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
+template <bool VEC>
+__device__ __forceinline__ void planes_out(const BwdWide& a, const CellUnits& q, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dgates for the weight gradients
+  const size_t o = ((size_t)t * a.B + n) * a.dn_pitch + q.u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float4 hi, lo;
+    split_tf32(p[k].x, hi.x, lo.x); split_tf32(p[k].y, hi.y, lo.y); split_tf32(p[k].z, hi.z, lo.z); split_tf32(p[k].w, hi.w, lo.w);
+    stu<VEC>(a.dn_hi + o + (size_t)k * a.H, hi, q.left); stu<VEC>(a.dn_lo + o + (size_t)k * a.H, lo, q.left);
+  }
+}
+// Small quads: four neighbouring units' gradients of a gate, or four weights of a row side by side, that are not all zero and all lie 2^28 below the largest
+// value of their scale, so that pairs would keep little of them.  They are zeros in the pairs, bit 0 of the scale's word tells of them, and the warp that
+// finishes a column adds their products in fp32, from the planes of dgates for the weight gradients (small_parts).  So no value is further off than 2^-22 of
+// the largest of its quad, whatever else shares its scale.  The rule of the flush, there a row's blocks of eight columns, for the same reason.
+__device__ __forceinline__ uint32_t quad_mag(float4 v) { return max(max(finite_mag(v.x), finite_mag(v.y)), max(finite_mag(v.z), finite_mag(v.w))); }
+// What the cell pass does besides where it finds one (small), or the weights have some: the column's planes go out before they are published, and the pairs again.
+template <bool VEC>
+__device__ __forceinline__ void cell_small(const BwdWide& a, CellUnits q, float4 p0, float4 p1, float4 p2, float4 p3, uint32_t t, uint32_t n, uint32_t word) {
+  if (!q.own) return;
+  const float4 p[4] = {p0, p1, p2, p3};
+  planes_out<VEC>(a, q, p, t, n);
+  if (!word) return;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float v[4], h, l;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { split_tf32((&p[k].x)[i], h, l); v[i] = h + l; }   // (what small_parts will see)
+    if (!pair_loses(quad_mag(make_float4(v[0], v[1], v[2], v[3])), word)) continue;
+    const size_t o = (((size_t)t * a.B + n) * 4 + k) * a.Hp + q.u;
+    *reinterpret_cast<uint2*>(a.d16_hi + o) = *reinterpret_cast<uint2*>(a.d16_lo + o) = make_uint2(0, 0);
+  }
+}
+// Quad of gate k from unit u on, of a column's planes (zeros past the last unit)
+__device__ __forceinline__ float4 quad_of(const BwdWide& a, const float* hi, const float* lo, uint32_t k, uint32_t u) {
+  float v[4];
+#pragma unroll
+  for (uint32_t i = 0; i < 4; ++i) v[i] = u + i < a.H ? __ldcg(hi + k * a.H + u + i) + __ldcg(lo + k * a.H + u + i) : 0.f;
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+// The products of the small quads of column r (of the sequence) and of rows [m, + 4); a warp.
+__device__ __noinline__ float4 small_parts(const BwdWide& a, uint32_t r, uint32_t m) {
+  const uint32_t lane = threadIdx.x & 31, G = 4 * a.H;
+  const float *hi = a.dn_hi + (size_t)r * a.dn_pitch, *lo = a.dn_lo + (size_t)r * a.dn_pitch;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (uint32_t b = 0; b * BM < a.H; ++b) {
+    const uint32_t word = __ldcg(a.dsc + (size_t)b * a.dsc_ld + r);
+    if (!(word & 1)) continue;
+    float4 v[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) v[k] = quad_of(a, hi, lo, k, b * BM + 4 * lane);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+      for (uint32_t left = __ballot_sync(0xffffffffu, pair_loses(quad_mag(v[k]), word)); left; left &= left - 1) {
+        const uint32_t src = __ffs(left) - 1, u = b * BM + 4 * src;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+          const float x = __shfl_sync(0xffffffffu, (&v[k].x)[i], src);
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j)
+            if (u + i < a.H && m + j < a.M) acc[j] = fmaf(__ldg(a.W + k * a.H + u + i + (size_t)G * (m + j)), x, acc[j]);
+        }
+      }
+  }
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j)
+    for (uint32_t left = __ballot_sync(0xffffffffu, m + j < a.M && (__ldg(a.wscale + m + j) & 1)); left; left &= left - 1) {
+      const uint32_t src = __ffs(left) - 1, row = __shfl_sync(0xffffffffu, m, src) + j, word = __ldg(a.wscale + row);
+      const float* w = a.W + (size_t)G * row;
+      float sum = 0.f;
+      for (uint32_t e = 4 * lane; e < G; e += 128) {   // (G is a multiple of four)
+        const float4 x = make_float4(__ldg(w + e), __ldg(w + e + 1), __ldg(w + e + 2), __ldg(w + e + 3));
+        if (!pair_loses(quad_mag(x), word)) continue;
+        for (uint32_t i = 0; i < 4; ++i) {
+          const uint32_t k = (e + i) / a.H, u = (e + i) % a.H;
+          const float4 v = quad_of(a, hi, lo, k, u / 4 * 4);
+          if (!pair_loses(quad_mag(v), __ldcg(a.dsc + (size_t)(u / BM) * a.dsc_ld + r))) sum = fmaf((&x.x)[i], (&v.x)[u % 4], sum);   // (else it has been added above)
+        }
+      }
+      sum = warp_sum(sum);
+      if (lane == src) acc[j] += sum;
+    }
+  return make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
 // The cell pass of units [u, + 4), column n of step t from dE/dh: dE/dc of the step before, and dgates as fp16 pairs with the word of the warp's
 // (column, block).  The four gates' gradients come back in p and are added to rs.  (All lanes of a warp take part; those past the last unit with zeros.)
-__device__ __forceinline__ void cell(const BwdWide& a, const CellUnits& q, CellIn& in, float4 dh, uint32_t t, uint32_t n, float4 (&p)[4], float4 (&rs)[4]) {
-  uint32_t m = 0;
+// Returns its word where there are small quads, else 0.
+__device__ __forceinline__ uint32_t cell(const BwdWide& a, const CellUnits& q, CellIn& in, float4 dh, uint32_t t, uint32_t n, float4 (&p)[4], float4 (&rs)[4]) {
+  uint32_t m = 0, low = 0xffffffffu;   // the largest magnitude, and that of the smallest quad that is not zero, less one
 #pragma unroll
   for (int k = 0; k < 4; ++k) p[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (q.own) {
@@ -92,13 +178,14 @@ __device__ __forceinline__ void cell(const BwdWide& a, const CellUnits& q, CellI
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      m = max(m, max(max(finite_mag(p[k].x), finite_mag(p[k].y)), max(finite_mag(p[k].z), finite_mag(p[k].w))));
+      const uint32_t w = quad_mag(p[k]);
+      m = max(m, w);
+      low = min(low, w - 1);
       rs[k].x += p[k].x; rs[k].y += p[k].y; rs[k].z += p[k].z; rs[k].w += p[k].w;
     }
   }
   m = __reduce_max_sync(0xffffffffu, m);
   const size_t r = (size_t)t * a.B + n;
-  if ((threadIdx.x & 31) == 0) a.dsc[(size_t)q.blk * a.dsc_ld + r] = m;
   const float s = scale_of(m);
   if (q.u < a.Hp) {
 #pragma unroll
@@ -110,19 +197,16 @@ __device__ __forceinline__ void cell(const BwdWide& a, const CellUnits& q, CellI
       *reinterpret_cast<uint2*>(a.d16_lo + o) = *reinterpret_cast<const uint2*>(lo);
     }
   }
+  const uint32_t small = __any_sync(0xffffffffu, pair_loses(low + 1, m));
+  if ((threadIdx.x & 31) == 0) a.dsc[(size_t)q.blk * a.dsc_ld + r] = (m & ~1u) | small;
+  return small ? m | 1u : 0u;
 }
 template <bool VEC>
-__device__ __forceinline__ void cell_rest(const BwdWide& a, const CellUnits& q, const CellIn& in, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dE/dc of the step before, dgates for the weight gradients
+__device__ __forceinline__ void cell_rest(const BwdWide& a, const CellUnits& q, const CellIn& in, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dE/dc of the step before, the planes
   if (!q.own) return;
   float* dcp = t ? a.dc + (size_t)(t - 1) * a.H * a.B : a.dc_prev;
   if (dcp) stu<VEC>(dcp + (size_t)n * a.H + q.u, in.dcp, q.left);
-  const size_t o = ((size_t)t * a.B + n) * a.dn_pitch + q.u;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float4 hi, lo;
-    split_tf32(p[k].x, hi.x, lo.x); split_tf32(p[k].y, hi.y, lo.y); split_tf32(p[k].z, hi.z, lo.z); split_tf32(p[k].w, hi.w, lo.w);
-    stu<VEC>(a.dn_hi + o + (size_t)k * a.H, hi, q.left); stu<VEC>(a.dn_lo + o + (size_t)k * a.H, lo, q.left);
-  }
+  planes_out<VEC>(a, q, p, t, n);
 }
 // The row sums of a CTA's columns in a step (part: those of its column block and rank), through 4096 floats of shared memory: the eight warps' columns
 // in order.  te: thread of the 256.
@@ -165,7 +249,8 @@ __global__ void __launch_bounds__(256) k_bwd_cells(const __grid_constant__ BwdWi
     CellIn in = {};
     float4 dh = make_float4(0.f, 0.f, 0.f, 0.f), p[4];
     if (un.own) { cell_load<VEC>(a, un, in, 0, n); dh = ldu<VEC>(a.dh + (size_t)n * a.H + u, un.left); }
-    cell(a, un, in, dh, 0, n, p, rs);
+    const uint32_t word = cell(a, un, in, dh, 0, n, p, rs);
+    if (word) cell_small<VEC>(a, un, p[0], p[1], p[2], p[3], 0, n, word);
     cell_rest<VEC>(a, un, in, p, 0, n);
   }
   row_sums(a, rs, park, part_of(a, 0, blockIdx.y, gridDim.z, blockIdx.z), blockIdx.x, threadIdx.x, ew, 4 * (threadIdx.x & 31), true);
@@ -340,6 +425,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
       for (int q = 0; q < 4; ++q) rs[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     };
 
+    bool planes = false;   // small quads among the weights: the others look into the planes of every column
+    if (REC && a.T > 1) {
+      for (uint32_t k = te; k < a.M; k += 256) planes = planes || (__ldg(a.wscale + k) & 1);
+      planes = !bar_and(1, 256, !planes);
+    }
     for (uint32_t cb = 0; REC && a.T > 1 && cb < nblocks; ++cb) {   // the cell pass of the last step (of a single one: k_bwd_cells)
       const uint32_t t = a.T - 1, n0 = (block0 + cb) * BNT;
       clear_sums();
@@ -352,7 +442,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
           CellIn in = {};
           float4 dh = make_float4(0.f, 0.f, 0.f, 0.f), p[4];
           if (own_u) { cell_load<VEC>(a, un, in, t, n); dh = ldu<VEC>(a.dh + (size_t)t * HB + (size_t)n * a.H + u, left); }
-          cell(a, un, in, dh, t, n, p, rs);
+          const uint32_t word = cell(a, un, in, dh, t, n, p, rs);
+          if (word) cell_small<VEC>(a, un, p[0], p[1], p[2], p[3], t, n, word);
           cell_rest<VEC>(a, un, in, p, t, n);
         }
       row_sums(a, rs, park, part_of(a, 0, block0 + cb, S, rank), blockIdx.x, te, ew, uq, ok);
@@ -360,6 +451,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
     if (REC && a.T > 1)   // (all blocks at the end: the exchange buffer belongs to the others from the first one on)
       for (uint32_t cb = 0; cb < nblocks; ++cb) publish(cb);
 
+    auto rows_of = [&](uint32_t m) {   // whether there are small quads among the weights of rows [m, + 4)
+      uint32_t w = 0;
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) w |= m + q < a.M ? __ldg(a.wscale + m + q) : 0u;
+      return w & 1;
+    };
+    uint32_t small_rows = REC ? rows_of(u) : 0u;
     float row_f = REC ? inv_scale_of(blockIdx.x * BM + row < a.M ? __ldg(a.wscale + blockIdx.x * BM + row) : 0x3f800000u) : 1.f;
 #pragma unroll 1
     for (uint32_t it = item0; it < a.P; it += item_step)
@@ -373,6 +471,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
       float* const dst = REC ? (t ? a.dh + (size_t)(t - 1) * HB : a.dh_prev) : a.dx;
       const uint32_t m = m0 + uq;
       const bool own = m < a.M, vec = REC || ((a.M & 3) == 0 && aligned16(a.dx) && aligned16(a.mask));
+      if (!REC) small_rows = rows_of(m);
       if (!REC) row_f = inv_scale_of(m0 + row < a.M ? __ldg(a.wscale + m0 + row) : 0x3f800000u);
       if (REC && t) {   // what the cell pass will read from HBM is asked for now (a request per 128-byte line)
         if (own_u && (te & 7) == 0) {
@@ -404,6 +503,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
       for (uint32_t q = 0; q < kHalf; ++q) sum[q] = 0.f;
       // (a share without k-blocks waits too: once the counter is up, the others are done with their exchange buffers as scratch for row sums)
       if (REC && ok && !mbar_wait(&go[cb], it & 1)) ok = false;
+      // (the words of the columns that this warp finishes: looked at once the partial sums are on their way)
+      uint32_t words[KC * BNT / 64];
+#pragma unroll
+      for (uint32_t k = 0; k < KC * BNT / 64; ++k) {
+        const uint32_t n = col0 + column(k / KC, k % KC);
+        words[k] = ok && n < cols && lane * BM < a.H ? __ldcg(a.dsc + (size_t)lane * a.dsc_ld + seq0 + n) : 0u;
+        if (a.H > 32 * BM && ok && n < cols) for (uint32_t b = lane + 32; b * BM < a.H; b += 32) words[k] |= __ldcg(a.dsc + (size_t)b * a.dsc_ld + seq0 + n);
+      }
 #pragma unroll 1
       for (uint32_t c = 0; c < nchains; ++c, ++cg) {
         const uint32_t buf = cg % kBufs;
@@ -434,6 +541,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
       if (REC) clear_sums();
 #pragma unroll
       for (int hh = 0; hh < BNT / 64; ++hh) {
+        uint32_t any = small_rows;
+#pragma unroll
+        for (uint32_t k = 0; k < KC; ++k) any |= words[KC * hh + k];
+        const bool quads = __any_sync(0xffffffffu, any & 1);
         // ---- partial sums to the ranks that finish them ----
         if (S > 1 && ok && !mbar_wait_cluster(&park_free, pr_phase ^ 1)) ok = false;
         if (S > 1) {
@@ -449,15 +560,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
           for (uint32_t q = 0; q < 32; ++q) park[park_at(32 * half + q, row >> 2) + (row & 3)] = sum[32 * hh + q];
         }
         const bool last_pass = hh == BNT / 64 - 1;
+        if (quads) {   // ---- the products of small quads, into what these columns are added to ----
+#pragma unroll 1
+          for (uint32_t k = 0; k < KC; ++k) {
+            const uint32_t n = col0 + column(hh, k);
+            if (n >= cols || !ok) continue;   // (the same for a whole warp)
+            const float4 x = small_parts(a, seq0 + n, m);
+            for (uint32_t q = 0; q < 4 && m + q < a.M; ++q) {
+              float* d = dst + (size_t)n * a.M + m + q;
+              *d = __fmaf_rn((&x.x)[q], a.mask ? a.mask[m + q + (a.mask_full ? (size_t)(REC ? n : n % a.B) * a.M : 0)] : 1.f, __ldcg(d));
+            }
+          }
+        }
 #pragma unroll 1
         for (uint32_t kb = 0; kb < KC; kb += GB) {
           CellIn in[GB];
           float4 old[GB], mk[GB], p[GB][4];
-          uint32_t n[GB];
+          uint32_t n[GB], word[GB];
 #pragma unroll
           for (uint32_t g = 0; g < GB; ++g) {   // everything that comes from memory, before the wait
             n[g] = col0 + column(hh, kb + g);
             in[g] = CellIn{};
+            word[g] = 0;
             mk[g] = make_float4(1.f, 1.f, 1.f, 1.f);
             old[g] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (!own || n[g] >= cols || !vec) continue;
@@ -487,12 +611,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
               else v = make_float4(v.x + old[g].x, v.y + old[g].y, v.z + old[g].z, v.w + old[g].w);
             }
             old[g] = v;
-            if (REC && t && ok) cell(a, un, in[g], v, t - 1, n[g], p[g], rs);
+            if (REC && t && ok) word[g] = cell(a, un, in[g], v, t - 1, n[g], p[g], rs);
             if (vec || !own || !ok) continue;
             for (uint32_t q = 0; q < 4 && m + q < a.M; ++q) {
               float* d = dst + (size_t)n[g] * a.M + m + q;
               *d = __fmaf_rn((&v.x)[q], a.mask ? a.mask[m + q + (a.mask_full ? (size_t)(n[g] % a.B) * a.M : 0)] : 1.f, *d);
             }
+          }
+          if (REC && t && ok) {
+#pragma unroll
+            for (uint32_t g = 0; g < GB; ++g)
+              if ((word[g] || planes) && n[g] < cols) cell_small<VEC>(a, un, p[g][0], p[g][1], p[g][2], p[g][3], t - 1, n[g], word[g]);
           }
           if (REC && t && last_pass && kb + GB >= KC) {
             bar_sync(1, 256);   // all stores of the pairs and their words are issued; what nobody waits for goes out behind them
@@ -633,8 +762,8 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
       (rc = dyb200_scratch(ctx, (size_t)T * tiles_n * S * G * sizeof(float), &part))) return rc;
   // (a k-block's copy starts at a gate's units: on 16 bytes as the weights lie, or with the gates moved apart)
   const uint32_t pad = H % 8 == 0 ? 0 : H, K = pad ? 4 * Hp : G;
-  if ((rc = dyb200_f16_param(ctx, q.Wh, G, H, G, F16_LINE, &wh, pad))) return rc;
-  if (q.dx && (rc = dyb200_f16_param(ctx, q.Wx, G, I, G, F16_LINE, &wx, pad))) return rc;
+  if ((rc = dyb200_f16_param(ctx, q.Wh, G, H, G, F16_LINE, &wh, pad, 1))) return rc;
+  if (q.dx && (rc = dyb200_f16_param(ctx, q.Wx, G, I, G, F16_LINE, &wx, pad, 1))) return rc;
   BwdWide a;
   memset(&a, 0, sizeof(a));
   a.T = T; a.B = B; a.H = H; a.Hp = Hp; a.Ha = pad ? Hp : H; a.kbs = k_blocks(H); a.P = T - 1 + (q.dh_prev ? 1 : 0); a.M = H; a.tiles_m = tiles_m;
@@ -642,7 +771,7 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
   a.gates = q.gates; a.cs = q.c; a.c0 = q.c0; a.dh = q.dh; a.dc = q.dc; a.dh_prev = q.dh_prev; a.dc_prev = q.dc_prev;
   a.dn_hi = q.dn_hi; a.dn_lo = q.dn_lo; a.dn_pitch = q.dn_pitch;
   a.d16_hi = (__half*)p16; a.d16_lo = a.d16_hi + plane;
-  a.dsc = (uint32_t*)words; a.dsc_ld = columns; a.wscale = wh.scale; a.part = (float*)part;
+  a.dsc = (uint32_t*)words; a.dsc_ld = columns; a.W = q.Wh; a.wscale = wh.scale; a.part = (float*)part;
   a.mask = q.mh; a.mask_full = q.mh_full;
   a.done = ctx->dev_flags + DYB200_DEV_BWD0; a.flags = ctx->dev_flags;
   TmapPack tm;
@@ -664,7 +793,7 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
   if (T > 1 && (rc = dyb200_seq_db(ctx, a.part, T, tiles_n * S, G, q.db, a.done))) return rc;
   if (!q.dx) return DYB200_OK;
   // dx of all columns
-  a.M = I; a.tiles_m = (I + BM - 1) / BM; a.columns = columns; a.dx = q.dx; a.mask = q.mx; a.mask_full = q.mx_full; a.wscale = wx.scale;
+  a.M = I; a.tiles_m = (I + BM - 1) / BM; a.columns = columns; a.dx = q.dx; a.mask = q.mx; a.mask_full = q.mx_full; a.W = q.Wx; a.wscale = wx.scale;
   // The form by what a round of tiles was measured to take.  All give the same bits, whatever the number of columns: chains are added in the order of
   // the blocks of units.  (1024 x 64 of a single step: 17 us with two CTAs per tile, 9 with
   // eight; 1024 x 17 920: 350 on 128-column tiles.)

@@ -352,8 +352,8 @@ int dyb200_vanilla_lstm_seq_fwd(const dyb200_tensor* x_all, const dyb200_tensor*
  * 4096 units where they do not come in eights) Wh^T dgates alone
  * stays in the recurrence, one kernel for all steps, and dx of all columns is one product after it; the single-step calls form the same products for one step
  * and give the same bits.  Both are products of scaled fp16 pairs: a scale per row of Wh^T and Wx^T, and one per column of dgates and block of 128 units (all
- * four gates).  What lies 2^28 below its scale keeps an absolute error of 2^-50 of it: a sum that only such values reach - units 2^28 below others of their
- * block, the others' weights zero - loses bits that pairs with an exponent per value have.  Narrower layers and larger batches: when the shape allows (as for the forward call; deferred and dx_all given), the
+ * four gates); four units of a gate, or four weights of a row side by side, that all lie 2^28 below their scale are added in fp32, so that no value is further
+ * off than 2^-22 of the largest of its four.  Narrower layers and larger batches: when the shape allows (as for the forward call; deferred and dx_all given), the
  * steps run inside ONE kernel whose CTAs stay on the GPU: the cell pass and the [Wx; Wh]^T dgates product of a step hand
  * over through counters in device memory, and every CTA alternates between two independent blocks of batch columns so that
  * one block's hand-overs hide behind the other's products (the per-step call uses the same K splits for such shapes, which

@@ -236,18 +236,19 @@ def _dgates(gates, c, cp, dh, dc, H):
     return torch.cat([d * gg * i * (1 - i), d * cp.double() * f * (1 - f), dh.double() * tc * o * (1 - o), d * i * (1 - gg * gg)], dim=1)
 
 
-# A pair's scale belongs to a column and 128 units of all gates (dgates) or to a row (weights).  Odd units have gradients 2^-e below the even ones; every third
-# row of the weights is zero at the even units, every third 2^-e smaller there than at the odd ones.  Bar of a result: 1.45e-6 * 1.25 (as above) of the sum of its
-# products' magnitudes - never more than |row| |column|, and all that a product or a truncated sum can be off by in proportion - and 2^-49 of a scale's
-# largest value times the other factor's sum: what lies 2^28 below a scale keeps an absolute error of 2^-50 of it, and its lo part meets no lo part, half of that again.
-@pytest.mark.parametrize("I,H,B", [(96, 512, 64), (100, 777, 33)])
-@pytest.mark.parametrize("e", [10, 20, 28, 30, 40, 50])
-def test_values_that_differ_within_a_scale(I, H, B, e):
+# A pair's scale belongs to a column and 128 units of all gates (dgates) or to a row (weights).  Every other `run` of units has gradients 2^-e below the rest; every
+# third row of the weights is zero at the rest, every third 2^-e smaller there.  Bar of a result: 1.45e-6 * 1.25 (as above) of the sum of its products'
+# magnitudes - never more than |row| |column|, and all that a product or a truncated sum can be off by in proportion - and 2^-22 of what the sum would be with the
+# largest value of its quad (four units of a gate, four weights of a row side by side) in the place of one of the factors: a value keeps an absolute error of
+# 2^-50 of its scale's largest, and a quad that lies 2^28 below that is added in fp32.  (Runs of four: quads of one magnitude, which keep their own bits.)
+@pytest.mark.parametrize("I,H,B,run,e", [(*s, run, e) for s in ((96, 512, 64), (130, 1000, 130), (9, 777, 33)) for run in (1, 4) for e in (10, 20, 27, 28, 29, 30, 40, 50, 90)] +
+                         [(3, 4104, 16, 4, 40), (3, 4104, 16, 4, 29)])   # (rows of weights that are made into pairs in two passes)
+def test_values_that_differ_within_a_scale(I, H, B, run, e):
     import torch
     T = 2
     gen = torch.Generator("cuda").manual_seed(H + e)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
-    odd = torch.arange(H, device="cuda") % 2 == 1
+    odd = torch.arange(H, device="cuda") // run % 2 == 1
     weight = [torch.ones(H, device="cuda"), odd.float(), torch.where(odd, 1.0, 2.0 ** -e)]
     Wx, Wh = [torch.stack([weight[j % 3] for j in range(n)]).repeat(1, 4) * rnd(n, 4 * H) / H ** 0.5 for n in (I, H)]
     gates = torch.cat([torch.sigmoid(rnd(T * B, 3 * H)), torch.tanh(rnd(T * B, H))], dim=1)
@@ -256,12 +257,17 @@ def test_values_that_differ_within_a_scale(I, H, B, e):
     dh, dc, dx, _ = _sweep(I, H, B, T, Wx, Wh, gates, cs, c0, dh_in, dc_in)
     sl, pr = slice(B, 2 * B), slice(0, B)
     dg = _dgates(gates[sl], cs[sl], cs[pr], dh[sl], dc[sl], H)
-    block = dg.abs().view(B, 4, H)
-    top = torch.cat([block[:, :, u:u + 128].amax(dim=(1, 2), keepdim=True).expand(-1, 4, min(128, H - u)) for u in range(0, H, 128)], dim=2).reshape(B, 4 * H)
+
+    def quad(v):   # the largest magnitude of the quad of every value that is not zero
+        rows, n = v.shape
+        m = torch.nn.functional.pad(v.abs(), (0, -n % 4)).view(rows, -1, 4).amax(dim=2).repeat_interleave(4, dim=1)[:, :n]
+        return m * (v != 0)
+
+    qg = torch.cat([quad(g) for g in dg.split(H, dim=1)], dim=1)
     for W, got, old in ((Wx, dx[sl], None), (Wh, dh[pr], dh_in[pr])):
         W = W.double()
         want = dg @ W.t() + (0 if old is None else old.double())
-        bar = 1.45e-6 * 1.25 * (dg.abs() @ W.abs().t()) + 2.0 ** -49 * (top @ W.abs().t() + dg.abs().sum(dim=1)[:, None] * W.abs().amax(dim=1)[None, :]) + 1.3e-7 * want.abs()
+        bar = 1.45e-6 * 1.25 * (dg.abs() @ W.abs().t()) + 2.0 ** -22 * (qg @ W.abs().t() + dg.abs() @ quad(W).t()) + 1.3e-7 * want.abs()
         assert bool(((got - want).abs() <= bar).all()), float(((got - want).abs() / bar).max())
 
 
