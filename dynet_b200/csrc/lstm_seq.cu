@@ -50,7 +50,7 @@ __device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return
 // A column of x has a scale of its own, h .* mask_h one that is known beforehand (|h| < 1: the largest mask value of the column), h_{-1} the
 // larger of that and its own; so accumulation chains end between Wx x and Wh h, and a chain is unscaled as it is drained.  (Elements of h below 2^-28 of
 // the mask's largest value keep an absolute error of 2^-50 of it, as those of a column of x and of a row of weights do of theirs: below the 2^-24
-// that an activation is rounded to, as long as a column's largest |x| times a row's sum of |w| stays below 2^26.)
+// that an activation is rounded to, as long as a column's largest |x| times a row's sum of |w|, and a row's largest |w| times a column's sum of |x|, stay below 2^25.)
 // grid = (4H / 128, B / BNT, S); with S > 1 the S CTAs of a tile are one thread-block cluster (1 x 1 x S).  S (1, 2, 4 or 8) is
 // a template parameter so that the column exchange indexes registers statically.
 // VEC: units in fours, on 16 bytes (otherwise, F16 only, a value at a time; those on 128-column tiles spill 464 - 592 bytes: 512 x 777 x 500 columns 23 us a
