@@ -63,6 +63,9 @@ __device__ __forceinline__ KBlock k_block(uint32_t i, uint32_t H, uint32_t Ha, u
 }
 
 constexpr int kMaxBlocks = 4;   // column blocks per CTA
+// A CTA that adds many small quads (below) is milliseconds late, and the others wait for it.  ms a step where every quad but one of a scale is small, of dgates / of
+// weights: 1024 units, 512 columns 2.3 / 9, 2048 units, 500 columns 14 / 37, 3072 units, 1000 columns 93 / 148 (past the other kernels' bound).
+constexpr uint32_t kLongWait = 16 * kWaitLimit;
 
 struct CellIn { float4 gi, gf, go, gg, c, cp, dci, dcp; };
 // What a thread of the eight warps that share a CTA's columns does of the cell pass: units [u, + 4) of block `blk`, `left` of them there (own: any)
@@ -122,44 +125,83 @@ __device__ __forceinline__ float4 quad_of(const BwdWide& a, const float* hi, con
 __device__ __noinline__ float4 small_parts(const BwdWide& a, uint32_t r, uint32_t m) {
   const uint32_t lane = threadIdx.x & 31, G = 4 * a.H;
   const float *hi = a.dn_hi + (size_t)r * a.dn_pitch, *lo = a.dn_lo + (size_t)r * a.dn_pitch;
+  const bool vec = (a.H & 3) == 0 && aligned16(a.W);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (uint32_t b = 0; b * BM < a.H; ++b) {
     const uint32_t word = __ldcg(a.dsc + (size_t)b * a.dsc_ld + r);
     if (!(word & 1)) continue;
     float4 v[4];
+    uint32_t hits[4], n = 0;
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) v[k] = quad_of(a, hi, lo, k, b * BM + 4 * lane);
+    for (uint32_t k = 0; k < 4; ++k) {
+      v[k] = quad_of(a, hi, lo, k, b * BM + 4 * lane);
+      const bool hit = pair_loses(quad_mag(v[k]), word);
+      if (!hit) v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      hits[k] = __ballot_sync(0xffffffffu, hit);
+      n += __popc(hits[k]);
+    }
+    if (n <= 6) {   // a few: quad by quad, every lane its rows (32 sectors a load: 16 such loads a quad)
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k)
-      for (uint32_t left = __ballot_sync(0xffffffffu, pair_loses(quad_mag(v[k]), word)); left; left &= left - 1) {
-        const uint32_t src = __ffs(left) - 1, u = b * BM + 4 * src;
+      for (uint32_t k = 0; k < 4; ++k)
+        for (uint32_t left = hits[k]; left; left &= left - 1) {
+          const uint32_t src = __ffs(left) - 1, u = b * BM + 4 * src;
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-          const float x = __shfl_sync(0xffffffffu, (&v[k].x)[i], src);
+          for (uint32_t i = 0; i < 4; ++i) {
+            const float x = __shfl_sync(0xffffffffu, (&v[k].x)[i], src);
 #pragma unroll
-          for (uint32_t j = 0; j < 4; ++j)
-            if (u + i < a.H && m + j < a.M) acc[j] = fmaf(__ldg(a.W + k * a.H + u + i + (size_t)G * (m + j)), x, acc[j]);
+            for (uint32_t j = 0; j < 4; ++j)
+              if (u + i < a.H && m + j < a.M) acc[j] = fmaf(__ldg(a.W + k * a.H + u + i + (size_t)G * (m + j)), x, acc[j]);
+          }
         }
+    } else {   // many: row by row, every lane its quads (whole lines; 1024 units, 512 columns, all of them small: 39 ms -> 6.9 for three steps)
+      const uint32_t u = b * BM + 4 * lane, left = u < a.H ? a.H - u : 0;
+      for (uint32_t src = 0; src < 32; ++src)
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+          const uint32_t row = __shfl_sync(0xffffffffu, m, src) + j;
+          float sum = 0.f;
+          if (row < a.M && left) {
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+              const float* p = a.W + (size_t)G * row + k * a.H + u;
+              const float4 w = vec ? __ldg(reinterpret_cast<const float4*>(p)) : ldu<false>(p, left);
+              sum = fmaf(w.x, v[k].x, fmaf(w.y, v[k].y, fmaf(w.z, v[k].z, fmaf(w.w, v[k].w, sum))));
+            }
+          }
+          sum = warp_sum(sum);
+          if (lane == src) acc[j] += sum;
+        }
+    }
+  }
+  // those of the weights' rows, 32 quads at a time, with what has not been added above
+  uint32_t rows[4];
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j) rows[j] = __ballot_sync(0xffffffffu, m + j < a.M && (__ldg(a.wscale + m + j) & 1));
+  if ((rows[0] | rows[1] | rows[2] | rows[3]) == 0) return make_float4(acc[0], acc[1], acc[2], acc[3]);
+  for (uint32_t e = 4 * lane; e < (G + 127) / 128 * 128; e += 128) {   // (G is a multiple of four)
+    float v[4];
+    bool have = false;   // (the dgates, once a row wants them)
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+      for (uint32_t left = rows[j]; left; left &= left - 1) {
+        const uint32_t src = __ffs(left) - 1, row = __shfl_sync(0xffffffffu, m, src) + j;
+        const float* w = a.W + (size_t)G * row + e;
+        const float4 x = e >= G ? make_float4(0.f, 0.f, 0.f, 0.f) : aligned16(a.W) ? __ldg(reinterpret_cast<const float4*>(w)) : make_float4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+        const bool hit = pair_loses(quad_mag(x), __ldg(a.wscale + row));
+        if (!__any_sync(0xffffffffu, hit)) continue;
+        if (!have) {
+          have = true;
+#pragma unroll
+          for (uint32_t i = 0; i < 4; ++i) {
+            const uint32_t k = (e + i) / a.H, u = (e + i) % a.H;
+            const float4 q = e < G ? quad_of(a, hi, lo, k, u / 4 * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[i] = e < G && !pair_loses(quad_mag(q), __ldcg(a.dsc + (size_t)(u / BM) * a.dsc_ld + r)) ? (u % 4 == 0 ? q.x : u % 4 == 1 ? q.y : u % 4 == 2 ? q.z : q.w) : 0.f;
+          }
+        }
+        const float sum = warp_sum(hit ? fmaf(x.x, v[0], fmaf(x.y, v[1], fmaf(x.z, v[2], x.w * v[3]))) : 0.f);
+        if (lane == src) acc[j] += sum;
       }
   }
-#pragma unroll
-  for (uint32_t j = 0; j < 4; ++j)
-    for (uint32_t left = __ballot_sync(0xffffffffu, m + j < a.M && (__ldg(a.wscale + m + j) & 1)); left; left &= left - 1) {
-      const uint32_t src = __ffs(left) - 1, row = __shfl_sync(0xffffffffu, m, src) + j, word = __ldg(a.wscale + row);
-      const float* w = a.W + (size_t)G * row;
-      float sum = 0.f;
-      for (uint32_t e = 4 * lane; e < G; e += 128) {   // (G is a multiple of four)
-        const float4 x = make_float4(__ldg(w + e), __ldg(w + e + 1), __ldg(w + e + 2), __ldg(w + e + 3));
-        if (!pair_loses(quad_mag(x), word)) continue;
-        for (uint32_t i = 0; i < 4; ++i) {
-          const uint32_t k = (e + i) / a.H, u = (e + i) % a.H;
-          const float4 v = quad_of(a, hi, lo, k, u / 4 * 4);
-          if (!pair_loses(quad_mag(v), __ldcg(a.dsc + (size_t)(u / BM) * a.dsc_ld + r))) sum = fmaf((&x.x)[i], (&v.x)[u % 4], sum);   // (else it has been added above)
-        }
-      }
-      sum = warp_sum(sum);
-      if (lane == src) acc[j] += sum;
-    }
   return make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 // The cell pass of units [u, + 4), column n of step t from dE/dh: dE/dc of the step before, and dgates as fp16 pairs with the word of the warp's
@@ -346,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
           if (fail) break;
         }
         for (; i < total; ++i) {
-          if (!mbar_wait(&empty_bar[s], ph ^ 1)) { fail = true; break; }
+          if (!mbar_wait(&empty_bar[s], ph ^ 1, kLongWait)) { fail = true; break; }
           unsigned char* st = ring + (size_t)s * kStageBytes;
           const KBlock kb = k_block(k0 + i, a.H, a.Ha, a.Hp);
           mbar_expect_tx(&full_bar[s], kStageBytes);
@@ -377,9 +419,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
         uint32_t in_chain = 0;
         for (uint32_t i = 0; i < total; ++i) {
           if (in_chain == 0 && chain >= kBufs) {
-            if (!mbar_wait(&acc_empty[buf], ((chain / kBufs) - 1) & 1)) { fail = true; break; }
+            if (!mbar_wait(&acc_empty[buf], ((chain / kBufs) - 1) & 1, kLongWait)) { fail = true; break; }
           }
-          if (!mbar_wait(&full_bar[s], ph)) { fail = true; break; }
+          if (!mbar_wait(&full_bar[s], ph, kLongWait)) { fail = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           uint64_t a_hi, a_lo, b;   // select without dynamic register indexing
           if (s == 0) { a_hi = d_a_hi[0]; a_lo = d_a_lo[0]; b = d_b[0]; }
@@ -502,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
 #pragma unroll
       for (uint32_t q = 0; q < kHalf; ++q) sum[q] = 0.f;
       // (a share without k-blocks waits too: once the counter is up, the others are done with their exchange buffers as scratch for row sums)
-      if (REC && ok && !mbar_wait(&go[cb], it & 1)) ok = false;
+      if (REC && ok && !mbar_wait(&go[cb], it & 1, kLongWait)) ok = false;
       // (the words of the columns that this warp finishes: looked at once the partial sums are on their way)
       uint32_t words[KC * BNT / 64];
 #pragma unroll
@@ -521,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
           const uint32_t n = col0 + half * kHalf + 32 * k + lane;
           f[k] = inv_scale_of(n < cols ? __ldcg(a.dsc + (size_t)((k0 >> 3) + c) * a.dsc_ld + seq0 + n) : 0x3f800000u);
         }
-        if (!mbar_wait(&acc_full[buf], (cg / kBufs) & 1)) { ok = false; continue; }
+        if (!mbar_wait(&acc_full[buf], (cg / kBufs) & 1, kLongWait)) { ok = false; continue; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t taddr = tmem_base + buf * kAccCols + ((quarter * 32) << 16) + half * kHalf;
 #pragma unroll
@@ -546,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
         for (uint32_t k = 0; k < KC; ++k) any |= words[KC * hh + k];
         const bool quads = __any_sync(0xffffffffu, any & 1);
         // ---- partial sums to the ranks that finish them ----
-        if (S > 1 && ok && !mbar_wait_cluster(&park_free, pr_phase ^ 1)) ok = false;
+        if (S > 1 && ok && !mbar_wait_cluster(&park_free, pr_phase ^ 1, kLongWait)) ok = false;
         if (S > 1) {
 #pragma unroll
           for (uint32_t rr = 0; rr < S / 2; ++rr) {
@@ -593,7 +635,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             if (REC && t) cell_load<VEC>(a, un, in[g], t - 1, n[g]);
           }
           if (kb == 0) {
-            const bool got = S > 1 ? mbar_wait_cluster(&park_full, pf_phase) : true;
+            const bool got = S > 1 ? mbar_wait_cluster(&park_full, pf_phase, kLongWait) : true;
             ok = bar_and(1, 256, ok && got) != 0;
             pf_phase ^= 1; pr_phase ^= 1;
             if (S > 1 && te == 0) mbar_expect_tx(&park_full, kParkBytes);   // (the next pass; it begins when this CTA has arrived on the others' park_free)

@@ -27,9 +27,9 @@ __device__ __forceinline__ void signal_counter(uint32_t* p) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 // mbarrier wait that also orders after arrivals from other CTAs of the cluster
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, uint32_t limit = kWaitLimit) {
   uint32_t done = 0;
-  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+  for (uint32_t it = 0; it < limit; ++it) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"

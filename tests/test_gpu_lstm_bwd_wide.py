@@ -319,3 +319,34 @@ def test_infinities_and_nans_stay_in_their_column_and_row(I, H, B):
     assert torch.equal(dx[2 * B:, rest], clean[2][2 * B:, rest]) and not bool(torch.isfinite(dx[2 * B:, [7, I - 1]]).any())
     units = [r for r in range(H) if r != 200]
     assert torch.equal(dh[B:2 * B, units], clean[0][B:2 * B, units]) and not bool(torch.isfinite(dh[B:2 * B, 200]).any())
+
+
+@pytest.mark.parametrize("I,H,B", [(64, 1024, 512), (9, 777, 100), (64, 2048, 500)])
+@pytest.mark.parametrize("where", ["weights", "dgates"])
+def test_small_quads_everywhere(I, H, B, where):
+    """Every quad of a scale but one lies 2^-40 below it: the slowest such calls can be, well inside the bounds of the waits, and right."""
+    import torch
+    T = 3
+    gen = torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)   # noqa: E731
+    keep = torch.arange(H, device="cuda") % 128 < 4                  # (units of quad 0 of every block; H % 4: of gate 0's at least)
+    low = torch.where(keep, 1.0, 2.0 ** -40)
+    Wx, Wh = [rnd(n, 4 * H) / H ** 0.5 * (torch.where(torch.arange(4 * H, device="cuda") < 4, 1.0, 2.0 ** -40) if where == "weights" else 1.0 - keep.float().repeat(4))
+              for n in (I, H)]
+    gates = torch.cat([torch.sigmoid(rnd(T * B, 3 * H)), torch.tanh(rnd(T * B, H))], dim=1)
+    cs, c0, dh_in, dc_in = rnd(T * B, H), rnd(B, H), rnd(T * B, H), rnd(T * B, H)
+    if where == "dgates":
+        dh_in *= low
+        dc_in *= low
+    dh, dc, dx, _ = _sweep(I, H, B, T, Wx, Wh, gates, cs, c0, dh_in, dc_in)
+    for t in range(T - 1, -1, -1):
+        sl, pr = slice(t * B, (t + 1) * B), slice((t - 1) * B, t * B)
+        dg = _dgates(gates[sl], cs[sl], cs[pr] if t else c0, dh[sl], dc[sl], H)
+        for W, got, old in ((Wx, dx[sl], None), (Wh, dh[pr], dh_in[pr]))[:2 if t else 1]:
+            W = W.double()
+            want = dg @ W.t() + (0 if old is None else old.double())
+            bar = (1.45e-6 * 1.25 + 2.0 ** -21) * (dg.abs() @ W.abs().t()) + 1.3e-7 * want.abs()
+            if where == "dgates" and H % 4 == 0:   # (nothing but small quads meets these rows)
+                assert bool(((got - want).abs() <= bar).all()), (t, float(((got - want).abs() / bar).max()))
+            bar = 1.45e-6 * 1.25 * dg.norm(dim=1)[:, None] * W.norm(dim=1)[None, :] + 1.3e-7 * want.abs()
+            assert bool(((got - want).abs() <= bar).all()), (t, float(((got - want).abs() / bar).max()))
