@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(256) k_f16_split(const __grid_constant__ F16Jo
         s = make_float4(scale_of(__ldg(j.scale + min(e[k], top))), scale_of(__ldg(j.scale + min(e[k] + 1, top))), scale_of(__ldg(j.scale + min(e[k] + 2, top))), 1.f);
       }
     } else {
-      const uint32_t word = __ldcg(j.scale + line[k]);   // (bit 0 may be set meanwhile)
+      const uint32_t word = j.mark ? __ldcg(j.scale + line[k]) : __ldg(j.scale + line[k]);   // (bit 0 may be set meanwhile)
       s.x = s.y = s.z = s.w = scale_of(word);
       if (j.mark && pair_loses(mag4(v[k]), word)) { v[k] = make_float4(0.f, 0.f, 0.f, 0.f); atomicOr(j.scale + line[k], 1u); }
     }
@@ -1025,7 +1025,7 @@ __global__ void __launch_bounds__(256) k_f16_strip(const __grid_constant__ F16Jo
 }
 // Lines: a warp per line of up to 1024 values, a CTA per longer one.
 constexpr uint32_t kOneLine = kF16PadMax, kOneStrip = 1024;   // longest line, most lines of a strip
-template <uint32_t R, bool PAD>
+template <uint32_t R, bool PAD, bool MARK>
 __device__ __forceinline__ void line_pairs(const F16Job& j, uint32_t line, uint32_t e0, uint32_t step, uint32_t* red) {
   const float* p = j.src + (size_t)j.ld * line;
   const bool vec = aligned16(p);
@@ -1047,7 +1047,7 @@ __device__ __forceinline__ void line_pairs(const F16Job& j, uint32_t line, uint3
 #pragma unroll
     for (int w = 0; w < 8; ++w) m = max(m, red[w]);
   }
-  if (j.mark) {
+  if (MARK && j.mark) {
     bool loses = false;
 #pragma unroll
     for (uint32_t k = 0; k < R; ++k)
@@ -1083,17 +1083,17 @@ __device__ __forceinline__ void line_pairs(const F16Job& j, uint32_t line, uint3
     }
   }
 }
-template <uint32_t R, bool PAD>   // (R 16: lines of more than 8192; PAD: jobs with pad_H)
+template <uint32_t R, bool PAD, bool MARK>   // (R 16: lines of more than 8192; PAD, MARK: jobs with pad_H, with mark - registers that the others do without, 95 against 80)
 __global__ void __launch_bounds__(256) k_f16_line(const __grid_constant__ F16Jobs jobs) {
   dyb_grid_dep_sync();
   __shared__ uint32_t red[8];
   const uint32_t z = f16_job_of(jobs), unit = blockIdx.x - jobs.start[z];
   const F16Job& j = jobs.job[z];
   if (j.n > 1024) {
-    line_pairs<R, PAD>(j, unit, 4 * threadIdx.x, 1024, red);
+    line_pairs<R, PAD, MARK>(j, unit, 4 * threadIdx.x, 1024, red);
   } else {
     const uint32_t line = 8 * unit + (threadIdx.x >> 5);
-    if (line < j.lines) line_pairs<8, PAD>(j, line, 4 * (threadIdx.x & 31), 128, nullptr);
+    if (line < j.lines) line_pairs<8, PAD, MARK>(j, line, 4 * (threadIdx.x & 31), 128, nullptr);
   }
 }
 constexpr uint64_t kOneValues = 12u << 20;   // (48 MB and as much again of pairs: L2 still holds most of both)
@@ -1292,21 +1292,22 @@ int dyb200_f16_pack(dyb200_ctx* ctx, F16Jobs* jobs) {
     F16Jobs part;
     part.n = 0; part.start[0] = 0;
     uint32_t lines = 0, longest = 0;
-    bool odd = false, pad = false;
+    bool odd = false, pad = false, mark = false;   // (pad: only with mark)
     for (int k = 0; k < jobs->n; ++k) {
       const F16Job& j = jobs->job[k];
       if (j.mode != mode) continue;
       if (!f16_one_pass(j)) { rest.job[rest.n++] = j; continue; }
       if (j.lines > lines) lines = j.lines;
       if (j.n > longest) longest = j.n;
-      odd = odd || j.perm_H % 4 != 0; pad = pad || j.pad_H;
+      odd = odd || j.perm_H % 4 != 0; pad = pad || j.pad_H; mark = mark || j.mark || j.pad_H;
       part.job[part.n] = j;
       part.start[part.n + 1] = part.start[part.n] + (mode == F16_ELEM ? (j.n + 31) / 32 : j.n > 1024 ? j.lines : (j.lines + 7) / 8);
       ++part.n;
     }
     if (part.n == 0 || part.start[part.n] == 0) continue;
     void (*k)(F16Jobs);
-    if (mode == F16_LINE) k = longest <= 8192 ? (pad ? k_f16_line<8, true> : k_f16_line<8, false>) : pad ? k_f16_line<16, true> : k_f16_line<16, false>;
+    if (mode == F16_LINE && !mark) k = longest <= 8192 ? k_f16_line<8, false, false> : k_f16_line<16, false, false>;
+    else if (mode == F16_LINE) k = longest <= 8192 ? (pad ? k_f16_line<8, true, true> : k_f16_line<8, false, true>) : pad ? k_f16_line<16, true, true> : k_f16_line<16, false, true>;
     else if (odd) k = lines <= 512 ? k_f16_strip<16, true> : k_f16_strip<32, true>;
     else k = lines <= 256 ? k_f16_strip<8> : lines <= 512 ? k_f16_strip<16> : k_f16_strip<32>;
     dyb_launch(k, part.start[part.n], 256, 0, ctx, part);
