@@ -88,6 +88,9 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
                "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// four bytes of global memory into this thread's place in shared memory, beside everything else it does
+__device__ __forceinline__ void copy4(uint32_t dst, const float* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // p + col * bytes: one multiply-add of 32 x 32 + 64 bits (indexing by floats adds a shift of 64 bits to every address; addresses were a
 // third of the cell passes' instructions)
 __device__ __forceinline__ float* at(float* p, uint32_t col, uint32_t bytes) { return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + (uint64_t)col * bytes); }
@@ -113,9 +116,11 @@ __device__ __forceinline__ void tc_kstep(uint32_t wide, uint32_t narrow, uint32_
 }
 
 // grid (C, clusters x directions), cluster (C, 1, 1).  Dynamic shared memory (1024-byte aligned), for each group:
-// h [2][2 KB blocks of 32 units][NC hi rows, NC lo rows][64 bytes]; gates on their way [NC][4][32]; KB = ceil(H / 64).
+// h [2][2 KB blocks of 32 units][NC hi rows, NC lo rows][64 bytes], then gates on their way [NC][4][32], then Wx x + b [2][2 cells x 4 gates][threads];
+// KB = ceil(H / 64).
 // TMEM: each group's accumulators (3 NC columns: A_hi B_hi, A_hi B_lo, A_lo B_hi - the last apart, so that the chain of one waits on
 // the other's MMAs, not on its own), Wh_hi and Wh_lo (32 KB columns each).
+template <uint32_t kH>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_constant__ RecFwd a) {
   constexpr uint32_t NC = kTcCols, kBlock = 2 * NC * 64;   // bytes of a CTA's part of h
   extern __shared__ unsigned char smem_raw[];
@@ -125,12 +130,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t grp = warp < kGroups ? warp : (warp - kGroups) / kGroupWarps, gw = (warp - kGroups) % kGroupWarps;   // (gw: cell warps)
   const RecDirF d = dir ? a.d[1] : a.d[0];
-  const uint32_t H = a.H, rank = blockIdx.x, C = gridDim.x, KB = (H + 63) / 64;
+  const uint32_t H = kH ? kH : a.H, rank = blockIdx.x, C = kH ? kH / kTcUnits : gridDim.x, KB = (H + 63) / 64;
   const uint32_t base = (blockIdx.y / ndir * kGroups + grp) * NC;
   const uint32_t hbytes = 2 * KB * kBlock;
   unsigned char* hall = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* hbuf = hall + grp * 2 * hbytes;
   float* exch = reinterpret_cast<float*>(hall + kGroups * 2 * hbytes) + grp * NC * 128;
+  float* ahead = reinterpret_cast<float*>(hall + kGroups * 2 * hbytes) + (kGroups + 2 * grp) * NC * 128;
   uint64_t *got = got_[grp], &acc_full = acc_full_[grp], &h_ready = h_ready_[grp];
   uint32_t* hword = hword_[grp];
   if (tid == 0) {
@@ -260,7 +266,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       col1 = col2; col2 = col3; n = n1;
     }
   } else {
-    // reads gate `quad` of the columns 16 j + c8 .. + 7, finishes columns 16 j + c8 + quad and + 4; lane = unit
+    // reads gate `quad` of the columns c8 .. c8 + 7, finishes columns c8 + quad + 4 j; lane = unit
     constexpr int kCells = NC / 8;
     const uint32_t quad = warp & 3, c8 = 8 * (gw >> 2), u = rank * kTcUnits + lane, i0 = c8 + quad;
     const bool live_u = u < H;
@@ -270,20 +276,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     const uint32_t tq = tmem + grp * 3 * NC + ((32 * quad) << 16) + c8;
     const float* mask = d.mask ? d.mask + uc : nullptr;
     float *pg = d.gates + uc, *pc = d.c + uc, *ph = d.h + uc, *phi = d.hn_hi ? d.hn_hi + uc : nullptr, *plo = phi ? d.hn_lo + uc : nullptr;
-    float pre[kCells][4], ahead[kCells][4], cst[kCells], mk[kCells];   // (ahead: of the next step, requested a whole step before its use)
+    float cst[kCells], mk[kCells];
+    // Wx x + b of this thread's cells, of this step and of the next, asked for a whole step before its use.  (In registers the wait for it fell wherever the
+    // compiler's few scoreboards put it, before the cell pass of the step that asked: 1187 us forward, 1110 - 1350 with other forms of the same loads, 1039 like this.)
+    float* const mine = ahead + gt0;
+    const uint32_t pitch = kH ? kH : a.hn_pitch;
     uint32_t ho[kCells];                                   // where h of cell j goes in this CTA's block
-    auto fetch = [&](uint32_t c0, uint32_t nact) {
+    auto fetch = [&](uint32_t to, uint32_t c0, uint32_t nact) {
+      const float* p = at(pg, c0 + base + i0, 16 * H);
+      const uint32_t dst = smem_u32(mine) + to * (NC * 128 * 4);
 #pragma unroll
-      for (int j = 0; j < kCells; ++j) {
-        const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), col = c0 + base + (i < nact ? i : 0);
+      for (int j = 0; j < kCells; ++j)
+        if (i0 + 4 * j < nact) {                           // (the same for the whole warp)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) ahead[j][q] = at(pg, col, 16 * H)[(size_t)q * H];
-      }
+          for (int q = 0; q < 4; ++q) copy4(dst + (4 * j + q) * (kGroupThreads * 4), p + (size_t)(16 * j + q) * H);
+        }
     };
-    if (n) fetch(0, n);          // (a group may have no column at all)
+    if (n) fetch(0, 0, n);          // (a group may have no column at all)
 #pragma unroll
     for (int j = 0; j < kCells; ++j) {
-      const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), sc = base + i;
+      const uint32_t i = i0 + 4 * j, sc = base + i;
       cst[j] = d.c0 && i < ncol ? __ldg(at(d.c0 + uc, sc, 4 * H)) : 0.f;
       mk[j] = mask && i < ncol ? __ldg(at(mask, a.mask_full ? sc : 0, 4 * H)) : 1.f;
       ho[j] = h_off(2 * NC, i, rank * kTcUnits + lane);
@@ -293,36 +305,33 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       unsigned char* hnext = hbuf + ((t & 1) ^ 1) * hbytes;
       const int ts = t ? t1 : t0, th = ts >> 1;
       const float f0 = __int_as_float((th + 127) << 23), f1 = __int_as_float((ts - th + 127) << 23);
-#pragma unroll
-      for (int j = 0; j < kCells; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) pre[j][q] = ahead[j][q];
-      if (n1) fetch(col1, n1);
+      const float* const pre = mine + (t & 1) * (NC * 128);
+      copies_done();
+      if (n1) fetch((t & 1) ^ 1, col1, n1);
       ok = ok && mbar_wait(&acc_full, t & 1);
       tc_after();
-#pragma unroll
-      for (int j = 0; j < (int)NC / 16; ++j) {
+      {
         float z[8], z2[8], z3[8];
-        tmem_ld8(tq + 16 * j, z);
-        tmem_ld8(tq + NC + 16 * j, z2);
-        tmem_ld8(tq + 2 * NC + 16 * j, z3);
+        tmem_ld8(tq, z);
+        tmem_ld8(tq + NC, z2);
+        tmem_ld8(tq + 2 * NC, z3);
         tmem_ld_wait();
 #pragma unroll
-        for (int x = 0; x < 8; ++x) exch[((16 * j + c8 + x) * 4 + quad) * 32 + lane] = (fmaf(z2[x] + z3[x], kLoScale, z[x]) * f0) * f1;
+        for (int x = 0; x < 8; ++x) exch[((c8 + x) * 4 + quad) * 32 + lane] = (fmaf(z2[x] + z3[x], kLoScale, z[x]) * f0) * f1;
       }
       tc_before();
       bar_sync(2 + 2 * grp + c8 / 8, 128);
       float hv[kCells], hm[kCells], y[kCells][4];
 #pragma unroll
       for (int j = 0; j < kCells; ++j) {
-        const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1);
+        const uint32_t i = i0 + 4 * j;
 #pragma unroll
         for (int q = 0; q < 4; ++q) y[j][q] = exch[(i * 4 + q) * 32 + lane];
         if (i >= n) continue;                            // (the same for the whole warp)
-        y[j][0] = gate_sigmoid(y[j][0] + pre[j][0]);
-        y[j][1] = gate_sigmoid(y[j][1] + pre[j][1] + a.fb);
-        y[j][2] = gate_sigmoid(y[j][2] + pre[j][2]);
-        y[j][3] = gate_tanh(y[j][3] + pre[j][3]);
+        y[j][0] = gate_sigmoid(y[j][0] + pre[4 * j * kGroupThreads]);
+        y[j][1] = gate_sigmoid(y[j][1] + pre[(4 * j + 1) * kGroupThreads] + a.fb);
+        y[j][2] = gate_sigmoid(y[j][2] + pre[(4 * j + 2) * kGroupThreads]);
+        y[j][3] = gate_tanh(y[j][3] + pre[(4 * j + 3) * kGroupThreads]);
         cst[j] = lstm_cell_c(y[j][0], y[j][3], y[j][1], cst[j]);
         hv[j] = lstm_cell_h(y[j][2], cst[j]);
         hm[j] = hv[j] * mk[j];
@@ -336,19 +345,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       fence_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&h_ready);
+      // (cell j: four columns on)
+      float *const og = at(pg, col0 + base + i0, 16 * H), *const oc = at(pc, col0 + base + i0, 4 * H), *const oh = at(ph, col0 + base + i0, 4 * H);
+      float *const ohi = at(phi, col1 + base + i0, 4 * pitch), *const olo = at(plo, col1 + base + i0, 4 * pitch);
 #pragma unroll
       for (int j = 0; j < kCells; ++j) {
-        const uint32_t i = 8 * (j & ~1) + i0 + 4 * (j & 1), sc = base + i;
+        const uint32_t i = i0 + 4 * j;
         if (!live_u || i >= n) continue;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) at(pg, col0 + sc, 16 * H)[(size_t)q * H] = y[j][q];
-        *at(pc, col0 + sc, 4 * H) = cst[j];
-        *at(ph, col0 + sc, 4 * H) = hv[j];
+        for (int q = 0; q < 4; ++q) og[(size_t)(16 * j + q) * H] = y[j][q];
+        oc[(size_t)(4 * j) * H] = cst[j];
+        oh[(size_t)(4 * j) * H] = hv[j];
         if (phi && i < n1) {
           float hi, lo;
           split_tf32(hm[j], hi, lo);
-          *at(phi, col1 + sc, 4 * a.hn_pitch) = hi;
-          *at(plo, col1 + sc, 4 * a.hn_pitch) = lo;
+          ohi[(size_t)(4 * j) * pitch] = hi;
+          olo[(size_t)(4 * j) * pitch] = lo;
         }
       }
       col0 = col1; col1 = col2; col2 = col3; n = n1;
@@ -370,7 +382,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
 // units the accumulators (2 NC columns); then Wh^T hi and lo (64 columns each per row tile).  The slots of the sums that have just been
 // read hold the outgoing ones: what comes into slot r next, rank r sends after it has what went out of that slot.  Gate row (unit ul,
 // gate q) is element 4 ul + q of the reduction.
-template <bool DC>
+template <bool DC, uint32_t kH>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_constant__ RecBwd a) {
   constexpr uint32_t NC = kTcCols, kSlot = NC * kTcUnits;
   extern __shared__ unsigned char smem_raw[];
@@ -381,7 +393,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t grp = warp < kGroups ? warp : (warp - kGroups) / kGroupWarps, gw = (warp - kGroups) % kGroupWarps;   // (gw: cell warps)
   const RecDirB d = dir ? a.d[1] : a.d[0];
-  const uint32_t H = a.H, rank = blockIdx.x, C = gridDim.x, MT = (H + 127) / 128;
+  const uint32_t H = kH ? kH : a.H, rank = blockIdx.x, C = kH ? kH / kTcUnits : gridDim.x, MT = (H + 127) / 128;
   const uint32_t base = (g * kGroups + grp) * NC;
   unsigned char* dgall = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* dgb = dgall + grp * 2 * 2 * NC * 128;
@@ -491,6 +503,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     const uint32_t tq = tmem + (grp * MT + mt) * 2 * NC + ((32 * quad) << 16);
     const float *pg = d.gates + uc, *pc = d.c + uc, *pc0 = d.c0 ? d.c0 + uc : nullptr;
     float *pdh = d.dh + uc, *pdc = DC ? d.dc + uc : nullptr, *phi = d.dn_hi + uc, *plo = d.dn_lo + uc;
+    const uint32_t pitch = kH ? 4 * kH : a.dn_pitch;
     uint32_t phase[2] = {0, 0};
     float gt[kCells][4], cv[kCells], cp[kCells], dhv[kCells], dcv[kCells], dcs[kCells];
     unsigned char* dgo = dgb + op_off(2 * NC, gw, 4 * lane);   // (eight columns on: 1024 bytes)
@@ -579,8 +592,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
           db[q] += pr[j][q];
           float hi, lo;
           split_tf32(pr[j][q], hi, lo);
-          at(phi, col + sc, 4 * a.dn_pitch)[(size_t)q * H] = hi;
-          at(plo, col + sc, 4 * a.dn_pitch)[(size_t)q * H] = lo;
+          at(phi, col + sc, 4 * pitch)[(size_t)q * H] = hi;
+          at(plo, col + sc, 4 * pitch)[(size_t)q * H] = lo;
         }
       }
       if (t == 0) break;           // (no earlier state to hand dE/dh to)
@@ -651,7 +664,34 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
 uint32_t tc_smem(bool bwd, uint32_t H) {
   const uint32_t NC = kTcCols, KB = (H + 63) / 64, C = (H + kTcUnits - 1) / kTcUnits;
   // (the partial sums' room also holds the row sums of dgates at the end, 512 bytes per cell warp)
-  return 1024 + kGroups * (bwd ? 2 * 2 * NC * 128 + 2 * C * NC * kTcUnits * 4 : 2 * 2 * KB * 2 * NC * 64 + NC * 512);
+  return 1024 + kGroups * (bwd ? 2 * 2 * NC * 128 + 2 * C * NC * kTcUnits * 4 : 2 * 2 * KB * 2 * NC * 64 + 3 * NC * 512);
+}
+
+typedef void (*TcFwd)(RecFwd);
+typedef void (*TcBwd)(RecBwd);
+// The instance of a launch.  Widths in whole 64 units (whose planes have no padding) have instances of their own: with the strides known the addresses of a
+// cell's 16 - 23 accesses are a base and immediates instead of a third of all instructions.  256 units, 4096 columns of up to 100 steps: 1039 against 961 us
+// forward, 1392 against 1194 backward.
+TcFwd tc_fwd_kernel(uint32_t H, uint32_t pitch) {
+  if (pitch && pitch != H) return k_rec_tc_fwd<0>;
+  switch (H) {
+    case 64: return k_rec_tc_fwd<64>;
+    case 128: return k_rec_tc_fwd<128>;
+    case 192: return k_rec_tc_fwd<192>;
+    case 256: return k_rec_tc_fwd<256>;
+    default: return k_rec_tc_fwd<0>;
+  }
+}
+template <bool DC>
+TcBwd tc_bwd_kernel(uint32_t H, uint32_t pitch) {
+  if (pitch != 4 * H) return k_rec_tc_bwd<DC, 0>;
+  switch (H) {
+    case 64: return k_rec_tc_bwd<DC, 64>;
+    case 128: return k_rec_tc_bwd<DC, 128>;
+    case 192: return k_rec_tc_bwd<DC, 192>;
+    case 256: return k_rec_tc_bwd<DC, 256>;
+    default: return k_rec_tc_bwd<DC, 0>;
+  }
 }
 
 }  // namespace
@@ -663,7 +703,7 @@ bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int n
   const uint32_t C = (H + kTcUnits - 1) / kTcUnits;
   int16_t& fit = ctx->rec_tc_fit[bwd][C - 1];
   if (fit == 0) {   // (asked once: whether a cluster fits this device at all)
-    const void* k = bwd ? (const void*)k_rec_tc_bwd<true> : (const void*)k_rec_tc_fwd;
+    const void* k = bwd ? (const void*)tc_bwd_kernel<true>(H, 4 * H) : (const void*)tc_fwd_kernel(H, H);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     if (dyb200_rec_launch_cfg(ctx, k, &cfg, attr, dim3(C, 1, 1), kTcThreads, tc_smem(bwd, H))) return false;
@@ -677,17 +717,18 @@ bool dyb200_rec_tc_plan(dyb200_ctx* ctx, bool bwd, uint32_t H, uint32_t N, int n
 }
 int dyb200_rec_tc_fwd(dyb200_ctx* ctx, const RecTcPlan& p, RecFwd* a, int ndir) {
   a->G = p.G; a->ndir = (uint32_t)ndir; a->flags = ctx->dev_flags;
+  const TcFwd k = tc_fwd_kernel(a->H, a->hn_pitch);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  int rc = dyb200_rec_launch_cfg(ctx, (const void*)k_rec_tc_fwd, &cfg, attr, dim3((a->H + kTcUnits - 1) / kTcUnits, p.G * ndir, 1), kTcThreads, tc_smem(false, a->H));
+  int rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3((a->H + kTcUnits - 1) / kTcUnits, p.G * ndir, 1), kTcThreads, tc_smem(false, a->H));
   if (rc) return rc;
-  cudaLaunchKernelEx(&cfg, k_rec_tc_fwd, *a);
+  cudaLaunchKernelEx(&cfg, k, *a);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
 int dyb200_rec_tc_bwd(dyb200_ctx* ctx, const RecTcPlan& p, RecBwd* a, int ndir) {
   a->G = p.G; a->ndir = (uint32_t)ndir; a->flags = ctx->dev_flags;
-  void (*k)(RecBwd) = a->d[0].dc ? k_rec_tc_bwd<true> : k_rec_tc_bwd<false>;   // (both directions give dE/dc or neither)
+  const TcBwd k = a->d[0].dc ? tc_bwd_kernel<true>(a->H, a->dn_pitch) : tc_bwd_kernel<false>(a->H, a->dn_pitch);   // (both directions give dE/dc or neither)
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
   int rc = dyb200_rec_launch_cfg(ctx, (const void*)k, &cfg, attr, dim3((a->H + kTcUnits - 1) / kTcUnits, p.G * ndir, 1), kTcThreads, tc_smem(true, a->H));
