@@ -245,12 +245,26 @@ def _native_call(*args):
     global _native_call
     try:
         from . import _call
-        _call.setup(C.Structure, DyTensor, C.c_void_p, C.sizeof(DyTensor))
+        sample = DyTensor()
+        _call.setup(C.Structure, DyTensor, C.c_void_p, C.sizeof(DyTensor), sample, C.addressof(sample))
         _native_call = _call.call
     except ImportError:
         def _native_call(*args):
             return NotImplemented
     return _native_call(*args)
+
+
+def _native_methods():
+    """Context.fwd and .bwd in C (host/py/call.c), from the first context on; what they do not take goes to the functions of the class."""
+    global _native_methods
+    _native_methods = lambda: None   # noqa: E731
+    try:
+        from . import _call
+    except ImportError:
+        return
+    _native_call(None)
+    Context.fwd = _call.method(Context.fwd, "_fwd", 6, "_hv", "check")
+    Context.bwd = _call.method(Context.bwd, "_bwd", 9, "_hv", "check")
 
 
 _ENTRIES = {}
@@ -303,6 +317,7 @@ class Context:
         self.h = h
         self._hv = h.value
         self._fwd, self._bwd = {}, {}
+        _native_methods()
 
     def _run(self, name, *args):
         rc = _native_call(_entry(name), *args, self._hv)
