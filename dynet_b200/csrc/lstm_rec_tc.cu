@@ -278,18 +278,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     float *pg = d.gates + uc, *pc = d.c + uc, *ph = d.h + uc, *phi = d.hn_hi ? d.hn_hi + uc : nullptr, *plo = phi ? d.hn_lo + uc : nullptr;
     float cst[kCells], mk[kCells];
     // Wx x + b of this thread's cells, of this step and of the next, asked for a whole step before its use.  (In registers the wait for it fell wherever the
-    // compiler's few scoreboards put it, before the cell pass of the step that asked: 1187 us forward, 1110 - 1350 with other forms of the same loads, 1039 like this.)
+    // compiler's few scoreboards put it, before the cell pass of the step that asked: 256 units 1187 us forward, 1039 like this; 200 units, 600 sentences 250 against
+    // 230; 99 units, where rows start on any four bytes, 116 against 120.)
     float* const mine = ahead + gt0;
     const uint32_t pitch = kH ? kH : a.hn_pitch;
     uint32_t ho[kCells];                                   // where h of cell j goes in this CTA's block
     auto fetch = [&](uint32_t to, uint32_t c0, uint32_t nact) {
-      const float* p = at(pg, c0 + base + i0, 16 * H);
       const uint32_t dst = smem_u32(mine) + to * (NC * 128 * 4);
 #pragma unroll
       for (int j = 0; j < kCells; ++j)
-        if (i0 + 4 * j < nact) {                           // (the same for the whole warp)
+        if (live_u && i0 + 4 * j < nact) {   // (units that are not there ask for nothing: 29 lanes on one address took 0.9 us a step, 99 units)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) copy4(dst + (4 * j + q) * (kGroupThreads * 4), p + (size_t)(16 * j + q) * H);
+          for (int q = 0; q < 4; ++q) copy4(dst + (4 * j + q) * (kGroupThreads * 4), at(pg, c0 + base + i0 + 4 * j, 16 * H) + (size_t)q * H);
         }
     };
     if (n) fetch(0, 0, n);          // (a group may have no column at all)
@@ -345,22 +345,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       fence_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&h_ready);
-      // (cell j: four columns on)
-      float *const og = at(pg, col0 + base + i0, 16 * H), *const oc = at(pc, col0 + base + i0, 4 * H), *const oh = at(ph, col0 + base + i0, 4 * H);
-      float *const ohi = at(phi, col1 + base + i0, 4 * pitch), *const olo = at(plo, col1 + base + i0, 4 * pitch);
 #pragma unroll
       for (int j = 0; j < kCells; ++j) {
-        const uint32_t i = i0 + 4 * j;
+        const uint32_t i = i0 + 4 * j, sc = base + i;
         if (!live_u || i >= n) continue;
+        float* const og = at(pg, col0 + sc, 16 * H);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) og[(size_t)(16 * j + q) * H] = y[j][q];
-        oc[(size_t)(4 * j) * H] = cst[j];
-        oh[(size_t)(4 * j) * H] = hv[j];
+        for (int q = 0; q < 4; ++q) og[(size_t)q * H] = y[j][q];
+        *at(pc, col0 + sc, 4 * H) = cst[j];
+        *at(ph, col0 + sc, 4 * H) = hv[j];
         if (phi && i < n1) {
           float hi, lo;
           split_tf32(hm[j], hi, lo);
-          ohi[(size_t)(4 * j) * pitch] = hi;
-          olo[(size_t)(4 * j) * pitch] = lo;
+          *at(phi, col1 + sc, 4 * pitch) = hi;
+          *at(plo, col1 + sc, 4 * pitch) = lo;
         }
       }
       col0 = col1; col1 = col2; col2 = col3; n = n1;
@@ -670,8 +668,8 @@ uint32_t tc_smem(bool bwd, uint32_t H) {
 typedef void (*TcFwd)(RecFwd);
 typedef void (*TcBwd)(RecBwd);
 // The instance of a launch.  Widths in whole 64 units (whose planes have no padding) have instances of their own: with the strides known the addresses of a
-// cell's 16 - 23 accesses are a base and immediates instead of a third of all instructions.  256 units, 4096 columns of up to 100 steps: 1039 against 961 us
-// forward, 1392 against 1194 backward.
+// cell's 16 - 23 accesses are a base and immediates instead of a third of all instructions.  256 units, 4096 columns of up to 100 steps: 1039 against 951 us
+// forward, 1392 against 1194 backward; 64 and 128 units, 1400 columns: 108 -> 96 and 130 -> 106 with the copies, 142 -> 128 and 147 -> 135.
 TcFwd tc_fwd_kernel(uint32_t H, uint32_t pitch) {
   if (pitch && pitch != H) return k_rec_tc_fwd<0>;
   switch (H) {
