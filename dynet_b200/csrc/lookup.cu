@@ -317,26 +317,36 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_ids32(const uint32_t* __r
 // Merges the sorted runs of k_sort_ids (run p = positions [p kSortMax, ...), sorted by (id, position)) into one sorted list:
 // one thread per element, whose place is the number of smaller keys in every run.  Positions grow with the run number, so
 // among equal ids the earlier run comes first: runs before the element's own count their ids <= id, later runs their ids < id.
+// A search is a chain of loads; eight runs are searched side by side, in steps of halving length (107 000 ids, 27 runs: 51 us one after
+// the other, 29 here; 13 400 ids, 4 runs: 15 and 7).
 __global__ void __launch_bounds__(256) k_merge_runs(const uint32_t* __restrict__ pos_run, const uint32_t* __restrict__ id_run,
                                                    uint32_t n, uint32_t* __restrict__ pos_out, uint32_t* __restrict__ id_out) {
   dyb_grid_dep_sync();
+  constexpr int kSide = 8;
   const uint32_t e = blockIdx.x * 256 + threadIdx.x;
   if (e >= n) return;
-  const uint32_t p = e / kSortMax, id = id_run[e];
+  const uint32_t p = e / kSortMax, id = id_run[e], pos = pos_run[e];
   const uint32_t npass = (n + kSortMax - 1) / kSortMax;
   uint32_t rank = e - p * kSortMax;
-  for (uint32_t q = 0; q < npass; ++q) {
-    if (q == p) continue;
-    const uint32_t* run = id_run + (size_t)q * kSortMax;
-    uint32_t lo = 0, hi = min((uint32_t)kSortMax, n - q * kSortMax);
-    const uint32_t bound = q < p ? id + 1 : id;   // count ids < bound  (id + 1 does not wrap: ids are below the vocabulary size)
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (run[mid] < bound) lo = mid + 1; else hi = mid;
+  for (uint32_t q0 = 0; q0 < npass; q0 += kSide) {
+    uint32_t at[kSide] = {};   // ids of run q0 + x known to lie below the bound
+#pragma unroll 1
+    for (uint32_t step = kSortMax; step; step >>= 1) {
+      uint32_t v[kSide];
+#pragma unroll
+      for (int x = 0; x < kSide; ++x) {
+        const uint32_t q = q0 + x, k = q * kSortMax + at[x] + step - 1;
+        v[x] = q < npass && at[x] + step <= (uint32_t)kSortMax && k < n ? id_run[k] : 0xffffffffu;
+      }
+#pragma unroll
+      for (int x = 0; x < kSide; ++x)
+        if (v[x] < (q0 + x < p ? id + 1 : id)) at[x] += step;   // (ids are below the vocabulary size: id + 1 does not wrap)
     }
-    rank += lo;
+#pragma unroll
+    for (int x = 0; x < kSide; ++x)
+      if (q0 + x != p) rank += at[x];
   }
-  pos_out[rank] = pos_run[e];
+  pos_out[rank] = pos;
   id_out[rank] = id;
 }
 
@@ -403,42 +413,78 @@ __global__ void __launch_bounds__(256) k_chunk_add(const float* __restrict__ g, 
     }
   }
 }
-// Pass B: the chunk in which a multi-chunk run starts adds the later pieces in chunk order and writes the row.
+// Pass B: the chunk in which a multi-chunk run starts adds the later pieces in chunk order and writes the row.  A frequent id runs over hundreds of chunks
+// (the most frequent word of a 107 k-token batch: ~500), which one warp adds 16 at a time, a round trip to memory each: runs of more than kCombineLong pieces are
+// left to the CTA, whose warps add a stretch each, the stretches' sums in order (107 000 tokens x 128:
+// 32 -> 8.8 us, 13 400: 10.2 -> 5.5).
+constexpr uint32_t kCombineLong = 32;
+template <int U>
+__device__ __forceinline__ void combine_pieces(float4& acc, const float* head, uint32_t slices, uint32_t c, uint32_t c_end) {
+#pragma unroll 1
+  for (; c < c_end; c += U) {
+    float4 piece[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c + u < c_end) piece[u] = ld4(head + (size_t)(c + u) * slices * 128);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c + u < c_end) add4(acc, piece[u]);
+  }
+}
 __global__ void __launch_bounds__(256) k_chunk_combine(float* __restrict__ all_grads, uint32_t E, const uint32_t* __restrict__ id_at,
                                                       uint32_t n, uint32_t slices, const float* __restrict__ head,
                                                       const float* __restrict__ tail) {
   dyb_grid_dep_sync();
+  __shared__ uint32_t long_first[8], long_end[8];   // (of warp w's run: its first later chunk, the chunk behind its last; equal: none)
+  __shared__ float4 part[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t nchunks = (n + kChunk - 1) / kChunk;
   const size_t work = (size_t)nchunks * slices;
-  for (size_t w = (size_t)blockIdx.x * 8 + warp; w < work; w += (size_t)gridDim.x * 8) {
+  for (size_t w0 = (size_t)blockIdx.x * 8; w0 < work; w0 += (size_t)gridDim.x * 8) {
+    const size_t w = w0 + warp;
     const uint32_t c = (uint32_t)(w / slices), sl = (uint32_t)(w % slices);
     const uint32_t k0 = c * kChunk, k1 = min(n, k0 + kChunk);
-    const uint32_t col = sl * 128 + lane * 4;
-    if (col >= E || k1 >= n) continue;
-    const uint32_t id = id_at[k1 - 1];
-    if (id_at[k1] != id) continue;                         // last run of the chunk does not continue
-    if (id_at[k0] == id && k0 > 0 && id_at[k0 - 1] == id) continue;   // it started earlier: not the owner
-    float4 acc = ld4(tail + ((size_t)c * slices + sl) * 128 + lane * 4);
-    // A frequent id runs over hundreds of chunks (the most frequent word of a 107 k-token batch: ~500).  The last chunk of
-    // the run is found by a binary search over the chunk heads (ids are sorted), then sixteen pieces are requested at a
-    // time; the adds stay in chunk order.
-    uint32_t lo = c + 1, hi = nchunks;   // first chunk in [lo, hi) whose head is another id
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (id_at[mid * kChunk] == id) lo = mid + 1; else hi = mid;
+    uint32_t first = 0, end = 0;
+    if (w < work && k1 < n) {
+      const uint32_t id = id_at[k1 - 1];
+      // its last run continues, and began here
+      if (id_at[k1] == id && !(id_at[k0] == id && k0 > 0 && id_at[k0 - 1] == id)) {
+        // The last chunk of the run by a binary search over the chunk heads (ids are sorted).
+        uint32_t lo = c + 1, hi = nchunks;   // first chunk in [lo, hi) whose head is another id
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (id_at[mid * kChunk] == id) lo = mid + 1; else hi = mid;
+        }
+        const uint32_t col = sl * 128 + lane * 4;
+        if (lo - c - 1 > kCombineLong) { first = c + 1; end = lo; }
+        else if (col < E) {
+          float4 acc = ld4(tail + ((size_t)c * slices + sl) * 128 + lane * 4);
+          combine_pieces<16>(acc, head + (size_t)sl * 128 + lane * 4, slices, c + 1, lo);
+          st4(all_grads + (size_t)id * E + col, acc);
+        }
+      }
     }
-    const uint32_t c_end = lo;
-    for (uint32_t c2 = c + 1; c2 < c_end; c2 += 16) {
-      float4 piece[16];
+    if (lane == 0) { long_first[warp] = first; long_end[warp] = end; }
+    if (!__syncthreads_or(first != end)) continue;
+    for (int x = 0; x < 8; ++x) {
+      const uint32_t from = long_first[x], to = long_end[x];
+      if (from == to) continue;
+      const uint32_t xc = (uint32_t)((w0 + x) / slices), xs = (uint32_t)((w0 + x) % slices), each = (to - from + 7) / 8, col = xs * 128 + lane * 4;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (col < E) {
+        if (warp == 0) acc = ld4(tail + ((size_t)xc * slices + xs) * 128 + lane * 4);
+        combine_pieces<8>(acc, head + (size_t)xs * 128 + lane * 4, slices, from + warp * each, min(to, from + (warp + 1) * each));
+      }
+      part[warp][lane] = acc;
+      __syncthreads();
+      if (warp == 0 && col < E) {
 #pragma unroll
-      for (int u = 0; u < 16; ++u)
-        if (c2 + u < c_end) piece[u] = ld4(head + ((size_t)(c2 + u) * slices + sl) * 128 + lane * 4);
-#pragma unroll
-      for (int u = 0; u < 16; ++u)
-        if (c2 + u < c_end) add4(acc, piece[u]);
+        for (int y = 1; y < 8; ++y) add4(acc, part[y][lane]);
+        st4(all_grads + (size_t)id_at[min(n, xc * kChunk + kChunk) - 1] * E + col, acc);
+      }
+      __syncthreads();
     }
-    st4(all_grads + (size_t)id * E + col, acc);
+    __syncthreads();   // (the next items' runs are not noted before every warp has seen these)
   }
 }
 
