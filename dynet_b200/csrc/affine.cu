@@ -8,6 +8,7 @@
 // A left operand with one batch element multiplies all batch columns of the right operand in one
 // product (N = cols * bd); otherwise the batch elements are multiplied one by one, a batch-1 operand
 // being reused for every element (and a batch-1 result summed over them).
+#include "lstm_rec_api.h"
 #include "common.cuh"
 #include "gemm.cuh"
 #include "reduce.cuh"
@@ -75,15 +76,16 @@ int mm_fwd(dyb200_ctx* ctx, const dyb200_tensor* l, const dyb200_tensor* r, dyb2
   return DYB200_OK;
 }
 
-// y += l^T * r   (l: M x K, r: M x N, y: K x N)
-int mm_transp_l_acc(dyb200_ctx* ctx, const dyb200_tensor* l, const dyb200_tensor* r, dyb200_tensor* y, int a_is_param) {
+// y (+)= l^T * r   (l: M x K, r: M x N, y: K x N)
+int mm_transp_l_acc(dyb200_ctx* ctx, const dyb200_tensor* l, const dyb200_tensor* r, dyb200_tensor* y, int a_is_param, bool overwrite) {
   const uint32_t M = t_rows(l), K = t_cols(l), N = t_cols(r);
   const uint32_t max_b = l->bd > r->bd ? l->bd : r->bd;
   if (l->bd == 1 && y->bd == r->bd) {
     GemmPair p{l->v, M, 1, r->v, M, 0, M, nullptr, 0, 0, a_is_param};
-    GemmEpilogue e{EPI_ACCUM, y->v, K, nullptr, 0, 0.f, nullptr, 0, 0};
+    GemmEpilogue e{overwrite ? EPI_STORE : EPI_ACCUM, y->v, K, nullptr, 0, 0.f, nullptr, 0, 0};
     return dyb200_gemm_fused(ctx, K, N * y->bd, 1, &p, e);
   }
+  if (overwrite) DYB_CUDA(ctx, cudaMemsetAsync(y->v, 0, t_size(y) * sizeof(float), ctx->stream));
   for (uint32_t b = 0; b < max_b; ++b) {
     GemmPair p{batch_ptr(l, b), M, 1, batch_ptr(r, b), M, 0, M, nullptr, 0, 0, 0};
     GemmEpilogue e{EPI_ACCUM, y->v + (size_t)(b % y->bd) * K * N, K, nullptr, 0, 0.f, nullptr, 0, 0};
@@ -93,15 +95,16 @@ int mm_transp_l_acc(dyb200_ctx* ctx, const dyb200_tensor* l, const dyb200_tensor
   return DYB200_OK;
 }
 
-// y += l * r^T   (l: M x N, r: K x N, y: M x K)
-int mm_transp_r_acc(dyb200_ctx* ctx, const dyb200_tensor* l, const dyb200_tensor* r, dyb200_tensor* y) {
+// y (+)= l * r^T   (l: M x N, r: K x N, y: M x K)
+int mm_transp_r_acc(dyb200_ctx* ctx, const dyb200_tensor* l, const dyb200_tensor* r, dyb200_tensor* y, bool overwrite) {
   const uint32_t M = t_rows(l), N = t_cols(l), K = t_rows(r);
   const uint32_t max_b = l->bd > r->bd ? l->bd : r->bd;
   if (y->bd == 1 && l->bd == r->bd) {
     GemmPair p{l->v, M, 0, r->v, K, 1, N * l->bd, nullptr, 0, 0, 0};
-    GemmEpilogue e{EPI_ACCUM, y->v, M, nullptr, 0, 0.f, nullptr, 0, 0};
+    GemmEpilogue e{overwrite ? EPI_STORE : EPI_ACCUM, y->v, M, nullptr, 0, 0.f, nullptr, 0, 0};
     return dyb200_gemm_fused(ctx, M, K, 1, &p, e);
   }
+  if (overwrite) DYB_CUDA(ctx, cudaMemsetAsync(y->v, 0, t_size(y) * sizeof(float), ctx->stream));
   for (uint32_t b = 0; b < max_b; ++b) {
     GemmPair p{batch_ptr(l, b), M, 0, batch_ptr(r, b), K, 1, N, nullptr, 0, 0, 0};
     GemmEpilogue e{EPI_ACCUM, y->v + (size_t)(b % y->bd) * M * K, M, nullptr, 0, 0.f, nullptr, 0, 0};
@@ -145,8 +148,9 @@ int dyb200_matmul_bwd(DYB200_BWD_ARGS) {
   if (rc) return rc;
   DYB_CHECK_ARG(ctx, dEdxi && dEdxi->v && t_batch_size(dEdxi) == t_batch_size(&xs[i]) && dEdxi->bd == xs[i].bd,
                 "MatrixMultiply: gradient shape differs from argument %u", i);
-  if (i == 0) return mm_transp_r_acc(ctx, dEdf, &xs[1], dEdxi);
-  return mm_transp_l_acc(ctx, &xs[0], dEdf, dEdxi, (attr_flags(attrs) & DYB200_GEMM_A_IS_PARAM) ? 1 : 0);
+  const bool overwrite = (attr_flags(attrs) & DYB200I_OVERWRITE) != 0;
+  if (i == 0) return mm_transp_r_acc(ctx, dEdf, &xs[1], dEdxi, overwrite);
+  return mm_transp_l_acc(ctx, &xs[0], dEdf, dEdxi, (attr_flags(attrs) & DYB200_GEMM_A_IS_PARAM) ? 1 : 0, overwrite);
 }
 
 int dyb200_affine_transform_fwd(DYB200_FWD_ARGS) {
@@ -194,8 +198,10 @@ int dyb200_affine_transform_bwd(DYB200_BWD_ARGS) {
   DYB_CHECK_ARG(ctx, dEdf && dEdf->v && dEdxi && dEdxi->v, "AffineTransform: null tensor");
   DYB_CHECK_ARG(ctx, t_batch_size(dEdxi) == t_batch_size(&xs[i]) && dEdxi->bd == xs[i].bd,
                 "AffineTransform: gradient shape differs from argument %u", i);
+  const bool overwrite = (attr_flags(attrs) & DYB200I_OVERWRITE) != 0;
   if (i == 0) {
     const size_t dx_size = t_size(dEdxi), df_size = t_size(dEdf);
+    if (overwrite) DYB_CUDA(ctx, cudaMemsetAsync(dEdxi->v, 0, dx_size * sizeof(float), ctx->stream));
     if (dx_size == df_size) {
       const int vec = dx_size % 4 == 0 && aligned16(dEdf->v) && aligned16(dEdxi->v);
       dyb_launch(k_add_into, stream_grid(ctx, dx_size / 4 + 1, kThreads), kThreads, 0, ctx, dEdf->v, dEdxi->v, dx_size, vec);
@@ -209,8 +215,8 @@ int dyb200_affine_transform_bwd(DYB200_BWD_ARGS) {
   const int k = (i % 2 == 1) ? (int)i : (int)i - 1;   // index of the left operand of this product
   int rc = check_product(ctx, &xs[k], &xs[k + 1], dEdf, "AffineTransform");
   if (rc) return rc;
-  if (i % 2 == 1) return mm_transp_r_acc(ctx, dEdf, &xs[i + 1], dEdxi);
-  return mm_transp_l_acc(ctx, &xs[i - 1], dEdf, dEdxi, (attr_flags(attrs) & DYB200_GEMM_A_IS_PARAM) ? 1 : 0);
+  if (i % 2 == 1) return mm_transp_r_acc(ctx, dEdf, &xs[i + 1], dEdxi, overwrite);
+  return mm_transp_l_acc(ctx, &xs[i - 1], dEdf, dEdxi, (attr_flags(attrs) & DYB200_GEMM_A_IS_PARAM) ? 1 : 0, overwrite);
 }
 
 }  // extern "C"

@@ -287,6 +287,7 @@ struct BwdWideCall {
   float* dx; const float* mx; int mx_full; const float* mh; int mh_full;   // (dx null: not wanted)
   float* db;
   float *dn_hi, *dn_lo; uint32_t dn_pitch;   // TF32 planes of the columns' dgates, to be filled
+  int fresh_dx, fresh_dc;        // dx is written, whatever it holds; dc holds nothing yet: zeros from outside
 };
 int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q);
 // db += row sums of dgates, part = [step][tile][G], tiles in order and then the steps (at most kDbMaxSteps); clears the counters at `done`, if any

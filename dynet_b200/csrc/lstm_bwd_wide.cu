@@ -48,6 +48,7 @@ struct BwdWide {
   float* part;                      // row sums of dgates: [step in sweep order][column block, rank][4H]
   const float* mask; int mask_full; // of the result's rows; full: one column per batch column
   float* dx; uint32_t columns;      // dx only
+  int fresh_dx, fresh_dc;           // dx is written and not added to; dE/dc of a step before it is added to: zeros, whatever dc holds
   uint32_t* done;                   // a counter per column block, zero at launch (cleared by the launch that sums up db)
   uint32_t* flags;
 };
@@ -79,8 +80,8 @@ __device__ __forceinline__ void cell_load(const BwdWide& a, const CellUnits& q, 
   in.c = ldu<VEC>(a.cs + (size_t)t * HB + e, q.left);
   in.cp = ldu<VEC>((t ? a.cs + (size_t)(t - 1) * HB : a.c0) + e, q.left);
   const float* dcp = t ? a.dc + (size_t)(t - 1) * HB : a.dc_prev;
-  in.dci = a.dc ? ldu_cg<VEC>(a.dc + (size_t)t * HB + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
-  in.dcp = dcp ? ldu_cg<VEC>(dcp + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
+  in.dci = a.dc && !(a.fresh_dc && t == a.T - 1) ? ldu_cg<VEC>(a.dc + (size_t)t * HB + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
+  in.dcp = dcp && !a.fresh_dc ? ldu_cg<VEC>(dcp + e, q.left) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 template <bool VEC>
 __device__ __forceinline__ void planes_out(const BwdWide& a, const CellUnits& q, const float4 (&p)[4], uint32_t t, uint32_t n) {   // dgates for the weight gradients
@@ -525,13 +526,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
               if (n >= a.B) continue;
               const size_t e = (size_t)n * a.H + u;
               const float* g = a.gates + (size_t)(t - 1) * 4 * HB + (size_t)n * 4 * a.H + u;
-              const float* ps[7] = {g, g + a.H, g + 2 * a.H, g + 3 * a.H, (t > 1 ? a.cs + (size_t)(t - 2) * HB : a.c0) + e, dst + e, t > 1 ? a.dc + (size_t)(t - 2) * HB + e : dst + e};
+              const float* ps[7] = {g, g + a.H, g + 2 * a.H, g + 3 * a.H, (t > 1 ? a.cs + (size_t)(t - 2) * HB : a.c0) + e, dst + e, t > 1 && !a.fresh_dc ? a.dc + (size_t)(t - 2) * HB + e : dst + e};
 #pragma unroll
               for (int q = 0; q < 7; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(ps[q]));
             }
         }
       }
-      if (!REC && own && (te & 7) == 0)   // (the values that this tile adds to)
+      if (!REC && own && !a.fresh_dx && (te & 7) == 0)   // (the values that this tile adds to)
 #pragma unroll
         for (int hh = 0; hh < BNT / 64; ++hh)
 #pragma unroll
@@ -610,7 +611,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             const float4 x = small_parts(a, seq0 + n, m);
             for (uint32_t q = 0; q < 4 && m + q < a.M; ++q) {
               float* d = dst + (size_t)n * a.M + m + q;
-              *d = __fmaf_rn((&x.x)[q], a.mask ? a.mask[m + q + (a.mask_full ? (size_t)(REC ? n : n % a.B) * a.M : 0)] : 1.f, __ldcg(d));
+              *d = __fmaf_rn((&x.x)[q], a.mask ? a.mask[m + q + (a.mask_full ? (size_t)(REC ? n : n % a.B) * a.M : 0)] : 1.f, !REC && a.fresh_dx ? 0.f : __ldcg(d));
             }
           }
         }
@@ -627,7 +628,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             mk[g] = make_float4(1.f, 1.f, 1.f, 1.f);
             old[g] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (!own || n[g] >= cols || !vec) continue;
-            old[g] = REC ? ldu_cg<VEC>(dst + (size_t)n[g] * a.M + m, left) : __ldcg(reinterpret_cast<const float4*>(dst + (size_t)n[g] * a.M + m));
+            if (REC || !a.fresh_dx || quads) old[g] = REC ? ldu_cg<VEC>(dst + (size_t)n[g] * a.M + m, left) : __ldcg(reinterpret_cast<const float4*>(dst + (size_t)n[g] * a.M + m));
             if (a.mask) {
               const float* mp = a.mask + m + (a.mask_full ? (size_t)(REC ? n[g] : n[g] % a.B) * a.M : 0);
               mk[g] = REC ? ldu<VEC>(mp, left) : ld4(mp);
@@ -657,7 +658,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bwd_wide(const __grid_constant_
             if (vec || !own || !ok) continue;
             for (uint32_t q = 0; q < 4 && m + q < a.M; ++q) {
               float* d = dst + (size_t)n[g] * a.M + m + q;
-              *d = __fmaf_rn((&v.x)[q], a.mask ? a.mask[m + q + (a.mask_full ? (size_t)(n[g] % a.B) * a.M : 0)] : 1.f, *d);
+              *d = __fmaf_rn((&v.x)[q], a.mask ? a.mask[m + q + (a.mask_full ? (size_t)(n[g] % a.B) * a.M : 0)] : 1.f, !REC && a.fresh_dx && !quads ? 0.f : *d);
             }
           }
           if (REC && t && ok) {
@@ -814,7 +815,7 @@ int dyb200_bwd_wide(dyb200_ctx* ctx, const BwdWideCall& q) {
   a.dn_hi = q.dn_hi; a.dn_lo = q.dn_lo; a.dn_pitch = q.dn_pitch;
   a.d16_hi = (__half*)p16; a.d16_lo = a.d16_hi + plane;
   a.dsc = (uint32_t*)words; a.dsc_ld = columns; a.W = q.Wh; a.wscale = wh.scale; a.part = (float*)part;
-  a.mask = q.mh; a.mask_full = q.mh_full;
+  a.mask = q.mh; a.mask_full = q.mh_full; a.fresh_dx = q.fresh_dx; a.fresh_dc = q.fresh_dc;
   a.done = ctx->dev_flags + DYB200_DEV_BWD0; a.flags = ctx->dev_flags;
   TmapPack tm;
   memset(&tm, 0, sizeof(tm));

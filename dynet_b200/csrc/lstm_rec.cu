@@ -630,13 +630,13 @@ int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float
 // ---- products over all columns around the recurrence -----------------------------------------------------------------------
 namespace {
 
-// dst += src .* mask, all `rows` x n; the mask repeats every `period` columns (0: one column for all)
+// dst (+)= src .* mask, all `rows` x n; the mask repeats every `period` columns (0: one column for all)
 __global__ void __launch_bounds__(256) k_masked_add(const float* __restrict__ src, const float* __restrict__ mask, uint32_t rows, uint32_t period,
-                                                    size_t total, float* __restrict__ dst) {
+                                                    size_t total, float* __restrict__ dst, int overwrite) {
   dyb_grid_dep_sync();
   for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (size_t)gridDim.x * 256) {
     const uint32_t n = (uint32_t)(e / rows), r = (uint32_t)(e % rows);
-    dst[e] = __fmaf_rn(src[e], mask[r + (period ? (size_t)rows * (n % period) : 0)], dst[e]);
+    dst[e] = __fmaf_rn(src[e], mask[r + (period ? (size_t)rows * (n % period) : 0)], overwrite ? 0.f : dst[e]);
   }
 }
 
@@ -708,7 +708,7 @@ int dyb200i_rec_bwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint
 }
 
 int dyb200i_rec_dx(dyb200_ctx* ctx, dyb200_wgrad* w, const float* Wx, uint32_t I, uint32_t H, uint32_t columns, const float* mask_x, int mask_full,
-                   uint32_t period, float* dx) {
+                   uint32_t period, float* dx, int overwrite) {
   { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
   const uint32_t G = 4 * H;
   PackedOp A, D;
@@ -716,7 +716,7 @@ int dyb200i_rec_dx(dyb200_ctx* ctx, dyb200_wgrad* w, const float* Wx, uint32_t I
   int rc = dyb200_tc_param(ctx, Wx, G, true, I, G, &A);
   if (rc) return rc;
   if (!mask_x) {
-    GemmEpilogue e{EPI_ACCUM, dx, I, nullptr, 0, 0.f, nullptr, 0, 0};
+    GemmEpilogue e{overwrite ? EPI_STORE : EPI_ACCUM, dx, I, nullptr, 0, 0.f, nullptr, 0, 0};
     return dyb200_tc_gemm_packed(ctx, I, columns, 1, &A, &D, e);
   }
   void* tmp;
@@ -724,7 +724,7 @@ int dyb200i_rec_dx(dyb200_ctx* ctx, dyb200_wgrad* w, const float* Wx, uint32_t I
   GemmEpilogue e{EPI_STORE, (float*)tmp, I, nullptr, 0, 0.f, nullptr, 0, 0};
   if ((rc = dyb200_tc_gemm_packed(ctx, I, columns, 1, &A, &D, e))) return rc;
   const size_t total = (size_t)I * columns;
-  dyb_launch(k_masked_add, stream_grid(ctx, total, 256), 256, 0, ctx, (const float*)tmp, mask_x, I, mask_full ? period : 0u, total, dx);
+  dyb_launch(k_masked_add, stream_grid(ctx, total, 256), 256, 0, ctx, (const float*)tmp, mask_x, I, mask_full ? period : 0u, total, dx, overwrite);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }

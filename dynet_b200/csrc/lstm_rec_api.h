@@ -29,9 +29,20 @@ int dyb200i_rec_fwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint
 /* columns = all of them: marks the gate-gradient planes of w as filled. */
 int dyb200i_rec_bwd(dyb200_ctx* ctx, int ndir, const dyb200i_rec_dir* dirs, uint32_t H, uint32_t T, uint32_t N, const uint32_t* prefix_dev,
                     int mask_full, uint32_t columns);
-/* dx += Wx^T dgates (.* mask_x, which repeats every `period` columns when mask_full), dgates = the planes left in w by rec_bwd. */
+/* dx += Wx^T dgates (.* mask_x, which repeats every `period` columns when mask_full), dgates = the planes left in w by rec_bwd; overwrite: dx = that. */
 int dyb200i_rec_dx(dyb200_ctx* ctx, struct dyb200_wgrad* w, const float* Wx, uint32_t I, uint32_t H, uint32_t columns, const float* mask_x,
-                   int mask_full, uint32_t period, float* dx);
+                   int mask_full, uint32_t period, float* dx, int overwrite);
+
+/* A driver whose gradient buffers hold nothing yet says so instead of clearing them: the clear is a pass of writes, and adding to zeros one of reads.
+ * A bit of the flags of dyb200_affine_transform_bwd and dyb200_matmul_bwd (the gradient wanted) and of dyb200_softmax_output_bwd_fused (dh alone): */
+#define DYB200I_OVERWRITE 0x80000000u
+/* dyb200_vanilla_lstm_seq_bwd with `fresh` bits: dx_all is written, whatever it holds; dE/dc is zero from outside and not wanted (dc_all: scratch memory). */
+enum { DYB200I_FRESH_DX = 1, DYB200I_FRESH_DC = 2 };
+int dyb200i_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0, const dyb200_tensor* Wx, const dyb200_tensor* Wh,
+                         const dyb200_tensor* mask_x, const dyb200_tensor* mask_h, const dyb200_lstm_gates_attrs* attrs, const dyb200_tensor* gates_all,
+                         const dyb200_tensor* c_all, const dyb200_tensor* h_all, dyb200_tensor* dh_all, dyb200_tensor* dc_all, dyb200_tensor* dx_all,
+                         dyb200_tensor* dWx, dyb200_tensor* dWh, dyb200_tensor* db, struct dyb200_wgrad* deferred, uint32_t steps, unsigned fresh,
+                         dyb200_ctx* ctx);
 
 /* The dependent-launch setting in force.  set >= 0 changes it, unless the caller of the library has chosen one. */
 int dyb200i_dependent_launch(dyb200_ctx* ctx, int set);

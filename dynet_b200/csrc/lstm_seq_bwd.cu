@@ -609,6 +609,13 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
                                 const dyb200_tensor* c_all, const dyb200_tensor* h_all, dyb200_tensor* dh_all, dyb200_tensor* dc_all,
                                 dyb200_tensor* dx_all, dyb200_tensor* dWx, dyb200_tensor* dWh, dyb200_tensor* db,
                                 dyb200_wgrad* deferred, uint32_t steps, dyb200_ctx* ctx) {
+  return dyb200i_lstm_seq_bwd(x_all, h0, c0, Wx, Wh, mask_x, mask_h, attrs, gates_all, c_all, h_all, dh_all, dc_all, dx_all, dWx, dWh, db, deferred, steps, 0, ctx);
+}
+
+int dyb200i_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0, const dyb200_tensor* Wx, const dyb200_tensor* Wh,
+                         const dyb200_tensor* mask_x, const dyb200_tensor* mask_h, const dyb200_lstm_gates_attrs* attrs, const dyb200_tensor* gates_all,
+                         const dyb200_tensor* c_all, const dyb200_tensor* h_all, dyb200_tensor* dh_all, dyb200_tensor* dc_all, dyb200_tensor* dx_all,
+                         dyb200_tensor* dWx, dyb200_tensor* dWh, dyb200_tensor* db, dyb200_wgrad* deferred, uint32_t steps, unsigned fresh, dyb200_ctx* ctx) {
   DYB_CHECK_ARG(ctx, x_all && h0 && c0 && Wx && Wh && attrs && gates_all && c_all && h_all && dh_all && dc_all && db && steps > 0 &&
                          (deferred || (dWx && dWh)), "lstm_seq_bwd: null argument");
   DYB_CHECK_ARG(ctx, (attrs->dropout != 0) == (mask_x != nullptr && mask_h != nullptr), "lstm_seq_bwd: masks must be given exactly when dropout is set");
@@ -635,12 +642,19 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
       dyb200_bwd_wide_plan(ctx, H, B, &wide_ncb, &wide_S)) {
     { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
     BwdWideCall q{I, H, B, T, Wx->v, Wh->v, gates_all->v, c_all->v, c0->v, dh_all->v, dc_all->v, nullptr, nullptr, dx_all ? dx_all->v : nullptr,
-                  mx, mx_full, mh, mh_full, db->v, nullptr, nullptr, 0};
+                  mx, mx_full, mh, mh_full, db->v, nullptr, nullptr, 0, (fresh & DYB200I_FRESH_DX) != 0, (fresh & DYB200I_FRESH_DC) != 0};
     if ((rc = dyb200_wgrad_reserve_a_at(deferred, 0, T * B, &q.dn_hi, &q.dn_lo, &q.dn_pitch, ctx))) return rc;
     rc = dyb200_bwd_wide(ctx, q);
     if (rc != DYB200_ENOMEM) return rc;
     wide_fits = false;   // (no room for the pairs of all steps: the single-step calls, with those of one)
   }
+
+  // (the forms below that know no fresh buffers get cleared ones)
+  auto clear_fresh = [&]() -> int {
+    if ((fresh & DYB200I_FRESH_DX) && dx_all) DYB_CUDA(ctx, cudaMemsetAsync(dx_all->v, 0, IB * T * sizeof(float), ctx->stream));
+    if (fresh & DYB200I_FRESH_DC) DYB_CUDA(ctx, cudaMemsetAsync(dc_all->v, 0, HB * T * sizeof(float), ctx->stream));
+    return DYB200_OK;
+  };
 
   // ---- all steps in one kernel, when its CTAs can all be resident ----
   LstmBwdTiling tl{64, 1, 1};
@@ -687,6 +701,7 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
     a.flags = ctx->dev_flags;
     const dim3 grid(tiles_m, tiles_n / ncb, S);
     const double flops = 2.0 * (I + H) * (double)B * G * T;
+    if ((rc = clear_fresh())) return rc;
     if (S > 1) rc = bn == 64 ? launch_seq_bwd<64, true>(ctx, tm, a, grid, flops) : launch_seq_bwd<128, true>(ctx, tm, a, grid, flops);
     else rc = bn == 64 ? launch_seq_bwd<64, false>(ctx, tm, a, grid, flops) : launch_seq_bwd<128, false>(ctx, tm, a, grid, flops);
     if (rc) return rc;
@@ -701,12 +716,13 @@ int dyb200_vanilla_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor*
       dyb200i_rec_takes(ctx, H, T, B, 1)) {
     dyb200i_rec_dir d;
     memset(&d, 0, sizeof(d));
-    d.Wh = Wh->v; d.c0 = c0->v; d.mask_h = mh; d.gates = gates_all->v; d.c = c_all->v; d.dh = dh_all->v; d.dc = dc_all->v; d.db = db->v; d.w = deferred;
+    d.Wh = Wh->v; d.c0 = c0->v; d.mask_h = mh; d.gates = gates_all->v; d.c = c_all->v; d.dh = dh_all->v; d.dc = fresh & DYB200I_FRESH_DC ? nullptr : dc_all->v; d.db = db->v; d.w = deferred;
     if ((rc = dyb200i_rec_bwd(ctx, 1, &d, H, T, B, nullptr, mh_full, T * B))) return rc;
-    return dyb200i_rec_dx(ctx, deferred, Wx->v, I, H, T * B, mx, mx_full, B, dx_all->v);
+    return dyb200i_rec_dx(ctx, deferred, Wx->v, I, H, T * B, mx, mx_full, B, dx_all->v, (fresh & DYB200I_FRESH_DX) != 0);
   }
 
   // ---- without the kernel: one call per time step ----
+  if (first > 0 && (rc = clear_fresh())) return rc;
   for (uint32_t t = first; t-- > 0;) {
     dyb200_tensor x = *x_all, hp = *h0, cp = *c0, g = *gates_all, c = *c_all, dh = *dh_all, dc = *dc_all, dx, dhp = *dh_all, dcp = *dc_all;
     x.bd = B; x.v = x_all->v + (size_t)t * IB;

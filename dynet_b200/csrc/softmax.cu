@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "gemm.cuh"
+#include "lstm_rec_api.h"
 #include "reduce.cuh"
 
 namespace {
@@ -990,9 +991,10 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
     dyb200_tensor dv = *x;   // the gradient of x, with x's shape
     dv.v = dx_scratch->v;
     dyb200_tensor xs[3] = {*db, *R, *h};
-    dyb200_affine_attrs at = {flags};
-    for (unsigned i = 0; i < 3 && !rc; ++i)
+    for (unsigned i = 0; i < 3 && !rc; ++i) {
+      dyb200_affine_attrs at = {i == 2 ? flags : flags & ~DYB200I_OVERWRITE};
       rc = dyb200_affine_transform_bwd(xs, 3, x, &dv, i, i == 0 ? db : i == 1 ? dR : dh, &at, nullptr, ctx);
+    }
     return rc;
   }
   int rc;
@@ -1045,8 +1047,8 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
     GemmEpilogue e{EPI_ACCUM, dR->v, V, nullptr, 0, 0.f, nullptr, 0, 0};
     if ((rc = dyb200_tc_gemm_packed(ctx, V, H, 1, &dA, &hT, e))) return rc;
   }
-  // dh += R^T d : M = H, N = n, K = V
-  GemmEpilogue e{EPI_ACCUM, dh->v, H, nullptr, 0, 0.f, nullptr, 0, 0};
+  // dh (+)= R^T d : M = H, N = n, K = V
+  GemmEpilogue e{flags & DYB200I_OVERWRITE ? EPI_STORE : EPI_ACCUM, dh->v, H, nullptr, 0, 0.f, nullptr, 0, 0};
   return dyb200_tc_gemm_packed(ctx, H, n, 1, &RT, &dB, e);
 }
 

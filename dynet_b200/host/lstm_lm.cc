@@ -120,7 +120,7 @@ size_t plan(const dyb200h_lm_config& c, Lm* m, char* base, size_t size) {
   float* dh = a.take<float>(TL * HB);
   float* dc = a.take<float>(TL * HB);
   float* dgates = a.take<float>(TL * GB);
-  // (the fused driver never stores the gate gradients in fp32: their part is not cleared)
+  // (the fused driver never stores the gate gradients in fp32: their part is not cleared.  Layer by layer nothing is: every buffer is written before it is added to)
   size_t d1 = c.fused ? (size_t)((char*)dgates - base) : a.off;
   if (m) {
     m->tok = tok; m->x = x; m->gates = gates; m->cs = cs; m->hs = hs; m->r = r; m->aux = aux; m->errs = errs;
@@ -271,7 +271,7 @@ void step_body(Lm& m, const float* const* masks, float* loss_dev, int phase = -1
   if (do_fwd) throw_status(dev, dyb200_sum_all(m.errs, (size_t)T * B, loss_dev, 0, dev.ctx));
 
   // ---------------- backward ----------------
-  if (do_fwd) CU(cudaMemsetAsync(m.dact, 0, m.dact_bytes, st));
+  if (do_fwd && !layer_major) CU(cudaMemsetAsync(m.dact, 0, m.dact_bytes, st));
   Tensor tgR(Dim({V, H}), m.g[1 + 3 * L]), tgbias(Dim({V}), m.g[2 + 3 * L]);
   if (do_fwd && c.fused) {
     Tensor tones(Dim({1}, TB), m.ones), tdr(Dim({V}, TB), m.dr), tdhall(Dim({H}, TB), m.dh + at(0, L - 1) * HB);
@@ -279,7 +279,8 @@ void step_body(Lm& m, const float* const* masks, float* loss_dev, int phase = -1
     // dh += R^T dr) in one: dr is written straight into the operand layouts of the two products
     dyb200_tensor cr = to_c(rall), ch = to_c(hall), cR = to_c(tR), cones = to_c(tones), cdr = to_c(tdr);
     dyb200_tensor cgb = to_c(tgbias), cgR = to_c(tgR), cdh = to_c(tdhall);
-    throw_status(dev, dyb200_softmax_output_bwd_fused(&cr, &ch, &cR, &cones, m.aux, &cgR, &cgb, &cdh, &cdr, DYB200_GEMM_A_IS_PARAM, dev.ctx));
+    throw_status(dev, dyb200_softmax_output_bwd_fused(&cr, &ch, &cR, &cones, m.aux, &cgR, &cgb, &cdh, &cdr,
+                                                     DYB200_GEMM_A_IS_PARAM | (layer_major ? DYB200I_OVERWRITE : 0u), dev.ctx));
   }
   Tensor tones(Dim({1}, B), m.ones);
   const uint32_t pass0 = phase < 0 ? 0u : (phase == 0 ? L : (uint32_t)phase - 1), pass1 = phase < 0 ? (layer_major ? L : 1u) : (phase == 0 ? L : (uint32_t)phase);
@@ -300,8 +301,8 @@ void step_body(Lm& m, const float* const* masks, float* loss_dev, int phase = -1
                   cg = to_c(gall), cc = to_c(call), ch = to_c(hall_l), cdh = to_c(dhall), cdc = to_c(dcall), cdx = to_c(dxall),
                   cgWx = to_c(gWx), cgWh = to_c(gWh), cgb = to_c(gb);
     dyb200_lstm_gates_attrs at = {c.dropout ? 1 : 0, 0.f, 1.f};
-    throw_status(dev, dyb200_vanilla_lstm_seq_bwd(&cxa, &ch0, &cc0, &cWx, &cWh, c.dropout ? &cmx : nullptr, c.dropout ? &cmh : nullptr, &at,
-                                                  &cg, &cc, &ch, &cdh, &cdc, &cdx, &cgWx, &cgWh, &cgb, m.wg_layer[l], T, dev.ctx));
+    throw_status(dev, dyb200i_lstm_seq_bwd(&cxa, &ch0, &cc0, &cWx, &cWh, c.dropout ? &cmx : nullptr, c.dropout ? &cmh : nullptr, &at,
+                                           &cg, &cc, &ch, &cdh, &cdc, &cdx, &cgWx, &cgWh, &cgb, m.wg_layer[l], T, DYB200I_FRESH_DX | DYB200I_FRESH_DC, dev.ctx));
   } else
   for (uint32_t tt = T; tt-- > 0;) {
     if (!c.fused) {

@@ -138,15 +138,16 @@ size_t plan(const dyb200h_tagger_config& c, uint32_t S, uint32_t N, Tagger* t, c
   float* errs = a.take<float>(N); uint32_t* ids = a.take<uint32_t>(ids_words(N, N)); float* ones = a.take<float>(N);
   float* zeros = a.take<float>(H * S); float* scalars = a.take<float>(64);
   float** tbl = a.take<float*>(8 * (size_t)N); size_t* len = a.take<size_t>(N);
+  // written before anything is added to them
+  for (int k = 0; k < 2; ++k) d[k].dh = a.take<float>(H * N);
+  float* dhf = a.take<float>(H * N); float* dhr = a.take<float>(H * N);
+  float* dth = a.take<float>((size_t)c.TH * N);
   // everything below is zeroed by one memset per pass
   a.off = (a.off + 255) & ~(size_t)255;
   const size_t z0 = a.off;
-  for (int k = 0; k < 2; ++k) d[k].dh = a.take<float>(H * N);
+  float* dpre = a.take<float>((size_t)c.TH * N); float* dlogits = a.take<float>((size_t)c.NT * N);
+  const size_t z_rec = a.off;                     // (with the recurrence kernels dx is written, and dE/dc zero where none is given)
   d[0].dx = d[1].dx = a.take<float>(2 * E * N);   // (the reverse direction's columns follow the forward direction's)
-  float* dhf = a.take<float>(H * N); float* dhr = a.take<float>(H * N);
-  float* dth = a.take<float>((size_t)c.TH * N); float* dpre = a.take<float>((size_t)c.TH * N);
-  float* dlogits = a.take<float>((size_t)c.NT * N);
-  const size_t z_rec = a.off;                     // (the recurrence kernels take dE/dc as zero where none is given)
   for (int k = 0; k < 2; ++k) d[k].dc = a.take<float>(H * N);
   const size_t z1 = a.off;
   if (t) {
@@ -307,17 +308,25 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   pnls.backward_dev_impl(dev, {&tlog}, terrs, tones, 0, tdlog);
   affine.backward_dev_impl(dev, xs2, tlog, tdlog, 0, gtbias);
   affine.backward_dev_impl(dev, xs2, tlog, tdlog, 1, gth2t);
-  affine.backward_dev_impl(dev, xs2, tlog, tdlog, 2, tdth);
+  // (the gradients of activations are written, not added to a cleared buffer)
+  auto input_grad = [&](const std::vector<const Tensor*>& xs, const Tensor& fx, const Tensor& dEdf, unsigned i, Tensor& dEdxi) {
+    dyb200_tensor cxs[5], cfx = to_c(fx), cd = to_c(dEdf), cdx = to_c(dEdxi);
+    for (size_t k = 0; k < xs.size(); ++k) cxs[k] = to_c(*xs[k]);
+    const dyb200_affine_attrs fresh = {DYB200I_OVERWRITE};
+    throw_status(dev, dyb200_affine_transform_bwd(cxs, (int)xs.size(), &cfx, &cd, i, &cdx, &fresh, nullptr, dev.ctx));
+  };
+  input_grad(xs2, tlog, tdlog, 2, tdth);
   tanh_node.backward_dev_impl(dev, {&tpre}, tth, tdth, 0, tdpre);
   affine.backward_dev_impl(dev, xs1, tpre, tdpre, 0, gthb);
   affine.backward_dev_impl(dev, xs1, tpre, tdpre, 1, gl2th);
-  affine.backward_dev_impl(dev, xs1, tpre, tdpre, 2, tdhf);
+  input_grad(xs1, tpre, tdpre, 2, tdhf);
   affine.backward_dev_impl(dev, xs1, tpre, tdpre, 3, gr2th);
-  affine.backward_dev_impl(dev, xs1, tpre, tdpre, 4, tdhr);
-  // accumulate_tensors: the token-major gradients back into the steps' dE/dh
+  input_grad(xs1, tpre, tdpre, 4, tdhr);
+  // accumulate_tensors: the token-major gradients back into the steps' dE/dh.  Every column of dE/dh belongs to one token and holds nothing yet, so that it is a copy
+  // (16 bytes of traffic per value less: a clear, and reading what is added to).
   for (int dr = 0; dr < 2; ++dr) {
     if (m.time_movers) CU(cudaEventRecord(m.ev[4 + 2 * dr], st));
-    gpu::parallel_accumulate(dev, (int)N, (int)H, m.tbl_dev + (4 + 2 * (size_t)dr) * N, m.tbl_dev + (5 + 2 * (size_t)dr) * N, m.len_dev);
+    gpu::parallel_memcpy(dev, (int)N, (int)H, m.tbl_dev + (4 + 2 * (size_t)dr) * N, m.tbl_dev + (5 + 2 * (size_t)dr) * N, m.len_dev);
     if (m.time_movers) CU(cudaEventRecord(m.ev[5 + 2 * dr], st));
   }
   Tensor gEmb(Dim({E}, V), m.g[P_EMB]);
@@ -331,7 +340,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
     Tensor gb(Dim({4 * H}), m.g[P_BF + 3 * dr]);
     const dyb200_tensor cWx = to_c(tWx), cWh = to_c(tWh);
     dyb200_tensor cgb = to_c(gb);
-    if (rec) throw_status(dev, dyb200i_rec_dx(dev.ctx, d.wg, m.p[P_WXF + 3 * dr], E, H, N, nullptr, 0, 0, d.dx));
+    if (rec) throw_status(dev, dyb200i_rec_dx(dev.ctx, d.wg, m.p[P_WXF + 3 * dr], E, H, N, nullptr, 0, 0, d.dx, 1));
     for (uint32_t k = rec ? 0 : Lmax; k-- > 0;) {
       const uint32_t B = Bk[k];
       const dyb200_tensor cx = to_c(col(d.x, E, prefix[k], B));
