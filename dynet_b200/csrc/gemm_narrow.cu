@@ -14,7 +14,7 @@ namespace {
 constexpr int kThreadsN = 256;
 constexpr uint32_t kNarrow = 64;                 // what counts as narrow
 constexpr uint32_t kSmallMax = 16 * 1024;        // floats of op(A) kept in shared memory
-constexpr size_t kSmemNarrow = 200 * 1024;       // above what any shape takes: 64 KB of op(A) and three pieces of up to 35 KB; 96 KB
+constexpr size_t kSmemNarrow = 224 * 1024;       // (the most a launch takes)
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(void* dst, const float* src, uint32_t bytes) {   // bytes < 16: the rest is zero
@@ -164,6 +164,169 @@ __global__ void __launch_bounds__(kThreadsN) k_gemm_narrow(const Narrow a) {
   cp_wait<0>();
 }
 
+// ---- few rows, a reduction of more than 64 ----
+struct Slices {
+  const float *A, *B; uint32_t lda, ldb; int transA;
+  uint32_t M, N, K;   // (at most 64 rows: one row block)
+  uint32_t KS, CS;    // KS CS = 8: slices of a piece's reduction and stretches of columns that the warps share out
+  uint32_t KC, pieces, TN, pitch;   // k per piece of B and pieces of the reduction; columns per tile; floats per column of a piece (an odd number of float4: eight columns, eight bank groups)
+  int vec_b, vec_c;   // 16-byte loads of B / accesses of C
+  float* C; uint32_t ldc; const float* bias; int mode;
+};
+
+// Lane: 8 rows x NJ columns, ML lanes along the rows, so that a warp has 8 ML rows x 32 / ML NJ columns: per four k a lane reads 8 + NJ float4 for 32 NJ multiply-adds,
+// with NJ = 8 half as many reads per multiply-add as 8 x 4 per thread.  What bounds it then is two warps per scheduler (58 % of the issue slots, 42 % of the
+// multiply-adds' rate at 32 x 107 000 x 256).  B comes in pieces of 64 k (of 16 each piece took a barrier per 2000 cycles), one on its way while the other is used.
+// The eight warps share out columns and, where there are fewer tiles than SMs, slices of a piece's reduction, whose sums meet, in their order, in the buffer just read:
+// without slices a few hundred columns were 15 us of one CTA's latencies.
+// us, k_gemm_narrow / here, by columns:  520  2300  13 400  107 000
+//   32 rows, K = 256   15.2 / 5.9  15.3 / 9.4  28.0 / 18.6  99 / 67      K = 128   8.7 / 5.7  8.8 / 5.7  15.3 / 12.8  52 / 37
+//   64 rows, K = 256   16.4 / 7.3  18.7 / 10.7  31.1 / 26.2  142 / 109   K = 128   9.3 / 6.1  9.3 / 7.4  17.3 / 16.5  76 / 59
+// Up to 64 k k_gemm_narrow is the faster one (32 rows, K = 32, 13 400 columns 5.5 / 8.8): there B's pieces are few and its tiles store while others load.
+template <int ML, int NJ>
+__global__ void __launch_bounds__(kThreadsN) k_gemm_slices(const Slices a) {
+  dyb_grid_dep_sync();
+  constexpr uint32_t NL = 32 / ML, WN = NL * NJ, MB = 8 * ML;   // NL: lanes along the columns; WN: columns of a warp
+  extern __shared__ __align__(16) float nsm[];
+  float* As = nsm;                                   // [K][MB]
+  float* ring = nsm + (size_t)a.K * MB;              // [2][TN][pitch]
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mg = lane % ML, nl = lane / ML;
+  const uint32_t ks = warp % a.KS, cs = warp / a.KS, buffer = a.TN * a.pitch, tiles = (a.N + a.TN - 1) / a.TN;
+  const uint32_t my_tiles = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0, items = my_tiles * a.pieces;
+  // this thread's part of a piece: the same k of every f_step-th column
+  const uint32_t f_q = a.vec_b ? a.KC / 4 : a.KC, f_step = kThreadsN / f_q, f_k = (tid % f_q) * (a.vec_b ? 4 : 1), f_n = tid / f_q;
+  auto fetch = [&](uint32_t item) {
+    if (item < items && f_n < f_step) {
+      const uint32_t n0 = (blockIdx.x + item / a.pieces * gridDim.x) * a.TN, k = item % a.pieces * a.KC + f_k, cols = min(a.TN, a.N - n0);
+      if (k < a.K) {
+        float* d = ring + (item & 1) * buffer + f_n * a.pitch + f_k;
+        const float* src = a.B + (size_t)a.ldb * (n0 + f_n) + k;
+        const uint32_t bytes = 4 * min(4u, a.K - k);
+        for (uint32_t n = f_n; n < cols; n += f_step, d += f_step * a.pitch, src += (size_t)a.ldb * f_step) {
+          if (a.vec_b) cp_async16(d, src, bytes); else cp_async4(d, src, 4);
+        }
+      }
+    }
+    cp_commit();
+  };
+  fetch(0);
+  for (uint32_t m = lane; m < MB; m += 32) {
+    const size_t step = a.transA ? 1 : a.lda;
+    const float* src = a.A + (m < a.M ? a.transA ? (size_t)a.lda * m : m : 0);
+#pragma unroll 8
+    for (uint32_t k = warp; k < a.K; k += kThreadsN / 32) As[(size_t)k * MB + m] = m < a.M ? src[k * step] : 0.f;
+  }
+  const uint32_t per = a.KC / a.KS, k_of = ks * per;                                          // this warp's slice of a piece
+  // the thread's part of a tile's results, where they go by shared memory
+  const uint32_t o_q = a.vec_c ? a.M / 4 : a.M, o_step = kThreadsN / o_q, o_m = (tid % o_q) * (a.vec_c ? 4 : 1), o_n = tid / o_q;
+  float acc[8][NJ];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) acc[i][j] = 0.f;
+  uint32_t piece = 0, tile = blockIdx.x;
+  for (uint32_t item = 0; item < items; ++item) {
+    float* const st = ring + (item & 1) * buffer;
+    fetch(item + 1);
+    cp_wait<1>();
+    __syncthreads();            // this piece (the first time: A too) is here
+    const uint32_t n0 = tile * a.TN, k0 = piece * a.KC, kn = min(per, k0 + k_of < a.K ? a.K - k0 - k_of : 0);   // k of this warp's slice
+    const float *bs = st + (size_t)(cs * WN + nl) * a.pitch + k_of, *as = As + (size_t)(k0 + k_of) * MB + 4 * mg;
+    float4 b[NJ];
+    if (kn >= 4) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) b[j] = ld4(bs + NL * j * a.pitch);
+    }
+    uint32_t k = 0;
+#pragma unroll 2
+    for (; k + 4 <= kn; k += 4, as += 4 * MB) {
+      float4 next[NJ];
+      const uint32_t kx = k + 8 <= kn ? k + 4 : k;   // (asked for a step ahead)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) next[j] = ld4(bs + NL * j * a.pitch + kx);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        float w[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 v = ld4(as + (size_t)kk * MB + 4 * ML * h);
+          w[4 * h] = v.x; w[4 * h + 1] = v.y; w[4 * h + 2] = v.z; w[4 * h + 3] = v.w;
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const float x = kk == 0 ? b[j].x : kk == 1 ? b[j].y : kk == 2 ? b[j].z : b[j].w;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(w[i], x, acc[i][j]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) b[j] = next[j];
+    }
+    for (; k < kn; ++k, as += MB)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 v = ld4(as + 4 * ML * h);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const float x = bs[NL * j * a.pitch + k];
+          acc[4 * h][j] = fmaf(v.x, x, acc[4 * h][j]);
+          acc[4 * h + 1][j] = fmaf(v.y, x, acc[4 * h + 1][j]);
+          acc[4 * h + 2][j] = fmaf(v.z, x, acc[4 * h + 2][j]);
+          acc[4 * h + 3][j] = fmaf(v.w, x, acc[4 * h + 3][j]);
+        }
+      }
+    __syncthreads();            // everybody is done with the buffer
+    if (++piece < a.pieces) continue;
+    piece = 0;
+    tile += gridDim.x;
+    if (a.KS == 1 && a.vec_c) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t n = n0 + cs * WN + nl + NL * j, m = 4 * mg + 4 * ML * h;
+          float4 v = make_float4(acc[4 * h][j], acc[4 * h + 1][j], acc[4 * h + 2][j], acc[4 * h + 3][j]);
+          acc[4 * h][j] = acc[4 * h + 1][j] = acc[4 * h + 2][j] = acc[4 * h + 3][j] = 0.f;
+          if (n >= a.N || m >= a.M) continue;
+          float* c = a.C + m + (size_t)a.ldc * n;
+          if (a.mode == EPI_BIAS) { const float4 o = ld4(a.bias + m); v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+          if (a.mode == EPI_ACCUM) { const float4 o = ld4(c); v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+          st4(c, v);
+        }
+      continue;
+    }
+    // the slices' sums side by side: [slice][column][row]
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        st4(st + ((size_t)ks * a.TN + cs * WN + nl + NL * j) * MB + 4 * mg + 4 * ML * h, make_float4(acc[4 * h][j], acc[4 * h + 1][j], acc[4 * h + 2][j], acc[4 * h + 3][j]));
+        acc[4 * h][j] = acc[4 * h + 1][j] = acc[4 * h + 2][j] = acc[4 * h + 3][j] = 0.f;
+      }
+    __syncthreads();
+    const uint32_t slice = a.TN * MB, cols = min(a.TN, a.N - n0);
+    if (o_n < o_step)
+      for (uint32_t n = o_n; n < cols; n += o_step) {
+        float* c = a.C + o_m + (size_t)a.ldc * (n0 + n);
+        const float* v = st + (size_t)n * MB + o_m;
+        if (a.vec_c) {
+          float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (a.mode == EPI_BIAS) o = ld4(a.bias + o_m);
+          if (a.mode == EPI_ACCUM) o = ld4(c);
+          float4 r = ld4(v);
+          for (uint32_t x = 1; x < a.KS; ++x) { const float4 w = ld4(v + x * slice); r.x += w.x; r.y += w.y; r.z += w.z; r.w += w.w; }
+          st4(c, make_float4(r.x + o.x, r.y + o.y, r.z + o.z, r.w + o.w));
+        } else {
+          float r = *v;
+          for (uint32_t x = 1; x < a.KS; ++x) r += v[x * slice];
+          *c = r + (a.mode == EPI_BIAS ? a.bias[o_m] : a.mode == EPI_ACCUM ? *c : 0.f);
+        }
+      }
+    __syncthreads();            // the buffer is free again
+  }
+  cp_wait<0>();
+}
+
 // ---- long reductions -------------------------------------------------------------------------------------------------------
 struct NarrowK {
   const float *A, *B; uint32_t lda, ldb;
@@ -279,6 +442,8 @@ __global__ void __launch_bounds__(256) k_narrow_reduce(const float* __restrict__
   *c = accumulate ? *c + s : s;
 }
 
+uint32_t up(uint32_t v, uint32_t step) { return (v + step - 1) / step * step; }
+
 template <int ML, int NJ>
 int launch_narrow(dyb200_ctx* ctx, Narrow a) {
   const uint32_t TN = kThreadsN / ML * NJ, tiles = (a.N + TN - 1) / TN, blocks = (a.M + 8 * ML - 1) / (8 * ML);
@@ -295,7 +460,32 @@ int launch_narrow(dyb200_ctx* ctx, Narrow a) {
   return DYB200_OK;
 }
 
-uint32_t up(uint32_t v, uint32_t step) { return (v + step - 1) / step * step; }
+// -1: the tile does not fit shared memory
+template <int ML, int NJ>
+int launch_slices(dyb200_ctx* ctx, Slices a) {
+  constexpr uint32_t MB = 8 * ML, WN = 32 / ML * NJ;
+  const uint32_t sms = (uint32_t)ctx->sm_count;
+  // slices by what the fullest SM has to do: whole rounds of tiles, 6 % more for each doubling (the sums' way through shared memory)
+  double best = 0;
+  size_t smem = 0;
+  for (uint32_t KS = 1; KS <= 8 && (KS == 1 || 16 * KS <= up(a.K, 8)); KS *= 2) {
+    const uint32_t TN = 8 / KS * WN, tiles = (a.N + TN - 1) / TN;
+    // k per piece; floats per column of the slices' sums (rows stored one by one go by the buffer as well)
+    const uint32_t most = KS == 8 ? 128 : 64, KC = a.K <= most ? up(a.K, 4 * KS) : most, need = KS > 1 || !a.vec_c ? KS * MB : 0;
+    const uint32_t pitch = (((KC > need ? KC : need) + 3) / 4 | 1) * 4;
+    const size_t bytes = sizeof(float) * ((size_t)a.K * MB + 2 * (size_t)TN * pitch);
+    const double t = (double)((tiles + sms - 1) / sms) * TN * (KS == 1 ? 1.0 : KS == 2 ? 1.06 : KS == 4 ? 1.12 : 1.18);
+    if (bytes > kSmemNarrow || (best != 0 && t >= best)) continue;
+    best = t; smem = bytes;
+    a.KS = KS; a.CS = 8 / KS; a.TN = TN; a.KC = KC; a.pitch = pitch; a.pieces = (a.K + KC - 1) / KC;
+  }
+  if (best == 0) return -1;
+  DYB_CUDA(ctx, dyb_smem_limit(k_gemm_slices<ML, NJ>, smem, kSmemNarrow));
+  const uint32_t tiles = (a.N + a.TN - 1) / a.TN, cap = (smem <= 72 * 1024 ? 3 : smem <= 110 * 1024 ? 2 : 1) * sms;
+  dyb_launch(k_gemm_slices<ML, NJ>, tiles < cap ? tiles : cap, kThreadsN, smem, ctx, a);
+  DYB_LAUNCHED(ctx);
+  return DYB200_OK;
+}
 
 // Row block: 32 rows, or 64 where that leaves less padding or reads the pieces less often.
 uint32_t row_block(uint32_t M) { return M <= 32 || (M > kNarrow && up(M, 32) < up(M, 64)) ? 32 : 64; }
@@ -320,6 +510,20 @@ int dyb200_gemm_narrow(dyb200_ctx* ctx, uint32_t M, uint32_t N, const GemmPair& 
   GemmProfScope scope(ctx, 2.0 * M * N * p.K, 0, M, N, p.K, (uint32_t)epi.mode);
   if (!p.transB) {
     const uint32_t mb = row_block(M);
+    if (p.K > 64) {   // (M <= 64)
+      Slices a{p.A, p.B, p.lda, p.ldb, p.transA, M, N, p.K, 0, 0, 0, 0, 0, 0, 0, 0, epi.C, epi.ldc, epi.bias, epi.mode};
+      a.vec_b = p.ldb % 4 == 0 && aligned16(p.B);
+      a.vec_c = epi.ldc % 4 == 0 && M % 4 == 0 && aligned16(epi.C) && (epi.mode != EPI_BIAS || aligned16(epi.bias));
+      // eight columns per lane, fewer where those tiles would leave SMs without one or do not fit
+      const uint32_t sms = (uint32_t)ctx->sm_count;
+      int rc = -1;
+      for (uint32_t nj = 8; nj >= 1 && rc == -1; nj /= 2) {
+        if (nj > 1 && (uint64_t)N < (uint64_t)sms * nj * (mb == 32 ? 8 : 4)) continue;
+        if (mb == 32) rc = nj == 8 ? launch_slices<4, 8>(ctx, a) : nj == 4 ? launch_slices<4, 4>(ctx, a) : nj == 2 ? launch_slices<4, 2>(ctx, a) : launch_slices<4, 1>(ctx, a);
+        else rc = nj == 8 ? launch_slices<8, 8>(ctx, a) : nj == 4 ? launch_slices<8, 4>(ctx, a) : nj == 2 ? launch_slices<8, 2>(ctx, a) : launch_slices<8, 1>(ctx, a);
+      }
+      return rc == -1 ? dyb200_fail(ctx, DYB200_ERUNTIME, "narrow product: %u x %u x %u does not fit shared memory", M, N, p.K) : rc;
+    }
     Narrow a{p.A, p.B, p.lda, p.ldb, p.transA, M, N, p.K, 0, 0, 0, 0, 0, epi.C, epi.ldc, epi.bias, epi.mode};
     // one piece holds the whole reduction when there are several row blocks (then it is at most 64 long)
     const bool several = M > mb;
