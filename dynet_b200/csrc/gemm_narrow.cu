@@ -335,7 +335,8 @@ struct NarrowK {
   uint32_t groups, KC;      // groups of threads that share a piece's k; k per piece (a multiple of `groups`)
   uint32_t kspan;           // k per CTA
   int vec_a, vec_b;
-  float* part;              // [grid.x][M N]
+  int meet;                 // the groups' sums meet in shared memory (else: a partial product per group)
+  float* part;              // [grid.x][groups, or 1][M N]
 };
 constexpr uint32_t kTilesMax = kThreadsN / 2;   // 8 x 8 outputs per thread and at least two groups: 8192 outputs per CTA
 
@@ -357,7 +358,11 @@ __global__ void __launch_bounds__(kThreadsN) k_gemm_narrow_k(const NarrowK a) {
       const uint32_t q = width / 4, step = kThreadsN / q;
       if (tid >= q * step) return;
       const uint32_t r = 4 * (tid % q), left = r < have ? min(4u, have - r) * 4 : 0;
-      for (uint32_t k = tid / q; k < a.KC; k += step) cp_async16(dst + k * row + r, src + (left && k < kn ? (size_t)ld * (k0 + k) + r : 0), k < kn ? left : 0);
+      uint32_t k = tid / q;
+      float* d = dst + k * row + r;
+      const float* from = src + (left ? (size_t)ld * (k0 + k) + r : 0);
+      for (; k < kn; k += step, d += step * row, from += left ? (size_t)ld * step : 0) cp_async16(d, from, left);
+      for (; k < a.KC; k += step, d += step * row) cp_async16(d, src, 0);
     } else {
       for (uint32_t r = tid & 31; r < width; r += 32)
         for (uint32_t k = tid >> 5; k < a.KC; k += kThreadsN / 32) {
@@ -387,11 +392,11 @@ __global__ void __launch_bounds__(kThreadsN) k_gemm_narrow_k(const NarrowK a) {
     __syncthreads();
     fetch(p + 2);
     if (!on) continue;
-    const float* st = nsm + (size_t)(p % kStagesN) * stage;
-#pragma unroll 2
-    for (uint32_t k = grp; k < a.KC; k += a.groups) {   // (k beyond the end are zeros)
-      const float4 x = ld4(st + k * row + 4 * mi), y = ld4(st + k * row + 4 * (mi + mt));
-      const float4 b = ld4(st + k * row + a.MT + 4 * ni), d = ld4(st + k * row + a.MT + 4 * (ni + nt));
+    const float* st = nsm + (size_t)(p % kStagesN) * stage + grp * row + 4 * mi;
+    const uint32_t to_y = 4 * mt, to_b = a.MT + 4 * ni - 4 * mi, to_d = to_b + 4 * nt;
+#pragma unroll 4
+    for (uint32_t k = grp; k < a.KC; k += a.groups, st += a.groups * row) {   // (k beyond the end are zeros)
+      const float4 x = ld4(st), y = ld4(st + to_y), b = ld4(st + to_b), d = ld4(st + to_d);
       const float w[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w}, c[8] = {b.x, b.y, b.z, b.w, d.x, d.y, d.z, d.w};
 #pragma unroll
       for (int i = 0; i < 8; ++i)
@@ -400,8 +405,33 @@ __global__ void __launch_bounds__(kThreadsN) k_gemm_narrow_k(const NarrowK a) {
     }
   }
   cp_wait<0>();
-  // the groups' sums, then out: each output's group sums are added in group order
   const uint32_t outs = a.MT * a.NT;
+  float* const out = a.part + (size_t)blockIdx.x * (a.meet ? 1 : a.groups) * a.M * a.N + m0 + (size_t)a.M * n0;
+  if (!a.meet) {
+    // every group's sums go out as they are: the launch that adds up the CTAs adds the groups too, in order
+    if (!on) return;
+    float* o = out + (size_t)grp * a.M * a.N;
+    const bool quads = a.M % 4 == 0;   // (the partial products start on 16 bytes)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t n = 4 * (ni + j / 4 * nt) + j % 4;
+      if (n >= nn) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t m = 4 * (mi + h * mt);
+        float* c = o + m + (size_t)a.M * n;
+        if (quads) {
+          if (m < mn) st4(c, make_float4(acc[4 * h][j], acc[4 * h + 1][j], acc[4 * h + 2][j], acc[4 * h + 3][j]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (m + i < mn) c[i] = acc[4 * h + i][j];
+        }
+      }
+    }
+    return;
+  }
+  // the groups' sums, then out: each output's group sums are added in group order
   __syncthreads();
   if (on) {
 #pragma unroll
@@ -411,13 +441,12 @@ __global__ void __launch_bounds__(kThreadsN) k_gemm_narrow_k(const NarrowK a) {
         st4(nsm + (size_t)grp * outs + (size_t)(4 * (ni + j / 4 * nt) + j % 4) * a.MT + 4 * (mi + h * mt), make_float4(acc[4 * h][j], acc[4 * h + 1][j], acc[4 * h + 2][j], acc[4 * h + 3][j]));
   }
   __syncthreads();
-  float* out = a.part + (size_t)blockIdx.x * a.M * a.N;
   for (uint32_t e = tid; e < outs; e += kThreadsN) {
     const uint32_t m = e % a.MT, n = e / a.MT;
     if (m >= mn || n >= nn) continue;
     float s = nsm[e];
     for (uint32_t g = 1; g < a.groups; ++g) s += nsm[(size_t)g * outs + e];
-    out[(m0 + m) + (size_t)a.M * (n0 + n)] = s;
+    out[m + (size_t)a.M * n] = s;
   }
 }
 
@@ -552,7 +581,11 @@ int dyb200_gemm_narrow(dyb200_ctx* ctx, uint32_t M, uint32_t N, const GemmPair& 
   }
   const uint32_t by = M <= kNarrow ? (N + a.NT - 1) / a.NT : (M + a.MT - 1) / a.MT;
   a.groups = kThreadsN / (a.MT / 8 * (a.NT / 8));
-  a.KC = up(4096 / (a.MT + a.NT), a.groups);   // 16 KB a piece
+  // Two groups or one write their sums as they are: where the outputs are many, meeting in shared memory and a thread adding the groups of 32 outputs one after the
+  // other took longer than twice the partial products do (us: 32 x 256 x 520 11.3 / 5.7, x 13 400 27.2 / 20.6, x 107 000 80 / 66, the last with pieces of 32 KB and
+  // addresses that walk; with 10 groups of 48 x 32 meeting is the faster one, 7.8 / 14.6 at 520).
+  a.meet = a.groups > 2;
+  a.KC = a.meet ? up(4096 / (a.MT + a.NT), a.groups) : up(8192 / (a.MT + a.NT), 4 * a.groups);   // 16 or 32 KB a piece
   a.vec_a = p.lda % 4 == 0 && aligned16(p.A);
   a.vec_b = p.ldb % 4 == 0 && aligned16(p.B);
   uint32_t gx = 2 * (uint32_t)ctx->sm_count / by;
@@ -560,15 +593,15 @@ int dyb200_gemm_narrow(dyb200_ctx* ctx, uint32_t M, uint32_t N, const GemmPair& 
   a.kspan = up((p.K + gx - 1) / gx, a.KC);
   gx = (p.K + a.kspan - 1) / a.kspan;
   void* part;
-  int rc = dyb200_scratch(ctx, (size_t)gx * M * N * sizeof(float), &part);
+  int rc = dyb200_scratch(ctx, (size_t)gx * (a.meet ? 1 : a.groups) * M * N * sizeof(float), &part);
   if (rc) return rc;
   a.part = (float*)part;
-  const size_t ring = (size_t)kStagesN * a.KC * (a.MT + a.NT), sums = (size_t)a.groups * a.MT * a.NT;
+  const size_t ring = (size_t)kStagesN * a.KC * (a.MT + a.NT), sums = a.meet ? (size_t)a.groups * a.MT * a.NT : 0;
   const size_t smem = sizeof(float) * (ring > sums ? ring : sums);
   DYB_CUDA(ctx, dyb_smem_limit(k_gemm_narrow_k, smem, kSmemNarrow));
   dyb_launch(k_gemm_narrow_k, dim3(gx, by), kThreadsN, smem, ctx, a);
   DYB_LAUNCHED(ctx);
-  dyb_launch(k_narrow_reduce, (M * N + 31) / 32, 256, 0, ctx, (const float*)a.part, gx, M, N, epi.C, epi.ldc, epi.mode == EPI_ACCUM ? 1 : 0);
+  dyb_launch(k_narrow_reduce, (M * N + 31) / 32, 256, 0, ctx, (const float*)a.part, gx * (a.meet ? 1 : a.groups), M, N, epi.C, epi.ldc, epi.mode == EPI_ACCUM ? 1 : 0);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;
 }
