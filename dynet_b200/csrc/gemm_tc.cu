@@ -13,7 +13,7 @@
 //   warps 2-9  add every finished chunk (tcgen05.ld of their 32 accumulator lanes x 64 columns) into fp32
 //              registers, park the finished tile in the idle operand ring and run the epilogue as a short
 //              cooperative loop over it: 16-byte accesses along the rows (whole 512-byte tile columns per warp),
-//              read-modify-write epilogues with 8 loads in flight; the LSTM epilogue reads the four gates of a
+//              what it adds to fetched while the last MMAs run; the LSTM epilogue reads the four gates of a
 //              hidden unit from the tile and also forms c and h
 // Products with few output tiles are split along K over blockIdx.z; the splits store raw partial
 // tiles and a second kernel adds them in split order and applies the epilogue (deterministic).
@@ -47,6 +47,85 @@ __device__ __forceinline__ void unscale_tile(const TmapPack& tm, float (&sum)[64
   for (int j = 0; j < 64; ++j) sum[j] = unscale(sum[j], ea + __shfl_sync(0xffffffffu, j < 32 ? f0 : f1, j & 31));
 }
 
+// The epilogue is what a short product spends its time on, and cold code is what an epilogue spends it on: a CTA runs it once, and
+// unrolled or with the modes told apart inside, its instructions took longer to fetch than its data.  So: one short loop per mode,
+// and what a tile adds to is copied into an idle stage of the operand ring while the last MMAs run, each thread's pieces by itself.
+// us for a launch in a running program, before / after (fetched at the end, by the pass that knows every mode, and by K splits with their
+// ranks' words read one after another): 1024 x 320 x 128 stored 8.2 / 6.0, 2000 x 256 x 320 added to 14.8 / 9.7, 1024 x 384 x 320 13.4 / 9.6,
+// 5003 x 300 x 1050 (pieces of 4 bytes) 31 / 25, 1024 x 384 x 1600 in six splits 15.0 / 13.2, 300 x 1050 x 1200 in four 15.5 / 12.5.
+template <int BYTES>
+__device__ __forceinline__ void copy_piece(float* dst, const float* src) {
+  if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// columns [c, c_hi) of the tile, STEP apart: what is there already, to the same place in `old` (stored like the tile)
+template <int BYTES, int STEP>
+__device__ __forceinline__ void fetch_old(float* old, const float* src, size_t ldc, uint32_t c, uint32_t c_hi) {
+  src += ldc * c;
+#pragma unroll 4
+  for (; c < c_hi; c += STEP, src += STEP * ldc) copy_piece<BYTES>(old + (size_t)c * BM, src);
+}
+__device__ __forceinline__ float piece_add(float a, float b) { return a + b; }
+__device__ __forceinline__ float4 piece_add(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+// (rounded as in every kernel with this epilogue)
+__device__ __forceinline__ float piece_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float4 piece_fma(float4 a, float4 b, float4 c) {
+  return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z), __fmaf_rn(a.w, b.w, c.w));
+}
+// The plain epilogues on columns [c, c_hi) of a tile in shared memory, STEP apart, a piece V (4 rows or one) per thread and column;
+// dst, mask and bias are those of the thread's first row, in column 0 of the tile.
+template <class V, int STEP>
+__device__ __forceinline__ void write_pieces(int mode, const float* tile, const float* old, float* dst, size_t ldc, const float* mask,
+                                             size_t mstep, const float* bias, uint32_t c, uint32_t c_hi) {
+  auto at = [](const float* p) { return *reinterpret_cast<const V*>(p); };
+  dst += ldc * c;
+  tile += (size_t)c * BM; old += (size_t)c * BM;
+  if (mode == EPI_STORE) {
+#pragma unroll 4
+    for (; c < c_hi; c += STEP, dst += STEP * ldc, tile += STEP * BM) *reinterpret_cast<V*>(dst) = at(tile);
+  } else if (mode == EPI_BIAS) {
+    const V b = at(bias);
+#pragma unroll 4
+    for (; c < c_hi; c += STEP, dst += STEP * ldc, tile += STEP * BM) *reinterpret_cast<V*>(dst) = piece_add(at(tile), b);
+  } else if (mode == EPI_ACCUM) {
+#pragma unroll 4
+    for (; c < c_hi; c += STEP, dst += STEP * ldc, tile += STEP * BM, old += STEP * BM) *reinterpret_cast<V*>(dst) = piece_add(at(tile), at(old));
+  } else {
+    mask += mstep * c;
+#pragma unroll 4
+    for (; c < c_hi; c += STEP, dst += STEP * ldc, tile += STEP * BM, old += STEP * BM, mask += STEP * mstep)
+      *reinterpret_cast<V*>(dst) = piece_fma(at(tile), at(mask), at(old));
+  }
+}
+// K splits as a cluster: the sums over the S partial tiles of the 16-byte pieces of columns [c, c_hi), 8 apart, in split order, put into
+// this CTA's own tile; BATCH columns x RANKS tiles requested at a time.
+template <int RANKS, int BATCH>
+__device__ __forceinline__ void slice_sums(float* tile, uint32_t S, uint32_t rq, uint32_t c, uint32_t c_hi) {
+  const uint32_t here = smem_u32(tile) + 16 * rq;
+  uint32_t base[RANKS];
+#pragma unroll
+  for (int r = 0; r < RANKS; ++r) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[r]) : "r"(here), "r"(min((uint32_t)r, S - 1)));
+#pragma unroll 1
+  for (; c < c_hi; c += 8 * BATCH) {
+    float4 p[BATCH][RANKS];
+#pragma unroll
+    for (int k = 0; k < BATCH; ++k)
+#pragma unroll
+      for (int r = 0; r < RANKS; ++r)
+        if ((uint32_t)r < S && c + 8 * k < c_hi)
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p[k][r].x), "=f"(p[k][r].y), "=f"(p[k][r].z), "=f"(p[k][r].w)
+                       : "r"(base[r] + 4u * BM * (c + 8u * k)) : "memory");
+#pragma unroll
+    for (int k = 0; k < BATCH; ++k) {
+      float4 a = p[k][0];
+#pragma unroll
+      for (int r = 1; r < RANKS; ++r)
+        if ((uint32_t)r < S) a = piece_add(a, p[k][r]);
+      if (c + 8 * k < c_hi) st4(tile + (size_t)(c + 8 * k) * BM + 4 * rq, a);
+    }
+  }
+}
+
 // BNT = columns of the output tile: 128, or 64 for products with N <= 64 (small per-GPU batches), where a 128-wide tile
 // would spend half of every MMA and half of the B traffic on padding.
 // CLUSTER: the gridDim.z K-splits of a tile form one thread-block cluster (1 x 1 x S); every CTA parks its partial tile in
@@ -66,7 +145,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
     if (!*(const volatile uint32_t*)tm.sa) return;   // (the same in every CTA)
   }
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2], old_free;
   __shared__ uint32_t tmem_base_slot;
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -83,11 +162,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
   constexpr int EL = F16 ? 64 : 32;
   const uint32_t nchunks = (total + kChunk - 1) / kChunk;
   if (!CLUSTER && gridDim.z > 1) epi.C += (size_t)blockIdx.z * epi.ldc * N;   // raw partial tile of this split (mode is EPI_STORE)
+  // What the tile adds to goes into the stage after the last k-block's (not the first one, where the tile will be), once k-block
+  // it_old - STAGES has been read from it.
+  const uint32_t it_old = total + (total % STAGES == 0 ? 1 : 0);
   __shared__ uint32_t split_ok;   // CLUSTER: this CTA's partial tile is complete
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int q = 0; q < 2; ++q) { mbar_init(&acc_full[q], 1); mbar_init(&acc_empty[q], kEpiWarps); }
+    mbar_init(&old_free, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -166,6 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
         if (F16) issue_kblock_f16(acc, acc + BNT, a_hi, a_lo, b_hi, idesc_wide, idesc, in_chunk, a_step, b_step);
         else issue_kblock(acc, a_hi, a_lo, b_hi, b_lo, idesc, in_chunk, a_step, b_step);
         umma_commit(&empty_bar[s]);   // frees the stage once these MMAs have read it
+        if (it + STAGES == it_old) umma_commit(&old_free);
         const bool chunk_ends = in_chunk == kChunk - 1 || it == total - 1;
         if (chunk_ends) { umma_commit(&acc_full[buf]); in_chunk = 0; ++chunk; buf ^= 1; }
         else ++in_chunk;
@@ -193,6 +277,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
         cprev[k] = n < N ? ld4(epi.c_prev + u + (size_t)epi.H * n) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
+    uint32_t ne0 = n0, Ne = N;
+    if (TWO) epi_side(epi, ne0, Ne);
+    // the columns this CTA finishes (K splits as a cluster: its slice), and the pieces of them this thread does in the plain epilogues:
+    // 4 rows of every eighth column where rows and destinations allow it, a row of every second one otherwise
+    const uint32_t S = CLUSTER ? gridDim.z : 1, w = CLUSTER ? ((BNT + S - 1) / S + 7) & ~7u : BNT;
+    const uint32_t c_lo = CLUSTER ? min(blockIdx.z * w, (uint32_t)BNT) : 0, c_hi = CLUSTER ? min(c_lo + w, (uint32_t)BNT) : BNT;
+    const bool adds = epi.mode == EPI_ACCUM || epi.mode == EPI_ACCUM_MASK;
+    const bool plain = adds || epi.mode == EPI_STORE || epi.mode == EPI_BIAS, vec = plain && epi_in_pieces(epi, M);
+    const uint32_t my_r = vec ? 4 * (te & 31) : te & 127, my_c = c_lo + (vec ? te >> 5 : te >> 7);
+    const uint32_t my_hi = m0 + my_r < M && ne0 < Ne ? min(c_hi, Ne - ne0) : 0;
+    const EpiRow row = epi_row(epi, min(m0 + my_r, M - 1));
+    float* const dst = row.c + (size_t)row.ldc * ne0;
+    float* const old = reinterpret_cast<float*>(ring + (size_t)(it_old % STAGES) * STAGE_BYTES) + my_r;
     float sum[64];   // this thread's row of the tile, columns [64 half, 64 half + 64)
 #pragma unroll
     for (int j = 0; j < 64; ++j) sum[j] = 0.f;
@@ -200,6 +297,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
 #pragma unroll 1
     for (uint32_t c = 0; c < nchunks; ++c) {
       const uint32_t buf = c & 1;
+      if (adds && c == nchunks - 1) {   // (the chunks before are drained: the MMAs that free the stage wait for nothing here)
+        if (it_old >= STAGES && !mbar_wait(&old_free, 0)) { ok = false; break; }
+        if (vec) fetch_old<16, 8>(old, dst, row.ldc, my_c, my_hi);
+        else fetch_old<4, 2>(old, dst, row.ldc, my_c, my_hi);
+      }
       if (!mbar_wait(&acc_full[buf], (c >> 1) & 1)) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (64 * half < BNT) {   // (with a 64-column tile the second column half does not exist)
@@ -238,54 +340,48 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
 #pragma unroll
       for (int j = 0; j < 64; ++j) col[(size_t)j * BM] = sum[j];
     }
-    uint32_t ne0 = n0, Ne = N;
-    if (TWO) epi_side(epi, ne0, Ne);
+    if (adds) asm volatile("cp.async.wait_all;" ::: "memory");   // (each thread reads what it has fetched itself)
     uint32_t all_ok;
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, 1, 256, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(all_ok) : "r"((uint32_t)ok) : "memory");
+    auto finish = [&]() {
+      const float* mask = epi.mode == EPI_ACCUM_MASK ? row.mask + (row.mask_full ? (size_t)row.mask_ld * ne0 : 0) : nullptr;
+      const size_t mstep = row.mask_full ? row.mask_ld : 0;
+      const float* bias = epi.bias + min(m0 + my_r, M - 1);
+      if (vec) write_pieces<float4, 8>(epi.mode, tile + my_r, old, dst, row.ldc, mask, mstep, bias, my_c, my_hi);
+      else if (plain) write_pieces<float, 2>(epi.mode, tile + my_r, old, dst, row.ldc, mask, mstep, bias, my_c, my_hi);
+      else epilogue_pass<BNT, 256>(epi, tile, te, blockIdx.x, m0, ne0, M, Ne, cprev, c_lo, c_hi);
+    };
     if (!CLUSTER) {
-      if (all_ok) epilogue_pass<BNT, 256>(epi, tile, te, blockIdx.x, m0, ne0, M, Ne, cprev);
+      if (all_ok) finish();
     } else {
       // every thread of every CTA of the cluster takes part in the two cluster barriers below (the TMA and MMA warps
       // reach them further down); between them rank 0 reads the other CTAs' tiles
       if (te == 0) split_ok = all_ok;
       asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-      {
-        // Rank r (= blockIdx.z: the cluster is 1 x 1 x gridDim.z) finishes columns [c_lo, c_hi) of the tile: it adds the
-        // S partial tiles of that slice in split order (the order of the split-K reduction kernel), its own from its
-        // shared memory and the others through distributed shared memory, and runs the epilogue on the slice.
-        const uint32_t S = gridDim.z, rank = blockIdx.z;
-        const uint32_t w = ((BNT + S - 1) / S + 7) & ~7u;
-        const uint32_t c_lo = min(rank * w, (uint32_t)BNT), c_hi = min(c_lo + w, (uint32_t)BNT);
-        uint32_t ok_all = all_ok, base[8];
-        for (uint32_t r = 0; r < S; ++r) {
-          uint32_t ra, v;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(&split_ok)), "r"(r));
-          asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(ra) : "memory");
-          ok_all &= v;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[r & 7]) : "r"(smem_u32(tile)), "r"(r));
-        }
-        if (ok_all) {
-          const uint32_t f_lo = c_lo * (BM / 4), f_hi = c_hi * (BM / 4);   // 16-byte pieces of the slice
-          float4* t4 = reinterpret_cast<float4*>(tile);
-          for (uint32_t f = f_lo + te; f < f_hi; f += 256) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (uint32_t r = 0; r < S; ++r) {
-              float4 pv;
-              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                           : "=f"(pv.x), "=f"(pv.y), "=f"(pv.z), "=f"(pv.w) : "r"(base[r & 7] + 16u * f) : "memory");
-              if (r == 0) acc = pv;
-              else { acc.x += pv.x; acc.y += pv.y; acc.z += pv.z; acc.w += pv.w; }
-            }
-            t4[f] = acc;
-          }
-          asm volatile("barrier.cta.sync 1, 256;" ::: "memory");   // the pass below reads other threads' pieces
-          epilogue_pass<BNT, 256>(epi, tile, te, blockIdx.x, m0, ne0, M, Ne, cprev, c_lo, c_hi);
-        } else if (te == 0 && rank == 0) {
-          atomicOr(flags, DYB200_FLAG_WAIT_TIMEOUT);
-        }
+      // Rank r (= blockIdx.z: the cluster is 1 x 1 x gridDim.z) finishes columns [c_lo, c_hi) of the tile: it adds the
+      // S partial tiles of that slice in split order (the order of the split-K reduction kernel), its own from its
+      // shared memory and the others through distributed shared memory, and runs the epilogue on the slice.
+      uint32_t ra, v;   // (one rank's word per lane)
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(&split_ok)), "r"(min((uint32_t)lane, S - 1)));
+      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(ra) : "memory");
+      {   // (whatever the words say: the sums go no further than this tile yet)
+        const uint32_t rq = te & 31, c = c_lo + (te >> 5);
+        if (S <= 2) slice_sums<2, 4>(tile, S, rq, c, c_hi);
+        else if (S <= 4) slice_sums<4, 2>(tile, S, rq, c, c_hi);
+        else slice_sums<8, 2>(tile, S, rq, c, c_hi);
       }
-      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // every tile stays until all ranks have read it
+      const bool ok_all = __all_sync(0xffffffffu, v != 0);
+      if (!ok_all && te == 0 && blockIdx.z == 0) atomicOr(flags, DYB200_FLAG_WAIT_TIMEOUT);
+      __syncwarp();
+      // every tile stays until all ranks have read it
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      if (ok_all) {
+        if (!vec) asm volatile("barrier.cta.sync 1, 256;" ::: "memory");   // the pass below reads other threads' pieces
+        finish();
+      }
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

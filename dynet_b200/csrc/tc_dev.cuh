@@ -222,6 +222,16 @@ __device__ __forceinline__ void issue_kblock_f16(uint32_t acc, uint32_t acc2, ui
       : "memory");
 }
 
+// Whether the rows, destinations, biases and masks of an epilogue can be handled as 16-byte pieces of four rows.
+__device__ __forceinline__ bool epi_in_pieces(const GemmEpilogue& epi, uint32_t M) {
+  return (M & 3) == 0 && (epi.split_m & 3) == 0 && (epi.ldc & 3) == 0 && aligned16(epi.C) &&
+         (epi.split_m == 0 || ((epi.ldc2 & 3) == 0 && aligned16(epi.C2))) &&
+         (epi.mode != EPI_BIAS || aligned16(epi.bias)) && (epi.mode != EPI_GATES || (aligned16(epi.bias) && (epi.H & 3) == 0)) &&
+         (epi.mode != EPI_ACCUM_MASK ||
+          (aligned16(epi.maskC) && (!epi.maskc_full || (epi.maskc_ld & 3) == 0) &&
+           (epi.split_m == 0 || (aligned16(epi.maskC2) && (!epi.maskc2_full || (epi.maskc2_ld & 3) == 0)))));
+}
+
 // The cooperative pass over NC finished columns parked in shared memory (column-major, BM rows per column): called by
 // NT epilogue threads (te = 0..NT-1).  mt is the tile's row-block index (m0 = BM mt), n0 the global column of the first
 // parked column, cprev the previous cell states the caller fetched for EPI_LSTM_CELL (hidden units
@@ -263,12 +273,7 @@ __device__ __forceinline__ void epilogue_pass(const GemmEpilogue& epi, const flo
       }
     }
   } else {
-    const bool vec = (M & 3) == 0 && (epi.split_m & 3) == 0 && (epi.ldc & 3) == 0 && aligned16(epi.C) &&
-                     (epi.split_m == 0 || ((epi.ldc2 & 3) == 0 && aligned16(epi.C2))) &&
-                     (epi.mode != EPI_BIAS || aligned16(epi.bias)) && (epi.mode != EPI_GATES || (aligned16(epi.bias) && (epi.H & 3) == 0)) &&
-                     (epi.mode != EPI_ACCUM_MASK ||
-                      (aligned16(epi.maskC) && (!epi.maskc_full || (epi.maskc_ld & 3) == 0) &&
-                       (epi.split_m == 0 || (aligned16(epi.maskC2) && (!epi.maskc2_full || (epi.maskc2_ld & 3) == 0)))));
+    const bool vec = epi_in_pieces(epi, M);
     if (vec) {
       // 32 row quads x NC columns; a thread keeps its row quad and walks the columns te / 32 + (NT / 32) k
       const uint32_t rq = te & 31, m = m0 + 4 * rq;

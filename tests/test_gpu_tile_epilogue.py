@@ -1,0 +1,26 @@
+"""Tensor-pipe products of one tile per CTA: what a tile adds to waits in a stage of the operand ring that the last k-blocks leave
+idle.  Reductions of every remainder of the three stages and of the eight k-blocks of an accumulation chunk, rows and destinations in
+16-byte pieces and not, stored and added to (dynet/nodes-affinetransform.cc:77-157: y = b + A x, dA += dy x^T)."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("add", [0, 1])
+@pytest.mark.parametrize("M,N,ldc", [(260, 130, 260), (259, 200, 261), (384, 64, 388), (130, 100, 130)])
+@pytest.mark.parametrize("K", [70, 96, 129, 160, 200, 256, 288, 300, 352, 520, 1050, 2080])
+def test_epilogue_of_a_tile(K, M, N, ldc, add):
+    import torch
+    import gpu_util as g
+    ctx = g.ctx()
+    torch.manual_seed(K + M)
+    a, b, c = torch.randn(K, M, device="cuda"), torch.randn(N, K, device="cuda"), torch.randn(N, ldc, device="cuda")
+    want = c.double().clone()
+    want[:, :M] = b.double() @ a.double() + (want[:, :M] if add else 0)
+    ctx.gemm(0, 0, M, N, K, a.data_ptr(), M, b.data_ptr(), K, c.data_ptr(), ldc, add)
+    assert ctx.device_errors() == 0
+    # a product of the split operands is off by less than 2^-20 of the sum of magnitudes (the dropped lo * lo term 2^-22, the rounding
+    # of lo 2^-22, and fp32 sums over chunks of at most 8 k-blocks); an addition by half an ulp of its result
+    bound = 2.0 ** -20 * (b.double().abs() @ a.double().abs()) + 2.0 ** -23 * want[:, :M].abs()
+    assert ((c.double()[:, :M] - want[:, :M]).abs() <= bound).all()
+    assert torch.equal(c.double()[:, M:], want[:, M:])   # the rows past M stay
