@@ -147,7 +147,7 @@ static inline unsigned stream_grid(const dyb200_ctx* ctx, size_t work_items, uns
 // dyb_grid_dep_sync() overlap the predecessor's tail; nothing after that call runs before the predecessor has completed
 // and its writes are visible.  With it off the launch is an ordinary stream-ordered one and the device call is a no-op.
 template <class... KArgs, class... Args>
-inline void dyb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, dyb200_ctx* ctx, Args&&... args) {
+inline void dyb_launch_as(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, dyb200_ctx* ctx, Args&&... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = ctx->stream;
@@ -155,10 +155,15 @@ inline void dyb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // (not for kernels that take most of an SM's shared memory: scheduled early, they would keep other streams' work off the SMs
-  // they wait on, and their own prologue is nothing beside their run time)
-  cfg.numAttrs = ctx->pdl && smem <= 96 * 1024 ? 1 : 0;
+  cfg.numAttrs = ctx->pdl && dependent ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);   // a failure is picked up by DYB_LAUNCHED (cudaGetLastError)
+}
+template <class... KArgs, class... Args>
+inline void dyb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, dyb200_ctx* ctx, Args&&... args) {
+  // (not for kernels that take most of an SM's shared memory: scheduled early, they would keep other streams' work off the SMs
+  // they wait on, and their own prologue is nothing beside their run time.  The one-tile products of gemm_tc.cu ask for it all the same:
+  // they take 6 to 25 us, 0.7 of them before the wait)
+  dyb_launch_as(smem <= 96 * 1024, kernel, grid, block, smem, ctx, static_cast<Args&&>(args)...);
 }
 // dyb_grid_dep_sync also lets the next kernel of the stream start now; after dyb_grid_dep_wait alone it starts when this one's CTAs end.
 // The branch behind the wait is never taken (no launch has that much shared memory).  It is what keeps the kernel's loads behind the

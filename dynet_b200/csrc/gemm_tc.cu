@@ -1611,6 +1611,10 @@ int dyb200_tc_param2(dyb200_ctx* ctx, const float* src, uint32_t rows, const flo
   return rc;
 }
 
+// One-tile products start under the kernel before them (see dyb_launch): 0.7 us of barriers, TMEM and descriptors, and the launch itself.  One
+// layer of 256 units on 32 sequences, forward and backward: 227.5 -> 222.6 us; steps of models on several streams are the same within the
+// noise; the persistent kernel so launched gained nothing and is not.  (A CTA that waits holds TMEM: no kernel that allocates any
+// fits beside its shared memory, so none before it in the stream can be waiting for what it holds.)
 // The kernels by tile width and form.  Their limit on dynamic shared memory is raised when one is first asked for (function attributes are per
 // device, so the context remembers what it has set on its own; a limit loads its kernel, and a program needs a few of them).
 using TcKernel = void (*)(TmapPack, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, GemmEpilogue, uint32_t*);
@@ -1720,11 +1724,13 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ctx->pdl ? 2 : 1;
     // (a smaller cluster size that fits was tried when the model's count does not - batch 64, 16 tiles: 7 instead of 8 -
     // and measured slower than the workspace form of the model's count: 4.73 vs 4.60 ms per step)
     const uint32_t Sc = (S <= 8 && cluster_fits(ctx, bn, S, grid.x * grid.y)) ? S : 0;
@@ -1825,7 +1831,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
     GemmProfScope scope(ctx, flops, f16 ? 2 : 1, M, N, kb_total * el, (uint32_t)epi.mode);
     TcKernel kern;
     if ((rc = tc_kernel(ctx, bn, false, f16 ? TC_F16 : TC_TF32, &kern))) return rc;
-    dyb_launch(kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb0, kb1, kb_per_split, kepi, ctx->dev_flags);
+    dyb_launch_as(true, kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb0, kb1, kb_per_split, kepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);
     if (S > 1 && epi.mode == EPI_LSTM_CELL) {
       dyb_launch(k_splitk_reduce_cell, stream_grid(ctx, (size_t)M / 16 * N + 1, 256), 256, 0, ctx, part, S, M, N, epi);
@@ -1918,15 +1924,17 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
     if ((rc = tc_kernel(ctx, bn, Sc > 1, TC_TWO, &kern))) return rc;
     GemmProfScope scope(ctx, only_if ? 0.0 : flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);   // (under a condition: the products on pairs have been counted)
     if (Sc == 1) {
-      dyb_launch(kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
+      dyb_launch_as(true, kern, grid, kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u, kb, epi, ctx->dev_flags);
     } else {
       cudaLaunchConfig_t cfg;
       memset(&cfg, 0, sizeof(cfg));
       cfg.gridDim = dim3(grid.x, grid.y, Sc); cfg.blockDim = dim3(kThreads, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = ctx->stream;
-      cudaLaunchAttribute attr[1];
+      cudaLaunchAttribute attr[2];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = Sc;
-      cfg.attrs = attr; cfg.numAttrs = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr; cfg.numAttrs = ctx->pdl ? 2 : 1;
       cudaLaunchKernelEx(&cfg, kern, tm, M, N, kb, 0u, (kb + Sc - 1) / Sc, epi, ctx->dev_flags);
     }
     DYB_LAUNCHED(ctx);
@@ -1938,7 +1946,7 @@ int dyb200_tc_gemm_packed2(dyb200_ctx* ctx, uint32_t M, const PackedOp& A, const
   if (through_memory) {
     if ((rc = tc_kernel(ctx, bn, false, TC_TWO, &kern))) return rc;
     GemmProfScope scope(ctx, flops, 1, M, N0 + N1, kb * 32, (uint32_t)EPI_ACCUM);
-    dyb_launch(kern, dim3(grid.x, grid.y, Sp), kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u,
+    dyb_launch_as(true, kern, dim3(grid.x, grid.y, Sp), kThreads, SMEM_BYTES, ctx, tm, M, N, kb, 0u,
                (kb + Sp - 1) / Sp, pepi, ctx->dev_flags);
     DYB_LAUNCHED(ctx);
   } else {
