@@ -1302,10 +1302,11 @@ int gates_f16_pack(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I
   return dyb200_f16_pack(ctx, &jobs);
 }
 
-// Returns the cached packed form of a parameter matrix, packing it first if it is new or stale.
+// Returns the cached packed form of a parameter matrix, packing it first if it is new or stale (3xTF32 planes: as jobs of `queue` if there is
+// one, which the caller then launches whatever happens: the entry counts as packed).
 // (k_is_fast = kLayoutF16 + F16_LINE or F16_ELEM: fp16 planes of the matrix as it lies, its scale words behind the hi plane)
 int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_fast, uint32_t rows, uint32_t K, uint32_t pitch,
-                      float** hi, float** lo, const float* src2 = nullptr, uint32_t rows2 = 0) {
+                      float** hi, float** lo, const float* src2 = nullptr, uint32_t rows2 = 0, PackJobs* queue = nullptr) {
   const int cap = (int)(sizeof(ctx->param_pack) / sizeof(ctx->param_pack[0]));
   dyb200_ctx::ParamPack* hit = nullptr;
   dyb200_ctx::ParamPack* victim = &ctx->param_pack[0];
@@ -1350,11 +1351,12 @@ int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_f
     if (rc) return rc;
     e->version = ctx->param_version;
   } else if (e->version != ctx->param_version) {
-    PackJobs batch;
-    dyb200_tc_pack_begin(&batch);
-    int rc = pack(ctx, src, ld, k_is_fast, rows, K, nullptr, 0, 0, e->hi, e->lo, pitch, &batch);
-    if (!rc && rows2) rc = pack(ctx, src2, ld, k_is_fast, rows2, K, nullptr, 0, 0, e->hi + (size_t)rows * pitch, e->lo + (size_t)rows * pitch, pitch, &batch);
-    if (!rc) rc = pack_flush_impl(ctx, &batch);
+    PackJobs own;
+    dyb200_tc_pack_begin(&own);
+    PackJobs* const batch = queue ? queue : &own;
+    int rc = pack(ctx, src, ld, k_is_fast, rows, K, nullptr, 0, 0, e->hi, e->lo, pitch, batch);
+    if (!rc && rows2) rc = pack(ctx, src2, ld, k_is_fast, rows2, K, nullptr, 0, 0, e->hi + (size_t)rows * pitch, e->lo + (size_t)rows * pitch, pitch, batch);
+    if (!rc && !queue) rc = pack_flush_impl(ctx, &own);
     if (rc) return rc;
     e->version = ctx->param_version;
   }
@@ -1501,10 +1503,10 @@ int dyb200_tc_planes(dyb200_ctx* ctx, uint32_t rows, uint32_t K, PackedOp* out) 
   return DYB200_OK;
 }
 
-int dyb200_tc_param(dyb200_ctx* ctx, const float* src, uint32_t ld, bool k_is_fast, uint32_t rows, uint32_t K, PackedOp* out) {
-  if (!ctx->param_cache_on) return dyb200_tc_pack(ctx, src, ld, k_is_fast, rows, K, nullptr, 0, 0, out, nullptr);
+int dyb200_tc_param(dyb200_ctx* ctx, const float* src, uint32_t ld, bool k_is_fast, uint32_t rows, uint32_t K, PackedOp* out, PackJobs* batch) {
+  if (!ctx->param_cache_on) return dyb200_tc_pack(ctx, src, ld, k_is_fast, rows, K, nullptr, 0, 0, out, batch);
   out->rows = rows; out->K = K; out->pitch = round_up(K, 32);
-  return cached_param_pack(ctx, src, ld, k_is_fast ? 1 : 0, rows, K, out->pitch, &out->hi, &out->lo);
+  return cached_param_pack(ctx, src, ld, k_is_fast ? 1 : 0, rows, K, out->pitch, &out->hi, &out->lo, nullptr, 0, batch);
 }
 
 int dyb200_tc_param_gates(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t rows, uint32_t K, PackedOp* out) {
@@ -2001,24 +2003,25 @@ int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const Ge
     A[0] = dyb200_f16_op(ja, a_mn); B[0] = dyb200_f16_op(jb, b_mn);
     return dyb200_tc_gemm_packed(ctx, M, N, 1, A, B, epi);
   }
-  PackJobs batch;   // all operands that need packing go out in one launch
+  PackJobs batch;   // all operands that need packing go out in one launch, also when a later one fails (a parameter's planes count as packed)
   dyb200_tc_pack_begin(&batch);
-  for (int p = 0; p < npairs; ++p) {
+  int rcp = DYB200_OK;
+  for (int p = 0; p < npairs && !rcp; ++p) {
     const GemmPair& g = pairs[p];
     // A: rows = m. op(A)(m,k) = transA ? A[k + lda*m] : A[m + lda*k]  -> k is fast iff transA.  An operand whose rows are
     // the fast index is split as it lies (K rows of M values) and read MN-major (single products only): no transposing
     // pass, and a parameter then has ONE set of planes for this product and for the one that uses it transposed.
     const bool a_mn = npairs == 1 && g.transA == 0, b_mn = npairs == 1 && g.transB != 0;
-    int rc;
+    int& rc = rcp;
     if (a_mn) {
-      rc = g.a_is_param ? dyb200_tc_param(ctx, g.A, g.lda, true, g.K, M, &A[p])
+      rc = g.a_is_param ? dyb200_tc_param(ctx, g.A, g.lda, true, g.K, M, &A[p], &batch)
                         : dyb200_tc_pack(ctx, g.A, g.lda, true, g.K, M, nullptr, 0, 0, &A[p], &batch);
       A[p].rows = M; A[p].K = g.K; A[p].mn_major = 1;
     } else {
-      rc = g.a_is_param ? dyb200_tc_param(ctx, g.A, g.lda, g.transA != 0, M, g.K, &A[p])
+      rc = g.a_is_param ? dyb200_tc_param(ctx, g.A, g.lda, g.transA != 0, M, g.K, &A[p], &batch)
                         : dyb200_tc_pack(ctx, g.A, g.lda, g.transA != 0, M, g.K, nullptr, 0, 0, &A[p], &batch);
     }
-    if (rc) return rc;
+    if (rc) break;
     // B: rows = n. op(B)(k,n) = transB ? B[n + ldb*k] : B[k + ldb*n]  -> k is fast iff !transB
     if (b_mn) {
       rc = dyb200_tc_pack(ctx, g.B, g.ldb, true, g.K, N, g.maskB, g.mask_ld, g.mask_full, &B[p], &batch);
@@ -2026,10 +2029,9 @@ int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const Ge
     } else {
       rc = dyb200_tc_pack(ctx, g.B, g.ldb, g.transB == 0, N, g.K, g.maskB, g.mask_ld, g.mask_full, &B[p], &batch);
     }
-    if (rc) return rc;
   }
-  int rcf = dyb200_tc_pack_flush(ctx, &batch);
-  if (rcf) return rcf;
+  const int rcf = dyb200_tc_pack_flush(ctx, &batch);
+  if (rcp || rcf) return rcp ? rcp : rcf;
   return dyb200_tc_gemm_packed(ctx, M, N, npairs, A, B, epi);
 }
 
