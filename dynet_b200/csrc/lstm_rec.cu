@@ -39,8 +39,10 @@ namespace {
 
 __device__ __forceinline__ float xor_add(float keep, float send, int m) { return keep + __shfl_xor_sync(0xffffffffu, send, m); }
 
-// columns of cluster g that are active at a step of width B: those i with g + G i < B
-__device__ __forceinline__ uint32_t active_cols(uint32_t B, uint32_t g, uint32_t G) { return B > g ? (B - g + G - 1) / G : 0; }
+// columns of a cluster that are active at a step of width B: those i < cap with first + step i < B
+__device__ __forceinline__ uint32_t active_cols(uint32_t B, uint32_t first, uint32_t step, uint32_t cap) {
+  return B > first ? min((B - first + step - 1) / step, cap) : 0;
+}
 
 // grid (C, G, directions), cluster (C, 1, 1); block = 8 U threads.
 // Dynamic shared memory: h[2][ncap][16 KD], c[ncap][U].  NB columns per block, NF of them computed (3 of 4, or all).
@@ -51,7 +53,7 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
   __shared__ __align__(8) uint64_t got[2];
   __shared__ __align__(16) float stage_all[8][NB * 4];
   const RecDirF d = blockIdx.z ? a.d[1] : a.d[0];
-  const uint32_t H = a.H, U = a.U, G = a.G, g = blockIdx.y, rank = blockIdx.x, C = gridDim.x, ncap = a.ncap;
+  const uint32_t H = a.H, U = a.U, g = blockIdx.y, g0 = g * a.first, gi = a.step, gc = a.cap, rank = blockIdx.x, C = gridDim.x, ncap = a.ncap;
   const uint32_t tid = threadIdx.x, s = tid & 15, ul0 = 2 * (tid >> 4);   // slice, first of the lane's two units
   const uint32_t ul = ul0 + (s >> 3), u = rank * U + ul;                  // the unit this lane finishes
   const bool live_u = u < H;
@@ -69,16 +71,16 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
   // the column of a block that this lane finishes; 8 / NB lanes share one (they hold equal values; dup == 0 stores)
   const uint32_t lc = NB == 8 ? (s & 7) : NB == 4 ? (s & 7) >> 1 : NB == 2 ? (s & 7) >> 2 : 0;
   const uint32_t dup = NB == 8 ? 0 : NB == 4 ? (s & 1) : NB == 2 ? (s & 3) : (s & 7);
-  const uint32_t ncol = active_cols(a.N, g, G);
+  const uint32_t ncol = active_cols(a.N, g0, gi, gc);
   uint32_t phase[2] = {0, 0};
   bool ok = true;
   uint32_t col0 = 0, B = a.prefix ? a.prefix[1] : a.N;      // first column and width of the step
-  uint32_t n = active_cols(B, g, G);
+  uint32_t n = active_cols(B, g0, gi, gc);
   float pre[4], mk, pre_next[4], mk_next;
   // Wx x + b and the mask of this lane's column of a block, asked for a block or step ahead.  (Behind a block's stores they came in after the h they are
   // added to: 200 - 480 of a step's 3 800 cycles at 256 units and 3 columns.)
   auto fetch = [&](uint32_t c0, uint32_t nact, uint32_t nb) {
-    const uint32_t i = nb + lc, sc = g + G * i;
+    const uint32_t i = nb + lc, sc = g0 + gi * i;
     if (live_u && i < nact) {
       const float* p = d.gates + u + (size_t)4 * H * (c0 + sc);
 #pragma unroll
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
   __syncthreads();
 #pragma unroll 2
   for (uint32_t e = tid; e < ncol * H; e += blockDim.x) {
-    const uint32_t i = e / H, k = e % H, sc = g + G * i;
+    const uint32_t i = e / H, k = e % H, sc = g0 + gi * i;
     const bool own = k / U == rank;
     float v = d.h0 ? __ldg(d.h0 + k + (size_t)H * sc) : 0.f;
     const float m = d.mask ? __ldg(d.mask + k + (a.mask_full ? (size_t)H * sc : 0)) : 1.f, c = own && d.c0 ? __ldg(d.c0 + k + (size_t)H * sc) : 0.f;
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
     const uint32_t hnext = smem_addr(hbuf + (size_t)pn * ncap * HP);
     const uint32_t col1 = col0 + B;                                          // the next step
     const uint32_t B1 = t + 1 < a.T ? (a.prefix ? a.prefix[t + 2] - a.prefix[t + 1] : a.N) : 0;
-    const uint32_t n1 = active_cols(B1, g, G);
+    const uint32_t n1 = active_cols(B1, g0, gi, gc);
     if (n1 && tid == 0) msg_expect(&got[pn], n1 * C * U * 4);   // (only the columns that go on are handed over)
     if (t > 0) {
       ok = ok && msg_wait(&got[pt], phase[pt]);
@@ -226,7 +228,7 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
         }
         z[q] = v[0];
       }
-      const uint32_t i = nb + lc, sc = g + G * i;
+      const uint32_t i = nb + lc, sc = g0 + gi * i;
       const bool mine = live_u && i < n;
       float cn = 0.f, hv = 0.f, hm = 0.f;
       if (mine) {
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(MT, 1) k_lstm_rec_bwd(const __grid_constant__ 
   __shared__ __align__(8) uint64_t got[2];
   __shared__ __align__(16) float stage_all[12][NB * 32];
   const RecDirB d = blockIdx.z ? a.d[1] : a.d[0];
-  const uint32_t H = a.H, U = a.U, G = a.G, g = blockIdx.y, rank = blockIdx.x, C = gridDim.x, ncap = a.ncap;
+  const uint32_t H = a.H, U = a.U, g = blockIdx.y, g0 = g * a.first, gi = a.step, gc = a.cap, rank = blockIdx.x, C = gridDim.x, ncap = a.ncap;
   const uint32_t tid = threadIdx.x, s = tid & 7, og = tid >> 3;
   float* part = rec_smem;                                   // [parity][source rank][column][unit]
   float* dg = part + (size_t)2 * C * ncap * U;
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(MT, 1) k_lstm_rec_bwd(const __grid_constant__ 
   cluster_wait();
   // the last step that has a column of this cluster: widths never grow, so the steps before it have one too
   uint32_t T = a.T;
-  while (a.prefix && T > 0 && active_cols(a.prefix[T] - a.prefix[T - 1], g, G) == 0) --T;
+  while (a.prefix && T > 0 && active_cols(a.prefix[T] - a.prefix[T - 1], g0, gi, gc) == 0) --T;
 
   // saved values of the first (column, unit) item of the cell pass of a step, requested one step ahead
   float gt[4], cv, cp, dhv, dcv;
@@ -349,8 +351,8 @@ __global__ void __launch_bounds__(MT, 1) k_lstm_rec_bwd(const __grid_constant__ 
   auto start_of = [&](uint32_t t) { return a.prefix ? a.prefix[t] : t * a.N; };
   uint32_t n_later = 0;            // columns that were active at step t + 1
   uint32_t col = T ? start_of(T - 1) : 0;
-  uint32_t n = T ? active_cols(start_of(T) - col, g, G) : 0;
-  if (T && c_live && c_i0 < n) fetch(T - 1, col, T > 1 ? start_of(T - 2) : 0, g + G * c_i0);
+  uint32_t n = T ? active_cols(start_of(T) - col, g0, gi, gc) : 0;
+  if (T && c_live && c_i0 < n) fetch(T - 1, col, T > 1 ? start_of(T - 2) : 0, g0 + gi * c_i0);
   for (uint32_t t = T; t-- > 0;) {
     const uint32_t colm1 = t ? start_of(t - 1) : 0, pin = (t + 1) & 1, pout = t & 1;
     const float* from = part + (size_t)pin * C * ncap * U;
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(MT, 1) k_lstm_rec_bwd(const __grid_constant__ 
     // ---- gradients of the gate pre-activations of this CTA's units ----
     if (c_live)
       for (uint32_t i = c_i0; i < n; i += c_step) {
-        const uint32_t sc = g + G * i;
+        const uint32_t sc = g0 + gi * i;
         if (i != c_i0) fetch(t, col, colm1, sc);
         float dh = dhv;
         if (i < n_later) {
@@ -392,8 +394,8 @@ __global__ void __launch_bounds__(MT, 1) k_lstm_rec_bwd(const __grid_constant__ 
       }
     if (t == 0) break;             // (no earlier state to hand dE/dh to)
     __syncthreads();
-    const uint32_t nm1 = active_cols(col - colm1, g, G);
-    if (c_live && c_i0 < nm1) fetch(t - 1, colm1, t > 1 ? start_of(t - 2) : 0, g + G * c_i0);
+    const uint32_t nm1 = active_cols(col - colm1, g0, gi, gc);
+    if (c_live && c_i0 < nm1) fetch(t - 1, colm1, t > 1 ? start_of(t - 2) : 0, g0 + gi * c_i0);
     // ---- partial sums of dE/dh_{t-1} over this CTA's gate rows ----
 #pragma unroll 1
     for (uint32_t nb = 0; nb < n; nb += NB) {
@@ -594,15 +596,28 @@ bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan*
 // clusters are two columns' time, and so they are over 8).  The others' SMs are left to other streams: three language models of 256
 // units and 16 columns on three streams 103.6 -> 85.9 us a step, of 300 units and 30 columns 475 -> 440; a layer by itself is as fast.  (Where the width shrinks from step to step
 // more clusters have fewer columns for longer.)
+constexpr uint32_t kBlockCols = 4;   // the most columns an instance of the kernels takes at a time
 static uint32_t clusters_needed(uint32_t N, uint32_t G, const uint32_t* prefix) {
   const uint32_t cols = (N + G - 1) / G;
-  return prefix ? G : (N + cols - 1) / cols;
+  return prefix && cols > kBlockCols ? G : (N + cols - 1) / cols;
+}
+// Which columns cluster g has: first * g + step * i, i < cap.  Neighbouring ones where they are one block of the kernel, which costs the same whatever is
+// left of it: the clusters of a ragged batch's short sequences then end early: taggers of 16 sentences of 5 to
+// 60 tokens on three streams 198 -> 188 us a step (one by itself: forward 100 -> 103 us, where the last steps of every cluster had a column left, backward
+// 97 both).  More than a block: every G-th column, so that all
+// clusters lose columns alike.
+template <class Args>
+static void deal(Args* a, uint32_t G) {
+  const uint32_t cols = (a->N + G - 1) / G;
+  const bool block = cols <= kBlockCols;
+  a->G = G; a->first = block ? cols : 1u; a->step = block ? 1u : G; a->cap = block ? cols : 0xffffffffu;
 }
 
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
   if (p.tcf) return dyb200_rec_tc_fwd(ctx, p.tf, a, ndir);
   const uint32_t G = clusters_needed(a->N, p.Gf, a->prefix);
-  a->U = p.U; a->G = G; a->ncap = p.ncapf; a->flags = ctx->dev_flags;
+  deal(a, G);
+  a->U = p.U; a->ncap = p.ncapf; a->flags = ctx->dev_flags;
   FwdKernel k = fwd_kernel(p.KD, (a->N + G - 1) / G);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
@@ -615,7 +630,8 @@ int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir) {
 
 int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db) {
   const uint32_t rows = 4 * a->H, G = p.tcb ? p.tb.G : clusters_needed(a->N, p.Gb, a->prefix);
-  a->U = p.U; a->G = G; a->ncap = p.ncapb; a->flags = ctx->dev_flags;
+  deal(a, G);
+  a->U = p.U; a->ncap = p.ncapb; a->flags = ctx->dev_flags;
   void* part;
   int rc = dyb200_scratch(ctx, (size_t)ndir * G * rows * sizeof(float), &part);
   if (rc) return rc;

@@ -16,7 +16,8 @@ struct RecDirF {
 struct RecFwd {
   RecDirF d[2];
   uint32_t H, U, T, N, G, ncap, hn_pitch;
-  uint32_t ndir;   // directions in the grid of lstm_rec_tc.cu, whose groups take neighbouring columns (lstm_rec.cu: every G-th)
+  uint32_t first, step, cap;   // (lstm_rec.cu) cluster g has the columns first * g + step * i, i < cap
+  uint32_t ndir;   // directions in the grid of lstm_rec_tc.cu, whose groups take neighbouring columns
   int mask_full;
   float fb;
   const uint32_t* prefix;   // device, T + 1 entries: step t has the columns [prefix[t], prefix[t + 1]), widths never grow (null: N each)
@@ -34,6 +35,7 @@ struct RecDirB {
 struct RecBwd {
   RecDirB d[2];
   uint32_t H, U, T, N, G, ncap, dn_pitch;
+  uint32_t first, step, cap;
   uint32_t ndir;
   int mask_full;
   const uint32_t* prefix;
@@ -47,7 +49,7 @@ struct RecTcPlan { uint32_t G; };
 struct RecPlan { uint32_t U, C, KD, KD2, Gf, Gb, ncapf, ncapb; bool tcf, tcb; RecTcPlan tf, tb; };
 // False when the width is outside what the registers of a cluster hold, or N columns are more than the clusters can carry.
 bool dyb200_rec_plan(dyb200_ctx* ctx, uint32_t H, uint32_t N, int ndir, RecPlan* out);
-// ndir directions (1 or 2) share T, N and prefix.  U, G, ncap and flags are filled in here.
+// ndir directions (1 or 2) share T, N and prefix.  U, G, ncap, the dealing of the columns and flags are filled in here.
 int dyb200_rec_fwd(dyb200_ctx* ctx, const RecPlan& p, RecFwd* a, int ndir);
 // db[dir] (4H) += row sums of dgates over all columns (partial sums in scratch memory).
 int dyb200_rec_bwd(dyb200_ctx* ctx, const RecPlan& p, RecBwd* a, int ndir, float* const* db);
