@@ -154,7 +154,6 @@ __device__ __forceinline__ void pair_issue(const TmapPack* tm, const PairArgs* a
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_constant__ TmapPack tm, const __grid_constant__ PairArgs a) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (a.unless) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (*(const volatile uint32_t*)a.unless) return;   // (the same in every CTA)

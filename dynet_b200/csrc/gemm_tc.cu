@@ -504,7 +504,7 @@ template <int BNT, bool F16 = false>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm_persist(const __grid_constant__ TmapPack tm, uint32_t M, uint32_t N,
                                                               uint32_t kb0, uint32_t kb1, uint32_t tiles_m, uint32_t tiles,
                                                               uint32_t gm, uint32_t S, GemmEpilogue epi, uint32_t* flags) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // (no early start of the next kernel: this one has every SM for its whole time)
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[kPersistBufs], acc_empty[kPersistBufs];
   __shared__ uint32_t tmem_base_slot;

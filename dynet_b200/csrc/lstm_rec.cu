@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256, 1) k_lstm_rec_fwd(const __grid_constant__
     msg_init(&got[1]);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  dyb_grid_dep_sync();
+  dyb_grid_dep_wait();   // (the next kernel starts when this one's CTAs end: early, its own would hold SMs for a whole sequence)
 
   // the column of a block that this lane finishes; 8 / NB lanes share one (they hold equal values; dup == 0 stores)
   const uint32_t lc = NB == 8 ? (s & 7) : NB == 4 ? (s & 7) >> 1 : NB == 2 ? (s & 7) >> 2 : 0;
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(MT, 1) k_lstm_rec_bwd(const __grid_constant__ 
     msg_init(&got[1]);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  dyb_grid_dep_sync();
+  dyb_grid_dep_wait();
 
   // weights: outputs o = 8 og + 0..7 (units of h_{t-1}) x this CTA's gate rows kk = q U + unit, slice s
   float w[8][KD];

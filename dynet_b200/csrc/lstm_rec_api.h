@@ -48,11 +48,11 @@ int dyb200i_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, co
 int dyb200i_dependent_launch(dyb200_ctx* ctx, int set);
 #ifdef __cplusplus
 }
-/* A driver's own launches are ordinary ones unless the caller has chosen otherwise; the context is left as it was found. */
+/* A driver's own launches are ordinary ones (or what it says) unless the caller has chosen otherwise; the context is left as it was found. */
 struct dyb200i_ordinary_launches {
   dyb200_ctx* ctx;
   int was;
-  explicit dyb200i_ordinary_launches(dyb200_ctx* c) : ctx(c), was(dyb200i_dependent_launch(c, 0)) {}
+  explicit dyb200i_ordinary_launches(dyb200_ctx* c, int dependent = 0) : ctx(c), was(dyb200i_dependent_launch(c, dependent)) {}
   ~dyb200i_ordinary_launches() { dyb200i_dependent_launch(ctx, was); }
   dyb200i_ordinary_launches(const dyb200i_ordinary_launches&) = delete;
 };

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols(kGroups * 3 * NC + 64 * KB)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  dyb_grid_dep_sync();
+  dyb_grid_dep_wait();
   tc_before();
   __syncthreads();
   tc_after();
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols(MT * (kGroups * 2 * NC + 128))) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  dyb_grid_dep_sync();
+  dyb_grid_dep_wait();
   tc_before();
   __syncthreads();
   tc_after();

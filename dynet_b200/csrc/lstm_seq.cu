@@ -57,7 +57,7 @@ __device__ __forceinline__ uint32_t h_word(const SeqFwd& a, uint32_t n) { return
 // step, launch by launch 53).
 template <int BNT, uint32_t S, bool F16, bool VEC = true>
 __global__ void __launch_bounds__(kThreads, 1) k_lstm_seq_fwd(const __grid_constant__ TmapPack tm, const SeqFwd a) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (a.T == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (behind a sequence the next kernel starts when this one ends)
   // 64-column tiles need 48 KiB per stage, so the ring holds four of them: at 0.4 us per k-block three stages do not cover
   // the latency of a tile fetch
   constexpr int kStages = BNT == 64 ? 4 : 3;

@@ -373,7 +373,16 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
 }
 
 int guarded(Tagger* m, const PassArgs& a) {
-  const dyb200i_ordinary_launches ordinary(m->dev.ctx);
+  // A pass is 50 launches one behind the other on two streams.  While their kernels take a few microseconds each, dependent launches save the gaps
+  // between them; longer ones keep CTAs that wait on SMs that the other direction, or another model, could use.  us, ordinary / dependent launches,
+  // one tagger of 256 units waited for, and a step of three on three streams: 520 tokens 500 / 446, 188 / 170; 1200 605 / 553, 235 / 229;
+  // 4000 794 / 749, 334 / 336; 8400 1004 / 968, 478 / 482; 13 400 1196 / 1135, 667 / 692.
+  constexpr uint64_t kDependentTokens = 6144;
+  uint64_t tokens = 0;
+  for (uint32_t s = 0; a.lens && s < a.S; ++s) tokens += a.lens[s];
+  const int dependent = tokens <= kDependentTokens;
+  const dyb200i_ordinary_launches first(m->dev.ctx, dependent);
+  const dyb200i_ordinary_launches second(m->dev2.ctx, dependent && dyb200i_dependent_launch(m->dev.ctx, -1));   // (the caller's choice holds for both)
   try {
     tagger_pass(*m, a);
     return DYB200_OK;
@@ -420,9 +429,7 @@ int dyb200h_tagger_create(const dyb200h_tagger_config* c, float* params, float* 
   if (!rc && cudaStreamCreateWithFlags(&m->stream2, cudaStreamNonBlocking) != cudaSuccess) rc = DYB200_ECUDA;
   if (!rc) rc = dyb200_ctx_create(device, m->stream2, &m->dev2.ctx);
   if (!rc) dyb200_ctx_param_cache(m->dev2.ctx, 1);
-  // (two streams: a kernel scheduled early would hold SMs that the other direction's kernels could use)
   const dyb200i_ordinary_launches ordinary(ctx);
-  if (!rc) dyb200_ctx_dependent_launch(m->dev2.ctx, 0);
   if (!rc && (cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming) != cudaSuccess)) rc = DYB200_ECUDA;
   for (int k = 0; k < 2 && !rc; ++k) rc = dyb200_wgrad_create(k ? m->dev2.ctx : ctx, 4 * c->H, c->E, c->H, max_tokens, &m->d[k].wg);
