@@ -1,6 +1,7 @@
 // Products with one narrow side and a long one, in fp32 on the CUDA cores: the per-token layers of a tagger (32 or 45 rows times
 // 100 000 tokens), their gradients by the tokens and by the weights.
-//   few rows or a short reduction, many columns:  C (M x N) = epilogue(op(A) B)      k_gemm_narrow
+//   a short reduction (up to 64), many columns:   C (M x N) = epilogue(op(A) B)      k_gemm_narrow
+//   few rows, more to reduce over, many columns:  the same                           k_gemm_slices
 //   both sides small, a long reduction:           C (M x N) (+)= A B^T               k_gemm_narrow_k
 // On the tensor path such a product is bound by everything but its arithmetic: the long operand is read, written as two split planes
 // and read again, three quarters of the rows of a 128-row tile are padding, and accumulating stores go by registers.  32 x 107 000 x 256

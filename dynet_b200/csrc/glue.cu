@@ -13,9 +13,10 @@ __global__ void __launch_bounds__(kBlock) k_fill(float* __restrict__ p, size_t n
   for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (size_t)gridDim.x * kBlock) p[i] = v;
 }
 
-// partial[blk] = sum over this CTA's grid-stride slice of x (SQUARE: of x^2)
+// partial[blk] = sum over this CTA's grid-stride slice of x (SQUARE: of x^2); a single CTA's goes to `out` itself
 template <bool SQUARE>
-__global__ void __launch_bounds__(kBlock) k_sum_partial(const float* __restrict__ x, size_t n, float* __restrict__ partial) {
+__global__ void __launch_bounds__(kBlock) k_sum_partial(const float* __restrict__ x, size_t n, float* __restrict__ partial, float* __restrict__ out,
+                                                       int accumulate) {
   dyb_grid_dep_sync();
   __shared__ float red[32];
   float acc = 0.f;
@@ -34,7 +35,9 @@ __global__ void __launch_bounds__(kBlock) k_sum_partial(const float* __restrict_
       acc += SQUARE ? x[i] * x[i] : x[i];
   }
   acc = block_sum(acc, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+  if (threadIdx.x) return;
+  if (gridDim.x > 1) partial[blockIdx.x] = acc;
+  else out[0] = accumulate ? out[0] + acc : acc;
 }
 __global__ void __launch_bounds__(kBlock) k_sum_final(const float* __restrict__ partial, int np, float* __restrict__ out,
                                                      int accumulate) {
@@ -80,13 +83,14 @@ int dyb200_fill(float* p, size_t n, float value, dyb200_ctx* ctx) {
 
 static int sum_impl(const float* x, size_t n, float* out, int square, int accumulate, dyb200_ctx* ctx) {
   DYB_CHECK_ARG(ctx, x != nullptr && out != nullptr, "sum: null pointer");
-  int np = ctx->sm_count * 4;
-  void* partial;
-  int rc = dyb200_scratch(ctx, np * sizeof(float), &partial);
+  // (the losses of a step, say, are one CTA's work of 2.2 us, at four 16-byte pieces a thread, and no second launch of 2)
+  const int np = n <= 16 * kBlock ? 1 : ctx->sm_count * 4;
+  void* partial = nullptr;
+  int rc = np > 1 ? dyb200_scratch(ctx, np * sizeof(float), &partial) : DYB200_OK;
   if (rc) return rc;
-  if (square) dyb_launch(k_sum_partial<true>, np, kBlock, 0, ctx, x, n, (float*)partial);
-  else dyb_launch(k_sum_partial<false>, np, kBlock, 0, ctx, x, n, (float*)partial);
+  dyb_launch(square ? k_sum_partial<true> : k_sum_partial<false>, np, kBlock, 0, ctx, x, n, (float*)partial, out, accumulate);
   DYB_LAUNCHED(ctx);
+  if (np == 1) return DYB200_OK;
   dyb_launch(k_sum_final, 1, kBlock, 0, ctx, (const float*)partial, np, out, accumulate);
   DYB_LAUNCHED(ctx);
   return DYB200_OK;

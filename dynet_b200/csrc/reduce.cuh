@@ -74,6 +74,34 @@ static __global__ void __launch_bounds__(128) k_batch_reduce_final_warp(const fl
   if (lane == 0) out[r] += acc;
 }
 
+// Both stages in one CTA per 32 outputs, for few terms: 32 warps add a stretch of b each, in ascending order, then a warp per output the 32 stretches
+// by a butterfly.  (5003 outputs of some 50 terms: 2.0 + 2.0 us in two launches, 3.1 in
+// one; a pass of a tagger of 520 tokens, three launches less, 447 -> 444.5.)
+constexpr uint32_t kReduceOneCols = 1024;
+constexpr size_t kReduceOneTerms = 1u << 18;
+template <class F>
+__global__ void __launch_bounds__(1024) k_batch_reduce_one(F f, size_t n, uint32_t B, float* __restrict__ out) {
+  dyb_grid_dep_sync();
+  __shared__ float part[32][33];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, per = (B + 31) / 32, b0 = min(w * per, B), b1 = min(b0 + per, B);
+  const size_t r = (size_t)blockIdx.x * 32 + lane, mine = (size_t)blockIdx.x * 32 + w;
+  float acc = 0.f;
+  if (r < n)
+#pragma unroll 1
+    for (uint32_t b = b0; b < b1; b += 8) {
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = f(r, min(b + q, b1 - 1));
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (b + q < b1) acc += v[q];
+    }
+  part[w][lane] = acc;
+  __syncthreads();
+  acc = warp_sum(part[lane][w]);
+  if (lane == 0 && mine < n) out[mine] += acc;
+}
+
 template <class F>
 static int batch_reduce_add(dyb200_ctx* ctx, F f, size_t n, uint32_t B, float* out) {
   if (n == 0 || B == 0) return DYB200_OK;
@@ -86,6 +114,11 @@ static int batch_reduce_add(dyb200_ctx* ctx, F f, size_t n, uint32_t B, float* o
   S = (B + chunk - 1) / chunk;
   if (S == 1) {
     dyb_launch(k_batch_reduce_partial<F>, dim3(gx, 1), 128, 0, ctx, f, n, B, chunk, nullptr, out, 1);
+    DYB_LAUNCHED(ctx);
+    return DYB200_OK;
+  }
+  if (B <= kReduceOneCols && n * B <= kReduceOneTerms) {
+    dyb_launch(k_batch_reduce_one<F>, (unsigned)((n + 31) / 32), 1024, 0, ctx, f, n, B, out);
     DYB_LAUNCHED(ctx);
     return DYB200_OK;
   }
