@@ -148,9 +148,8 @@ int dyb200_matmul_bwd(DYB200_BWD_ARGS) {
   if (rc) return rc;
   DYB_CHECK_ARG(ctx, dEdxi && dEdxi->v && t_batch_size(dEdxi) == t_batch_size(&xs[i]) && dEdxi->bd == xs[i].bd,
                 "MatrixMultiply: gradient shape differs from argument %u", i);
-  const bool overwrite = (attr_flags(attrs) & DYB200I_OVERWRITE) != 0;
-  if (i == 0) return mm_transp_r_acc(ctx, dEdf, &xs[1], dEdxi, overwrite);
-  return mm_transp_l_acc(ctx, &xs[0], dEdf, dEdxi, (attr_flags(attrs) & DYB200_GEMM_A_IS_PARAM) ? 1 : 0, overwrite);
+  if (i == 0) return mm_transp_r_acc(ctx, dEdf, &xs[1], dEdxi, false);
+  return mm_transp_l_acc(ctx, &xs[0], dEdf, dEdxi, (attr_flags(attrs) & DYB200_GEMM_A_IS_PARAM) ? 1 : 0, false);
 }
 
 int dyb200_affine_transform_fwd(DYB200_FWD_ARGS) {
@@ -191,14 +190,16 @@ int dyb200_affine_transform_fwd(DYB200_FWD_ARGS) {
   return DYB200_OK;
 }
 
-int dyb200_affine_transform_bwd(DYB200_BWD_ARGS) {
+int dyb200_affine_transform_bwd(DYB200_BWD_ARGS) { return dyb200i_affine_transform_bwd(xs, nxs, fx, dEdf, i, dEdxi, attrs, aux_mem, 0, ctx); }
+
+int dyb200i_affine_transform_bwd(const dyb200_tensor* xs, int nxs, const dyb200_tensor* fx, const dyb200_tensor* dEdf, unsigned i, dyb200_tensor* dEdxi,
+                                 const void* attrs, void* aux_mem, int overwrite, dyb200_ctx* ctx) {
   { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
   (void)aux_mem; (void)fx;
   DYB_CHECK_ARG(ctx, nxs >= 1 && (nxs - 1) % 2 == 0 && (int)i < nxs, "AffineTransform: failed boundary check in backward");
   DYB_CHECK_ARG(ctx, dEdf && dEdf->v && dEdxi && dEdxi->v, "AffineTransform: null tensor");
   DYB_CHECK_ARG(ctx, t_batch_size(dEdxi) == t_batch_size(&xs[i]) && dEdxi->bd == xs[i].bd,
                 "AffineTransform: gradient shape differs from argument %u", i);
-  const bool overwrite = (attr_flags(attrs) & DYB200I_OVERWRITE) != 0;
   if (i == 0) {
     const size_t dx_size = t_size(dEdxi), df_size = t_size(dEdf);
     if (overwrite) DYB_CUDA(ctx, cudaMemsetAsync(dEdxi->v, 0, dx_size * sizeof(float), ctx->stream));

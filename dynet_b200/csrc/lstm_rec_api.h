@@ -34,8 +34,12 @@ int dyb200i_rec_dx(dyb200_ctx* ctx, struct dyb200_wgrad* w, const float* Wx, uin
                    int mask_full, uint32_t period, float* dx, int overwrite);
 
 /* A driver whose gradient buffers hold nothing yet says so instead of clearing them: the clear is a pass of writes, and adding to zeros one of reads.
- * A bit of the flags of dyb200_affine_transform_bwd and dyb200_matmul_bwd (the gradient wanted) and of dyb200_softmax_output_bwd_fused (dh alone): */
-#define DYB200I_OVERWRITE 0x80000000u
+ * dyb200_affine_transform_bwd and dyb200_softmax_output_bwd_fused with `overwrite`: dEdxi, or dh alone, is written, whatever it holds. */
+int dyb200i_affine_transform_bwd(const dyb200_tensor* xs, int nxs, const dyb200_tensor* fx, const dyb200_tensor* dEdf, unsigned i, dyb200_tensor* dEdxi,
+                                 const void* attrs, void* aux_mem, int overwrite, dyb200_ctx* ctx);
+int dyb200i_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor* h, const dyb200_tensor* R, const dyb200_tensor* dEdf, const void* aux_mem,
+                                     dyb200_tensor* dR, dyb200_tensor* db, dyb200_tensor* dh, dyb200_tensor* dx_scratch, uint32_t flags, int overwrite,
+                                     dyb200_ctx* ctx);
 /* dyb200_vanilla_lstm_seq_bwd with `fresh` bits: dx_all is written, whatever it holds; dE/dc is zero from outside and not wanted (dc_all: scratch memory). */
 enum { DYB200I_FRESH_DX = 1, DYB200I_FRESH_DC = 2 };
 int dyb200i_lstm_seq_bwd(const dyb200_tensor* x_all, const dyb200_tensor* h0, const dyb200_tensor* c0, const dyb200_tensor* Wx, const dyb200_tensor* Wh,

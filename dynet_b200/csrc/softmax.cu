@@ -970,6 +970,12 @@ int dyb200_pickneglogsoftmax_bwd(DYB200_BWD_ARGS) {
 int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor* h, const dyb200_tensor* R,
                                     const dyb200_tensor* dEdf, const void* aux_mem, dyb200_tensor* dR, dyb200_tensor* db,
                                     dyb200_tensor* dh, dyb200_tensor* dx_scratch, uint32_t flags, dyb200_ctx* ctx) {
+  return dyb200i_softmax_output_bwd_fused(x, h, R, dEdf, aux_mem, dR, db, dh, dx_scratch, flags, 0, ctx);
+}
+
+int dyb200i_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor* h, const dyb200_tensor* R, const dyb200_tensor* dEdf, const void* aux_mem,
+                                     dyb200_tensor* dR, dyb200_tensor* db, dyb200_tensor* dh, dyb200_tensor* dx_scratch, uint32_t flags, int overwrite,
+                                     dyb200_ctx* ctx) {
   { int rc0__ = dyb200_scratch_begin(ctx); if (rc0__) return rc0__; }
   DYB_CHECK_ARG(ctx, x && h && R && dEdf && aux_mem && dR && db && dh && x->v && h->v && R->v && dEdf->v && dR->v && db->v && dh->v,
                 "softmax_output_bwd_fused: null argument");
@@ -991,10 +997,9 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
     dyb200_tensor dv = *x;   // the gradient of x, with x's shape
     dv.v = dx_scratch->v;
     dyb200_tensor xs[3] = {*db, *R, *h};
-    for (unsigned i = 0; i < 3 && !rc; ++i) {
-      dyb200_affine_attrs at = {i == 2 ? flags : flags & ~DYB200I_OVERWRITE};
-      rc = dyb200_affine_transform_bwd(xs, 3, x, &dv, i, i == 0 ? db : i == 1 ? dR : dh, &at, nullptr, ctx);
-    }
+    dyb200_affine_attrs at = {flags};
+    for (unsigned i = 0; i < 3 && !rc; ++i)
+      rc = dyb200i_affine_transform_bwd(xs, 3, x, &dv, i, i == 0 ? db : i == 1 ? dR : dh, &at, nullptr, i == 2 && overwrite, ctx);
     return rc;
   }
   int rc;
@@ -1048,7 +1053,7 @@ int dyb200_softmax_output_bwd_fused(const dyb200_tensor* x, const dyb200_tensor*
     if ((rc = dyb200_tc_gemm_packed(ctx, V, H, 1, &dA, &hT, e))) return rc;
   }
   // dh (+)= R^T d : M = H, N = n, K = V
-  GemmEpilogue e{flags & DYB200I_OVERWRITE ? EPI_STORE : EPI_ACCUM, dh->v, H, nullptr, 0, 0.f, nullptr, 0, 0};
+  GemmEpilogue e{overwrite ? EPI_STORE : EPI_ACCUM, dh->v, H, nullptr, 0, 0.f, nullptr, 0, 0};
   return dyb200_tc_gemm_packed(ctx, H, n, 1, &RT, &dB, e);
 }
 

@@ -279,8 +279,8 @@ void step_body(Lm& m, const float* const* masks, float* loss_dev, int phase = -1
     // dh += R^T dr) in one: dr is written straight into the operand layouts of the two products
     dyb200_tensor cr = to_c(rall), ch = to_c(hall), cR = to_c(tR), cones = to_c(tones), cdr = to_c(tdr);
     dyb200_tensor cgb = to_c(tgbias), cgR = to_c(tgR), cdh = to_c(tdhall);
-    throw_status(dev, dyb200_softmax_output_bwd_fused(&cr, &ch, &cR, &cones, m.aux, &cgR, &cgb, &cdh, &cdr,
-                                                     DYB200_GEMM_A_IS_PARAM | (layer_major ? DYB200I_OVERWRITE : 0u), dev.ctx));
+    throw_status(dev, dyb200i_softmax_output_bwd_fused(&cr, &ch, &cR, &cones, m.aux, &cgR, &cgb, &cdh, &cdr,
+                                                      DYB200_GEMM_A_IS_PARAM, layer_major, dev.ctx));
   }
   Tensor tones(Dim({1}, B), m.ones);
   const uint32_t pass0 = phase < 0 ? 0u : (phase == 0 ? L : (uint32_t)phase - 1), pass1 = phase < 0 ? (layer_major ? L : 1u) : (phase == 0 ? L : (uint32_t)phase);

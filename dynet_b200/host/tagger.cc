@@ -312,8 +312,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   auto input_grad = [&](const std::vector<const Tensor*>& xs, const Tensor& fx, const Tensor& dEdf, unsigned i, Tensor& dEdxi) {
     dyb200_tensor cxs[5], cfx = to_c(fx), cd = to_c(dEdf), cdx = to_c(dEdxi);
     for (size_t k = 0; k < xs.size(); ++k) cxs[k] = to_c(*xs[k]);
-    const dyb200_affine_attrs fresh = {DYB200I_OVERWRITE};
-    throw_status(dev, dyb200_affine_transform_bwd(cxs, (int)xs.size(), &cfx, &cd, i, &cdx, &fresh, nullptr, dev.ctx));
+    throw_status(dev, dyb200i_affine_transform_bwd(cxs, (int)xs.size(), &cfx, &cd, i, &cdx, nullptr, nullptr, 1, dev.ctx));
   };
   input_grad(xs2, tlog, tdlog, 2, tdth);
   tanh_node.backward_dev_impl(dev, {&tpre}, tth, tdth, 0, tdpre);
