@@ -73,10 +73,12 @@ __device__ __forceinline__ float4 piece_fma(float4 a, float4 b, float4 c) {
   return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z), __fmaf_rn(a.w, b.w, c.w));
 }
 // The plain epilogues on columns [c, c_hi) of a tile in shared memory, STEP apart, a piece V (4 rows or one) per thread and column;
-// dst, mask and bias are those of the thread's first row, in column 0 of the tile.
+// dst, mask and bias are those of the thread's first row, in column 0 of the tile; a thread whose rows are not there (no columns: c >= c_hi) reads none of them -
+// its bias would be one value short of a whole piece, or beyond the last.
 template <class V, int STEP>
 __device__ __forceinline__ void write_pieces(int mode, const float* tile, const float* old, float* dst, size_t ldc, const float* mask,
                                              size_t mstep, const float* bias, uint32_t c, uint32_t c_hi) {
+  if (c >= c_hi) return;
   auto at = [](const float* p) { return *reinterpret_cast<const V*>(p); };
   dst += ldc * c;
   tile += (size_t)c * BM; old += (size_t)c * BM;

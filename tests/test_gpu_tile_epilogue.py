@@ -24,3 +24,26 @@ def test_epilogue_of_a_tile(K, M, N, ldc, add):
     bound = 2.0 ** -20 * (b.double().abs() @ a.double().abs()) + 2.0 ** -23 * want[:, :M].abs()
     assert ((c.double()[:, :M] - want[:, :M]).abs() <= bound).all()
     assert torch.equal(c.double()[:, M:], want[:, M:])   # the rows past M stay
+
+
+@pytest.mark.parametrize("M", [260, 259, 388, 1000])
+@pytest.mark.parametrize("N,K", [(130, 160), (130, 1050), (130, 2080), (2500, 96)])   # a tile per CTA, its K splits in clusters, the persistent kernel
+@pytest.mark.parametrize("off", [0, 1])
+def test_bias_of_ragged_rows(M, N, K, off):
+    """y = b + W x with rows that end inside a tile, b on 16 bytes and off them, K splits in clusters and through memory."""
+    import torch
+    import gpu_util as g
+    ctx = g.ctx()
+    torch.manual_seed(K + M)
+    w, x = torch.randn(K, M, device="cuda"), torch.randn(N, K, device="cuda")
+    b = torch.randn(M + off, device="cuda")[off:]
+    want, sums = b.double() + x.double() @ w.double(), x.double().abs() @ w.double().abs()
+    for clusters in (True, False):
+        y = torch.full((N, M), 7.0, device="cuda")
+        try:
+            ctx.cluster_splitk(clusters)
+            ctx.fwd("affine_transform", [g.T(b, [M], 1), g.T(w, [M, K], 1), g.T(x, [K], N)], g.T(y, [M], N))
+        finally:
+            ctx.cluster_splitk(True)
+        assert ctx.device_errors() == 0
+        assert ((y.double() - want).abs() <= 2.0 ** -20 * sums + 2.0 ** -23 * want.abs()).all()   # (the bound above)
