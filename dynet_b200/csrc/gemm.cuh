@@ -196,7 +196,7 @@ int dyb200_tc_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, bool k_is_fas
                    const float* mask, uint32_t mask_ld, int mask_full, PackedOp* out, PackJobs* batch = nullptr);
 // Same for a parameter matrix: served from the parameter cache when it is on.
 int dyb200_tc_param(dyb200_ctx* ctx, const float* src, uint32_t ld, bool k_is_fast, uint32_t rows, uint32_t K, PackedOp* out,
-                    PackJobs* batch = nullptr);   // (batch: the caller launches it whatever happens afterwards)
+                    PackJobs* batch = nullptr);   // (batch: a caller that cannot launch it increments ctx->param_version)
 // A gate weight matrix (rows = 4H, element (r, k) at src[r + ld * k]) with its rows interleaved for EPI_LSTM_CELL.
 int dyb200_tc_param_gates(dyb200_ctx* ctx, const float* src, uint32_t ld, uint32_t rows, uint32_t K, PackedOp* out);
 // Number of K splits dyb200_tc_gemm_packed will use for this shape (1 = the epilogue runs in the MMA kernel).

@@ -1316,7 +1316,7 @@ int gates_f16_pack(dyb200_ctx* ctx, const float* Wx, const float* Wh, uint32_t I
 }
 
 // Returns the cached packed form of a parameter matrix, packing it first if it is new or stale (3xTF32 planes: as jobs of `queue` if there is
-// one, which the caller then launches whatever happens: the entry counts as packed).
+// one; the entry then counts as packed, and a caller that does not launch the queue, or fails to, makes the cache stale).
 // (k_is_fast = kLayoutF16 + F16_LINE or F16_ELEM: fp16 planes of the matrix as it lies, its scale words behind the hi plane)
 int cached_param_pack(dyb200_ctx* ctx, const float* src, uint32_t ld, int k_is_fast, uint32_t rows, uint32_t K, uint32_t pitch,
                       float** hi, float** lo, const float* src2 = nullptr, uint32_t rows2 = 0, PackJobs* queue = nullptr) {
@@ -2016,7 +2016,7 @@ int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const Ge
     A[0] = dyb200_f16_op(ja, a_mn); B[0] = dyb200_f16_op(jb, b_mn);
     return dyb200_tc_gemm_packed(ctx, M, N, 1, A, B, epi);
   }
-  PackJobs batch;   // all operands that need packing go out in one launch, also when a later one fails (a parameter's planes count as packed)
+  PackJobs batch;   // all operands that need packing go out in one launch
   dyb200_tc_pack_begin(&batch);
   int rcp = DYB200_OK;
   for (int p = 0; p < npairs && !rcp; ++p) {
@@ -2043,8 +2043,11 @@ int dyb200_gemm_tc(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, const Ge
       rc = dyb200_tc_pack(ctx, g.B, g.ldb, g.transB == 0, N, g.K, g.maskB, g.mask_ld, g.mask_full, &B[p], &batch);
     }
   }
-  const int rcf = dyb200_tc_pack_flush(ctx, &batch);
-  if (rcp || rcf) return rcp ? rcp : rcf;
+  if (!rcp) rcp = dyb200_tc_pack_flush(ctx, &batch);
+  if (rcp) {   // (planes of a parameter that were queued count as packed, and were not: nothing that is cached does any more)
+    ctx->param_version++;
+    return rcp;
+  }
   return dyb200_tc_gemm_packed(ctx, M, N, npairs, A, B, epi);
 }
 
