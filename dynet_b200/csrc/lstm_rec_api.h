@@ -60,4 +60,10 @@ struct dyb200i_ordinary_launches {
   ~dyb200i_ordinary_launches() { dyb200i_dependent_launch(ctx, was); }
   dyb200i_ordinary_launches(const dyb200i_ordinary_launches&) = delete;
 };
+/* The same for a driver with a second context of its own beside the caller's: what is in force on the caller's - its choice, or else `dependent` - holds for both. */
+struct dyb200i_both_launches {
+  dyb200i_ordinary_launches first, second;
+  dyb200i_both_launches(dyb200_ctx* caller, dyb200_ctx* own, int dependent)
+      : first(caller, dependent), second(own, dyb200i_dependent_launch(caller, -1)) {}
+};
 #endif

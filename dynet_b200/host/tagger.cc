@@ -379,9 +379,7 @@ int guarded(Tagger* m, const PassArgs& a) {
   constexpr uint64_t kDependentTokens = 6144;
   uint64_t tokens = 0;
   for (uint32_t s = 0; a.lens && s < a.S; ++s) tokens += a.lens[s];
-  const int dependent = tokens <= kDependentTokens;
-  const dyb200i_ordinary_launches first(m->dev.ctx, dependent);
-  const dyb200i_ordinary_launches second(m->dev2.ctx, dependent && dyb200i_dependent_launch(m->dev.ctx, -1));   // (the caller's choice holds for both)
+  const dyb200i_both_launches launches(m->dev.ctx, m->dev2.ctx, tokens <= kDependentTokens);
   try {
     tagger_pass(*m, a);
     return DYB200_OK;
