@@ -19,6 +19,7 @@
 // tok0[s] + t.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cstring>
 #include <string>
@@ -372,14 +373,18 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
 }
 
 int guarded(Tagger* m, const PassArgs& a) {
-  // A pass is 50 launches one behind the other on two streams.  While their kernels take a few microseconds each, dependent launches save the gaps
-  // between them; longer ones keep CTAs that wait on SMs that the other direction, or another model, could use.  us, ordinary / dependent launches,
-  // one tagger of 256 units waited for, and a step of three on three streams: 520 tokens 500 / 446, 188 / 170; 1200 605 / 553, 235 / 229;
-  // 4000 794 / 749, 334 / 336; 8400 1004 / 968, 478 / 482; 13 400 1196 / 1135, 667 / 692.
-  constexpr uint64_t kDependentTokens = 6144;
+  // A pass is 50 launches one behind the other on two streams.  Dependent launches save the gaps between them, so that a pass by itself is faster with them at
+  // every size; where several models share the GPU, CTAs that wait hold SMs that another's kernels could use, the longer the longer the kernels are, which goes
+  // by tokens and units.  us, ordinary / dependent launches, one tagger waited for, and a step of three on three streams:
+  //   256 units   1200 tokens 530 / 480, 199 / 187   3800 768 / 724, 306 / 307   6300 949 / 881, 383 / 393   8400 1007 / 966, 455 / 471   13 400 1201 / 1145, 670 / 691
+  //   128 units   1200 tokens 454 / 401, 171 / 159   6300 819 / 748, 286 / 284   8400 855 / 790, 321 / 313   13 400 996 / 917, 399 / 404   26 900 1269 / 1186, 627 / 641
+  //    64 units   1200 tokens 427 / 372, 173 / 158   8400 781 / 717, 272 / 252   13 400 898 / 825, 342 / 304   26 900 1113 / 1057, 472 / 438
+  // The line: 6144 tokens of 256 units, where three lose about a third of what one gains, and past which it is more than half; fewer units, more tokens, but no more
+  // than 64 units' (below, the tag layer and the lookups, which know no units, are most of a pass).
+  constexpr uint64_t kDependentWork = 6144 * 256;
   uint64_t tokens = 0;
   for (uint32_t s = 0; a.lens && s < a.S; ++s) tokens += a.lens[s];
-  const dyb200i_both_launches launches(m->dev.ctx, m->dev2.ctx, tokens <= kDependentTokens);
+  const dyb200i_both_launches launches(m->dev.ctx, m->dev2.ctx, tokens * std::max(m->c.H, 64u) <= kDependentWork);
   try {
     tagger_pass(*m, a);
     return DYB200_OK;
