@@ -1730,7 +1730,7 @@ int dyb200_tc_gemm_packed(dyb200_ctx* ctx, uint32_t M, uint32_t N, int npairs, c
   // Split K when the output has too few tiles to occupy the SMs (e.g. dx = W^T dgate: 16-32 tiles, K = 4096).
   uint32_t S = force_splits ? (force_splits < kb_total ? force_splits : kb_total) : dyb200_tc_splits(ctx, M, N, kb_total);
   uint32_t kb_per_split = (kb_total + S - 1) / S;
-  S = (kb_total + kb_per_split - 1) / kb_per_split;
+  S = k_splits_used(kb0, kb1, (kb_total + kb_per_split - 1) / kb_per_split);
   GemmEpilogue kepi = epi;
   float* part = nullptr;
   // K splits as one thread-block cluster per tile (partial tiles meet in distributed shared memory) when every cluster

@@ -39,13 +39,32 @@ constexpr uint32_t kEpiWarps = 8;
 
 // The k-blocks of K split z of S: [b0, b0 + n0) of pair 0, then [b1, b1 + n1) of pair 1 (each pair cut into S equal shares).
 struct KSplit { uint32_t b0, n0, b1, n1; };
-__device__ __forceinline__ KSplit k_split(uint32_t kb0, uint32_t kb1, uint32_t z, uint32_t S) {
+__host__ __device__ constexpr uint32_t k_min(uint32_t a, uint32_t b) { return a < b ? a : b; }
+__host__ __device__ constexpr KSplit k_split(uint32_t kb0, uint32_t kb1, uint32_t z, uint32_t S) {
   const uint32_t per0 = (kb0 + S - 1) / S, per1 = (kb1 + S - 1) / S;
-  KSplit k;
-  k.b0 = min(z * per0, kb0); k.n0 = min(k.b0 + per0, kb0) - k.b0;
-  k.b1 = min(z * per1, kb1); k.n1 = min(k.b1 + per1, kb1) - k.b1;
-  return k;
+  const uint32_t b0 = k_min(z * per0, kb0), b1 = k_min(z * per1, kb1);
+  return KSplit{b0, k_min(b0 + per0, kb0) - b0, b1, k_min(b1 + per1, kb1) - b1};
 }
+// How many of S splits have any k-block: cut into that many, each has the k-blocks it has among S.  (A split without one would be a CTA that adds
+// to a destination it has never read: what a tile adds to is fetched under its MMAs.)
+constexpr uint32_t k_splits_used(uint32_t kb0, uint32_t kb1, uint32_t S) {
+  const uint32_t per0 = (kb0 + S - 1) / S, per1 = (kb1 + S - 1) / S, s0 = per0 ? (kb0 + per0 - 1) / per0 : 0, s1 = per1 ? (kb1 + per1 - 1) / per1 : 0;
+  return s0 > s1 ? s0 : s1;
+}
+constexpr bool k_splits_hold(uint32_t most_kb, uint32_t most_S) {
+  for (uint32_t kb0 = 1; kb0 <= most_kb; ++kb0)
+    for (uint32_t kb1 = 0; kb1 <= most_kb; ++kb1)
+      for (uint32_t S = 1; S <= most_S; ++S) {
+        const uint32_t used = k_splits_used(kb0, kb1, S);
+        for (uint32_t z = 0; z < S; ++z) {
+          const KSplit a = k_split(kb0, kb1, z, S), b = k_split(kb0, kb1, z, used);
+          const bool some = a.n0 + a.n1 > 0;
+          if (some != (z < used) || (some && (a.b0 != b.b0 || a.n0 != b.n0 || a.b1 != b.b1 || a.n1 != b.n1))) return false;
+        }
+      }
+  return true;
+}
+static_assert(k_splits_hold(20, 9), "K splits without a k-block");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

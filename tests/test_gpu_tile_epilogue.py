@@ -47,3 +47,33 @@ def test_bias_of_ragged_rows(M, N, K, off):
             ctx.cluster_splitk(True)
         assert ctx.device_errors() == 0
         assert ((y.double() - want).abs() <= 2.0 ** -20 * sums + 2.0 ** -23 * want.abs()).all()   # (the bound above)
+
+
+@pytest.mark.parametrize("I,H,B", [(300, 300, 100), (160, 300, 70), (90, 290, 40), (330, 100, 64)])
+def test_two_products_in_splits_of_unlike_shares(I, H, B):
+    """Wx x + Wh h where the shares of the two reductions end before the number of K splits does (10 + 10 k-blocks in seven): no split is empty."""
+    import torch
+    import gpu_util as g
+    from dynet_b200 import capi
+    ctx = g.ctx()
+    torch.manual_seed(I + H)
+    x, h, c = torch.randn(B, I, device="cuda"), torch.randn(B, H, device="cuda") * 0.5, torch.randn(B, H, device="cuda")
+    wx, wh, b = torch.randn(I, 4 * H, device="cuda") * 0.1, torch.randn(H, 4 * H, device="cuda") * 0.1, torch.randn(4 * H, device="cuda")
+    z = (x.double() @ wx.double() + h.double() @ wh.double() + b.double()).view(B, 4, H)
+    z[:, 1] += 1.0
+    want = torch.cat([torch.sigmoid(z[:, :3]), torch.tanh(z[:, 3:])], 1).view(B, 4 * H)
+    sums = x.double().abs() @ wx.double().abs() + h.double().abs() @ wh.double().abs() + b.double().abs()
+    got = []
+    for clusters in (True, False):
+        gates, c1, h1 = torch.empty(B, 4 * H, device="cuda"), torch.empty(B, H, device="cuda"), torch.empty(B, H, device="cuda")
+        try:
+            ctx.cluster_splitk(clusters)
+            ctx.lstm_fwd_fused(g.T(x, [I], B), g.T(h, [H], B), g.T(c, [H], B), g.T(wx, [4 * H, I], 1), g.T(wh, [4 * H, H], 1), g.T(b, [4 * H], 1), None, None,
+                               capi.LstmGatesAttrs(0, 0.0, 1.0), g.T(gates, [4 * H], B), g.T(c1, [H], B), g.T(h1, [H], B))
+        finally:
+            ctx.cluster_splitk(True)
+        assert ctx.device_errors() == 0
+        # the bound above through a function of slope at most one, and a few ulp of values below one for the function itself
+        assert ((gates.double() - want).abs() <= 2.0 ** -20 * sums + 2.0 ** -21).all()
+        got.append((gates, c1, h1))
+    assert all(torch.equal(p, q) for p, q in zip(*got))
