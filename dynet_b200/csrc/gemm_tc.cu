@@ -1629,7 +1629,7 @@ int dyb200_tc_param2(dyb200_ctx* ctx, const float* src, uint32_t rows, const flo
 // One-tile products start under the kernel before them (see dyb_launch): 0.7 us of barriers, TMEM and descriptors, and the launch itself.  One
 // layer of 256 units on 32 sequences, forward and backward: 227.5 -> 222.6 us; steps of models on several streams are the same within the
 // noise; the persistent kernel so launched gained nothing and is not.  (A CTA that waits holds TMEM: no kernel that allocates any
-// fits beside its shared memory, so none before it in the stream can be waiting for what it holds.)
+// fits beside it, kTmemSmem sees to that, so none can be waiting for what it holds.)
 // The kernels by tile width and form.  Their limit on dynamic shared memory is raised when one is first asked for (function attributes are per
 // device, so the context remembers what it has set on its own; a limit loads its kernel, and a program needs a few of them).
 using TcKernel = void (*)(TmapPack, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, GemmEpilogue, uint32_t*);

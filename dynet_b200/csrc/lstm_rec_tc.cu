@@ -659,11 +659,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_bwd(const __grid_const
   }
 }
 
-uint32_t tc_smem(bool bwd, uint32_t H) {
+constexpr uint32_t tc_smem(bool bwd, uint32_t H) {
   const uint32_t NC = kTcCols, KB = (H + 63) / 64, C = (H + kTcUnits - 1) / kTcUnits;
   // (the partial sums' room also holds the row sums of dgates at the end, 512 bytes per cell warp)
-  return 1024 + kGroups * (bwd ? 2 * 2 * NC * 128 + 2 * C * NC * kTcUnits * 4 : 2 * 2 * KB * 2 * NC * 64 + 3 * NC * 512);
+  const uint32_t need = 1024 + kGroups * (bwd ? 2 * 2 * NC * 128 + 2 * C * NC * kTcUnits * 4 : 2 * 2 * KB * 2 * NC * 64 + 3 * NC * 512);
+  return need > kTmemSmem ? need : kTmemSmem;
 }
+static_assert(tc_smem(true, 1) >= kTmemSmem && tc_smem(false, 1) >= kTmemSmem, "a recurrence that fits beside a waiting product");
 
 typedef void (*TcFwd)(RecFwd);
 typedef void (*TcBwd)(RecBwd);

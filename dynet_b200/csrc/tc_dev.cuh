@@ -28,7 +28,12 @@ constexpr int STAGE_BYTES = 4 * TILE_BYTES;      // A_hi, A_lo, B_hi, B_lo
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;   // + slack to align the ring to 1 KiB
 constexpr int kThreads = 320;              // TMA warp, MMA warp, 8 epilogue warps
 constexpr uint32_t kWaitLimit = 1u << 20;
-constexpr uint32_t kTmemCols = 256;       // two 128-column accumulators, used alternately       // two 128-column accumulators, used alternately
+constexpr uint32_t kTmemCols = 256;       // two 128-column accumulators, used alternately
+// The least dynamic shared memory of a kernel that allocates TMEM: too much to fit on an SM beside a one-tile product (228 KB, of which each CTA reserves one).  A
+// product that starts under the kernel before it holds TMEM while it waits; a CTA of another kernel beside it could wait for that TMEM, and a neighbour that its own
+// cluster or stream needs for that CTA.  (Registers keep them apart as well, as the kernels are compiled now.)
+constexpr uint32_t kTmemSmem = 34 * 1024;
+static_assert(SMEM_BYTES + kTmemSmem + 2 * 1024 > 228 * 1024, "a kernel with TMEM fits beside a one-tile product");
 // k-blocks accumulated in TMEM before the sum moves to registers.  Measured against a float64 product (randn operands,
 // worst element / rms of the result): one unbroken chain 1.9e-5 at K = 2048 and 1.6e-4 at K = 17920 (biased towards
 // zero); chains of 8 k-blocks 8.7e-6 at both, against 2.6e-6 .. 9.3e-6 for cuBLAS SGEMM.  Each flush costs about
