@@ -357,8 +357,8 @@ __device__ __forceinline__ void add4(float4& a, const float4& b) { a.x += b.x; a
 // earlier chunk begins from zero and goes to head[chunk]; a run that continues goes to tail[chunk].
 // A chunk is a trip to memory for its ids, one for all its gradient rows and table rows together (copied to shared memory, every lane its
 // own four columns) and a chain of adds: requested 8 at a time into registers it was four trips, and an unrolled body that a
-// short call fetches for longer than its data.  us, before / after: 320 ids of 128 columns 9.7 / 6.5, 1050 of 200 12.2 / 7.5, 13 400 of 128
-// 13.0 / 7.0, 107 000 of 128 24.6 / 20.9; 17 920 of 512, which is memory, 16.0 / 17.5.
+// short call fetches for longer than its data.  Six chunks fit an SM at a time, though, where registers hold sixteen warps: with more chunks than that, rounds of them cost
+// more than the two extra trips do (k_chunk_add_rows, and staged_chunks for the line).
 constexpr unsigned kAddCtas = 6;   // CTAs (of one warp) on an SM: 32 KB each
 __global__ void __launch_bounds__(32) k_chunk_add(const float* __restrict__ g, float* __restrict__ all_grads, uint32_t E,
                                                  const uint32_t* __restrict__ pos_sorted, const uint32_t* __restrict__ id_at,
@@ -416,6 +416,77 @@ __global__ void __launch_bounds__(32) k_chunk_add(const float* __restrict__ g, f
       else st4(all_grads + (size_t)cur * E + col, acc);              // whole run
     }
   }
+}
+// The same with rows in registers, eight positions at a time: a warp per (chunk, slice), sixteen on an SM.
+__global__ void __launch_bounds__(256, 2) k_chunk_add_rows(const float* __restrict__ g, float* __restrict__ all_grads, uint32_t E,
+                                                  const uint32_t* __restrict__ pos_sorted, const uint32_t* __restrict__ id_at,
+                                                  uint32_t n, uint32_t slices, float* __restrict__ head, float* __restrict__ tail) {
+  dyb_grid_dep_sync();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t nchunks = (n + kChunk - 1) / kChunk;
+  const size_t work = (size_t)nchunks * slices;
+  for (size_t w = (size_t)blockIdx.x * 8 + warp; w < work; w += (size_t)gridDim.x * 8) {
+    const uint32_t c = (uint32_t)(w / slices), sl = (uint32_t)(w % slices);
+    const uint32_t k0 = c * kChunk, k1 = min(n, k0 + kChunk);
+    const uint32_t col = sl * 128 + lane * 4;
+    const bool live = col < E;   // lanes past the row end still take part in the shuffles
+    const uint32_t my_id = k0 + lane < k1 ? id_at[k0 + lane] : 0xffffffffu;
+    const uint32_t my_pos = k0 + lane < k1 ? pos_sorted[k0 + lane] : 0;
+    uint32_t cur = __shfl_sync(0xffffffffu, my_id, 0);
+    bool started_before = k0 > 0 && id_at[k0 - 1] == cur;
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 acc = (started_before || !live) ? zero4 : ld4(all_grads + (size_t)cur * E + col);
+    float* hslot = head + ((size_t)c * slices + sl) * 128 + lane * 4;
+    float* tslot = tail + ((size_t)c * slices + sl) * 128 + lane * 4;
+    for (uint32_t j0 = 0; j0 < k1 - k0; j0 += 8) {
+      // the gradient rows of the next 8 positions and the table rows that runs start from are requested together; the adds stay in order
+      float4 rows[8], start[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t pos = __shfl_sync(0xffffffffu, my_pos, (j0 + u) & 31), id = __shfl_sync(0xffffffffu, my_id, (j0 + u) & 31);
+        const uint32_t before = __shfl_sync(0xffffffffu, my_id, (j0 + u - 1) & 31);
+        const bool in = live && j0 + u < k1 - k0;
+        rows[u] = in ? ld4_stream(g + (size_t)pos * E + col) : zero4;
+        start[u] = in && j0 + u > 0 && id != before ? ld4(all_grads + (size_t)id * E + col) : zero4;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t id = __shfl_sync(0xffffffffu, my_id, (j0 + u) & 31);
+        if (j0 + u < k1 - k0) {
+          if (id != cur) {   // the run of `cur` ends inside this chunk
+            if (live) {
+              if (started_before) st4(hslot, acc);
+              else st4(all_grads + (size_t)cur * E + col, acc);
+            }
+            cur = id;
+            started_before = false;
+            acc = start[u];
+          }
+          add4(acc, rows[u]);
+        }
+      }
+    }
+    const bool continues = k1 < n && id_at[k1] == cur;
+    if (live) {
+      if (started_before) st4(hslot, acc);                           // middle or last piece
+      else if (continues) st4(tslot, acc);                           // first piece (holds the row)
+      else st4(all_grads + (size_t)cur * E + col, acc);              // whole run
+    }
+  }
+}
+// Whether `work` pairs of chunk and slice go by shared memory.  us (cold caches), registers / staged, by ids of `columns` columns: Zipf ids, and ids without repeats
+//   up to six chunks an SM, one round:         4096 x 128 14.5 / 8.4, 14.6 / 8.6    13 000 x 256 14.6 / 8.9, 15.3 / 11.0
+//   to sixteen, two and three rounds for one:  9000 x 512 14.9 / 13.2, 15.6 / 16.3  17 920 x 512 16.1 / 17.8, 18.0 / 23.6   (gradients still in L2: 11.0 / 11.3 and 12.7 / 14.6)
+//   to twenty-four, up to four for two:        107 000 x 128 26.0 / 21.9, 27.7 / 25.7   26 000 x 512 26.5 / 22.1, 30.6 / 30.7
+//   more:                                      36 000 x 512 27.8 / 31.8, 32.4 / 42.9    107 000 x 512 71.6 / 74.8, 82.9 / 90.4
+static bool staged_chunks(const dyb200_ctx* ctx, size_t work) {
+  const size_t sms = (size_t)ctx->sm_count;
+  return work <= kAddCtas * sms || (work > 16 * sms && work <= 24 * sms);
+}
+static void launch_chunk_add(dyb200_ctx* ctx, size_t work, const float* g, float* all_grads, uint32_t E, const uint32_t* pos_sorted, const uint32_t* id_at, uint32_t n,
+                             uint32_t slices, float* head, float* tail) {
+  if (staged_chunks(ctx, work)) dyb_launch(k_chunk_add, stream_grid(ctx, work, 1, kAddCtas), 32, 0, ctx, g, all_grads, E, pos_sorted, id_at, n, slices, head, tail);
+  else dyb_launch(k_chunk_add_rows, stream_grid(ctx, work, 8), 256, 0, ctx, g, all_grads, E, pos_sorted, id_at, n, slices, head, tail);
 }
 // Pass B: the chunk in which a multi-chunk run starts adds the later pieces in chunk order and writes the row.  A frequent id runs over hundreds of chunks
 // (the most frequent word of a 107 k-token batch: ~500), which one warp adds 16 at a time, a round trip to memory each: runs of more than kCombineLong pieces are
@@ -524,7 +595,7 @@ static int scatter_run_chunked(dyb200_ctx* ctx, unsigned n, const unsigned* ids_
     dyb_launch(k_merge_runs, (n + 255) / 256, 256, 0, ctx, (const uint32_t*)pos_all, (const uint32_t*)id_all, n, pos_m, id_m);
     DYB_LAUNCHED(ctx);
     const size_t work = (size_t)((n + kChunk - 1) / kChunk) * slices;
-    dyb_launch(k_chunk_add, stream_grid(ctx, work, 1, kAddCtas), 32, 0, ctx, g, all_grads, E, pos_m, id_m, n, slices, head, tail);
+    launch_chunk_add(ctx, work, g, all_grads, E, pos_m, id_m, n, slices, head, tail);
     DYB_LAUNCHED(ctx);
     dyb_launch(k_chunk_combine, stream_grid(ctx, work, 8), 256, 0, ctx, all_grads, E, id_m, n, slices, head, tail);
     DYB_LAUNCHED(ctx);
@@ -537,7 +608,7 @@ static int scatter_run_chunked(dyb200_ctx* ctx, unsigned n, const unsigned* ids_
     uint32_t* pos_sorted = pos_all + base;
     uint32_t* id_at = id_all + base;
     size_t work = (size_t)nchunks * slices;
-    dyb_launch(k_chunk_add, stream_grid(ctx, work, 1, kAddCtas), 32, 0, ctx, g, all_grads, E, pos_sorted, id_at, np, slices, head, tail);
+    launch_chunk_add(ctx, work, g, all_grads, E, pos_sorted, id_at, np, slices, head, tail);
     DYB_LAUNCHED(ctx);
     dyb_launch(k_chunk_combine, stream_grid(ctx, work, 8), 256, 0, ctx, all_grads, E, id_at, np, slices, head, tail);
     DYB_LAUNCHED(ctx);

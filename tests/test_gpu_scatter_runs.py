@@ -30,3 +30,25 @@ def test_sums(E, kind):
         ctx.lookup_accumulate_grads([], ids32.data_ptr(), grad.data_ptr(), table.data_ptr(), E, V, n=n)
         assert torch.equal(table, want), "n = %d: %d of %d values" % (n, int((table != want).sum()), want.numel())
     assert ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("chunks_per_sm", [6, 16, 24])
+@pytest.mark.parametrize("E,V", [(128, 3000), (200, 400), (128, 0)])   # (V = 0: no repeats)
+def test_sums_where_the_form_changes(chunks_per_sm, E, V):
+    """Both sides of the lines up to which chunks go by shared memory: whole chunks and one id more, on (chunk, slice) pairs of the whole GPU."""
+    import torch
+    import gpu_util as g
+    ctx = g.ctx()
+    slices = (E + 127) // 128
+    at = 32 * (chunks_per_sm * torch.cuda.get_device_properties(0).multi_processor_count // slices)
+    for n in (at, at + 1):
+        gen = torch.Generator("cuda").manual_seed(n)
+        rows = V or n
+        ids = torch.randint(0, rows, (n,), device="cuda", generator=gen) if V else torch.randperm(n, device="cuda", generator=gen)
+        grad = torch.randint(-2048, 2049, (n, E), device="cuda", generator=gen).float() / 1024
+        table = torch.randint(-2048, 2049, (rows, E), device="cuda", generator=gen).float() / 1024
+        want = table.double().index_add_(0, ids, grad.double()).float()
+        ids32 = ids.to(torch.int32)
+        ctx.lookup_accumulate_grads([], ids32.data_ptr(), grad.data_ptr(), table.data_ptr(), E, rows, n=n)
+        assert torch.equal(table, want)
+    assert ctx.device_errors() == 0
