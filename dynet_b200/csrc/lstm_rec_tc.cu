@@ -120,7 +120,7 @@ __device__ __forceinline__ void tc_kstep(uint32_t wide, uint32_t narrow, uint32_
 // KB = ceil(H / 64).
 // TMEM: each group's accumulators (3 NC columns: A_hi B_hi, A_hi B_lo, A_lo B_hi - the last apart, so that the chain of one waits on
 // the other's MMAs, not on its own), Wh_hi and Wh_lo (32 KB columns each).
-template <uint32_t kH>
+template <uint32_t kH, bool kCopies = true>
 __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_constant__ RecFwd a) {
   constexpr uint32_t NC = kTcCols, kBlock = 2 * NC * 64;   // bytes of a CTA's part of h
   extern __shared__ unsigned char smem_raw[];
@@ -279,11 +279,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     float cst[kCells], mk[kCells];
     // Wx x + b of this thread's cells, of this step and of the next, asked for a whole step before its use.  (In registers the wait for it fell wherever the
     // compiler's few scoreboards put it, before the cell pass of the step that asked: 256 units 1187 us forward, 1039 like this; 200 units, 600 sentences 250 against
-    // 230; 99 units, where rows start on any four bytes, 116 against 120.)
+    // 230; 99 units, 600 sentences 127 against 119.  Fewer than 64 units, whose steps are the shortest, keep the registers, kCopies off: 600 sentences, 8 units 95 against 101, 33
+    // 102 against 105, 56 100 against 104; 64 units 102 against 94.)
     float* const mine = ahead + gt0;
     const uint32_t pitch = kH ? kH : a.hn_pitch;
     uint32_t ho[kCells];                                   // where h of cell j goes in this CTA's block
+    float next[kCells][4];   // (without copies)
     auto fetch = [&](uint32_t to, uint32_t c0, uint32_t nact) {
+      if (!kCopies) {
+#pragma unroll
+        for (int j = 0; j < kCells; ++j) {   // (columns and units that are not there: another's)
+          const uint32_t i = i0 + 4 * j;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) next[j][q] = at(pg, c0 + base + (i < nact ? i : 0), 16 * H)[(size_t)q * H];
+        }
+        return;
+      }
       const uint32_t dst = smem_u32(mine) + to * (NC * 128 * 4);
 #pragma unroll
       for (int j = 0; j < kCells; ++j)
@@ -305,8 +316,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       unsigned char* hnext = hbuf + ((t & 1) ^ 1) * hbytes;
       const int ts = t ? t1 : t0, th = ts >> 1;
       const float f0 = __int_as_float((th + 127) << 23), f1 = __int_as_float((ts - th + 127) << 23);
-      const float* const pre = mine + (t & 1) * (NC * 128);
-      copies_done();
+      float pre[kCells][4];
+      if (kCopies) copies_done();
+      else
+#pragma unroll
+        for (int j = 0; j < kCells; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) pre[j][q] = next[j][q];
+      auto in = [&](int j, int q) { return kCopies ? mine[(t & 1) * (NC * 128) + (4 * j + q) * kGroupThreads] : pre[j][q]; };
       if (n1) fetch((t & 1) ^ 1, col1, n1);
       ok = ok && mbar_wait(&acc_full, t & 1);
       tc_after();
@@ -328,10 +345,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
 #pragma unroll
         for (int q = 0; q < 4; ++q) y[j][q] = exch[(i * 4 + q) * 32 + lane];
         if (i >= n) continue;                            // (the same for the whole warp)
-        y[j][0] = gate_sigmoid(y[j][0] + pre[4 * j * kGroupThreads]);
-        y[j][1] = gate_sigmoid(y[j][1] + pre[(4 * j + 1) * kGroupThreads] + a.fb);
-        y[j][2] = gate_sigmoid(y[j][2] + pre[(4 * j + 2) * kGroupThreads]);
-        y[j][3] = gate_tanh(y[j][3] + pre[(4 * j + 3) * kGroupThreads]);
+        y[j][0] = gate_sigmoid(y[j][0] + in(j, 0));
+        y[j][1] = gate_sigmoid(y[j][1] + in(j, 1) + a.fb);
+        y[j][2] = gate_sigmoid(y[j][2] + in(j, 2));
+        y[j][3] = gate_tanh(y[j][3] + in(j, 3));
         cst[j] = lstm_cell_c(y[j][0], y[j][3], y[j][1], cst[j]);
         hv[j] = lstm_cell_h(y[j][2], cst[j]);
         hm[j] = hv[j] * mk[j];
@@ -673,6 +690,7 @@ typedef void (*TcBwd)(RecBwd);
 // cell's 16 - 23 accesses are a base and immediates instead of a third of all instructions.  256 units, 4096 columns of up to 100 steps: 1039 against 951 us
 // forward, 1392 against 1194 backward; 64 and 128 units, 1400 columns: 108 -> 96 and 130 -> 106 with the copies, 142 -> 128 and 147 -> 135.
 TcFwd tc_fwd_kernel(uint32_t H, uint32_t pitch) {
+  if (H < 64) return k_rec_tc_fwd<0, false>;   // (see its inputs)
   if (pitch && pitch != H) return k_rec_tc_fwd<0>;
   switch (H) {
     case 64: return k_rec_tc_fwd<64>;
