@@ -586,15 +586,23 @@ int dyb200_gemm_narrow(dyb200_ctx* ctx, uint32_t M, uint32_t N, const GemmPair& 
   // other took longer than twice the partial products do (us: 32 x 256 x 520 11.3 / 5.7, x 13 400 27.2 / 20.6, x 107 000 80 / 66, the last with pieces of 32 KB and
   // addresses that walk; with 10 groups of 48 x 32 meeting is the faster one, 7.8 / 14.6 at 520).
   a.meet = a.groups > 2;
-  a.KC = a.meet ? up(4096 / (a.MT + a.NT), a.groups) : up(8192 / (a.MT + a.NT), 4 * a.groups);   // 16 or 32 KB a piece
   a.vec_a = p.lda % 4 == 0 && aligned16(p.A);
   a.vec_b = p.ldb % 4 == 0 && aligned16(p.B);
-  uint32_t gx = 2 * (uint32_t)ctx->sm_count / by;
-  if (gx < 1) gx = 1;
-  a.kspan = up((p.K + gx - 1) / gx, a.KC);
-  gx = (p.K + a.kspan - 1) / a.kspan;
+  uint32_t gx;
   void* part;
-  int rc = dyb200_scratch(ctx, (size_t)gx * (a.meet ? 1 : a.groups) * M * N * sizeof(float), &part);
+  auto cut = [&]() {
+    a.KC = a.meet ? up(4096 / (a.MT + a.NT), a.groups) : up(8192 / (a.MT + a.NT), 4 * a.groups);   // 16 or 32 KB a piece
+    gx = 2 * (uint32_t)ctx->sm_count / by;
+    if (gx < 1) gx = 1;
+    a.kspan = up((p.K + gx - 1) / gx, a.KC);
+    gx = (p.K + a.kspan - 1) / a.kspan;
+    return dyb200_scratch(ctx, (size_t)gx * (a.meet ? 1 : a.groups) * M * N * sizeof(float), &part);
+  };
+  int rc = cut();
+  if (rc == DYB200_ENOMEM && !a.meet) {   // (half as much, up to 10 MB, may still fit)
+    a.meet = 1;
+    rc = cut();
+  }
   if (rc) return rc;
   a.part = (float*)part;
   const size_t ring = (size_t)kStagesN * a.KC * (a.MT + a.NT), sums = a.meet ? (size_t)a.groups * a.MT * a.NT : 0;
