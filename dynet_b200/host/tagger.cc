@@ -11,7 +11,8 @@
 // nodes of the tag layer are batched over ALL tokens; their inputs, the hidden states of (sentence, position), sit in
 // the outputs of different LSTM steps and are gathered into one contiguous matrix by combine_tensors (exec.cc:298-361 ->
 // gpu::parallel_memcpy); the gradients go back through accumulate_tensors (exec.cc:363-411 -> gpu::parallel_accumulate).
-// This driver makes exactly those calls.  The pointer tables of the movers are built on the host per mini-batch and
+// This driver makes the same calls, but for the way back: there every target holds nothing yet and is met once, so that it is a
+// parallel_memcpy too.  The pointer tables of the movers are built on the host per mini-batch and
 // uploaded, as the executor does (exec.cc:346-356).
 //
 // Device layout: per direction the columns of all steps sit side by side in step order ("step-major"): column
@@ -322,7 +323,7 @@ void tagger_pass(Tagger& m, const PassArgs& a) {
   input_grad(xs1, tpre, tdpre, 2, tdhf);
   affine.backward_dev_impl(dev, xs1, tpre, tdpre, 3, gr2th);
   input_grad(xs1, tpre, tdpre, 4, tdhr);
-  // accumulate_tensors: the token-major gradients back into the steps' dE/dh.  Every column of dE/dh belongs to one token and holds nothing yet, so that it is a copy
+  // in place of accumulate_tensors: the token-major gradients back into the steps' dE/dh.  Every column of dE/dh belongs to one token and holds nothing yet, so that it is a copy
   // (16 bytes of traffic per value less: a clear, and reading what is added to).
   for (int dr = 0; dr < 2; ++dr) {
     if (m.time_movers) CU(cudaEventRecord(m.ev[4 + 2 * dr], st));
@@ -489,7 +490,7 @@ int dyb200h_tagger_side_stats(void* h, uint64_t* launches, uint32_t* error_flags
 }
 
 // Measurement hooks: with timing on, the four mover calls of a pass are bracketed by CUDA events; dyb200h_tagger_mover_ms
-// waits for the pass and returns {copy fwd, copy bwd direction, accumulate fwd, accumulate bwd direction} in ms, plus the host
+// waits for the pass and returns {states fwd, bwd direction, their gradients back fwd, bwd direction} in ms, plus the host
 // time spent building the schedule and the pointer tables of the last pass.
 int dyb200h_tagger_time_movers(void* h, int enable) { ((Tagger*)h)->time_movers = enable != 0; return DYB200_OK; }
 int dyb200h_tagger_mover_ms(void* h, float ms_out[4], double* host_schedule_ms) {

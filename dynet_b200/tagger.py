@@ -155,7 +155,7 @@ class Tagger:
         self._check(self.H.dyb200h_tagger_time_movers(self.h, int(enable)))
 
     def mover_ms(self):
-        """({copy fwd-direction, copy bwd-direction, accumulate fwd-direction, accumulate bwd-direction} in ms, host ms spent on the
+        """({states of the fwd-direction, of the bwd-direction, their gradients back, fwd-direction and bwd-direction: copies all} in ms, host ms spent on the
         schedule and pointer tables) of the last pass; waits for it."""
         ms, host = (C.c_float * 4)(), C.c_double(0)
         self._check(self.H.dyb200h_tagger_mover_ms(self.h, ms, C.byref(host)))
