@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
     // Wx x + b of this thread's cells, of this step and of the next, asked for a whole step before its use.  (In registers the wait for it fell wherever the
     // compiler's few scoreboards put it, before the cell pass of the step that asked: 256 units 1187 us forward, 1039 like this; 200 units, 600 sentences 250 against
     // 230; 99 units, 600 sentences 127 against 119.  Fewer than 64 units, whose steps are the shortest, keep the registers, kCopies off: 600 sentences, 8 units 95 against 101, 33
-    // 102 against 105, 56 100 against 104; 64 units 102 against 94.)
+    // 102 against 105, 56 100 against 104; 64 units 102 against 94.  160 steps of 600 columns, inputs out of L2: 8 units 237 against 254, 56 272 against 264.)
     float* const mine = ahead + gt0;
     const uint32_t pitch = kH ? kH : a.hn_pitch;
     uint32_t ho[kCells];                                   // where h of cell j goes in this CTA's block
@@ -316,14 +316,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
       unsigned char* hnext = hbuf + ((t & 1) ^ 1) * hbytes;
       const int ts = t ? t1 : t0, th = ts >> 1;
       const float f0 = __int_as_float((th + 127) << 23), f1 = __int_as_float((ts - th + 127) << 23);
-      float pre[kCells][4];
+      const float* const pre = mine + (t & 1) * (NC * 128);
+      float now[kCells][4];
       if (kCopies) copies_done();
       else
 #pragma unroll
         for (int j = 0; j < kCells; ++j)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) pre[j][q] = next[j][q];
-      auto in = [&](int j, int q) { return kCopies ? mine[(t & 1) * (NC * 128) + (4 * j + q) * kGroupThreads] : pre[j][q]; };
+          for (int q = 0; q < 4; ++q) now[j][q] = next[j][q];
       if (n1) fetch((t & 1) ^ 1, col1, n1);
       ok = ok && mbar_wait(&acc_full, t & 1);
       tc_after();
@@ -345,10 +345,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_rec_tc_fwd(const __grid_const
 #pragma unroll
         for (int q = 0; q < 4; ++q) y[j][q] = exch[(i * 4 + q) * 32 + lane];
         if (i >= n) continue;                            // (the same for the whole warp)
-        y[j][0] = gate_sigmoid(y[j][0] + in(j, 0));
-        y[j][1] = gate_sigmoid(y[j][1] + in(j, 1) + a.fb);
-        y[j][2] = gate_sigmoid(y[j][2] + in(j, 2));
-        y[j][3] = gate_tanh(y[j][3] + in(j, 3));
+        y[j][0] = gate_sigmoid(y[j][0] + (kCopies ? pre[4 * j * kGroupThreads] : now[j][0]));
+        y[j][1] = gate_sigmoid(y[j][1] + (kCopies ? pre[(4 * j + 1) * kGroupThreads] : now[j][1]) + a.fb);
+        y[j][2] = gate_sigmoid(y[j][2] + (kCopies ? pre[(4 * j + 2) * kGroupThreads] : now[j][2]));
+        y[j][3] = gate_tanh(y[j][3] + (kCopies ? pre[(4 * j + 3) * kGroupThreads] : now[j][3]));
         cst[j] = lstm_cell_c(y[j][0], y[j][3], y[j][1], cst[j]);
         hv[j] = lstm_cell_h(y[j][2], cst[j]);
         hm[j] = hv[j] * mk[j];
