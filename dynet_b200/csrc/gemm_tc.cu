@@ -190,7 +190,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__
   const uint32_t tmem_base = tmem_base_slot;
   // Barrier initialisation and the TMEM allocation above may overlap the previous kernel of the stream; nothing below
   // (TMA loads, c_prev prefetch, stores) starts before that kernel has completed.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (the scales of fp16 pairs go by __ldg, which an asm statement alone does not keep behind it)
+  dyb_grid_dep_wait();
 
   if (warp == 0) {
     if (elect_one()) {
